@@ -242,7 +242,7 @@ int qpam_head_logits(const qpam_ce_args* args, void* logits, int64_t ld, void* s
  *               (NULL: all hist_cols entries count); append != 0 stores the drawn id at history[row][hist_len]
  *               and increments hist_len
  *   next_ids    int64 [n];  stats optional float [n,4] = (max, kept mass, kept count, mass after top-k)
- *   workspace   qpam_sample_workspace_bytes(n, V) bytes (0 while a row fits in shared memory, V <= ~56k) */
+ *   workspace   qpam_sample_workspace_bytes(n, V) bytes (0 while one bit per token fits in shared memory, V <= 1.3 M) */
 size_t qpam_sample_workspace_bytes(int32_t n, int32_t V);
 int qpam_sample_logits(const void* logits, int32_t io_dtype, int32_t n, int32_t V, int64_t ld_logits,
                        float temperature, int32_t top_k, float top_p, float repetition_penalty,

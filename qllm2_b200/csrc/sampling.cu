@@ -6,21 +6,33 @@
 //   top-k : drop x < (k-th largest x)                            (ties with the k-th value stay)
 //   top-p : in descending order, drop a token when the probability mass BEFORE it is >= top_p
 //   draw from softmax of what is left
-// The row lives in shared memory (V <= ~56k floats) or in a caller workspace; the k-th largest value and the
-// nucleus threshold are found without sorting: the k-th largest value by radix selection over order-preserving
-// integer keys (4 passes of 8 bits over count histograms), the nucleus threshold by a 4-way search over the bit
-// patterns of the unnormalised probabilities (each probe a deterministic block reduction); the draw is the inverse
-// CDF in vocabulary order of a uniform number the caller supplies.  Nothing depends on the order of atomics, so the
-// same inputs give the same token on every run.  Tokens that tie with the nucleus threshold are all kept (a sort would keep an arbitrary
-// subset of them).
+// The draw is the inverse CDF in vocabulary order of a uniform number the caller supplies.  Nothing depends on the
+// order of atomics, so the same inputs give the same token on every run.  Tokens that tie with the nucleus threshold are
+// all kept (a sort would keep an arbitrary subset of them).
+//
+// What bounds it: the row is 100 KB (bf16, V = 50 k) and the 256 rows of a full engine are 26 MB, 4 us of HBM, so the
+// work is the number of passes over the row and the block-wide steps between them.  A row is never copied: every pass
+// streams it again with 16-byte loads (L1 / L2 hits after the first), which leaves room for two CTAs per SM, and the
+// tokens of the penalty are one bit each in shared memory.
+//   small top-k   pass 1 takes every thread's largest value; the k-th largest of those is a lower bound of the k-th
+//                 largest of the row, so pass 2 collects the few values at or above it (about k + k^2 / threads) and
+//                 everything after that works on that list: ranks by counting, no search.
+//   otherwise     counts or probability mass over 2048 bins LINEAR in x (leading bits of the float pattern put most of a
+//                 row into a dozen bins, whose atomics serialise), the bin in which the k-th value / the nucleus closes,
+//                 and the exact threshold from the elements of that bin.  Masses are accumulated in fixed point: the
+//                 sums do not depend on the order of the atomics.
+// 256 rows x 50261 bf16 logits, top-k 50 + top-p 0.9 + penalty: 34.8 us a call; 128.9 us for the version that kept
+// the row as floats in shared memory (one CTA per SM, two waves) and searched it by radix passes.
 #include "common.cuh"
 
 namespace qpam {
 namespace {
 
-constexpr int SAMPLE_THREADS = 1024;
-constexpr int SAMPLE_SMEM_EXTRA = 12288;  // histograms, scan scratch, scalars, compact list of the top-k survivors
-constexpr int SAMPLE_COMPACT = 1024;       // survivors of top-k that the later stages handle one per thread
+constexpr int SAMPLE_LIST = 1024;            // values that the list steps can hold
+constexpr int SAMPLE_LIST_TOP_K = 384;       // top-k up to which the list is expected to fit (512 threads: ~710 values)
+constexpr int SAMPLE_BINS = 2048;
+constexpr float SAMPLE_BINS_PER_UNIT = 64.f;  // bins reach 32 units below the maximum (e^-32 of its mass)
+constexpr size_t SAMPLE_SMEM_BITMAP = 160 * 1024;
 
 struct SampleParams {
   const void* logits;
@@ -32,8 +44,9 @@ struct SampleParams {
   const float* uniforms;
   int64_t* next_ids;
   float* stats;
-  float* work;
-  int32_t n, V, n_hist_rows, hist_cols, top_k, append, row_in_smem;
+  uint32_t* bitmaps;      // [n][words] in the workspace when a bitmap does not fit in shared memory
+  int32_t n, V, n_hist_rows, hist_cols, top_k, append, bitmap_words;
+  int32_t mass_half;      // masses are integers of 2 * mass_half bits; V sums of one half fit 32 bits
   float inv_temperature, top_p, penalty;
 };
 
@@ -41,75 +54,186 @@ __device__ __forceinline__ uint32_t order_key(float x) {
   const uint32_t u = __float_as_uint(x);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-
-// Histogram update of a whole warp (every lane calls; bin < 0 = this lane adds nothing).  Lanes that hit the same
-// bin are combined before the shared-memory atomic, so a row whose keys share their leading bits (the usual case
-// at the first radix level) does not serialise 32 ways on one address.
-__device__ __forceinline__ void warp_hist_count(uint32_t* hist, int bin) {
-  const unsigned peers = __match_any_sync(0xffffffffu, bin);
-  if (bin >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&hist[bin], (uint32_t)__popc(peers));
+__device__ __forceinline__ float key_value(uint32_t k) {
+  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
 struct Scratch {
-  uint32_t count[256];
-  float mass[256];
+  union {
+    uint32_t bins[3][SAMPLE_BINS];     // counts | low and high half of the masses
+    struct {
+      float e[SAMPLE_LIST];            // survivors of top-k in vocabulary order
+      int idx[SAMPLE_LIST];
+    } sorted;
+  };
+  uint32_t key[SAMPLE_LIST];           // collected values (any order); 0 = none
+  int idx[SAMPLE_LIST];
+  double warp_d[32];
   float warp_f[32];
-  float bcast_f[4];
-  uint32_t prefix;
-  uint32_t remaining;
-  int chosen;
-  int last_kept;
+  int n_list, cross_bin, chosen, last_kept, warp_i[32];
+  double cross_before;
+  uint32_t limit;
 };
 
+template <int NT>
 __device__ __forceinline__ float block_max(float v, Scratch* sc) {
   for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   __syncthreads();
   if ((threadIdx.x & 31) == 0) sc->warp_f[threadIdx.x >> 5] = v;
   __syncthreads();
-  float r = sc->warp_f[threadIdx.x & 31];
-  for (int o = 16; o; o >>= 1) r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, o));
+  float r = sc->warp_f[threadIdx.x & (NT / 32 - 1)];
+  for (int o = NT / 64; o; o >>= 1) r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, o));
   return r;
 }
 
-__device__ __forceinline__ float block_sum(float v, Scratch* sc) {
+template <int NT>
+__device__ __forceinline__ double block_sum(double v, Scratch* sc) {
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) sc->warp_f[threadIdx.x >> 5] = v;
+  if ((threadIdx.x & 31) == 0) sc->warp_d[threadIdx.x >> 5] = v;
   __syncthreads();
-  float r = sc->warp_f[threadIdx.x & 31];
-  for (int o = 16; o; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  double r = sc->warp_d[threadIdx.x & (NT / 32 - 1)];
+  for (int o = NT / 64; o; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
   return r;
 }
 
-// exclusive prefix of v over the block (thread order); *total = sum over the block
-__device__ __forceinline__ float block_exclusive_scan(float v, Scratch* sc, float* total) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  float inc = v;
+// The row as groups of 16 aligned bytes.  Group g holds the elements [g * VEC - lead, (g + 1) * VEC - lead): rows need
+// not start on a 16-byte boundary, and the first and last group are read element by element.
+template <typename T>
+struct Row {
+  static constexpr int VEC = 16 / (int)sizeof(T);
+  const T* base;
+  const uint32_t* bits;    // penalised elements by shifted position (index + lead); null = none
+  int V, lead, groups;
+  float inv_t, penalty;
+
+  __device__ __forceinline__ void init(const T* row, int V_) {
+    base = row;
+    V = V_;
+    lead = (int)((reinterpret_cast<uintptr_t>(row) & 15u) / sizeof(T));
+    groups = (V + lead + VEC - 1) / VEC;
+  }
+  __device__ __forceinline__ uint4 raw(int g) const {
+    const int i0 = g * VEC - lead;
+    if (i0 >= 0 && i0 + VEC <= V) return __ldg(reinterpret_cast<const uint4*>(base + i0));
+    union { uint4 u; T t[VEC]; } r;
+    r.u = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int j = 0; j < VEC; ++j)
+      if (i0 + j >= 0 && i0 + j < V) r.t[j] = base[i0 + j];
+    return r.u;
+  }
+  // temperature and penalty; elements outside the row become -inf
+  __device__ __forceinline__ void values(int g, uint4 u, float (&x)[VEC]) const {
+    if constexpr (sizeof(T) == 2) {
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        x[2 * j] = __uint_as_float(w[j] << 16) * inv_t;
+        x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u) * inv_t;
+      }
+    } else {
+      x[0] = __uint_as_float(u.x) * inv_t;
+      x[1] = __uint_as_float(u.y) * inv_t;
+      x[2] = __uint_as_float(u.z) * inv_t;
+      x[3] = __uint_as_float(u.w) * inv_t;
+    }
+    if (bits) {
+      const int s = g * VEC;
+      const uint32_t m = (bits[s >> 5] >> (s & 31)) & ((1u << VEC) - 1u);
+      if (m) {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j)
+          if (m >> j & 1u) x[j] = x[j] > 0.f ? x[j] / penalty : x[j] * penalty;
+      }
+    }
+    if (g == 0 || g == groups - 1) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) {
+        const int i = g * VEC - lead + j;
+        if (i < 0 || i >= V) x[j] = -INFINITY;
+      }
+    }
+  }
+};
+
+// Every warp walks its own contiguous stretch of the row, four groups in flight per lane.  f(index of x[0], x).
+template <int NT, typename T, typename F>
+__device__ __forceinline__ void for_each(const Row<T>& r, F f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (r.groups + NT / 32 - 1) / (NT / 32);
+  const int g1 = min(r.groups, (warp + 1) * per);
+  for (int g = warp * per + lane; g < g1; g += 128) {
+    uint4 u[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (g + 32 * k < g1) u[k] = r.raw(g + 32 * k);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (g + 32 * k < g1) {
+        float x[Row<T>::VEC];
+        r.values(g + 32 * k, u[k], x);
+        f((g + 32 * k) * Row<T>::VEC - r.lead, x);
+      }
+  }
+}
+
+__device__ __forceinline__ void list_add(Scratch* sc, uint32_t key, int i) {
+  const int at = atomicAdd(&sc->n_list, 1);
+  if (at < SAMPLE_LIST) {
+    sc->key[at] = key;
+    sc->idx[at] = i;
+  }
+}
+
+__device__ __forceinline__ int bin_of(float x, float mx) {
+  return (int)fminf(fmaxf((mx - x) * SAMPLE_BINS_PER_UNIT, 0.f), (float)(SAMPLE_BINS - 1));
+}
+
+// First bin at which the running sum over the bins (counts, or masses) reaches `target`, and the sum before it; the
+// last bin when the target is never reached.  All threads call.
+template <int NT, bool MASS>
+__device__ __forceinline__ void find_crossing(Scratch* sc, double target, double lo_unit, double hi_unit) {
+  constexpr int PER = SAMPLE_BINS / NT;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double v[PER], mine = 0.0;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int b = tid * PER + j;
+    v[j] = MASS ? (double)sc->bins[2][b] * hi_unit + (double)sc->bins[1][b] * lo_unit : (double)sc->bins[0][b];
+    mine += v[j];
+  }
+  double inc = mine;
   for (int o = 1; o < 32; o <<= 1) {
-    const float t = __shfl_up_sync(0xffffffffu, inc, o);
+    const double t = __shfl_up_sync(0xffffffffu, inc, o);
     if (lane >= o) inc += t;
   }
   __syncthreads();
-  if (lane == 31) sc->warp_f[w] = inc;
+  if (lane == 31) sc->warp_d[warp] = inc;
+  if (tid == 0) { sc->cross_bin = SAMPLE_BINS - 1; sc->cross_before = 0.0; }
   __syncthreads();
-  float ws = sc->warp_f[lane];
-  float winc = ws;
-  for (int o = 1; o < 32; o <<= 1) {
-    const float t = __shfl_up_sync(0xffffffffu, winc, o);
-    if (lane >= o) winc += t;
+  double before = inc - mine;
+  for (int w = 0; w < warp; ++w) before += sc->warp_d[w];
+  if ((before < target && target <= before + mine) || tid == NT - 1) {
+    // (the last thread also covers a target that rounding put above the total)
+    double cum = before;
+    int b = 0;
+#pragma unroll
+    for (; b < PER - 1; ++b) {
+      if (cum + v[b] >= target) break;
+      cum += v[b];
+    }
+    if (before < target) { sc->cross_bin = tid * PER + b; sc->cross_before = cum; }
   }
-  const float before_warp = __shfl_sync(0xffffffffu, winc - ws, w);
-  *total = __shfl_sync(0xffffffffu, winc, 31);
-  return before_warp + inc - v;
+  __syncthreads();
 }
 
-template <typename T>
-__global__ void __launch_bounds__(SAMPLE_THREADS) k_sample_rows(SampleParams p) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Scratch* sc = reinterpret_cast<Scratch*>(smem_raw);
-  const int row = blockIdx.x, tid = threadIdx.x, V = p.V;
-  float* w = p.row_in_smem ? reinterpret_cast<float*>(smem_raw + SAMPLE_SMEM_EXTRA) : p.work + (size_t)row * V;
-  const T* lg = reinterpret_cast<const T*>(p.logits) + (size_t)row * p.ldl;
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sample_rows(SampleParams p) {
+  extern __shared__ __align__(16) unsigned char dyn_smem[];
+  __shared__ __align__(16) Scratch scratch;
+  Scratch* sc = &scratch;
+  const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   int hrow = -1;
   if (p.history) {
@@ -120,242 +244,360 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample_rows(SampleParams p) 
     if (tid == 0) p.next_ids[row] = 0;
     return;
   }
-
-  for (int i = tid; i < V; i += SAMPLE_THREADS) w[i] = IO<T>::ld(lg + i) * p.inv_temperature;
-  __syncthreads();
-  int hlen = 0;
-  if (hrow >= 0) {
-    hlen = p.hist_len ? p.hist_len[hrow] : p.hist_cols;
+  Row<T> r;
+  r.init(reinterpret_cast<const T*>(p.logits) + (size_t)row * p.ldl, p.V);
+  r.inv_t = p.inv_temperature;
+  r.penalty = p.penalty;
+  r.bits = nullptr;
+  if (hrow >= 0 && p.penalty != 1.0f) {
+    uint32_t* bm = p.bitmaps ? p.bitmaps + (size_t)row * p.bitmap_words : reinterpret_cast<uint32_t*>(dyn_smem);
+    for (int i = tid; i < p.bitmap_words; i += NT) bm[i] = 0u;
+    __syncthreads();
+    int hlen = p.hist_len ? p.hist_len[hrow] : p.hist_cols;
     hlen = max(0, min(hlen, p.hist_cols));
-    if (p.penalty != 1.0f) {
-      const int64_t* hist = p.history + (size_t)hrow * p.ld_hist;
-      for (int j = tid; j < hlen; j += SAMPLE_THREADS) {
-        const int64_t h = hist[j];
-        if (h >= 0 && h < V) {
-          const float x = IO<T>::ld(lg + h) * p.inv_temperature;  // from the ORIGINAL value: repeats write the same
-          w[h] = x > 0.f ? x / p.penalty : x * p.penalty;
-        }
-      }
+    const int64_t* hist = p.history + (size_t)hrow * p.ld_hist;
+    for (int j = tid; j < hlen; j += NT) {
+      const int64_t h = hist[j];
+      if (h >= 0 && h < p.V) atomicOr(&bm[((int)h + r.lead) >> 5], 1u << (((int)h + r.lead) & 31));
     }
+    r.bits = bm;
   }
+  if (tid == 0) { sc->n_list = 0; sc->chosen = 0x7fffffff; sc->last_kept = -1; }
   __syncthreads();
 
-  // ---- top-k: key of the k-th largest value (0 keeps everything)
-  uint32_t key_k = 0;
-  if (p.top_k > 0 && p.top_k < V) {
-    if (tid == 0) { sc->prefix = 0; sc->remaining = (uint32_t)p.top_k; }
-    for (int shift = 24; shift >= 0; shift -= 8) {
-      if (tid < 256) sc->count[tid] = 0;
-      __syncthreads();
-      const uint32_t prefix = sc->prefix;
-      const uint32_t himask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
-      for (int base = 0; base < V; base += SAMPLE_THREADS) {
-        const int i = base + tid;
-        const uint32_t key = i < V ? order_key(w[i]) : 0u;
-        const bool in = i < V && (key & himask) == prefix;
-        if (__ballot_sync(0xffffffffu, in) == 0u) continue;     // below the first level few warps hold a candidate
-        // first level: few distinct leading bytes, lanes are combined; deeper levels spread over the bins
-        if (shift == 24) warp_hist_count(sc->count, in ? (int)((key >> shift) & 255u) : -1);
-        else if (in) atomicAdd(&sc->count[(key >> shift) & 255u], 1u);
-      }
-      __syncthreads();
-      if (tid < 32) {  // warp 0: lane l owns bins 255-8l .. 248-8l (descending order of keys)
-        const uint32_t rem = sc->remaining;
-        const int top = 255 - 8 * tid;
-        uint32_t mine = 0;
+  // ---- pass 1: the maximum, and every thread's own
+  float mine = -INFINITY;
+  for_each<NT>(r, [&](int, const float (&x)[Row<T>::VEC]) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) mine += sc->count[top - j];
-        uint32_t inc = mine;
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-          if (tid >= o) inc += t;
-        }
-        const uint32_t before = inc - mine;
-        const unsigned hit = __ballot_sync(0xffffffffu, before < rem && rem <= inc);
-        const int owner = hit ? __ffs(hit) - 1 : 31;
-        if (tid == owner) {
-          uint32_t cum = before;
-          int b = top;
-          for (; b > top - 7; --b) {
-            if (cum + sc->count[b] >= rem) break;
-            cum += sc->count[b];
-          }
-          sc->remaining = rem - cum;
-          sc->prefix = prefix | ((uint32_t)b << shift);
-        }
-      }
-      __syncthreads();
+    for (int j = 0; j < Row<T>::VEC; ++j) mine = fmaxf(mine, x[j]);
+  });
+  const float mx = block_max<NT>(mine, sc);
+
+  const bool use_k = p.top_k > 0 && p.top_k < p.V;
+  const bool use_p = p.top_p > 0.f && p.top_p < 1.f;
+  const float u = p.uniforms[row];
+  float kept_mass = 0.f, kept_count = 0.f, z = 0.f;
+  int pick = 0;
+  bool listed = false;
+
+  if (use_k && p.top_k <= SAMPLE_LIST_TOP_K) {
+    // k-th largest of the threads' maxima, to its leading 20 bits (rounded down: still a lower bound)
+    const uint32_t my_key = order_key(mine);
+    uint32_t bound = 0;
+    for (int b = 31; b >= 12; --b) {
+      const uint32_t t = bound | (1u << b);
+      if (__syncthreads_count(my_key >= t) >= p.top_k) bound = t;
     }
-    key_k = sc->prefix;
-  }
-
-  // ---- what top-k left, as unnormalised probabilities e = exp(x - max) in place of the logits (0 = dropped).
-  // e is monotone in x, and for non-negative floats the bit pattern orders like the value.
-  float mx = -INFINITY;
-  for (int i = tid; i < V; i += SAMPLE_THREADS) mx = fmaxf(mx, w[i]);
-  mx = block_max(mx, sc);
-  float z = 0.f;
-  for (int i = tid; i < V; i += SAMPLE_THREADS) {
-    const float x = w[i];
-    const float e = order_key(x) >= key_k ? __expf(x - mx) : 0.f;
-    w[i] = e;
-    z += e;
-  }
-  z = block_sum(z, sc);
-
-  // ---- a short list of survivors (top-k with a small k): the nucleus search and the draw then touch one element
-  // per thread instead of the whole row.  The list keeps vocabulary order.
-  float* cval = reinterpret_cast<float*>(smem_raw + sizeof(Scratch));
-  int* cidx = reinterpret_cast<int*>(cval + SAMPLE_COMPACT);
-  const float* ev = w;
-  int n_el = V;
-  if (p.top_k > 0 && p.top_k <= SAMPLE_COMPACT / 2 && p.top_k < V) {
-    const int per_v = (V + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
-    const int a0 = min(V, tid * per_v), a1 = min(V, a0 + per_v);
-    int c = 0;
-    for (int i = a0; i < a1; ++i) c += w[i] > 0.f ? 1 : 0;
-    float tot;
-    const int at = (int)block_exclusive_scan((float)c, sc, &tot);      // counts <= V: exact in float
-    if ((int)tot <= SAMPLE_COMPACT) {                                    // block-uniform
-      int o = at;
-      for (int i = a0; i < a1; ++i) {
-        const float e = w[i];
-        if (e > 0.f) {
-          cval[o] = e;
-          cidx[o] = i;
-          ++o;
-        }
-      }
-      ev = cval;
-      n_el = (int)tot;
-      __syncthreads();
-    }
-  }
-  const bool compact = ev != w;
-
-  // ---- top-p: the largest threshold t (as a bit pattern) with mass{e >= t} >= top_p * z, i.e. the value at which
-  // the descending cumulative mass first reaches the target; found by a 4-way search over the bit patterns of
-  // (0, 1].  Every probe is one pass with a fixed reduction tree: no atomics, the same result on every run.
-  uint32_t bits_min = 1u;                       // keeps every e > 0
-  if (p.top_p > 0.f && p.top_p < 1.f && compact && n_el <= 256) {
-    // a short list: one warp holds it in registers (eight per lane) and runs the same search with shuffles only
-    const float target = p.top_p * z;
-    if (tid < 32) {
-      float e8[8];
+    if (__any_sync(0xffffffffu, my_key >= bound)) {       // most warps hold no value of the list: they skip the pass
+      const float floor_x = key_value(bound);
+      const bool all = bound <= 0x007fffffu;         // fewer than k threads hold a finite value
+      for_each<NT>(r, [&](int i0, const float (&x)[Row<T>::VEC]) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) e8[j] = (tid + 32 * j < n_el) ? ev[tid + 32 * j] : 0.f;
-      uint32_t lo = 1u, hi = 0x3f800001u;
-      while (hi - lo > 1u) {
-        const uint32_t step = (hi - lo) >> 2;
-        const uint32_t m2 = lo + ((hi - lo) >> 1);
-        const uint32_t m1 = step ? lo + step : m2, m3 = step ? m2 + step : m2;
-        float f1 = 0.f, f2 = 0.f, f3 = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const uint32_t eb = __float_as_uint(e8[j]);
-          f1 += eb >= m1 ? e8[j] : 0.f;
-          f2 += eb >= m2 ? e8[j] : 0.f;
-          f3 += eb >= m3 ? e8[j] : 0.f;
-        }
-        for (int o = 16; o; o >>= 1) {
-          f1 += __shfl_xor_sync(0xffffffffu, f1, o);
-          f2 += __shfl_xor_sync(0xffffffffu, f2, o);
-          f3 += __shfl_xor_sync(0xffffffffu, f3, o);
-        }
-        if (f3 >= target && m3 > m2) lo = m3;
-        else if (f2 >= target) { lo = m2; if (m3 > m2) hi = m3; }
-        else if (f1 >= target && m1 < m2) { lo = m1; hi = m2; }
-        else hi = (m1 < m2) ? m1 : m2;
-      }
-      if (tid == 0) sc->prefix = lo;
+        for (int j = 0; j < Row<T>::VEC; ++j)
+          if ((all || x[j] >= floor_x) && (unsigned)(i0 + j) < (unsigned)r.V) list_add(sc, order_key(x[j]), i0 + j);
+      });
     }
     __syncthreads();
-    bits_min = sc->prefix;
-  } else if (p.top_p > 0.f && p.top_p < 1.f) {
-    const float target = p.top_p * z;
-    uint32_t lo = 1u, hi = 0x3f800001u;         // mass{>= lo} >= target > mass{>= hi}
-    while (hi - lo > 1u) {
-      const uint32_t step = (hi - lo) >> 2;
-      const uint32_t m2 = lo + ((hi - lo) >> 1);
-      const uint32_t m1 = step ? lo + step : m2, m3 = step ? m2 + step : m2;
-      float f1 = 0.f, f2 = 0.f, f3 = 0.f;
-      for (int i = tid; i < n_el; i += SAMPLE_THREADS) {
-        const float e = ev[i];
-        const uint32_t eb = __float_as_uint(e);
-        f1 += eb >= m1 ? e : 0.f;
-        f2 += eb >= m2 ? e : 0.f;
-        f3 += eb >= m3 ? e : 0.f;
-      }
-      // one reduction for the three sums
-      for (int o = 16; o; o >>= 1) {
-        f1 += __shfl_xor_sync(0xffffffffu, f1, o);
-        f2 += __shfl_xor_sync(0xffffffffu, f2, o);
-        f3 += __shfl_xor_sync(0xffffffffu, f3, o);
+    const int m = sc->n_list;
+    listed = m <= SAMPLE_LIST;                             // block-uniform
+    if (listed) {
+      const int m4 = (m + 3) & ~3;
+      for (int j = m + tid; j < m4; j += NT) { sc->key[j] = 0u; sc->idx[j] = 0x7fffffff; }
+      __syncthreads();
+      // the k largest (ties with the k-th stay): fewer than k values above
+      uint32_t kk[SAMPLE_LIST / NT];
+#pragma unroll
+      for (int c = 0; c < SAMPLE_LIST / NT; ++c) {
+        const int j = tid + c * NT;
+        kk[c] = 0u;
+        if (j < m) {
+          const uint32_t key = sc->key[j];
+          int above = 0;
+          for (int i = 0; i < m4; i += 4) {
+            const uint4 o = *reinterpret_cast<const uint4*>(&sc->key[i]);
+            above += (o.x > key) + (o.y > key) + (o.z > key) + (o.w > key);
+          }
+          if (above < p.top_k && __expf(key_value(key) - mx) > 0.f) kk[c] = key;
+        }
       }
       __syncthreads();
-      if ((tid & 31) == 0) {
-        sc->mass[tid >> 5] = f1;
-        sc->mass[32 + (tid >> 5)] = f2;
-        sc->mass[64 + (tid >> 5)] = f3;
+#pragma unroll
+      for (int c = 0; c < SAMPLE_LIST / NT; ++c)
+        if (tid + c * NT < m) sc->key[tid + c * NT] = kk[c];
+      __syncthreads();
+      // vocabulary order: position = kept values with a smaller index
+      int n_keep = 0;
+#pragma unroll
+      for (int c = 0; c < SAMPLE_LIST / NT; ++c) {
+        const int j = tid + c * NT;
+        if (kk[c]) {
+          const int idx = sc->idx[j];
+          int before = 0;
+          for (int i = 0; i < m4; i += 4) {
+            const uint4 o = *reinterpret_cast<const uint4*>(&sc->key[i]);
+            const int4 q = *reinterpret_cast<const int4*>(&sc->idx[i]);
+            before += (o.x && q.x < idx) + (o.y && q.y < idx) + (o.z && q.z < idx) + (o.w && q.w < idx);
+          }
+          sc->sorted.e[before] = __expf(key_value(kk[c]) - mx);
+          sc->sorted.idx[before] = idx;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < SAMPLE_LIST / NT; ++c) n_keep += __syncthreads_count(kk[c] != 0u);
+      // nucleus: keep a value when the mass above it is below top_p of the whole
+      float e[SAMPLE_LIST / NT];
+      if (tid < n_keep || tid == 0) {
+        for (int i = 0; i < n_keep; ++i) z += sc->sorted.e[i];
+      }
+#pragma unroll
+      for (int c = 0; c < SAMPLE_LIST / NT; ++c) {
+        const int j = tid + c * NT;
+        e[c] = 0.f;
+        if (j < n_keep) {
+          e[c] = sc->sorted.e[j];
+          if (use_p) {
+            float above = 0.f;
+            for (int i = 0; i < n_keep; ++i) {
+              const float o = sc->sorted.e[i];
+              above += o > e[c] ? o : 0.f;
+            }
+            if (!(above < p.top_p * z)) e[c] = 0.f;
+          }
+        }
       }
       __syncthreads();
-      f1 = sc->mass[tid & 31];
-      f2 = sc->mass[32 + (tid & 31)];
-      f3 = sc->mass[64 + (tid & 31)];
-      for (int o = 16; o; o >>= 1) {
-        f1 += __shfl_xor_sync(0xffffffffu, f1, o);
-        f2 += __shfl_xor_sync(0xffffffffu, f2, o);
-        f3 += __shfl_xor_sync(0xffffffffu, f3, o);
+#pragma unroll
+      for (int c = 0; c < SAMPLE_LIST / NT; ++c)
+        if (tid + c * NT < n_keep) sc->sorted.e[tid + c * NT] = e[c];
+      __syncthreads();
+      // inverse CDF
+#pragma unroll
+      for (int c = 0; c < SAMPLE_LIST / NT; ++c) {
+        const int j = tid + c * NT;
+        if (e[c] > 0.f || j == 0) {
+          float cum = 0.f, upto = 0.f, cnt = 0.f;
+          for (int i = 0; i < n_keep; ++i) {
+            const float o = sc->sorted.e[i];
+            cum += o;
+            cnt += o > 0.f ? 1.f : 0.f;
+            if (i == j) upto = cum;
+          }
+          kept_mass = cum;
+          kept_count = cnt;
+          if (e[c] > 0.f) {
+            atomicMax(&sc->last_kept, j);
+            if (upto > u * cum) atomicMin(&sc->chosen, j);
+          }
+        }
       }
-      if (f3 >= target && m3 > m2) lo = m3;
-      else if (f2 >= target) { lo = m2; if (m3 > m2) hi = m3; }
-      else if (f1 >= target && m1 < m2) { lo = m1; hi = m2; }
-      else hi = (m1 < m2) ? m1 : m2;
+      __syncthreads();
+      if (tid == 0) {
+        const int at = sc->chosen != 0x7fffffff ? sc->chosen : sc->last_kept;
+        pick = at >= 0 ? sc->sorted.idx[at] : 0;
+      }
     }
-    bits_min = lo;
   }
 
-  // ---- the draw: inverse CDF in vocabulary order over the kept tokens
-  const int per = (n_el + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
-  const int i0 = min(n_el, tid * per), i1 = min(n_el, i0 + per);
-  float mine = 0.f;
-  int last = -1, cnt = 0;
-  for (int i = i0; i < i1; ++i) {
-    const float e = ev[i];
-    if (__float_as_uint(e) >= bits_min) {
-      mine += e;
-      last = i;
-      ++cnt;
-    }
-  }
-  if (tid == 0) { sc->chosen = -1; sc->last_kept = -1; }
-  float total;
-  const float before = block_exclusive_scan(mine, sc, &total);
-  const float kept = block_sum((float)cnt, sc);
-  if (last >= 0) atomicMax(&sc->last_kept, last);
-  const float target = p.uniforms[row] * total;
-  if (cnt > 0 && before <= target && target < before + mine) {
-    float cum = before;
-    int pick = last;
-    for (int i = i0; i < i1; ++i) {
-      const float e = ev[i];
-      if (__float_as_uint(e) >= bits_min) {
-        cum += e;
-        if (cum > target) { pick = i; break; }
+  if (!listed) {
+    uint32_t key_k = 0u;                     // top-k: keep keys >= key_k
+    int cross = SAMPLE_BINS;                 // top-p: keep bins < cross, and in bin `cross` the masses >= e_min
+    uint32_t e_min = 1u;                     //        (cross == SAMPLE_BINS: e_min alone decides)
+    if (use_k) {
+      for (int b = tid; b < SAMPLE_BINS; b += NT) sc->bins[0][b] = 0u;
+      if (tid == 0) sc->n_list = 0;
+      __syncthreads();
+      for_each<NT>(r, [&](int i0, const float (&x)[Row<T>::VEC]) {
+#pragma unroll
+        for (int j = 0; j < Row<T>::VEC; ++j)
+          if ((unsigned)(i0 + j) < (unsigned)r.V) atomicAdd(&sc->bins[0][bin_of(x[j], mx)], 1u);
+      });
+      __syncthreads();
+      find_crossing<NT, false>(sc, (double)p.top_k, 0.0, 0.0);
+      const int cb = sc->cross_bin;
+      const int need = p.top_k - (int)sc->cross_before;      // values to keep inside the bin
+      for_each<NT>(r, [&](int i0, const float (&x)[Row<T>::VEC]) {
+#pragma unroll
+        for (int j = 0; j < Row<T>::VEC; ++j)
+          if ((unsigned)(i0 + j) < (unsigned)r.V && bin_of(x[j], mx) == cb) list_add(sc, order_key(x[j]), i0 + j);
+      });
+      if (tid == 0) sc->limit = 0xffffffffu;
+      __syncthreads();
+      const int m = sc->n_list;
+      if (m <= SAMPLE_LIST) {
+        for (int j = tid; j < m; j += NT) {
+          const uint32_t key = sc->key[j];
+          int above = 0;
+          for (int i = 0; i < m; ++i) above += sc->key[i] > key;
+          if (above < need) atomicMin(&sc->limit, key);
+        }
+        __syncthreads();
+        key_k = sc->limit;
+      } else {                               // a bin with more values than the list holds (mass ties): search the key's bits
+        for (int b = 31; b >= 0; --b) {
+          const uint32_t t = key_k | (1u << b);
+          double c = 0.0;
+          for_each<NT>(r, [&](int i0, const float (&x)[Row<T>::VEC]) {
+#pragma unroll
+            for (int j = 0; j < Row<T>::VEC; ++j)
+              if ((unsigned)(i0 + j) < (unsigned)r.V && order_key(x[j]) >= t) c += 1.0;
+          });
+          if (block_sum<NT>(c, sc) >= (double)p.top_k) key_k = t;
+        }
       }
     }
-    atomicMax(&sc->chosen, pick);
+    if (use_p) {
+      for (int b = tid; b < SAMPLE_BINS; b += NT) sc->bins[1][b] = sc->bins[2][b] = 0u;
+      __syncthreads();
+      if (tid == 0) sc->n_list = 0;
+      double zz = 0.0;
+      const uint32_t half_mask = (1u << p.mass_half) - 1u;
+      const float one = (float)(1u << (2 * p.mass_half));            // the integer that stands for e = 1
+      const double unit = 1.0 / (double)one;
+      for_each<NT>(r, [&](int, const float (&x)[Row<T>::VEC]) {
+#pragma unroll
+        for (int j = 0; j < Row<T>::VEC; ++j) {
+          const float e = order_key(x[j]) >= key_k ? __expf(x[j] - mx) : 0.f;
+          const uint32_t q = __float2uint_rn(e * one);
+          const int b = bin_of(x[j], mx);
+          if (q & half_mask) atomicAdd(&sc->bins[1][b], q & half_mask);
+          if (q >> p.mass_half) atomicAdd(&sc->bins[2][b], q >> p.mass_half);
+          zz += (double)q;
+        }
+      });
+      const double zq = block_sum<NT>(zz, sc) * unit;     // exact: integers below 2^53
+      const double target = (double)p.top_p * zq;
+      find_crossing<NT, true>(sc, target, unit, unit * (double)(half_mask + 1u));
+      cross = sc->cross_bin;
+      const double before = sc->cross_before;
+      for_each<NT>(r, [&](int i0, const float (&x)[Row<T>::VEC]) {
+#pragma unroll
+        for (int j = 0; j < Row<T>::VEC; ++j)
+          if (bin_of(x[j], mx) == cross && order_key(x[j]) >= key_k && __expf(x[j] - mx) > 0.f)
+            list_add(sc, __float_as_uint(__expf(x[j] - mx)), i0 + j);
+      });
+      if (tid == 0) sc->limit = 0xffffffffu;
+      __syncthreads();
+      const int m = sc->n_list;
+      if (m <= SAMPLE_LIST) {
+        for (int j = tid; j < m; j += NT) {
+          const uint32_t eb = sc->key[j];
+          unsigned long long above = 0ull;
+          for (int i = 0; i < m; ++i) {
+            const uint32_t o = sc->key[i];
+            if (o > eb) above += __float2uint_rn(__uint_as_float(o) * one);
+          }
+          if (before + (double)above * unit < target) atomicMin(&sc->limit, eb);
+        }
+        __syncthreads();
+        e_min = sc->limit;
+      } else {                               // mass ties: search the bits of the probability
+        cross = SAMPLE_BINS;
+        e_min = 0u;
+        for (int b = 29; b >= 0; --b) {
+          const uint32_t t = e_min | (1u << b);
+          double c = 0.0;
+          for_each<NT>(r, [&](int, const float (&x)[Row<T>::VEC]) {
+#pragma unroll
+            for (int j = 0; j < Row<T>::VEC; ++j) {
+              const float e = order_key(x[j]) >= key_k ? __expf(x[j] - mx) : 0.f;
+              if (__float_as_uint(e) >= t) c += (double)__float2uint_rn(e * one);
+            }
+          });
+          if (block_sum<NT>(c, sc) * unit >= target) e_min = t;
+        }
+        e_min = max(e_min, 1u);
+      }
+    }
+    auto keep = [&](float x) -> float {      // unnormalised probability of a kept value, 0 for a dropped one
+      const float e = order_key(x) >= key_k ? __expf(x - mx) : 0.f;
+      if (cross < SAMPLE_BINS) {
+        const int b = bin_of(x, mx);
+        return b < cross || (b == cross && __float_as_uint(e) >= e_min) ? e : 0.f;
+      }
+      return __float_as_uint(e) >= e_min ? e : 0.f;
+    };
+    // ---- masses of the warps' stretches (vocabulary order), then the stretch that holds the target is walked again
+    float acc = 0.f, all = 0.f;
+    int cnt = 0;
+    for_each<NT>(r, [&](int, const float (&x)[Row<T>::VEC]) {
+#pragma unroll
+      for (int j = 0; j < Row<T>::VEC; ++j) {
+        const float e = keep(x[j]);
+        acc += e;
+        cnt += e > 0.f;
+        if (use_p) all += order_key(x[j]) >= key_k ? __expf(x[j] - mx) : 0.f;
+      }
+    });
+    for (int o = 16; o; o >>= 1) {
+      acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    }
+    __syncthreads();
+    if (lane == 0) { sc->warp_f[warp] = acc; sc->warp_i[warp] = cnt; }
+    __syncthreads();
+    int total_cnt = 0, own = -1, last = -1;
+    for (int w = 0; w < NT / 32; ++w) { kept_mass += sc->warp_f[w]; total_cnt += sc->warp_i[w]; }
+    kept_count = (float)total_cnt;
+    const float target = u * kept_mass;
+    float before = 0.f, cum = 0.f;
+    for (int w = 0; w < NT / 32; ++w) {
+      if (sc->warp_i[w]) {
+        last = w;
+        if (own < 0 && cum + sc->warp_f[w] > target) { own = w; before = cum; }
+      }
+      cum += sc->warp_f[w];
+    }
+    const bool past_end = own < 0;           // u * total rounded up to the total: the last kept token
+    if (past_end) own = last;
+    z = use_p ? (float)block_sum<NT>((double)all, sc) : kept_mass;
+    if (warp == own) {
+      const int per = (r.groups + NT / 32 - 1) / (NT / 32);
+      const int g0 = warp * per, g1 = min(r.groups, (warp + 1) * per);
+      int found = 0x7fffffff, last_i = -1;
+      for (int g = g0; g < g1; g += 32) {    // 32 groups at a time: prefix over the lanes, then inside the lane
+        float x[Row<T>::VEC], e[Row<T>::VEC], s = 0.f;
+        const bool on = g + lane < g1;
+        if (on) r.values(g + lane, r.raw(g + lane), x);
+#pragma unroll
+        for (int j = 0; j < Row<T>::VEC; ++j) {
+          e[j] = on ? keep(x[j]) : 0.f;
+          s += e[j];
+          if (e[j] > 0.f) last_i = (g + lane) * Row<T>::VEC - r.lead + j;
+        }
+        float inc = s;
+        for (int o = 1; o < 32; o <<= 1) {
+          const float t = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += t;
+        }
+        if (!past_end) {
+          float c = before + (inc - s);
+#pragma unroll
+          for (int j = 0; j < Row<T>::VEC; ++j) {
+            c += e[j];
+            if (e[j] > 0.f && c > target) found = min(found, (g + lane) * Row<T>::VEC - r.lead + j);
+          }
+          if (__any_sync(0xffffffffu, found != 0x7fffffff)) break;
+        }
+        before += __shfl_sync(0xffffffffu, inc, 31);
+      }
+      for (int o = 16; o; o >>= 1) {
+        found = min(found, __shfl_xor_sync(0xffffffffu, found, o));
+        last_i = max(last_i, __shfl_xor_sync(0xffffffffu, last_i, o));
+      }
+      if (lane == 0) sc->chosen = found != 0x7fffffff ? found : last_i;
+    }
+    __syncthreads();
+    pick = sc->chosen;
+    if (pick < 0 || pick >= p.V) pick = 0;
   }
-  __syncthreads();
+
   if (tid == 0) {
-    int pick = sc->chosen >= 0 ? sc->chosen : sc->last_kept;
-    if (compact) pick = cidx[pick];
     p.next_ids[row] = pick;
     if (p.stats) {
       float* s = p.stats + 4 * (size_t)row;
       s[0] = mx;
-      s[1] = total;
-      s[2] = kept;
+      s[1] = kept_mass;
+      s[2] = kept_count;
       s[3] = z;
     }
     if (p.append && hrow >= 0 && p.hist_len) {
@@ -368,6 +610,14 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample_rows(SampleParams p) 
   }
 }
 
+template <typename T, int NT>
+int sample_launch(const SampleParams& p, size_t smem, cudaStream_t st) {
+  if (smem > 0) QPAM_CUDA(cudaFuncSetAttribute(k_sample_rows<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_sample_rows<T, NT><<<p.n, NT, smem, st>>>(p);
+  QPAM_LAUNCH_CHECK("k_sample_rows");
+  return QPAM_OK;
+}
+
 }  // namespace
 }  // namespace qpam
 
@@ -375,8 +625,8 @@ using namespace qpam;
 
 extern "C" size_t qpam_sample_workspace_bytes(int32_t n, int32_t V) {
   if (n <= 0 || V <= 0) return 0;
-  if ((size_t)V * 4 + SAMPLE_SMEM_EXTRA <= 227u * 1024u) return 0;
-  return (size_t)n * V * 4;
+  const size_t words = ((size_t)V + 8 + 31) / 32;
+  return words * 4 <= SAMPLE_SMEM_BITMAP ? 0 : (size_t)n * words * 4;      // one bit per token, only for vocabularies beyond 1.3 M
 }
 
 extern "C" int qpam_sample_logits(const void* logits, int32_t io_dtype, int32_t n, int32_t V, int64_t ld_logits,
@@ -400,23 +650,19 @@ extern "C" int qpam_sample_logits(const void* logits, int32_t io_dtype, int32_t 
   p.n = n; p.V = V; p.n_hist_rows = n_hist_rows; p.hist_cols = hist_cols; p.top_k = top_k; p.append = append;
   p.inv_temperature = 1.f / temperature; p.top_p = top_p; p.penalty = repetition_penalty;
   const size_t need = qpam_sample_workspace_bytes(n, V);
-  p.row_in_smem = need == 0;
-  size_t smem = SAMPLE_SMEM_EXTRA;
-  if (p.row_in_smem) {
-    smem += (size_t)V * 4;
-  } else {
+  p.bitmap_words = (int)(((size_t)V + 8 + 31) / 32);
+  p.mass_half = 15;
+  while (p.mass_half > 1 && ((int64_t)V << p.mass_half) > (1ll << 32)) --p.mass_half;
+  size_t smem = repetition_penalty != 1.f && history ? (size_t)p.bitmap_words * 4 : 0;
+  if (need) {
     QPAM_REQUIRE(workspace && workspace_bytes >= need, "sample: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
-    p.work = reinterpret_cast<float*>(workspace);
+    p.bitmaps = reinterpret_cast<uint32_t*>(workspace);
+    smem = 0;
   }
-  static_assert(sizeof(Scratch) + SAMPLE_COMPACT * 8 <= SAMPLE_SMEM_EXTRA, "scratch does not fit");
+  // more rows than SMs: two CTAs of 512 threads share an SM, so that one row's block-wide steps run under the other's
+  // passes; otherwise a row has an SM to itself and takes 1024 threads
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (io_dtype == QPAM_F32) {
-    QPAM_CUDA(cudaFuncSetAttribute(k_sample_rows<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_sample_rows<float><<<n, SAMPLE_THREADS, smem, st>>>(p);
-  } else {
-    QPAM_CUDA(cudaFuncSetAttribute(k_sample_rows<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_sample_rows<__nv_bfloat16><<<n, SAMPLE_THREADS, smem, st>>>(p);
-  }
-  QPAM_LAUNCH_CHECK("k_sample_rows");
-  return QPAM_OK;
+  const bool wide = n <= 148;
+  if (io_dtype == QPAM_F32) return wide ? sample_launch<float, 1024>(p, smem, st) : sample_launch<float, 512>(p, smem, st);
+  return wide ? sample_launch<__nv_bfloat16, 1024>(p, smem, st) : sample_launch<__nv_bfloat16, 512>(p, smem, st);
 }

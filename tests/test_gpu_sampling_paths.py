@@ -1,0 +1,37 @@
+"""The sampler's dispatch at its edges: list and bin paths around the list's top-k limit, rows that start off a 16-byte
+boundary, rows shorter than the block, and rows whose ties overflow the list."""
+import pytest
+import torch
+
+from qllm2_b200 import ops
+from tests.test_gpu_sampling import _check_rows
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("n", [3, 150])
+@pytest.mark.parametrize("dtype,V,lead", [(torch.bfloat16, 50261, 0), (torch.bfloat16, 4099, 3), (torch.float32, 1027, 1), (torch.float32, 9, 0)])
+@pytest.mark.parametrize("top_k,top_p", [(384, 0.9), (385, 0.9), (1500, 0.0), (0, 0.6)])
+def test_paths(n, dtype, V, lead, top_k, top_p):
+    g = torch.Generator().manual_seed(V + top_k + n)
+    store = (torch.randn(n, V + 11, generator=g) * 2.0).to(dtype).to(DEV)
+    logits = store[:, lead:lead + V]
+    hist = torch.randint(0, V, (n, 33), generator=g)
+    u = torch.rand(n, generator=g)
+    cfg = dict(temperature=0.8, top_k=top_k, top_p=top_p, repetition_penalty=1.2345)
+    ids, stats = ops.sample_logits(logits, u.to(DEV), history=hist.to(DEV), return_stats=True, **cfg)
+    _check_rows(logits, hist.numpy(), None, u.numpy(), ids.cpu().numpy(), stats.cpu().numpy(), cfg, count_exact=dtype == torch.float32)
+
+
+@pytest.mark.parametrize("top_k,top_p", [(50, 0.9), (900, 0.5), (0, 0.5)])
+def test_ties_beyond_the_list(top_k, top_p):
+    """Every token at one of two values: all of the upper ones tie with the threshold and stay."""
+    n, V = 4, 20000
+    g = torch.Generator().manual_seed(3)
+    logits = (torch.rand(n, V, generator=g) < 0.5).float().to(DEV)
+    u = torch.rand(n, generator=g)
+    cfg = dict(temperature=1.0, top_k=top_k, top_p=top_p, repetition_penalty=1.0)
+    ids, stats = ops.sample_logits(logits, u.to(DEV), return_stats=True, **cfg)
+    _check_rows(logits, None, None, u.numpy(), ids.cpu().numpy(), stats.cpu().numpy(), cfg)
+    assert stats[:, 2].tolist() == (logits == 1).sum(1).tolist()
