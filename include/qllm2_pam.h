@@ -337,6 +337,38 @@ typedef struct qpam_front_args {
 } qpam_front_args;
 int qpam_pam_front_fwd(const qpam_front_args* args, void* stream);
 
+/* One decode step of a whole model for a handful of sequences (n <= 16, bf16 weights, head dim 64): token ids ->
+ * arg-max ids or bf16 logits, the slots' states updated in place (the per-token loop body of V11LM.generate,
+ * v11/model.py:1206-1245).  Weights are the packed block matrices of an inference forward: complex projections
+ * [2*out, 2*in] with rows (o,re) = (Wr,-Wi), (o,im) = (Wi,Wr) over interleaved columns (only the (o,re) rows are read),
+ * w_front = qkv block matrix [6*H*d] followed by rows_a real rows (biases at the same rows of b_front), w_mag the
+ * rows_m real rows that read |x|.  col_* are columns of the combined gate values [rows_a | rows_m], -1 = absent.
+ * `layers` is an array in HOST memory; every other pointer is a device pointer. */
+typedef struct qpam_step_layer {
+  const void *w_gu, *w_down, *w_front, *b_front, *w_mag, *b_mag, *w_o;      /* bf16 */
+  const float *n1, *n2, *act_bias, *act_beta, *cgu_scale, *pam_scale, *dt_bias, *dt_off;
+  int32_t col_dt, col_pg, col_phase, col_score;
+  float gamma_floor;
+} qpam_step_layer;
+typedef struct qpam_step_args {
+  const qpam_step_layer* layers;
+  const void *embed_real, *embed_imag, *w_head, *b_head, *w_vocab;          /* bf16; b_head may be NULL */
+  const float *embed_scale, *out_scale, *head_norm_scale, *rope;            /* rope [rope_len, d, 2] or NULL */
+  const int64_t *ids, *positions;                                           /* [n] */
+  const int32_t* slot_ids;                                                  /* [n], outside [0, n_slots): padded row */
+  void* pool;                                                               /* [n_slots, n_layers, K, H, d, d, 2] */
+  int64_t* next_ids;                                                        /* [n], or */
+  void* logits;                                                             /* bf16 [n, ld_logits] */
+  void* workspace;
+  size_t workspace_bytes;
+  int64_t n_slots, rope_len, ld_logits;
+  int32_t n, n_layers, D, H, d, K, hidden, V, rows_a, rows_m, state_dtype;
+  float q_scale;
+} qpam_step_args;
+int32_t qpam_step_supported(int32_t n, int32_t D, int32_t H, int32_t d, int32_t K, int32_t hidden, int32_t V);
+size_t qpam_step_workspace_bytes(const qpam_step_args* args);
+int qpam_step_fwd(const qpam_step_args* args, void* stream);
+
 /* Residual with a learnable scalar (V11Block.forward: x + mixed * cgu_scale, x + pam_out * pam_scale):
  * out[i] = x[i] + scale[0] * delta[i] over n scalars (n a multiple of 4; x/out and delta may differ in
  * dtype).  Backward: ddelta = scale[0] * dout, dscale = sum of the P partials, d(x) = dout. */

@@ -52,6 +52,20 @@ class FrontArgs(C.Structure):
     ]
 
 
+class StepLayer(C.Structure):
+    _fields_ = [(n, c_void_p) for n in ("w_gu", "w_down", "w_front", "b_front", "w_mag", "b_mag", "w_o", "n1", "n2", "act_bias", "act_beta",
+                                        "cgu_scale", "pam_scale", "dt_bias", "dt_off")] + \
+        [(n, c_int32) for n in ("col_dt", "col_pg", "col_phase", "col_score")] + [("gamma_floor", c_float)]
+
+
+class StepArgs(C.Structure):
+    _fields_ = [("layers", C.POINTER(StepLayer))] + \
+        [(n, c_void_p) for n in ("embed_real", "embed_imag", "w_head", "b_head", "w_vocab", "embed_scale", "out_scale", "head_norm_scale", "rope",
+                                 "ids", "positions", "slot_ids", "pool", "next_ids", "logits", "workspace")] + \
+        [("workspace_bytes", c_size_t)] + [(n, c_int64) for n in ("n_slots", "rope_len", "ld_logits")] + \
+        [(n, c_int32) for n in ("n", "n_layers", "D", "H", "d", "K", "hidden", "V", "rows_a", "rows_m", "state_dtype")] + [("q_scale", c_float)]
+
+
 SIGNATURES = {
     "qpam_scan_workspace_bytes": (c_size_t, [C.POINTER(ScanArgs), c_int32]),
     "qpam_scan_fwd": (c_int32, [C.POINTER(ScanArgs), c_void_p]),
@@ -106,6 +120,9 @@ SIGNATURES = {
     "qpam_residual_cnorm_fwd": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int64,
                                           c_int32, C.c_float, c_void_p]),
     "qpam_pam_front_fwd": (c_int32, [C.POINTER(FrontArgs), c_void_p]),
+    "qpam_step_supported": (c_int32, [c_int32] * 7),
+    "qpam_step_workspace_bytes": (c_size_t, [C.POINTER(StepArgs)]),
+    "qpam_step_fwd": (c_int32, [C.POINTER(StepArgs), c_void_p]),
     "qpam_scaled_residual_fwd": (c_int32, [c_void_p, c_int32, c_void_p, c_int32, c_void_p, c_void_p, c_int64, c_void_p]),
     "qpam_scaled_residual_bwd": (c_int32, [c_void_p, c_int32, c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_int32,
                                            c_int64, c_void_p]),

@@ -111,11 +111,13 @@ namespace qpam {
 int ce_tc_device_status(int* value, bool clear);
 int scan_tc_device_status(int* value, bool clear);
 int decode_device_status(int* value, bool clear);
+int step_device_status(int* value, bool clear);
 }
 
 extern "C" int qpam_device_status(int32_t* status, int32_t clear) {
   int first = 0;
-  int (*readers[])(int*, bool) = {qpam::ce_tc_device_status, qpam::scan_tc_device_status, qpam::decode_device_status};
+  int (*readers[])(int*, bool) = {qpam::ce_tc_device_status, qpam::scan_tc_device_status, qpam::decode_device_status,
+                                 qpam::step_device_status};
   for (auto rd : readers) {
     int v = 0;
     const int rc = rd(&v, clear != 0);

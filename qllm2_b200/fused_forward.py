@@ -52,6 +52,7 @@ class FusedForward:
                             torch.stack([hp.bias_real, hp.bias_imag], -1).reshape(-1).detach().to(self.dtype))
         self.w_vocab = torch.cat([model.embed.embed_real.weight, model.embed.embed_imag.weight], -1).detach().to(self.dtype).contiguous()
         self.layers = [self.pack_block(blk, self.dtype) for blk in model.blocks]
+        self._step_layers = None
 
     @staticmethod
     def unsupported_reason(model: V11LM) -> Optional[str]:
@@ -207,6 +208,62 @@ class FusedForward:
         h = F.linear(xn.reshape(n, 2 * self.D), self.w_head_proj, self.b_head_proj).view(n, self.D, 2)
         h, _ = self._res_norm(h, None, None, self.head_norm_scale)
         return h
+
+    # ---------------------------------------------------------------------------------- decode step for few rows
+    def step_supported(self, n: int) -> bool:
+        """Whether `step` covers a batch of n rows: few enough that the weights' bytes, not the arithmetic, set the
+        time (there the step reads half of them in a third of the launches), bf16 weights, head dim 64."""
+        return (self.dtype == torch.bfloat16 and self.model.embed.embed_real.weight.dtype == torch.bfloat16 and
+                bool(_lib.lib().qpam_step_supported(n, self.D, self.H, self.d, self.K, self.layers[0].hidden, self.w_vocab.shape[0])))
+
+    def _pack_step_layers(self):
+        H, inner = self.H, self.inner
+        arr = (_lib.StepLayer * len(self.layers))()
+        for s, L in zip(arr, self.layers):
+            for name in ("w_gu", "w_down", "w_front", "b_front", "w_mag", "b_mag", "w_o", "n1", "n2", "act_bias", "act_beta", "cgu_scale",
+                         "pam_scale", "dt_bias"):
+                setattr(s, name, ptr(getattr(L, name)))
+            s.dt_off = ptr(L.dt_off)
+            s.gamma_floor = L.gamma_floor
+            rows_a = L.w_front.shape[0] - 6 * inner
+            for name in ("dt", "pg", "phase", "score"):
+                src, off = L.cols.get(name, ("", -1))
+                setattr(s, "col_" + name, off - 6 * inner if src == "a" else rows_a + off if src == "m" else -1)
+        return arr
+
+    @torch.no_grad()
+    def step(self, ids, positions, slots, pool, logits: bool = False):
+        """One decode step of the whole model (qpam_step_fwd): ids, positions int64 [n], slots int32 [n], `pool`
+        [n_slots, L, K, H, d, d, 2] updated in place.  Returns the arg-max ids [n], or bf16 logits [n, V]."""
+        if self._step_layers is None:
+            self._step_layers = self._pack_step_layers()
+        n, V, L0 = ids.numel(), self.w_vocab.shape[0], self.layers[0]
+        dev, emb = self.device, self.model.embed
+        a = _lib.StepArgs()
+        a.layers = self._step_layers
+        er, ei = emb.embed_real.weight, emb.embed_imag.weight
+        a.embed_real, a.embed_imag, a.w_head, a.b_head, a.w_vocab = ptr(er), ptr(ei), ptr(self.w_head_proj), ptr(self.b_head_proj), ptr(self.w_vocab)
+        a.embed_scale, a.out_scale, a.head_norm_scale, a.rope = ptr(self.embed_scale), ptr(self.out_scale), ptr(self.head_norm_scale), ptr(self.rope)
+        ids, positions = ids.reshape(-1).contiguous(), positions.reshape(-1).to(torch.int64).contiguous()
+        a.ids, a.positions, a.slot_ids, a.pool = ptr(ids), ptr(positions), ptr(slots), ptr(pool)
+        if slots.dtype != torch.int32 or slots.numel() != n or positions.numel() != n or ids.dtype != torch.int64:
+            raise _lib.QPamError("step: ids / positions int64 [n] and slots int32 [n] expected")
+        if pool.dim() != 7 or not pool.is_contiguous() or tuple(pool.shape[1:]) != (len(self.layers), self.K, self.H, self.d, self.d, 2):
+            raise _lib.QPamError(f"step: state pool {tuple(pool.shape)} does not fit this model")
+        a.n, a.n_layers, a.D, a.H, a.d, a.K, a.hidden, a.V = n, len(self.layers), self.D, self.H, self.d, self.K, L0.hidden, V
+        a.rows_a, a.rows_m = L0.w_front.shape[0] - 6 * self.inner, 0 if L0.w_mag is None else L0.w_mag.shape[0]
+        a.n_slots, a.rope_len, a.state_dtype, a.q_scale = pool.shape[0], 0 if self.rope is None else self.rope.shape[0], dtype_code(pool.dtype), self.d ** -0.5
+        if logits:
+            ld = (V + 7) // 8 * 8
+            out = torch.empty(n, ld, dtype=torch.bfloat16, device=dev)
+            a.logits, a.ld_logits = ptr(out), ld
+        else:
+            out = torch.empty(n, dtype=torch.int64, device=dev)
+            a.next_ids = ptr(out)
+        ws = torch.empty(_lib.lib().qpam_step_workspace_bytes(a), dtype=torch.uint8, device=dev)
+        a.workspace, a.workspace_bytes = ptr(ws), ws.numel()
+        check(_lib.lib().qpam_step_fwd(a, stream_ptr()), "qpam_step_fwd")
+        return out[:, :V] if logits else out
 
     @torch.no_grad()
     def logits(self, lm: torch.Tensor) -> torch.Tensor:

@@ -196,8 +196,8 @@ class ContinuousBatcher:
             self._hist = torch.zeros(n_slots, max_position + 1, dtype=torch.long, device=self.device)
             self._hist_len = torch.zeros(n_slots, dtype=torch.int32, device=self.device)
         if cuda_graph:
-            self._g_ids = torch.zeros(n_slots, 1, dtype=torch.long, device=self.device)
-            self._g_pos = torch.zeros(n_slots, 1, dtype=torch.long, device=self.device)
+            self._g_io = torch.zeros(2, n_slots, dtype=torch.long, device=self.device)
+            self._g_ids, self._g_pos = self._g_io[0][:, None], self._g_io[1][:, None]
             self._g_slots = torch.full((n_slots,), -1, dtype=torch.int32, device=self.device)
             self._g_out = None
 
@@ -231,6 +231,9 @@ class ContinuousBatcher:
         else:
             Hm, W = self.model.tied_head_matrices(lm_rows.unsqueeze(1))
             logits = (Hm @ W.to(Hm.dtype).T).float()
+        return self._draw(logits, slots)
+
+    def _draw(self, logits, slots):
         return ops.sample_logits(logits, history=self._hist, hist_len=self._hist_len, slot_ids=slots, append=True,
                                  **self.sampling)
 
@@ -240,13 +243,23 @@ class ContinuousBatcher:
         state its predecessor left in the slot; a request emits its first token when its last piece is done."""
         lens = [take for _, _, take in items]
         self._ensure_rope(max(st + take for _, st, take in items))
-        # token ids and positions are assembled on the host and copied once each
-        ids = torch.cat([torch.as_tensor(r.prompt[st:st + take], dtype=torch.long) for r, st, take in items]).to(self.device)[None]
-        positions = torch.cat([torch.arange(st, st + take) for _, st, take in items]).to(self.device)[None]
-        cu = torch.zeros(len(items) + 1, dtype=torch.int32)
-        cu[1:] = torch.tensor(lens).cumsum(0).int()
-        cu = cu.to(self.device)
-        slots = torch.tensor([r.slot for r, _, _ in items], dtype=torch.int32, device=self.device)
+        # token ids, positions and descriptors are assembled on the host and copied once each
+        toks: List[int] = []
+        for r, st, take in items:
+            toks += r.prompt[st:st + take] if take < len(r.prompt) else r.prompt
+        n_tok, count = len(toks), torch.tensor(lens)
+        ends = count.cumsum(0)
+        starts = torch.tensor([st for _, st, _ in items])
+        both = torch.empty(2, n_tok, dtype=torch.long)
+        both[0] = torch.tensor(toks, dtype=torch.long)
+        both[1] = torch.arange(n_tok) + (starts - ends + count).repeat_interleave(count)
+        both = both.to(self.device)
+        ids, positions = both[0][None], both[1][None]
+        meta = torch.zeros(2, len(items) + 1, dtype=torch.int32)
+        meta[0, 1:] = ends
+        meta[1, :-1] = torch.tensor([r.slot for r, _, _ in items], dtype=torch.int32)
+        meta = meta.to(self.device)
+        cu, slots = meta[0], meta[1, :-1]
         s0_of = None
         if any(st > 0 for _, st, _ in items):
             resumed = torch.tensor([1.0 if st > 0 else 0.0 for _, st, _ in items], device=self.device)
@@ -255,8 +268,7 @@ class ContinuousBatcher:
                 s = self.pool[slots.long(), layer].float() * resumed[:, None, None, None, None, None]
                 return s.permute(1, 0, 2, 3, 4, 5).contiguous()
         if self.sampling is not None:      # the penalty looks at the whole prompt: load the slots' histories
-            for r, st, take in items:
-                self._hist[r.slot, st:st + take] = torch.as_tensor(r.prompt[st:st + take], dtype=torch.long).to(self.device)
+            self._hist[slots.long().repeat_interleave(count.to(self.device), output_size=n_tok), both[1]] = both[0]
             self._hist_len[slots.long()] = torch.tensor([st + take for _, st, take in items], dtype=torch.int32, device=self.device)
             # a piece that ends mid-prompt draws nothing: its row is padded out (slot -1)
             pick_slots = torch.tensor([r.slot if st + take == len(r.prompt) else -1 for r, st, take in items],
@@ -304,35 +316,47 @@ class ContinuousBatcher:
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             self._g_out = self._decode_tensors(self._g_ids, self._g_pos, self._g_slots)
+            # the next step's inputs, so that steps can follow one another without the host (`_decode` sets them anew)
+            self._g_ids[:, 0].copy_(self._g_out)
+            self._g_pos.add_(1)
         self._graph = graph
 
     @torch.no_grad()
-    def _decode(self, live: List[Request]):
+    def _decode(self, live: List[Request], steps: int = 1):
+        """`steps` decode steps of the live sequences; more than one only while none of them finishes (captured steps feed
+        each other on the device, and the host reads all their tokens at once)."""
         n = len(live)
-        self._ensure_rope(max(r.position for r in live) + 1)
-        ids = torch.tensor([r.generated[-1] for r in live], dtype=torch.long)
-        positions = torch.tensor([r.position for r in live], dtype=torch.long)
-        slots = torch.tensor([r.slot for r in live], dtype=torch.int32)
+        self._ensure_rope(max(r.position for r in live) + steps)
+        ids, positions, slots = [r.generated[-1] for r in live], [r.position for r in live], [r.slot for r in live]
         if self.cuda_graph:
-            self._g_ids.zero_()
-            self._g_pos.zero_()
-            self._g_slots.fill_(-1)
-            self._g_ids[:n, 0] = ids.to(self.device)
-            self._g_pos[:n, 0] = positions.to(self.device)
-            self._g_slots[:n] = slots.to(self.device)
             self.warmup()
-            self._graph.replay()
-            nxt = self._g_out[:n]
+            pad = [0] * (self.n_slots - n)
+            self._g_io.copy_(torch.tensor([ids + pad, positions + pad], dtype=torch.long))
+            self._g_slots.copy_(torch.tensor(slots + [-1] * (self.n_slots - n), dtype=torch.int32))
+            if steps == 1:
+                self._graph.replay()
+                rows = [self._g_out[:n].tolist()]
+            else:
+                log = torch.empty(steps, self.n_slots, dtype=torch.long, device=self.device)
+                for i in range(steps):
+                    self._graph.replay()
+                    log[i].copy_(self._g_out)
+                rows = log[:, :n].tolist()
         else:
-            nxt = self._decode_tensors(ids.to(self.device)[:, None], positions.to(self.device)[:, None],
-                                       slots.to(self.device))
-        for r, t in zip(live, nxt.tolist()):
-            r.generated.append(int(t))
-        self.decoded_tokens += n
+            dev = self.device
+            rows = [self._decode_tensors(torch.tensor(ids, dtype=torch.long, device=dev)[:, None], torch.tensor(positions, dtype=torch.long, device=dev)[:, None],
+                                         torch.tensor(slots, dtype=torch.int32, device=dev)).tolist()]
+        for row in rows:
+            for r, t in zip(live, row):
+                r.generated.append(t)
+        self.decoded_tokens += n * len(rows)
 
     @torch.no_grad()
     def _decode_tensors(self, ids, positions, slots):
         """One decode step for rows (ids [n,1], positions [n,1], slots [n]); returns next ids [n]."""
+        if self.ff is not None and self.ff.step_supported(ids.shape[0]):
+            out = self.ff.step(ids, positions, slots, self.pool, logits=self.sampling is not None)
+            return out if self.sampling is None else self._draw(out, slots)
         if self.ff is not None:
             xn = self.ff.hidden(ids, _DecodeMix(self, slots), positions=positions)
             return self._pick(self.ff.head_hidden(xn), slots)
@@ -409,9 +433,25 @@ class ContinuousBatcher:
             _lib.raise_on_device_error("ContinuousBatcher.step")
         return len(live_before) + len(batch)
 
+    def _quiet_steps(self, most: int = 64) -> int:
+        """Decode steps during which the batch cannot change: nothing is admitted or prefilled, and nobody finishes before
+        the last of them.  1 when steps have to be taken one by one."""
+        live = self.sched.live.values()
+        if not self.cuda_graph or not live or (self.sched.waiting and self.sched.free) or any(r.prefilling or r.done for r in live):
+            return 1
+        return min(most, min(r.max_new_tokens - len(r.generated) for r in live))
+
     def run(self) -> Dict[int, List[int]]:
         while not self.sched.idle:
-            self.step()
+            k = self._quiet_steps()
+            if k <= 1:
+                self.step()
+                continue
+            self._decode(self.sched.live_requests(), k)       # what k calls of step() do, without the host in between
+            self.sched.retire_finished()
+            self.steps += k
+            if self.steps % 64 < k:
+                _lib.raise_on_device_error("ContinuousBatcher.run")
         _lib.raise_on_device_error("ContinuousBatcher.run")
         return {r.rid: r.generated for r in self.sched.finished}
 
@@ -471,6 +511,14 @@ def generate_fused(model: V11LM, input_ids, max_new_tokens, sample, eos_token_id
         lm = ff.head_hidden(xn_rows)
         return ff.greedy_next(lm)[:, None] if greedy else ff.logits(lm)
 
+    small = ff.step_supported(B)
+
+    def step(ids, positions):
+        if small:
+            got = ff.step(ids, positions, slots, pool, logits=not greedy)
+            return got[:, None] if greedy else got.float()
+        return head(ff.hidden(ids, mix, positions=positions))
+
     out = input_ids.clone()
     xn = ff.hidden(out, _BatchPrefillMix(pool, slots))
     res = head(xn.view(B, T0, cfg.dim, 2)[:, -1])
@@ -491,11 +539,11 @@ def generate_fused(model: V11LM, input_ids, max_new_tokens, sample, eos_token_id
         ids_buf.copy_(nxt)
         pos_buf.fill_(T0 + i)
         if graph is None and i == 0:
-            res = head(ff.hidden(ids_buf, mix, positions=pos_buf))          # first step eagerly (warms every kernel up)
+            res = step(ids_buf, pos_buf)                                    # first step eagerly (warms every kernel up)
         elif graph is None:
             graph = torch.cuda.CUDAGraph()                                  # capture records the step, it does not run it
             with torch.cuda.graph(graph):
-                g_res = head(ff.hidden(ids_buf, mix, positions=pos_buf))
+                g_res = step(ids_buf, pos_buf)
             graph.replay()
             res = g_res.clone()
         else:
