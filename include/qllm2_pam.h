@@ -206,6 +206,11 @@ int qpam_ce_finalize(const qpam_ce_args* args, const float* row_max, const float
                      const float* row_tgt, const int64_t* row_argmax, float* lse, float* per_token,
                      float* loss_sum, float* denom, float* correct, float* tokens, void* stream);
 
+/* qpam_ce_partial and qpam_ce_finalize of an unsharded w in one call (N > 0), without the row statistics in between;
+ * loss[0] = loss_sum / denom.  Any output may be NULL except lse. */
+int qpam_ce_loss(const qpam_ce_args* args, float* lse, float* loss, float* per_token, float* denom,
+                 float* loss_sum, float* correct, float* tokens, void* stream);
+
 /* Gradients: dh [N,F], dw [V,F] (io_dtype) of  grad_scale[0] * loss_sum / denom[0]
  * given lse from qpam_ce_finalize.  grad_scale and denom are device scalars. */
 int qpam_ce_bwd(const qpam_ce_args* args, const float* lse, const float* grad_scale,

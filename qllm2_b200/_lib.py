@@ -10,6 +10,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libqllm2_pam_b200.so")
+HOST_PATH = os.path.join(HERE, "_host.so")
 
 QPAM_F32, QPAM_BF16 = 0, 1
 MAX_STATES = 4
@@ -87,6 +88,7 @@ SIGNATURES = {
     "qpam_ce_partial": (c_int32, [C.POINTER(CEArgs), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "qpam_ce_finalize": (c_int32, [C.POINTER(CEArgs), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                    c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "qpam_ce_loss": (c_int32, [C.POINTER(CEArgs)] + [c_void_p] * 8),
     "qpam_ce_bwd": (c_int32, [C.POINTER(CEArgs), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "qpam_ce_bwd_overlap": (c_int32, [C.POINTER(CEArgs), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                       c_void_p]),
@@ -163,6 +165,26 @@ def lib() -> C.CDLL:
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host runtime (_host.so, built beside the library): whole calls of the hot path -- checks, allocation,
+    autograd nodes, launches -- without the interpreter in between."""
+    global _host
+    if _host is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries must be loaded first)
+        if not os.path.exists(HOST_PATH):
+            raise QPamError(f"{HOST_PATH} is missing: build it with `python -m qllm2_b200.build`")
+        lib()
+        spec = importlib.util.spec_from_file_location("qllm2_b200._host", HOST_PATH)
+        _host = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_host)
+    return _host
 
 
 def check(rc: int, what: str) -> None:

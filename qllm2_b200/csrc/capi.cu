@@ -39,6 +39,30 @@ int sm_count() {
   return cached[dev];
 }
 
+int allow_smem(const void* kernel, size_t bytes) {
+  struct Entry {
+    const void* kernel;
+    int device;
+    size_t bytes;
+  };
+  static std::mutex mu;
+  static std::vector<Entry> seen;
+  if (bytes <= 48 * 1024) return QPAM_OK;
+  int dev = 0;
+  QPAM_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  for (auto& e : seen)
+    if (e.kernel == kernel && e.device == dev) {
+      if (e.bytes >= bytes) return QPAM_OK;
+      QPAM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+      e.bytes = bytes;
+      return QPAM_OK;
+    }
+  QPAM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  seen.push_back({kernel, dev, bytes});
+  return QPAM_OK;
+}
+
 // ------------------------------------------------------------------ launch accounting
 static std::atomic<long long> g_launches{0};
 static std::atomic<bool> g_profiling{false};

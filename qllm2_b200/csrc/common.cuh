@@ -28,6 +28,10 @@ int sm_count();   // multiprocessors of the current device
     if (e__ != cudaSuccess) return ::qpam::cuda_fail(e__, #call);    \
   } while (0)
 
+// Opt-in of a kernel to `bytes` of dynamic shared memory, asked of the runtime once per kernel, size and device (the call
+// costs about as much as a third of a launch).
+int allow_smem(const void* kernel, size_t bytes);
+
 // Counts the launch and, while profiling is on, records an event behind it on `stream_`.
 void note_launch(const char* name, cudaStream_t stream_);
 // True while qpam_profile_begin .. qpam_profile_end is recording (entry points then keep to one stream).

@@ -1,0 +1,59 @@
+// Host runtime of the package: the per-call work around the C ABI (argument checks, allocation, autograd bookkeeping,
+// launch order) as native code.  A small scan is five kernels of 2..10 us; driven from Python its call took 170 us, of
+// which the interpreter, ctypes and the hand-over of the GIL to autograd's worker thread were about 110.
+#pragma once
+#include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include "qllm2_pam.h"
+
+namespace qhost {
+
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+// Turned into qllm2_b200._lib.QPamError by the module's exception translator.
+struct Error : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
+
+template <typename... Args>
+[[noreturn]] inline void fail(const Args&... args) {
+  throw Error(c10::str(args...));
+}
+#define QH_REQUIRE(cond, ...)                  \
+  do {                                         \
+    if (!(cond)) ::qhost::fail(__VA_ARGS__);   \
+  } while (0)
+
+inline void check(int rc, const char* what) {
+  if (rc != 0) fail(what, " failed with code ", rc, ": ", qpam_last_error());
+}
+
+inline void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
+inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+inline float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
+inline Tensor value(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
+
+inline int dtype_code(at::ScalarType t) {
+  if (t == at::kFloat) return QPAM_F32;
+  if (t == at::kBFloat16) return QPAM_BF16;
+  fail("unsupported dtype ", t, ": the PAM kernels take float32 or bfloat16");
+}
+inline Tensor workspace(size_t bytes, const Tensor& like) {
+  return at::empty({(int64_t)std::max<size_t>(bytes, 256)}, like.options().dtype(at::kByte));
+}
+inline Tensor f32(const Tensor& t) { return t.defined() ? t.to(at::kFloat).contiguous() : t; }
+inline bool needs_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
+inline std::string shape(const Tensor& t) { return c10::str(t.sizes()); }
+
+inline bool autocast_bf16() {
+  return at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) == at::kBFloat16;
+}
+
+void bind_scan(pybind11::module_& m);
+void bind_loss(pybind11::module_& m);
+
+}  // namespace qhost

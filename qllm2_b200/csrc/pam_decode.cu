@@ -241,7 +241,8 @@ template <typename T>
 static int launch_decode_bulk(const DecodeParams& p, cudaStream_t st) {
   const size_t smem = (size_t)p.K * DEC_BULK_STATE_BYTES;
   auto kern = k_decode_step_bulk<T>;
-  QPAM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int rc = allow_smem(reinterpret_cast<const void*>(kern), smem);
+  if (rc) return rc;
   kern<<<p.n * p.H, 256, smem, st>>>(p);
   QPAM_LAUNCH_CHECK("k_decode_step_bulk");
   return QPAM_OK;

@@ -152,10 +152,7 @@ static ScanParams make_params(const qpam_scan_args* a, const ScanLayout& L) {
 }
 
 template <typename KernelT>
-static int set_smem(KernelT kern, size_t bytes) {
-  if (bytes > 48 * 1024) QPAM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return QPAM_OK;
-}
+static int set_smem(KernelT kern, size_t bytes) { return allow_smem(reinterpret_cast<const void*>(kern), bytes); }
 
 template <int D>
 constexpr size_t outer_smem() { return sizeof(float2) * 2 * CH * (D + 1) + sizeof(float) * CH; }

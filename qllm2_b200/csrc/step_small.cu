@@ -1123,7 +1123,8 @@ __global__ void __launch_bounds__(ONE_THREADS, 1) k_step_one(const __grid_consta
 // ------------------------------------------------------------------------------------------------ host
 template <typename... Params, typename... Args>
 int launch_pdl(const char* name, void (*kern)(Params...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t st, Args... args) {
-  if (smem > 48 * 1024) QPAM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int rc = allow_smem(reinterpret_cast<const void*>(kern), smem);
+  if (rc) return rc;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
@@ -1218,7 +1219,8 @@ int launch_one(const qpam_step_args* a, const StepWs& w, cudaStream_t st) {
   QPAM_CUDA(cudaMemsetAsync(w.best, 0, (size_t)a->n * 8 + 256, st));
   void* args[] = {&p, &layers};
   auto kern = a->state_dtype == QPAM_F32 ? (const void*)k_step_one<float> : (const void*)k_step_one<bf16>;
-  QPAM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int rc = allow_smem(kern, smem);
+  if (rc) return rc;
   QPAM_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(ONE_THREADS), args, smem, st));
   QPAM_LAUNCH_CHECK("k_step_one");
   return QPAM_OK;

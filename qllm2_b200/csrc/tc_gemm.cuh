@@ -46,6 +46,7 @@ struct GemmParams {
   float *pm, *ps, *pt, *pbest;
   int32_t* pidx;
   int64_t stats_ld;         // = rows of the whole problem (partials are [split][rows])
+  unsigned int* zero_word;  // a counter of the next kernel, cleared here (or null)
   int64_t row_base;         // global row of tile row 0 of blockIdx.y == 0
   // EPI_PROBS
   __nv_bfloat16* pbuf;
@@ -115,6 +116,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
     // one read of the device error word for the whole CTA: every warp must take the same side of has_work
     // (the epilogue warps meet at a named barrier), whatever another CTA writes meanwhile
     *err_slot = (uint32_t) * reinterpret_cast<volatile int*>(&g_device_error);
+    if (EPI == EPI_STATS && p.zero_word && blockIdx.x == 0 && blockIdx.y == 0) *p.zero_word = 0u;
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);

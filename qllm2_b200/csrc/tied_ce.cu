@@ -10,7 +10,7 @@ static inline size_t dtype_size(int dt) { return dt == QPAM_BF16 ? 2 : 4; }
 struct CELayout {
   int32_t nsplit, tiles_per_split;
   int64_t ldp, chunk_rows;
-  size_t off_pm, off_ps, off_pt, off_pbest, off_pidx, total_fwd;
+  size_t off_pm, off_ps, off_pt, off_pbest, off_pidx, off_sums, total_fwd;   // off_sums: arrival counter, then four doubles per CTA of k_ce_rows
   size_t off_pbuf, off_dwacc, off_dhpart, total_bwd;
   CETcPlan tc;  // tensor-core path (bf16 inputs)
 };
@@ -36,6 +36,7 @@ static CELayout ce_layout(const qpam_ce_args* a) {
   L.off_pt = off; off += ce_align(n * 4);
   L.off_pbest = off; off += ce_align(n * 4);
   L.off_pidx = off; off += ce_align(n * 4);
+  L.off_sums = off; off += 256 + ce_align(((size_t)(a->N > 0 ? a->N : 1) + CE_ROWS - 1) / CE_ROWS * 4 * sizeof(double));
   L.total_fwd = off;
   L.ldp = (a->V + 7) & ~(int64_t)7;
   const size_t row_bytes = (size_t)L.ldp * dtype_size(a->io_dtype);
@@ -183,6 +184,37 @@ extern "C" int qpam_ce_partial(const qpam_ce_args* a, float* row_max, float* row
   }
   return a->io_dtype == QPAM_BF16 ? ce_partial_t<__nv_bfloat16>(a, L, row_max, row_sumexp, row_tgt, row_argmax, st)
                                   : ce_partial_t<float>(a, L, row_max, row_sumexp, row_tgt, row_argmax, st);
+}
+
+extern "C" int qpam_ce_loss(const qpam_ce_args* a, float* lse, float* loss, float* per_token, float* denom, float* loss_sum, float* correct,
+                            float* tokens, void* stream) {
+  int rc = check_ce_args(a, true);
+  if (rc) return rc;
+  QPAM_REQUIRE(lse != nullptr && a->N > 0, "ce loss: lse must not be NULL, N must be positive");
+  const CELayout L = ce_layout(a);
+  if (a->workspace_bytes < L.total_fwd) {
+    set_error("ce loss: workspace %zu bytes < required %zu", a->workspace_bytes, L.total_fwd);
+    return QPAM_EWORKSPACE;
+  }
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  char* ws = reinterpret_cast<char*>(a->workspace);
+  unsigned int* arrived = reinterpret_cast<unsigned int*>(ws + L.off_sums);
+  CEParams p = ce_params(a, L);
+  if (tc_usable(a, L)) {
+    p.nsplit = L.tc.nsplit;
+    rc = ce_tc_partial(a, L.tc, tc_buffers(a, L), st, arrived);
+    if (rc) return rc;
+  } else {
+    QPAM_CUDA(cudaMemsetAsync(arrived, 0, sizeof(*arrived), st));
+    const dim3 grid(L.nsplit, (unsigned)((a->N + CE_TM - 1) / CE_TM));
+    if (a->io_dtype == QPAM_BF16) k_ce_partial<__nv_bfloat16><<<grid, 256, 0, st>>>(p);
+    else k_ce_partial<float><<<grid, 256, 0, st>>>(p);
+    QPAM_LAUNCH_CHECK("k_ce_partial");
+  }
+  k_ce_rows<<<(unsigned)((a->N + CE_ROWS - 1) / CE_ROWS), 256, 0, st>>>(p, lse, loss, per_token, denom, loss_sum, correct, tokens,
+                                                                         reinterpret_cast<double*>(ws + L.off_sums + 256), arrived);
+  QPAM_LAUNCH_CHECK("k_ce_rows");
+  return QPAM_OK;
 }
 
 extern "C" int qpam_ce_finalize(const qpam_ce_args* a, const float* row_max, const float* row_sumexp,

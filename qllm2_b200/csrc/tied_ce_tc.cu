@@ -7,10 +7,7 @@
 namespace qpam {
 
 template <typename K>
-static int opt_in_smem(K kern, size_t bytes) {
-  QPAM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return QPAM_OK;
-}
+static int opt_in_smem(K kern, size_t bytes) { return allow_smem(reinterpret_cast<const void*>(kern), bytes); }
 
 // Launch a kernel of CTA pairs: clusters of two CTAs along x (pair_axis 0) or y (pair_axis 1).
 template <typename... KArgs, typename... Args>
@@ -93,7 +90,7 @@ static int probs_tiles_per_cta(int64_t row_tiles, int n_tiles) {
 }
 
 // ------------------------------------------------------------------ forward statistics
-int ce_tc_partial(const qpam_ce_args* a, const CETcPlan& pl, const CETcBuffers& b, cudaStream_t st) {
+int ce_tc_partial(const qpam_ce_args* a, const CETcPlan& pl, const CETcBuffers& b, cudaStream_t st, unsigned int* zero_word) {
   CUtensorMap tmH, tmW;
   int rc = make_map(&tmH, a->h, a->F, a->N, a->F, tc::BK, tc::BM);
   if (rc) return rc;
@@ -108,6 +105,7 @@ int ce_tc_partial(const qpam_ce_args* a, const CETcPlan& pl, const CETcBuffers& 
   p.targets = a->targets; p.v_offset = a->v_offset; p.ignore_index = a->ignore_index;
   p.pm = b.pm; p.ps = b.ps; p.pt = b.pt; p.pbest = b.pbest; p.pidx = b.pidx;
   p.stats_ld = a->N; p.row_base = 0;
+  p.zero_word = zero_word;
   // CTA pairs (cta_group::2): two row tiles share one 256-column B tile, each CTA loading half of it
   auto kern = tc::k_tc_gemm<256, tc::EPI_STATS, false, false, 1, true>;
   using CfgP = tc::Cfg<256, 1, true>;

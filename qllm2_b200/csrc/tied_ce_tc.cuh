@@ -26,7 +26,8 @@ struct CETcBuffers {
 };
 
 // per-row partial statistics [nsplit][N] via the tensor-core logits GEMM
-int ce_tc_partial(const qpam_ce_args* a, const CETcPlan& plan, const CETcBuffers& b, cudaStream_t st);
+// zero_word: a counter of the next kernel, cleared by this one (or null)
+int ce_tc_partial(const qpam_ce_args* a, const CETcPlan& plan, const CETcBuffers& b, cudaStream_t st, unsigned int* zero_word = nullptr);
 // out[N][ld] (bf16) = h w^T through the same GEMM, tiles stored by TMA (ld a multiple of 8, out 16-byte aligned)
 int ce_tc_logits(const qpam_ce_args* a, const CETcPlan& plan, void* out, int64_t ld, cudaStream_t st);
 // dH, dW via recomputed probabilities (bf16 tiles) and two tensor-core GEMMs per row chunk

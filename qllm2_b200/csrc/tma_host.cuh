@@ -33,6 +33,16 @@ static inline int make_map(CUtensorMap* m, const void* base, int64_t inner, int6
     set_error("cuTensorMapEncodeTiled is not available from the CUDA driver");
     return QPAM_ECUDA;
   }
+  // the encoder is a driver call and wants the device's context current; a thread that has only been given a device (an
+  // autograd worker) gets it from the runtime here
+  static thread_local int bound = -1;
+  int dev = 0;
+  QPAM_CUDA(cudaGetDevice(&dev));
+  if (dev != bound) {
+    QPAM_CUDA(cudaSetDevice(dev));
+    QPAM_CUDA(cudaFree(nullptr));
+    bound = dev;
+  }
   QPAM_REQUIRE(((uintptr_t)base & 15) == 0 && (row_stride * 2) % 16 == 0, "TMA operand is not 16-byte aligned");
   cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
   cuuint64_t strides[1] = {(cuuint64_t)row_stride * 2};

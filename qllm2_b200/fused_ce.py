@@ -17,7 +17,7 @@ from typing import Optional
 
 import torch
 
-from . import ops
+from . import _lib, ops
 
 
 def _combine_stats(stats, group):
@@ -50,7 +50,9 @@ def _comm_stream(device):
     return _COMM_STREAMS[key]
 
 
-class _FusedLinearCE(torch.autograd.Function):
+class _ShardedLinearCE(torch.autograd.Function):
+    """The vocabulary-parallel form; one GPU's whole head is a native node (csrc/host/loss.cpp)."""
+
     @staticmethod
     def forward(ctx, hidden_rows, weight_matrix, targets, mask, ignore_index, group, vocab_start):
         h = hidden_rows.contiguous()
@@ -65,9 +67,7 @@ class _FusedLinearCE(torch.autograd.Function):
         if ctx.empty:   # nothing to launch; the reference returns 0 / clamp_min(1) = 0
             ctx.save_for_backward(h, w)
             return torch.zeros((), dtype=torch.float32, device=h.device)
-        stats = ops.ce_row_stats(h, w, targets, ignore_index=ignore_index, v_offset=vocab_start)
-        if group is not None:
-            stats = _combine_stats(stats, group)
+        stats = _combine_stats(ops.ce_row_stats(h, w, targets, ignore_index=ignore_index, v_offset=vocab_start), group)
         fin = ops.ce_finalize(h, w, targets, maskf, stats, ignore_index=ignore_index)
         loss = (fin["loss_sum"] / fin["denom"]).reshape(())
         ctx.save_for_backward(h, w, targets, maskf, fin["lse"], fin["denom"])
@@ -82,19 +82,16 @@ class _FusedLinearCE(torch.autograd.Function):
         h, w, targets, maskf, lse, denom = ctx.saved_tensors
         ignore_index, group, vocab_start, h_dtype, w_dtype = ctx.cfg
         gs = grad_output.detach().float().reshape(1).contiguous()
-        if group is None:
-            dh, dw = ops.ce_backward(h, w, targets, maskf, lse, gs, denom, ignore_index=ignore_index, v_offset=vocab_start)
-        else:
-            # dH of the shards is summed over the group on a side stream that the library releases as soon as dH
-            # is complete: the exchange runs under the dW products, which stay local to the shard
-            import torch.distributed as dist
-            cur, comm = torch.cuda.current_stream(h.device), _comm_stream(h.device)
-            dh, dw = ops.ce_backward(h, w, targets, maskf, lse, gs, denom, ignore_index=ignore_index, v_offset=vocab_start,
-                                     dh_ready_stream=comm)
-            with torch.cuda.stream(comm):
-                dist.all_reduce(dh, op=dist.ReduceOp.SUM, group=group)
-            dh.record_stream(comm)
-            cur.wait_stream(comm)
+        # dH of the shards is summed over the group on a side stream that the library releases as soon as dH
+        # is complete: the exchange runs under the dW products, which stay local to the shard
+        import torch.distributed as dist
+        cur, comm = torch.cuda.current_stream(h.device), _comm_stream(h.device)
+        dh, dw = ops.ce_backward(h, w, targets, maskf, lse, gs, denom, ignore_index=ignore_index, v_offset=vocab_start,
+                                 dh_ready_stream=comm)
+        with torch.cuda.stream(comm):
+            dist.all_reduce(dh, op=dist.ReduceOp.SUM, group=group)
+        dh.record_stream(comm)
+        cur.wait_stream(comm)
         return dh.to(h_dtype), dw.to(w_dtype), None, None, None, None, None
 
 
@@ -110,27 +107,25 @@ def fused_linear_cross_entropy(
 ) -> torch.Tensor:
     """Mean cross-entropy of (hidden_rows @ weight_matrix.T) vs targets (fp32 0-dim tensor)."""
     del chunk
-    return _FusedLinearCE.apply(hidden_rows, weight_matrix, targets, mask, ignore_index, group, vocab_start)
+    if mask is not None and mask.numel() != hidden_rows.shape[0]:
+        raise ValueError("mask must have one entry per row of hidden_rows")
+    if group is not None or hidden_rows.shape[0] == 0:
+        return _ShardedLinearCE.apply(hidden_rows, weight_matrix, targets, mask, ignore_index, group, vocab_start)
+    return _lib.host().linear_ce(hidden_rows, weight_matrix, targets, mask, ignore_index, vocab_start)
 
 
 @torch.no_grad()
 def linear_ce_per_token(hidden_rows, weight_matrix, targets, chunk: int = 4096, ignore_index: int = -100):
     """Detached per-row cross-entropy [N]; rows whose target is ignore_index give 0.0."""
     del chunk
-    h, w = hidden_rows.contiguous(), weight_matrix.contiguous().to(hidden_rows.dtype)
-    stats = ops.ce_row_stats(h, w, targets.contiguous(), ignore_index=ignore_index)
-    fin = ops.ce_finalize(h, w, targets.contiguous(), None, stats, ignore_index=ignore_index)
-    return fin["per_token"].to(hidden_rows.dtype)
+    rows, _ = _lib.host().linear_ce_rows(hidden_rows, weight_matrix, targets, None, ignore_index)
+    return rows.to(hidden_rows.dtype)
 
 
 @torch.no_grad()
 def linear_ce_stats(hidden_rows, weight_matrix, targets, mask=None, chunk: int = 4096, ignore_index: int = -100):
     """(loss_sum, correct, tokens) as Python floats, without materialising logits."""
     del chunk
-    h, w = hidden_rows.contiguous(), weight_matrix.contiguous().to(hidden_rows.dtype)
-    targets = targets.contiguous()
-    maskf = None if mask is None else mask.float().contiguous()
-    stats = ops.ce_row_stats(h, w, targets, ignore_index=ignore_index)
-    fin = ops.ce_finalize(h, w, targets, maskf, stats, ignore_index=ignore_index)
-    vals = torch.cat([fin["loss_sum"], fin["correct"], fin["tokens"]]).tolist()
+    _, sums = _lib.host().linear_ce_rows(hidden_rows, weight_matrix, targets, mask, ignore_index)
+    vals = sums.tolist()
     return vals[0], vals[1], vals[2]

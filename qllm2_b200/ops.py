@@ -41,142 +41,6 @@ def _scan_args(q, k, v, gamma, coef, s0, cu_seqlens, y, s_final, q_scale, eps, c
     return a
 
 
-class _PamScanFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, gamma, coef, s0, cu_seqlens, q_scale, eps, chunk, save_states):
-        L = _lib.lib()
-        _require_cuda(q, k, v, gamma)
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        gamma = gamma.float().contiguous()
-        coef = None if coef is None else coef.float().contiguous()
-        s0 = None if s0 is None else s0.float().contiguous()
-        B, H, T, d = q.shape[:4]
-        K = gamma.shape[0]
-        S = B if cu_seqlens is None else cu_seqlens.numel() - 1
-        y = torch.empty_like(q)
-        s_final = torch.empty(K, S, H, d, d, 2, dtype=torch.float32, device=q.device)
-        need_bwd = any(t is not None and t.requires_grad for t in (q, k, v, gamma, coef, s0))
-        a = _scan_args(q, k, v, gamma, coef, s0, cu_seqlens, y, s_final, q_scale, eps, chunk)
-        nbytes = L.qpam_scan_workspace_bytes(C.byref(a), 1 if (need_bwd and save_states) else 0)
-        ws = _workspace(nbytes, q.device)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-        check(L.qpam_scan_fwd(C.byref(a), stream_ptr()), "qpam_scan_fwd")
-        ctx.save_for_backward(q, k, v, gamma, coef, s0, cu_seqlens, ws if (need_bwd and save_states) else None)
-        ctx.cfg = (q_scale, eps, chunk)
-        ctx.set_materialize_grads(False)
-        return y, s_final
-
-    @staticmethod
-    def backward(ctx, dy, ds_final):
-        L = _lib.lib()
-        q, k, v, gamma, coef, s0, cu_seqlens, ws = ctx.saved_tensors
-        q_scale, eps, chunk = ctx.cfg
-        dy = torch.zeros_like(q) if dy is None else dy.contiguous().to(q.dtype)
-        if dy.shape != q.shape:
-            raise _lib.QPamError(f"dy shape {tuple(dy.shape)} != y shape {tuple(q.shape)}")
-        if ds_final is not None and ds_final.numel() != gamma.shape[0] * (q.shape[0] if cu_seqlens is None else cu_seqlens.numel() - 1) * q.shape[1] * q.shape[3] ** 2 * 2:
-            raise _lib.QPamError("ds_final has the wrong number of elements")
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        dgamma = torch.empty_like(gamma)
-        dcoef = torch.empty_like(coef) if coef is not None else None
-        ds0 = torch.empty_like(s0) if (s0 is not None and ctx.needs_input_grad[5]) else None
-        if ds_final is not None:
-            ds_final = ds_final.float().contiguous()
-        a = _scan_args(q, k, v, gamma, coef, s0, cu_seqlens, None, None, q_scale, eps, chunk)
-        states_valid = 1
-        if ws is None:
-            ws = _workspace(L.qpam_scan_workspace_bytes(C.byref(a), 1), q.device)
-            states_valid = 0
-        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-        check(L.qpam_scan_bwd(C.byref(a), ptr(dy), ptr(dq), ptr(dk), ptr(dv), ptr(dgamma), ptr(dcoef),
-                              ptr(ds_final), ptr(ds0), states_valid, stream_ptr()), "qpam_scan_bwd")
-        return dq, dk, dv, dgamma, dcoef, ds0, None, None, None, None, None
-
-
-class _PamScanStatesFn(torch.autograd.Function):
-    """K single-state scans over the same q, k, v (bf16, d = 64: the tensor-core kernels), one per decay row of
-    `gamma` [K,B,H,T]: returns the per-state outputs ys [K,B,H,T,d,2] and final states [K,S,H,d,d,2].  The
-    backward runs the K backward scans into ONE set of dq, dk, dv buffers: the first writes, the others add
-    (qpam_scan_bwd_accumulate), so the sum over the states costs no extra pass."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, gamma, s0, cu_seqlens, q_scale, eps, chunk):
-        L = _lib.lib()
-        _require_cuda(q, k, v, gamma)
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        gamma = gamma.float().contiguous()
-        s0 = None if s0 is None else s0.float().contiguous()
-        B, H, T, d = q.shape[:4]
-        K = gamma.shape[0]
-        S = B if cu_seqlens is None else cu_seqlens.numel() - 1
-        ys = torch.empty((K,) + tuple(q.shape), dtype=q.dtype, device=q.device)
-        s_final = torch.empty(K, S, H, d, d, 2, dtype=torch.float32, device=q.device)
-        need_bwd = any(t is not None and t.requires_grad for t in (q, k, v, gamma, s0))
-        if 2 <= K <= 4 and T > 0:
-            # one call: the chunk sums of all states from one pass over k and v, one carry launch, then the output
-            # kernel per state; the workspace keeps every state's chunk states for the per-state backward calls
-            a = _scan_args(q, k, v, gamma, None, s0, cu_seqlens, None, s_final, q_scale, eps, chunk)
-            ws = _workspace(L.qpam_scan_workspace_bytes(C.byref(a), 1 if need_bwd else 0), q.device)
-            a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-            check(L.qpam_scan_fwd_states(C.byref(a), ptr(ys), stream_ptr()), "qpam_scan_fwd_states")
-            ctx.save_for_backward(q, k, v, gamma, s0, cu_seqlens, *([ws] if need_bwd else []))
-            ctx.cfg = (q_scale, eps, chunk, need_bwd)
-            ctx.shared = True
-            ctx.set_materialize_grads(False)
-            return ys, s_final
-        ctx.shared = False
-        wss = []
-        for kk in range(K):
-            a = _scan_args(q, k, v, gamma[kk:kk + 1], None, None if s0 is None else s0[kk:kk + 1], cu_seqlens, ys[kk],
-                           s_final[kk:kk + 1], q_scale, eps, chunk)
-            ws = _workspace(L.qpam_scan_workspace_bytes(C.byref(a), 1 if need_bwd else 0), q.device)
-            a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-            check(L.qpam_scan_fwd(C.byref(a), stream_ptr()), "qpam_scan_fwd")
-            wss.append(ws if need_bwd else None)
-        ctx.save_for_backward(q, k, v, gamma, s0, cu_seqlens, *[w_ for w_ in wss if w_ is not None])
-        ctx.cfg = (q_scale, eps, chunk, need_bwd)
-        ctx.set_materialize_grads(False)
-        return ys, s_final
-
-    @staticmethod
-    def backward(ctx, dys, ds_final):
-        L = _lib.lib()
-        q, k, v, gamma, s0, cu_seqlens, *wss = ctx.saved_tensors
-        q_scale, eps, chunk, _ = ctx.cfg
-        K = gamma.shape[0]
-        dys = torch.zeros((K,) + tuple(q.shape), dtype=q.dtype, device=q.device) if dys is None else dys.contiguous().to(q.dtype)
-        if dys.shape != (K,) + tuple(q.shape):
-            raise _lib.QPamError(f"dys shape {tuple(dys.shape)} != ys shape {(K,) + tuple(q.shape)}")
-        if ds_final is not None:
-            ds_final = ds_final.float().contiguous()
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        dgamma = torch.empty_like(gamma)
-        ds0 = torch.empty_like(s0) if (s0 is not None and ctx.needs_input_grad[4]) else None
-        if ctx.shared:
-            a = _scan_args(q, k, v, gamma, None, s0, cu_seqlens, None, None, q_scale, eps, chunk)
-            a.workspace, a.workspace_bytes = wss[0].data_ptr(), wss[0].numel()
-            for kk in range(K):
-                dsf = None if ds_final is None else ds_final[kk:kk + 1]
-                d0 = None if ds0 is None else ds0[kk:kk + 1]
-                check(L.qpam_scan_bwd_state(C.byref(a), kk, ptr(dys[kk]), ptr(dq), ptr(dk), ptr(dv), ptr(dgamma[kk:kk + 1]),
-                                            ptr(dsf), ptr(d0), 1 if kk > 0 else 0, stream_ptr()), "qpam_scan_bwd_state")
-            return dq, dk, dv, dgamma, ds0, None, None, None, None
-        for kk in range(K):
-            a = _scan_args(q, k, v, gamma[kk:kk + 1], None, None if s0 is None else s0[kk:kk + 1], cu_seqlens, None, None,
-                           q_scale, eps, chunk)
-            ws = wss[kk]
-            a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-            dsf = None if ds_final is None else ds_final[kk:kk + 1]
-            d0 = None if ds0 is None else ds0[kk:kk + 1]
-            if kk == 0:
-                check(L.qpam_scan_bwd(C.byref(a), ptr(dys[kk]), ptr(dq), ptr(dk), ptr(dv), ptr(dgamma[kk:kk + 1]), None,
-                                      ptr(dsf), ptr(d0), 1, stream_ptr()), "qpam_scan_bwd")
-            else:
-                check(L.qpam_scan_bwd_accumulate(C.byref(a), ptr(dys[kk]), ptr(dq), ptr(dk), ptr(dv), ptr(dgamma[kk:kk + 1]),
-                                                 ptr(dsf), ptr(d0), 1, stream_ptr()), "qpam_scan_bwd_accumulate")
-        return dq, dk, dv, dgamma, ds0, None, None, None, None
-
-
 def pam_scan(q, k, v, gamma, *, coef=None, s0=None, cu_seqlens=None, head_dim: Optional[int] = None,
              eps: float = GAMMA_EPS, chunk: int = 64, save_states: bool = True, token_major: bool = False):
     """Chunked dual-form PAM scan on the GPU.  (token_major=True returns y as [B, T, H*d, 2], the head merge
@@ -187,81 +51,26 @@ def pam_scan(q, k, v, gamma, *, coef=None, s0=None, cu_seqlens=None, head_dim: O
     gamma    [B,H,T] or [K,B,H,T] decay in (0,1];  coef optional [K,B,H,T,2] read-out weights
     s0       optional [K,S,H,d,d,2] initial state;  cu_seqlens optional int32 [S+1] (then B == 1)
     Returns (y [B,H,T,d,2] in q's dtype, s_final float32 [K,S,H,d,d,2]).
+
+    Checks, autograd node and launches are native (csrc/host/scan.cpp).  K > 1 states in bf16 at d = 64 with gradients:
+    y = sum_k c_k y^(k), where y^(k) is the single-state scan with decay gamma^(k) on the same q, k, v (the fused K-state form
+    of the reference, v11/model.py:657-781, is algebraically this sum), as one node whose backward accumulates dq, dk, dv of
+    the states in place.
     """
-    # one dtype for the token tensors: under bf16 autocast the reference's matmuls round their inputs to
-    # bf16 anyway, so mixed fp32/bf16 operands (RoPE promotes q and k to fp32) are taken as bf16;
-    # otherwise they are promoted to the widest dtype present.  The C ABI reads all three through
-    # q's dtype, so they must agree before the pointers are handed over.
-    if torch.is_autocast_enabled() and torch.get_autocast_dtype("cuda") == torch.bfloat16:
-        io = torch.bfloat16
-    else:
-        io = torch.promote_types(torch.promote_types(q.dtype, k.dtype), v.dtype)
-    q, k, v = q.to(io), k.to(io), v.to(io)
-    if not (q.shape == k.shape == v.shape and q.dim() == 5 and q.shape[-1] == 2):
-        raise _lib.QPamError(f"q, k, v must share one shape [B,H,T,d,2]; got {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}")
-    B_, H_, T_ = q.shape[:3]
+    y, s = _lib.host().pam_scan(q, k, v, gamma, coef, s0, cu_seqlens, head_dim or 0, eps, chunk, save_states, token_major)
+    if y is not None:
+        return y, s
+    # K tensor-core states recomputed in the backward: one scan per state, autograd sums the gradients
     gamma = gamma.float()
-    if gamma.dim() == 3:
-        gamma = gamma.unsqueeze(0)
-    if gamma.shape[1:] != (B_, H_, T_):
-        raise _lib.QPamError(f"gamma shape {tuple(gamma.shape)} does not match q {tuple(q.shape)}")
-    if coef is not None:
-        coef = coef.float()
-        if coef.dim() == 4:
-            coef = coef.unsqueeze(0)
-    if coef is not None and coef.shape != gamma.shape + (2,):
-        raise _lib.QPamError(f"coef shape {tuple(coef.shape)} != gamma shape + (2,)")
-    n_seq = B_ if cu_seqlens is None else cu_seqlens.numel() - 1
-    if s0 is not None:
-        s0 = s0.float()
-        if s0.shape != (gamma.shape[0], n_seq, H_, q.shape[3], q.shape[3], 2):
-            raise _lib.QPamError(f"s0 shape {tuple(s0.shape)} != [K,S,H,d,d,2]")
-    if cu_seqlens is not None and B_ != 1:
-        raise _lib.QPamError("packed mode (cu_seqlens) needs B == 1")
-    d = q.shape[3]
-    head_dim = d if head_dim is None else head_dim
-    if cu_seqlens is not None:
-        if not cu_seqlens.is_cuda:
-            # a host descriptor is checked here (the kernels check a device descriptor themselves and report
-            # through the status word, see _lib.device_status)
-            c = cu_seqlens.to(torch.int64)
-            if c.numel() < 2 or int(c[0]) != 0 or bool((c[1:] < c[:-1]).any()) or int(c[-1]) > T_:
-                raise _lib.QPamError(f"cu_seqlens must start at 0, never decrease and end at or before T={T_}; got {c.tolist()[:8]}...")
-        cu_seqlens = cu_seqlens.to(device=q.device, dtype=torch.int32).contiguous()
-    K = gamma.shape[0]
-    needs_grad = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (q, k, v, gamma, coef, s0))
-    if K > 1 and q.dtype == torch.bfloat16 and d == 64 and needs_grad:
-        # Phase-routed K-state scan on the tensor-core kernels: y = sum_k c_k y^(k), where y^(k) is the
-        # single-state scan with decay gamma^(k) on the same q, k, v (the fused K-state form of the
-        # reference, v11/model.py:657-781, is algebraically this sum).  autograd composes the backward:
-        # K single-state backward scans with upstream conj(c_k) dy, and dc_k = <dy, y^(k)>.  With the chunk states kept
-        # for the backward (save_states) the K scans share one autograd node whose backward accumulates dq, dk, dv in
-        # place (qpam_scan_bwd_accumulate) instead of leaving K partial gradients for autograd to add.
-        if save_states:
-            ys_all, finals = _PamScanStatesFn.apply(q, k, v, gamma, s0, cu_seqlens, head_dim ** -0.5, eps, chunk)
-            if coef is not None:
-                from .fused_elementwise import state_combine_stacked
-                return state_combine_stacked(coef, ys_all, token_major=token_major), finals
-            y = ys_all.sum(dim=0)
-            return (_merge_heads(y) if token_major else y), finals
-        ys, finals = [], []
-        for kk in range(K):        # states recomputed in the backward: one scan per state, autograd sums the gradients
-            yk, sk = _PamScanFn.apply(q, k, v, gamma[kk:kk + 1], None, None if s0 is None else s0[kk:kk + 1],
-                                      cu_seqlens, head_dim ** -0.5, eps, chunk, save_states)
-            ys.append(yk)
-            finals.append(sk)
-        if coef is None:
-            y = ys[0]
-            for yk in ys[1:]:
-                y = y + yk
-        else:
-            from .fused_elementwise import state_combine
-            return state_combine(coef, ys, token_major=token_major), torch.cat(finals, dim=0)
+    ys, finals = zip(*(pam_scan(q, k, v, gamma[kk:kk + 1], s0=None if s0 is None else s0[kk:kk + 1], cu_seqlens=cu_seqlens, head_dim=head_dim,
+                                eps=eps, chunk=chunk, save_states=False) for kk in range(gamma.shape[0])))
+    if coef is None:
+        y = ys[0]
+        for yk in ys[1:]:
+            y = y + yk
         return (_merge_heads(y) if token_major else y), torch.cat(finals, dim=0)
-    if token_major and not needs_grad:
-        return pam_scan_tokens(q, k, v, gamma, coef=coef, s0=s0, cu_seqlens=cu_seqlens, head_dim=head_dim, eps=eps, chunk=chunk)
-    y, s = _PamScanFn.apply(q, k, v, gamma, coef, s0, cu_seqlens, head_dim ** -0.5, eps, chunk, save_states)
-    return (_merge_heads(y) if token_major else y), s
+    from .fused_elementwise import state_combine
+    return state_combine(coef.float(), ys, token_major=token_major), torch.cat(finals, dim=0)
 
 
 def _merge_heads(y):
@@ -311,37 +120,7 @@ def pam_scan_tokens(q, k, v, gamma, coef=None, s0=None, cu_seqlens=None, *, head
     """Inference form of `pam_scan`: same arguments, but Y comes back token-major, [B, T, H*d, 2] -- the layout
     the output projection reads (the head merge of v11/model.py:835-836) -- and nothing is kept for a backward
     pass (K phase-routed states in bf16 at d = 64 then run the fused K-state output kernel)."""
-    B, H, T, d = q.shape[:4]
-    gamma4 = gamma if gamma.dim() == 4 else gamma.unsqueeze(0)
-    K = gamma4.shape[0]
-    direct = (q.is_cuda and d == 64 and q.dtype == k.dtype == v.dtype == torch.bfloat16 and T > 0
-              and (K > 1 or coef is None) and tuple(gamma4.shape) == (K, B, H, T)
-              and q.shape == k.shape == v.shape and (cu_seqlens is None or B == 1))
-    if not direct:
-        y, s = pam_scan(q, k, v, gamma, coef=coef, s0=s0, cu_seqlens=cu_seqlens, head_dim=head_dim, eps=eps, chunk=chunk)
-        return y.transpose(1, 2).reshape(B, T, H * d, 2), s
-    # tensor-core path: the output kernel writes [B,T,H,d,2] itself
-    L = _lib.lib()
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    gamma4 = gamma4.float().contiguous()
-    if coef is not None:
-        if tuple(coef.shape) != (K, B, H, T, 2):
-            raise _lib.QPamError(f"coef must be [K,B,H,T,2] = {(K, B, H, T, 2)}, got {tuple(coef.shape)}")
-        coef = coef.float().contiguous()
-    if cu_seqlens is not None:
-        cu_seqlens = cu_seqlens.to(device=q.device, dtype=torch.int32).contiguous()
-    S = B if cu_seqlens is None else cu_seqlens.numel() - 1
-    if s0 is not None:
-        if s0.numel() != K * S * H * d * d * 2:
-            raise _lib.QPamError(f"s0 must be [K,S,H,d,d,2] = {(K, S, H, d, d, 2)}, got {tuple(s0.shape)}")
-        s0 = s0.float().contiguous()
-    y = torch.empty(B, T, H * d, 2, dtype=q.dtype, device=q.device)
-    s_final = torch.empty(K, S, H, d, d, 2, dtype=torch.float32, device=q.device)
-    a = _scan_args(q, k, v, gamma4, coef, s0, cu_seqlens, y, s_final, (d if head_dim is None else head_dim) ** -0.5, eps, chunk)
-    ws = _workspace(L.qpam_scan_workspace_bytes(C.byref(a), 0), q.device)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-    check(L.qpam_scan_fwd_tokens(C.byref(a), stream_ptr()), "qpam_scan_fwd_tokens")
-    return y, s_final
+    return _lib.host().pam_scan_tokens(q, k, v, gamma, coef, s0, cu_seqlens, head_dim or 0, eps, chunk)
 
 
 # --------------------------------------------------------------------------------------- decode
