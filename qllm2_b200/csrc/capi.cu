@@ -47,7 +47,7 @@ int allow_smem(const void* kernel, size_t bytes) {
   };
   static std::mutex mu;
   static std::vector<Entry> seen;
-  if (bytes <= 48 * 1024) return QPAM_OK;
+  if (bytes <= 32 * 1024) return QPAM_OK;     // (static shared memory counts towards the default limit of 48 KB too)
   int dev = 0;
   QPAM_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
