@@ -53,7 +53,12 @@ inline bool autocast_bf16() {
   return at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) == at::kBFloat16;
 }
 
+// Forward scan with token-major output [B,T,H*d,2] and the final states [K,S,H,d,d,2]; inputs contiguous, of the scan's dtypes.
+std::tuple<Tensor, Tensor> scan_tokens(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gamma, const Tensor& coef, const Tensor& s0,
+                                       const Tensor& cu, double q_scale);
+
 void bind_scan(pybind11::module_& m);
 void bind_loss(pybind11::module_& m);
+void bind_forward(pybind11::module_& m);
 
 }  // namespace qhost

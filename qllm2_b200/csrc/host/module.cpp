@@ -13,4 +13,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   qhost::bind_scan(m);
   qhost::bind_loss(m);
+  qhost::bind_forward(m);
 }

@@ -277,6 +277,11 @@ std::tuple<Tensor, Tensor> pam_scan_tokens(const Tensor& q, const Tensor& k, con
 
 }  // namespace
 
+std::tuple<Tensor, Tensor> scan_tokens(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gamma, const Tensor& coef, const Tensor& s0,
+                                       const Tensor& cu, double q_scale) {
+  return forward_only(Inputs{q, k, v, gamma, coef, s0, cu, q_scale}, 1e-6, 64, true);
+}
+
 void bind_scan(pybind11::module_& m) {
   namespace py = pybind11;
   m.def("pam_scan", &pam_scan, py::call_guard<py::gil_scoped_release>());

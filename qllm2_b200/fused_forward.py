@@ -53,6 +53,7 @@ class FusedForward:
         self.w_vocab = torch.cat([model.embed.embed_real.weight, model.embed.embed_imag.weight], -1).detach().to(self.dtype).contiguous()
         self.layers = [self.pack_block(blk, self.dtype) for blk in model.blocks]
         self._step_layers = None
+        self._native = _lib.host().Packed(self.D, self.H, self.d, self.K, self.layers, self.embed_scale, self.out_scale, self.rope)
 
     @staticmethod
     def unsupported_reason(model: V11LM) -> Optional[str]:
@@ -125,6 +126,10 @@ class FusedForward:
             bias_a.append(torch.zeros(pad, device=device))
         L.w_front = torch.cat([r.float() for r in rows_a], 0).to(T).contiguous()
         L.b_front = torch.cat([b.float() for b in bias_a], 0).to(T).contiguous()
+        if rows_m and (-sum(r.shape[0] for r in rows_m)) % 8:
+            pad = (-sum(r.shape[0] for r in rows_m)) % 8     # aligned output rows here too: a ragged width costs the GEMM its tensor-core kernels
+            rows_m.append(torch.zeros(pad, D, device=device))
+            bias_m.append(torch.zeros(pad, device=device))
         L.w_mag = torch.cat([r.float() for r in rows_m], 0).to(T).contiguous() if rows_m else None
         L.b_mag = torch.cat([b.float() for b in bias_m], 0).to(T).contiguous() if rows_m else None
         return L
@@ -208,6 +213,14 @@ class FusedForward:
         h = F.linear(xn.reshape(n, 2 * self.D), self.w_head_proj, self.b_head_proj).view(n, self.D, 2)
         h, _ = self._res_norm(h, None, None, self.head_norm_scale)
         return h
+
+    def prefill(self, ids, pool, slots, cu=None, positions=None, resumed=None):
+        """Absorb prompts: ids [B, T] (cu None: a prompt per row; otherwise the pieces of one packed row, cu int32 [S+1]) into the
+        states of `slots` int32 [S] of `pool` [n_slots, L, K, H, d, d, 2].  resumed float32 [S]: 1 for pieces that continue from
+        their slot's state.  Returns what `hidden` does.  (csrc/host/forward.cpp: the same launches as `hidden` around a scan,
+        ~15 per block; issuing them from Python took longer than the GPU needs for a few hundred tokens.)"""
+        emb = self.model.embed
+        return self._native.prefill(emb.embed_real.weight, emb.embed_imag.weight, ids, pool, slots, cu, positions, resumed)
 
     # ---------------------------------------------------------------------------------- decode step for few rows
     def step_supported(self, n: int) -> bool:

@@ -12,6 +12,7 @@ per-sequence RoPE positions.  New sequences are prefetched in one packed ragged 
 from __future__ import annotations
 
 from collections import deque
+from contextlib import contextmanager
 from dataclasses import dataclass, field
 from typing import Deque, Dict, List, Optional, Sequence
 
@@ -126,18 +127,16 @@ class SlotScheduler:
 
 
 # ------------------------------------------------------------------------------------ engine
-class _PrefillMix:
-    """Sequence mixing at prefill: the packed ragged scan; final states go to the sequences' slots."""
-    q_scale = 1.0     # the scan applies head_dim^-0.5 itself
-
-    def __init__(self, eng, cu, slots, s0_of=None):
-        self.eng, self.cu, self.slots, self.s0_of = eng, cu, slots, s0_of
-
-    def __call__(self, layer, q, k, v, gamma, coef):
-        y, s = ops.pam_scan_tokens(q, k, v, gamma, coef=coef, cu_seqlens=self.cu, head_dim=q.shape[3],
-                                   s0=None if self.s0_of is None else self.s0_of(layer))
-        ops.pam_pool_store(self.eng.pool, self.slots, s, layer=layer)
-        return y.view(q.shape[2], -1)
+@contextmanager
+def _captured():
+    """A graph whose capture the body begins on a stream of its own and this ends.  (torch.cuda.graph would also collect
+    garbage and hand every cached block back to the driver, which an engine beside other work then pays for twice.)"""
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        yield graph
+        graph.capture_end()
+    torch.cuda.current_stream().wait_stream(side)
 
 
 class _DecodeMix:
@@ -260,13 +259,7 @@ class ContinuousBatcher:
         meta[1, :-1] = torch.tensor([r.slot for r, _, _ in items], dtype=torch.int32)
         meta = meta.to(self.device)
         cu, slots = meta[0], meta[1, :-1]
-        s0_of = None
-        if any(st > 0 for _, st, _ in items):
-            resumed = torch.tensor([1.0 if st > 0 else 0.0 for _, st, _ in items], device=self.device)
-
-            def s0_of(layer):      # [K,S,H,d,d,2] float32; fresh sequences start from zero whatever the slot held
-                s = self.pool[slots.long(), layer].float() * resumed[:, None, None, None, None, None]
-                return s.permute(1, 0, 2, 3, 4, 5).contiguous()
+        resumed = torch.tensor([1.0 if st > 0 else 0.0 for _, st, _ in items], device=self.device) if any(st > 0 for _, st, _ in items) else None
         if self.sampling is not None:      # the penalty looks at the whole prompt: load the slots' histories
             self._hist[slots.long().repeat_interleave(count.to(self.device), output_size=n_tok), both[1]] = both[0]
             self._hist_len[slots.long()] = torch.tensor([st + take for _, st, take in items], dtype=torch.int32, device=self.device)
@@ -276,17 +269,24 @@ class ContinuousBatcher:
         else:
             pick_slots = slots
         if self.ff is not None:
-            xn = self.ff.hidden(ids, _PrefillMix(self, cu, slots, s0_of), positions=positions)
+            xn = self.ff.prefill(ids, self.pool, slots, cu, positions, resumed)
             nxt = self._pick(self.ff.head_hidden(xn[(cu[1:] - 1).long()]), pick_slots)
         else:
-            nxt = self._prefill_modules(ids, positions, cu, slots, s0_of, pick_slots)
+            nxt = self._prefill_modules(ids, positions, cu, slots, resumed, pick_slots)
         for (r, st, take), t in zip(items, nxt.tolist()):
             r.prefilled = st + take
             if not r.prefilling:
                 r.generated.append(int(t))
 
-    def _prefill_modules(self, ids, positions, cu, slots, s0_of=None, pick_slots=None):
+    def _prefill_modules(self, ids, positions, cu, slots, resumed=None, pick_slots=None):
         m = self.model
+
+        def s0_of(layer):      # [K,S,H,d,d,2] float32; fresh sequences start from zero whatever the slot held
+            if resumed is None:
+                return None
+            s = self.pool[slots.long(), layer].float() * resumed[:, None, None, None, None, None]
+            return s.permute(1, 0, 2, 3, 4, 5).contiguous()
+
         z = m.embed_norm(m.embed(ids))
         for li, blk in enumerate(m.blocks):
             z = z + blk.cgu(blk.norm1(z)) * blk.cgu_scale
@@ -294,7 +294,7 @@ class ContinuousBatcher:
             pam = blk.pam
             q, k, vprime, gamma, coef = pam.project_gated(xn, positions=positions)
             y, s = ops.pam_scan(q, k, vprime, gamma, coef=coef, cu_seqlens=cu, head_dim=pam.head_dim,
-                                s0=None if s0_of is None else s0_of(li))
+                                s0=s0_of(li))
             ops.pam_pool_store(self.pool, slots, s, layer=li)
             out = pam.o_proj(y.transpose(1, 2).contiguous().view(1, ids.shape[1], pam.inner_dim, 2))
             z = z + out * blk.pam_scale
@@ -308,13 +308,9 @@ class ContinuousBatcher:
         idle rows only (slot id -1, no state changes), then the capture, which records and does not execute."""
         if not self.cuda_graph or self._graph is not None:
             return
-        side = torch.cuda.Stream()
-        side.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(side):
+        with _captured() as graph:
             self._decode_tensors(self._g_ids, self._g_pos, torch.full_like(self._g_slots, -1))
-        torch.cuda.current_stream().wait_stream(side)
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph):
+            graph.capture_begin()
             self._g_out = self._decode_tensors(self._g_ids, self._g_pos, self._g_slots)
             # the next step's inputs, so that steps can follow one another without the host (`_decode` sets them anew)
             self._g_ids[:, 0].copy_(self._g_out)
@@ -457,19 +453,6 @@ class ContinuousBatcher:
 
 
 # ------------------------------------------------------------------------------------ V11LM.generate
-class _BatchPrefillMix:
-    """Sequence mixing at the prefill of `generate`: B equal-length rows, final states into slots 0..B-1."""
-    q_scale = 1.0
-
-    def __init__(self, pool, slots):
-        self.pool, self.slots = pool, slots
-
-    def __call__(self, layer, q, k, v, gamma, coef):
-        y, s = ops.pam_scan_tokens(q, k, v, gamma, coef=coef, head_dim=q.shape[3])
-        ops.pam_pool_store(self.pool, self.slots, s, layer=layer)
-        return y.view(q.shape[0] * q.shape[2], -1)
-
-
 class _PoolDecodeMix:
     def __init__(self, pool, slots, head_dim):
         self.pool, self.slots, self.q_scale = pool, slots, head_dim ** -0.5
@@ -520,7 +503,7 @@ def generate_fused(model: V11LM, input_ids, max_new_tokens, sample, eos_token_id
         return head(ff.hidden(ids, mix, positions=positions))
 
     out = input_ids.clone()
-    xn = ff.hidden(out, _BatchPrefillMix(pool, slots))
+    xn = ff.prefill(out, pool, slots)
     res = head(xn.view(B, T0, cfg.dim, 2)[:, -1])
     ids_buf = torch.zeros(B, 1, dtype=torch.long, device=dev)
     pos_buf = torch.zeros(B, 1, dtype=torch.long, device=dev)
@@ -541,8 +524,8 @@ def generate_fused(model: V11LM, input_ids, max_new_tokens, sample, eos_token_id
         if graph is None and i == 0:
             res = step(ids_buf, pos_buf)                                    # first step eagerly (warms every kernel up)
         elif graph is None:
-            graph = torch.cuda.CUDAGraph()                                  # capture records the step, it does not run it
-            with torch.cuda.graph(graph):
+            with _captured() as graph:                                      # capture records the step, it does not run it
+                graph.capture_begin()
                 g_res = step(ids_buf, pos_buf)
             graph.replay()
             res = g_res.clone()
