@@ -92,6 +92,11 @@ int qpam_scan_fwd(const qpam_scan_args* args, void* stream);
  * available where the tensor-core kernels run (bf16, d = 64), QPAM_EUNSUPPORTED otherwise. */
 int qpam_scan_fwd_tokens(const qpam_scan_args* args, void* stream);
 
+/* qpam_scan_fwd_tokens followed by qpam_pool_store of the final states, in one call and without the fp32 states in
+ * between: sequence s leaves its states in pool [n_slots,L,K,H,d,d,2] at slot_ids[s] (outside [0, n_slots): nowhere). */
+int qpam_scan_prefill(const qpam_scan_args* args, void* pool, int32_t state_dtype, int64_t n_slots, int32_t L,
+                      int32_t layer, const int32_t* slot_ids, void* stream);
+
 /* Forward scan with no workspace argument, for hosts that are not allowed to allocate device
  * memory: a server whose memory pool took the whole GPU at start-up, a sandboxed plugin, or a
  * latency-critical loop where cudaMalloc (which may synchronise the device) is forbidden.  The

@@ -57,6 +57,10 @@ inline bool autocast_bf16() {
 std::tuple<Tensor, Tensor> scan_tokens(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gamma, const Tensor& coef, const Tensor& s0,
                                        const Tensor& cu, double q_scale);
 
+// The same with the final states going straight to the slots of a state pool; false where the kernels do not offer it.
+bool scan_prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gamma, const Tensor& coef, const Tensor& s0, const Tensor& cu, double q_scale,
+                  const Tensor& pool, const Tensor& slots, int64_t layer, Tensor& y);
+
 void bind_scan(pybind11::module_& m);
 void bind_loss(pybind11::module_& m);
 void bind_forward(pybind11::module_& m);

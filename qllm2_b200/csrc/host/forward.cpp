@@ -108,10 +108,15 @@ class Packed {
       Tensor s0;
       if (resumed.defined())     // fresh sequences start from zero whatever their slot held
         s0 = (pool.select(1, (int64_t)li).index_select(0, slots_long).to(at::kFloat) * resumed.view({-1, 1, 1, 1, 1, 1})).transpose(0, 1).contiguous();
-      auto [y, s] = scan_tokens(q, k, v, gamma, coef, s0, cu, 1.0 / std::sqrt((double)d_));
-      check(qpam_pool_store(pool.data_ptr(), pool_code, n_slots, (int)L, (int)li, static_cast<int32_t*>(slots.data_ptr()), fptr(s), (int)s.size(1), (int)H_,
-                            (int)d_, (int)K_, st),
-            "qpam_pool_store");
+      const double q_scale = 1.0 / std::sqrt((double)d_);
+      Tensor y;
+      if (!scan_prefill(q, k, v, gamma, coef, s0, cu, q_scale, pool, slots, (int64_t)li, y)) {
+        Tensor s;
+        std::tie(y, s) = scan_tokens(q, k, v, gamma, coef, s0, cu, q_scale);
+        check(qpam_pool_store(pool.data_ptr(), pool_code, n_slots, (int)L, (int)li, static_cast<int32_t*>(slots.data_ptr()), fptr(s), (int)s.size(1), (int)H_,
+                              (int)d_, (int)K_, st),
+              "qpam_pool_store");
+      }
       const Tensor o = at::linear(y.view({N, 2 * inner}), l.w_o);
       const Tensor& next = li + 1 < layers_.size() ? layers_[li + 1].n1 : out_scale_;
       check(qpam_residual_cnorm_fwd(z.data_ptr(), o.data_ptr(), fptr(l.pam_scale), fptr(next), xn.data_ptr(), nullptr, code, N, (int)D_, 1e-6f, st),

@@ -282,6 +282,20 @@ std::tuple<Tensor, Tensor> scan_tokens(const Tensor& q, const Tensor& k, const T
   return forward_only(Inputs{q, k, v, gamma, coef, s0, cu, q_scale}, 1e-6, 64, true);
 }
 
+bool scan_prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gamma, const Tensor& coef, const Tensor& s0, const Tensor& cu, double q_scale,
+                  const Tensor& pool, const Tensor& slots, int64_t layer, Tensor& y) {
+  const int64_t B = q.size(0), H = q.size(1), T = q.size(2), d = q.size(3), K = gamma.size(0);
+  if (d != 64 || q.scalar_type() != at::kBFloat16 || T == 0 || (K == 1 && coef.defined())) return false;
+  y = at::empty({B, T, H * d, 2}, q.options());
+  qpam_scan_args a = scan_args(q, k, v, gamma, coef, s0, cu, y, Tensor(), {q_scale, 1e-6, 64});
+  Tensor ws = workspace(qpam_scan_workspace_bytes(&a, 0), q);
+  set_workspace(a, ws);
+  check(qpam_scan_prefill(&a, pool.data_ptr(), dtype_code(pool.scalar_type()), pool.size(0), (int)pool.size(1), (int)layer,
+                          static_cast<const int32_t*>(slots.data_ptr()), stream()),
+        "qpam_scan_prefill");
+  return true;
+}
+
 void bind_scan(pybind11::module_& m) {
   namespace py = pybind11;
   m.def("pam_scan", &pam_scan, py::call_guard<py::gil_scoped_release>());

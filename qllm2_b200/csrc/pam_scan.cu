@@ -234,6 +234,22 @@ static int tc_states(const ScanParams& p, const ScanLayout& L, const qpam_scan_a
   return QPAM_OK;
 }
 
+// Destination of the final states of a forward of which no backward will follow.
+struct PoolDest {
+  void* pool;
+  const int32_t* slot_ids;
+  int64_t n_slots;
+  int32_t dtype, L, layer;
+};
+// A workspace without room for the backward's part cannot be handed to one (qpam_scan_bwd refuses it): forward only.
+static void set_forward_only(ScanParams& p, const qpam_scan_args* a, const ScanLayout& L, const PoolDest* dest) {
+  p.fwd_only = dest != nullptr || a->workspace_bytes < L.total_bwd;
+  if (dest) {
+    p.pool = dest->pool; p.slot_ids = dest->slot_ids; p.n_slots = dest->n_slots;
+    p.pool_bf16 = dest->dtype == QPAM_BF16; p.pool_L = dest->L; p.pool_layer = dest->layer;
+  }
+}
+
 // Output tensor as the target of the chunk kernels' TMA stores (boxes of 64 elements x 32 rows): [B*H*T rows][128], or
 // for the token-major layout [B*T rows][H*128].
 static int make_out_map(CUtensorMap* m, const qpam_scan_args* a, bool token_major) {
@@ -242,9 +258,10 @@ static int make_out_map(CUtensorMap* m, const qpam_scan_args* a, bool token_majo
 }
 
 // bf16 / d = 64 / one state: tensor-core kernels on 128-token chunks
-static int scan_fwd_tc(const qpam_scan_args* a, const ScanLayout& L, cudaStream_t st, bool token_major = false) {
+static int scan_fwd_tc(const qpam_scan_args* a, const ScanLayout& L, cudaStream_t st, bool token_major = false, const PoolDest* dest = nullptr) {
   ScanParams p = make_params(a, L);
   p.y_token_major = token_major ? 1 : 0;
+  set_forward_only(p, a, L, dest);
   if (a->cu_seqlens != nullptr) {
     k_chunk_prefix_checked<<<1, 256, 0, st>>>(a->cu_seqlens, const_cast<int32_t*>(p.geom.chunk_prefix), a->S, L.ch, a->T);
     QPAM_LAUNCH_CHECK("k_chunk_prefix");
@@ -267,9 +284,10 @@ static int scan_fwd_tc(const qpam_scan_args* a, const ScanLayout& L, cudaStream_
 }
 
 // bf16 / d = 64 / K = 2..4 states: state sums and carry per state, then ONE fused output kernel
-static int scan_fwd_tcK(const qpam_scan_args* a, const ScanLayout& L, cudaStream_t st, bool token_major = false) {
+static int scan_fwd_tcK(const qpam_scan_args* a, const ScanLayout& L, cudaStream_t st, bool token_major = false, const PoolDest* dest = nullptr) {
   ScanParams p = make_params(a, L);
   p.y_token_major = token_major ? 1 : 0;
+  set_forward_only(p, a, L, dest);
   if (a->cu_seqlens != nullptr) {
     k_chunk_prefix_checked<<<1, 256, 0, st>>>(a->cu_seqlens, const_cast<int32_t*>(p.geom.chunk_prefix), a->S, L.ch, a->T);
     QPAM_LAUNCH_CHECK("k_chunk_prefix");
@@ -482,6 +500,27 @@ static int scan_fwd_any(const qpam_scan_args* a, void* stream, bool token_major)
 extern "C" int qpam_scan_fwd(const qpam_scan_args* a, void* stream) { return scan_fwd_any(a, stream, false); }
 
 extern "C" int qpam_scan_fwd_tokens(const qpam_scan_args* a, void* stream) { return scan_fwd_any(a, stream, true); }
+
+extern "C" int qpam_scan_prefill(const qpam_scan_args* a, void* pool, int32_t state_dtype, int64_t n_slots, int32_t L_, int32_t layer,
+                                 const int32_t* slot_ids, void* stream) {
+  int rc = check_scan_args(a);
+  if (rc) return rc;
+  QPAM_REQUIRE(a->y && pool && slot_ids && ((uintptr_t)pool & 15) == 0, "scan prefill: NULL pointer argument or unaligned pool");
+  QPAM_REQUIRE(state_dtype == QPAM_F32 || state_dtype == QPAM_BF16, "scan prefill: state_dtype %d unknown", state_dtype);
+  QPAM_REQUIRE(L_ >= 1 && layer >= 0 && layer < L_ && n_slots >= 0, "scan prefill: bad pool shape");
+  const ScanLayout L = scan_layout(a, fwd_chunk_len(a));
+  if (L.ch != tcs::TC) {
+    set_error("scan prefill: offered on the tensor-core path only (bf16, d = 64)");
+    return QPAM_EUNSUPPORTED;
+  }
+  if (a->workspace_bytes < L.total_fwd) {
+    set_error("scan prefill: workspace %zu bytes < required %zu", a->workspace_bytes, L.total_fwd);
+    return QPAM_EWORKSPACE;
+  }
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const PoolDest dest{pool, slot_ids, n_slots, state_dtype, L_, layer};
+  return tc_fwdK_eligible(a) ? scan_fwd_tcK(a, L, st, true, &dest) : scan_fwd_tc(a, L, st, true, &dest);
+}
 
 extern "C" int qpam_scan_bwd(const qpam_scan_args* a, const void* dy, void* dq, void* dk, void* dv,
                              float* dgamma, float* dcoef, const float* ds_final, float* ds0,

@@ -69,6 +69,34 @@ __device__ __forceinline__ void warp_cumsum128(float* A, const float* __restrict
   warp_cumsum128_finish(A, g, len, eps, lane);
 }
 
+// Where a chunk's sums go when they are a sequence's final state already (fwd_only, one chunk, no initial state): s_final
+// and / or the sequence's pool slot.  A lane holds one column (n' = q4 * 32 + lane) of every row.
+struct FinalDest {
+  float* f;                 // s_final block, or null
+  int64_t pool;             // first scalar of the pool block, or -1
+  __device__ __forceinline__ void init(const ScanParams& p, int seq, int k, int h) {
+    f = p.s_final ? p.s_final + (((size_t)k * p.geom.S + seq) * p.H + h) * (size_t)(TD * TD) * 2 : nullptr;
+    pool = p.pool ? pool_base(p, seq, k, h, TD) : -1;
+  }
+  // rows i and i + 1 (u0, u1) of the lane's column; off: the scalar of row i
+  __device__ __forceinline__ void store2(const ScanParams& p, int off, float u0, float u1, bool even, bool ok) const {
+    if (f && ok) {
+      f[off] = u0;
+      f[off + 2 * TD] = u1;
+    }
+    if (pool >= 0) {
+      if (p.pool_bf16) {         // the even lane of a pair takes both columns of row i, the odd lane those of row i + 1
+        const float x = __shfl_xor_sync(0xffffffffu, even ? u1 : u0, 1);
+        const int at = even ? off : off - 1 + 2 * TD;
+        if (ok) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.pool) + pool + at) = even ? pack_bf162(u0, x) : pack_bf162(x, u1);
+      } else if (ok) {
+        reinterpret_cast<float*>(p.pool)[pool + off] = u0;
+        reinterpret_cast<float*>(p.pool)[pool + off + 2 * TD] = u1;
+      }
+    }
+  }
+};
+
 // ---------------------------------------------------------------------------------------------
 // Chunk-local state sum  U[i][j] = sum_s w_s v_s[i] conj(k_s[j])  in transposed form, from the key tile AS THE TMA
 // DELIVERS IT (interleaved re, im: no operand is built from it) and the value tile split into two weighted planes:
@@ -180,11 +208,22 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + cc * 32, d1);
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + 64 + cc * 32, d2);
     const bool even = (lane & 1) == 0;
+    const bool final_now = !DSTATE && p.fwd_only && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
+    if (final_now) {
+      FinalDest fin;
+      fin.init(p, L.seq, kst, h);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float other = __shfl_xor_sync(0xffffffffu, d2[i], 1);      // D2 of the neighbouring key column
-      const float u = even ? d1[i] + other : other - d1[i];
-      if (ok) dst[(size_t)(cc * 32 + i) * 128] = u;
+      for (int i = 0; i < 32; i += 2) {
+        const float o0 = __shfl_xor_sync(0xffffffffu, d2[i], 1), o1 = __shfl_xor_sync(0xffffffffu, d2[i + 1], 1);
+        fin.store2(p, (cc * 32 + i) * 128 + q4 * 32 + lane, even ? d1[i] + o0 : o0 - d1[i], even ? d1[i + 1] + o1 : o1 - d1[i + 1], even, ok);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float other = __shfl_xor_sync(0xffffffffu, d2[i], 1);      // D2 of the neighbouring key column
+        const float u = even ? d1[i] + other : other - d1[i];
+        if (ok) dst[(size_t)(cc * 32 + i) * 128] = u;
+      }
     }
     if (ok && !DSTATE && tid == 0) p.chunk_decay[((size_t)kst * p.H + h) * p.nslots + L.slot0 + L.c + 1] = __expf(a_last);
   }
@@ -298,16 +337,27 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
     // Re U = D1[2j] + D2[2j+1], Im U = D2[2j] - D1[2j+1]: lane n' = 2j+c holds column i, state[i][j][c] at i*128 + n'
     float2* slot = p.states + state_base(p, k, h, L.slot0 + L.c + 1, TD);
     float* dst = reinterpret_cast<float*>(slot) + (q4 * 32 + lane);
+    const bool final_now = p.fwd_only && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
 #pragma unroll 1
     for (int hh = 0; hh < 2; ++hh) {          // 16 columns at a time: the value tile stays in registers beside them
       float d1[16], d2[16];
       const uint32_t col = (uint32_t)(cc * 32 + hh * 16);
       tmem_ld16x2(tmem + ((uint32_t)(q4 * 32) << 16) + col, d1, tmem + ((uint32_t)(q4 * 32) << 16) + 64 + col, d2);
+      if (final_now) {
+        FinalDest fin;
+        fin.init(p, L.seq, k, h);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float other = __shfl_xor_sync(0xffffffffu, d2[i], 1);
-        const float u = even ? d1[i] + other : other - d1[i];
-        if (ok) dst[(size_t)(col + i) * 128] = u;
+        for (int i = 0; i < 16; i += 2) {
+          const float o0 = __shfl_xor_sync(0xffffffffu, d2[i], 1), o1 = __shfl_xor_sync(0xffffffffu, d2[i + 1], 1);
+          fin.store2(p, (int)(col + i) * 128 + q4 * 32 + lane, even ? d1[i] + o0 : o0 - d1[i], even ? d1[i + 1] + o1 : o1 - d1[i + 1], even, ok);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float other = __shfl_xor_sync(0xffffffffu, d2[i], 1);
+          const float u = even ? d1[i] + other : other - d1[i];
+          if (ok) dst[(size_t)(col + i) * 128] = u;
+        }
       }
     }
     if (ok && tid == 0) p.chunk_decay[((size_t)k * p.H + h) * p.nslots + L.slot0 + L.c + 1] = __expf(a_last);
