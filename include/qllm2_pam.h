@@ -345,7 +345,61 @@ typedef struct qpam_front_args {
   float gamma_floor, q_scale;
   int32_t B, T, H, d, K, io_dtype;
 } qpam_front_args;
+struct qpam_front_bwd_args {
+  qpam_front_args f;
+  void *d_raw, *d_rawm;
+  int64_t ld_raw, ld_rawm;
+  float* part;
+  int32_t P, used_raw, used_rawm;
+  int32_t col[4], from_mag[4];
+};
 int qpam_pam_front_fwd(const qpam_front_args* args, void* stream);
+
+/* ------------------------------------------------------------------------------------------
+ * Training-step fusions of a block (bf16 activations, fp32 parameters): the element-wise work of
+ * V11Block.forward (v11/model.py:1021-1049) and its backward around the library GEMMs and the scan.
+ * ------------------------------------------------------------------------------------------ */
+#define QPAM_PACK_COMPLEX 0     /* a, b [out,in] = Wr, Wi  <->  packed [2*out, 2*in] block matrix */
+#define QPAM_PACK_INTERLEAVE 1  /* a [out, 2*in], columns [re | im]  <->  packed [out, 2*in], interleaved columns */
+#define QPAM_PACK_PLAIN 2       /* a [out,in] (NULL when packing: zeros)  <->  packed [out,in] */
+typedef struct qpam_pack_item {
+  float *a, *b;       /* fp32 parameters (pack) or their gradients (unpack) */
+  void* packed;       /* bf16, 16-byte aligned rows */
+  int32_t out, in, kind;
+} qpam_pack_item;
+int qpam_pack_block(const qpam_pack_item* items, int32_t n, void* stream);     /* items in HOST memory, n <= 24 */
+int qpam_unpack_block(const qpam_pack_item* items, int32_t n, void* stream);
+typedef struct qpam_colsum_item {
+  const float* part;  /* P rows of ld, the first C columns of each */
+  float* out;         /* [C] */
+  int32_t P, C, ld;
+} qpam_colsum_item;
+int qpam_colsum(const qpam_colsum_item* items, int32_t n, void* stream);       /* items in HOST memory, n <= 12 */
+/* Training forward (bf16, one pass, same bits as the separate operators): out = gated unit of gate and act(up), each [N,C,2]. */
+int qpam_act_gate_train_fwd(const void* gate, const void* up, const float* bias, const float* beta, void* out, int64_t N, int32_t C,
+                            void* stream);
+/* Its backward: dgate_up [N,4C] = (d gate | d up); part [P][2C] (modSwish: d(bias), d(beta)) or [P][C] (modReLU), P as
+ * qpam_act_gate_bwd_parts suggests. */
+int32_t qpam_act_gate_bwd_parts(int64_t N, int32_t C);
+int qpam_act_gate_bwd(const void* gate, const void* up, const void* dout, const float* bias, const float* beta, void* dgate_up,
+                      float* part, int32_t P, int64_t N, int32_t C, void* stream);
+/* Training forward of residual add and norm (bf16, D <= 768, same bits as the separate operators): z_out = z + s * delta (both NULL:
+ * the norm of z), xn = norm(z_out) * scale, mag = |xn| (NULL: not wanted). */
+int qpam_norm_train_fwd(const void* z, const void* delta, const float* s, const float* scale, void* z_out, void* xn, void* mag,
+                        int64_t N, int32_t D, float eps, void* stream);
+/* Its backward (bf16, D <= 768): dz = dres + d(norm)(dxn) [+ the gradient through |xn|, dmag], ddelta = s * dz; part [P][D+1] =
+ * d(norm_scale), d(s).  z is the stored sum.  dmag, dres, delta (with s and ddelta) may be NULL. */
+int qpam_cnorm_res_bwd(const void* z, const float* scale, const void* dxn, const void* dmag, const void* dres, const void* delta,
+                       const float* s, void* dz, void* ddelta, float* part, int32_t P, int64_t N, int32_t D, float eps, void* stream);
+/* Backward of qpam_pam_front_fwd: args.f as in the forward with q, k, v, gamma, coef holding the incoming gradients; writes the
+ * gradient of the projection output into d_raw [B*T, ld_raw] (qkv columns first) and of the |x| projection into d_rawm.
+ * col / from_mag: where dt, pg, phase, score sit (-1 absent); columns from used_raw / used_rawm on are zeroed.
+ * part [P][H][3K+1] = sums of d(x_k), d(pg), d(phase_k), d(score_k). */
+typedef struct qpam_front_bwd_args qpam_front_bwd_args;
+int qpam_pam_front_bwd(const qpam_front_bwd_args* args, void* stream);
+/* Parameter gradients from those sums added up over P, sums [H][3K+1]; pointers of absent parameters NULL. */
+int qpam_front_params(const float* sums, int32_t H, int32_t K, float* dt_bias, float* dt_proj_bias, float* dt_off,
+                      float* pg_bias, float* phase_bias, float* score_bias, void* stream);
 
 /* One decode step of a whole model for a handful of sequences (n <= 16, bf16 weights, head dim 64): token ids ->
  * arg-max ids or bf16 logits, the slots' states updated in place (the per-token loop body of V11LM.generate,

@@ -123,6 +123,16 @@ SIGNATURES = {
     "qpam_residual_cnorm_fwd": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int64,
                                           c_int32, C.c_float, c_void_p]),
     "qpam_pam_front_fwd": (c_int32, [C.POINTER(FrontArgs), c_void_p]),
+    "qpam_pack_block": (c_int32, [c_void_p, c_int32, c_void_p]),
+    "qpam_unpack_block": (c_int32, [c_void_p, c_int32, c_void_p]),
+    "qpam_colsum": (c_int32, [c_void_p, c_int32, c_void_p]),
+    "qpam_act_gate_train_fwd": (c_int32, [c_void_p] * 5 + [c_int64, c_int32, c_void_p]),
+    "qpam_act_gate_bwd_parts": (c_int32, [c_int64, c_int32]),
+    "qpam_act_gate_bwd": (c_int32, [c_void_p] * 7 + [c_int32, c_int64, c_int32, c_void_p]),
+    "qpam_norm_train_fwd": (c_int32, [c_void_p] * 7 + [c_int64, c_int32, c_float, c_void_p]),
+    "qpam_cnorm_res_bwd": (c_int32, [c_void_p] * 10 + [c_int32, c_int64, c_int32, c_float, c_void_p]),
+    "qpam_pam_front_bwd": (c_int32, [c_void_p, c_void_p]),
+    "qpam_front_params": (c_int32, [c_void_p, c_int32, c_int32] + [c_void_p] * 7),
     "qpam_step_supported": (c_int32, [c_int32] * 7),
     "qpam_step_workspace_bytes": (c_size_t, [C.POINTER(StepArgs)]),
     "qpam_step_fwd": (c_int32, [C.POINTER(StepArgs), c_void_p]),

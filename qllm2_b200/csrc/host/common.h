@@ -64,5 +64,6 @@ bool scan_prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
 void bind_scan(pybind11::module_& m);
 void bind_loss(pybind11::module_& m);
 void bind_forward(pybind11::module_& m);
+void bind_block(pybind11::module_& m);
 
 }  // namespace qhost

@@ -14,4 +14,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   qhost::bind_scan(m);
   qhost::bind_loss(m);
   qhost::bind_forward(m);
+  qhost::bind_block(m);
 }

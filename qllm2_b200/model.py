@@ -409,13 +409,16 @@ class V11PAMLayer(nn.Module):
         gamma, omp, coef = self.gates_and_coef(x)
         rope = None
         if self.use_rope:
-            if positions is None and step_offset + x.shape[1] > self.rope_cache.shape[0]:
-                self.register_buffer("rope_cache", build_rope_cache((step_offset + x.shape[1]) * 2, self.head_dim).to(x.device),
-                                     persistent=False)
-            rope = self.rope_cache
+            rope = self.rope_table(x, step_offset) if positions is None else self.rope_cache
         q, k, vprime = FE.pam_prep(self.qkv_proj(x), rope, omp, n_heads=self.num_heads, head_dim=self.head_dim,
                                    positions=positions, offset=step_offset)
         return q, k, vprime, gamma, coef
+
+    def rope_table(self, x: torch.Tensor, step_offset: int) -> torch.Tensor:
+        """The rotary table, grown to cover positions step_offset .. step_offset + T - 1."""
+        if step_offset + x.shape[1] > self.rope_cache.shape[0]:
+            self.register_buffer("rope_cache", build_rope_cache((step_offset + x.shape[1]) * 2, self.head_dim).to(x.device), persistent=False)
+        return self.rope_cache
 
     def _gamma_and_vprime(self, x, values, state_offset: float = 0.0):
         """Single-state form kept for callers of the reference API (v11/model.py:308-350)."""
@@ -504,7 +507,41 @@ class V11Block(nn.Module):
         self.pam = V11PAMLayer(cfg, layer_idx=layer_idx)
         self.pam_scale = nn.Parameter(torch.tensor(0.1))
 
-    def forward(self, x, pam_state=None, step_offset: int = 0):
+    def _native_ok(self, x, pam_state) -> bool:
+        """Whether the whole block can run as one native node (csrc/host/block.cpp): bf16 autocast over fp32 parameters from
+        a zero state, in the shape its kernels cover, with nothing attached to the operators in between."""
+        pam = self.pam
+        if (pam_state is not None or not x.is_cuda or x.dtype != torch.bfloat16 or x.shape[1] < 2 or not torch.is_autocast_enabled("cuda")
+                or torch.get_autocast_dtype("cuda") != torch.bfloat16):
+            return False
+        if pam.head_dim != 64 or pam.num_heads > 64 or not pam.fused_qkv or pam.qk_norm or pam.dim % 4 or pam.dim > 768 or not pam._fused_gates_ok(x):
+            return False
+        if self.training and (self.cgu_dropout.p > 0 or pam.dropout.p > 0):
+            return False
+        if any(p.dtype != torch.float32 for p in self.parameters()):
+            return False
+        return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in self.modules() if m is not self)
+
+    def _native(self, x, step_offset: int):
+        cgu, pam = self.cgu, self.pam
+        act, K, gsp = cgu.act, pam.n_states, pam.use_gsp
+        rope = pam.rope_table(x, step_offset) if pam.use_rope else None
+        score = pam.score_proj if K > 1 and pam.state_compete else None
+        params = [self.norm1.scale, cgu.gate_proj.weight_real, cgu.gate_proj.weight_imag, cgu.up_proj.weight_real, cgu.up_proj.weight_imag,
+                  cgu.down_proj.weight_real, cgu.down_proj.weight_imag, act.bias, getattr(act, "beta", None), self.cgu_scale, self.norm2.scale,
+                  pam.qkv_proj.weight_real, pam.qkv_proj.weight_imag, pam.o_proj.weight_real, pam.o_proj.weight_imag, pam.dt_proj.weight, pam.dt_proj.bias,
+                  pam.dt_bias, pam.protect_gate.weight if gsp else None, pam.protect_gate.bias if gsp else None, pam.state_dt_offset if K > 1 else None,
+                  pam.phase_proj.weight if K > 1 else None, pam.phase_proj.bias if K > 1 else None, None if score is None else score.weight,
+                  None if score is None else score.bias, self.pam_scale]
+        pam._route_aux = None
+        return _lib.host().block(x, params, rope, pam.num_heads, pam.head_dim, K, pam.gate_content_aware, pam.routing_content_aware,
+                                 float(pam.gamma_floor or 0.0), step_offset)
+
+    def forward(self, x, pam_state=None, step_offset: int = 0, want_state: bool = True):
+        """want_state=False: the caller drops the new state (training), None is returned in its place where that saves work."""
+        if self._native_ok(x, pam_state):
+            out, s = self._native(x, step_offset)
+            return out, ((s[0] if self.pam.n_states == 1 else s).to(x.dtype) if want_state else None)
         mixed = self.cgu(self.norm1(x))
         if self.training and self.cgu_dropout.p > 0:
             mixed = mixed * _dropout_mask(self.cgu_dropout, mixed)
@@ -581,15 +618,15 @@ class V11LM(nn.Module):
                 total = a if total is None else total + a
         return total if total is not None else torch.zeros((), device=device)
 
-    def _run_blocks(self, z, states, step_offset, checkpoint):
+    def _run_blocks(self, z, states, step_offset, checkpoint, want_states=True):
         new_states = []
         for i, blk in enumerate(self.blocks):
             s = states[i] if states is not None else None
             if checkpoint:
                 from torch.utils.checkpoint import checkpoint as ckpt
-                z, ns = ckpt(lambda zz, b=blk: b(zz, pam_state=None, step_offset=step_offset), z, use_reentrant=False)
+                z, ns = ckpt(lambda zz, b=blk: b(zz, pam_state=None, step_offset=step_offset, want_state=want_states), z, use_reentrant=False)
             else:
-                z, ns = blk(z, pam_state=s, step_offset=step_offset)
+                z, ns = blk(z, pam_state=s, step_offset=step_offset, want_state=want_states)
             new_states.append(ns)
         return z, new_states
 
@@ -607,7 +644,7 @@ class V11LM(nn.Module):
     def _hidden_to_lm(self, input_ids, step_offset: int = 0):
         z = self._embed(input_ids, step_offset)
         ckpt = self.config.gradient_checkpointing and self.training
-        z, _ = self._run_blocks(z, None, step_offset, ckpt)
+        z, _ = self._run_blocks(z, None, step_offset, ckpt, want_states=False)
         lm = self._head_hidden(z)
         probs = [b.pam._gate_prob_bt for b in self.blocks if getattr(b.pam, "_gate_prob_bt", None) is not None]
         return lm, self._aux(input_ids.device), (torch.stack(probs, dim=0) if probs else None)
