@@ -122,6 +122,11 @@ int qpam_scan_fwd_static(const qpam_scan_args* args, void* stream);
 int qpam_scan_bwd(const qpam_scan_args* args, const void* dy, void* dq, void* dk, void* dv,
                   float* dgamma, float* dcoef, const float* ds_final, float* ds0,
                   int32_t states_valid, void* stream);
+/* The same with dy token-major, [B,T,H,d,2], as the projection behind the scan leaves it (bf16, d = 64, 2..4 states;
+ * QPAM_EUNSUPPORTED otherwise). */
+int qpam_scan_bwd_tokens(const qpam_scan_args* args, const void* dy, void* dq, void* dk, void* dv,
+                         float* dgamma, float* dcoef, const float* ds_final, float* ds0,
+                         int32_t states_valid, void* stream);
 
 /* qpam_scan_bwd for one state with dq, dk, dv ADDED to the values the buffers already hold (dgamma, ds0 are
  * written as usual).  The K phase-routed states of a layer (v11/model.py:657-781) are K scans over the same

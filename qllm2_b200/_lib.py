@@ -75,6 +75,8 @@ SIGNATURES = {
     "qpam_scan_fwd_static": (c_int32, [C.POINTER(ScanArgs), c_void_p]),
     "qpam_scan_bwd": (c_int32, [C.POINTER(ScanArgs), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_void_p, c_void_p, c_int32, c_void_p]),
+    "qpam_scan_bwd_tokens": (c_int32, [C.POINTER(ScanArgs), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                c_void_p, c_void_p, c_void_p, c_int32, c_void_p]),
     "qpam_scan_bwd_accumulate": (c_int32, [C.POINTER(ScanArgs), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                            c_void_p, c_int32, c_void_p]),
     "qpam_scan_fwd_states": (c_int32, [C.POINTER(ScanArgs), c_void_p, c_void_p]),

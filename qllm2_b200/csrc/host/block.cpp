@@ -178,7 +178,7 @@ struct Block : Function<Block> {
     qpam_front_args f = front_args(s, p, qkv, logits, rope, offset, gamma_floor);
     f.q = q.data_ptr(); f.k = k.data_ptr(); f.v = v.data_ptr(); f.gamma = fptr(gamma); f.coef = fptr(coef);
     check(qpam_pam_front_fwd(&f, st), "qpam_pam_front_fwd");
-    Tensor y = at::empty({N, 2 * s.inner}, o), s_final = at::empty({K, s.B, H, d, d, 2}, f32o), ys;
+    Tensor y = at::empty({N, 2 * s.inner}, o), s_final = at::empty({K, s.B, H, d, d, 2}, f32o);
     qpam_scan_args a = scan_args(s, q, k, v, gamma);
     a.s_final = fptr(s_final);
     if (K > 1 && !bwd) a.coef = fptr(coef);
@@ -189,7 +189,7 @@ struct Block : Function<Block> {
       a.y = y.data_ptr();
       check(qpam_scan_fwd_tokens(&a, st), "qpam_scan_fwd_tokens");
     } else {
-      ys = at::empty({K, s.B, H, s.T, d, 2}, o);
+      const Tensor ys = at::empty({K, s.B, H, s.T, d, 2}, o);
       check(qpam_scan_fwd_states(&a, ys.data_ptr(), st), "qpam_scan_fwd_states");
       void* yk[QPAM_MAX_STATES];
       state_ptrs(ys, yk);
@@ -199,7 +199,7 @@ struct Block : Function<Block> {
     Tensor x2 = at::empty_like(x);
     check(qpam_scaled_residual_fwd(x1.data_ptr(), QPAM_BF16, out.data_ptr(), QPAM_BF16, fptr(p[PAM_SCALE]), x2.data_ptr(), x.numel(), st), "qpam_scaled_residual_fwd");
     if (bwd) {
-      variable_list keep = {x, xn, gate, up, gated, mixed, x1, xn2, mag, qkv, logits[0], logits[1], logits[2], logits[3], q, k, v, gamma, coef, ws, ys, y, out, w.w_gu, w.w_down, w.w_front, w.w_mag, w.w_o, rope};
+      variable_list keep = {x, xn, gate, up, gated, mixed, x1, xn2, mag, qkv, logits[0], logits[1], logits[2], logits[3], q, k, v, gamma, coef, ws, y, out, w.w_gu, w.w_down, w.w_front, w.w_mag, w.w_o, rope};
       keep.insert(keep.end(), p.begin(), p.end());
       ctx->save_for_backward(std::move(keep));
       ctx->saved_data["H"] = H;
@@ -217,7 +217,7 @@ struct Block : Function<Block> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
     const auto sv = ctx->get_saved_variables();
-    enum { X, XN, GATE, UP, GATED, MIXED, X1, XN2, MAG, QKV, LOGITS, LOGITS_END = LOGITS + 3, Q, KK, V, GAMMA, COEF, WS, YS, Y, OUT, W_GU, W_DOWN, W_FRONT, W_MAG, W_O, ROPE, FIRST_PARAM };
+    enum { X, XN, GATE, UP, GATED, MIXED, X1, XN2, MAG, QKV, LOGITS, LOGITS_END = LOGITS + 3, Q, KK, V, GAMMA, COEF, WS, Y, OUT, W_GU, W_DOWN, W_FRONT, W_MAG, W_O, ROPE, FIRST_PARAM };
     const variable_list p(sv.begin() + FIRST_PARAM, sv.end());
     const int64_t H = ctx->saved_data["H"].toInt(), d = ctx->saved_data["d"].toInt(), K = ctx->saved_data["K"].toInt();
     const Tensor& x = sv[X];
@@ -260,17 +260,9 @@ struct Block : Function<Block> {
       check(qpam_scan_bwd(&a, dyh.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), fptr(dgamma), nullptr, fptr(ds), nullptr, 1, st), "qpam_scan_bwd");
     } else {
       dcoef = at::empty_like(sv[COEF]);
-      Tensor dys = at::empty_like(sv[YS]);
-      void *yk[QPAM_MAX_STATES], *dyk[QPAM_MAX_STATES];
-      state_ptrs(sv[YS], yk);
-      state_ptrs(dys, dyk);
-      check(qpam_state_combine_tokens_bwd(yk, fptr(sv[COEF]), dy.data_ptr(), dyk, fptr(dcoef), QPAM_BF16, (int)K, (int)s.B, (int)H, (int)s.T, (int)d, st),
-            "qpam_state_combine_tokens_bwd");
-      const int64_t row = s.B * H * s.T, sb = s.B * H * d * d * 2;
-      for (int64_t i = 0; i < K; ++i)
-        check(qpam_scan_bwd_state(&a, (int)i, dyk[i], dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), fptr(dgamma) + i * row, ds.defined() ? fptr(ds) + i * sb : nullptr,
-                                  nullptr, i > 0 ? 1 : 0, st),
-              "qpam_scan_bwd_state");
+      a.coef = fptr(sv[COEF]);
+      check(qpam_scan_bwd_tokens(&a, dy.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), fptr(dgamma), fptr(dcoef), fptr(ds), nullptr, 1, st),
+            "qpam_scan_bwd_tokens");
     }
     // ---- front
     Tensor d_raw = at::empty({N, s.rows_a}, o), d_rawm = s.rows_m ? at::empty({N, s.rows_m}, o) : Tensor();

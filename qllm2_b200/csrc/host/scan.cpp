@@ -90,8 +90,9 @@ void state_ptrs(const Tensor& ys, void** out) {
 }
 
 // K = 2..4 states over the same bf16 q, k, v (d = 64), with gradients: the chunk sums of all states from one pass, the output
-// kernel per state, and the read-out sum_k c_k y^(k) of the per-state outputs; the backward adds the states' dq, dk, dv in
-// one set of buffers (qpam_scan_bwd_state).  Without read-out weights the per-state outputs themselves are returned.
+// kernel per state, and the read-out sum_k c_k y^(k) of the per-state outputs; the backward takes all states at once.  Without
+// read-out weights the per-state outputs themselves are returned, and their gradients' dq, dk, dv added up in one set of
+// buffers (qpam_scan_bwd_state).
 struct ScanStates : Function<ScanStates> {
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gamma, const OptTensor& coef_,
                                const OptTensor& s0_, const OptTensor& cu_, double q_scale, double eps, int64_t chunk, bool token_major) {
@@ -119,7 +120,7 @@ struct ScanStates : Function<ScanStates> {
         check(qpam_state_combine_fwd(yk, fptr(coef), y.data_ptr(), QPAM_BF16, (int)K, B * H * T, (int)d, stream()), "qpam_state_combine_fwd");
       }
     }
-    ctx->save_for_backward({q, k, v, gamma, coef, s0, cu, bwd ? ws : Tensor(), coef.defined() && bwd ? ys : Tensor()});
+    ctx->save_for_backward({q, k, v, gamma, coef, s0, cu, bwd ? ws : Tensor()});
     ctx->saved_data["q_scale"] = q_scale;
     ctx->saved_data["eps"] = eps;
     ctx->saved_data["chunk"] = chunk;
@@ -130,37 +131,23 @@ struct ScanStates : Function<ScanStates> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
-    const Tensor &q = s[0], &k = s[1], &v = s[2], &gamma = s[3], &coef = s[4], &s0 = s[5], &cu = s[6], &ws = s[7], &ys = s[8];
+    const Tensor &q = s[0], &k = s[1], &v = s[2], &gamma = s[3], &coef = s[4], &s0 = s[5], &cu = s[6], &ws = s[7];
     const Config c{ctx->saved_data["q_scale"].toDouble(), ctx->saved_data["eps"].toDouble(), ctx->saved_data["chunk"].toInt()};
     const bool tokens = ctx->saved_data["tokens"].toBool();
     const int64_t B = q.size(0), H = q.size(1), T = q.size(2), d = q.size(3), K = gamma.size(0);
-    qpam_scan_args a = scan_args(q, k, v, gamma, Tensor(), s0, cu, Tensor(), Tensor(), c);
+    qpam_scan_args a = scan_args(q, k, v, gamma, coef, s0, cu, Tensor(), Tensor(), c);
     set_workspace(a, ws);
     const Tensor ds = grad_states(grads[1], a);
-    Tensor dys, dcoef;
-    if (coef.defined()) {
-      dys = at::empty({K, B, H, T, d, 2}, q.options());
-      dcoef = at::empty_like(coef);
-      if (grads[0].defined()) {
-        const Tensor dy = grads[0].to(q.scalar_type()).contiguous();
-        void *yk[QPAM_MAX_STATES], *dyk[QPAM_MAX_STATES];
-        state_ptrs(ys, yk);
-        state_ptrs(dys, dyk);
-        if (tokens)
-          check(qpam_state_combine_tokens_bwd(yk, fptr(coef), dy.data_ptr(), dyk, fptr(dcoef), QPAM_BF16, (int)K, (int)B, (int)H, (int)T, (int)d, stream()),
-                "qpam_state_combine_tokens_bwd");
-        else
-          check(qpam_state_combine_bwd(yk, fptr(coef), dy.data_ptr(), dyk, fptr(dcoef), QPAM_BF16, (int)K, B * H * T, (int)d, stream()),
-                "qpam_state_combine_bwd");
-      } else {
-        dys.zero_();
-        dcoef.zero_();
-      }
-    } else {
-      dys = grads[0].defined() ? grads[0].to(q.scalar_type()).contiguous() : at::zeros({K, B, H, T, d, 2}, q.options());
-    }
-    Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), dgamma = at::empty_like(gamma);
+    Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), dgamma = at::empty_like(gamma), dcoef;
     Tensor ds0 = s0.defined() && ctx->saved_data["ds0"].toBool() ? at::empty_like(s0) : Tensor();
+    if (coef.defined()) {
+      dcoef = at::empty_like(coef);
+      const Tensor dy = grads[0].defined() ? grads[0].to(q.scalar_type()).contiguous() : at::zeros({q.numel()}, q.options());
+      const auto bwd = tokens ? &qpam_scan_bwd_tokens : &qpam_scan_bwd;
+      check(bwd(&a, dy.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), fptr(dgamma), fptr(dcoef), fptr(ds), fptr(ds0), 1, stream()), "qpam_scan_bwd");
+      return {dq, dk, dv, dgamma, dcoef, ds0, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+    const Tensor dys = grads[0].defined() ? grads[0].to(q.scalar_type()).contiguous() : at::zeros({K, B, H, T, d, 2}, q.options());
     void* dyk[QPAM_MAX_STATES];
     state_ptrs(dys, dyk);
     const int64_t row = B * H * T, st = (int64_t)a.S * H * d * d * 2;

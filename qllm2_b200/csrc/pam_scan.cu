@@ -5,6 +5,7 @@
 #include "pam_scan_tc.cuh"
 #include "pam_scan_tc2.cuh"
 #include "pam_scan_tc3.cuh"
+#include "pam_scan_tc4.cuh"
 #include "tma_host.cuh"
 
 namespace qpam {
@@ -211,13 +212,13 @@ static ScanParams one_state_view(const ScanParams& pK, const qpam_scan_args* a, 
 // chunk-local state sums on tensor cores, then the carry over the chunk axis
 static int tc_states(const ScanParams& p, const ScanLayout& L, const qpam_scan_args* a, cudaStream_t st) {
   if (L.grid_chunks > 0 && a->K > 1) {      // all states from one load of the key / value tiles
-    int rc = set_smem(tcs::k_tc_chunk_outerK, tcs::OUTERK_SMEM);
+    int rc = set_smem(tcs::k_tc_chunk_outerK<false>, tcs::OUTERK_SMEM);
     if (rc) return rc;
     CUtensorMap mk, mv;
     const int64_t rows = (int64_t)a->B * a->H * a->T;
     if ((rc = make_map(&mk, a->k, 128, rows, 128, 64, 128))) return rc;
     if ((rc = make_map(&mv, a->v, 128, rows, 128, 64, 128))) return rc;
-    tcs::k_tc_chunk_outerK<<<dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st>>>(mk, mv, p);
+    tcs::k_tc_chunk_outerK<false><<<dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st>>>(mk, mv, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outerK");
   } else if (L.grid_chunks > 0) {
     int rc = set_smem(tcs::k_tc_chunk_outer<false>, tcs::OUTER_SMEM);
@@ -398,6 +399,62 @@ static int scan_bwd_tc(const qpam_scan_args* a, const ScanLayout& L, const void*
   return QPAM_OK;
 }
 
+template <int K>
+static int launch_bwdK(const tcs::BwdMaps& maps, const ScanParams& p, const ScanLayout& L, const float* anchors, cudaStream_t st) {
+  int rc = set_smem(tcs::k_tc_scan_bwdK<K>, tcs::BWDK_SMEM);
+  if (rc) return rc;
+  tcs::k_tc_scan_bwdK<K><<<dim3(L.grid_chunks, p.H), tcs::BT, tcs::BWDK_SMEM, st>>>(maps, p, anchors);
+  QPAM_LAUNCH_CHECK("k_tc_scan_bwdK");
+  return QPAM_OK;
+}
+
+// bf16 / d = 64 / K = 2..4 states, backward: gradient state sums of all states -> reverse carry (with the anchors of the
+// decay gradient) -> every gradient of every chunk.  Everything stays on the caller's stream.
+static int scan_bwd_tcK(const qpam_scan_args* a, const ScanLayout& L, const void* dy, void* dq, void* dk, void* dv, float* dgamma, float* dcoef,
+                        const float* ds_final, float* ds0, int states_valid, bool dy_tokens, cudaStream_t st) {
+  ScanParams p = make_params(a, L);
+  p.dy = dy; p.dq = dq; p.dk = dk; p.dv = dv;
+  p.dgamma = dgamma; p.dcoef = dcoef; p.ds_final = ds_final; p.ds0 = ds0;
+  p.dy_tokens = dy_tokens ? 1 : 0;
+  p.sms = sm_count();
+  int rc;
+  if (!states_valid) {
+    ScanParams pf = p;
+    pf.s_final = nullptr;
+    if (a->cu_seqlens != nullptr) {
+      k_chunk_prefix_checked<<<1, 256, 0, st>>>(a->cu_seqlens, const_cast<int32_t*>(p.geom.chunk_prefix), a->S, L.ch, a->T);
+      QPAM_LAUNCH_CHECK("k_chunk_prefix");
+    }
+    rc = tc_states(pf, L, a, st);
+    if (rc) return rc;
+  }
+  float* anchors = reinterpret_cast<float*>(reinterpret_cast<char*>(a->workspace) + L.off_anchors);
+  tcs::BwdMaps maps;
+  const int64_t rows = (int64_t)a->B * a->H * a->T;
+  if (L.grid_chunks > 0) {
+    if ((rc = make_map(&maps.q, a->q, 128, rows, 128, 64, 128))) return rc;
+    if ((rc = make_map(&maps.k, a->k, 128, rows, 128, 64, 128))) return rc;
+    if ((rc = make_map(&maps.v, a->v, 128, rows, 128, 64, 128))) return rc;
+    if (dy_tokens) rc = make_map(&maps.dy, dy, (int64_t)a->H * 128, (int64_t)a->B * a->T, (int64_t)a->H * 128, 64, 128);
+    else rc = make_map(&maps.dy, dy, 128, rows, 128, 64, 128);
+    if (rc) return rc;
+    if ((rc = make_map(&maps.dq, dq, 128, rows, 128, 64, 32))) return rc;
+    if ((rc = make_map(&maps.dk, dk, 128, rows, 128, 64, 32))) return rc;
+    if ((rc = make_map(&maps.dv, dv, 128, rows, 128, 64, 32))) return rc;
+    if ((rc = set_smem(tcs::k_tc_chunk_outerK<true>, tcs::OUTERK_SMEM))) return rc;
+    tcs::k_tc_chunk_outerK<true><<<dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st>>>(maps.q, maps.dy, p);
+    QPAM_LAUNCH_CHECK("k_tc_chunk_outerK<dstate>");
+  }
+  tcs::k_tc_state_scan_rev<<<dim3(a->S, a->H * a->K, 64 * 64 / 2 / 256), 256, 0, st>>>(p, anchors);
+  QPAM_LAUNCH_CHECK("k_tc_state_scan_rev");
+  if (L.grid_chunks == 0) return QPAM_OK;
+  switch (a->K) {
+    case 2: return launch_bwdK<2>(maps, p, L, anchors, st);
+    case 3: return launch_bwdK<3>(maps, p, L, anchors, st);
+    default: return launch_bwdK<4>(maps, p, L, anchors, st);
+  }
+}
+
 template <int D, typename T>
 static int scan_bwd_t(const qpam_scan_args* a, const ScanLayout& L, const void* dy, void* dq, void* dk,
                       void* dv, float* dgamma, float* dcoef, const float* ds_final, float* ds0,
@@ -522,24 +579,39 @@ extern "C" int qpam_scan_prefill(const qpam_scan_args* a, void* pool, int32_t st
   return tc_fwdK_eligible(a) ? scan_fwd_tcK(a, L, st, true, &dest) : scan_fwd_tc(a, L, st, true, &dest);
 }
 
-extern "C" int qpam_scan_bwd(const qpam_scan_args* a, const void* dy, void* dq, void* dk, void* dv,
-                             float* dgamma, float* dcoef, const float* ds_final, float* ds0,
-                             int32_t states_valid, void* stream) {
+static int scan_bwd_any(const qpam_scan_args* a, const void* dy, void* dq, void* dk, void* dv, float* dgamma, float* dcoef, const float* ds_final,
+                        float* ds0, int32_t states_valid, void* stream, bool dy_tokens) {
   int rc = check_scan_args(a);
   if (rc) return rc;
   QPAM_REQUIRE(dy && dq && dk && dv && dgamma, "scan bwd: dy/dq/dk/dv/dgamma must not be NULL");
   QPAM_REQUIRE(dcoef == nullptr || a->coef != nullptr, "scan bwd: dcoef requested but coef is NULL");
-  const bool tc_bwd = tc_fwd_eligible(a) && a->T > 0 && dcoef == nullptr &&
-                      (((uintptr_t)dy | (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv) & 15) == 0;
-  const ScanLayout L = scan_layout(a, tc_bwd ? tcs::TC : CH);
+  const bool aligned = a->T > 0 && (((uintptr_t)dy | (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv) & 15) == 0;
+  const bool tcK = tc_fwdK_eligible(a) && aligned, tc1 = tc_fwd_eligible(a) && aligned && dcoef == nullptr;
+  if (dy_tokens && !tcK) {
+    set_error("scan bwd: the token-major output gradient exists for 2..4 states on the tensor-core path only (bf16, d = 64)");
+    return QPAM_EUNSUPPORTED;
+  }
+  const ScanLayout L = scan_layout(a, tcK || tc1 ? tcs::TC : CH);
   if (fwd_chunk_len(a) != L.ch) states_valid = 0;  // the forward left states of another chunking
   if (a->workspace_bytes < L.total_bwd) {
     set_error("scan bwd: workspace %zu bytes < required %zu", a->workspace_bytes, L.total_bwd);
     return QPAM_EWORKSPACE;
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (tc_bwd) return scan_bwd_tc(a, L, dy, dq, dk, dv, dgamma, ds_final, ds0, states_valid, st);
+  if (tcK) return scan_bwd_tcK(a, L, dy, dq, dk, dv, dgamma, dcoef, ds_final, ds0, states_valid, dy_tokens, st);
+  if (tc1) return scan_bwd_tc(a, L, dy, dq, dk, dv, dgamma, ds_final, ds0, states_valid, st);
   QPAM_DISPATCH_SCAN(scan_bwd_t, a, L, dy, dq, dk, dv, dgamma, dcoef, ds_final, ds0, states_valid, st);
+}
+
+extern "C" int qpam_scan_bwd(const qpam_scan_args* a, const void* dy, void* dq, void* dk, void* dv,
+                             float* dgamma, float* dcoef, const float* ds_final, float* ds0,
+                             int32_t states_valid, void* stream) {
+  return scan_bwd_any(a, dy, dq, dk, dv, dgamma, dcoef, ds_final, ds0, states_valid, stream, false);
+}
+extern "C" int qpam_scan_bwd_tokens(const qpam_scan_args* a, const void* dy, void* dq, void* dk, void* dv,
+                                    float* dgamma, float* dcoef, const float* ds_final, float* ds0,
+                                    int32_t states_valid, void* stream) {
+  return scan_bwd_any(a, dy, dq, dk, dv, dgamma, dcoef, ds_final, ds0, states_valid, stream, true);
 }
 
 // The same backward with dq, dk, dv ADDED to what the buffers hold: the K phase-routed states of a layer are K

@@ -236,14 +236,16 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
 }
 
 // ---------------------------------------------------------------------------------------------
-// State sums of K states from ONE load of the key / value tiles (forward only, 2 <= K <= 4).  As in k_tc_chunk_outer
+// State sums of K states from ONE load of the key / value tiles (2 <= K <= 4).  As in k_tc_chunk_outer
 // the key tile is the A operand as the TMA delivers it and the decay weights sit on the value planes, so a state costs
 // one rewrite of the planes B_k = w^k_s (Re v_s ; Im v_s) from the registers that hold the value tile, its two MMA
 // chains into the same 128 TMEM columns, and its epilogue; the states follow one another.
 // grid = (chunks, H); 256 threads; 70 KB shared memory, 128 TMEM columns: three CTAs per SM.
 // ---------------------------------------------------------------------------------------------
-constexpr size_t OUTERK_SMEM = 1024 + 65536 + 4096;
+// DSTATE: the gradient counterpart, G_k = sum_t scale conj(c_kt) e^{A^k_t} dy_t (x) conj(q_t), into dstate slot c.
+constexpr size_t OUTERK_SMEM = 1024 + 65536 + KMAX * TC * 12 + 256;
 
+template <bool DSTATE>
 __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constant__ CUtensorMap mk,
                                                             const __grid_constant__ CUtensorMap mv, ScanParams p) {
   using namespace umma;
@@ -252,7 +254,8 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
   unsigned char* sA = smem;            // key tile: [2 boxes of 64 columns][128 rows][128 B]
   unsigned char* sB = smem + 32768;    // value tile, then per state [256 rows][128 B]: w Re v_s ; w Im v_s
   float* Acum = reinterpret_cast<float*>(smem + 65536);           // [KMAX][128]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(Acum + KMAX * TC);  // one per state, [KMAX]: the token tiles
+  float2* wrow = reinterpret_cast<float2*>(Acum + KMAX * TC);     // DSTATE: [KMAX][128] weight of a token
+  uint64_t* bar = reinterpret_cast<uint64_t*>(wrow + KMAX * TC);  // one per state, [KMAX]: the token tiles
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + KMAX + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const ChunkLoc L = locate_chunk(p.geom, blockIdx.x);
@@ -266,11 +269,12 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
     mbar_init(&bar[KMAX], 1);
     fence_barrier_init();
     const int row0 = (L.b * p.H + h) * p.T + L.t0;
+    const bool tok = DSTATE && p.dy_tokens;
     mbar_arrive_expect_tx(&bar[KMAX], 4 * 16384);
 #pragma unroll
     for (int kb = 0; kb < 2; ++kb) {
       tma_load_2d(sA + kb * 16384, &mk, &bar[KMAX], kb * 64, row0);
-      tma_load_2d(sB + kb * 16384, &mv, &bar[KMAX], kb * 64, row0);
+      tma_load_2d(sB + kb * 16384, &mv, &bar[KMAX], (tok ? h * 128 : 0) + kb * 64, tok ? L.b * p.T + L.t0 : row0);
     }
   }
   __syncwarp();
@@ -280,6 +284,15 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (DSTATE) {
+    for (int e = tid; e < K * TC; e += 256) {          // (read after the barrier in front of the first planes)
+      const int k = e / TC, t = e - k * TC;
+      float2 c = make_float2(1.f, 0.f);
+      if (p.coef != nullptr && t < L.len) c = __ldg(reinterpret_cast<const float2*>(p.coef + gamma_base(p, k, L.b, h, L.t0 + t) * 2));
+      const float f = p.q_scale * __expf(Acum[e]);
+      wrow[e] = make_float2(c.x * f, -c.y * f);
+    }
+  }
   bool ok = mbar_wait(&bar[KMAX], 0, 206);
   // this thread's 16-byte pieces of the value tile (rows past the chunk's end: zeros, which also cancel whatever the
   // key tile holds in those rows)
@@ -304,14 +317,14 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
       const int idx = tid + 256 * it;
       const int row = idx >> 4, c16 = idx & 15;
       const uint4 vx = vxa[it];
-      const float w = __expf(fminf(0.f, a_last - Acum[k * TC + row]));
+      const float2 w = DSTATE ? wrow[k * TC + row] : make_float2(__expf(fminf(0.f, a_last - Acum[k * TC + row])), 0.f);
       const uint32_t vw[4] = {vx.x, vx.y, vx.z, vx.w};
       float vr[4], vi[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float2 vv = unpack_bf162(vw[e]);
-        vr[e] = w * vv.x;
-        vi[e] = w * vv.y;
+        vr[e] = DSTATE ? w.x * vv.x - w.y * vv.y : w.x * vv.x;
+        vi[e] = DSTATE ? w.x * vv.y + w.y * vv.x : w.x * vv.y;
       }
       const uint32_t boff = (c16 & 1) * 8;
       *reinterpret_cast<uint2*>(sB + sw128(row, c16 >> 1) + boff) = make_uint2(pack_bf162(vr[0], vr[1]), pack_bf162(vr[2], vr[3]));
@@ -335,9 +348,9 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
     ok = mbar_wait(&bar[k], 0, 205) && ok;
     tc_fence_after();
     // Re U = D1[2j] + D2[2j+1], Im U = D2[2j] - D1[2j+1]: lane n' = 2j+c holds column i, state[i][j][c] at i*128 + n'
-    float2* slot = p.states + state_base(p, k, h, L.slot0 + L.c + 1, TD);
+    float2* slot = DSTATE ? p.dstates + state_base(p, k, h, L.slot0 + L.c, TD) : p.states + state_base(p, k, h, L.slot0 + L.c + 1, TD);
     float* dst = reinterpret_cast<float*>(slot) + (q4 * 32 + lane);
-    const bool final_now = p.fwd_only && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
+    const bool final_now = !DSTATE && p.fwd_only && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
 #pragma unroll 1
     for (int hh = 0; hh < 2; ++hh) {          // 16 columns at a time: the value tile stays in registers beside them
       float d1[16], d2[16];
@@ -360,7 +373,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
         }
       }
     }
-    if (ok && tid == 0) p.chunk_decay[((size_t)k * p.H + h) * p.nslots + L.slot0 + L.c + 1] = __expf(a_last);
+    if (ok && !DSTATE && tid == 0) p.chunk_decay[((size_t)k * p.H + h) * p.nslots + L.slot0 + L.c + 1] = __expf(a_last);
   }
   tc_fence_before();
   __syncthreads();

@@ -567,15 +567,15 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_bwd(const __grid_constant__
 }
 
 // ---------------------------------------------------------------------------------------------
-// Reverse inter-chunk carry of the tensor-core backward (d = 64, one state), with the anchors of the decay
+// Reverse inter-chunk carry of the tensor-core backward (d = 64), with the anchors of the decay
 // gradient:  dS_c = g_c dS_c+1 + G_c  in place over the chunk axis, and for every state slot the partial sums of
 // Re<dS_slot, S_slot> (S: forward state of the slot) -- one value per warp, ANCHOR_PARTS per slot, summed by the
 // chunk kernel.  Scaling S_c by e^x changes the loss by x Re<dS_c, S_c>, so that inner product is the exact
 // value of the suffix sum da at the first token of chunk c, known from fp32 quantities.
-// grid = (S, H, 8), 256 threads: every thread owns one float4 (two complex entries) of the state.
+// grid = (S, H * K, 8), 256 threads: every thread owns one float4 (two complex entries) of the state.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_tc_state_scan_rev(ScanParams p, float* __restrict__ anchor_parts) {
-  const int seq = blockIdx.x, h = blockIdx.y;
+  const int seq = blockIdx.x, h = blockIdx.y % p.H, k = blockIdx.y / p.H;
   const int e4 = blockIdx.z * 256 + threadIdx.x;
   constexpr int n4 = TD * TD / 2;
   const int lane = threadIdx.x & 31, part = blockIdx.z * 8 + (threadIdx.x >> 5);
@@ -588,11 +588,11 @@ __global__ void __launch_bounds__(256) k_tc_state_scan_rev(ScanParams p, float* 
     nc = p.geom.chunk_prefix[seq + 1] - p.geom.chunk_prefix[seq];
     slot0 = (int64_t)p.geom.chunk_prefix[seq] + seq;
   }
-  float4* st = reinterpret_cast<float4*>(p.dstates + state_base(p, 0, h, slot0, TD)) + e4;
-  const float4* fs = reinterpret_cast<const float4*>(p.states + state_base(p, 0, h, slot0, TD)) + e4;
-  const float* dec = p.chunk_decay + (size_t)h * p.nslots + slot0;
-  float* parts = anchor_parts + ((size_t)h * p.nslots + slot0) * ANCHOR_PARTS + part;
-  const size_t ext = (((size_t)seq * p.H + h) * (size_t)(TD * TD)) / 2 + e4;
+  float4* st = reinterpret_cast<float4*>(p.dstates + state_base(p, k, h, slot0, TD)) + e4;
+  const float4* fs = reinterpret_cast<const float4*>(p.states + state_base(p, k, h, slot0, TD)) + e4;
+  const float* dec = p.chunk_decay + ((size_t)k * p.H + h) * p.nslots + slot0;
+  float* parts = anchor_parts + (((size_t)k * p.H + h) * p.nslots + slot0) * ANCHOR_PARTS + part;
+  const size_t ext = ((((size_t)k * p.geom.S + seq) * p.H + h) * (size_t)(TD * TD)) / 2 + e4;
   float4 cur = make_float4(0.f, 0.f, 0.f, 0.f);
   if (p.ds_final != nullptr) cur = reinterpret_cast<const float4*>(p.ds_final)[ext];
   auto anchor = [&](int slot, const float4& a, const float4& b) {

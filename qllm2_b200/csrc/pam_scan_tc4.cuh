@@ -1,0 +1,650 @@
+// Backward of the chunked PAM scan on tensor cores for 2 <= K <= 4 phase-routed states: ALL gradients of a 128-token chunk,
+// for every state, in one CTA (bf16 token tensors, head dim 64).  With A^k the cumulative log decay of state k inside the chunk,
+// D^k_ts = e^{A^k_t - A^k_s} (s <= t < len), c_k the read-out weights, sigma the query scale:
+//
+//   X_ts = dy_t . conj(v_s)      Y_ts = q_t . conj(k_s)      G_ts = sigma sum_k conj(c_kt) D^k_ts
+//   dq_t = sum_s (G X)_ts k_s                 + sum_k sigma conj(c_kt) e^{A^k_t} (S^k_c)^H dy_t
+//   dk_s = sum_t conj((G X)_ts) q_t           + sum_k e^{A^k_last - A^k_s} (dS^k_c+1)^H v_s
+//   dv_s = sum_t (G conj(Y))_ts dy_t          + sum_k e^{A^k_last - A^k_s} dS^k_c+1 k_s
+//   dc_kt        = sigma [ sum_s D^k_ts Z_ts + e^{A^k_t} conj(q_t) . (S^k_c)^H dy_t ],     Z_ts = X_ts conj(Y_ts)
+//   Re<q,dq>_kt  = Re(conj(c_kt) dc_kt)
+//   Re<k,dk>_ks  = sigma sum_t D^k_ts Re(conj(c_kt) Z_ts) + e^{A^k_last - A^k_s} Re<k_s, (dS^k_c+1)^H v_s>
+//
+// The scores do not depend on the state, so K states cost one pass of the tile products; what a state adds is its term of
+// the weight G, its sums of Z and its carried-state products.  dc and the decay gradient come from the fp32 scores (no
+// per-state output is needed, and the contribution of every (t, s) pair to Re<q,dq> - Re<k,dk> cancels to fp32 rounding).
+//
+//
+// (One state keeps the three-job kernel of pam_scan_tc2.cuh: two CTAs on an SM hide each other's waits there, 108 us against
+// 118 us here at 8 x 6 x 2048; three states took 420 us that way, read-out weights included, and take 235 us.)
+//
+// Every score is formed twice, once per direction of the sum (a row of the tile is a TMEM lane, so sums along a row stay
+// inside threads): pass A has tokens t as rows (dq, dc), pass B tokens s (dk, dv, Re<k,dk>).  512 threads: a thread owns a
+// row and 32 columns of both score tiles in a pass and 16 channels of its row in the outputs.
+//
+//   TMEM        [0,128)              [128,256)           [256,384)            [384,512)
+//   scores      X real               X imaginary         Y real               Y imaginary
+//   dq          G X (bf16)           dq accumulator      (S^0)^H dy           (S^1)^H dy
+//               (S^2)^H dy                               (S^3)^H dy
+//   scores      X^H real             X^H imaginary       Y^H real             Y^H imaginary
+//   dk, dv      conj(G X)^T (bf16)   dk accumulator      (G conj Y)^T (bf16)  dv accumulator
+//   carried     (dS^0)^H v           (dS^1)^H v          dS^0 k               dS^1 k         (then states 2, 3)
+//
+// Decay: D factors as e^{A_t - A_m} e^{A_m - A_s} around the middle of the chunk; a state whose chunk decays by more than
+// e^-80 takes one exponential per score instead (see pam_scan_tc2.cuh).
+#pragma once
+#include "pam_scan_tc2.cuh"
+
+namespace qpam {
+namespace tcs {
+
+constexpr int BT = 512;                    // threads
+constexpr size_t BWDK_SMEM = 1024 + 4 * 32768 + 4 * 16384 + KMAX * TC * (4 + 4 + 8 + 4) + 4 * KMAX * TC * 8 + 256;
+
+// acc (real parts at acc, imaginary at acc + 64) = A (.) state planes, as bw_issue_state
+template <bool OP_H>
+__device__ __forceinline__ void issue_state(uint32_t acc, uint32_t a_r, uint32_t s_r) { bw_issue_state<OP_H>(acc - 128, a_r, s_r, false); }
+
+// acc = T X2, T's packed scores in the columns its fp32 scores had: of every 16 columns the first 8 hold the real parts
+__device__ __forceinline__ void issue_rows(uint32_t t, uint32_t acc, uint32_t x_r) {
+  using namespace umma;
+  constexpr uint32_t id = idesc_bf16(128, 64, false, true);
+  constexpr uint32_t idn = idesc_bf16_nega(128, 64, false, true);
+  const uint32_t x_i = x_r + 16384;
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk)
+    mma_bf16_ts(acc, t + 16 * kk, smem_desc_sw128(x_r + kk * 2048, 16, 1024), id, kk > 0);
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk)
+    mma_bf16_ts(acc, t + 16 * kk + 8, smem_desc_sw128(x_i + kk * 2048, 16, 1024), idn, true);
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk)
+    mma_bf16_ts(acc + 64, t + 16 * kk, smem_desc_sw128(x_i + kk * 2048, 16, 1024), id, kk > 0);
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk)
+    mma_bf16_ts(acc + 64, t + 16 * kk + 8, smem_desc_sw128(x_r + kk * 2048, 16, 1024), id, true);
+}
+
+struct BwdTables {
+  float* A;        // [K][128] cumulative log decay
+  float* col;      // [K][128] e^{A_m - A_s}                       (strong: 1)
+  float* row;      // [K][128] sigma e^{A_t - A_m}, 0 past the end (strong: sigma)
+  float2* w;       // [K][128] conj(c_t) row_t
+};
+
+// Pass A for 16 columns of row r: T = G X over the columns of X, sums of col_s D Z over the columns into zs.
+template <int K, bool STRONG>
+__device__ __forceinline__ void pass_a16(uint32_t tl, int c0, int q4, int r, const BwdTables& tb, uint32_t strong, const float2 (&wk)[K],
+                                         const float (&ar)[K], float2 (&zs)[K]) {
+  using namespace umma;
+  uint32_t out[16];
+  if (c0 > q4 * 32 + 31) {                  // warp-uniform: above the diagonal
+#pragma unroll
+    for (int j = 0; j < 16; ++j) out[j] = 0u;
+  } else {
+    uint32_t xr[16], xi[16], yr[16], yi[16];
+    tmem_ld16x4(tl + c0, xr, tl + 128 + c0, xi, tl + 256 + c0, yr, tl + 384 + c0, yi);
+    const int last = c0 + 15 <= q4 * 32 ? TC : r;      // no diagonal inside the block: every column counts
+#pragma unroll
+    for (int j4 = 0; j4 < 16; j4 += 4) {
+      float cf[K][4];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const float4 v = *reinterpret_cast<const float4*>(tb.col + k * TC + c0 + j4);
+        cf[k][0] = v.x; cf[k][1] = v.y; cf[k][2] = v.z; cf[k][3] = v.w;
+        if (STRONG && ((strong >> k) & 1u)) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) cf[k][e] = __expf(fminf(0.f, ar[k] - tb.A[k * TC + c0 + j4 + e]));
+        }
+      }
+      float tr[4], ti[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int j = j4 + e;
+        const bool on = c0 + j <= last;
+        const float a = __uint_as_float(xr[j]), b = __uint_as_float(xi[j]), c = __uint_as_float(yr[j]), d = __uint_as_float(yi[j]);
+        float gr = 0.f, gi = 0.f;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          gr = fmaf(wk[k].x, cf[k][e], gr);
+          gi = fmaf(wk[k].y, cf[k][e], gi);
+        }
+        float zr = fmaf(a, c, b * d), zi = fmaf(b, c, -(a * d));
+        if (!on) gr = gi = zr = zi = 0.f;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          zs[k].x = fmaf(cf[k][e], zr, zs[k].x);
+          zs[k].y = fmaf(cf[k][e], zi, zs[k].y);
+        }
+        tr[e] = gr * a - gi * b;
+        ti[e] = gr * b + gi * a;
+      }
+      out[j4 >> 1] = pack_bf162(tr[0], tr[1]);
+      out[(j4 >> 1) + 1] = pack_bf162(tr[2], tr[3]);
+      out[8 + (j4 >> 1)] = pack_bf162(ti[0], ti[1]);
+      out[8 + (j4 >> 1) + 1] = pack_bf162(ti[2], ti[3]);
+    }
+  }
+  tmem_st16(tl + c0, out);
+}
+
+// Pass B for 16 columns (tokens t) of row s = r: conj(G X)^T over the columns of X^H, (G conj Y)^T over those of Y^H, sums
+// of sigma e^{A_t - A_m} Re(conj(c) Z) into cs.
+template <int K, bool STRONG>
+__device__ __forceinline__ void pass_b16(uint32_t tl, int c0, int q4, int r, const BwdTables& tb, uint32_t strong, const float (&ck)[K],
+                                         const float (&ar)[K], float (&cs)[K]) {
+  using namespace umma;
+  uint32_t ox[16], oy[16];
+  if (c0 + 15 < q4 * 32) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) ox[j] = oy[j] = 0u;
+  } else {
+    uint32_t xr[16], xi[16], yr[16], yi[16];
+    tmem_ld16x4(tl + c0, xr, tl + 128 + c0, xi, tl + 256 + c0, yr, tl + 384 + c0, yi);
+    const int first = c0 >= q4 * 32 + 31 ? 0 : r;
+#pragma unroll
+    for (int j2 = 0; j2 < 16; j2 += 2) {
+      float2 w[K][2];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const float4 v = *reinterpret_cast<const float4*>(tb.w + k * TC + c0 + j2);
+        w[k][0] = make_float2(v.x, v.y);
+        w[k][1] = make_float2(v.z, v.w);
+        if (STRONG && ((strong >> k) & 1u)) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float f = __expf(fminf(0.f, tb.A[k * TC + c0 + j2 + e] - ar[k]));
+            w[k][e].x *= f;
+            w[k][e].y *= f;
+          }
+        }
+      }
+      float xo[2], xp[2], yo[2], yp[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int j = j2 + e;
+        const bool on = c0 + j >= first;
+        const float a = __uint_as_float(xr[j]), b = __uint_as_float(xi[j]), c = __uint_as_float(yr[j]), d = __uint_as_float(yi[j]);
+        float gr = 0.f, gi = 0.f;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          gr = fmaf(w[k][e].x, ck[k], gr);
+          gi = fmaf(w[k][e].y, ck[k], gi);
+        }
+        float zr = fmaf(a, c, b * d), zi = fmaf(a, d, -(b * c));      // conj(X^H) Y^H
+        if (!on) gr = gi = zr = zi = 0.f;
+#pragma unroll
+        for (int k = 0; k < K; ++k) cs[k] = fmaf(w[k][e].x, zr, fmaf(-w[k][e].y, zi, cs[k]));
+        xo[e] = gr * a + gi * b; xp[e] = gr * b - gi * a;
+        yo[e] = gr * c - gi * d; yp[e] = gr * d + gi * c;
+      }
+      ox[j2 >> 1] = pack_bf162(xo[0], xo[1]);
+      ox[8 + (j2 >> 1)] = pack_bf162(xp[0], xp[1]);
+      oy[j2 >> 1] = pack_bf162(yo[0], yo[1]);
+      oy[8 + (j2 >> 1)] = pack_bf162(yp[0], yp[1]);
+    }
+  }
+  tmem_st16(tl + c0, ox);
+  tmem_st16(tl + 256 + c0, oy);
+}
+
+// carried state (fp32 [64][64] re, im) -> bf16 planes of a slot
+__device__ __forceinline__ void stage_state(unsigned char* slot, const float2* __restrict__ state, int tid) {
+  const float4* sg = reinterpret_cast<const float4*>(state);
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const int idx = tid + BT * it;          // (i, c16): state[i][4*c16 .. +3]
+    const float4 s01 = __ldg(sg + idx * 2), s23 = __ldg(sg + idx * 2 + 1);
+    const int i = idx >> 4, c16 = idx & 15;
+    const uint32_t off = sw128(i, c16 >> 1) + (c16 & 1) * 8;
+    *reinterpret_cast<uint2*>(slot + off) = make_uint2(pack_bf162(s01.x, s01.z), pack_bf162(s23.x, s23.z));
+    *reinterpret_cast<uint2*>(slot + 8192 + off) = make_uint2(pack_bf162(s01.y, s01.w), pack_bf162(s23.y, s23.w));
+  }
+}
+
+// 16 channels of row r (channels [16 cq, 16 cq + 16)) of a de-interleaved tile
+__device__ __forceinline__ void row16(const unsigned char* planes, int r, int cq, float (&re)[16], float (&im)[16]) {
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    const uint4 a = *reinterpret_cast<const uint4*>(planes + sw128(r, 2 * cq + g)), b = *reinterpret_cast<const uint4*>(planes + 16384 + sw128(r, 2 * cq + g));
+    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 x = unpack_bf162(aw[e]), y = unpack_bf162(bw[e]);
+      re[g * 8 + 2 * e] = x.x; re[g * 8 + 2 * e + 1] = x.y;
+      im[g * 8 + 2 * e] = y.x; im[g * 8 + 2 * e + 1] = y.y;
+    }
+  }
+}
+
+// 16 finished channels of a row: into the staging block [2 boxes of 32 channels][128 rows][128 B] of a TMA store, or (a
+// ragged chunk: rows past the end belong to someone else) straight to global memory
+__device__ __forceinline__ void put16(const float (&re)[16], const float (&im)[16], unsigned char* stage, __nv_bfloat16* __restrict__ row, int r, int cq,
+                                      bool bulk, bool valid) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const uint4 pk = make_uint4(pack_bf162(re[4 * g], im[4 * g]), pack_bf162(re[4 * g + 1], im[4 * g + 1]), pack_bf162(re[4 * g + 2], im[4 * g + 2]),
+                          pack_bf162(re[4 * g + 3], im[4 * g + 3]));
+    if (bulk) {
+      *reinterpret_cast<uint4*>(stage + (cq >> 1) * 16384 + r * 128 + (((4 * (cq & 1) + g) ^ (r & 7)) << 4)) = pk;
+    } else if (valid) {
+      *reinterpret_cast<uint4*>(row + cq * 32 + g * 8) = pk;
+    }
+  }
+}
+// box b (0..7: 32 rows of 32 channels) of a staging block leaves by TMA; one thread
+__device__ __forceinline__ void store_box(const CUtensorMap* map, const unsigned char* stage, int b, int row0) {
+  const unsigned char* box = stage + (b >> 2) * 16384 + (b & 3) * 4096;
+  umma::tma_store_2d_keep(map, box, (b >> 2) * 64, row0 + (b & 3) * 32);
+}
+
+// What the CTA that will follow on this SM reads -- tiles, carried states, decays, read-out weights -- into L2, while this
+// one computes (without it every wave of CTAs waits for HBM at its start and at both stagings of the states).  One warp.
+template <int K>
+__device__ __forceinline__ void prefetch_next(const BwdMaps& maps, const ScanParams& p, int lane) {
+  const int next = blockIdx.y * gridDim.x + blockIdx.x + p.sms, h = next / gridDim.x;
+  if (h >= (int)gridDim.y) return;
+  const ChunkLoc N = locate_chunk(p.geom, next - h * gridDim.x);
+  if (!N.valid) return;
+  if (lane < 2) {
+    const int row0 = (N.b * p.H + h) * p.T + N.t0;
+    umma::tma_prefetch_2d(&maps.dy, (p.dy_tokens ? h * 128 : 0) + lane * 64, p.dy_tokens ? N.b * p.T + N.t0 : row0);
+    umma::tma_prefetch_2d(&maps.v, lane * 64, row0);
+    umma::tma_prefetch_2d(&maps.q, lane * 64, row0);
+    umma::tma_prefetch_2d(&maps.k, lane * 64, row0);
+  } else if (lane < 2 + K) {
+    umma::bulk_prefetch(p.states + state_base(p, lane - 2, h, N.slot0 + N.c, TD), 32768);
+    umma::bulk_prefetch(p.dstates + state_base(p, lane - 2, h, N.slot0 + N.c + 1, TD), 32768);
+  }
+  const int k = lane >> 3, i = (lane & 7) * 16;
+  if (k < K && i < N.len) {
+    const size_t g = gamma_base(p, k, N.b, h, N.t0 + i);
+    umma::prefetch_l2(p.gamma + g);
+    if (p.coef) umma::prefetch_l2(p.coef + 2 * g);
+  }
+}
+
+// grid = (chunks, H)
+template <int K>
+__global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ BwdMaps maps, ScanParams p, const float* __restrict__ anchor_parts) {
+  using namespace umma;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char *TQ = smem, *TK = TQ + 32768, *TV = TK + 32768, *TY = TV + 32768;      // q, k, v, dy: real plane, imaginary plane
+  unsigned char* SL = TY + 32768;                                                     // 4 slots of carried-state planes, 16 KB each
+  BwdTables tb;
+  tb.A = reinterpret_cast<float*>(SL + 4 * 16384);
+  tb.col = tb.A + KMAX * TC;
+  tb.w = reinterpret_cast<float2*>(tb.col + KMAX * TC);
+  tb.row = reinterpret_cast<float*>(tb.w + KMAX * TC);
+  float2* dcp = reinterpret_cast<float2*>(tb.row + KMAX * TC);      // [4 channel groups][K][128] shares of dc
+  float* kdp = reinterpret_cast<float*>(SL + 2 * 16384);            // [4][K][128] shares of Re<k, dk>, once no MMA reads the slots
+  uint64_t* bars = reinterpret_cast<uint64_t*>(dcp + 4 * KMAX * TC);
+  enum { B_VY, B_QK, B_SA, B_SB, B_DQ, B_DKV, B_U0, B_C0 = B_U0 + KMAX, N_BARS = B_C0 + KMAX };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + N_BARS);
+  int* failed = reinterpret_cast<int*>(tmem_slot + 1);
+  float* wsum = reinterpret_cast<float*>(failed + 1);               // [K][4]
+  float* anc = wsum + 4 * KMAX;                                     // [K][2]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const ChunkLoc L = locate_chunk(p.geom, blockIdx.x);
+  if (!L.valid) return;
+  const int h = blockIdx.y, len = L.len;
+  const bool has_s = L.c > 0 || p.s0 != nullptr, has_ds = L.c < L.nc - 1 || p.ds_final != nullptr;
+  const int row0 = (L.b * p.H + h) * p.T + L.t0;
+  if (tid == BT - 1) *failed = device_error_now();
+  float graw[4] = {1.f, 1.f, 1.f, 1.f};
+  if (warp >= 1 && warp <= K) warp_cumsum128_load(graw, p.gamma + gamma_base(p, warp - 1, L.b, h, L.t0), len, lane);
+  if (tid == 0) {
+#pragma unroll
+    for (int i = 0; i < N_BARS; ++i) mbar_init(&bars[i], 1);
+    fence_barrier_init();
+    const int dx = p.dy_tokens ? h * 128 : 0, dr = p.dy_tokens ? L.b * p.T + L.t0 : row0;
+    mbar_arrive_expect_tx(&bars[B_VY], 4 * 16384);
+#pragma unroll
+    for (int kb = 0; kb < 2; ++kb) {
+      tma_load_2d(TY + kb * 16384, &maps.dy, &bars[B_VY], dx + kb * 64, dr);
+      tma_load_2d(TV + kb * 16384, &maps.v, &bars[B_VY], kb * 64, row0);
+    }
+    mbar_arrive_expect_tx(&bars[B_QK], 4 * 16384);
+#pragma unroll
+    for (int kb = 0; kb < 2; ++kb) {
+      tma_load_2d(TQ + kb * 16384, &maps.q, &bars[B_QK], kb * 64, row0);
+      tma_load_2d(TK + kb * 16384, &maps.k, &bars[B_QK], kb * 64, row0);
+    }
+  }
+  __syncwarp();
+  const int ek = tid >> 7, et = tid & 127;          // this thread's (state, token) in the tables
+  const size_t eg = gamma_base(p, ek, L.b, h, L.t0 + et);
+  float2 c_e = make_float2(1.f, 0.f);
+  if (p.coef != nullptr && ek < K && et < len) c_e = __ldg(reinterpret_cast<const float2*>(p.coef + eg * 2));
+  // what the decay gradient needs at the end, requested now: the decay of this thread's token, and per state the partial
+  // sums of the anchors at the chunk's first token and just after the chunk (two warps of the state's four)
+  const int et_rev = TC - 1 - et;
+  float g_e = 1.f, an0 = 0.f, an1 = 0.f;
+  if (ek < K) {
+    if (et_rev < len) g_e = __ldg(p.gamma + eg - et + et_rev);
+    if ((warp & 3) < 2) {
+      const float* ap = anchor_parts + (((size_t)ek * p.H + h) * p.nslots + L.slot0 + L.c + (warp & 3)) * ANCHOR_PARTS;
+      an0 = __ldg(ap + lane);
+      an1 = __ldg(ap + lane + 32);
+    }
+  }
+  if (warp == 0) tmem_alloc<512>(tmem_slot);
+  if (warp >= 1 && warp <= K) warp_cumsum128_finish(tb.A + (warp - 1) * TC, graw, len, p.eps, lane);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  if (*failed != 0) {       // an earlier launch gave up on a wait: outputs stay untouched (the tiles still have to land)
+    mbar_wait(&bars[B_VY], 0, 250);
+    mbar_wait(&bars[B_QK], 0, 250);
+    __syncthreads();
+    if (warp == 0) tmem_dealloc<512>(tmem);
+    return;
+  }
+  uint32_t strong = 0;
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (tb.A[k * TC + TC - 1] < STRONG_DECAY) strong |= 1u << k;
+  if (ek < K) {
+    const bool st = (strong >> ek) & 1u;
+    const float a = tb.A[ek * TC + et], a_mid = tb.A[ek * TC + TC / 2 - 1];
+    const float rf = et < len ? p.q_scale * (st ? 1.f : __expf(a - a_mid)) : 0.f;
+    tb.col[ek * TC + et] = st ? 1.f : __expf(a_mid - a);
+    tb.row[ek * TC + et] = rf;
+    tb.w[ek * TC + et] = make_float2(c_e.x * rf, -c_e.y * rf);
+    if ((warp & 3) < 2) {
+      double a2 = (double)an0 + (double)an1;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+      if (lane == 0) anc[ek * 2 + (warp & 3)] = (float)a2;
+    }
+  }
+  const uint32_t q_r = smem_u32(TQ), k_r = smem_u32(TK), v_r = smem_u32(TV), y_r = smem_u32(TY), sl = smem_u32(SL);
+  const bool issuer = warp == 0 && elect_one();
+  // de-interleave dy and v, start X; then q and k, start Y
+  bool ok = mbar_wait(&bars[B_VY], 0, 251);
+  {
+    const int row = tid & 127, hb = (tid >> 7) & 1;
+    unsigned char* tile = tid < 256 ? TY : TV;
+    uint4 ra[8];
+    deint_read(tile, row, hb, ra);
+    __syncthreads();
+    deint_write(tile, row, hb, ra);
+    fence_proxy_async();
+    __syncthreads();
+    if (issuer) bw_issue_scores(tmem, y_r, v_r);
+    __syncwarp();
+    ok = mbar_wait(&bars[B_QK], 0, 252) && ok;
+    tile = tid < 256 ? TQ : TK;
+    deint_read(tile, row, hb, ra);
+    __syncthreads();
+    deint_write(tile, row, hb, ra);
+    fence_proxy_async();
+    __syncthreads();
+    if (issuer) {
+      bw_issue_scores(tmem + 256, q_r, k_r);
+      mma_commit(&bars[B_SA]);
+    }
+    __syncwarp();
+  }
+  if (has_s) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) stage_state(SL + k * 16384, p.states + state_base(p, k, h, L.slot0 + L.c, TD), tid);
+  }
+  const int q4 = warp & 3, cq = warp >> 2;
+  const int r = q4 * 32 + lane;                                   // this thread's row (TMEM lane)
+  const uint32_t tl = tmem + ((uint32_t)(q4 * 32) << 16);
+  const bool valid = r < len;
+  const size_t obase = token_base(p, L.b, h, L.t0 + r, TD);
+  float ar[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) ar[k] = tb.A[k * TC + r];
+
+  // ---- pass A: rows t
+  float2 wk[K], zs[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    wk[k] = tb.w[k * TC + r];
+    zs[k] = make_float2(0.f, 0.f);
+  }
+  ok = mbar_wait(&bars[B_SA], 0, 253) && ok;
+  tc_fence_after();
+#pragma unroll 1
+  for (int hh = 0; hh < 2; ++hh) {
+    const int c0 = cq * 32 + hh * 16;
+    if (strong == 0u) pass_a16<K, false>(tl, c0, q4, r, tb, 0u, wk, ar, zs);
+    else pass_a16<K, true>(tl, c0, q4, r, tb, strong, wk, ar, zs);
+  }
+  tmem_st_wait();
+  fence_proxy_async();
+  tc_fence_before();
+  __syncthreads();
+  if (issuer) {
+    tc_fence_after();
+    issue_rows(tmem, tmem + 128, k_r);
+    mma_commit(&bars[B_DQ]);
+    if (has_s) {
+      issue_state<true>(tmem + 256, y_r, sl);
+      mma_commit(&bars[B_U0]);
+      issue_state<true>(tmem + 384, y_r, sl + 16384);
+      mma_commit(&bars[B_U0 + 1]);
+      if (K > 2 && mbar_wait(&bars[B_DQ], 0, 254)) {      // the packed scores have been consumed: state 2 takes their columns
+        issue_state<true>(tmem, y_r, sl + 2 * 16384);
+        mma_commit(&bars[B_U0 + 2]);
+      }
+    }
+  }
+  __syncwarp();
+  if (warp == 8) prefetch_next<K>(maps, p, lane);
+  ok = mbar_wait(&bars[B_DQ], 0, 254) && ok;
+  tc_fence_after();
+  {
+    float vr[16], vi[16];
+    tmem_ld16x2(tl + 128 + 16 * cq, vr, tl + 192 + 16 * cq, vi);
+    if (has_s) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        ok = mbar_wait(&bars[B_U0 + k], 0, 255) && ok;
+        tc_fence_after();
+        const uint32_t at = tl + (k == 1 ? 384u : k == 2 ? 0u : 256u) + 16 * cq;
+        float ur[16], ui[16], xr[16], xi[16];
+        tmem_ld16x2(at, ur, at + 64, ui);
+        if (k == 0 && K > 3) {              // read by everyone: state 3 takes the columns of state 0
+          tc_fence_before();
+          __syncthreads();
+          if (issuer) {
+            tc_fence_after();
+            issue_state<true>(tmem + 256, y_r, sl + 3 * 16384);
+            mma_commit(&bars[B_U0 + 3]);
+          }
+          __syncwarp();
+        }
+        row16(TQ, r, cq, xr, xi);
+        const float f = __expf(((strong >> k) & 1u) ? ar[k] : tb.A[k * TC + TC / 2 - 1]);      // row_t f = sigma e^{A_t}
+        const float wr = wk[k].x * f, wi = wk[k].y * f;
+        float er = 0.f, ei = 0.f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          er = fmaf(xr[j], ur[j], fmaf(xi[j], ui[j], er));
+          ei = fmaf(xr[j], ui[j], fmaf(-xi[j], ur[j], ei));
+          vr[j] += wr * ur[j] - wi * ui[j];
+          vi[j] += wr * ui[j] + wi * ur[j];
+        }
+        zs[k].x = fmaf(f, er, zs[k].x);
+        zs[k].y = fmaf(f, ei, zs[k].y);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float rw = tb.row[k * TC + r];
+      dcp[(cq * K + k) * TC + r] = make_float2(rw * zs[k].x, rw * zs[k].y);
+    }
+    tc_fence_before();
+    __syncthreads();                        // accumulators and state slots have been read
+    if (issuer) {
+      tc_fence_after();
+      bw_issue_scores(tmem, v_r, y_r);
+      bw_issue_scores(tmem + 256, k_r, q_r);
+      mma_commit(&bars[B_SB]);
+    }
+    __syncwarp();
+    put16(vr, vi, SL, reinterpret_cast<__nv_bfloat16*>(p.dq) + obase, r, cq, len == TC, valid && ok);
+  }
+  fence_proxy_async();
+  __syncthreads();
+  if (warp >= 8 && lane == 0 && len == TC && ok) {
+    store_box(&maps.dq, SL, warp - 8, row0);
+    if (K > 2) tma_store_wait_read();
+  }
+  if (K > 2) __syncthreads();               // the staging block has left: its slots are free
+  if (has_ds) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) stage_state(SL + ((k + 2) & 3) * 16384, p.dstates + state_base(p, k, h, L.slot0 + L.c + 1, TD), tid);
+  }
+
+  // ---- pass B: rows s
+  float ck[K], cs[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    ck[k] = tb.col[k * TC + r];
+    cs[k] = 0.f;
+  }
+  ok = mbar_wait(&bars[B_SB], 0, 256) && ok;
+  tc_fence_after();
+#pragma unroll 1
+  for (int hh = 0; hh < 2; ++hh) {
+    const int c0 = cq * 32 + hh * 16;
+    if (strong == 0u) pass_b16<K, false>(tl, c0, q4, r, tb, 0u, ck, ar, cs);
+    else pass_b16<K, true>(tl, c0, q4, r, tb, strong, ck, ar, cs);
+  }
+  tmem_st_wait();
+  fence_proxy_async();
+  tc_fence_before();
+  __syncthreads();
+  if (issuer) {
+    tc_fence_after();
+    issue_rows(tmem, tmem + 128, q_r);
+    issue_rows(tmem + 256, tmem + 384, y_r);
+    mma_commit(&bars[B_DKV]);
+    if (has_ds && mbar_wait(&bars[B_DKV], 0, 257)) {       // the packed scores have been consumed: state 0 takes their columns
+      issue_state<true>(tmem, v_r, sl + 2 * 16384);
+      issue_state<false>(tmem + 256, k_r, sl + 2 * 16384);
+      mma_commit(&bars[B_C0]);
+    }
+  }
+  __syncwarp();
+  ok = mbar_wait(&bars[B_DKV], 0, 257) && ok;
+  tc_fence_after();
+  {
+    float kr[16], ki[16], vr[16], vi[16];           // dk, dv
+    tmem_ld16x2(tl + 128 + 16 * cq, kr, tl + 192 + 16 * cq, ki);
+    tmem_ld16x2(tl + 384 + 16 * cq, vr, tl + 448 + 16 * cq, vi);
+#pragma unroll
+    for (int k = 0; k < K; ++k) cs[k] *= ck[k];
+    if (has_ds) {
+      // state k uses the columns of the packed scores (k even) or of the accumulators (k odd); it is issued as soon as
+      // everyone has read what was there
+      auto issue_carried = [&](int k) {
+        tc_fence_before();
+        __syncthreads();
+        if (issuer) {
+          tc_fence_after();
+          const uint32_t s_r = sl + ((k + 2) & 3) * 16384;
+          issue_state<true>(tmem + 128 * (k & 1), v_r, s_r);
+          issue_state<false>(tmem + 256 + 128 * (k & 1), k_r, s_r);
+          mma_commit(&bars[B_C0 + k]);
+        }
+        __syncwarp();
+      };
+      issue_carried(1);
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        ok = mbar_wait(&bars[B_C0 + k], 0, 258) && ok;
+        tc_fence_after();
+        const uint32_t at = tl + 128 * (k & 1) + 16 * cq;
+        const float e = __expf(fminf(0.f, tb.A[k * TC + TC - 1] - ar[k]));
+        float ur[16], ui[16];
+        {
+          float xr[16], xi[16];
+          tmem_ld16x2(at, ur, at + 64, ui);
+          row16(TK, r, cq, xr, xi);
+          float d = 0.f;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            d = fmaf(xr[j], ur[j], fmaf(xi[j], ui[j], d));
+            kr[j] = fmaf(e, ur[j], kr[j]);
+            ki[j] = fmaf(e, ui[j], ki[j]);
+          }
+          cs[k] = fmaf(e, d, cs[k]);
+        }
+        tmem_ld16x2(at + 256, ur, at + 320, ui);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          vr[j] = fmaf(e, ur[j], vr[j]);
+          vi[j] = fmaf(e, ui[j], vi[j]);
+        }
+        if (k + 2 < K) issue_carried(k + 2);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) kdp[(cq * K + k) * TC + r] = cs[k];
+    // q and dy have no reader left: their tiles take the rows of dk and dv
+    put16(kr, ki, TQ, reinterpret_cast<__nv_bfloat16*>(p.dk) + obase, r, cq, len == TC, valid && ok);
+    put16(vr, vi, TY, reinterpret_cast<__nv_bfloat16*>(p.dv) + obase, r, cq, len == TC, valid && ok);
+  }
+  fence_proxy_async();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc<512>(tmem);
+  }
+  if (lane == 0 && len == TC && ok) {
+    if (warp < 8) store_box(&maps.dk, TQ, warp, row0);
+    else store_box(&maps.dv, TY, warp - 8, row0);
+  }
+
+  // ---- dc, and the decay gradient: da_u = sum_{t >= u} (Re<q,dq> - Re<k,dk>)_t.  The raw values would accumulate their
+  // errors as a random walk over the whole sequence, so the suffix sum is anchored at every chunk boundary with the value
+  // the reverse carry left there (Re<dS, S>, fp32) and the small mismatch of the chunk is spread linearly over its tokens.
+  float suffix = 0.f;
+  if (ek < K) {
+    float2 dc = make_float2(0.f, 0.f);
+    float kd = 0.f;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const float2 a = dcp[(g * K + ek) * TC + et];
+      dc.x += a.x;
+      dc.y += a.y;
+      kd += kdp[(g * K + ek) * TC + et];
+    }
+    if (p.dcoef != nullptr && et < len && ok) *reinterpret_cast<float2*>(p.dcoef + eg * 2) = dc;
+    tb.row[ek * TC + et] = et < len ? c_e.x * dc.x + c_e.y * dc.y - kd : 0.f;
+  }
+  __syncthreads();
+  if (ek < K) {
+    suffix = tb.row[ek * TC + et_rev];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float n = __shfl_up_sync(0xffffffffu, suffix, o);
+      if (lane >= o) suffix += n;
+    }
+    if (lane == 31) wsum[ek * 4 + (warp & 3)] = suffix;
+  }
+  __syncthreads();
+  if (ek < K) {
+    const int w = warp & 3;
+    for (int i = 0; i < w; ++i) suffix += wsum[ek * 4 + i];
+    const float total = wsum[ek * 4] + wsum[ek * 4 + 1] + wsum[ek * 4 + 2] + wsum[ek * 4 + 3];
+    const float lo = anc[ek * 2], hi = anc[ek * 2 + 1], mismatch = total - (lo - hi);
+    if (et_rev < len && ok) {
+      const size_t gi = gamma_base(p, ek, L.b, h, L.t0 + et_rev);
+      p.dgamma[gi] = (hi + suffix - mismatch * (float)(len - et_rev) / (float)len) / (g_e + p.eps);
+    }
+  }
+  if (lane == 0) tma_store_wait_read();     // the staging blocks are read before this CTA's shared memory goes away
+}
+
+}  // namespace tcs
+}  // namespace qpam
