@@ -416,7 +416,6 @@ static int scan_bwd_tcK(const qpam_scan_args* a, const ScanLayout& L, const void
   p.dy = dy; p.dq = dq; p.dk = dk; p.dv = dv;
   p.dgamma = dgamma; p.dcoef = dcoef; p.ds_final = ds_final; p.ds0 = ds0;
   p.dy_tokens = dy_tokens ? 1 : 0;
-  p.sms = sm_count();
   int rc;
   if (!states_valid) {
     ScanParams pf = p;

@@ -110,7 +110,6 @@ struct ScanParams {
   float q_scale, eps;
   int32_t y_token_major;   // tensor-core forward kernels only: y laid out [B,T,H,d,2] instead of [B,H,T,d,2]
   int32_t dy_tokens;       // K-state tensor-core backward only: the same for dy
-  int32_t sms;             // multiprocessors (K-state tensor-core backward: whose tiles to prefetch)
   // Tensor-core forward of which no backward will read the states: what only a backward needs is not written (see
   // k_state_scan), and the final states may go to slots of a state pool [n_slots,L,K,H,D,D,2] instead of s_final.
   int32_t fwd_only;

@@ -16,7 +16,7 @@
 //
 //
 // (One state keeps the three-job kernel of pam_scan_tc2.cuh: two CTAs on an SM hide each other's waits there, 108 us against
-// 118 us here at 8 x 6 x 2048; three states took 420 us that way, read-out weights included, and take 235 us.)
+// 118 us here at 8 x 6 x 2048; three states took 420 us that way, read-out weights included, and take 229 us.)
 //
 // Every score is formed twice, once per direction of the sum (a row of the tile is a TMEM lane, so sums along a row stay
 // inside threads): pass A has tokens t as rows (dq, dc), pass B tokens s (dk, dv, Re<k,dk>).  512 threads: a thread owns a
@@ -24,11 +24,10 @@
 //
 //   TMEM        [0,128)              [128,256)           [256,384)            [384,512)
 //   scores      X real               X imaginary         Y real               Y imaginary
-//   dq          G X (bf16)           dq accumulator      (S^0)^H dy           (S^1)^H dy
-//               (S^2)^H dy                               (S^3)^H dy
+//   dq          G X (bf16)           dq accumulator      (S^0)^H dy           (S^1)^H dy     (then states 2, 3)
 //   scores      X^H real             X^H imaginary       Y^H real             Y^H imaginary
 //   dk, dv      conj(G X)^T (bf16)   dk accumulator      (G conj Y)^T (bf16)  dv accumulator
-//   carried     (dS^0)^H v           (dS^1)^H v          dS^0 k               dS^1 k         (then states 2, 3)
+//   carried     (dS^0)^H v                               dS^0 k                              (then states 1, 2; then 3)
 //
 // Decay: D factors as e^{A_t - A_m} e^{A_m - A_s} around the middle of the chunk; a state whose chunk decays by more than
 // e^-80 takes one exponential per score instead (see pam_scan_tc2.cuh).
@@ -188,17 +187,18 @@ __device__ __forceinline__ void pass_b16(uint32_t tl, int c0, int q4, int r, con
   tmem_st16(tl + 256 + c0, oy);
 }
 
-// carried state (fp32 [64][64] re, im) -> bf16 planes of a slot
+// carried state (fp32 [64][64] re, im) -> bf16 planes of a slot; a warp's 512 consecutive bytes are one row
 __device__ __forceinline__ void stage_state(unsigned char* slot, const float2* __restrict__ state, int tid) {
   const float4* sg = reinterpret_cast<const float4*>(state);
+  float4 v[4];
 #pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int idx = tid + BT * it;          // (i, c16): state[i][4*c16 .. +3]
-    const float4 s01 = __ldg(sg + idx * 2), s23 = __ldg(sg + idx * 2 + 1);
-    const int i = idx >> 4, c16 = idx & 15;
-    const uint32_t off = sw128(i, c16 >> 1) + (c16 & 1) * 8;
-    *reinterpret_cast<uint2*>(slot + off) = make_uint2(pack_bf162(s01.x, s01.z), pack_bf162(s23.x, s23.z));
-    *reinterpret_cast<uint2*>(slot + 8192 + off) = make_uint2(pack_bf162(s01.y, s01.w), pack_bf162(s23.y, s23.w));
+  for (int it = 0; it < 4; ++it) v[it] = __ldg(sg + tid + BT * it);
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int i = (tid + BT * it) >> 5, c = tid & 31;      // row i, columns 2c and 2c + 1
+    const uint32_t off = sw128(i, c >> 2) + (c & 3) * 4;
+    *reinterpret_cast<uint32_t*>(slot + off) = pack_bf162(v[it].x, v[it].z);
+    *reinterpret_cast<uint32_t*>(slot + 8192 + off) = pack_bf162(v[it].y, v[it].w);
   }
 }
 
@@ -238,32 +238,6 @@ __device__ __forceinline__ void store_box(const CUtensorMap* map, const unsigned
   umma::tma_store_2d_keep(map, box, (b >> 2) * 64, row0 + (b & 3) * 32);
 }
 
-// What the CTA that will follow on this SM reads -- tiles, carried states, decays, read-out weights -- into L2, while this
-// one computes (without it every wave of CTAs waits for HBM at its start and at both stagings of the states).  One warp.
-template <int K>
-__device__ __forceinline__ void prefetch_next(const BwdMaps& maps, const ScanParams& p, int lane) {
-  const int next = blockIdx.y * gridDim.x + blockIdx.x + p.sms, h = next / gridDim.x;
-  if (h >= (int)gridDim.y) return;
-  const ChunkLoc N = locate_chunk(p.geom, next - h * gridDim.x);
-  if (!N.valid) return;
-  if (lane < 2) {
-    const int row0 = (N.b * p.H + h) * p.T + N.t0;
-    umma::tma_prefetch_2d(&maps.dy, (p.dy_tokens ? h * 128 : 0) + lane * 64, p.dy_tokens ? N.b * p.T + N.t0 : row0);
-    umma::tma_prefetch_2d(&maps.v, lane * 64, row0);
-    umma::tma_prefetch_2d(&maps.q, lane * 64, row0);
-    umma::tma_prefetch_2d(&maps.k, lane * 64, row0);
-  } else if (lane < 2 + K) {
-    umma::bulk_prefetch(p.states + state_base(p, lane - 2, h, N.slot0 + N.c, TD), 32768);
-    umma::bulk_prefetch(p.dstates + state_base(p, lane - 2, h, N.slot0 + N.c + 1, TD), 32768);
-  }
-  const int k = lane >> 3, i = (lane & 7) * 16;
-  if (k < K && i < N.len) {
-    const size_t g = gamma_base(p, k, N.b, h, N.t0 + i);
-    umma::prefetch_l2(p.gamma + g);
-    if (p.coef) umma::prefetch_l2(p.coef + 2 * g);
-  }
-}
-
 // grid = (chunks, H)
 template <int K>
 __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ BwdMaps maps, ScanParams p, const float* __restrict__ anchor_parts) {
@@ -280,7 +254,7 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   float2* dcp = reinterpret_cast<float2*>(tb.row + KMAX * TC);      // [4 channel groups][K][128] shares of dc
   float* kdp = reinterpret_cast<float*>(SL + 2 * 16384);            // [4][K][128] shares of Re<k, dk>, once no MMA reads the slots
   uint64_t* bars = reinterpret_cast<uint64_t*>(dcp + 4 * KMAX * TC);
-  enum { B_VY, B_QK, B_SA, B_SB, B_DQ, B_DKV, B_U0, B_C0 = B_U0 + KMAX, N_BARS = B_C0 + KMAX };
+  enum { B_VY, B_QK, B_SA, B_SB, B_DQ, B_U2, B_DKV, B_C0, B_C1, B_C2, N_BARS };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + N_BARS);
   int* failed = reinterpret_cast<int*>(tmem_slot + 1);
   float* wsum = reinterpret_cast<float*>(failed + 1);               // [K][4]
@@ -362,6 +336,11 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   }
   const uint32_t q_r = smem_u32(TQ), k_r = smem_u32(TK), v_r = smem_u32(TV), y_r = smem_u32(TY), sl = smem_u32(SL);
   const bool issuer = warp == 0 && elect_one();
+  // the states entering the chunk, while the tiles are on their way
+  if (has_s) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) stage_state(SL + k * 16384, p.states + state_base(p, k, h, L.slot0 + L.c, TD), tid);
+  }
   // de-interleave dy and v, start X; then q and k, start Y
   bool ok = mbar_wait(&bars[B_VY], 0, 251);
   {
@@ -387,10 +366,6 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
       mma_commit(&bars[B_SA]);
     }
     __syncwarp();
-  }
-  if (has_s) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) stage_state(SL + k * 16384, p.states + state_base(p, k, h, L.slot0 + L.c, TD), tid);
   }
   const int q4 = warp & 3, cq = warp >> 2;
   const int r = q4 * 32 + lane;                                   // this thread's row (TMEM lane)
@@ -423,20 +398,13 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   if (issuer) {
     tc_fence_after();
     issue_rows(tmem, tmem + 128, k_r);
-    mma_commit(&bars[B_DQ]);
     if (has_s) {
       issue_state<true>(tmem + 256, y_r, sl);
-      mma_commit(&bars[B_U0]);
       issue_state<true>(tmem + 384, y_r, sl + 16384);
-      mma_commit(&bars[B_U0 + 1]);
-      if (K > 2 && mbar_wait(&bars[B_DQ], 0, 254)) {      // the packed scores have been consumed: state 2 takes their columns
-        issue_state<true>(tmem, y_r, sl + 2 * 16384);
-        mma_commit(&bars[B_U0 + 2]);
-      }
     }
+    mma_commit(&bars[B_DQ]);
   }
   __syncwarp();
-  if (warp == 8) prefetch_next<K>(maps, p, lane);
   ok = mbar_wait(&bars[B_DQ], 0, 254) && ok;
   tc_fence_after();
   {
@@ -445,21 +413,22 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
     if (has_s) {
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        ok = mbar_wait(&bars[B_U0 + k], 0, 255) && ok;
-        tc_fence_after();
-        const uint32_t at = tl + (k == 1 ? 384u : k == 2 ? 0u : 256u) + 16 * cq;
-        float ur[16], ui[16], xr[16], xi[16];
-        tmem_ld16x2(at, ur, at + 64, ui);
-        if (k == 0 && K > 3) {              // read by everyone: state 3 takes the columns of state 0
+        if (k == 2) {                       // both accumulators have been read: states 2 and 3
           tc_fence_before();
           __syncthreads();
           if (issuer) {
             tc_fence_after();
-            issue_state<true>(tmem + 256, y_r, sl + 3 * 16384);
-            mma_commit(&bars[B_U0 + 3]);
+            issue_state<true>(tmem + 256, y_r, sl + 2 * 16384);
+            if (K > 3) issue_state<true>(tmem + 384, y_r, sl + 3 * 16384);
+            mma_commit(&bars[B_U2]);
           }
           __syncwarp();
+          ok = mbar_wait(&bars[B_U2], 0, 255) && ok;
+          tc_fence_after();
         }
+        const uint32_t at = tl + 256 + 128 * (k & 1) + 16 * cq;
+        float ur[16], ui[16], xr[16], xi[16];
+        tmem_ld16x2(at, ur, at + 64, ui);
         row16(TQ, r, cq, xr, xi);
         const float f = __expf(((strong >> k) & 1u) ? ar[k] : tb.A[k * TC + TC / 2 - 1]);      // row_t f = sigma e^{A_t}
         const float wr = wk[k].x * f, wi = wk[k].y * f;
@@ -493,14 +462,20 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   }
   fence_proxy_async();
   __syncthreads();
-  if (warp >= 8 && lane == 0 && len == TC && ok) {
-    store_box(&maps.dq, SL, warp - 8, row0);
-    if (K > 2) tma_store_wait_read();
-  }
-  if (K > 2) __syncthreads();               // the staging block has left: its slots are free
+  const bool storing = warp >= 8 && lane == 0 && len == TC && ok;
+  if (storing) store_box(&maps.dq, SL, warp - 8, row0);
+  auto stage_grad = [&](int k) { stage_state(SL + ((k + 2) & 3) * 16384, p.dstates + state_base(p, k, h, L.slot0 + L.c + 1, TD), tid); };
   if (has_ds) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) stage_state(SL + ((k + 2) & 3) * 16384, p.dstates + state_base(p, k, h, L.slot0 + L.c + 1, TD), tid);
+    stage_grad(0);
+    stage_grad(1);
+  }
+  if (K > 2) {
+    if (storing) tma_store_wait_read();
+    __syncthreads();                        // the staging block has left: slots 0 and 1 are free
+    if (has_ds) {
+      stage_grad(2);
+      if (K > 3) stage_grad(3);
+    }
   }
 
   // ---- pass B: rows s
@@ -543,26 +518,28 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
 #pragma unroll
     for (int k = 0; k < K; ++k) cs[k] *= ck[k];
     if (has_ds) {
-      // state k uses the columns of the packed scores (k even) or of the accumulators (k odd); it is issued as soon as
-      // everyone has read what was there
-      auto issue_carried = [&](int k) {
-        tc_fence_before();
-        __syncthreads();
-        if (issuer) {
-          tc_fence_after();
-          const uint32_t s_r = sl + ((k + 2) & 3) * 16384;
-          issue_state<true>(tmem + 128 * (k & 1), v_r, s_r);
-          issue_state<false>(tmem + 256 + 128 * (k & 1), k_r, s_r);
-          mma_commit(&bars[B_C0 + k]);
-        }
-        __syncwarp();
-      };
-      issue_carried(1);
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        ok = mbar_wait(&bars[B_C0 + k], 0, 258) && ok;
-        tc_fence_after();
-        const uint32_t at = tl + 128 * (k & 1) + 16 * cq;
+        if (k == 1 || k == 3) {                     // every accumulator has been read: the next states
+          tc_fence_before();
+          __syncthreads();
+          if (issuer) {
+            tc_fence_after();
+            issue_state<true>(tmem, v_r, sl + ((k + 2) & 3) * 16384);
+            issue_state<false>(tmem + 256, k_r, sl + ((k + 2) & 3) * 16384);
+            if (k == 1 && K > 2) {
+              issue_state<true>(tmem + 128, v_r, sl);
+              issue_state<false>(tmem + 384, k_r, sl);
+            }
+            mma_commit(&bars[k == 1 ? B_C1 : B_C2]);
+          }
+          __syncwarp();
+        }
+        if (k != 2) {
+          ok = mbar_wait(&bars[k == 0 ? B_C0 : k == 1 ? B_C1 : B_C2], 0, 258) && ok;
+          tc_fence_after();
+        }
+        const uint32_t at = tl + (k == 2 ? 128u : 0u) + 16 * cq;
         const float e = __expf(fminf(0.f, tb.A[k * TC + TC - 1] - ar[k]));
         float ur[16], ui[16];
         {
@@ -584,7 +561,6 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
           vr[j] = fmaf(e, ur[j], vr[j]);
           vi[j] = fmaf(e, ui[j], vi[j]);
         }
-        if (k + 2 < K) issue_carried(k + 2);
       }
     }
 #pragma unroll
