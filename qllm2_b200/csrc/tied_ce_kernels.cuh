@@ -248,15 +248,25 @@ __global__ void __launch_bounds__(256) k_ce_rows(CEParams p, float* lse, float* 
   float M = -INFINITY, S = 0.f, tz = 0.f, best = -INFINITY;
   int bi = 0x7fffffff;
   if (n < p.N) {
-    for (int s = part; s < p.nsplit; s += 8) {
-      const size_t o = (size_t)s * p.N + n;
-      const float m = p.pm[o], b = p.pbest[o];
-      const int i = p.pidx[o];
-      const float Mn = fmaxf(M, m);
-      if (Mn > -INFINITY) S = S * expf(M - Mn) + p.ps[o] * expf(m - Mn);
-      M = Mn;
-      tz += p.pt[o];
-      if (b > best || (b == best && i < bi)) { best = b; bi = i; }
+    // four splits' values requested together: the folding is a chain, the loads need not be (99 splits of 100 rows: 16 us)
+    for (int s0 = part; s0 < p.nsplit; s0 += 32) {
+      float m[4], w[4], t[4], b[4];
+      int i[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int s = s0 + 8 * u;
+        const size_t o = (size_t)(s < p.nsplit ? s : part) * p.N + n;
+        m[u] = p.pm[o]; w[u] = p.ps[o]; t[u] = p.pt[o]; b[u] = p.pbest[o]; i[u] = p.pidx[o];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (s0 + 8 * u >= p.nsplit) break;
+        const float Mn = fmaxf(M, m[u]);
+        if (Mn > -INFINITY) S = S * expf(M - Mn) + w[u] * expf(m[u] - Mn);
+        M = Mn;
+        tz += t[u];
+        if (b[u] > best || (b[u] == best && i[u] < bi)) { best = b[u]; bi = i[u]; }
+      }
     }
   }
   sm[part][r] = M; ss[part][r] = S; st_[part][r] = tz; sb[part][r] = best; si[part][r] = bi;

@@ -32,7 +32,7 @@ CETcPlan ce_tc_plan(const qpam_ce_args* a) {
   CETcPlan pl{};
   pl.enabled = a->io_dtype == QPAM_BF16 && (a->F % 8) == 0 && a->N > 0;
   pl.n_tiles = (int32_t)((a->V + 255) / 256);
-  const int64_t row_tiles = (a->N + tc::BM - 1) / tc::BM;
+  const int64_t row_tiles = ((a->N + tc::BM - 1) / tc::BM + 1) & ~(int64_t)1;      // of CTA pairs: an odd last tile has an idle partner
   // vocabulary splits: fill the SMs in whole waves (one CTA per SM: the ring takes ~193 KB)
   const int sms = sm_count();
   int best = 1;
@@ -56,12 +56,15 @@ CETcPlan ce_tc_plan(const qpam_ce_args* a) {
   if (rows < tc::BM) rows = tc::BM;
   pl.chunk_rows = rows;
   const int64_t f_tiles = (a->F + 255) / 256;
-  // split-K of dH: one CTA per SM, so the cost is (waves of CTAs) x (K blocks per split)
+  // split-K of dH: one CTA per SM, so the cost is (waves of CTAs) x (K blocks per split), in K blocks of ~0.55 us, and the
+  // fp32 partials of a split are written and read once more (~5 TB/s).  Few rows take many splits: 509 rows x 768 use 48 of
+  // 148 SMs with eight (77 us) and all of them with 24 (38 us).
   const int64_t kb_total = (a->V + tc::BK - 1) / tc::BK;
   int64_t ks = 1, ks_cost = -1;
-  for (int64_t s = 1; s <= 8 && s <= kb_total; ++s) {
+  for (int64_t s = 1; s <= 48 && s <= kb_total; ++s) {
     const int64_t ctas = f_tiles * ((rows + 2 * tc::BM - 1) / (2 * tc::BM)) * s;     // CTAs of two row tiles
-    const int64_t cost = ((ctas + sms - 1) / sms) * ((kb_total + s - 1) / s + 8);   // + 8: prologue and epilogue of a CTA
+    const int64_t cost = ((ctas + sms - 1) / sms) * ((kb_total + s - 1) / s + 8) +      // + 8: prologue and epilogue of a CTA
+                         s * rows * a->F * 8 / 2750000;
     if (ks_cost < 0 || cost < ks_cost) { ks_cost = cost; ks = s; }
   }
   pl.ksplit = (int32_t)ks;
@@ -76,6 +79,7 @@ CETcPlan ce_tc_plan(const qpam_ce_args* a) {
 // Vocabulary tiles one CTA of the probability pass walks for its row tile: more tiles hide the epilogue of one
 // tile behind the MMAs of the next (two accumulator buffers), fewer fill the last wave better.
 static int probs_tiles_per_cta(int64_t row_tiles, int n_tiles) {
+  row_tiles = (row_tiles + 1) & ~(int64_t)1;      // CTA pairs
   const int sms = sm_count();
   int best = 1;
   double best_eff = -1.0;
