@@ -221,13 +221,14 @@ static int tc_states(const ScanParams& p, const ScanLayout& L, const qpam_scan_a
     tcs::k_tc_chunk_outerK<false><<<dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st>>>(mk, mv, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outerK");
   } else if (L.grid_chunks > 0) {
-    int rc = set_smem(tcs::k_tc_chunk_outer<false>, tcs::OUTER_SMEM);
+    const auto kern = p.fwd_only ? tcs::k_tc_chunk_outer<false, true> : tcs::k_tc_chunk_outer<false>;
+    int rc = set_smem(kern, tcs::OUTER_SMEM);
     if (rc) return rc;
     CUtensorMap mk, mv;
     const int64_t rows = (int64_t)a->B * a->H * a->T;
     if ((rc = make_map(&mk, a->k, 128, rows, 128, 64, 128))) return rc;
     if ((rc = make_map(&mv, a->v, 128, rows, 128, 64, 128))) return rc;
-    tcs::k_tc_chunk_outer<false><<<dim3(L.grid_chunks, a->H, a->K), 256, tcs::OUTER_SMEM, st>>>(mk, mv, p);
+    kern<<<dim3(L.grid_chunks, a->H, a->K), 256, tcs::OUTER_SMEM, st>>>(mk, mv, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outer<state>");
   }
   k_state_scan<false><<<dim3(a->S, a->H * a->K, (64 * 64 / 2 + 255) / 256), 256, 0, st>>>(p, 64);
@@ -444,7 +445,7 @@ static int scan_bwd_tcK(const qpam_scan_args* a, const ScanLayout& L, const void
     tcs::k_tc_chunk_outerK<true><<<dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st>>>(maps.q, maps.dy, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outerK<dstate>");
   }
-  tcs::k_tc_state_scan_rev<<<dim3(a->S, a->H * a->K, 64 * 64 / 2 / 256), 256, 0, st>>>(p, anchors);
+  tcs::k_tc_state_scan_rev<<<dim3(a->S, a->H, 8 * a->K), 256, 0, st>>>(p, anchors);
   QPAM_LAUNCH_CHECK("k_tc_state_scan_rev");
   if (L.grid_chunks == 0) return QPAM_OK;
   switch (a->K) {

@@ -113,7 +113,7 @@ constexpr size_t OUTER_SMEM = 1024 + 32768 + 32768 + 1024;
 // The two token tiles (k and v, or q and dy; maps of [B*H*T rows][128 bf16], boxes of 64 x 128, 128-byte swizzle)
 // arrive by TMA; the value tile lands in the region its planes are then built in: every thread reads its pieces, a
 // barrier, and the planes are written over them.
-template <bool DSTATE>
+template <bool DSTATE, bool FWD_ONLY = false>
 __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant__ CUtensorMap mk,
                                                            const __grid_constant__ CUtensorMap mv, ScanParams p) {
   using namespace umma;
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + cc * 32, d1);
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + 64 + cc * 32, d2);
     const bool even = (lane & 1) == 0;
-    const bool final_now = !DSTATE && p.fwd_only && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
+    const bool final_now = FWD_ONLY && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
     if (final_now) {
       FinalDest fin;
       fin.init(p, L.seq, kst, h);

@@ -572,13 +572,13 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_bwd(const __grid_constant__
 // Re<dS_slot, S_slot> (S: forward state of the slot) -- one value per warp, ANCHOR_PARTS per slot, summed by the
 // chunk kernel.  Scaling S_c by e^x changes the loss by x Re<dS_c, S_c>, so that inner product is the exact
 // value of the suffix sum da at the first token of chunk c, known from fp32 quantities.
-// grid = (S, H * K, 8), 256 threads: every thread owns one float4 (two complex entries) of the state.
+// grid = (S, H, 8 K), 256 threads: every thread owns one float4 (two complex entries) of the state.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_tc_state_scan_rev(ScanParams p, float* __restrict__ anchor_parts) {
-  const int seq = blockIdx.x, h = blockIdx.y % p.H, k = blockIdx.y / p.H;
-  const int e4 = blockIdx.z * 256 + threadIdx.x;
+  const int seq = blockIdx.x, h = blockIdx.y, k = blockIdx.z >> 3, z = blockIdx.z & 7;
+  const int e4 = z * 256 + threadIdx.x;
   constexpr int n4 = TD * TD / 2;
-  const int lane = threadIdx.x & 31, part = blockIdx.z * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, part = z * 8 + (threadIdx.x >> 5);
   int64_t slot0;
   int nc;
   if (p.geom.cu_seqlens == nullptr) {
