@@ -189,6 +189,8 @@ struct Block : Function<Block> {
       a.y = y.data_ptr();
       check(qpam_scan_fwd_tokens(&a, st), "qpam_scan_fwd_tokens");
     } else {
+      // every state's output rounded to bf16 before the read-out, as the per-state form always did: the fused output kernel
+      // rounds once, which is enough to move a gate's phase (see the top of this file)
       const Tensor ys = at::empty({K, s.B, H, s.T, d, 2}, o);
       check(qpam_scan_fwd_states(&a, ys.data_ptr(), st), "qpam_scan_fwd_states");
       void* yk[QPAM_MAX_STATES];

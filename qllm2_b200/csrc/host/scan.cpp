@@ -89,37 +89,26 @@ void state_ptrs(const Tensor& ys, void** out) {
   for (int64_t i = 0; i < K; ++i) out[i] = static_cast<char*>(ys.data_ptr()) + i * step;
 }
 
-// K = 2..4 states over the same bf16 q, k, v (d = 64), with gradients: the chunk sums of all states from one pass, the output
-// kernel per state, and the read-out sum_k c_k y^(k) of the per-state outputs; the backward takes all states at once.  Without
-// read-out weights the per-state outputs themselves are returned, and their gradients' dq, dk, dv added up in one set of
-// buffers (qpam_scan_bwd_state).
+// K = 2..4 states over the same bf16 q, k, v (d = 64), with gradients: the fused K-state kernels, forward and backward (8 x 6 x
+// 2048, three states: 500 us with the output kernel once per state and the read-out as a pass of its own).  Without read-out
+// weights the per-state outputs themselves are returned, and their gradients' dq, dk, dv added up in one set of buffers
+// (qpam_scan_bwd_state).
 struct ScanStates : Function<ScanStates> {
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gamma, const OptTensor& coef_,
                                const OptTensor& s0_, const OptTensor& cu_, double q_scale, double eps, int64_t chunk, bool token_major) {
     const Tensor coef = value(coef_), s0 = value(s0_), cu = value(cu_);
     const Config c{q_scale, eps, chunk};
     const int64_t B = q.size(0), H = q.size(1), T = q.size(2), d = q.size(3), K = gamma.size(0);
-    Tensor ys = at::empty({K, B, H, T, d, 2}, q.options());
-    qpam_scan_args a = scan_args(q, k, v, gamma, Tensor(), s0, cu, Tensor(), Tensor(), c);
+    Tensor y = !coef.defined() ? at::empty({K, B, H, T, d, 2}, q.options()) : token_major ? at::empty({B, T, H * d, 2}, q.options()) : at::empty_like(q);
+    qpam_scan_args a = scan_args(q, k, v, gamma, coef, s0, cu, coef.defined() ? y : Tensor(), Tensor(), c);
     Tensor s_final = final_states(a, q);
     a.s_final = fptr(s_final);
     const bool bwd = needs_grad(q) || needs_grad(k) || needs_grad(v) || needs_grad(gamma) || needs_grad(coef) || needs_grad(s0);
     Tensor ws = workspace(qpam_scan_workspace_bytes(&a, bwd ? 1 : 0), q);
     set_workspace(a, ws);
-    check(qpam_scan_fwd_states(&a, ys.data_ptr(), stream()), "qpam_scan_fwd_states");
-    Tensor y = ys;
-    if (coef.defined()) {
-      void* yk[QPAM_MAX_STATES];
-      state_ptrs(ys, yk);
-      if (token_major) {
-        y = at::empty({B, T, H * d, 2}, q.options());
-        check(qpam_state_combine_tokens_fwd(yk, fptr(coef), y.data_ptr(), QPAM_BF16, (int)K, (int)B, (int)H, (int)T, (int)d, stream()),
-              "qpam_state_combine_tokens_fwd");
-      } else {
-        y = at::empty_like(q);
-        check(qpam_state_combine_fwd(yk, fptr(coef), y.data_ptr(), QPAM_BF16, (int)K, B * H * T, (int)d, stream()), "qpam_state_combine_fwd");
-      }
-    }
+    if (!coef.defined()) check(qpam_scan_fwd_states(&a, y.data_ptr(), stream()), "qpam_scan_fwd_states");
+    else if (token_major) check(qpam_scan_fwd_tokens(&a, stream()), "qpam_scan_fwd_tokens");
+    else check(qpam_scan_fwd(&a, stream()), "qpam_scan_fwd");
     ctx->save_for_backward({q, k, v, gamma, coef, s0, cu, bwd ? ws : Tensor()});
     ctx->saved_data["q_scale"] = q_scale;
     ctx->saved_data["eps"] = eps;

