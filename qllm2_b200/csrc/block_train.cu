@@ -30,6 +30,14 @@ __device__ __forceinline__ uint2 pack4(float a, float b, float c, float d) {
   const __nv_bfloat162 x = __floats2bfloat162_rn(a, b), y = __floats2bfloat162_rn(c, d);
   return make_uint2(*reinterpret_cast<const uint32_t*>(&x), *reinterpret_cast<const uint32_t*>(&y));
 }
+__device__ __forceinline__ void unpack8(const uint4& u, float (&r)[4], float (&i)[4]) {      // four interleaved complex values
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    r[j] = __uint_as_float(w[j] << 16);
+    i[j] = __uint_as_float(w[j] & 0xffff0000u);
+  }
+}
 __device__ __forceinline__ float2 unpack2(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 
 // A CTA takes 256 groups of four source columns of one item.
@@ -193,12 +201,22 @@ __global__ void __launch_bounds__(512) k_act_gate_bwd(const bf16* __restrict__ g
     b4[j] = bias[g * 4 + j];
     be4[j] = SWISH ? beta[g * 4 + j] : 0.f;
   }
+  // the next row is on its way while this one is computed (~100 instructions and six special functions for 20 bytes)
+  uint4 na = make_uint4(0u, 0u, 0u, 0u), nu = na, ng = na;
+  auto request = [&](int64_t row) {
+    if (row >= N) return;
+    const int64_t at = (row * C + g * 4) * 2;
+    na = *reinterpret_cast<const uint4*>(gate + at);
+    nu = *reinterpret_cast<const uint4*>(up + at);
+    ng = *reinterpret_cast<const uint4*>(dout + at);
+  };
+  request(blockIdx.y);
   for (int64_t row = blockIdx.y; row < N; row += gridDim.y) {
     float ar[4], ai[4], ur[4], ui[4], gr[4], gi[4], dr[4], di[4];
-    const int64_t at = (row * C + g * 4) * 2;
-    V4<bf16>::ld(gate + at, ar, ai);
-    V4<bf16>::ld(up + at, ur, ui);
-    V4<bf16>::ld(dout + at, gr, gi);
+    unpack8(na, ar, ai);
+    unpack8(nu, ur, ui);
+    unpack8(ng, gr, gi);
+    request(row + gridDim.y);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const MagInv um = mag_inv(ur[j] * ur[j] + ui[j] * ui[j] + MAG_EPS), gm = mag_inv(ar[j] * ar[j] + ai[j] * ai[j] + MAG_EPS);
@@ -269,17 +287,37 @@ __global__ void __launch_bounds__(128) k_cnorm_res_bwd(const bf16* __restrict__ 
     for (int j = 0; j < 4; ++j) acc[v][j] = 0.f;
   for (int64_t row = warp; row < N; row += nwarps) {
     const int64_t base = row * (int64_t)D * 2;
-    float re[MAXV][4], im[MAXV][4], gr[MAXV][4], gi[MAXV][4], ss = 0.f;
+    // everything the row needs is requested before the first reduction (as it arrives: 16 bytes are eight scalars)
+    uint4 zp[MAXV], rp[MAXV], dp[MAXV];
+    uint2 mp[MAXV];
+    float gr[MAXV][4], gi[MAXV][4], ss = 0.f;
 #pragma unroll
     for (int v = 0; v < MAXV; ++v) {
       const int g = v * 32 + lane;
       if (g < groups) {
-        V4<bf16>::ld(z + base + g * 8, re[v], im[v]);
+        zp[v] = *reinterpret_cast<const uint4*>(z + base + g * 8);
         V4<bf16>::ld(dxn + base + g * 8, gr[v], gi[v]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) ss += re[v][j] * re[v][j] + im[v][j] * im[v][j] + MAG_EPS;
       }
     }
+#pragma unroll
+    for (int v = 0; v < MAXV; ++v) {
+      const int g = v * 32 + lane;
+      rp[v] = dp[v] = make_uint4(0u, 0u, 0u, 0u);
+      mp[v] = make_uint2(0u, 0u);
+      if (g < groups) {
+        if (dres) rp[v] = *reinterpret_cast<const uint4*>(dres + base + g * 8);
+        if (dmag) mp[v] = *reinterpret_cast<const uint2*>(dmag + row * (int64_t)D + g * 4);
+        if (delta) dp[v] = *reinterpret_cast<const uint4*>(delta + base + g * 8);
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < MAXV; ++v)
+      if (v * 32 + lane < groups) {
+        float re[4], im[4];
+        unpack8(zp[v], re, im);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ss += re[j] * re[j] + im[j] * im[j] + MAG_EPS;
+      }
     ss = warp_sum(ss);
     const float rrms = rsqrtf(ss / (float)D + eps);
     float cs = 0.f;
@@ -289,20 +327,22 @@ __global__ void __launch_bounds__(128) k_cnorm_res_bwd(const bf16* __restrict__ 
       if (g < groups) {
         const float4 sc = *reinterpret_cast<const float4*>(scale + g * 4);
         const float s4[4] = {sc.x, sc.y, sc.z, sc.w};
-        float dm[4] = {0.f, 0.f, 0.f, 0.f};
-        if (dmag) E4<bf16>::ld(dmag + row * (int64_t)D + g * 4, dm);
+        const float2 m01 = unpack2(mp[v].x), m23 = unpack2(mp[v].y);
+        const float dm[4] = {m01.x, m01.y, m23.x, m23.y};
+        float re[4], im[4];
+        unpack8(zp[v], re, im);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const MagInv m = mag_inv(re[v][j] * re[v][j] + im[v][j] * im[v][j] + MAG_EPS);
+          const MagInv m = mag_inv(re[j] * re[j] + im[j] * im[j] + MAG_EPS);
           const float mi = m.mag * m.inv;
           if (dmag) {                         // d|xn| / dxn = xn / |xn| at the rounded xn
             const float wv = mi * rrms * s4[j];
-            const float xr = round_bf16(re[v][j] * wv), xi = round_bf16(im[v][j] * wv);
+            const float xr = round_bf16(re[j] * wv), xi = round_bf16(im[j] * wv);
             const float q = dm[j] * mag_inv(xr * xr + xi * xi + MAG_EPS).rmag;
             gr[v][j] = fmaf(q, xr, gr[v][j]);
             gi[v][j] = fmaf(q, xi, gi[v][j]);
           }
-          cs += (gr[v][j] * re[v][j] + gi[v][j] * im[v][j]) * s4[j] * mi;
+          cs += (gr[v][j] * re[j] + gi[v][j] * im[j]) * s4[j] * mi;
         }
       }
     }
@@ -314,23 +354,24 @@ __global__ void __launch_bounds__(128) k_cnorm_res_bwd(const bf16* __restrict__ 
       if (g < groups) {
         const float4 sc = *reinterpret_cast<const float4*>(scale + g * 4);
         const float s4[4] = {sc.x, sc.y, sc.z, sc.w};
-        float rr[4] = {0.f, 0.f, 0.f, 0.f}, ri[4] = {0.f, 0.f, 0.f, 0.f};
-        if (dres) V4<bf16>::ld(dres + base + g * 8, rr, ri);
+        float re[4], im[4], rr[4], ri[4];
+        unpack8(zp[v], re, im);
+        unpack8(rp[v], rr, ri);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const MagInv m = mag_inv(re[v][j] * re[v][j] + im[v][j] * im[v][j] + MAG_EPS);
+          const MagInv m = mag_inv(re[j] * re[j] + im[j] * im[j] + MAG_EPS);
           const float mi = m.mag * m.inv;
-          const float q = gr[v][j] * re[v][j] + gi[v][j] * im[v][j];
+          const float q = gr[v][j] * re[j] + gi[v][j] * im[j];
           const float wv = mi * rrms * s4[j];
           const float kk = q * s4[j] * MAG_EPS * rrms * m.inv * m.inv * m.rmag - common;
           acc[v][j] += q * mi * rrms;
-          rr[j] = round_bf16(rr[j] + gr[v][j] * wv + re[v][j] * kk);
-          ri[j] = round_bf16(ri[j] + gi[v][j] * wv + im[v][j] * kk);
+          rr[j] = round_bf16(rr[j] + gr[v][j] * wv + re[j] * kk);
+          ri[j] = round_bf16(ri[j] + gi[v][j] * wv + im[j] * kk);
         }
         V4<bf16>::st(dz + base + g * 8, rr, ri);
         if (delta) {
           float xr[4], xi[4];
-          V4<bf16>::ld(delta + base + g * 8, xr, xi);
+          unpack8(dp[v], xr, xi);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             ds = fmaf(rr[j], xr[j], ds);
@@ -358,22 +399,23 @@ __global__ void __launch_bounds__(128) k_cnorm_res_bwd(const bf16* __restrict__ 
 }
 
 // ------------------------------------------------------------------------------------------------ PAM front
-// The adjoint of k_pam_front.  A CTA walks tiles of FRONT_TOK tokens: threads own (token, head, group of 4 channels) of
+// The adjoint of k_pam_front.  A CTA walks tiles of `tile_tok` tokens: threads own (token, head, group of 4 channels) of
 // q, k, v; d/4 neighbouring lanes sum a head's Re<dv, v>, which the gate threads -- one (token, head) each -- turn into
-// the protect gate's gradient beside the decay's and the read-out weights'.
-constexpr int FRONT_TOK = 4;
-__global__ void __launch_bounds__(1024) k_front_bwd(const __grid_constant__ qpam_front_bwd_args p, int per_tok_pad) {
+// the protect gate's gradient beside the decay's and the read-out weights'.  A tile is as long as the grid allows (28 tokens
+// at 16384 tokens): its two barriers and the gates' chain of small loads and transcendentals are paid once for all its
+// tokens, while another CTA of the SM streams (112 us with tiles of four tokens, 27 us of traffic).
+__global__ void __launch_bounds__(1024) k_front_bwd(const __grid_constant__ qpam_front_bwd_args p, int per_tok_pad, int tile_tok) {
   const qpam_front_args& a = p.f;
-  extern __shared__ float domp[];             // [FRONT_TOK][H], then the CTA's sums [FRONT_TOK * H][3K + 1]
+  extern __shared__ float domp[];             // [tile_tok][H], then the CTA's sums [tile_tok * H][3K + 1]
   const int H = a.H, K = a.K, d = a.d, gph = d >> 2, tid = threadIdx.x;
-  const int64_t ntok = (int64_t)a.B * a.T, ntile = (ntok + FRONT_TOK - 1) / FRONT_TOK;
+  const int64_t ntok = (int64_t)a.B * a.T, ntile = (ntok + tile_tok - 1) / tile_tok;
   const int64_t side = (int64_t)H * d * 2;
   const int slots = blockDim.x / per_tok_pad;   // tokens in flight
   const int my_u = tid / per_tok_pad, idx = tid - my_u * per_tok_pad;
   const bool main_on = my_u < slots && idx < H * gph;
   const int h = main_on ? idx / gph : 0, g = main_on ? idx - h * gph : 0;
   const int NS = 3 * K + 1;
-  const bool gate_on = tid < FRONT_TOK * H;
+  const bool gate_on = tid < tile_tok * H;
   const int gu = gate_on ? tid / H : 0, gh = gate_on ? tid - gu * H : 0;
   float sx[QPAM_MAX_STATES], sp = 0.f, sph[QPAM_MAX_STATES], ssc[QPAM_MAX_STATES];
 #pragma unroll
@@ -381,10 +423,10 @@ __global__ void __launch_bounds__(1024) k_front_bwd(const __grid_constant__ qpam
   bf16* draw = reinterpret_cast<bf16*>(p.d_raw);
   bf16* drawm = reinterpret_cast<bf16*>(p.d_rawm);
   for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-    for (int u0 = 0; u0 < FRONT_TOK; u0 += slots) {
+    for (int u0 = 0; u0 < tile_tok; u0 += slots) {
       const int u = u0 + my_u;
-      const int64_t tok = tile * FRONT_TOK + u;
-      const bool on = main_on && u < FRONT_TOK && tok < ntok;
+      const int64_t tok = tile * tile_tok + u;
+      const bool on = main_on && u < tile_tok && tok < ntok;
       float dot = 0.f;
       if (on) {
         const int b = (int)(tok / a.T), t = (int)(tok - (int64_t)b * a.T);
@@ -423,7 +465,7 @@ __global__ void __launch_bounds__(1024) k_front_bwd(const __grid_constant__ qpam
       if (on && g == 0) domp[u * H + h] = dot;
     }
     __syncthreads();
-    const int64_t tok = tile * FRONT_TOK + gu;
+    const int64_t tok = tile * tile_tok + gu;
     if (gate_on && tok < ntok) {
       const int b = (int)(tok / a.T), t = (int)(tok - (int64_t)b * a.T);
       const float dtv = __bfloat162float(reinterpret_cast<const bf16*>(a.dt)[tok * a.ld_dt + gh]) + a.dt_bias[gh];
@@ -502,7 +544,7 @@ __global__ void __launch_bounds__(1024) k_front_bwd(const __grid_constant__ qpam
   for (int c = tid; c < H * NS; c += blockDim.x) {
     float v = 0.f;
     const int hh = c / NS, i = c - hh * NS;
-    for (int u = 0; u < FRONT_TOK; ++u) v += domp[(u * H + hh) * NS + i];
+    for (int u = 0; u < tile_tok; ++u) v += domp[(u * H + hh) * NS + i];
     p.part[(int64_t)blockIdx.x * H * NS + c] = v;
   }
 }
@@ -676,11 +718,14 @@ extern "C" int qpam_pam_front_bwd(const qpam_front_bwd_args* p, void* stream) {
   for (int i = 0; i < 4; ++i) QPAM_REQUIRE(p->col[i] < 0 || !p->from_mag[i] || p->d_rawm, "front_bwd: gate columns without their buffer");
   const int per_tok = (a.H * (a.d / 4) + 31) / 32 * 32;
   QPAM_REQUIRE(per_tok <= 1024, "front_bwd: H * d too large");
-  const int slots = std::max(1, std::min(FRONT_TOK, 384 / per_tok));
-  int threads = std::max(per_tok * slots, (FRONT_TOK * a.H + 31) / 32 * 32);
-  const size_t smem = std::max((size_t)FRONT_TOK * a.H * (3 * a.K + 1), (size_t)FRONT_TOK * a.H) * sizeof(float);
+  const int slots = std::max(1, std::min(4, 384 / per_tok));        // tokens in flight
+  const int threads = std::max(per_tok * slots, (slots * a.H + 31) / 32 * 32);
+  const int64_t share = ((int64_t)a.B * a.T + p->P - 1) / p->P;
+  const int most = std::max(slots, std::min(threads, 900) / a.H / slots * slots);     // a gate thread per (token, head); 48 KB of sums
+  const int tile = (int)std::min<int64_t>(most, (share + slots - 1) / slots * slots);
+  const size_t smem = (size_t)tile * a.H * (3 * a.K + 1) * sizeof(float);
   cudaStream_t st = (cudaStream_t)stream;
-  k_front_bwd<<<p->P, threads, smem, st>>>(*p, per_tok);
+  k_front_bwd<<<p->P, threads, smem, st>>>(*p, per_tok, tile);
   QPAM_LAUNCH_CHECK("k_front_bwd");
   return QPAM_OK;
 }

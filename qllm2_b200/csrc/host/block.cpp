@@ -269,7 +269,7 @@ struct Block : Function<Block> {
     // ---- front
     Tensor d_raw = at::empty({N, s.rows_a}, o), d_rawm = s.rows_m ? at::empty({N, s.rows_m}, o) : Tensor();
     const int NS = (int)(3 * K + 1);
-    const int Pf = parts_of((N + 3) / 4, 6);
+    const int Pf = parts_of((N + 3) / 4, 4);
     qpam_front_bwd_args fb{};
     fb.f = front_args(s, p, sv[QKV], &sv[LOGITS], sv[ROPE], ctx->saved_data["offset"].toInt(), ctx->saved_data["floor"].toDouble());
     fb.f.q = dq.data_ptr(); fb.f.k = dk.data_ptr(); fb.f.v = dv.data_ptr(); fb.f.gamma = fptr(dgamma); fb.f.coef = fptr(dcoef);

@@ -17,10 +17,10 @@ CONFIGS = {
 
 
 @pytest.mark.parametrize("name", CONFIGS)
-@pytest.mark.parametrize("B,T,dim,heads", [(2, 130, 64, 2), (1, 5, 388, 3), (3, 257, 768, 2)])
+@pytest.mark.parametrize("B,T,dim,heads", [(2, 130, 64, 2), (1, 5, 388, 3), (3, 257, 768, 2), (2, 1531, 128, 12)])
 def test_native_block_matches_operators(name, B, T, dim, heads):
     torch.manual_seed(11)
-    cfg = M.V11Config(vocab_size=64, dim=dim, n_heads=heads, head_dim=64, n_layers=1, dropout=0.0, gradient_checkpointing=False, max_seq_len=512, **CONFIGS[name])
+    cfg = M.V11Config(vocab_size=64, dim=dim, n_heads=heads, head_dim=64, n_layers=1, dropout=0.0, gradient_checkpointing=False, max_seq_len=2048, **CONFIGS[name])
     blk = M.V11Block(cfg).to(DEV).train()
     with torch.no_grad():
         for k, p in blk.named_parameters():
