@@ -11,10 +11,11 @@ per-sequence RoPE positions.  New sequences are prefetched in one packed ragged 
 """
 from __future__ import annotations
 
+from array import array
 from collections import deque
 from contextlib import contextmanager
 from dataclasses import dataclass, field
-from typing import Deque, Dict, List, Optional, Sequence
+from typing import Deque, Dict, Iterable, List, Optional
 
 import torch
 
@@ -67,12 +68,13 @@ class SlotScheduler:
         self.finished: List[Request] = []
         self._next_id = 0
 
-    def submit(self, prompt: Sequence[int], max_new_tokens: int) -> int:
-        if len(prompt) == 0:
+    def submit(self, prompt: Iterable[int], max_new_tokens: int) -> int:
+        prompt = list(prompt)
+        if not prompt:
             raise ValueError("empty prompt")
         rid = self._next_id
         self._next_id += 1
-        self.waiting.append(Request(rid, list(prompt), max_new_tokens))
+        self.waiting.append(Request(rid, prompt, max_new_tokens))
         return rid
 
     def admit(self) -> List[Request]:
@@ -201,7 +203,7 @@ class ContinuousBatcher:
             self._g_out = None
 
     def submit(self, prompt, max_new_tokens):
-        return self.sched.submit([int(t) for t in prompt], max_new_tokens)
+        return self.sched.submit(map(int, prompt), max_new_tokens)
 
     def _ensure_rope(self, need: int):
         """Rotary tables must cover every position before a step that cannot look at its positions on the host."""
@@ -250,7 +252,7 @@ class ContinuousBatcher:
         ends = count.cumsum(0)
         starts = torch.tensor([st for _, st, _ in items])
         both = torch.empty(2, n_tok, dtype=torch.long)
-        both[0] = torch.tensor(toks, dtype=torch.long)
+        both[0] = torch.frombuffer(array("q", toks), dtype=torch.long)        # 18 k ids: 0.25 ms; torch.tensor of the list 0.84
         both[1] = torch.arange(n_tok) + (starts - ends + count).repeat_interleave(count)
         both = both.to(self.device)
         ids, positions = both[0][None], both[1][None]
