@@ -63,7 +63,7 @@ struct ScanLayout {
   int32_t ch;           // tokens per chunk of this layout
   int32_t nc_uniform;
   int32_t grid_chunks;  // upper bound on the number of chunks (grid.x of the chunk kernels)
-  size_t off_prefix, off_states, off_decay, off_dstates, off_anchors, off_dak, total_fwd, total_bwd;
+  size_t off_prefix, off_states, off_decay, off_dstates, off_anchors, off_dak, off_jobs, total_fwd, total_bwd;
 };
 
 // Tensor-core kernels take bf16 token tensors with head dim 64 and a single state; their chunk is
@@ -102,6 +102,8 @@ static ScanLayout scan_layout(const qpam_scan_args* a, int ch) {
   off += align256(sizeof(float2) * (size_t)a->K * a->H * L.nslots * dd);
   L.off_decay = off;
   off += align256(sizeof(float) * (size_t)a->K * a->H * L.nslots);
+  L.off_jobs = off;      // ticket counter, then the jobs of the carrying chunk sums (packed calls)
+  if (a->cu_seqlens != nullptr) off += align256(256 + sizeof(ChunkJob) * (size_t)L.grid_chunks);
   L.total_fwd = off;
   L.off_dstates = off;
   off += align256(sizeof(float2) * (size_t)a->K * a->H * L.nslots * dd);
@@ -209,8 +211,67 @@ static ScanParams one_state_view(const ScanParams& pK, const qpam_scan_args* a, 
   return p;
 }
 
+// Jobs of the carrying chunk sums: CTA s places the chunks of sequence s.  Chunk c of nc sits at (c + 1/2) / nc of the way, so
+// that all sequences end together and the chunks of the longest are as far apart as they can be.  The rank of a chunk is the
+// number of chunks before that point, plus the earlier sequences that have one at the same point.
+// A link of a chain takes ~2.2 us and the chip does 67 jobs a us, so the sums carry (ticket[1]) where the longest sequence has at
+// most 1/CARRY_WIDTH of all jobs; a pass of its own for the carry costs ~9 ns a job.
+// Clears the flags and the ticket counter.
+constexpr int CARRY_WIDTH = 160;
+__global__ void __launch_bounds__(256) k_chunk_jobs(ScanParams p, ChunkJob* jobs) {
+  const int s = blockIdx.x, S = p.geom.S;
+  const int32_t *cu = p.geom.cu_seqlens, *pre = p.geom.chunk_prefix;
+  if (s == 0) {
+    int longest = 1;
+    for (int o = threadIdx.x; o < S; o += 256) longest = max(longest, pre[o + 1] - pre[o]);
+    const bool narrow = __syncthreads_or((int64_t)pre[S] * p.H < (int64_t)longest * CARRY_WIDTH);
+    if (threadIdx.x == 0) {
+      p.ticket[0] = 0u;
+      p.ticket[1] = narrow ? 0u : 1u;
+    }
+  }
+  const int64_t flags = (int64_t)p.K * p.H * p.nslots;
+  for (int64_t i = (int64_t)s * 256 + threadIdx.x; i < flags; i += (int64_t)S * 256) p.ready[i] = 0u;
+  const int nc = pre[s + 1] - pre[s], a = cu[s], len = cu[s + 1] - a;
+  for (int c = threadIdx.x; c < nc; c += 256) {
+    int rank = 0;
+    for (int o = 0; o < S; ++o) {
+      const int n = pre[o + 1] - pre[o];            // chunks x of o with (2x + 1) / n < (2c + 1) / nc
+      int up;
+      bool tie;
+      if (pre[S] <= 32768) {
+        const uint32_t at = (uint32_t)(2 * c + 1) * (uint32_t)n;
+        up = (int)((at + (uint32_t)nc - 1u) / (uint32_t)nc);
+        tie = (uint32_t)up * (uint32_t)nc == at;
+      } else {
+        const int64_t at = (int64_t)(2 * c + 1) * n;
+        up = (int)((at + nc - 1) / nc);
+        tie = (int64_t)up * nc == at;
+      }
+      rank += up >> 1;
+      if (o < s && (up & 1) && tie) ++rank;
+    }
+    jobs[rank] = ChunkJob{s, c, nc, a + c * p.geom.ch, min(p.geom.ch, len - c * p.geom.ch), pre[s] + s, {0, 0}};
+  }
+}
+
 // chunk-local state sums on tensor cores, then the carry over the chunk axis
-static int tc_states(const ScanParams& p, const ScanLayout& L, const qpam_scan_args* a, cudaStream_t st) {
+static int tc_states(const ScanParams& p0, const ScanLayout& L, const qpam_scan_args* a, cudaStream_t st) {
+  ScanParams p = p0;
+  // Where the carry is likely to pay: the lengths are on the device, so by their average (eight chunks and more: short
+  // sequences have few links to save) and by how many sequences and heads run side by side (of 384, with lengths anywhere
+  // up to the longest, about 190 on average).  Drawing jobs costs 10 % of the chunk sums if the device then decides against it.
+  const bool carry = a->cu_seqlens != nullptr && a->K == 1 && p.fwd_only && p.s0 == nullptr && a->T >= (int64_t)8 * tcs::TC * a->S &&
+                     (int64_t)a->S * a->H >= 384;
+  if (carry) {
+    char* ws = reinterpret_cast<char*>(a->workspace);
+    ChunkJob* jobs = reinterpret_cast<ChunkJob*>(ws + L.off_jobs + 256);
+    p.jobs = jobs;
+    p.ticket = reinterpret_cast<unsigned int*>(ws + L.off_jobs);
+    p.ready = reinterpret_cast<unsigned int*>(p.chunk_decay);
+    k_chunk_jobs<<<a->S, 256, 0, st>>>(p, jobs);
+    QPAM_LAUNCH_CHECK("k_chunk_jobs");
+  }
   if (L.grid_chunks > 0 && a->K > 1) {      // all states from one load of the key / value tiles
     int rc = set_smem(tcs::k_tc_chunk_outerK<false>, tcs::OUTERK_SMEM);
     if (rc) return rc;
@@ -221,7 +282,7 @@ static int tc_states(const ScanParams& p, const ScanLayout& L, const qpam_scan_a
     tcs::k_tc_chunk_outerK<false><<<dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st>>>(mk, mv, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outerK");
   } else if (L.grid_chunks > 0) {
-    const auto kern = p.fwd_only ? tcs::k_tc_chunk_outer<false, true> : tcs::k_tc_chunk_outer<false>;
+    const auto kern = carry ? tcs::k_tc_chunk_outer<false, tcs::OUTER_CARRY> : p.fwd_only ? tcs::k_tc_chunk_outer<false, tcs::OUTER_FWD_ONLY> : tcs::k_tc_chunk_outer<false>;
     int rc = set_smem(kern, tcs::OUTER_SMEM);
     if (rc) return rc;
     CUtensorMap mk, mv;

@@ -89,6 +89,12 @@ __device__ __forceinline__ void warp_chunk_cumsum(float* A, const float* __restr
   A[t + 1] = excl + x0 + x1;
 }
 
+// One chunk of a packed batch as a job of the carrying chunk sums (pam_scan_tc.cuh)
+struct ChunkJob {
+  int32_t seq, c, nc, t0, len, slot0;
+  int32_t pad[2];
+};
+
 struct ScanParams {
   const void *q, *k, *v, *dy;
   const float* gamma;   // [K,B,H,T]
@@ -117,6 +123,12 @@ struct ScanParams {
   void* pool;
   const int32_t* slot_ids;
   int64_t n_slots;
+  // Packed forward-only calls from zero states: jobs[0 .. chunk_prefix[S]) in an order in which a sequence's chunks follow one
+  // another; the tickets drawn so far, [1]: whether the chunk sums carry; a flag for every state slot, set once the state is
+  // there.
+  const ChunkJob* jobs;
+  unsigned int* ticket;
+  unsigned int* ready;     // [K,H,nslots] (in the place of chunk_decay)
 };
 
 __device__ __forceinline__ size_t token_base(const ScanParams& p, int b, int h, int t, int D) {
@@ -233,6 +245,7 @@ __global__ void __launch_bounds__(256) k_state_scan(ScanParams p, int D) {
   }
   const bool from_zero = !REVERSE && p.s0 == nullptr;
   if (!REVERSE && p.fwd_only && nc == 1 && from_zero) return;
+  if (!REVERSE && p.jobs != nullptr && p.ticket[1] != 0u && nc > 1) return;      // the chunk sums have carried already
   const int e4 = blockIdx.z * 256 + threadIdx.x;  // float4 index within the D*D*2 floats
   if (e4 >= n4) return;
   float4* st = reinterpret_cast<float4*>((REVERSE ? p.dstates : p.states) + state_base(p, k, h, slot0, D)) + e4;

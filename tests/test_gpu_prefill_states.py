@@ -52,3 +52,15 @@ def test_forward_only_states(K, H, copies, with_s0):
         a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
         check(_lib.lib().qpam_scan_prefill(C.byref(a), pool.data_ptr(), dtype_code(dtype), n + 2, 2, 1, ptr(slots), stream_ptr()), "qpam_scan_prefill")
         assert torch.equal(y2, y) and torch.equal(pool, want)
+
+
+@pytest.mark.parametrize("lens", [[0, 1, 128, 129] + [1000 + 37 * i for i in range(20)],          # wide: the chunk sums carry
+                                  [20000, 0] + [255 + i for i in range(22)]])                    # one long chain: they do not
+def test_carry_in_the_chunk_sums(lens):
+    H = 16
+    q, k, v, gamma, _, cu, _ = _inputs(1, H, lens, False)
+    assert len(lens) * H >= 384 and sum(lens) >= 1024 * len(lens)      # the batches the carrying form is chosen for
+    y_ref, s_ref = ops.pam_scan(q, k, v, gamma.clone().requires_grad_(True), cu_seqlens=cu, token_major=True)
+    for _ in range(3):
+        y, s = ops.pam_scan_tokens(q, k, v, gamma, cu_seqlens=cu)
+        assert torch.equal(s, s_ref) and torch.equal(y, y_ref)
