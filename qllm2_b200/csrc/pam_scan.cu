@@ -261,6 +261,9 @@ static int tc_states(const ScanParams& p0, const ScanLayout& L, const qpam_scan_
   // Where the carry is likely to pay: the lengths are on the device, so by their average (eight chunks and more: short
   // sequences have few links to save) and by how many sequences and heads run side by side (of 384, with lengths anywhere
   // up to the longest, about 190 on average).  Drawing jobs costs 10 % of the chunk sums if the device then decides against it.
+  // every sequence one chunk, from zero: its sums are its final state, and nothing is left for the carry
+  const bool single = a->cu_seqlens == nullptr && L.nc_uniform == 1 && p.s0 == nullptr;
+  p.single = single && !p.fwd_only;
   const bool carry = a->cu_seqlens != nullptr && a->K == 1 && p.fwd_only && p.s0 == nullptr && a->T >= (int64_t)8 * tcs::TC * a->S &&
                      (int64_t)a->S * a->H >= 384;
   if (carry) {
@@ -282,7 +285,7 @@ static int tc_states(const ScanParams& p0, const ScanLayout& L, const qpam_scan_
     tcs::k_tc_chunk_outerK<false><<<dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st>>>(mk, mv, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outerK");
   } else if (L.grid_chunks > 0) {
-    const auto kern = carry ? tcs::k_tc_chunk_outer<false, tcs::OUTER_CARRY> : p.fwd_only ? tcs::k_tc_chunk_outer<false, tcs::OUTER_FWD_ONLY> : tcs::k_tc_chunk_outer<false>;
+    const auto kern = carry ? tcs::k_tc_chunk_outer<false, tcs::OUTER_CARRY> : p.fwd_only || single ? tcs::k_tc_chunk_outer<false, tcs::OUTER_FWD_ONLY> : tcs::k_tc_chunk_outer<false>;
     int rc = set_smem(kern, tcs::OUTER_SMEM);
     if (rc) return rc;
     CUtensorMap mk, mv;
@@ -292,6 +295,7 @@ static int tc_states(const ScanParams& p0, const ScanLayout& L, const qpam_scan_
     kern<<<dim3(L.grid_chunks, a->H, a->K), 256, tcs::OUTER_SMEM, st>>>(mk, mv, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outer<state>");
   }
+  if (single) return QPAM_OK;
   k_state_scan<false><<<dim3(a->S, a->H * a->K, (64 * 64 / 2 + 255) / 256), 256, 0, st>>>(p, 64);
   QPAM_LAUNCH_CHECK("k_state_scan<fwd>");
   return QPAM_OK;
@@ -400,6 +404,13 @@ static int scan_fwd_tc_states(const qpam_scan_args* a, const ScanLayout& L, void
   return QPAM_OK;
 }
 
+// No state enters a chunk and no gradient reaches one: every sequence is one chunk, without initial state, gradient of its final
+// state or request for that of its initial state.  The gradient state sums and the reverse carry have nothing to compute then
+// (93 tokens, forward and backward: seven launches to four, 96 -> 89 us, all of it host time).
+static bool chunks_alone(const qpam_scan_args* a, const ScanLayout& L, const float* ds_final, const float* ds0) {
+  return a->cu_seqlens == nullptr && L.nc_uniform == 1 && a->s0 == nullptr && ds_final == nullptr && ds0 == nullptr;
+}
+
 // bf16 / d = 64 / one state, backward: gradient state sums -> reverse carry (with the anchors of the decay
 // gradient) -> ONE launch for the dq, dv, dk jobs of every chunk -> dgamma.  Everything stays on the caller's stream.
 // state >= 0: `a` describes K states whose forward (qpam_scan_fwd_states) left its states in the workspace; the backward of
@@ -412,7 +423,8 @@ static int scan_bwd_tc(const qpam_scan_args* a, const ScanLayout& L, const void*
   p.dy = dy; p.dq = dq; p.dk = dk; p.dv = dv;
   p.dgamma = dgamma; p.dcoef = nullptr; p.ds_final = ds_final; p.ds0 = ds0;
   int rc;
-  if (!states_valid) {
+  const bool alone = chunks_alone(a, L, ds_final, ds0);
+  if (!states_valid && !alone) {
     ScanParams pf = p;
     pf.s_final = nullptr;
     if (a->cu_seqlens != nullptr) {
@@ -425,7 +437,7 @@ static int scan_bwd_tc(const qpam_scan_args* a, const ScanLayout& L, const void*
   float* anchors = reinterpret_cast<float*>(reinterpret_cast<char*>(a->workspace) + L.off_anchors) +
                    (state > 0 ? (size_t)state * a->H * L.nslots * tcs::ANCHOR_PARTS : 0);
   p.dA_k = reinterpret_cast<float*>(reinterpret_cast<char*>(a->workspace) + L.off_dak);
-  if (L.grid_chunks > 0) {
+  if (L.grid_chunks > 0 && !alone) {
     rc = set_smem(tcs::k_tc_chunk_outer<true>, tcs::OUTER_SMEM);
     if (rc) return rc;
     CUtensorMap mq, mdy;
@@ -435,8 +447,10 @@ static int scan_bwd_tc(const qpam_scan_args* a, const ScanLayout& L, const void*
     tcs::k_tc_chunk_outer<true><<<dim3(L.grid_chunks, a->H), 256, tcs::OUTER_SMEM, st>>>(mq, mdy, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outer<dstate>");
   }
-  tcs::k_tc_state_scan_rev<<<dim3(a->S, a->H, 64 * 64 / 2 / 256), 256, 0, st>>>(p, anchors);
-  QPAM_LAUNCH_CHECK("k_tc_state_scan_rev");
+  if (!alone) {
+    tcs::k_tc_state_scan_rev<<<dim3(a->S, a->H, 64 * 64 / 2 / 256), 256, 0, st>>>(p, anchors);
+    QPAM_LAUNCH_CHECK("k_tc_state_scan_rev");
+  }
   if (L.grid_chunks > 0) {
     tcs::BwdMaps maps;
     const int64_t rows = (int64_t)a->B * a->H * a->T;
@@ -455,7 +469,7 @@ static int scan_bwd_tc(const qpam_scan_args* a, const ScanLayout& L, const void*
       tcs::k_tc_chunk_bwd<false><<<dim3(3 * L.grid_chunks, a->H), 256, tcs::CHUNK2_SMEM, st>>>(maps, p);
     }
     QPAM_LAUNCH_CHECK("k_tc_chunk<dq,dv,dk>");
-    tcs::k_tc_dgamma_finalize<<<dim3(L.grid_chunks, a->H), 128, 0, st>>>(p, anchors);
+    tcs::k_tc_dgamma_finalize<<<dim3(L.grid_chunks, a->H), 128, 0, st>>>(p, alone ? nullptr : anchors);
     QPAM_LAUNCH_CHECK("k_tc_dgamma_finalize");
   }
   return QPAM_OK;
@@ -479,7 +493,8 @@ static int scan_bwd_tcK(const qpam_scan_args* a, const ScanLayout& L, const void
   p.dgamma = dgamma; p.dcoef = dcoef; p.ds_final = ds_final; p.ds0 = ds0;
   p.dy_tokens = dy_tokens ? 1 : 0;
   int rc;
-  if (!states_valid) {
+  const bool alone = chunks_alone(a, L, ds_final, ds0);
+  if (!states_valid && !alone) {
     ScanParams pf = p;
     pf.s_final = nullptr;
     if (a->cu_seqlens != nullptr) {
@@ -502,12 +517,18 @@ static int scan_bwd_tcK(const qpam_scan_args* a, const ScanLayout& L, const void
     if ((rc = make_map(&maps.dq, dq, 128, rows, 128, 64, 32))) return rc;
     if ((rc = make_map(&maps.dk, dk, 128, rows, 128, 64, 32))) return rc;
     if ((rc = make_map(&maps.dv, dv, 128, rows, 128, 64, 32))) return rc;
-    if ((rc = set_smem(tcs::k_tc_chunk_outerK<true>, tcs::OUTERK_SMEM))) return rc;
-    tcs::k_tc_chunk_outerK<true><<<dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st>>>(maps.q, maps.dy, p);
-    QPAM_LAUNCH_CHECK("k_tc_chunk_outerK<dstate>");
+    if (!alone) {
+      if ((rc = set_smem(tcs::k_tc_chunk_outerK<true>, tcs::OUTERK_SMEM))) return rc;
+      tcs::k_tc_chunk_outerK<true><<<dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st>>>(maps.q, maps.dy, p);
+      QPAM_LAUNCH_CHECK("k_tc_chunk_outerK<dstate>");
+    }
   }
-  tcs::k_tc_state_scan_rev<<<dim3(a->S, a->H, 8 * a->K), 256, 0, st>>>(p, anchors);
-  QPAM_LAUNCH_CHECK("k_tc_state_scan_rev");
+  if (alone) {
+    anchors = nullptr;
+  } else {
+    tcs::k_tc_state_scan_rev<<<dim3(a->S, a->H, 8 * a->K), 256, 0, st>>>(p, anchors);
+    QPAM_LAUNCH_CHECK("k_tc_state_scan_rev");
+  }
   if (L.grid_chunks == 0) return QPAM_OK;
   switch (a->K) {
     case 2: return launch_bwdK<2>(maps, p, L, anchors, st);
@@ -524,13 +545,14 @@ static int scan_bwd_t(const qpam_scan_args* a, const ScanLayout& L, const void* 
   p.dy = dy; p.dq = dq; p.dk = dk; p.dv = dv;
   p.dgamma = dgamma; p.dcoef = dcoef; p.ds_final = ds_final; p.ds0 = ds0;
   int rc;
-  if (!states_valid) {
+  const bool alone = chunks_alone(a, L, ds_final, ds0);
+  if (!states_valid && !alone) {
     ScanParams pf = p;
     pf.s_final = nullptr;
     rc = launch_states<D, T>(pf, L, a, st);
     if (rc) return rc;
   }
-  if (L.grid_chunks > 0) {
+  if (L.grid_chunks > 0 && !alone) {
     auto kern = k_chunk_outer<D, T, true>;
     rc = set_smem(kern, outer_smem<D>());
     if (rc) return rc;
@@ -538,8 +560,10 @@ static int scan_bwd_t(const qpam_scan_args* a, const ScanLayout& L, const void* 
     QPAM_LAUNCH_CHECK("k_chunk_outer<dstate>");
   }
   const int n4 = D * D / 2;
-  k_state_scan<true><<<dim3(a->S, a->H * a->K, (n4 + 255) / 256), 256, 0, st>>>(p, D);
-  QPAM_LAUNCH_CHECK("k_state_scan<rev>");
+  if (!alone) {
+    k_state_scan<true><<<dim3(a->S, a->H * a->K, (n4 + 255) / 256), 256, 0, st>>>(p, D);
+    QPAM_LAUNCH_CHECK("k_state_scan<rev>");
+  }
   if (L.grid_chunks > 0) {
     auto kern = k_bwd_chunk<D, T>;
     rc = set_smem(kern, bwd_chunk_smem<D>());

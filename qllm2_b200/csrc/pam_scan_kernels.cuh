@@ -119,6 +119,7 @@ struct ScanParams {
   // Tensor-core forward of which no backward will read the states: what only a backward needs is not written (see
   // k_state_scan), and the final states may go to slots of a state pool [n_slots,L,K,H,D,D,2] instead of s_final.
   int32_t fwd_only;
+  int32_t single;          // a backward may follow, but every sequence is one chunk from zero: the chunk sums write s_final as well
   int32_t pool_bf16, pool_L, pool_layer;
   void* pool;
   const int32_t* slot_ids;

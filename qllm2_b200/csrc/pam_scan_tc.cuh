@@ -306,14 +306,19 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + cc * 32, d1);
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + 64 + cc * 32, d2);
     const bool even = (lane & 1) == 0;
-    const bool final_now = MODE == OUTER_FWD_ONLY && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
+    const bool final_now = MODE == OUTER_FWD_ONLY && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform (fwd_only or single)
     if (final_now) {
       FinalDest fin;
       fin.init(p, L.seq, kst, h);
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
         const float o0 = __shfl_xor_sync(0xffffffffu, d2[i], 1), o1 = __shfl_xor_sync(0xffffffffu, d2[i + 1], 1);
-        fin.store2(p, (cc * 32 + i) * 128 + q4 * 32 + lane, even ? d1[i] + o0 : o0 - d1[i], even ? d1[i + 1] + o1 : o1 - d1[i + 1], even, ok);
+        const float u0 = even ? d1[i] + o0 : o0 - d1[i], u1 = even ? d1[i + 1] + o1 : o1 - d1[i + 1];
+        fin.store2(p, (cc * 32 + i) * 128 + q4 * 32 + lane, u0, u1, even, ok);
+        if (p.single && ok) {
+          dst[(size_t)(cc * 32 + i) * 128] = u0;
+          dst[(size_t)(cc * 32 + i + 1) * 128] = u1;
+        }
       }
     } else {
 #pragma unroll
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
     // Re U = D1[2j] + D2[2j+1], Im U = D2[2j] - D1[2j+1]: lane n' = 2j+c holds column i, state[i][j][c] at i*128 + n'
     float2* slot = DSTATE ? p.dstates + state_base(p, k, h, L.slot0 + L.c, TD) : p.states + state_base(p, k, h, L.slot0 + L.c + 1, TD);
     float* dst = reinterpret_cast<float*>(slot) + (q4 * 32 + lane);
-    const bool final_now = !DSTATE && p.fwd_only && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
+    const bool final_now = !DSTATE && (p.fwd_only || p.single) && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
 #pragma unroll 1
     for (int hh = 0; hh < 2; ++hh) {          // 16 columns at a time: the value tile stays in registers beside them
       float d1[16], d2[16];
@@ -460,7 +465,12 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
           const float o0 = __shfl_xor_sync(0xffffffffu, d2[i], 1), o1 = __shfl_xor_sync(0xffffffffu, d2[i + 1], 1);
-          fin.store2(p, (int)(col + i) * 128 + q4 * 32 + lane, even ? d1[i] + o0 : o0 - d1[i], even ? d1[i + 1] + o1 : o1 - d1[i + 1], even, ok);
+          const float u0 = even ? d1[i] + o0 : o0 - d1[i], u1 = even ? d1[i + 1] + o1 : o1 - d1[i + 1];
+          fin.store2(p, (int)(col + i) * 128 + q4 * 32 + lane, u0, u1, even, ok);
+          if (p.single && ok) {
+            dst[(size_t)(col + i) * 128] = u0;
+            dst[(size_t)(col + i + 1) * 128] = u1;
+          }
         }
       } else {
 #pragma unroll

@@ -611,7 +611,8 @@ __global__ void __launch_bounds__(256) k_tc_state_scan_rev(ScanParams p, float* 
     for (int i = 0; i < UN; ++i)
       if (c - i >= 0) {
         u[i] = st[(size_t)(c - i) * n4];
-        f[i] = __ldg(fs + (size_t)(c - i) * n4);
+        // (the state before the first chunk is zero and not always stored without s0)
+        f[i] = c - i > 0 || p.s0 != nullptr ? __ldg(fs + (size_t)(c - i) * n4) : make_float4(0.f, 0.f, 0.f, 0.f);
         g[i] = dec[c - i + 1];
       }
 #pragma unroll
@@ -645,7 +646,9 @@ __global__ void __launch_bounds__(128) k_tc_dgamma_finalize(ScanParams p, const 
   const size_t base = gamma_base(p, 0, L.b, h, L.t0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int len = L.len;
-  if (warp < 2) {      // warp 0: anchor at the chunk's first token, warp 1: just after the chunk
+  if (anchor_parts == nullptr) {      // one chunk from zero and no gradient of its final state: both anchors are zero
+    if (tid < 2) anc[tid] = 0.f;
+  } else if (warp < 2) {      // warp 0: anchor at the chunk's first token, warp 1: just after the chunk
     const float* ap = anchor_parts + ((size_t)h * p.nslots + L.slot0 + L.c + warp) * ANCHOR_PARTS;
     double a = (double)ap[lane] + (double)ap[lane + 32];
 #pragma unroll

@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   float g_e = 1.f, an0 = 0.f, an1 = 0.f;
   if (ek < K) {
     if (et_rev < len) g_e = __ldg(p.gamma + eg - et + et_rev);
-    if ((warp & 3) < 2) {
+    if ((warp & 3) < 2 && anchor_parts != nullptr) {      // (null: zero, see scan_bwd_tc)
       const float* ap = anchor_parts + (((size_t)ek * p.H + h) * p.nslots + L.slot0 + L.c + (warp & 3)) * ANCHOR_PARTS;
       an0 = __ldg(ap + lane);
       an1 = __ldg(ap + lane + 32);

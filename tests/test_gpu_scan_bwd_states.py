@@ -39,3 +39,22 @@ def test_bwd_of_all_states(K, B, T, lengths, strong, tokens):
         assert torch.isfinite(a).all(), name
         err = float((a.float() - b).norm() / b.norm())
         assert err < 1e-2, (name, err)
+
+
+@pytest.mark.parametrize("dtype,K,T", [(torch.bfloat16, 1, 1), (torch.bfloat16, 1, 93), (torch.bfloat16, 1, 128), (torch.bfloat16, 3, 128),
+                                       (torch.bfloat16, 2, 17), (torch.float32, 1, 64), (torch.float32, 2, 5)])
+@pytest.mark.parametrize("state_grad", [False, True])
+def test_one_chunk_alone_equals_packed(dtype, K, T, state_grad):
+    """A batch of one-chunk sequences runs without carries; the same sequence described by cu_seqlens takes every launch."""
+    g = torch.Generator(device=DEV).manual_seed(T + K)
+    H, d = 3, 64
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    data = [(rnd(1, H, T, d, 2) * 0.09).to(dtype) for _ in range(3)] + [torch.sigmoid(rnd(K, 1, H, T) + 2)] + ([rnd(K, 1, H, T, 2)] if K > 1 else [])
+    dy, ds = rnd(1, H, T, d, 2).to(dtype), rnd(K, 1, H, d, d, 2)
+    res = []
+    for cu in (None, torch.tensor([0, T], device=DEV, dtype=torch.int32)):
+        leaves = [t.clone().requires_grad_() for t in data]
+        y, s = ops.pam_scan(*leaves[:4], coef=leaves[4] if K > 1 else None, cu_seqlens=cu)
+        res.append([y, s, *torch.autograd.grad([y, s] if state_grad else [y], leaves, [dy, ds] if state_grad else [dy])])
+    for a, b in zip(*res):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
