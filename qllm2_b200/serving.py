@@ -13,7 +13,7 @@ from __future__ import annotations
 
 from array import array
 from collections import deque
-from contextlib import contextmanager
+from contextlib import contextmanager, suppress
 from dataclasses import dataclass, field
 from typing import Deque, Dict, Iterable, List, Optional
 
@@ -135,10 +135,20 @@ def _captured():
     garbage and hand every cached block back to the driver, which an engine beside other work then pays for twice.)"""
     side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
     side.wait_stream(torch.cuda.current_stream())
-    with torch.cuda.stream(side):
-        yield graph
-        graph.capture_end()
-    torch.cuda.current_stream().wait_stream(side)
+    try:
+        with torch.cuda.stream(side):
+            try:
+                yield graph
+            except BaseException:
+                # the stream must not stay in capture (whatever comes next on it would be recorded or refused); the graph is
+                # dropped, and the body's own error is the one to report
+                if torch.cuda.is_current_stream_capturing():
+                    with suppress(RuntimeError):
+                        graph.capture_end()
+                raise
+            graph.capture_end()
+    finally:
+        torch.cuda.current_stream().wait_stream(side)
 
 
 class _DecodeMix:
