@@ -24,6 +24,7 @@ from typing import Dict, List, Optional
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _lib
 from . import fused_elementwise as FE
@@ -494,16 +495,27 @@ class V11PAMLayer(nn.Module):
 
 
 # ------------------------------------------------------------------------------------ block / LM
-def _plain_fp32(module, inner: bool = True) -> bool:
-    """Whether every parameter below `module` is fp32 and no module inside it has hooks.  (Asked at every call of every block:
-    a walk over the plain dictionaries takes 8 us where modules() and parameters() take 40.)"""
-    if inner and (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks):
-        return False
-    for p in module._parameters.values():
-        if p is not None and p.dtype is not torch.float32:
+def _stock(module) -> bool:
+    """Whether a module of one of these classes, and every operator below it, is as this file builds it: exactly the class,
+    forward not replaced on the instance, no hooks (the module itself is being called: its own have run), fp32 parameters.
+    (Asked at every call of every block: a walk over the plain dictionaries, where modules() and parameters() take 40 us.)"""
+    cls = type(module)
+    for name, p in module._parameters.items():
+        if p is None:
+            if cls is nn.Linear:                            # the kernels read its bias
+                return False
+        elif p.dtype is not torch.float32 or (cls is ComplexLinear and name[0] == "b"):   # these projections have none
             return False
-    for m in module._modules.values():
-        if m is not None and not _plain_fp32(m):
+    if cls is ComplexNorm and module.eps != 1e-6:
+        return False
+    parts = module._modules
+    for name, classes in _STOCK.get(cls, ()):
+        m = parts.get(name)
+        if m is None:
+            continue
+        if type(m) not in classes or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__:
+            return False
+        if not _stock(m):
             return False
     return True
 
@@ -523,16 +535,16 @@ class V11Block(nn.Module):
 
     def _native_ok(self, x, pam_state) -> bool:
         """Whether the whole block can run as one native node (csrc/host/block.cpp): bf16 autocast over fp32 parameters from
-        a zero state, in the shape its kernels cover, with nothing attached to the operators in between."""
-        pam = self.pam
+        a zero state, in the shape its kernels cover, with nothing replaced among, or attached to, the operators in between."""
         if (pam_state is not None or not x.is_cuda or x.dtype != torch.bfloat16 or x.shape[1] < 2 or not torch.is_autocast_enabled("cuda")
                 or torch.get_autocast_dtype("cuda") != torch.bfloat16):
             return False
+        if type(self) is not V11Block or _has_any_global_hook() or not _stock(self):
+            return False
+        pam = self.pam
         if pam.head_dim != 64 or pam.num_heads > 64 or not pam.fused_qkv or pam.qk_norm or pam.dim % 4 or pam.dim > 768 or not pam._fused_gates_ok(x):
             return False
-        if self.training and (self.cgu_dropout.p > 0 or pam.dropout.p > 0):
-            return False
-        return _plain_fp32(self, inner=False)
+        return not (self.training and (self.cgu_dropout.p > 0 or pam.dropout.p > 0))
 
     def _native(self, x, step_offset: int):
         cgu, pam = self.cgu, self.pam
@@ -568,6 +580,17 @@ class V11Block(nn.Module):
         if x.numel() % 4 == 0 and x.dtype in (torch.float32, torch.bfloat16) and delta.dtype in (torch.float32, torch.bfloat16):
             return FE.scaled_residual(x, delta, scale)
         return x + delta * scale        # other dtypes (fp16, fp64): the residual add stays a torch operator
+
+
+#: the operators that a native block stands for: the attribute each is kept under, and the class it has to be exactly (a
+#: subclass or an adapter in its place may compute something else from the same parameters)
+_STOCK = {
+    ComplexGatedUnit: (("gate_proj", (ComplexLinear,)), ("up_proj", (ComplexLinear,)), ("down_proj", (ComplexLinear,)), ("act", (ModSwish, ModReLU))),
+    V11PAMLayer: (("qkv_proj", (ComplexLinear,)), ("o_proj", (ComplexLinear,)), ("dt_proj", (nn.Linear,)), ("protect_gate", (nn.Linear,)),
+                    ("phase_proj", (nn.Linear,)), ("score_proj", (nn.Linear,)), ("dropout", (nn.Dropout,))),
+    V11Block: (("norm1", (ComplexNorm,)), ("cgu", (ComplexGatedUnit,)), ("cgu_dropout", (nn.Dropout,)), ("norm2", (ComplexNorm,)),
+                 ("pam", (V11PAMLayer,))),
+}
 
 
 class ComplexPosEmbed(nn.Module):
