@@ -144,7 +144,7 @@ struct Block : Function<Block> {
     variable_list p(N_PARAMS);
     for (int i = 0, at = 0; i < N_PARAMS; ++i)
       if (present >> i & 1) p[i] = params[at++];
-    const Tensor x = x_.contiguous(), rope = value(rope_);
+    const Tensor x = x_, rope = value(rope_);
     const Shape s(x, p, H, d, K, pg_content, routing_content);
     void* st = stream();
     bool bwd = x_.requires_grad();
@@ -229,7 +229,7 @@ struct Block : Function<Block> {
     const auto f32o = o.dtype(at::kFloat);
     const int64_t N = s.N, D = s.D;
     const float eps = 1e-6f;
-    const Tensor dx2 = grads[0].defined() ? grads[0].to(at::kBFloat16).contiguous() : at::zeros_like(x);
+    const Tensor dx2 = grads[0].defined() ? dense(grads[0].to(at::kBFloat16)) : at::zeros_like(x);
     variable_list g(N_PARAMS);
     for (int i = 0; i < N_PARAMS; ++i)
       if (p[i].defined()) g[i] = at::empty_like(p[i]);
@@ -331,20 +331,69 @@ struct Block : Function<Block> {
   }
 };
 
-std::tuple<Tensor, Tensor> block(const Tensor& x, const std::vector<OptTensor>& params, const OptTensor& rope, int64_t H, int64_t d, int64_t K, bool pg_content,
+// Rows and columns of parameter i (1-D parameters: their length by one).
+std::pair<int64_t, int64_t> param_shape(int i, const Shape& s) {
+  switch (i) {
+    case N1: case N2: return {s.D, 1};
+    case GATE_R: case GATE_I: case UP_R: case UP_I: return {s.hidden, s.D};
+    case DOWN_R: case DOWN_I: return {s.D, s.hidden};
+    case ACT_BIAS: case ACT_BETA: return {s.hidden, 1};
+    case CGU_SCALE: case PAM_SCALE: return {1, 1};
+    case QKV_R: case QKV_I: return {3 * s.inner, s.D};
+    case O_R: case O_I: return {s.D, s.inner};
+    case DT_W: return {s.H, 2 * s.D};
+    case DT_B: case DT_BIAS: case PG_B: return {s.H, 1};
+    case DT_OFF: return {s.K, 1};
+    case PG_W: return {s.H, s.mag[1] ? s.D : 2 * s.D};
+    case PHASE_W: case SCORE_W: return {s.H * s.K, s.mag[2] ? s.D : 2 * s.D};
+    default: return {s.H * s.K, 1};           // PHASE_B, SCORE_B
+  }
+}
+constexpr int64_t bits(std::initializer_list<int> l) {
+  int64_t b = 0;
+  for (int i : l) b |= (int64_t)1 << i;
+  return b;
+}
+
+// The operators this node stands for check their operands one by one; the kernels behind it take pointers and the sizes of x,
+// H, d and K, so all of it is checked here, before the first launch.
+std::tuple<Tensor, Tensor> block(const Tensor& x, const std::vector<OptTensor>& params, const OptTensor& rope_, int64_t H, int64_t d, int64_t K, bool pg_content,
                                  bool routing_content, double gamma_floor, int64_t offset) {
   QH_REQUIRE((int64_t)params.size() == N_PARAMS, "block: ", (int)N_PARAMS, " parameters expected");
-  variable_list p;
+  QH_REQUIRE(x.scalar_type() == at::kBFloat16 && x.dim() == 4 && x.size(3) == 2 && x.size(0) > 0 && x.size(1) > 0,
+             "block: bfloat16 x [B,T,D,2] expected; got ", shape(x));
+  QH_REQUIRE(d == 64 && H >= 1 && H <= 64 && K >= 1 && K <= QPAM_MAX_STATES, "block: d=", d, ", H=", H, ", K=", K, " are not covered");
+  QH_REQUIRE(x.size(2) % 4 == 0 && x.size(2) <= 768, "block: the channel count must be a multiple of 4 up to 768; got ", x.size(2));
+  variable_list p(N_PARAMS), present_params;
   int64_t present = 0;
   for (int i = 0; i < N_PARAMS; ++i) {
-    const auto& t = params[i];
-    if (!t.has_value()) continue;
-    QH_REQUIRE(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous(), "block: parameters must be contiguous float32 CUDA tensors");
-    p.push_back(*t);
+    if (!params[i].has_value()) continue;
+    QH_REQUIRE(params[i]->device() == x.device() && params[i]->scalar_type() == at::kFloat, "block: parameters must be float32 on x's device");
+    p[i] = dense(*params[i]);
+    present_params.push_back(p[i]);
     present |= (int64_t)1 << i;
   }
-  QH_REQUIRE(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 4 && x.size(3) == 2, "block: bfloat16 x [B,T,D,2] expected; got ", shape(x));
-  auto out = Block::apply(x, at::TensorList(p), rope, present, H, d, K, pg_content, routing_content, gamma_floor, offset);
+  const int64_t gsp = bits({PG_W, PG_B}), routing = bits({DT_OFF, PHASE_W, PHASE_B}), score = bits({SCORE_W, SCORE_B}), optional = gsp | routing | score | bits({ACT_BETA});
+  const int64_t all = ((int64_t)1 << N_PARAMS) - 1;
+  const auto whole = [&](int64_t group) { return (present & group) == 0 || (present & group) == group; };
+  QH_REQUIRE((present | optional) == all && whole(gsp) && whole(score) && (present & routing) == (K > 1 ? routing : 0) && (K > 1 || !(present & score)),
+             "block: parameters are missing or do not go together");
+  const Shape s(x, p, H, d, K, pg_content, routing_content);
+  QH_REQUIRE(s.hidden > 0 && s.hidden % 4 == 0, "block: the hidden width must be a multiple of 4; got ", s.hidden);
+  for (int i = 0; i < N_PARAMS; ++i) {
+    if (!p[i].defined()) continue;
+    const auto [rows, cols] = param_shape(i, s);
+    QH_REQUIRE(p[i].numel() == rows * cols && (cols == 1 || (p[i].dim() == 2 && p[i].size(0) == rows)), "block: parameter ", i, " is ", shape(p[i]), ", [", rows, ", ",
+               cols, "] expected for x ", shape(x));
+  }
+  OptTensor rope;
+  if (rope_.has_value()) {
+    QH_REQUIRE(rope_->device() == x.device() && rope_->dim() == 3 && rope_->size(1) == d && rope_->size(2) == 2 && offset + x.size(1) <= rope_->size(0),
+               "block: the rotary table must be [P, ", d, ", 2] with P >= offset + T = ", offset + x.size(1), "; got ", shape(*rope_));
+    rope = dense(rope_->detach().to(at::kFloat));
+  }
+  QH_REQUIRE(x.is_cuda(), "PAM kernels need CUDA tensors (there is no CPU path in this package)");
+  auto out = Block::apply(dense(x), at::TensorList(present_params), rope, present, H, d, K, pg_content, routing_content, gamma_floor, offset);
   return {out[0], out[1]};
 }
 

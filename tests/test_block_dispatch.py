@@ -3,6 +3,7 @@ import pytest
 import torch
 import torch.nn as nn
 
+from qllm2_b200 import _lib
 from qllm2_b200 import model as M
 
 
@@ -59,6 +60,69 @@ def test_changed_blocks_keep_their_operators(change):
     blk = _block()
     CHANGES[change](blk)
     assert not M._stock(blk)
+
+
+def _x(D=64, T=40):
+    return torch.zeros(1, T, D, 2, dtype=torch.bfloat16)
+
+
+MISFITS = {     # what is changed about the block, and the input it then gets
+    "other channel count": (lambda b: None, _x(D=68)),
+    "wider down projection": (lambda b: setattr(b.cgu, "down_proj", M.ComplexLinear(256, 64, bias=False)), _x()),
+    "fewer heads in the input projection": (lambda b: setattr(b.pam, "qkv_proj", M.ComplexLinear(64, 64, bias=False)), _x()),
+    "short activation bias": (lambda b: setattr(b.cgu.act, "bias", nn.Parameter(torch.zeros(100))), _x()),
+    "narrow routing": (lambda b: setattr(b.pam, "phase_proj", nn.Linear(32, 3)), _x()),
+    "scalar of two": (lambda b: setattr(b, "pam_scale", nn.Parameter(torch.ones(2))), _x()),
+    "short rotary table": (lambda b: setattr(b.pam, "rope_table", lambda x, o: b.pam.rope_cache[:39]), _x()),
+    "other rotary width": (lambda b: setattr(b.pam, "rope_cache", torch.zeros(64, 32, 2)), _x()),
+    "no input": (lambda b: None, _x(T=0)),
+}
+
+
+@pytest.mark.parametrize("case", MISFITS)
+def test_native_node_checks_every_shape(case):
+    """The node's kernels get pointers and sizes: operands that do not fit are refused before anything is launched."""
+    change, x = MISFITS[case]
+    blk = _block()
+    change(blk)
+    with pytest.raises(_lib.QPamError, match="block: "):
+        blk._native(x, 0)
+
+
+def test_native_node_has_no_cpu_path():
+    with pytest.raises(_lib.QPamError, match="need CUDA tensors"):
+        _block()._native(_x(), 0)
+
+
+@pytest.mark.gpu
+def test_parameters_of_any_layout():
+    """Parameters as views into one flat buffer, each starting off a 16-byte boundary, and transposed ones: the same results."""
+    ref, blk = _block().cuda(), _block().cuda()
+    buf = torch.zeros(sum(p.numel() + 9 for p in blk.parameters()), device="cuda")
+    at = 1
+    for i, p in enumerate(blk.parameters()):
+        if p.dim() == 2 and i % 2:
+            p.data = p.data.t().contiguous().t()
+        else:
+            flat = buf[at:at + p.numel()].view(p.shape)
+            flat.copy_(p.data)
+            p.data = flat
+            at = (at + p.numel() + 4) // 4 * 4 + 1
+    assert any(not p.is_contiguous() for p in blk.parameters()) and any(p.data_ptr() % 16 for p in blk.parameters())
+    g = torch.Generator(device="cuda").manual_seed(1)
+    xs = torch.randn(1 + 2 * 50 * 64 * 2, device="cuda", generator=g).bfloat16()
+    x = [t.requires_grad_() for t in (xs[1:].view(2, 50, 64, 2).clone(), xs[1:].view(2, 50, 64, 2).detach())]
+    dys = torch.randn(1 + 2 * 50 * 64 * 2, device="cuda", generator=g).bfloat16()[1:].view(2, 50, 64, 2)
+    assert x[0].data_ptr() % 16 == 0 and x[1].data_ptr() % 16 and dys.data_ptr() % 16
+    res = []
+    for b, xi, dy in ((ref, x[0], dys.clone()), (blk, x[1], dys)):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            assert b._native_ok(xi, None)
+            y, s = b._native(xi, 0)
+        y.backward(dy)
+        res.append([y, s, xi.grad] + [p.grad for p in b.parameters()])
+    for a, c in zip(*res):
+        assert torch.equal(a, c)
 
 
 @pytest.mark.gpu
