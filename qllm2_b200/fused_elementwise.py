@@ -82,7 +82,8 @@ class _ComplexNormFn(torch.autograd.Function):
         P = max(4, min((N + 3) // 4 * 4, 148 * 16))
         part = torch.empty(P, D, dtype=torch.float32, device=z.device)
         dz = torch.empty_like(z)
-        check(_lib.lib().qpam_cnorm_bwd(ptr(z), dtype_code(z.dtype), ptr(_param(scale, D, "scale")), ptr(dout),
+        sc = _param(scale, D, "scale")
+        check(_lib.lib().qpam_cnorm_bwd(ptr(z), dtype_code(z.dtype), ptr(sc), ptr(dout),
                                         dtype_code(ctx.out_dtype), ptr(dz), ptr(part), P, N, D, float(ctx.eps),
                                         stream_ptr()), "qpam_cnorm_bwd")
         return dz, part.sum(0).to(scale.dtype).view_as(scale), None, None
@@ -128,9 +129,11 @@ class _ModActFn(torch.autograd.Function):
         pb = torch.empty(P, C, dtype=torch.float32, device=z.device)
         pe = None if beta is None else torch.empty(P, C, dtype=torch.float32, device=z.device)
         dz = torch.empty_like(z)
-        check(_lib.lib().qpam_modact_bwd(ptr(z), dtype_code(z.dtype), ptr(_param(bias, C, "bias")),
-                                         None if beta is None else ptr(_param(beta, C, "beta")), ptr(dout), ptr(dz),
-                                         ptr(pb), ptr(pe), P, N, C, stream_ptr()), "qpam_modact_bwd")
+        # (names, not temporaries: a copy freed while the call is being put together gives its memory to the next one)
+        b = _param(bias, C, "bias")
+        be = None if beta is None else _param(beta, C, "beta")
+        check(_lib.lib().qpam_modact_bwd(ptr(z), dtype_code(z.dtype), ptr(b), ptr(be), ptr(dout), ptr(dz), ptr(pb), ptr(pe), P, N, C,
+                                         stream_ptr()), "qpam_modact_bwd")
         dbias = pb.sum(0).to(bias.dtype).view_as(bias)
         dbeta = None if beta is None else pe.sum(0).to(beta.dtype).view_as(beta)
         return dz, dbias, dbeta
