@@ -28,6 +28,13 @@ def _require_cuda(*ts):
             raise _lib.QPamError("the fused complex operators run on CUDA tensors only")
 
 
+def _dense(t: torch.Tensor) -> torch.Tensor:
+    """t contiguous and starting on a 16-byte boundary, as the kernels' vector accesses need it: a view into a flat buffer may
+    start anywhere."""
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
+
+
 def _rows(t: torch.Tensor):
     """(tensor, N, C, row stride in scalars) of a [..., C, 2] tensor; copies only if rows are not uniform."""
     if t.dim() < 2 or t.shape[-1] != 2:
@@ -46,7 +53,7 @@ def _rows(t: torch.Tensor):
     elif ok:
         ld = 2 * C
     if not ok:
-        t = t.contiguous()
+        t = _dense(t)
         ld = 2 * C
     N = t.numel() // (2 * C)
     return t, N, C, ld
@@ -55,14 +62,14 @@ def _rows(t: torch.Tensor):
 def _param(p: torch.Tensor, C: int, name: str) -> torch.Tensor:
     if p.numel() != C:
         raise _lib.QPamError(f"{name} must have {C} entries, got {p.numel()}")
-    return p.detach().float().contiguous()
+    return _dense(p.detach().float())
 
 
 # ------------------------------------------------------------------------------------ norm
 class _ComplexNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, z, scale, eps, out_dtype):
-        z = z.contiguous()
+        z = _dense(z)
         D = z.shape[-2]
         N = z.numel() // (2 * D)
         sc = _param(scale, D, "scale")
@@ -78,7 +85,7 @@ class _ComplexNormFn(torch.autograd.Function):
         z, scale = ctx.saved_tensors
         D = z.shape[-2]
         N = z.numel() // (2 * D)
-        dout = dout.to(ctx.out_dtype).contiguous()
+        dout = _dense(dout.to(ctx.out_dtype))
         P = max(4, min((N + 3) // 4 * 4, 148 * 16))
         part = torch.empty(P, D, dtype=torch.float32, device=z.device)
         dz = torch.empty_like(z)
@@ -108,7 +115,7 @@ def fused_complex_norm(z: torch.Tensor, scale: torch.Tensor, eps: float = 1e-6) 
 class _ModActFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, z, bias, beta):
-        z = z.contiguous()
+        z = _dense(z)
         C = z.shape[-2]
         N = z.numel() // (2 * C)
         out = torch.empty_like(z)
@@ -124,7 +131,7 @@ class _ModActFn(torch.autograd.Function):
         z, bias, beta = ctx.saved_tensors
         C = z.shape[-2]
         N = z.numel() // (2 * C)
-        dout = dout.to(z.dtype).contiguous()
+        dout = _dense(dout.to(z.dtype))
         P = max(1, min(N, 1024))        # rows of partial parameter gradients = row partitions of the launch
         pb = torch.empty(P, C, dtype=torch.float32, device=z.device)
         pe = None if beta is None else torch.empty(P, C, dtype=torch.float32, device=z.device)
@@ -178,7 +185,7 @@ class _CguGateFn(torch.autograd.Function):
         gate, up = ctx.saved_tensors
         gate, N, C, ldg = _rows(gate)
         up, _, _, ldu = _rows(up)
-        dout = dout.to(gate.dtype).contiguous()
+        dout = _dense(dout.to(gate.dtype))
         # two dense tensors: the consumers (the activation's backward, the projections' GEMMs) take them as they
         # are; halves of one buffer would be copied by the first consumer that needs dense rows
         dgate = torch.empty(*gate.shape[:-2], C, 2, dtype=gate.dtype, device=gate.device)
@@ -194,7 +201,7 @@ class _CguGatePackedFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, gu):
-        gu = gu.contiguous()
+        gu = _dense(gu)
         C = gu.shape[-2] // 2
         N = gu.numel() // (4 * C)
         out = torch.empty(*gu.shape[:-2], C, 2, dtype=gu.dtype, device=gu.device)
@@ -209,7 +216,7 @@ class _CguGatePackedFn(torch.autograd.Function):
         (gu,) = ctx.saved_tensors
         C = gu.shape[-2] // 2
         N = gu.numel() // (4 * C)
-        dout = dout.to(gu.dtype).contiguous()
+        dout = _dense(dout.to(gu.dtype))
         dgu = torch.empty_like(gu)
         base, dbase, off = gu.data_ptr(), dgu.data_ptr(), 2 * C * gu.element_size()
         check(_lib.lib().qpam_cgu_gate_bwd(base, 4 * C, base + off, 4 * C, ptr(dout), dtype_code(gu.dtype), dbase, 4 * C,
@@ -238,10 +245,10 @@ def fused_cgu_gate_packed(gate_up: torch.Tensor) -> torch.Tensor:
 class _PamPrepFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, rope, omp, positions, offset, H, d):
-        qkv = qkv.contiguous()
+        qkv = _dense(qkv)
         B, T = qkv.shape[0], qkv.shape[1]
         q, k, v = (torch.empty(B, H, T, d, 2, dtype=qkv.dtype, device=qkv.device) for _ in range(3))
-        ompf = None if omp is None else omp.detach().float().contiguous()
+        ompf = None if omp is None else _dense(omp.detach().float())
         check(_lib.lib().qpam_pam_prep_fwd(ptr(qkv), dtype_code(qkv.dtype), ptr(rope), 0 if rope is None else rope.shape[0],
                                            ptr(positions), int(offset), ptr(ompf), ptr(q), ptr(k), ptr(v), B, T, H, d,
                                            stream_ptr()), "qpam_pam_prep_fwd")
@@ -254,7 +261,7 @@ class _PamPrepFn(torch.autograd.Function):
         qkv, rope, ompf, positions = ctx.saved_tensors
         offset, H, d, omp_dtype = ctx.meta
         B, T = qkv.shape[0], qkv.shape[1]
-        dq, dk, dv = (g.to(qkv.dtype).contiguous() for g in (dq, dk, dv))
+        dq, dk, dv = (_dense(g.to(qkv.dtype)) for g in (dq, dk, dv))
         dqkv = torch.empty_like(qkv)
         domp = None if ompf is None else torch.empty(B, T, H, dtype=torch.float32, device=qkv.device)
         check(_lib.lib().qpam_pam_prep_bwd(ptr(qkv), dtype_code(qkv.dtype), ptr(rope), 0 if rope is None else rope.shape[0],
@@ -282,7 +289,7 @@ def pam_prep(qkv: torch.Tensor, rope: Optional[torch.Tensor], omp: Optional[torc
     if rope is not None:
         if rope.dim() != 3 or rope.shape[1:] != (d, 2):
             raise _lib.QPamError(f"pam_prep: rope must be [P, {d}, 2], got {tuple(rope.shape)}")
-        rope = rope.detach().float().contiguous()
+        rope = _dense(rope.detach().float())
         if positions is None and offset + T > rope.shape[0]:
             raise _lib.QPamError("pam_prep: the rotary table is shorter than offset + T")
     if omp is not None and tuple(omp.shape) != (B, T, H):
@@ -299,10 +306,10 @@ class _StateCombineFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, coef, token_major, *yks):
         K = len(yks)
-        yks = tuple(t.contiguous() for t in yks)
+        yks = tuple(_dense(t) for t in yks)
         d = yks[0].shape[-2]
         R = yks[0].numel() // (2 * d)
-        cf = coef.detach().float().contiguous()
+        cf = _dense(coef.detach().float())
         arr = (_lib.c_void_p * K)(*[t.data_ptr() for t in yks])
         if token_major:
             B, H, T = yks[0].shape[:3]
@@ -324,7 +331,7 @@ class _StateCombineFn(torch.autograd.Function):
         K = len(yks)
         d = yks[0].shape[-2]
         R = yks[0].numel() // (2 * d)
-        dy = dy.to(yks[0].dtype).contiguous()
+        dy = _dense(dy.to(yks[0].dtype))
         dyks = [torch.empty_like(t) for t in yks]
         dcoef = torch.empty_like(cf)
         arr = (_lib.c_void_p * K)(*[t.data_ptr() for t in yks])
@@ -343,7 +350,7 @@ class _StateCombineFn(torch.autograd.Function):
 def state_combine_tokens(coef: torch.Tensor, yks) -> torch.Tensor:
     """Inference form of `state_combine` for yks[k] [B, H, T, d, 2]: the result is written token-major,
     [B, T, H*d, 2], which is the layout the output projection reads (no transpose copy)."""
-    yks = [t.contiguous() for t in yks]
+    yks = [_dense(t) for t in yks]
     _require_cuda(coef, *yks)
     K = len(yks)
     B, H, T, d, two = yks[0].shape
@@ -353,7 +360,7 @@ def state_combine_tokens(coef: torch.Tensor, yks) -> torch.Tensor:
         raise _lib.QPamError(f"state_combine_tokens: bf16/f32 and d a power of two in [4,128]; got {yks[0].dtype}, d={d}")
     if tuple(coef.shape) != (K, B, H, T, 2):
         raise _lib.QPamError(f"state_combine_tokens: coef must be {(K, B, H, T, 2)}, got {tuple(coef.shape)}")
-    cf = coef.float().contiguous()
+    cf = _dense(coef.float())
     y = torch.empty(B, T, H * d, 2, dtype=yks[0].dtype, device=yks[0].device)
     arr = (_lib.c_void_p * K)(*[t.data_ptr() for t in yks])
     check(_lib.lib().qpam_state_combine_tokens_fwd(arr, ptr(cf), ptr(y), dtype_code(y.dtype), K, B, H, T, d, stream_ptr()),
@@ -387,7 +394,7 @@ def state_combine(coef: torch.Tensor, yks, token_major: bool = False) -> torch.T
 class _ScaledResidualFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, delta, scale):
-        x, delta = x.contiguous(), delta.contiguous()
+        x, delta = _dense(x), _dense(delta)
         sc = scale.detach().float().reshape(1)
         out = torch.empty_like(x)
         check(_lib.lib().qpam_scaled_residual_fwd(ptr(x), dtype_code(x.dtype), ptr(delta), dtype_code(delta.dtype), ptr(sc),
@@ -400,7 +407,7 @@ class _ScaledResidualFn(torch.autograd.Function):
     def backward(ctx, dout):
         delta, sc = ctx.saved_tensors
         s_dtype, s_shape, x_dtype = ctx.meta
-        dout = dout.to(x_dtype).contiguous()
+        dout = _dense(dout.to(x_dtype))
         P = max(1, min(148 * 8, delta.numel() // 4096 + 1))
         part = torch.empty(P, dtype=torch.float32, device=delta.device)
         ddelta = torch.empty_like(delta)
@@ -437,7 +444,7 @@ class _BlockWeightFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dw):
         w_dtype, out_dtype, out_dim, in_dim = ctx.meta
-        dw = dw.to(out_dtype).contiguous()
+        dw = _dense(dw.to(out_dtype))
         dwr = torch.empty(out_dim, in_dim, dtype=w_dtype, device=dw.device)
         dwi = torch.empty_like(dwr)
         check(_lib.lib().qpam_block_weight_bwd(ptr(dw), dtype_code(out_dtype), ptr(dwr), ptr(dwi), dtype_code(w_dtype), out_dim,
@@ -463,7 +470,7 @@ class _PamGatesFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, dt, pg, phase, score, dt_bias, dt_off, gamma_floor, K, want_coef):
         B, T, H = dt.shape
-        f = lambda t: None if t is None else t.detach().float().contiguous()
+        f = lambda t: None if t is None else _dense(t.detach().float())
         dtf, pgf, phf, scf, bf, of = f(dt), f(pg), f(phase), f(score), f(dt_bias), f(dt_off)
         dev = dt.device
         gamma = torch.empty(K, B, H, T, dtype=torch.float32, device=dev)
@@ -482,8 +489,8 @@ class _PamGatesFn(torch.autograd.Function):
         gamma_floor, K, dtypes = ctx.meta
         B, T, H = dtf.shape
         dev = dtf.device
-        g = lambda t, ok: None if (t is None or not ok or t.numel() == 0) else t.float().contiguous()
-        dgamma = torch.zeros(K, B, H, T, dtype=torch.float32, device=dev) if dgamma is None else dgamma.float().contiguous()
+        g = lambda t, ok: None if (t is None or not ok or t.numel() == 0) else _dense(t.float())
+        dgamma = torch.zeros(K, B, H, T, dtype=torch.float32, device=dev) if dgamma is None else _dense(dgamma.float())
         domp, dcoef = g(domp, pgf is not None), g(dcoef, True)
         ddt = torch.empty_like(dtf)
         dpg = None if pgf is None else torch.empty_like(pgf)
@@ -527,7 +534,7 @@ def pam_gates(dt, pg, phase, score, dt_bias, state_dt_offset, gamma_floor: float
 class _MagnitudeFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, z):
-        z = z.contiguous()
+        z = _dense(z)
         out = torch.empty(z.shape[:-1], dtype=z.dtype, device=z.device)
         check(_lib.lib().qpam_cmagnitude_fwd(ptr(z), dtype_code(z.dtype), ptr(out), out.numel(), stream_ptr()), "qpam_cmagnitude_fwd")
         ctx.save_for_backward(z)
@@ -536,7 +543,7 @@ class _MagnitudeFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dm):
         (z,) = ctx.saved_tensors
-        dm = dm.to(z.dtype).contiguous()
+        dm = _dense(dm.to(z.dtype))
         dz = torch.empty_like(z)
         check(_lib.lib().qpam_cmagnitude_bwd(ptr(z), ptr(dm), dtype_code(z.dtype), ptr(dz), dm.numel(), stream_ptr()),
               "qpam_cmagnitude_bwd")

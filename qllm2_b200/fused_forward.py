@@ -24,11 +24,12 @@ import torch.nn.functional as F
 
 from . import _lib, ops
 from ._lib import check, dtype_code, ptr, stream_ptr
+from .fused_elementwise import _dense
 from .model import ModSwish, V11LM, build_rope_cache
 
 
 def _f32(t: torch.Tensor) -> torch.Tensor:
-    return t.detach().float().contiguous()
+    return _dense(t.detach().float())
 
 
 class FusedForward:
