@@ -1,9 +1,14 @@
 """The block as one native node against the block operator by operator (torch autograd in between), each against the fp32 block:
-output, input gradient and every parameter's gradient, for each source of the gates and both activations."""
+output, input gradient and every parameter's gradient, for each source of the gates and both activations.  The node's forward has
+the bits of the operators with every state's output rounded to bf16 before the read-out (the form of their scan that keeps no
+chunk states; with one state there is only one form)."""
+import functools
+
 import pytest
 import torch
 
 from qllm2_b200 import model as M
+from qllm2_b200 import ops
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -18,7 +23,7 @@ CONFIGS = {
 
 @pytest.mark.parametrize("name", CONFIGS)
 @pytest.mark.parametrize("B,T,dim,heads", [(2, 130, 64, 2), (1, 5, 388, 3), (3, 257, 768, 2), (2, 1531, 128, 12)])
-def test_native_block_matches_operators(name, B, T, dim, heads):
+def test_native_block_matches_operators(name, B, T, dim, heads, monkeypatch):
     torch.manual_seed(11)
     cfg = M.V11Config(vocab_size=64, dim=dim, n_heads=heads, head_dim=64, n_layers=1, dropout=0.0, gradient_checkpointing=False, max_seq_len=2048, **CONFIGS[name])
     blk = M.V11Block(cfg).to(DEV).train()
@@ -34,10 +39,12 @@ def test_native_block_matches_operators(name, B, T, dim, heads):
     dy = torch.randn(B, T, dim, 2, device=DEV).bfloat16()
     ds = None
     res = {}
-    for mode in ("native", "operators", "fp32"):
+    scan = ops.pam_scan
+    for mode in ("native", "per_state", "operators", "fp32"):
         xi = (x.float() if mode == "fp32" else x).clone().requires_grad_(True)
         blk.zero_grad()
-        hook = blk.norm1.register_forward_hook(lambda *a: None) if mode == "operators" else None      # keeps the operators
+        hook = blk.norm1.register_forward_hook(lambda *a: None) if mode != "native" else None         # keeps the operators
+        monkeypatch.setattr(ops, "pam_scan", functools.partial(scan, save_states=False) if mode == "per_state" else scan)
         with torch.autocast("cuda", dtype=torch.bfloat16, enabled=mode != "fp32"):
             assert blk._native_ok(xi, None) == (mode == "native")
             out, state = blk(xi)
@@ -48,8 +55,8 @@ def test_native_block_matches_operators(name, B, T, dim, heads):
             hook.remove()
         res[mode] = [out.detach().float(), state.detach().float(), xi.grad.float()] + [p.grad for p in blk.parameters()]
     names = ["out", "state", "x"] + [k for k, _ in blk.named_parameters()]
-    if cfg.n_states == 1:
-        assert torch.equal(res["native"][0], res["operators"][0])   # the forward rounds where the operators do
+    for i in (0, 1):                                                # the forward rounds where these operators do
+        assert torch.equal(res["native"][i], res["per_state"][i])
     for n, a, b, ref in zip(names, res["native"], res["operators"], res["fp32"]):
         assert a is not None and torch.isfinite(a).all(), n
         err, err_ops = float((a - ref).norm() / ref.norm()), float((b - ref).norm() / ref.norm())

@@ -32,10 +32,7 @@ def test_forward_only_states(K, H, copies, with_s0):
     q, k, v, gamma, coef, cu, s0 = _inputs(K, H, lens, with_s0)
     y_ref, s_ref = ops.pam_scan(q, k, v, gamma.clone().requires_grad_(True), coef=coef, cu_seqlens=cu, s0=s0, token_major=True)
     y, s = ops.pam_scan_tokens(q, k, v, gamma, coef=coef, cu_seqlens=cu, s0=s0)
-    if K == 1:
-        assert torch.equal(y, y_ref)
-    assert (y.float() - y_ref.float()).norm() <= 1e-2 * y_ref.float().norm()
-    assert torch.equal(s, s_ref)
+    assert torch.equal(y, y_ref) and torch.equal(s, s_ref)
     for dtype in (torch.float32, torch.bfloat16):
         n = len(lens)
         slots = torch.randperm(n + 2, device=DEV)[:n].int()
