@@ -59,6 +59,10 @@ inline bool autocast_bf16() {
   return at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) == at::kBFloat16;
 }
 
+// Descriptor of a packed batch (int32 [S+1]) on the tokens' device; a host descriptor is checked here (the kernels check a
+// device descriptor themselves and report through the status word).
+Tensor descriptor(const Tensor& cu, int64_t T, at::Device device);
+
 // Forward scan with token-major output [B,T,H*d,2] and the final states [K,S,H,d,d,2]; inputs contiguous, of the scan's dtypes.
 std::tuple<Tensor, Tensor> scan_tokens(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gamma, const Tensor& coef, const Tensor& s0,
                                        const Tensor& cu, double q_scale);

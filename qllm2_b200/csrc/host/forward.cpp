@@ -50,17 +50,29 @@ class Packed {
   // ids [B,T]; every row (cu undefined) or every piece of the one packed row (cu [S+1]) belongs to slots[i], whose states
   // [n_slots, L, K, H, d, d, 2] it leaves at its end.  resumed [S] (fp32, 0 or 1): pieces that start from their slot's
   // state.  Returns the residual stream after the last block, normalised for the head, [B*T, D, 2].
-  Tensor prefill(const Tensor& embed_real, const Tensor& embed_imag, const Tensor& ids, const Tensor& pool, const Tensor& slots, const OptTensor& cu_,
+  Tensor prefill(const Tensor& embed_real, const Tensor& embed_imag, const Tensor& ids, const Tensor& pool, const Tensor& slots_, const OptTensor& cu_,
                  const OptTensor& positions_, const OptTensor& resumed_) {
     at::NoGradGuard no_grad;
-    const Tensor cu = value(cu_), resumed = value(resumed_);
-    const int64_t B = ids.size(0), T = ids.size(1), N = B * T, inner = H_ * d_;
+    QH_REQUIRE(ids.dim() == 2 && ids.numel() > 0, "prefill: ids [B,T] expected; got ", shape(ids));
+    const int64_t B = ids.size(0), T = ids.size(1), N = B * T, inner = H_ * d_, L = (int64_t)layers_.size();
     const at::ScalarType dt = layers_[0].w_gu.scalar_type();
-    const Tensor positions = positions_.has_value() ? positions_->reshape({-1}).to(at::kLong).contiguous() : Tensor();
-    QH_REQUIRE(!rope_.defined() || positions.defined() || T <= rope_.size(0), "position beyond max_position of this FusedForward");
-    QH_REQUIRE(pool.is_contiguous() && pool.dim() == 7 && pool.size(1) == (int64_t)layers_.size(), "prefill: state pool does not fit this model");
+    // what the kernels index by pointer: one slot (and one resumed flag) a sequence, a pool of this model's states
+    QH_REQUIRE(embed_real.dim() == 2 && embed_real.size(1) == D_ && embed_real.sizes() == embed_imag.sizes(), "prefill: embeddings [V,", D_, "] expected; got ",
+               shape(embed_real), ", ", shape(embed_imag));
+    QH_REQUIRE(!cu_.has_value() || (B == 1 && cu_->dim() == 1 && cu_->numel() >= 2), "prefill: a packed batch is one row of ids with cu [S+1]");
+    const int64_t n_seq = cu_.has_value() ? cu_->numel() - 1 : B;
+    QH_REQUIRE(slots_.numel() == n_seq && !slots_.is_floating_point() && (!resumed_.has_value() || resumed_->numel() == n_seq), "prefill: one slot a sequence expected, ", n_seq,
+               " in all; got ", shape(slots_));
+    QH_REQUIRE(pool.is_contiguous() && pool.device() == ids.device() && (pool.sizes().slice(1) == at::IntArrayRef{L, K_, H_, d_, d_, 2}) && pool.dim() == 7,
+               "prefill: state pool ", shape(pool), " does not fit this model");
+    QH_REQUIRE(!positions_.has_value() || positions_->numel() == N, "prefill: positions must have one entry per token");
+    QH_REQUIRE(!rope_.defined() || positions_.has_value() || T <= rope_.size(0), "position beyond max_position of this FusedForward");
+    const Tensor cu = descriptor(value(cu_), T, ids.device()), slots = slots_.to(ids.device(), at::kInt).contiguous();
+    const Tensor resumed = resumed_.has_value() ? resumed_->to(ids.device(), at::kFloat) : Tensor();
+    const Tensor positions = positions_.has_value() ? positions_->reshape({-1}).to(ids.device(), at::kLong).contiguous() : Tensor();
+    QH_REQUIRE(ids.is_cuda(), "PAM kernels need CUDA tensors (there is no CPU path in this package)");
     const int code = dtype_code(dt), pool_code = dtype_code(pool.scalar_type());
-    const int64_t n_slots = pool.size(0), L = pool.size(1);
+    const int64_t n_slots = pool.size(0);
     void* st = stream();
     Tensor z = at::stack({at::embedding(embed_real, ids), at::embedding(embed_imag, ids)}, -1).reshape({N, D_, 2}).to(dt);
     const auto opts = z.options();

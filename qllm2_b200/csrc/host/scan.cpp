@@ -152,20 +152,6 @@ Tensor merge_heads(const Tensor& y) {
   return y.transpose(1, 2).reshape({y.size(0), y.size(2), y.size(1) * y.size(3), 2});
 }
 
-// Descriptor of a packed batch on the tokens' device; a host descriptor is checked here (the kernels check a device
-// descriptor themselves and report through the status word).
-Tensor descriptor(const Tensor& cu, const Tensor& q) {
-  if (!cu.defined()) return cu;
-  if (!cu.is_cuda()) {
-    const Tensor c = cu.to(at::kLong).contiguous();
-    const int64_t* p = c.data_ptr<int64_t>();
-    bool ok = c.numel() >= 2 && p[0] == 0 && p[c.numel() - 1] <= q.size(2);
-    for (int64_t i = 1; ok && i < c.numel(); ++i) ok = p[i] >= p[i - 1];
-    QH_REQUIRE(ok, "cu_seqlens must start at 0, never decrease and end at or before T=", q.size(2), "; got ", c.slice(0, 0, 8));
-  }
-  return cu.to(q.device(), at::kInt).contiguous();
-}
-
 struct Inputs {
   Tensor q, k, v, gamma, coef, s0, cu;
   double q_scale;
@@ -201,7 +187,7 @@ Inputs checked(Tensor q, Tensor k, Tensor v, Tensor gamma, const OptTensor& coef
   in.gamma = gamma.contiguous();
   in.coef = coef.defined() ? coef.contiguous() : coef;
   in.s0 = s0.defined() ? s0.contiguous() : s0;
-  in.cu = descriptor(cu, q);
+  in.cu = descriptor(cu, q.size(2), q.device());
   in.q_scale = 1.0 / std::sqrt((double)(head_dim > 0 ? head_dim : d));
   return in;
 }
@@ -252,6 +238,18 @@ std::tuple<Tensor, Tensor> pam_scan_tokens(const Tensor& q, const Tensor& k, con
 }
 
 }  // namespace
+
+Tensor descriptor(const Tensor& cu, int64_t T, at::Device device) {
+  if (!cu.defined()) return cu;
+  if (!cu.is_cuda()) {
+    const Tensor c = cu.to(at::kLong).contiguous();
+    const int64_t* p = c.data_ptr<int64_t>();
+    bool ok = c.numel() >= 2 && p[0] == 0 && p[c.numel() - 1] <= T;
+    for (int64_t i = 1; ok && i < c.numel(); ++i) ok = p[i] >= p[i - 1];
+    QH_REQUIRE(ok, "cu_seqlens must start at 0, never decrease and end at or before T=", T, "; got ", c.slice(0, 0, 8));
+  }
+  return cu.to(device, at::kInt).contiguous();
+}
 
 std::tuple<Tensor, Tensor> scan_tokens(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gamma, const Tensor& coef, const Tensor& s0,
                                        const Tensor& cu, double q_scale) {
