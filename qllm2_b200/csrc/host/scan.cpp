@@ -211,8 +211,8 @@ std::tuple<Tensor, Tensor> forward_only(const Inputs& in, double eps, int64_t ch
   return {token_major && !direct ? merge_heads(y) : y, s_final};
 }
 
-// Returns (y, s_final), or (undefined, undefined) for the one form that is left to the caller: K > 1 tensor-core states
-// whose chunk states are to be recomputed in the backward (save_states = false).
+// Returns (y, s_final), or (undefined, undefined) for the forms that are left to the caller: K > 1 tensor-core states
+// whose chunk states are to be recomputed in the backward (save_states = false), and more of them than one call takes.
 std::tuple<Tensor, Tensor> pam_scan(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gamma, const OptTensor& coef, const OptTensor& s0,
                                     const OptTensor& cu, int64_t head_dim, double eps, int64_t chunk, bool save_states, bool token_major) {
   const Inputs in = checked(q, k, v, gamma, coef, s0, cu, head_dim);
@@ -221,7 +221,7 @@ std::tuple<Tensor, Tensor> pam_scan(const Tensor& q, const Tensor& k, const Tens
   if (!grad) return forward_only(in, eps, chunk, token_major);
   const int64_t K = in.gamma.size(0);
   if (K > 1 && in.q.scalar_type() == at::kBFloat16 && in.q.size(3) == 64 && in.q.size(2) > 0) {
-    if (!save_states) return {Tensor(), Tensor()};
+    if (!save_states || K > QPAM_MAX_STATES) return {Tensor(), Tensor()};
     auto out = ScanStates::apply(in.q, in.k, in.v, in.gamma, opt(in.coef), opt(in.s0), opt(in.cu), in.q_scale, eps, chunk, token_major);
     if (in.coef.defined()) return {out[0], out[1]};
     Tensor y = out[0].sum(0);

@@ -60,10 +60,11 @@ def pam_scan(q, k, v, gamma, *, coef=None, s0=None, cu_seqlens=None, head_dim: O
     y, s = _lib.host().pam_scan(q, k, v, gamma, coef, s0, cu_seqlens, head_dim or 0, eps, chunk, save_states, token_major)
     if y is not None:
         return y, s
-    # K tensor-core states recomputed in the backward: one scan per state, autograd sums the gradients
+    # K tensor-core states recomputed in the backward, or more of them than the fused kernels take: one scan per state, autograd
+    # sums the gradients
     gamma = gamma.float()
     ys, finals = zip(*(pam_scan(q, k, v, gamma[kk:kk + 1], s0=None if s0 is None else s0[kk:kk + 1], cu_seqlens=cu_seqlens, head_dim=head_dim,
-                                eps=eps, chunk=chunk, save_states=False) for kk in range(gamma.shape[0])))
+                                eps=eps, chunk=chunk, save_states=save_states) for kk in range(gamma.shape[0])))
     if coef is None:
         y = ys[0]
         for yk in ys[1:]:

@@ -1,0 +1,42 @@
+"""Ways to call the scan and the loss that a native node in their place has to serve as the operators did."""
+import pytest
+import torch
+
+from qllm2_b200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _data(K, T=140, S=1):
+    g = torch.Generator(device=DEV).manual_seed(K)
+    q, k, v = [(torch.randn(1, 2, T, 64, 2, device=DEV, generator=g) * 0.1).bfloat16() for _ in range(3)]
+    gamma = torch.sigmoid(torch.randn(K, 1, 2, T, device=DEV, generator=g) + 2)
+    return q, k, v, gamma, torch.randn(K, S, 2, 64, 64, 2, device=DEV, generator=g)
+
+
+@pytest.mark.parametrize("save_states", [True, False])
+@pytest.mark.parametrize("token_major", [True, False])
+def test_more_states_than_the_fused_kernels_take(save_states, token_major):
+    """Five states without read-out weights: the sum of five scans, outputs, states and gradients."""
+    q, k, v, gamma, s0 = _data(5, S=2)
+    cu = torch.tensor([0, 60, 140], dtype=torch.int32)
+    leaves = [t.clone().requires_grad_() for t in (q, k, v, gamma, s0)]
+    y, s = ops.pam_scan(*leaves[:4], s0=leaves[4], cu_seqlens=cu, save_states=save_states, token_major=token_major)
+    assert s.shape == (5, 2, 2, 64, 64, 2)
+    dy = torch.randn(y.shape, device=DEV, generator=torch.Generator(device=DEV).manual_seed(9)).bfloat16()
+    got = [y, s, *torch.autograd.grad([y, s], leaves, [dy, s0])]
+    refs = [t.clone().requires_grad_() for t in (q, k, v, gamma, s0)]
+    one = [ops.pam_scan(*refs[:3], refs[3][i:i + 1], s0=refs[4][i:i + 1], cu_seqlens=cu, token_major=token_major) for i in range(5)]
+    y_ref, s_ref = sum(o[0].float() for o in one), torch.cat([o[1] for o in one])
+    want = [y_ref, s_ref, *torch.autograd.grad([y_ref, s_ref], refs, [dy.float(), s0])]
+    for a, b in zip(got, want):       # (bf16 sums of five terms in another order: a few roundings of 2^-9)
+        assert float((a.float() - b.float()).norm() / b.float().norm()) < 1e-2
+
+
+def test_read_out_of_more_states_is_refused():
+    q, k, v, gamma, _ = _data(5)
+    with pytest.raises(_lib.QPamError):
+        ops.pam_scan(q.requires_grad_(), k, v, gamma, coef=torch.ones(5, 1, 2, 140, 2, device=DEV))
+    with pytest.raises(_lib.QPamError):
+        ops.pam_scan(q.detach(), k, v, gamma)
