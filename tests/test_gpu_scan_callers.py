@@ -1,6 +1,7 @@
 """Ways to call the scan and the loss that a native node in their place has to serve as the operators did."""
 import pytest
 import torch
+import torch.autograd.forward_ad as fwAD
 
 from qllm2_b200 import _lib, ops
 
@@ -40,3 +41,16 @@ def test_read_out_of_more_states_is_refused():
         ops.pam_scan(q.requires_grad_(), k, v, gamma, coef=torch.ones(5, 1, 2, 140, 2, device=DEV))
     with pytest.raises(_lib.QPamError):
         ops.pam_scan(q.detach(), k, v, gamma)
+
+
+@pytest.mark.parametrize("which", range(6))
+@pytest.mark.parametrize("call", ["scan", "token_major", "tokens"])
+def test_forward_mode_is_refused(which, call):
+    """Never silently without the tangent, whichever input carries one."""
+    q, k, v, gamma, s0 = _data(3)
+    args = [q, k, v, gamma, torch.ones(3, 1, 2, 140, 2, device=DEV), s0]
+    fn = {"scan": ops.pam_scan, "tokens": ops.pam_scan_tokens}.get(call, lambda *a, **kw: ops.pam_scan(*a, token_major=True, **kw))
+    with fwAD.dual_level():
+        args[which] = fwAD.make_dual(args[which], torch.ones_like(args[which]))
+        with pytest.raises(RuntimeError, match="forward-mode"):
+            fn(*args[:4], coef=args[4], s0=args[5])
