@@ -26,6 +26,34 @@ def _workspace(nbytes: int, device) -> torch.Tensor:
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
 
 
+# --------------------------------------------------------------------------------------- tracing
+class _Recorded(torch.autograd.Function):
+    """A native call as one operator of a torch.jit trace.  A trace records torch operators; the launches of a native call are
+    not among them, and replayed it would hand out its outputs' memory as allocated."""
+
+    @staticmethod
+    def forward(ctx, call, *tensors):
+        ctx.call = call
+        ctx.save_for_backward(*tensors)
+        ctx.set_materialize_grads(False)
+        return call(*tensors)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        leaves = [None if t is None else t.detach().requires_grad_(need) for t, need in zip(ctx.saved_tensors, ctx.needs_input_grad[1:])]
+        with torch.enable_grad():
+            outs = ctx.call(*leaves)
+        pairs = [(o, g) for o, g in zip(outs if isinstance(outs, tuple) else (outs,), grads) if g is not None]
+        wanted = [t for t in leaves if t is not None and t.requires_grad]
+        got = iter(torch.autograd.grad([o for o, _ in pairs], wanted, [g for _, g in pairs], allow_unused=True))
+        return (None, *(next(got) if t is not None and t.requires_grad else None for t in leaves))
+
+
+def recorded(call, *tensors):
+    """call(*tensors), recorded where a trace is being taken."""
+    return _Recorded.apply(call, *tensors) if torch.jit.is_tracing() else call(*tensors)
+
+
 # --------------------------------------------------------------------------------------- scan
 def _scan_args(q, k, v, gamma, coef, s0, cu_seqlens, y, s_final, q_scale, eps, chunk):
     B, H, T, d = q.shape[0], q.shape[1], q.shape[2], q.shape[3]
@@ -57,7 +85,17 @@ def pam_scan(q, k, v, gamma, *, coef=None, s0=None, cu_seqlens=None, head_dim: O
     of the reference, v11/model.py:657-781, is algebraically this sum), as one node whose backward accumulates dq, dk, dv of
     the states in place.
     """
-    y, s = _lib.host().pam_scan(q, k, v, gamma, coef, s0, cu_seqlens, head_dim or 0, eps, chunk, save_states, token_major)
+    def native(q, k, v, gamma, coef, s0, cu):
+        return _lib.host().pam_scan(q, k, v, gamma, coef, s0, cu, head_dim or 0, eps, chunk, save_states, token_major)
+
+    if not torch.jit.is_tracing():
+        y, s = native(q, k, v, gamma, coef, s0, cu_seqlens)
+    else:
+        if torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16:
+            q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()       # what autocast decides belongs to the trace, not to its replay
+        each = (gamma.dim() == 4 and gamma.shape[0] > 1 and (not save_states or gamma.shape[0] > _lib.MAX_STATES) and q.dtype == torch.bfloat16 and
+                q.shape[3] == 64 and torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (q, k, v, gamma, coef, s0)))
+        y, s = (None, None) if each else _Recorded.apply(native, q, k, v, gamma, coef, s0, cu_seqlens)
     if y is not None:
         return y, s
     # K tensor-core states recomputed in the backward, or more of them than the fused kernels take: one scan per state, autograd
@@ -121,7 +159,8 @@ def pam_scan_tokens(q, k, v, gamma, coef=None, s0=None, cu_seqlens=None, *, head
     """Inference form of `pam_scan`: same arguments, but Y comes back token-major, [B, T, H*d, 2] -- the layout
     the output projection reads (the head merge of v11/model.py:835-836) -- and nothing is kept for a backward
     pass (K phase-routed states in bf16 at d = 64 then run the fused K-state output kernel)."""
-    return _lib.host().pam_scan_tokens(q, k, v, gamma, coef, s0, cu_seqlens, head_dim or 0, eps, chunk)
+    return recorded(lambda q, k, v, gamma, coef, s0, cu: _lib.host().pam_scan_tokens(q, k, v, gamma, coef, s0, cu, head_dim or 0, eps, chunk),
+                    q, k, v, gamma, coef, s0, cu_seqlens)
 
 
 # --------------------------------------------------------------------------------------- decode

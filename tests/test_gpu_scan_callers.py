@@ -4,6 +4,8 @@ import torch
 import torch.autograd.forward_ad as fwAD
 
 from qllm2_b200 import _lib, ops
+from qllm2_b200 import model as M
+from qllm2_b200.fused_ce import fused_linear_cross_entropy
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -54,3 +56,43 @@ def test_forward_mode_is_refused(which, call):
         args[which] = fwAD.make_dual(args[which], torch.ones_like(args[which]))
         with pytest.raises(RuntimeError, match="forward-mode"):
             fn(*args[:4], coef=args[4], s0=args[5])
+
+
+@pytest.mark.parametrize("K,grad,call", [(1, False, "scan"), (1, True, "scan"), (3, True, "scan"), (3, True, "token_major"), (3, False, "tokens"), (3, True, "recompute")])
+def test_traced_scan_runs_its_kernels(K, grad, call):
+    """A replayed trace on other inputs equals the call itself, gradients included."""
+    q, k, v, gamma, _ = _data(K)
+    coef = torch.randn(K, 1, 2, 140, 2, device=DEV, generator=torch.Generator(device=DEV).manual_seed(2)) if K > 1 else None
+    kw = {"token_major": dict(token_major=True), "recompute": dict(save_states=False)}.get(call, {})
+    fn = lambda q, k, v, gamma: (ops.pam_scan_tokens if call == "tokens" else ops.pam_scan)(q, k, v, gamma, coef=coef, **kw)
+    inputs = [t.clone().requires_grad_(grad) for t in (q, k, v, gamma)]
+    traced = torch.jit.trace(fn, inputs, check_trace=False)
+    res = []
+    for f in (traced, fn):
+        leaves = [(t.detach() * 0.5).requires_grad_(grad) for t in inputs]
+        y, s = f(*leaves)
+        res.append([y, s, *(torch.autograd.grad([y, s], leaves, [torch.ones_like(y), torch.ones_like(s)]) if grad else ())])
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
+
+
+def test_traced_loss_and_block():
+    g = torch.Generator(device=DEV).manual_seed(3)
+    h, w = torch.randn(48, 64, device=DEV, generator=g).requires_grad_(), torch.randn(100, 64, device=DEV, generator=g).requires_grad_()
+    t = torch.randint(0, 100, (48,), device=DEV, generator=g)
+    traced = torch.jit.trace(fused_linear_cross_entropy, (h, w, t), check_trace=False)
+    res = []
+    for f in (traced, fused_linear_cross_entropy):
+        leaves = [(x.detach() * 0.5).requires_grad_() for x in (h, w)]
+        loss = f(*leaves, t)
+        res.append([loss, *torch.autograd.grad(loss, leaves)])
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
+    torch.manual_seed(0)
+    blk = M.V11Block(M.V11Config(vocab_size=64, dim=64, n_heads=1, head_dim=64, n_layers=1, dropout=0.0, max_seq_len=64)).to(DEV).requires_grad_(False)
+    x = torch.randn(1, 40, 64, 2, device=DEV, generator=g).bfloat16()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        traced = torch.jit.trace(lambda x: blk(x)[0], (x,), check_trace=False)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        want = blk(x * 0.5)[0]
+        assert torch.equal(traced(x * 0.5), want)
