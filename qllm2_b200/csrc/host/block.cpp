@@ -246,9 +246,9 @@ struct Block : Function<Block> {
 
     // ---- residual and output projection of the sequence mix
     Tensor dout = at::empty({N, 2 * D}, o);
-    const int64_t Pr = std::max<int64_t>(1, std::min<int64_t>(148 * 8, x.numel() / 4096 + 1));
+    const int Pr = parts_of(x.numel() / 4096 + 1, 8);
     float* part = partial(Pr, 1);
-    check(qpam_scaled_residual_bwd(dx2.data_ptr(), QPAM_BF16, sv[OUT].data_ptr(), QPAM_BF16, fptr(p[PAM_SCALE]), dout.data_ptr(), part, (int)Pr, x.numel(), st),
+    check(qpam_scaled_residual_bwd(dx2.data_ptr(), QPAM_BF16, sv[OUT].data_ptr(), QPAM_BF16, fptr(p[PAM_SCALE]), dout.data_ptr(), part, Pr, x.numel(), st),
           "qpam_scaled_residual_bwd");
     sum(part, Pr, 1, 1, g[PAM_SCALE]);
     const Tensor dy = at::mm(dout, sv[W_O]);

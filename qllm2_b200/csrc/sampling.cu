@@ -662,7 +662,7 @@ extern "C" int qpam_sample_logits(const void* logits, int32_t io_dtype, int32_t 
   // more rows than SMs: two CTAs of 512 threads share an SM, so that one row's block-wide steps run under the other's
   // passes; otherwise a row has an SM to itself and takes 1024 threads
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const bool wide = n <= 148;
+  const bool wide = n <= sm_count();
   if (io_dtype == QPAM_F32) return wide ? sample_launch<float, 1024>(p, smem, st) : sample_launch<float, 512>(p, smem, st);
   return wide ? sample_launch<__nv_bfloat16, 1024>(p, smem, st) : sample_launch<__nv_bfloat16, 512>(p, smem, st);
 }

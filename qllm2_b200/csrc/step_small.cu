@@ -1147,7 +1147,7 @@ int launch_pdl(const char* name, void (*kern)(Params...), dim3 grid, int threads
 // Cluster size that splits K so that a projection with few rows still covers the SMs
 int split_of(int tiles, int kblocks) {
   int cs = 1;
-  while (cs < 8 && tiles * cs < 148 && kblocks / (cs * 2) >= ST_WARPS / 2) cs *= 2;
+  while (cs < 8 && tiles * cs < sm_count() && kblocks / (cs * 2) >= ST_WARPS / 2) cs *= 2;
   return cs;
 }
 

@@ -35,6 +35,10 @@ def _dense(t: torch.Tensor) -> torch.Tensor:
     return t.clone() if t.data_ptr() % 16 else t
 
 
+def _sms(t: torch.Tensor) -> int:
+    return torch.cuda.get_device_properties(t.device).multi_processor_count
+
+
 def _rows(t: torch.Tensor):
     """(tensor, N, C, row stride in scalars) of a [..., C, 2] tensor; copies only if rows are not uniform."""
     if t.dim() < 2 or t.shape[-1] != 2:
@@ -86,7 +90,7 @@ class _ComplexNormFn(torch.autograd.Function):
         D = z.shape[-2]
         N = z.numel() // (2 * D)
         dout = _dense(dout.to(ctx.out_dtype))
-        P = max(4, min((N + 3) // 4 * 4, 148 * 16))
+        P = max(4, min((N + 3) // 4 * 4, _sms(z) * 16))
         part = torch.empty(P, D, dtype=torch.float32, device=z.device)
         dz = torch.empty_like(z)
         sc = _param(scale, D, "scale")
@@ -408,7 +412,7 @@ class _ScaledResidualFn(torch.autograd.Function):
         delta, sc = ctx.saved_tensors
         s_dtype, s_shape, x_dtype = ctx.meta
         dout = _dense(dout.to(x_dtype))
-        P = max(1, min(148 * 8, delta.numel() // 4096 + 1))
+        P = max(1, min(_sms(delta) * 8, delta.numel() // 4096 + 1))
         part = torch.empty(P, dtype=torch.float32, device=delta.device)
         ddelta = torch.empty_like(delta)
         check(_lib.lib().qpam_scaled_residual_bwd(ptr(dout), dtype_code(x_dtype), ptr(delta), dtype_code(delta.dtype), ptr(sc),
@@ -496,7 +500,7 @@ class _PamGatesFn(torch.autograd.Function):
         dpg = None if pgf is None else torch.empty_like(pgf)
         dph = None if phf is None else torch.empty_like(phf)
         dsc = None if scf is None else torch.empty_like(scf)
-        P = max(1, min(148 * 4, (dtf.numel() + 255) // 256))
+        P = max(1, min(_sms(dtf) * 4, (dtf.numel() + 255) // 256))
         part = torch.empty(P, H, K, dtype=torch.float32, device=dev)
         check(_lib.lib().qpam_pam_gates_bwd(ptr(dtf), ptr(pgf), ptr(phf), ptr(scf), ptr(bf), ptr(of), float(gamma_floor),
                                             ptr(dgamma), ptr(domp), ptr(dcoef), ptr(ddt), ptr(dpg), ptr(dph), ptr(dsc),
