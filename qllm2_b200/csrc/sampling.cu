@@ -612,7 +612,11 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sample_rows(SamplePar
 
 template <typename T, int NT>
 int sample_launch(const SampleParams& p, size_t smem, cudaStream_t st) {
-  if (smem > 0) QPAM_CUDA(cudaFuncSetAttribute(k_sample_rows<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the opt-in only ever grows (another thread may be between its opt-in and its launch for a larger vocabulary); allow_smem
+  // reckons with 16 KB of static shared memory
+  static_assert(sizeof(Scratch) >= 16 * 1024, "");
+  const int rc = allow_smem(reinterpret_cast<const void*>(k_sample_rows<T, NT>), smem + sizeof(Scratch) - 16 * 1024);
+  if (rc) return rc;
   k_sample_rows<T, NT><<<p.n, NT, smem, st>>>(p);
   QPAM_LAUNCH_CHECK("k_sample_rows");
   return QPAM_OK;

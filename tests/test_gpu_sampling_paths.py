@@ -1,5 +1,7 @@
 """The sampler's dispatch at its edges: list and bin paths around the list's top-k limit, rows that start off a 16-byte
 boundary, rows shorter than the block, and rows whose ties overflow the list."""
+import threading
+
 import pytest
 import torch
 
@@ -35,3 +37,33 @@ def test_ties_beyond_the_list(top_k, top_p):
     ids, stats = ops.sample_logits(logits, u.to(DEV), return_stats=True, **cfg)
     _check_rows(logits, None, None, u.numpy(), ids.cpu().numpy(), stats.cpu().numpy(), cfg)
     assert stats[:, 2].tolist() == (logits == 1).sum(1).tolist()
+
+
+def test_threads_with_vocabularies_of_different_size():
+    """The penalty's bitmap is sized by the vocabulary: threads with different ones do not shrink each other's shared memory."""
+    errors, want = [], {}
+
+    def draw(V):
+        g = torch.Generator().manual_seed(V)
+        logits, hist = torch.randn(2, V, generator=g).to(DEV), torch.randint(0, V, (2, 9), generator=g).to(DEV)
+        u = torch.rand(2, generator=g).to(DEV)
+        return lambda: ops.sample_logits(logits, u, history=hist, top_k=20, repetition_penalty=1.2)
+
+    calls = {V: draw(V) for V in (1000, 200_000, 1_200_000)}
+    for V, f in calls.items():
+        want[V] = f().tolist()
+
+    def work(V):
+        try:
+            for _ in range(200):
+                got = calls[V]()
+            assert got.tolist() == want[V]
+        except Exception as e:      # reported in the test's own thread
+            errors.append((V, e))
+
+    ts = [threading.Thread(target=work, args=(V,)) for V in calls]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors
