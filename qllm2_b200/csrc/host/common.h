@@ -45,13 +45,14 @@ inline int dtype_code(at::ScalarType t) {
 inline Tensor workspace(size_t bytes, const Tensor& like) {
   return at::empty({(int64_t)std::max<size_t>(bytes, 256)}, like.options().dtype(at::kByte));
 }
-inline Tensor f32(const Tensor& t) { return t.defined() ? t.to(at::kFloat).contiguous() : t; }
-// Contiguous and starting on a 16-byte boundary, as the kernels' vector accesses need it (a view into a flat buffer may start
-// anywhere).  Differentiable like the copies it is made of.
-inline Tensor dense(const Tensor& t) {
+// Contiguous and starting on a boundary of `align` bytes, as the kernels' vector accesses need it (a view into a flat buffer may
+// start anywhere).  Differentiable like the copies it is made of.
+inline Tensor dense(const Tensor& t, size_t align = 16) {
   const Tensor c = t.contiguous();
-  return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) ? c.clone() : c;
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % align ? c.clone() : c;
 }
+// Token tensors: whole complex numbers at least.  (Off a 16-byte boundary the scan takes them through its scalar kernels.)
+inline Tensor dense_tokens(const Tensor& t) { return dense(t, 2 * t.element_size()); }
 inline bool needs_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
 inline std::string shape(const Tensor& t) { return c10::str(t.sizes()); }
 

@@ -49,18 +49,21 @@ struct LinearCE : Function<LinearCE> {
   }
 };
 
-void check_rows(const Tensor& h, const Tensor& w, const Tensor& targets) {
-  QH_REQUIRE(h.is_cuda() && w.is_cuda(), "PAM kernels need CUDA tensors (there is no CPU path in this package)");
+void check_rows(const Tensor& h, const Tensor& w, const Tensor& targets, const Tensor& mask) {
+  QH_REQUIRE(h.is_cuda(), "PAM kernels need CUDA tensors (there is no CPU path in this package)");
+  for (const Tensor* t : {&w, &targets, &mask})
+    QH_REQUIRE(!t->defined() || t->device() == h.device(), "the loss's operands are on different devices: ", h.device(), " and ", t->device());
   QH_REQUIRE(h.dim() == 2 && w.dim() == 2 && h.size(1) == w.size(1), "h [N,F] and w [V,F] expected; got ", shape(h), ", ", shape(w));
   QH_REQUIRE(targets.scalar_type() == at::kLong && targets.numel() == h.size(0), "targets must be int64 with one entry per row of h");
+  QH_REQUIRE(!mask.defined() || mask.numel() == h.size(0), "mask must have one entry per row of hidden_rows");
 }
 
 Tensor linear_ce(const Tensor& hidden, const Tensor& weight, const Tensor& targets, const OptTensor& mask, int64_t ignore_index, int64_t v_offset) {
   Tensor h = hidden.contiguous(), w = weight.contiguous();
   if (w.scalar_type() != h.scalar_type()) w = w.to(h.scalar_type());
-  check_rows(h, w, targets);
   OptTensor m;
   if (mask.has_value()) m = mask->to(at::kFloat).contiguous();
+  check_rows(h, w, targets, value(m));
   return LinearCE::apply(h, w, targets.contiguous(), m, ignore_index, v_offset);
 }
 
@@ -68,8 +71,8 @@ Tensor linear_ce(const Tensor& hidden, const Tensor& weight, const Tensor& targe
 std::tuple<Tensor, Tensor> linear_ce_rows(const Tensor& hidden, const Tensor& weight, const Tensor& targets_, const OptTensor& mask, int64_t ignore_index) {
   at::NoGradGuard no_grad;
   const Tensor h = hidden.contiguous(), w = weight.to(hidden.scalar_type()).contiguous(), targets = targets_.contiguous();
-  check_rows(h, w, targets);
   const Tensor m = mask.has_value() ? mask->to(at::kFloat).contiguous() : Tensor();
+  check_rows(h, w, targets, m);
   qpam_ce_args a = ce_args(h, w, targets, m, ignore_index, 0);
   Tensor ws = workspace(qpam_ce_workspace_bytes(&a, 0), h);
   a.workspace = ws.data_ptr();

@@ -37,7 +37,7 @@ Tensor final_states(const qpam_scan_args& a, const Tensor& q) {
 Tensor grad_states(const Tensor& ds, const qpam_scan_args& a) {
   if (!ds.defined()) return ds;
   QH_REQUIRE(ds.numel() == (int64_t)a.K * a.S * a.H * a.d * a.d * 2, "ds_final has the wrong number of elements");
-  return f32(ds);
+  return dense(ds.to(at::kFloat));
 }
 
 // One scan (all K states in its kernels).  Inputs contiguous, gamma / coef / s0 fp32.
@@ -69,7 +69,7 @@ struct Scan : Function<Scan> {
     Tensor ws = s[7];
     const Config c{ctx->saved_data["q_scale"].toDouble(), ctx->saved_data["eps"].toDouble(), ctx->saved_data["chunk"].toInt()};
     qpam_scan_args a = scan_args(q, k, v, gamma, coef, s0, cu, Tensor(), Tensor(), c);
-    const Tensor dy = grads[0].defined() ? grads[0].to(q.scalar_type()).contiguous() : at::zeros_like(q);
+    const Tensor dy = grads[0].defined() ? dense_tokens(grads[0].to(q.scalar_type())) : at::zeros_like(q);
     QH_REQUIRE(dy.sizes() == q.sizes(), "dy shape ", shape(dy), " != y shape ", shape(q));
     const Tensor ds = grad_states(grads[1], a);
     Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), dgamma = at::empty_like(gamma);
@@ -131,12 +131,12 @@ struct ScanStates : Function<ScanStates> {
     Tensor ds0 = s0.defined() && ctx->saved_data["ds0"].toBool() ? at::empty_like(s0) : Tensor();
     if (coef.defined()) {
       dcoef = at::empty_like(coef);
-      const Tensor dy = grads[0].defined() ? grads[0].to(q.scalar_type()).contiguous() : at::zeros({q.numel()}, q.options());
+      const Tensor dy = grads[0].defined() ? dense(grads[0].to(q.scalar_type())) : at::zeros({q.numel()}, q.options());
       const auto bwd = tokens ? &qpam_scan_bwd_tokens : &qpam_scan_bwd;
       check(bwd(&a, dy.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), fptr(dgamma), fptr(dcoef), fptr(ds), fptr(ds0), 1, stream()), "qpam_scan_bwd");
       return {dq, dk, dv, dgamma, dcoef, ds0, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     }
-    const Tensor dys = grads[0].defined() ? grads[0].to(q.scalar_type()).contiguous() : at::zeros({K, B, H, T, d, 2}, q.options());
+    const Tensor dys = grads[0].defined() ? dense(grads[0].to(q.scalar_type())) : at::zeros({K, B, H, T, d, 2}, q.options());
     void* dyk[QPAM_MAX_STATES];
     state_ptrs(dys, dyk);
     const int64_t row = B * H * T, st = (int64_t)a.S * H * d * d * 2;
@@ -184,12 +184,14 @@ Inputs checked(Tensor q, Tensor k, Tensor v, Tensor gamma, const OptTensor& coef
     QH_REQUIRE((s0.sizes() == at::IntArrayRef{gamma.size(0), n_seq, q.size(1), d, d, 2}), "s0 shape ", shape(s0), " != [K,S,H,d,d,2]");
   }
   QH_REQUIRE(!cu.defined() || q.size(0) == 1, "packed mode (cu_seqlens) needs B == 1");
-  QH_REQUIRE(q.is_cuda() && k.is_cuda() && v.is_cuda() && gamma.is_cuda(), "PAM kernels need CUDA tensors (there is no CPU path in this package)");
+  for (const Tensor* t : {&k, &v, &gamma, &coef, &s0})
+    QH_REQUIRE(!t->defined() || t->device() == q.device(), "the scan's operands are on different devices: ", q.device(), " and ", t->device());
+  QH_REQUIRE(q.is_cuda(), "PAM kernels need CUDA tensors (there is no CPU path in this package)");
   Inputs in;
-  in.q = q.contiguous(); in.k = k.contiguous(); in.v = v.contiguous();
+  in.q = dense_tokens(q); in.k = dense_tokens(k); in.v = dense_tokens(v);
   in.gamma = gamma.contiguous();
-  in.coef = coef.defined() ? coef.contiguous() : coef;
-  in.s0 = s0.defined() ? s0.contiguous() : s0;
+  in.coef = coef.defined() ? dense(coef) : coef;
+  in.s0 = s0.defined() ? dense(s0) : s0;
   in.cu = descriptor(cu, q.size(2), q.device());
   in.q_scale = 1.0 / std::sqrt((double)(head_dim > 0 ? head_dim : d));
   return in;

@@ -171,7 +171,7 @@ def pam_decode_step(state_pool, slot_ids, q_scaled, k, v, gamma, coef=None, *, l
     slot_ids int32 [n].  Returns y [n,H,d,2].  (v11/model.py:927-965)
     """
     L = _lib.lib()
-    _require_cuda(state_pool, q_scaled)
+    _require_cuda(state_pool, q_scaled, k, v, gamma, coef)
     n_slots, n_layers, K, H, d = state_pool.shape[:5]
     if gamma.dim() == 2:
         gamma = gamma.unsqueeze(0)
@@ -203,6 +203,7 @@ def pam_decode_step(state_pool, slot_ids, q_scaled, k, v, gamma, coef=None, *, l
 def pam_pool_store(state_pool, slot_ids, states, *, layer: int = 0):
     """Write prefill states [K,S,H,d,d,2] (float32) into pool slots ``slot_ids`` [S]."""
     L = _lib.lib()
+    _require_cuda(state_pool, states)
     n_slots, n_layers, K, H, d = state_pool.shape[:5]
     states = states.float().contiguous()
     S = states.shape[1]

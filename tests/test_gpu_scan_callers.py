@@ -5,7 +5,7 @@ import torch.autograd.forward_ad as fwAD
 
 from qllm2_b200 import _lib, ops
 from qllm2_b200 import model as M
-from qllm2_b200.fused_ce import fused_linear_cross_entropy
+from qllm2_b200.fused_ce import fused_linear_cross_entropy, linear_ce_stats
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -96,3 +96,52 @@ def test_traced_loss_and_block():
     with torch.autocast("cuda", dtype=torch.bfloat16):
         want = blk(x * 0.5)[0]
         assert torch.equal(traced(x * 0.5), want)
+
+
+def _off(t, elements=1):
+    """The same values, `elements` behind an aligned address."""
+    v = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)[elements:elements + t.numel()].view(t.shape)
+    return v.copy_(t)
+
+
+@pytest.mark.parametrize("K,dtype", [(1, torch.bfloat16), (3, torch.bfloat16), (1, torch.float32), (2, torch.float32)])
+@pytest.mark.parametrize("token_major", [False, True])
+def test_operands_off_their_alignment(K, dtype, token_major):
+    """Every operand one element behind an aligned address: the results of the aligned ones."""
+    q, k, v, gamma, s0 = _data(K)
+    data = [t.to(dtype) for t in (q, k, v)] + [gamma, s0] + ([torch.randn(K, 1, 2, 140, 2, device=DEV)] if K > 1 else [])
+    res = []
+    for place in (torch.clone, _off):
+        leaves = [place(t).requires_grad_() for t in data]
+        y, s = ops.pam_scan(*leaves[:4], s0=leaves[4], coef=leaves[5] if K > 1 else None, token_major=token_major)
+        g = [place(torch.linspace(-1, 1, t.numel(), device=DEV).view(t.shape).to(t.dtype)) for t in (y, s)]
+        res.append([y, s, *torch.autograd.grad([y, s], leaves, g)])
+    for a, b in zip(*res):
+        if dtype is torch.float32:
+            assert torch.equal(a, b)
+        else:                     # (an output gradient off its alignment takes the scalar kernels backward: bf16 rounding apart)
+            assert float((a.detach().float() - b.detach().float()).norm() / a.detach().float().norm()) < 1e-2
+
+
+def test_operands_on_other_devices_are_refused():
+    """Host memory never reaches a kernel as a pointer."""
+    q, k, v, gamma, s0 = _data(3)
+    coef = torch.ones(3, 1, 2, 140, 2, device=DEV)
+    for i in range(1, 6):
+        a = [q, k, v, gamma, coef, s0]
+        a[i] = a[i].cpu()
+        with pytest.raises(_lib.QPamError, match="devices"):
+            ops.pam_scan(*a[:4], coef=a[4], s0=a[5])
+    h, w = torch.randn(8, 64, device=DEV), torch.randn(30, 64, device=DEV)
+    t, m = torch.randint(0, 30, (8,), device=DEV), torch.ones(8, device=DEV)
+    for a in ((h, w.cpu(), t, m), (h, w, t.cpu(), m), (h, w, t, m.cpu())):
+        for fn in (fused_linear_cross_entropy, linear_ce_stats):
+            with pytest.raises(_lib.QPamError, match="devices"):
+                fn(*a[:3], mask=a[3])
+    with pytest.raises(_lib.QPamError, match="one entry per row"):
+        linear_ce_stats(h, w, t, mask=m[:5])
+    pool, one = torch.zeros(2, 1, 1, 2, 64, 64, 2, device=DEV), torch.zeros(1, 2, 64, 2, device=DEV)
+    with pytest.raises(_lib.QPamError):
+        ops.pam_decode_step(pool, torch.tensor([0]), one, one.cpu(), one, torch.ones(1, 1, 2, device=DEV))
+    with pytest.raises(_lib.QPamError):
+        ops.pam_pool_store(pool, torch.tensor([0]), torch.zeros(1, 1, 2, 64, 64, 2))
