@@ -47,18 +47,19 @@ class Packed {
     }
   }
 
-  // ids [B,T]; every row (cu undefined) or every piece of the one packed row (cu [S+1]) belongs to slots[i], whose states
+  // embed_real, embed_imag [V,D], or the embedded tokens [B,T,D,2]; ids [B,T]; every row (cu undefined) or every piece of the one packed row (cu [S+1]) belongs to slots[i], whose states
   // [n_slots, L, K, H, d, d, 2] it leaves at its end.  resumed [S] (fp32, 0 or 1): pieces that start from their slot's
   // state.  Returns the residual stream after the last block, normalised for the head, [B*T, D, 2].
-  Tensor prefill(const Tensor& embed_real, const Tensor& embed_imag, const Tensor& ids, const Tensor& pool, const Tensor& slots_, const OptTensor& cu_,
+  Tensor prefill(const OptTensor& embed_real, const OptTensor& embed_imag, const OptTensor& embedded, const Tensor& ids, const Tensor& pool, const Tensor& slots_, const OptTensor& cu_,
                  const OptTensor& positions_, const OptTensor& resumed_) {
     at::NoGradGuard no_grad;
     QH_REQUIRE(ids.dim() == 2 && ids.numel() > 0, "prefill: ids [B,T] expected; got ", shape(ids));
     const int64_t B = ids.size(0), T = ids.size(1), N = B * T, inner = H_ * d_, L = (int64_t)layers_.size();
     const at::ScalarType dt = layers_[0].w_gu.scalar_type();
     // what the kernels index by pointer: one slot (and one resumed flag) a sequence, a pool of this model's states
-    QH_REQUIRE(embed_real.dim() == 2 && embed_real.size(1) == D_ && embed_real.sizes() == embed_imag.sizes(), "prefill: embeddings [V,", D_, "] expected; got ",
-               shape(embed_real), ", ", shape(embed_imag));
+    const auto is_table = [&](const OptTensor& t) { return t.has_value() && t->dim() == 2 && t->size(1) == D_; };
+    QH_REQUIRE(embedded.has_value() ? embedded->sizes() == at::IntArrayRef({B, T, D_, 2}) : is_table(embed_real) && is_table(embed_imag),
+               "prefill: embeddings [V,", D_, "] or embedded tokens [B,T,", D_, ",2] expected");
     QH_REQUIRE(!cu_.has_value() || (B == 1 && cu_->dim() == 1 && cu_->numel() >= 2), "prefill: a packed batch is one row of ids with cu [S+1]");
     const int64_t n_seq = cu_.has_value() ? cu_->numel() - 1 : B;
     QH_REQUIRE(slots_.numel() == n_seq && !slots_.is_floating_point() && (!resumed_.has_value() || resumed_->numel() == n_seq), "prefill: one slot a sequence expected, ", n_seq,
@@ -74,7 +75,8 @@ class Packed {
     const int code = dtype_code(dt), pool_code = dtype_code(pool.scalar_type());
     const int64_t n_slots = pool.size(0);
     void* st = stream();
-    Tensor z = at::stack({at::embedding(embed_real, ids), at::embedding(embed_imag, ids)}, -1).reshape({N, D_, 2}).to(dt);
+    Tensor z = (embedded.has_value() ? *embedded : at::stack({at::embedding(*embed_real, ids), at::embedding(*embed_imag, ids)}, -1)).reshape({N, D_, 2}).to(dt);
+    z = dense(z);
     const auto opts = z.options();
     Tensor xn = at::empty_like(z), mag;
     check(qpam_residual_cnorm_fwd(z.data_ptr(), nullptr, nullptr, fptr(embed_scale_), xn.data_ptr(), nullptr, code, N, (int)D_, 1e-6f, st),

@@ -21,6 +21,7 @@ from typing import Optional
 
 import torch
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _lib, ops
 from ._lib import check, dtype_code, ptr, stream_ptr
@@ -30,6 +31,14 @@ from .model import ModSwish, V11LM, build_rope_cache
 
 def _f32(t: torch.Tensor) -> torch.Tensor:
     return _dense(t.detach().float())
+
+
+def _is_table(m) -> bool:
+    """Whether an embedding is its weight's rows and nothing else (no subclass, hook or renormalisation), laid out as the kernels
+    read it; anything else is called as the module it is."""
+    w = m.weight if type(m) is torch.nn.Embedding else None
+    return (w is not None and m.max_norm is None and "forward" not in m.__dict__ and not m._forward_hooks and not m._forward_pre_hooks and
+            not _has_any_global_hook() and w.is_contiguous() and w.data_ptr() % 16 == 0)
 
 
 class FusedForward:
@@ -215,19 +224,23 @@ class FusedForward:
         h, _ = self._res_norm(h, None, None, self.head_norm_scale)
         return h
 
+    @torch.no_grad()
     def prefill(self, ids, pool, slots, cu=None, positions=None, resumed=None):
         """Absorb prompts: ids [B, T] (cu None: a prompt per row; otherwise the pieces of one packed row, cu int32 [S+1]) into the
         states of `slots` int32 [S] of `pool` [n_slots, L, K, H, d, d, 2].  resumed float32 [S]: 1 for pieces that continue from
         their slot's state.  Returns what `hidden` does.  (csrc/host/forward.cpp: the same launches as `hidden` around a scan,
         ~15 per block; issuing them from Python took longer than the GPU needs for a few hundred tokens.)"""
-        emb = self.model.embed
-        return self._native.prefill(emb.embed_real.weight, emb.embed_imag.weight, ids, pool, slots, cu, positions, resumed)
+        er, ei = self.model.embed.embed_real, self.model.embed.embed_imag
+        if _is_table(er) and _is_table(ei):
+            return self._native.prefill(er.weight, ei.weight, None, ids, pool, slots, cu, positions, resumed)
+        return self._native.prefill(None, None, torch.stack([er(ids), ei(ids)], dim=-1), ids, pool, slots, cu, positions, resumed)
 
     # ---------------------------------------------------------------------------------- decode step for few rows
     def step_supported(self, n: int) -> bool:
         """Whether `step` covers a batch of n rows: few enough that the weights' bytes, not the arithmetic, set the
         time (there the step reads half of them in a third of the launches), bf16 weights, head dim 64."""
-        return (self.dtype == torch.bfloat16 and self.model.embed.embed_real.weight.dtype == torch.bfloat16 and
+        er, ei = self.model.embed.embed_real, self.model.embed.embed_imag
+        return (self.dtype == torch.bfloat16 and _is_table(er) and _is_table(ei) and er.weight.dtype == ei.weight.dtype == torch.bfloat16 and
                 bool(_lib.lib().qpam_step_supported(n, self.D, self.H, self.d, self.K, self.layers[0].hidden, self.w_vocab.shape[0])))
 
     def _pack_step_layers(self):
