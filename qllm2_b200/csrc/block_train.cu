@@ -403,7 +403,8 @@ __global__ void __launch_bounds__(128) k_cnorm_res_bwd(const bf16* __restrict__ 
 // q, k, v; d/4 neighbouring lanes sum a head's Re<dv, v>, which the gate threads -- one (token, head) each -- turn into
 // the protect gate's gradient beside the decay's and the read-out weights'.  A tile is as long as the grid allows (28 tokens
 // at 16384 tokens): its two barriers and the gates' chain of small loads and transcendentals are paid once for all its
-// tokens, while another CTA of the SM streams (112 us with tiles of four tokens, 27 us of traffic).
+// tokens, while another CTA of the SM streams (112 us with tiles of four tokens, 47 us
+// so; 27 us of traffic).
 __global__ void __launch_bounds__(1024) k_front_bwd(const __grid_constant__ qpam_front_bwd_args p, int per_tok_pad, int tile_tok) {
   const qpam_front_args& a = p.f;
   extern __shared__ float domp[];             // [tile_tok][H], then the CTA's sums [tile_tok * H][3K + 1]

@@ -259,7 +259,7 @@ struct Block : Function<Block> {
     qpam_scan_args a = scan_args(s, sv[Q], sv[KK], sv[V], sv[GAMMA]);
     a.workspace = sv[WS].data_ptr();
     a.workspace_bytes = (size_t)sv[WS].numel();
-    const Tensor ds = grads[1].defined() ? grads[1].to(at::kFloat).contiguous() : Tensor();
+    const Tensor ds = grads[1].defined() ? dense(grads[1].to(at::kFloat)) : Tensor();
     if (K == 1) {
       const Tensor dyh = dy.view({s.B, s.T, H, d, 2}).transpose(1, 2).contiguous();
       check(qpam_scan_bwd(&a, dyh.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), fptr(dgamma), nullptr, fptr(ds), nullptr, 1, st), "qpam_scan_bwd");

@@ -5,6 +5,7 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/extension.h>
 
 #include "qllm2_pam.h"
@@ -14,9 +15,10 @@ namespace qhost {
 using at::Tensor;
 using OptTensor = std::optional<Tensor>;
 
-// Turned into qllm2_b200._lib.QPamError by the module's exception translator.
-struct Error : std::runtime_error {
-  using std::runtime_error::runtime_error;
+// qllm2_b200._lib.QPamError in Python: by the module's exception translator in a call, by torch's from a backward pass.
+struct Error : torch::PyTorchError {
+  using PyTorchError::PyTorchError;
+  PyObject* python_type() override;
 };
 
 template <typename... Args>

@@ -2,13 +2,14 @@
 
 namespace py = pybind11;
 
+PyObject* qhost::Error::python_type() { return py::module_::import("qllm2_b200._lib").attr("QPamError").ptr(); }   // (the module keeps it)
+
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   py::register_exception_translator([](std::exception_ptr p) {
     try {
       if (p) std::rethrow_exception(p);
-    } catch (const qhost::Error& e) {
-      py::object cls = py::module_::import("qllm2_b200._lib").attr("QPamError");
-      PyErr_SetString(cls.ptr(), e.what());
+    } catch (qhost::Error& e) {
+      PyErr_SetString(e.python_type(), e.what());
     }
   });
   qhost::bind_scan(m);

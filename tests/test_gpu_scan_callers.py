@@ -145,3 +145,14 @@ def test_operands_on_other_devices_are_refused():
         ops.pam_decode_step(pool, torch.tensor([0]), one, one.cpu(), one, torch.ones(1, 1, 2, device=DEV))
     with pytest.raises(_lib.QPamError):
         ops.pam_pool_store(pool, torch.tensor([0]), torch.zeros(1, 1, 2, 64, 64, 2))
+
+
+@pytest.mark.parametrize("K", [1, 3])
+def test_errors_of_a_backward_pass_are_qpam_errors(K):
+    """Here a workspace that comes back too small from a saved-tensor hook, which the call refuses before any launch."""
+    q, k, v, gamma, _ = _data(K)
+    q.requires_grad_()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t[:256].clone() if t.dtype == torch.uint8 else t):
+        y, _ = ops.pam_scan(q, k, v, gamma, coef=torch.ones(K, 1, 2, 140, 2, device=DEV) if K > 1 else None)
+    with pytest.raises(_lib.QPamError, match="workspace"):
+        y.float().sum().backward()
