@@ -119,8 +119,8 @@ constexpr size_t OUTER_SMEM = 1024 + 32768 + 32768 + 1024;
 // (k_chunk_jobs), so the predecessor of a job is usually done; a job only ever waits for a smaller ticket, whose CTA has
 // started, so the waiting ends (and is bounded like every other wait).  ticket[1] == 0: too few sequences side by side for
 // that, the sums are left to k_state_scan.
-// 32 documents of 512..16384 tokens, 16 heads: 692 us where the sums and the carry took 515 + 322.  (K states take their links
-// one after the other in a CTA; with three the pass of its own was as fast.)
+// 32 documents of 512..16384 tokens (241,740 in all), 16 heads: 676 us where the sums and a carry of its own take 516 + 334.  (K
+// states take their links one after the other in a CTA; with three the pass of its own was as fast.)
 enum OuterMode { OUTER_PLAIN = 0, OUTER_FWD_ONLY = 1, OUTER_CARRY = 2 };
 
 __device__ __forceinline__ bool wait_ready(const unsigned int* flag) {

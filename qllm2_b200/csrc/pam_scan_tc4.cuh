@@ -13,10 +13,8 @@
 // The scores do not depend on the state, so K states cost one pass of the tile products; what a state adds is its term of
 // the weight G, its sums of Z and its carried-state products.  dc and the decay gradient come from the fp32 scores (no
 // per-state output is needed, and the contribution of every (t, s) pair to Re<q,dq> - Re<k,dk> cancels to fp32 rounding).
-//
-//
-// (One state keeps the three-job kernel of pam_scan_tc2.cuh: two CTAs on an SM hide each other's waits there, 108 us against
-// 118 us here at 8 x 6 x 2048; three states took 420 us that way, read-out weights included, and take 229 us.)
+// (One state keeps the three-job kernel of pam_scan_tc2.cuh: two CTAs on an SM hide each other's waits there, 102-106 us against
+// 118 us here at 8 x 6 x 2048; three states took 420 us that way, read-out weights included, and take 230-235 us.)
 //
 // Every score is formed twice, once per direction of the sum (a row of the tile is a TMEM lane, so sums along a row stay
 // inside threads): pass A has tokens t as rows (dq, dc), pass B tokens s (dk, dv, Re<k,dk>).  512 threads: a thread owns a

@@ -111,6 +111,8 @@ def fused_linear_cross_entropy(
         raise ValueError("mask must have one entry per row of hidden_rows")
     if group is not None or hidden_rows.shape[0] == 0:
         return _ShardedLinearCE.apply(hidden_rows, weight_matrix, targets, mask, ignore_index, group, vocab_start)
+    if not ops.is_tracing():
+        return _lib.host().linear_ce(hidden_rows, weight_matrix, targets, mask, ignore_index, vocab_start)
     return ops.recorded(lambda h, w, t, m: _lib.host().linear_ce(h, w, t, m, ignore_index, vocab_start), hidden_rows, weight_matrix, targets, mask)
 
 

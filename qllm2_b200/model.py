@@ -539,7 +539,7 @@ class V11Block(nn.Module):
         if (pam_state is not None or not x.is_cuda or x.dtype != torch.bfloat16 or x.shape[1] < 2 or not torch.is_autocast_enabled("cuda")
                 or torch.get_autocast_dtype("cuda") != torch.bfloat16):
             return False
-        if type(self) is not V11Block or _has_any_global_hook() or not _stock(self) or torch.jit.is_tracing():   # (a trace records operators)
+        if type(self) is not V11Block or _has_any_global_hook() or not _stock(self) or ops.is_tracing():   # (a trace records operators)
             return False
         pam = self.pam
         if pam.head_dim != 64 or pam.num_heads > 64 or not pam.fused_qkv or pam.qk_norm or pam.dim % 4 or pam.dim > 768 or not pam._fused_gates_ok(x):

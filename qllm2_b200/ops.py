@@ -1,4 +1,4 @@
-"""torch-facing wrappers of the C ABI: autograd functions over raw device pointers.
+"""torch-facing wrappers of the C ABI: the scan through its native nodes (csrc/host), the rest over raw device pointers.
 
 torch is used here for what it is good at on this path -- owning device memory, the current
 stream and autograd bookkeeping.  All arithmetic happens in libqllm2_pam_b200.so.
@@ -50,8 +50,12 @@ class _Recorded(torch.autograd.Function):
 
 
 def recorded(call, *tensors):
-    """call(*tensors), recorded where a trace is being taken."""
-    return _Recorded.apply(call, *tensors) if torch.jit.is_tracing() else call(*tensors)
+    """call(*tensors) as one operator of the trace that is being taken."""
+    return _Recorded.apply(call, *tensors)
+
+
+#: torch.jit.is_tracing without its Python frames: asked at every call
+is_tracing = torch._C._is_tracing
 
 
 # --------------------------------------------------------------------------------------- scan
@@ -80,22 +84,22 @@ def pam_scan(q, k, v, gamma, *, coef=None, s0=None, cu_seqlens=None, head_dim: O
     s0       optional [K,S,H,d,d,2] initial state;  cu_seqlens optional int32 [S+1] (then B == 1)
     Returns (y [B,H,T,d,2] in q's dtype, s_final float32 [K,S,H,d,d,2]).
 
-    Checks, autograd node and launches are native (csrc/host/scan.cpp).  K > 1 states in bf16 at d = 64 with gradients:
+    Checks, autograd node and launches are native (csrc/host/scan.cpp).  K = 2..4 states in bf16 at d = 64:
     y = sum_k c_k y^(k), where y^(k) is the single-state scan with decay gamma^(k) on the same q, k, v (the fused K-state form
-    of the reference, v11/model.py:657-781, is algebraically this sum), as one node whose backward accumulates dq, dk, dv of
-    the states in place.
+    of the reference, v11/model.py:657-781, is algebraically this sum), through the fused K-state kernels, forward and backward.
+    Without read-out weights (coef) and with gradients: one output kernel per state, whose dq, dk, dv the backward accumulates
+    in place.  save_states=False with gradients, or more states than four: one single-state scan per state.
     """
-    def native(q, k, v, gamma, coef, s0, cu):
-        return _lib.host().pam_scan(q, k, v, gamma, coef, s0, cu, head_dim or 0, eps, chunk, save_states, token_major)
-
-    if not torch.jit.is_tracing():
-        y, s = native(q, k, v, gamma, coef, s0, cu_seqlens)
+    if not is_tracing():
+        y, s = _lib.host().pam_scan(q, k, v, gamma, coef, s0, cu_seqlens, head_dim or 0, eps, chunk, save_states, token_major)
     else:
         if torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16:
             q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()       # what autocast decides belongs to the trace, not to its replay
         each = (gamma.dim() == 4 and gamma.shape[0] > 1 and (not save_states or gamma.shape[0] > _lib.MAX_STATES) and q.dtype == torch.bfloat16 and
                 q.shape[3] == 64 and torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (q, k, v, gamma, coef, s0)))
-        y, s = (None, None) if each else _Recorded.apply(native, q, k, v, gamma, coef, s0, cu_seqlens)
+        y, s = (None, None) if each else recorded(
+            lambda q, k, v, gamma, coef, s0, cu: _lib.host().pam_scan(q, k, v, gamma, coef, s0, cu, head_dim or 0, eps, chunk, save_states, token_major),
+            q, k, v, gamma, coef, s0, cu_seqlens)
     if y is not None:
         return y, s
     # K tensor-core states recomputed in the backward, or more of them than the fused kernels take: one scan per state, autograd
@@ -159,6 +163,8 @@ def pam_scan_tokens(q, k, v, gamma, coef=None, s0=None, cu_seqlens=None, *, head
     """Inference form of `pam_scan`: same arguments, but Y comes back token-major, [B, T, H*d, 2] -- the layout
     the output projection reads (the head merge of v11/model.py:835-836) -- and nothing is kept for a backward
     pass (K phase-routed states in bf16 at d = 64 then run the fused K-state output kernel)."""
+    if not is_tracing():
+        return _lib.host().pam_scan_tokens(q, k, v, gamma, coef, s0, cu_seqlens, head_dim or 0, eps, chunk)
     return recorded(lambda q, k, v, gamma, coef, s0, cu: _lib.host().pam_scan_tokens(q, k, v, gamma, coef, s0, cu, head_dim or 0, eps, chunk),
                     q, k, v, gamma, coef, s0, cu_seqlens)
 
