@@ -159,8 +159,10 @@ struct Inputs {
 
 Inputs checked(Tensor q, Tensor k, Tensor v, Tensor gamma, const OptTensor& coef_, const OptTensor& s0_, const OptTensor& cu_, int64_t head_dim) {
   // (a call without reverse-mode gradients runs without a node, which would have refused these)
-  for (const Tensor& t : {q, k, v, gamma, value(coef_), value(s0_)})
-    QH_REQUIRE(!t.defined() || !t._fw_grad(0).defined(), "the scan has no forward-mode derivative");
+  const auto has_tangent = [](const Tensor& t) { return t.defined() && t._fw_grad(0).defined(); };
+  bool tangent = (coef_.has_value() && has_tangent(*coef_)) || (s0_.has_value() && has_tangent(*s0_));
+  for (const Tensor* t : {&q, &k, &v, &gamma}) tangent = tangent || has_tangent(*t);
+  QH_REQUIRE(!tangent, "the scan has no forward-mode derivative");
   // one dtype for the token tensors: under bf16 autocast the reference's matmuls round their inputs to bf16 anyway, so mixed
   // fp32 / bf16 operands (RoPE promotes q and k to fp32) are taken as bf16; otherwise they are promoted to the widest
   // dtype present.  The C ABI reads all three through q's dtype, so they must agree before the pointers are handed over.
