@@ -88,8 +88,9 @@ size_t qpam_scan_workspace_bytes(const qpam_scan_args* args, int32_t with_backwa
 int qpam_scan_fwd(const qpam_scan_args* args, void* stream);
 
 /* qpam_scan_fwd with y written token-major, [B,T,H,d,2] (packed mode: [T_total,H,d,2]): the head merge
- * that precedes the output projection (v11/model.py:835-836) without a transpose pass.  Forward only;
- * available where the tensor-core kernels run (bf16, d = 64), QPAM_EUNSUPPORTED otherwise. */
+ * that precedes the output projection (v11/model.py:835-836) without a transpose pass.  A backward may follow as after
+ * qpam_scan_fwd (2..4 states take its output gradient in the same layout, qpam_scan_bwd_tokens).
+ * Available where the tensor-core kernels run (bf16, d = 64), QPAM_EUNSUPPORTED otherwise. */
 int qpam_scan_fwd_tokens(const qpam_scan_args* args, void* stream);
 
 /* qpam_scan_fwd_tokens followed by qpam_pool_store of the final states, in one call and without the fp32 states in
