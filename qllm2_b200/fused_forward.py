@@ -271,7 +271,7 @@ class FusedForward:
         er, ei = emb.embed_real.weight, emb.embed_imag.weight
         a.embed_real, a.embed_imag, a.w_head, a.b_head, a.w_vocab = ptr(er), ptr(ei), ptr(self.w_head_proj), ptr(self.b_head_proj), ptr(self.w_vocab)
         a.embed_scale, a.out_scale, a.head_norm_scale, a.rope = ptr(self.embed_scale), ptr(self.out_scale), ptr(self.head_norm_scale), ptr(self.rope)
-        ids, positions = ids.reshape(-1).contiguous(), positions.reshape(-1).to(torch.int64).contiguous()
+        ids, positions, slots = ids.reshape(-1).contiguous(), positions.reshape(-1).to(torch.int64).contiguous(), slots.contiguous()
         a.ids, a.positions, a.slot_ids, a.pool = ptr(ids), ptr(positions), ptr(slots), ptr(pool)
         if slots.dtype != torch.int32 or slots.numel() != n or positions.numel() != n or ids.dtype != torch.int64:
             raise _lib.QPamError("step: ids / positions int64 [n] and slots int32 [n] expected")

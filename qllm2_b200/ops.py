@@ -241,6 +241,7 @@ def ce_row_stats(h, w, targets, *, ignore_index=-100, v_offset=0):
         raise _lib.QPamError(f"h [N,F] and w [V,F] expected; got {tuple(h.shape)}, {tuple(w.shape)}")
     if targets is not None and (targets.dtype != torch.int64 or targets.numel() != h.shape[0]):
         raise _lib.QPamError("targets must be int64 with one entry per row of h")
+    targets = None if targets is None else targets.contiguous()
     N = h.shape[0]
     f32 = dict(dtype=torch.float32, device=h.device)
     row_max, row_sum, row_tgt = torch.empty(N, **f32), torch.empty(N, **f32), torch.empty(N, **f32)
@@ -342,6 +343,11 @@ def sample_logits(logits, uniforms=None, *, temperature: float = 1.0, top_k: int
         raise _lib.QPamError("sample_logits: slot_ids must be int32 [n] on the device")
     if append and (history is None or hist_len is None):
         raise _lib.QPamError("sample_logits: append needs history and hist_len")
+    if append and not hist_len.is_contiguous():
+        raise _lib.QPamError("sample_logits: append advances hist_len in place, so it must be contiguous")
+    uniforms = uniforms.contiguous()
+    slot_ids = None if slot_ids is None else slot_ids.contiguous()
+    hist_len = None if hist_len is None else hist_len.contiguous()
     ids = torch.empty(n, dtype=torch.int64, device=dev)
     stats = torch.empty(n, 4, dtype=torch.float32, device=dev) if return_stats else None
     need = L.qpam_sample_workspace_bytes(n, V)

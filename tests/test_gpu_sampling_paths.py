@@ -5,7 +5,7 @@ import threading
 import pytest
 import torch
 
-from qllm2_b200 import ops
+from qllm2_b200 import _lib, ops
 from tests.test_gpu_sampling import _check_rows
 
 pytestmark = pytest.mark.gpu
@@ -37,6 +37,22 @@ def test_ties_beyond_the_list(top_k, top_p):
     ids, stats = ops.sample_logits(logits, u.to(DEV), return_stats=True, **cfg)
     _check_rows(logits, None, None, u.numpy(), ids.cpu().numpy(), stats.cpu().numpy(), cfg)
     assert stats[:, 2].tolist() == (logits == 1).sum(1).tolist()
+
+
+def test_strided_vectors():
+    """Uniforms, slots and lengths as columns of wider tensors mean what their values say."""
+    n, V = 5, 997
+    g = torch.Generator().manual_seed(8)
+    logits = (torch.randn(n, V, generator=g) * 3).to(DEV)
+    wide = lambda t: torch.stack([t, torch.zeros_like(t)], dim=1).to(DEV)[:, 0]
+    u, slots = torch.rand(n, generator=g), torch.tensor([4, 0, 2, 1, 3], dtype=torch.int32)
+    lens, hist = torch.tensor([3, 7, 1, 5, 9], dtype=torch.int32), torch.randint(0, V, (n, 12), generator=g)
+    cfg = dict(history=hist.to(DEV), top_p=0.9, repetition_penalty=1.5)
+    want = ops.sample_logits(logits, u.to(DEV), slot_ids=slots.to(DEV), hist_len=lens.to(DEV), **cfg)
+    got = ops.sample_logits(logits, wide(u), slot_ids=wide(slots), hist_len=wide(lens), **cfg)
+    assert torch.equal(got, want)
+    with pytest.raises(_lib.QPamError):
+        ops.sample_logits(logits, u.to(DEV), hist_len=wide(lens), append=True, **cfg)
 
 
 def test_threads_with_vocabularies_of_different_size():
