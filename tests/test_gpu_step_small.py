@@ -1,5 +1,5 @@
 """The decode step for few rows (qpam_step_fwd) against the block-by-block packed forward it replaces there, at the edges of
-its dispatch: rows around the fused-norm limit and the groups of four, split and unsplit projections, every gate source."""
+its dispatch: rows around the one-kernel limit (4) and the groups of four and eight, split and unsplit projections, every gate source."""
 import pytest
 import torch
 
