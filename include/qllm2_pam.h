@@ -158,7 +158,7 @@ int qpam_scan_bwd_state(const qpam_scan_args* args, int32_t state, const void* d
  * (note: gamma is used as is, without gamma_eps, exactly as the reference's recurrent path).
  *
  * state_pool: [n_slots, L, K, H, d, d, 2] (state_dtype); the step updates, in place, layer
- * `layer` of the slots named by slot_ids[n].  q (already scaled by d^-0.5), k, v, y: [n,H,d,2]
+ * `layer` of the slots named by slot_ids[n] (outside [0, n_slots): no state, y = 0).  q (already scaled by d^-0.5), k, v, y: [n,H,d,2]
  * io_dtype.  gamma fp32 [K,n,H]; coef fp32 [K,n,H,2] or NULL.
  * ------------------------------------------------------------------------------------------ */
 int qpam_decode_step(void* state_pool, int32_t state_dtype, int64_t n_slots, int32_t L, int32_t layer,

@@ -66,8 +66,11 @@ __global__ void __launch_bounds__(256) k_decode_step(DecodeParams p) {
   const int tid = threadIdx.x;
   const int seq = blockIdx.x / p.H, h = blockIdx.x - seq * p.H;
   const int slot = p.slot_ids[seq];
-  if (slot < 0 || slot >= p.n_slots) return;  // padded / retired entry: nothing to do
   const size_t vb = ((size_t)seq * p.H + h) * D * 2;
+  if (slot < 0 || slot >= p.n_slots) {        // padded / retired entry: no state, but a defined output (see k_decode_step_bulk)
+    for (int i = tid; i < D; i += NTH) IO<T>::st2(reinterpret_cast<T*>(p.y) + vb + 2 * i, make_float2(0.f, 0.f));
+    return;
+  }
   if (tid < D) {
     sq[tid] = IO<T>::ld2(reinterpret_cast<const T*>(p.q) + vb + 2 * tid);
     sk[tid] = IO<T>::ld2(reinterpret_cast<const T*>(p.k) + vb + 2 * tid);
@@ -153,7 +156,11 @@ __global__ void __launch_bounds__(256) k_decode_step_bulk(DecodeParams p) {
   const int tid = threadIdx.x;
   const int seq = blockIdx.x / p.H, h = blockIdx.x - seq * p.H;
   const int slot = p.slot_ids[seq];
-  if (slot < 0 || slot >= p.n_slots) return;  // padded / retired entry: nothing to do (whole CTA)
+  const size_t vb = ((size_t)seq * p.H + h) * D * 2;
+  if (slot < 0 || slot >= p.n_slots) {        // padded / retired entry (whole CTA): no state, but a defined output -- the row goes on
+    if (tid < D) IO<T>::st2(reinterpret_cast<T*>(p.y) + vb + 2 * tid, make_float2(0.f, 0.f));      // through the step to an id
+    return;
+  }
   __nv_bfloat16* pool = reinterpret_cast<__nv_bfloat16*>(p.pool);
   const size_t state_elems = (size_t)D * D * 2;
   const size_t base = (((size_t)slot * p.L + p.layer) * p.K) * p.H + h;  // + k * H per state
@@ -166,7 +173,6 @@ __global__ void __launch_bounds__(256) k_decode_step_bulk(DecodeParams p) {
                 DEC_BULK_STATE_BYTES, &bar[k]);
     }
   }
-  const size_t vb = ((size_t)seq * p.H + h) * D * 2;
   if (tid < D) {
     sq[tid] = IO<T>::ld2(reinterpret_cast<const T*>(p.q) + vb + 2 * tid);
     sk[tid] = IO<T>::ld2(reinterpret_cast<const T*>(p.k) + vb + 2 * tid);
