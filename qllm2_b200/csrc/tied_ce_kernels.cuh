@@ -189,7 +189,8 @@ __global__ void k_ce_merge(CEParams p, float* row_max, float* row_sumexp, float*
   if (row_max) row_max[n] = M;
   if (row_sumexp) row_sumexp[n] = S;
   if (row_tgt) row_tgt[n] = tz;
-  if (row_argmax) row_argmax[n] = (int64_t)bi + p.v_offset;
+  // (a row without a comparable logit, all NaN or -inf, has no arg-max: the first column, so that the id can be embedded)
+  if (row_argmax) row_argmax[n] = (bi == 0x7fffffff ? 0 : (int64_t)bi) + p.v_offset;
 }
 
 // Single CTA: lse, per-token loss and the scalar reductions (fixed summation order, double).

@@ -44,3 +44,18 @@ def test_captured_steps_feed_ids_of_the_vocabulary():
         if graph:
             assert int(eng._g_ids.min()) >= 0 and int(eng._g_ids.max()) < 101 and torch.isfinite(eng.pool.float()).all()
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("dtype,N,F,V", [(torch.float32, 9, 32, 101), (torch.bfloat16, 9, 64, 1003), (torch.bfloat16, 300, 64, 1003)])
+def test_arg_max_of_rows_without_a_number(dtype, N, F, V):
+    """A row of NaN has no arg-max; its id is one of the vocabulary all the same, and the other rows' are what they were."""
+    g = torch.Generator(device=DEV).manual_seed(V)
+    h, w = torch.randn(N, F, device=DEV, generator=g).to(dtype), torch.randn(V, F, device=DEV, generator=g).to(dtype)
+    want, _ = ops.head_argmax(h, w)
+    bad = h.clone()
+    bad[::4] = float("nan")
+    ids, _ = ops.head_argmax(bad, w)
+    assert int(ids.min()) >= 0 and int(ids.max()) < V
+    keep = torch.ones(N, dtype=torch.bool, device=DEV)
+    keep[::4] = False
+    assert torch.equal(ids[keep], want[keep])
