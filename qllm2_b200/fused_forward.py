@@ -26,7 +26,7 @@ from torch.nn.modules.module import _has_any_global_hook
 from . import _lib, ops
 from ._lib import check, dtype_code, ptr, stream_ptr
 from .fused_elementwise import _dense
-from .model import ModSwish, V11LM, build_rope_cache
+from .model import ModSwish, V11LM, _stock_operators, build_rope_cache
 
 
 def _f32(t: torch.Tensor) -> torch.Tensor:
@@ -77,6 +77,8 @@ class FusedForward:
             return "head_dim must be a power of two in [4,128] and n_heads <= 64"
         if cfg.dim % 4 or (cfg.dim * cfg.expand) % 4:
             return "dim and dim*expand must be multiples of 4"
+        if not _stock_operators(model):
+            return "operators of the model were replaced or have hooks: they are called as modules"
         p = next(model.parameters())
         if not p.is_cuda or p.dtype not in (torch.float32, torch.bfloat16):
             return "needs a CUDA model in float32 or bfloat16"

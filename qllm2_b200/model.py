@@ -495,16 +495,17 @@ class V11PAMLayer(nn.Module):
 
 
 # ------------------------------------------------------------------------------------ block / LM
-def _stock(module) -> bool:
+def _stock(module, dtype=None) -> bool:
     """Whether a module of one of these classes, and every operator below it, is as this file builds it: exactly the class,
-    forward not replaced on the instance, no hooks (the module itself is being called: its own have run), fp32 parameters.
+    forward not replaced on the instance, no hooks (the module itself is being called: its own have run), parameters of
+    `dtype` if one is given.
     (Asked at every call of every block: a walk over the plain dictionaries, where modules() and parameters() take 40 us.)"""
     cls = type(module)
     for name, p in module._parameters.items():
         if p is None:
             if cls is nn.Linear:                            # the kernels read its bias
                 return False
-        elif p.dtype is not torch.float32 or (cls is ComplexLinear and name[0] == "b"):   # these projections have none
+        elif (dtype is not None and p.dtype is not dtype) or (cls is ComplexLinear and name[0] == "b"):   # these projections have none
             return False
     if cls is ComplexNorm and module.eps != 1e-6:
         return False
@@ -515,9 +516,17 @@ def _stock(module) -> bool:
             continue
         if type(m) not in classes or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__:
             return False
-        if not _stock(m):
+        if not _stock(m, dtype):
             return False
     return True
+
+
+def _stock_operators(model) -> bool:
+    """Whether the packed inference forward computes what the model's modules would: stock blocks, norms and head projection."""
+    rest = [(model.embed_norm, ComplexNorm), (model.output_norm, ComplexNorm), (model.lm_head_norm, ComplexNorm), (model.lm_head_proj, ComplexLinear)]
+    if _has_any_global_hook() or any(type(m) is not cls or m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ for m, cls in rest):
+        return False
+    return all(m.eps == 1e-6 for m, cls in rest if cls is ComplexNorm) and all(type(b) is V11Block and _stock(b) for b in model.blocks)
 
 
 class V11Block(nn.Module):
@@ -539,7 +548,7 @@ class V11Block(nn.Module):
         if (pam_state is not None or not x.is_cuda or x.dtype != torch.bfloat16 or x.shape[1] < 2 or not torch.is_autocast_enabled("cuda")
                 or torch.get_autocast_dtype("cuda") != torch.bfloat16):
             return False
-        if type(self) is not V11Block or _has_any_global_hook() or not _stock(self) or ops.is_tracing():   # (a trace records operators)
+        if type(self) is not V11Block or _has_any_global_hook() or not _stock(self, torch.float32) or ops.is_tracing():   # (a trace records operators)
             return False
         pam = self.pam
         if pam.head_dim != 64 or pam.num_heads > 64 or not pam.fused_qkv or pam.qk_norm or pam.dim % 4 or pam.dim > 768 or not pam._fused_gates_ok(x):

@@ -5,6 +5,8 @@ import torch.nn as nn
 
 from qllm2_b200 import _lib
 from qllm2_b200 import model as M
+from qllm2_b200.fused_forward import FusedForward
+from qllm2_b200.serving import ContinuousBatcher
 
 
 def _block(**kw):
@@ -52,14 +54,37 @@ CHANGES = {
 
 def test_stock_blocks_are_recognised():
     for kw in (dict(), dict(n_states=1, use_gsp=False), dict(activation="modrelu", state_compete=False)):
-        assert M._stock(_block(**kw))
+        assert M._stock(_block(**kw), torch.float32)
 
 
 @pytest.mark.parametrize("change", CHANGES)
 def test_changed_blocks_keep_their_operators(change):
     blk = _block()
     CHANGES[change](blk)
-    assert not M._stock(blk)
+    assert not M._stock(blk, torch.float32)
+    assert M._stock(blk) == (change == "bf16 parameter")         # inference takes weights of any type
+
+
+def _net():
+    torch.manual_seed(3)
+    return M.V11LM(M.V11Config(vocab_size=64, dim=64, n_heads=1, head_dim=64, n_layers=2, dropout=0.0, gradient_checkpointing=False, max_seq_len=64))
+
+
+NET_CHANGES = {
+    "adapter": lambda n: _swap(n.blocks[1].cgu, "up_proj", _Adapter(64, 192, bias=False)),
+    "block subclass": lambda n: setattr(n.blocks[0], "__class__", _OtherBlock),
+    "hook": lambda n: n.blocks[1].pam.dt_proj.register_forward_hook(lambda *a: None),
+    "head epsilon": lambda n: setattr(n.lm_head_norm, "eps", 1e-5),
+    "head hook": lambda n: n.lm_head_proj.register_forward_hook(lambda *a: None),
+}
+
+
+@pytest.mark.parametrize("change", NET_CHANGES)
+def test_changed_models_are_not_packed(change):
+    net = _net()
+    assert M._stock_operators(net) and "CUDA" in FusedForward.unsupported_reason(net)
+    NET_CHANGES[change](net)
+    assert "called as modules" in FusedForward.unsupported_reason(net)
 
 
 def _x(D=64, T=40):
@@ -150,3 +175,22 @@ def test_native_node_does_not_bypass(case):
         blk.norm1.register_forward_hook(lambda *a: None)           # the operators, in any case
         want, _ = blk(x)
     assert torch.equal(y, want)
+
+
+@pytest.mark.gpu
+def test_adapters_take_part_in_generation_and_serving():
+    """A projection with a term of its own: its tokens are those of the module-by-module loop, not of the packed weights."""
+    net = _net().cuda().eval()
+    with torch.no_grad():
+        for p in net.parameters():
+            p.add_(torch.randn(p.shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(p.numel())) * 0.2)
+    ids = torch.randint(0, 64, (2, 9), device="cuda", generator=torch.Generator(device="cuda").manual_seed(5))
+    plain = net.generate(ids, 12, temperature=0)
+    NET_CHANGES["adapter"](net)
+    net.cuda()
+    got = net.generate(ids, 12, temperature=0)
+    assert torch.equal(got, net.generate(ids, 12, temperature=0, fused=False)) and not torch.equal(got, plain)
+    eng = ContinuousBatcher(net, n_slots=2, max_position=64)
+    rids = [eng.submit(row, 12) for row in ids.tolist()]
+    done = eng.run()
+    assert [done[r] for r in rids] == got[:, 9:].tolist()
