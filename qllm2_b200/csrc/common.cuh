@@ -46,6 +46,47 @@ bool profiling_active();
 // every launch site names its stream `st`
 #define QPAM_LAUNCH_CHECK(name) QPAM_LAUNCH_CHECK_ON(name, st)
 
+// ------------------------------------------------------------------ kernels that follow one another on a stream
+// Programmatic dependent launch: a kernel launched with launch_after() may have its first CTAs started once every CTA of its
+// predecessor has called pdl_trigger() (or has ended), so that a launch's start and the part of it that needs nothing from the
+// predecessor run in the predecessor's last wave.  What every such kernel keeps to:
+//   * pdl_wait() in every thread, before the first access to anything the predecessor writes (or still reads) and before any
+//     return: it returns when the predecessor has completed, which has waited for its own in turn;
+//   * the first kernel of a call waits at its very start and triggers only afterwards.  All its inputs have been written by
+//     then, so the kernels behind it may read the call's inputs (not its intermediate results) before their own wait;
+//   * tensor memory is allocated before the trigger: a CTA of the successor that holds columns while it waits can then not
+//     keep them from a CTA it waits for.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// 16 bytes that a predecessor may write while this kernel has begun already (behind pdl_wait): an ordinary load, not the
+// read-only path the compiler could choose.
+__device__ __forceinline__ float4 ld_dependent(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));      // (no memory clobber: loads may be batched ahead of
+  return v;                                                                                       // stores; volatile keeps them behind the wait)
+}
+
+// `first`: an ordinary launch, for a kernel that begins a call and reads its inputs without waiting.
+template <typename... Params, typename... Args>
+static inline void launch_kernel(bool first, void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = first ? 0 : 1;
+  cudaLaunchKernelEx(&cfg, kern, args...);      // (an error is found by the QPAM_LAUNCH_CHECK behind every launch)
+}
+template <typename... Params, typename... Args>
+static inline void launch_after(void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+  launch_kernel(false, kern, grid, threads, smem, st, args...);
+}
+
 // ------------------------------------------------------------------ io element access
 template <typename T>
 struct IO;

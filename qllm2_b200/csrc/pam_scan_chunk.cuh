@@ -29,7 +29,7 @@ __device__ __forceinline__ void load_state(float2* dst, const float2* __restrict
   constexpr int LD = D + 1;
   for (int e = tid; e < D * D; e += NT) {
     const int i = e / D, j = e - i * D;
-    dst[i * LD + j] = src[e];
+    dst[i * LD + j] = __ldcg(src + e);      // (not the read-only path: see ld_dependent)
   }
 }
 
@@ -54,8 +54,12 @@ __global__ void __launch_bounds__(NT) k_fwd_chunk(ScanParams p) {
   float* A = reinterpret_cast<float*>(X + CH * XS);           // [KMAX][CH]
   float2* cf = reinterpret_cast<float2*>(A + KMAX * CH);      // [KMAX][CH]
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  pdl_trigger();
   const ChunkLoc L = locate_chunk(p.geom, blockIdx.x);
-  if (!L.valid) return;
+  if (!L.valid) {
+    pdl_wait();
+    return;
+  }
   const int h = blockIdx.y;
   load_decay_coef(p, L, h, A, cf, tid);
   const size_t tb = token_base(p, L.b, h, L.t0, D);
@@ -87,6 +91,7 @@ __global__ void __launch_bounds__(NT) k_fwd_chunk(ScanParams p) {
   float2 acc[4][RD];
   czero(acc);
   cgemm<4, RD, false, false>(acc, X, XS, 1, Vs, 1, LD, CH, ty, tx);
+  pdl_wait();          // the carried states are the predecessor's; everything above is the call's inputs
   if (L.c > 0 || p.s0 != nullptr) {
     for (int k = 0; k < p.K; ++k) {
       __syncthreads();
@@ -161,8 +166,12 @@ __global__ void __launch_bounds__(NT) k_bwd_chunk(ScanParams p) {
   float* col = reinterpret_cast<float*>(dcI + KMAX * CH);
   float* colp = col + KMAX * CH;  // [8 warps][KMAX][CH]
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, warp = tid >> 5, lane = tid & 31;
+  pdl_trigger();
   const ChunkLoc L = locate_chunk(p.geom, blockIdx.x);
-  if (!L.valid) return;
+  if (!L.valid) {
+    pdl_wait();
+    return;
+  }
   const int h = blockIdx.y;
   load_decay_coef(p, L, h, A, cf, tid);
   const size_t tb = token_base(p, L.b, h, L.t0, D);
@@ -239,7 +248,8 @@ __global__ void __launch_bounds__(NT) k_bwd_chunk(ScanParams p) {
   cgemm<4, RD, false, false>(aQ, Z, XS, 1, Ks, 1, LD, CH, ty, tx);
   cgemm<4, RD, true, false>(aK, Z, 1, XS, Qs, 1, LD, CH, ty, tx);
 
-  // ---- inter-chunk terms through the carried state and its gradient
+  // ---- inter-chunk terms through the carried state and its gradient (the predecessor's; everything above is the call's inputs)
+  pdl_wait();
   const bool has_prev = (L.c > 0) || (p.s0 != nullptr);
   const bool has_next = (L.c < L.nc - 1) || (p.ds_final != nullptr);
   for (int k = 0; k < p.K; ++k) {
@@ -355,6 +365,8 @@ __global__ void __launch_bounds__(NT) k_bwd_chunk(ScanParams p) {
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_dgamma_finalize(ScanParams p, int D) {
   __shared__ double wsum[8];
+  pdl_trigger();
+  pdl_wait();
   const int seq = blockIdx.x, h = blockIdx.y, k = blockIdx.z;
   int b = seq, a = 0, e = p.T;
   int64_t slot_last;

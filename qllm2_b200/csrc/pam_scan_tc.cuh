@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr bool CARRY = MODE == OUTER_CARRY;
+  pdl_wait();
   int h;
   const ChunkLoc L = take_job<CARRY>(p, tmem_slot + 1, h);
   if (!L.valid) return;
@@ -232,6 +233,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
   if (warp == 1) warp_cumsum128_finish(Acum, graw, L.len, p.eps, lane);
   tc_fence_before();
   __syncthreads();
+  pdl_trigger();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const float a_last = Acum[TC - 1];
@@ -361,6 +363,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
   uint64_t* bar = reinterpret_cast<uint64_t*>(wrow + KMAX * TC);  // one per state, [KMAX]: the token tiles
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + KMAX + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_wait();
   const ChunkLoc L = locate_chunk(p.geom, blockIdx.x);
   if (!L.valid) return;
   const int h = blockIdx.y;
@@ -385,6 +388,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
   if (warp >= 1 && warp <= K) warp_cumsum128_finish(Acum + (warp - 1) * TC, graw, L.len, p.eps, lane);
   tc_fence_before();
   __syncthreads();
+  pdl_trigger();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   if (DSTATE) {

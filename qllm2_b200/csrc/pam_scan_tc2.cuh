@@ -313,8 +313,12 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
   int* failed = reinterpret_cast<int*>(tmem_slot + 1);      // error word as found at the start of this CTA
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // (chunk_prefix, read here, is older than the predecessor: see launch_after)
   const ChunkLoc L = locate_chunk(p.geom, chunk_x);
-  if (!L.valid) return;
+  if (!L.valid) {
+    pdl_wait();
+    return;
+  }
   if (tid == 64) *failed = device_error_now();     // not on warp 1: its cumulative decay is the prologue's critical path
   const bool has_state = LOWER ? ((L.c > 0) || (p.s0 != nullptr)) : ((L.c < L.nc - 1) || (p.ds_final != nullptr));
   const int row0 = (L.b * p.H + h) * p.T + L.t0;
@@ -340,8 +344,10 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem = *tmem_slot;
   if (*failed != 0) {
+    pdl_wait();
     // an earlier launch gave up on a wait: leave the outputs alone (the tiles still land; wait for them so that no
     // bulk copy is in flight into this CTA's shared memory when it exits)
     mbar_wait(&bars[0], 0, 225);
@@ -386,6 +392,9 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
   __syncwarp();
   ok = mbar_wait(&bars[1], 0, 222) && ok;
   tc_fence_after();
+  // the tiles, their scores and the decays are the call's inputs; the carried states (and, backward, the buffer of dA_k) are
+  // the predecessor's
+  pdl_wait();
   if (has_state && tid == 0) {
     // stage 1 has released the B1 region: the carried state (fp32, 32 KB, contiguous) comes into it by one bulk copy
     // while epilogue 1 runs
@@ -575,6 +584,8 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_bwd(const __grid_constant__
 // grid = (S, H, 8 K), 256 threads: every thread owns one float4 (two complex entries) of the state.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_tc_state_scan_rev(ScanParams p, float* __restrict__ anchor_parts) {
+  pdl_trigger();
+  pdl_wait();
   const int seq = blockIdx.x, h = blockIdx.y, k = blockIdx.z >> 3, z = blockIdx.z & 7;
   const int e4 = z * 256 + threadIdx.x;
   constexpr int n4 = TD * TD / 2;
@@ -640,6 +651,8 @@ __global__ void __launch_bounds__(256) k_tc_state_scan_rev(ScanParams p, float* 
 __global__ void __launch_bounds__(128) k_tc_dgamma_finalize(ScanParams p, const float* __restrict__ anchor_parts) {
   __shared__ float wsum[4];
   __shared__ float anc[2];
+  pdl_trigger();
+  pdl_wait();
   const ChunkLoc L = locate_chunk(p.geom, blockIdx.x);
   if (!L.valid) return;
   const int h = blockIdx.y;
@@ -650,7 +663,7 @@ __global__ void __launch_bounds__(128) k_tc_dgamma_finalize(ScanParams p, const 
     if (tid < 2) anc[tid] = 0.f;
   } else if (warp < 2) {      // warp 0: anchor at the chunk's first token, warp 1: just after the chunk
     const float* ap = anchor_parts + ((size_t)h * p.nslots + L.slot0 + L.c + warp) * ANCHOR_PARTS;
-    double a = (double)ap[lane] + (double)ap[lane + 32];
+    double a = (double)__ldcg(ap + lane) + (double)__ldcg(ap + lane + 32);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     if (lane == 0) anc[warp] = (float)a;

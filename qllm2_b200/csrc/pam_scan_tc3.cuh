@@ -42,7 +42,10 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   int* failed = reinterpret_cast<int*>(tmem_slot + 1);      // error word as found at the start of this CTA
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const ChunkLoc L = locate_chunk(p.geom, blockIdx.x);
-  if (!L.valid) return;
+  if (!L.valid) {
+    pdl_wait();
+    return;
+  }
   if (tid == 160) *failed = device_error_now();
   const int h = blockIdx.y;
   const int K = p.K;
@@ -76,8 +79,10 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem = *tmem_slot;
   if (*failed != 0) {       // an earlier launch gave up on a wait: outputs stay untouched (see pam_scan_tc2.cuh)
+    pdl_wait();
     mbar_wait(&bars[0], 0, 239);
     __syncthreads();
     if (warp == 0) tmem_dealloc<256>(tmem);
@@ -139,6 +144,7 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   __syncwarp();
   ok = mbar_wait(&bars[1], 0, 232) && ok;
   tc_fence_after();
+  pdl_wait();          // the carried states below are the predecessor's; everything above is the call's inputs
   const int q4 = warp & 3, hf = warp >> 2;
   const int r = q4 * 32 + lane;                               // this thread's row (TMEM lane)
   const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);
@@ -151,10 +157,13 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
     const float cst = ((strong_mask >> k) & 1u) ? 1.f : __expf(Acum[k * TC + TC / 2 - 1]);
     const float4* sg = reinterpret_cast<const float4*>(p.states + state_base(p, k, h, L.slot0 + L.c, TD));
     unsigned char* dstp = RB + s * 16384;
+    float4 v[8];                               // all of them requested before the first is used
+#pragma unroll
+    for (int it = 0; it < 8; ++it) v[it] = ld_dependent(sg + (tid + 256 * (it >> 1)) * 2 + (it & 1));
 #pragma unroll
     for (int it = 0; it < 4; ++it) {
       const int idx = tid + 256 * it;          // (i, c16): state[i][4*c16 .. +3]
-      const float4 s01 = __ldg(sg + idx * 2), s23 = __ldg(sg + idx * 2 + 1);
+      const float4 s01 = v[2 * it], s23 = v[2 * it + 1];
       const int i = idx >> 4, c16 = idx & 15;
       const uint32_t off = sw128(i, c16 >> 1) + (c16 & 1) * 8;
       *reinterpret_cast<uint2*>(dstp + off) = make_uint2(pack_bf162(cst * s01.x, cst * s01.z), pack_bf162(cst * s23.x, cst * s23.z));

@@ -190,7 +190,7 @@ __device__ __forceinline__ void stage_state(unsigned char* slot, const float2* _
   const float4* sg = reinterpret_cast<const float4*>(state);
   float4 v[4];
 #pragma unroll
-  for (int it = 0; it < 4; ++it) v[it] = __ldg(sg + tid + BT * it);
+  for (int it = 0; it < 4; ++it) v[it] = ld_dependent(sg + tid + BT * it);
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
     const int i = (tid + BT * it) >> 5, c = tid & 31;      // row i, columns 2c and 2c + 1
@@ -259,7 +259,10 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   float* anc = wsum + 4 * KMAX;                                     // [K][2]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const ChunkLoc L = locate_chunk(p.geom, blockIdx.x);
-  if (!L.valid) return;
+  if (!L.valid) {
+    pdl_wait();
+    return;
+  }
   const int h = blockIdx.y, len = L.len;
   const bool has_s = L.c > 0 || p.s0 != nullptr, has_ds = L.c < L.nc - 1 || p.ds_final != nullptr;
   const int row0 = (L.b * p.H + h) * p.T + L.t0;
@@ -289,25 +292,21 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   const size_t eg = gamma_base(p, ek, L.b, h, L.t0 + et);
   float2 c_e = make_float2(1.f, 0.f);
   if (p.coef != nullptr && ek < K && et < len) c_e = __ldg(reinterpret_cast<const float2*>(p.coef + eg * 2));
-  // what the decay gradient needs at the end, requested now: the decay of this thread's token, and per state the partial
-  // sums of the anchors at the chunk's first token and just after the chunk (two warps of the state's four)
+  // what the decay gradient needs at the end, requested as soon as it may be: the decay of this thread's token, and (further
+  // down, they are the predecessor's) per state the partial sums of the anchors at the chunk's first token and just after the
+  // chunk (two warps of the state's four)
   const int et_rev = TC - 1 - et;
   float g_e = 1.f, an0 = 0.f, an1 = 0.f;
-  if (ek < K) {
-    if (et_rev < len) g_e = __ldg(p.gamma + eg - et + et_rev);
-    if ((warp & 3) < 2 && anchor_parts != nullptr) {      // (null: zero, see scan_bwd_tc)
-      const float* ap = anchor_parts + (((size_t)ek * p.H + h) * p.nslots + L.slot0 + L.c + (warp & 3)) * ANCHOR_PARTS;
-      an0 = __ldg(ap + lane);
-      an1 = __ldg(ap + lane + 32);
-    }
-  }
+  if (ek < K && et_rev < len) g_e = __ldg(p.gamma + eg - et + et_rev);
   if (warp == 0) tmem_alloc<512>(tmem_slot);
   if (warp >= 1 && warp <= K) warp_cumsum128_finish(tb.A + (warp - 1) * TC, graw, len, p.eps, lane);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem = *tmem_slot;
   if (*failed != 0) {       // an earlier launch gave up on a wait: outputs stay untouched (the tiles still have to land)
+    pdl_wait();
     mbar_wait(&bars[B_VY], 0, 250);
     mbar_wait(&bars[B_QK], 0, 250);
     __syncthreads();
@@ -325,12 +324,6 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
     tb.col[ek * TC + et] = st ? 1.f : __expf(a_mid - a);
     tb.row[ek * TC + et] = rf;
     tb.w[ek * TC + et] = make_float2(c_e.x * rf, -c_e.y * rf);
-    if ((warp & 3) < 2) {
-      double a2 = (double)an0 + (double)an1;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-      if (lane == 0) anc[ek * 2 + (warp & 3)] = (float)a2;
-    }
   }
   const uint32_t q_r = smem_u32(TQ), k_r = smem_u32(TK), v_r = smem_u32(TV), y_r = smem_u32(TY), sl = smem_u32(SL);
   const bool issuer = warp == 0 && elect_one();
@@ -463,6 +456,14 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   const bool storing = warp >= 8 && lane == 0 && len == TC && ok;
   if (storing) store_box(&maps.dq, SL, warp - 8, row0);
   auto stage_grad = [&](int k) { stage_state(SL + ((k + 2) & 3) * 16384, p.dstates + state_base(p, k, h, L.slot0 + L.c + 1, TD), tid); };
+  // the gradients of the states and the anchors are the reverse carry's; everything above is the call's inputs and the forward
+  // states, which are older (see launch_after)
+  pdl_wait();
+  if (ek < K && (warp & 3) < 2 && anchor_parts != nullptr) {      // (null: zero, see scan_bwd_tc)
+    const float* ap = anchor_parts + (((size_t)ek * p.H + h) * p.nslots + L.slot0 + L.c + (warp & 3)) * ANCHOR_PARTS;
+    an0 = __ldcg(ap + lane);
+    an1 = __ldcg(ap + lane + 32);
+  }
   if (has_ds) {
     stage_grad(0);
     stage_grad(1);
@@ -595,6 +596,12 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
     }
     if (p.dcoef != nullptr && et < len && ok) *reinterpret_cast<float2*>(p.dcoef + eg * 2) = dc;
     tb.row[ek * TC + et] = et < len ? c_e.x * dc.x + c_e.y * dc.y - kd : 0.f;
+    if ((warp & 3) < 2) {
+      double a2 = (double)an0 + (double)an1;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+      if (lane == 0) anc[ek * 2 + (warp & 3)] = (float)a2;
+    }
   }
   __syncthreads();
   if (ek < K) {

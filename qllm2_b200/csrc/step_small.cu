@@ -33,9 +33,6 @@ constexpr int ST_PF = 6;             // 32-wide K blocks of weights requested ah
 constexpr int ST_ONE_N = 4;          // up to this many sequences the step is one persistent kernel
 constexpr int ST_ONE_LAYERS = 64;    // (its layer pointers are kernel parameters)
 
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 __device__ __forceinline__ uint4 ld_weight(const bf16* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
