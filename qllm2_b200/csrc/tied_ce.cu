@@ -38,7 +38,7 @@ static CELayout ce_layout(const qpam_ce_args* a) {
   L.off_pidx = off; off += ce_align(n * 4);
   L.off_sums = off; off += 256 + ce_align(((size_t)(a->N > 0 ? a->N : 1) + CE_ROWS - 1) / CE_ROWS * 4 * sizeof(double));
   L.total_fwd = off;
-  L.ldp = (a->V + 7) & ~(int64_t)7;
+  L.ldp = (a->V + 63) & ~(int64_t)63;
   const size_t row_bytes = (size_t)L.ldp * dtype_size(a->io_dtype);
   int64_t rows = (int64_t)(((size_t)256 << 20) / row_bytes);
   rows = (rows / CE_TM) * CE_TM;
