@@ -39,6 +39,7 @@ struct GemmParams {
   int32_t kb_total;         // K blocks in total
   int32_t kb_per_split;     // K blocks per blockIdx.z
   int32_t swap_xy;          // 1: blockIdx.x walks the M tiles (neighbouring CTAs share the B tile in L2)
+  int32_t walk;             // > 0 (WALK): tiles of 2 x 128 rows times BN columns, all of them, dealt to the grid's CTA pairs
   int64_t M, N;             // logical extents (rows / columns of D)
   // EPI_STATS
   const int64_t* targets;
@@ -68,6 +69,8 @@ struct GemmParams {
 // PAIR: two CTAs of a cluster (neighbouring SMs) work on one 256-row tile with cta_group::2 MMAs: each CTA loads
 // its own 128 rows of A and only HALF of the B tile, so the operand traffic per MAC drops by a third while both
 // accumulator buffers stay (short-K products with heavy epilogues).
+// WALK: the grid is one CTA pair per two SMs, and a pair takes every (pairs)-th tile of the whole output, columns first
+// (neighbours share the rows of A in L2): no last wave, and the epilogue of each tile runs under the MMAs of the next.
 template <int BN, int MT = 1, bool PAIR = false>
 struct Cfg {
   static constexpr int A_BYTES = MT * BM * BK * 2;           // 16 KB per row tile
@@ -82,14 +85,15 @@ struct Cfg {
   static constexpr size_t SMEM_BYTES_STAGED = SMEM_BYTES + (size_t)EPI_WARPS * EPI_STAGE_BYTES;
 };
 
-template <int BN, int EPI, bool A_MN, bool B_MN, int MT = 1, bool PAIR = false>
+template <int BN, int EPI, bool A_MN, bool B_MN, int MT = 1, bool PAIR = false, bool WALK = false>
 __global__ void __launch_bounds__(NTHREADS, 1)
 k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
           const __grid_constant__ CUtensorMap tmC, const GemmParams p) {   // tmC: EPI_PROBS output, boxes of 64 x 32
   using namespace umma;
   using C = Cfg<BN, MT, PAIR>;
   static_assert(MT == 1 || EPI == EPI_STORE || EPI == EPI_STORE_BF16, "two row tiles per CTA: plain stores only");
-  static_assert(!PAIR || (MT == 1 && !A_MN && !B_MN), "CTA pairs: K-major operands, one row tile per CTA");
+  static_assert(!PAIR || (MT == 1 && A_MN == B_MN), "CTA pairs: one row tile per CTA");
+  static_assert(!WALK || (PAIR && (EPI == EPI_STORE || EPI == EPI_STORE_BF16)), "tile walk: CTA pairs, plain stores");
   // PAIR: launched as clusters of two CTAs along the row-tile axis; tmB's box holds BN / 2 rows
   const uint32_t crank = PAIR ? cluster_ctarank() : 0u;
   const bool leader = crank == 0u;
@@ -105,9 +109,13 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::STAGES + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_tile = p.swap_xy ? blockIdx.x : blockIdx.y;
-  const int n_begin = (p.swap_xy ? blockIdx.y : blockIdx.x) * p.tiles_per_cta;
-  const int n_end = min(p.n_tiles, n_begin + p.tiles_per_cta);
+  const int m_tile0 = WALK ? 0 : p.swap_xy ? blockIdx.x : blockIdx.y;
+  const int n_begin = WALK ? blockIdx.x >> 1 : (p.swap_xy ? blockIdx.y : blockIdx.x) * p.tiles_per_cta;
+  const int n_end = WALK ? p.walk : min(p.n_tiles, n_begin + p.tiles_per_cta);
+  const int n_step = WALK ? gridDim.x >> 1 : 1;
+  // row tile and column tile of step n
+  auto tile_m = [&](int n) { return WALK ? 2 * (n / p.n_tiles) + (int)crank : m_tile0; };
+  auto tile_n = [&](int n) { return WALK ? n % p.n_tiles : n; };
   const int kb_begin = blockIdx.z * p.kb_per_split;
   const int kb_end = min(p.kb_total, kb_begin + p.kb_per_split);
   uint32_t* err_slot = tmem_slot + 1;
@@ -116,7 +124,6 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
     // one read of the device error word for the whole CTA: every warp must take the same side of has_work
     // (the epilogue warps meet at a named barrier), whatever another CTA writes meanwhile
     *err_slot = (uint32_t) * reinterpret_cast<volatile int*>(&g_device_error);
-    if (EPI == EPI_STATS && p.zero_word && blockIdx.x == 0 && blockIdx.y == 0) *p.zero_word = 0u;
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
@@ -126,7 +133,11 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
       mbar_init(&tempty[b], (PAIR ? 2 : 1) * EPI_WARPS);  // one arrival per epilogue warp (of both CTAs of a pair)
     }
     fence_barrier_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
   }
+  pdl_wait();      // (before the allocation: tensor memory held while waiting could be what another kernel waits for)
+  if (EPI == EPI_STATS && threadIdx.x == 0 && p.zero_word && blockIdx.x == 0 && blockIdx.y == 0) *p.zero_word = 0u;
   if (warp == 1) {
     if (PAIR) tmem_alloc_pair<C::TMEM_COLS>(tmem_slot);
     else tmem_alloc<C::TMEM_COLS>(tmem_slot);
@@ -135,6 +146,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
   if (PAIR) cluster_sync_all();   // the peer's barriers exist before anything signals them
   else __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
   // after a failed handshake anywhere on the device, later CTAs do not start new work
   const bool has_work = (n_begin < n_end) && (kb_begin < kb_end) && (*err_slot == 0);
@@ -143,12 +155,11 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
     if (warp == 0) {
       // ------------------------------------------------------------- TMA producer
       if (elect_one()) {
-        tma_prefetch_desc(&tmA);
-        tma_prefetch_desc(&tmB);
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
-        for (int n = n_begin; n < n_end && ok; ++n) {
+        for (int nn = n_begin; nn < n_end && ok; nn += n_step) {
+          const int n = tile_n(nn), m_tile = tile_m(nn);
           for (int kb = kb_begin; kb < kb_end; ++kb) {
             if (!mbar_wait(&empty[stage], phase ^ 1, 101)) { ok = false; break; }
             unsigned char* sa = smem + (size_t)stage * C::STAGE_BYTES;
@@ -157,8 +168,16 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
               // the leader's barrier counts the bytes of both CTAs; each CTA loads its rows of A and its half of B
               if (leader) mbar_arrive_expect_tx(&full[stage], 2 * C::STAGE_BYTES);
               const uint32_t fb = cluster_map(&full[stage], 0);
-              tma_load_2d_pair(sa, &tmA, fb, kb * BK, m_tile * BM);
-              tma_load_2d_pair(sb, &tmB, fb, kb * BK, n * BN + (int)crank * (BN / 2));
+              if constexpr (A_MN) {
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                  tma_load_2d_pair(sa + j * 8192, &tmA, fb, m_tile * BM + j * 64, kb * BK);
+                  tma_load_2d_pair(sb + j * 8192, &tmB, fb, n * BN + (int)crank * (BN / 2) + j * 64, kb * BK);
+                }
+              } else {
+                tma_load_2d_pair(sa, &tmA, fb, kb * BK, m_tile * BM);
+                tma_load_2d_pair(sb, &tmB, fb, kb * BK, n * BN + (int)crank * (BN / 2));
+              }
               if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
               continue;
             }
@@ -194,7 +213,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
         uint32_t phase = 0;
         bool ok = true;
         int it = 0;
-        for (int n = n_begin; n < n_end && ok; ++n, ++it) {
+        for (int nn = n_begin; nn < n_end && ok; nn += n_step, ++it) {
           const int buf = it % C::NBUF;
           const uint32_t bphase = (it / C::NBUF) & 1;
           if (!mbar_wait(&tempty[buf], bphase ^ 1, 102)) { ok = false; break; }
@@ -233,7 +252,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
       const int half = (warp - 2) >> 2;                        // which half of the tile's columns
       constexpr int CC_HALF = BN / 64;                         // 32-column groups per half
       const int r_tile = quarter * 32 + lane;                  // row within the tile == TMEM lane
-      const int64_t row = (int64_t)m_tile * BM + r_tile;       // row of D
+      const int64_t row = (int64_t)m_tile0 * BM + r_tile;      // row of D (statistics and probabilities)
       const bool row_ok = row < p.M;
       const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
       // EPI_STATS running state
@@ -260,7 +279,8 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
       const float mul_r = sc_pos ? 1.f : sc_r;
       bool ok = true;
       int it = 0;
-      for (int n = n_begin; n < n_end && ok; ++n, ++it) {
+      for (int nn = n_begin; nn < n_end && ok; nn += n_step, ++it) {
+        const int n = tile_n(nn), m_tile = tile_m(nn);
         const int buf = it % C::NBUF;
         const uint32_t bphase = (it / C::NBUF) & 1;
         if (!mbar_wait(&tfull[buf], bphase, 104)) { ok = false; break; }

@@ -178,7 +178,7 @@ extern "C" int qpam_ce_partial(const qpam_ce_args* a, float* row_max, float* row
     if (rc) return rc;
     CEParams p = ce_params(a, L);
     p.nsplit = L.tc.nsplit;
-    k_ce_merge<<<(unsigned)((a->N + 255) / 256), 256, 0, st>>>(p, row_max, row_sumexp, row_tgt, row_argmax);
+    launch_after(k_ce_merge, (unsigned)((a->N + 255) / 256), 256, 0, st, p, row_max, row_sumexp, row_tgt, row_argmax);
     QPAM_LAUNCH_CHECK("k_ce_merge");
     return QPAM_OK;
   }
@@ -211,8 +211,8 @@ extern "C" int qpam_ce_loss(const qpam_ce_args* a, float* lse, float* loss, floa
     else k_ce_partial<float><<<grid, 256, 0, st>>>(p);
     QPAM_LAUNCH_CHECK("k_ce_partial");
   }
-  k_ce_rows<<<(unsigned)((a->N + CE_ROWS - 1) / CE_ROWS), 256, 0, st>>>(p, lse, loss, per_token, denom, loss_sum, correct, tokens,
-                                                                         reinterpret_cast<double*>(ws + L.off_sums + 256), arrived);
+  launch_after(k_ce_rows, (unsigned)((a->N + CE_ROWS - 1) / CE_ROWS), 256, 0, st, p, lse, loss, per_token, denom, loss_sum, correct, tokens,
+               reinterpret_cast<double*>(ws + L.off_sums + 256), arrived);
   QPAM_LAUNCH_CHECK("k_ce_rows");
   return QPAM_OK;
 }

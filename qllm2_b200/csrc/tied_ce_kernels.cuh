@@ -169,6 +169,8 @@ __global__ void __launch_bounds__(256) k_ce_partial(CEParams p) {
 }
 
 __global__ void k_ce_merge(CEParams p, float* row_max, float* row_sumexp, float* row_tgt, int64_t* row_argmax) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= p.N) return;
   float M = -INFINITY;
@@ -244,6 +246,8 @@ __global__ void __launch_bounds__(256) k_ce_rows(CEParams p, float* lse, float* 
   __shared__ int si[8][CE_ROWS];
   __shared__ double red[4][8];
   __shared__ bool last;
+  pdl_trigger();
+  pdl_wait();
   const int r = threadIdx.x & 31, part = threadIdx.x >> 5;
   const int64_t n = (int64_t)blockIdx.x * CE_ROWS + r;
   float M = -INFINITY, S = 0.f, tz = 0.f, best = -INFINITY;

@@ -9,21 +9,23 @@ namespace qpam {
 template <typename K>
 static int opt_in_smem(K kern, size_t bytes) { return allow_smem(reinterpret_cast<const void*>(kern), bytes); }
 
-// Launch a kernel of CTA pairs: clusters of two CTAs along x (pair_axis 0) or y (pair_axis 1).
+// Launch a kernel of CTA pairs: clusters of two CTAs along x.  Like every kernel of this file it may start while its
+// predecessor ends (launch_after in common.cuh).
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_pairs(void (*kern)(KArgs...), dim3 grid, int pair_axis, size_t smem, cudaStream_t st, Args&&... args) {
+static cudaError_t launch_pairs(void (*kern)(KArgs...), dim3 grid, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(tc::NTHREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = pair_axis == 0 ? 2 : 1;
-  at[0].val.clusterDim.y = pair_axis == 1 ? 2 : 1;
-  at[0].val.clusterDim.z = 1;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
@@ -117,7 +119,7 @@ int ce_tc_partial(const qpam_ce_args* a, const CETcPlan& pl, const CETcBuffers& 
   if (rc) return rc;
   const unsigned row_tiles = (unsigned)((a->N + tc::BM - 1) / tc::BM);
   p.swap_xy = 1;      // blockIdx.x walks the row tiles: the two CTAs of a pair are neighbours in x
-  QPAM_CUDA(launch_pairs(kern, dim3((row_tiles + 1) & ~1u, pl.nsplit, 1), 0, CfgP::SMEM_BYTES, st, tmH, tmW, tmW, p));
+  QPAM_CUDA(launch_pairs(kern, dim3((row_tiles + 1) & ~1u, pl.nsplit, 1), CfgP::SMEM_BYTES, st, tmH, tmW, tmW, p));
   QPAM_LAUNCH_CHECK("k_tc_gemm<stats>");
   return QPAM_OK;
 }
@@ -143,7 +145,7 @@ int ce_tc_logits(const qpam_ce_args* a, const CETcPlan& pl, void* out, int64_t l
   p.kb_per_split = p.kb_total;
   p.M = a->N; p.N = a->V;
   p.swap_xy = 1;
-  QPAM_CUDA(launch_pairs(kern, dim3((row_tiles + 1) & ~1u, n_groups, 1), 0, CfgP::SMEM_BYTES_STAGED, st, tmH, tmW, tmO, p));
+  QPAM_CUDA(launch_pairs(kern, dim3((row_tiles + 1) & ~1u, n_groups, 1), CfgP::SMEM_BYTES_STAGED, st, tmH, tmW, tmO, p));
   QPAM_LAUNCH_CHECK("k_tc_gemm<logits>");
   return QPAM_OK;
 }
@@ -151,10 +153,12 @@ int ce_tc_logits(const qpam_ce_args* a, const CETcPlan& pl, void* out, int64_t l
 // ------------------------------------------------------------------ backward
 __global__ void k_reduce_splits_bf16(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int64_t n,
                                      int splits, int64_t split_stride) {
+  pdl_trigger();
+  pdl_wait();
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += (int64_t)gridDim.x * blockDim.x * 4) {
-    float4 acc = *reinterpret_cast<const float4*>(part + i);
+    float4 acc = __ldcg(reinterpret_cast<const float4*>(part + i));      // (not the read-only path: see ld_dependent)
     for (int s = 1; s < splits; ++s) {
-      const float4 x = *reinterpret_cast<const float4*>(part + s * split_stride + i);
+      const float4 x = __ldcg(reinterpret_cast<const float4*>(part + s * split_stride + i));
       acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
     }
     __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
@@ -183,20 +187,23 @@ int ce_tc_backward(const qpam_ce_args* a, const CETcPlan& pl, const CETcBuffers&
   const int64_t V = a->V;
   auto k_probs = tc::k_tc_gemm<256, tc::EPI_PROBS, false, false, 1, true>;      // CTA pairs, as the forward pass
   using CfgP = tc::Cfg<256, 1, true>;
-  // dH and dW run long K loops into few output tiles: two row tiles per CTA share every B block
+  // dH runs long K loops into few output tiles: two row tiles per CTA share every B block
   constexpr int MT = 2;
   auto k_dh = tc::k_tc_gemm<256, tc::EPI_STORE, false, true, MT>;
-  auto k_dw = tc::k_tc_gemm<256, tc::EPI_STORE, true, true, MT>;
+  // dW has many tiles (591 of 256 x 256 at V = 50261, F = 768) whose K is the number of rows: CTA pairs walk them, so that with
+  // few rows the stores of a tile hide behind the products of the next.  The bytes from L2 are those of two row tiles a CTA.
+  // 509 rows: 50 -> 38 us; 8192 rows (K long, four whole waves of either) the same 400.
+  auto k_dw = tc::k_tc_gemm<256, tc::EPI_STORE, true, true, 1, true, true>;
   int rc = opt_in_smem(k_probs, CfgP::SMEM_BYTES_STAGED);
   if (rc) return rc;
   rc = opt_in_smem(k_dh, tc::Cfg<256, MT>::SMEM_BYTES_STAGED);
   if (rc) return rc;
-  rc = opt_in_smem(k_dw, tc::Cfg<256, MT>::SMEM_BYTES_STAGED);
+  rc = opt_in_smem(k_dw, CfgP::SMEM_BYTES_STAGED);
   if (rc) return rc;
   // one row chunk: dW is complete after one product and leaves as bf16 straight from the accumulators
-  auto k_dw16 = tc::k_tc_gemm<256, tc::EPI_STORE_BF16, true, true, MT>;
+  auto k_dw16 = tc::k_tc_gemm<256, tc::EPI_STORE_BF16, true, true, 1, true, true>;
   const bool dw_direct = a->N <= pl.chunk_rows;
-  rc = opt_in_smem(k_dw16, tc::Cfg<256, MT>::SMEM_BYTES_STAGED);
+  rc = opt_in_smem(k_dw16, CfgP::SMEM_BYTES_STAGED);
   if (rc) return rc;
   CUtensorMap tmWk, tmWmn;
   rc = make_map(&tmWk, a->w, F, V, F, tc::BK, 128);   // K-major B of the logits GEMM: half a tile per CTA of a pair
@@ -227,7 +234,7 @@ int ce_tc_backward(const qpam_ce_args* a, const CETcPlan& pl, const CETcBuffers&
     p.swap_xy = 1;   // consecutive CTAs take the row tiles of one vocabulary tile: W is read from DRAM once
     CUtensorMap tmPst;                                                                 // P as the output of TMA stores
     if ((rc = make_map(&tmPst, b.pbuf, V, rows, b.ldp, 64, 32))) return rc;
-    QPAM_CUDA(launch_pairs(k_probs, dim3((row_tiles + 1) & ~1u, n_groups, 1), 0, CfgP::SMEM_BYTES_STAGED, st, tmHk, tmWk, tmPst, p));
+    QPAM_CUDA(launch_pairs(k_probs, dim3((row_tiles + 1) & ~1u, n_groups, 1), CfgP::SMEM_BYTES_STAGED, st, tmHk, tmWk, tmPst, p));
     QPAM_LAUNCH_CHECK("k_tc_gemm<probs>");
     // 2) dH[r0:r0+rows] = P W, split over the vocabulary (K) axis, fp32 partials then bf16
     tc::GemmParams g{};
@@ -237,10 +244,9 @@ int ce_tc_backward(const qpam_ce_args* a, const CETcPlan& pl, const CETcBuffers&
     const int ks = (g.kb_total + g.kb_per_split - 1) / g.kb_per_split;
     g.M = rows; g.N = F;
     g.c = b.dh_part; g.ldc = F; g.beta = 0;
-    k_dh<<<dim3(f_tiles, (row_tiles + MT - 1) / MT, ks), tc::NTHREADS, tc::Cfg<256, MT>::SMEM_BYTES_STAGED, st>>>(tmPk, tmWmn, tmWmn, g);
+    launch_after(k_dh, dim3(f_tiles, (row_tiles + MT - 1) / MT, ks), tc::NTHREADS, tc::Cfg<256, MT>::SMEM_BYTES_STAGED, st, tmPk, tmWmn, tmWmn, g);
     QPAM_LAUNCH_CHECK("k_tc_gemm<dH>");
-    k_reduce_splits_bf16<<<592, 256, 0, st>>>(b.dh_part, reinterpret_cast<__nv_bfloat16*>(dh) + r0 * F, rows * F, ks,
-                                             rows * F);
+    launch_after(k_reduce_splits_bf16, 592, 256, 0, st, b.dh_part, reinterpret_cast<__nv_bfloat16*>(dh) + r0 * F, rows * F, ks, rows * F);
     QPAM_LAUNCH_CHECK("k_reduce_splits_bf16");
     if (dh_ready_stream != nullptr && r0 + rows >= a->N) {
       // dH is complete: a caller's side stream (the all-reduce of the vocabulary-parallel form) may start on it
@@ -250,7 +256,10 @@ int ce_tc_backward(const qpam_ce_args* a, const CETcPlan& pl, const CETcBuffers&
     }
     // 3) dW (+)= P^T H[r0:r0+rows]
     tc::GemmParams w{};
-    w.n_tiles = f_tiles; w.tiles_per_cta = 1;
+    w.n_tiles = f_tiles;
+    const int64_t tiles = (V + 2 * tc::BM - 1) / (2 * tc::BM) * f_tiles;
+    w.walk = (int32_t)tiles;
+    const unsigned pairs = (unsigned)(tiles < sm_count() / 2 ? tiles : sm_count() / 2);
     w.kb_total = (int32_t)((rows + tc::BK - 1) / tc::BK); w.kb_per_split = w.kb_total;
     w.M = V; w.N = F;
     if (!dw_direct) { w.c = b.dwacc + (size_t)(chunk_idx % pl.dw_bufs) * V * F; w.beta = chunk_idx >= pl.dw_bufs ? 1 : 0; }
@@ -258,18 +267,16 @@ int ce_tc_backward(const qpam_ce_args* a, const CETcPlan& pl, const CETcBuffers&
     if (dw_direct) {
       CUtensorMap tmDw;
       if ((rc = make_map(&tmDw, dw, F, V, F, 64, 32))) return rc;
-      k_dw16<<<dim3(f_tiles, (unsigned)((V + MT * tc::BM - 1) / (MT * tc::BM)), 1), tc::NTHREADS,
-               tc::Cfg<256, MT>::SMEM_BYTES_STAGED, st>>>(tmPmn, tmHmn, tmDw, w);
+      QPAM_CUDA(launch_pairs(k_dw16, dim3(2 * pairs), CfgP::SMEM_BYTES_STAGED, st, tmPmn, tmHmn, tmDw, w));
     } else {
-      k_dw<<<dim3(f_tiles, (unsigned)((V + MT * tc::BM - 1) / (MT * tc::BM)), 1), tc::NTHREADS,
-             tc::Cfg<256, MT>::SMEM_BYTES_STAGED, st>>>(tmPmn, tmHmn, tmHmn, w);
+      QPAM_CUDA(launch_pairs(k_dw, dim3(2 * pairs), CfgP::SMEM_BYTES_STAGED, st, tmPmn, tmHmn, tmHmn, w));
     }
     QPAM_LAUNCH_CHECK("k_tc_gemm<dW>");
     ++chunk_idx;
   }
   if (!dw_direct) {
-    k_reduce_splits_bf16<<<1184, 256, 0, st>>>(b.dwacc, reinterpret_cast<__nv_bfloat16*>(dw), V * (int64_t)F,
-                                              chunk_idx < pl.dw_bufs ? (chunk_idx > 0 ? chunk_idx : 1) : pl.dw_bufs, V * (int64_t)F);
+    launch_after(k_reduce_splits_bf16, 1184, 256, 0, st, b.dwacc, reinterpret_cast<__nv_bfloat16*>(dw), V * (int64_t)F,
+                 chunk_idx < pl.dw_bufs ? (chunk_idx > 0 ? chunk_idx : 1) : pl.dw_bufs, V * (int64_t)F);
     QPAM_LAUNCH_CHECK("k_reduce_splits_bf16");
   }
   return QPAM_OK;

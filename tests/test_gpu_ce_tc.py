@@ -137,3 +137,25 @@ def test_head_logits_bf16_tiles(N, F, V):
     ref = ce_oracle.head_logits(h.float().numpy(), w.float().numpy())
     err = np.abs(z.float().cpu().numpy() - ref).max() / np.abs(ref).max()
     assert err <= 2.0 ** -8, err
+
+
+@pytest.mark.parametrize("N,D,V", [
+    (65, 260, 20001),           # 79 x 3 tiles of dW, more than pairs of SMs: ragged in both directions
+    (8192 + 65, 260, 20001),    # the same over two row chunks (fp32 sums)
+    (70, 130, 257),             # fewer tiles than pairs; the second row tile of the last pair has one row
+])
+def test_weight_gradient_tile_walk(N, D, V):
+    c = synthetic.ce_inputs(N, D, V, seed=N, dtype=torch.bfloat16)
+    w_host = (c.w.float() * 20).bfloat16()
+    h = c.h.to(DEV).requires_grad_(True)
+    w = w_host.to(DEV).requires_grad_(True)
+    loss = fused_ce.fused_linear_cross_entropy(h, w, c.targets.to(DEV))
+    loss.backward()
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    hd, wd, t = h.detach().double(), w.detach().double(), c.targets.to(DEV)
+    p = torch.softmax(hd @ wd.T, 1)
+    p[torch.arange(N, device=DEV), t] -= 1.0
+    p /= N
+    assert_close(w.grad.double().cpu().numpy(), (p.T @ hd).cpu().numpy(), 2e-2, "dW")
+    assert_close(h.grad.double().cpu().numpy(), (p @ wd).cpu().numpy(), 2e-2, "dH")
