@@ -10,19 +10,25 @@
 // order of atomics, so the same inputs give the same token on every run.  Tokens that tie with the nucleus threshold are
 // all kept (a sort would keep an arbitrary subset of them).
 //
-// What bounds it: the row is 100 KB (bf16, V = 50 k) and the 256 rows of a full engine are 26 MB, 4 us of HBM, so the
-// work is the number of passes over the row and the block-wide steps between them.  A row is never copied: every pass
-// streams it again with 16-byte loads (L1 / L2 hits after the first), which leaves room for two CTAs per SM, and the
-// tokens of the penalty are one bit each in shared memory.
-//   small top-k   pass 1 takes every thread's largest value; the k-th largest of those is a lower bound of the k-th
-//                 largest of the row, so pass 2 collects the few values at or above it (about k + k^2 / threads) and
-//                 everything after that works on that list: ranks by counting, no search.
+// What bounds it: the row is 100 KB (bf16, V = 50 k) and the 256 rows of a full engine are 26 MB, 4 us of HBM.  A row is never
+// copied: every pass streams it again with 16-byte loads (L1 / L2 hits after the first), which leaves room for two CTAs per
+// SM, and what a pass costs is its instructions for 98 elements a thread.  So a pass does per element only what it must:
+//   * the tokens of the penalty are one bit each in shared memory.  A pass drops them (-inf in the raw word) and takes them one
+//     by one afterwards, warp by warp for the warp's own stretch: some lane of a warp holds one in nine of ten steps, and the
+//     division and its tests for eight elements were then most of the pass;
+//   * the maximum is taken on the raw (packed) values, scaled once per block of four groups;
+//   * a comparison with a bin's rough edges decides for nearly every element whether its bin has to be formed at all.
+//   small top-k   pass 1 leaves the largest value of every block of four groups (32 or 16 values); the k-th largest of the
+//                 threads' maxima is a lower bound of the k-th largest of the row, so only blocks that reach it (about k) are
+//                 read again, a group for each thread; the values at or above the bound (about k + k^2 / threads) are a list
+//                 and everything after that works on that list: ranks by counting, no search.
 //   otherwise     counts or probability mass over 2048 bins LINEAR in x (leading bits of the float pattern put most of a
 //                 row into a dozen bins, whose atomics serialise), the bin in which the k-th value / the nucleus closes,
 //                 and the exact threshold from the elements of that bin.  Masses are accumulated in fixed point: the
 //                 sums do not depend on the order of the atomics.
-// 256 rows x 50261 bf16 logits, top-k 50 + top-p 0.9 + penalty: 34.8 us a call; 128.9 us for the version that kept
-// the row as floats in shared memory (one CTA per SM, two waves) and searched it by radix passes.
+// 256 rows x 50261 bf16 logits with a penalty over 16..513 tokens (a call, device): top-k 50 + top-p 0.9 34.8 -> 20.8 us; top-p 0.9 alone
+// 124 -> 82; neither 54 -> 29.  One row: 19 -> 16.7, 66 -> 51, 29 -> 19.8.  (Before: eight tests and a division for every group of
+// a pass, the small top-k reading the whole row twice, one warp walking the stretch of the draw.)
 #include "common.cuh"
 
 namespace qpam {
@@ -31,6 +37,8 @@ namespace {
 constexpr int SAMPLE_LIST = 1024;            // values that the list steps can hold
 constexpr int SAMPLE_LIST_TOP_K = 384;       // top-k up to which the list is expected to fit (512 threads: ~710 values)
 constexpr int SAMPLE_BINS = 2048;
+constexpr int SAMPLE_BLOCKS = 4096;          // blocks of a row (several of a thread's steps share one when a row has more)
+constexpr int SAMPLE_ITEMS = 2048;
 constexpr float SAMPLE_BINS_PER_UNIT = 64.f;  // bins reach 32 units below the maximum (e^-32 of its mass)
 constexpr size_t SAMPLE_SMEM_BITMAP = 160 * 1024;
 
@@ -62,6 +70,10 @@ struct Scratch {
   union {
     uint32_t bins[3][SAMPLE_BINS];     // counts | low and high half of the masses
     struct {
+      float top[SAMPLE_BLOCKS];        // [block][thread] largest value of a block
+      int item[SAMPLE_ITEMS];          // blocks to read again
+    } blocks;
+    struct {
       float e[SAMPLE_LIST];            // survivors of top-k in vocabulary order
       int idx[SAMPLE_LIST];
     } sorted;
@@ -70,7 +82,7 @@ struct Scratch {
   int idx[SAMPLE_LIST];
   double warp_d[32];
   float warp_f[32];
-  int n_list, cross_bin, chosen, last_kept, warp_i[32];
+  int n_list, n_item, cross_bin, chosen, last_kept, warp_i[32];
   double cross_before;
   uint32_t limit;
 };
@@ -98,7 +110,7 @@ __device__ __forceinline__ double block_sum(double v, Scratch* sc) {
 }
 
 // The row as groups of 16 aligned bytes.  Group g holds the elements [g * VEC - lead, (g + 1) * VEC - lead): rows need
-// not start on a 16-byte boundary, and the first and last group are read element by element.
+// not start on a 16-byte boundary; the first and last group are read element by element, with -inf outside the row.
 template <typename T>
 struct Row {
   static constexpr int VEC = 16 / (int)sizeof(T);
@@ -106,6 +118,7 @@ struct Row {
   const uint32_t* bits;    // penalised elements by shifted position (index + lead); null = none
   int V, lead, groups;
   float inv_t, penalty;
+  bool flat;               // infinite temperature: every finite logit is 0
 
   __device__ __forceinline__ void init(const T* row, int V_) {
     base = row;
@@ -115,50 +128,110 @@ struct Row {
   }
   __device__ __forceinline__ uint4 raw(int g) const {
     const int i0 = g * VEC - lead;
-    if (i0 >= 0 && i0 + VEC <= V) return __ldg(reinterpret_cast<const uint4*>(base + i0));
+    if (i0 >= 0 && i0 + VEC <= V && !flat) return __ldg(reinterpret_cast<const uint4*>(base + i0));
     union { uint4 u; T t[VEC]; } r;
-    r.u = make_uint4(0, 0, 0, 0);
+    const uint32_t none = sizeof(T) == 2 ? 0xff80ff80u : 0xff800000u;      // -inf
+    r.u = make_uint4(none, none, none, none);
 #pragma unroll
     for (int j = 0; j < VEC; ++j)
-      if (i0 + j >= 0 && i0 + j < V) r.t[j] = base[i0 + j];
+      if (i0 + j >= 0 && i0 + j < V) r.t[j] = flat ? (T)((float)base[i0 + j] * 0.f) : base[i0 + j];
     return r.u;
   }
-  // temperature and penalty; elements outside the row become -inf
-  __device__ __forceinline__ void values(int g, uint4 u, float (&x)[VEC]) const {
-    if constexpr (sizeof(T) == 2) {
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  __device__ __forceinline__ uint32_t marks(int g) const {      // one bit for each element of a group (a word holds whole groups)
+    const int s = g * VEC;
+    return (bits[s >> 5] >> (s & 31)) & ((1u << VEC) - 1u);
+  }
+  // the group with -inf for its penalised elements
+  __device__ __forceinline__ uint4 plain(int g, uint4 u) const {
+    if (bits == nullptr) return u;
+    const uint32_t m = marks(g);
+    if (m == 0u) return u;
+    uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 4; ++j) {
+      if constexpr (sizeof(T) == 2) {
+        if (m >> (2 * j) & 1u) w[j] = (w[j] & 0xffff0000u) | 0xff80u;
+        if (m >> (2 * j + 1) & 1u) w[j] = (w[j] & 0xffffu) | 0xff800000u;
+      } else {
+        if (m >> j & 1u) w[j] = 0xff800000u;
+      }
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  // divided by the temperature
+  __device__ __forceinline__ void scaled(uint4 u, float (&x)[VEC]) const {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if constexpr (sizeof(T) == 2) {
         x[2 * j] = __uint_as_float(w[j] << 16) * inv_t;
         x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u) * inv_t;
+      } else {
+        x[j] = __uint_as_float(w[j]) * inv_t;
       }
-    } else {
-      x[0] = __uint_as_float(u.x) * inv_t;
-      x[1] = __uint_as_float(u.y) * inv_t;
-      x[2] = __uint_as_float(u.z) * inv_t;
-      x[3] = __uint_as_float(u.w) * inv_t;
     }
+  }
+  __device__ __forceinline__ float penalised(float x) const { return x > 0.f ? x / penalty : x * penalty; }
+  __device__ __forceinline__ float penalised_at(int i) const {
+    return penalised((float)base[i] * (flat ? 0.f : inv_t));
+  }
+  // temperature and penalty, in vocabulary order
+  __device__ __forceinline__ void values(int g, uint4 u, float (&x)[VEC]) const {
+    scaled(u, x);
     if (bits) {
-      const int s = g * VEC;
-      const uint32_t m = (bits[s >> 5] >> (s & 31)) & ((1u << VEC) - 1u);
+      const uint32_t m = marks(g);
       if (m) {
 #pragma unroll
         for (int j = 0; j < VEC; ++j)
-          if (m >> j & 1u) x[j] = x[j] > 0.f ? x[j] / penalty : x[j] * penalty;
-      }
-    }
-    if (g == 0 || g == groups - 1) {
-#pragma unroll
-      for (int j = 0; j < VEC; ++j) {
-        const int i = g * VEC - lead + j;
-        if (i < 0 || i >= V) x[j] = -INFINITY;
+          if (m >> j & 1u) x[j] = penalised(x[j]);
       }
     }
   }
 };
 
-// Every warp walks its own contiguous stretch of the row, four groups in flight per lane.  f(index of x[0], x).
+// Running maximum of raw groups, a NaN losing to any number.
+template <typename T>
+struct RawMax;
+template <>
+struct RawMax<float> {
+  float m = -INFINITY;
+  __device__ __forceinline__ void add(uint4 u) {
+    m = fmaxf(fmaxf(m, fmaxf(__uint_as_float(u.x), __uint_as_float(u.y))), fmaxf(__uint_as_float(u.z), __uint_as_float(u.w)));
+  }
+  __device__ __forceinline__ float value() const { return m; }
+};
+template <>
+struct RawMax<__nv_bfloat16> {
+  uint32_t m = 0xff80ff80u;
+  static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
+    const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&r);
+  }
+  __device__ __forceinline__ void add(uint4 u) { m = max2(m, max2(max2(u.x, u.y), max2(u.z, u.w))); }
+  __device__ __forceinline__ float value() const { return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u)); }
+};
+
+// Every warp walks its own contiguous stretch of the row, four groups in flight per lane; f(index, x) for one element after another.
+// EXACT: every element in its place.  Otherwise the penalised elements are -inf there and come one by one afterwards
+// (for_marked), for the warp's own stretch.
 template <int NT, typename T, typename F>
+__device__ __forceinline__ void for_marked(const Row<T>& r, F one) {
+  if (r.bits == nullptr) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (r.groups + NT / 32 - 1) / (NT / 32);
+  const int s0 = warp * per * Row<T>::VEC, s1 = min(r.groups, (warp + 1) * per) * Row<T>::VEC;      // shifted positions
+  for (int w = (s0 >> 5) + lane; w * 32 < s1; w += 32) {
+    uint32_t m = r.bits[w];
+    if (w * 32 < s0) m &= ~0u << (s0 & 31);
+    if (s1 - w * 32 < 32) m &= (1u << (s1 & 31)) - 1u;
+    while (m) {
+      const int i = w * 32 + __ffs((int)m) - 1 - r.lead;
+      m &= m - 1;
+      one(i, r.penalised_at(i));
+    }
+  }
+}
+template <int NT, bool EXACT, typename T, typename F>
 __device__ __forceinline__ void for_each(const Row<T>& r, F f) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int per = (r.groups + NT / 32 - 1) / (NT / 32);
@@ -168,13 +241,17 @@ __device__ __forceinline__ void for_each(const Row<T>& r, F f) {
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       if (g + 32 * k < g1) u[k] = r.raw(g + 32 * k);
+#pragma unroll 1
+    for (int gk = g; gk < min(g1, g + 128); gk += 32) {
+      const uint4 c = EXACT ? u[0] : r.plain(gk, u[0]);
+      u[0] = u[1]; u[1] = u[2]; u[2] = u[3];
+      float x[Row<T>::VEC];
+      if (EXACT) r.values(gk, c, x);
+      else r.scaled(c, x);
+      const int i0 = gk * Row<T>::VEC - r.lead;
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (g + 32 * k < g1) {
-        float x[Row<T>::VEC];
-        r.values(g + 32 * k, u[k], x);
-        f((g + 32 * k) * Row<T>::VEC - r.lead, x);
-      }
+      for (int j = 0; j < Row<T>::VEC; ++j) f(i0 + j, x[j]);
+    }
   }
 }
 
@@ -186,8 +263,33 @@ __device__ __forceinline__ void list_add(Scratch* sc, uint32_t key, int i) {
   }
 }
 
-__device__ __forceinline__ int bin_of(float x, float mx) {
-  return (int)fminf(fmaxf((mx - x) * SAMPLE_BINS_PER_UNIT, 0.f), (float)(SAMPLE_BINS - 1));
+__device__ __forceinline__ int bin_of(float x, float mx) {      // (the conversion saturates: below zero and NaN give 0)
+  return (int)min(__float2uint_rz(fmaf(x, -SAMPLE_BINS_PER_UNIT, mx * SAMPLE_BINS_PER_UNIT)), (uint32_t)(SAMPLE_BINS - 1));
+}
+// exp(x - mx) as __expf gives it, without its care for denormal results (four of its six instructions; a value that small is
+// never drawn)
+__device__ __forceinline__ float mass_of(float x, float mx) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"((x - mx) * 1.4426950408889634f));
+  return y;
+}
+// What few elements of a pass need stays out of line: 32 copies of it in a loop that jumps over them cost more than the pass.
+__device__ __noinline__ void list_bin_value(Scratch* sc, float x, float mx, int i, int cross, uint32_t key_k) {
+  if (bin_of(x, mx) != cross || order_key(x) < key_k) return;
+  const float e = mass_of(x, mx);
+  if (e > 0.f) list_add(sc, __float_as_uint(e), i);
+}
+// unnormalised probability of a kept value, 0 for a dropped one
+__device__ __forceinline__ float kept_mass_of(float x, float mx, int cross, uint32_t e_min, uint32_t key_k) {
+  const float e = order_key(x) >= key_k ? mass_of(x, mx) : 0.f;
+  if (cross < SAMPLE_BINS) {
+    const int b = bin_of(x, mx);
+    return b < cross || (b == cross && __float_as_uint(e) >= e_min) ? e : 0.f;
+  }
+  return __float_as_uint(e) >= e_min ? e : 0.f;
+}
+__device__ __noinline__ float kept_mass_slow(float x, float mx, int cross, uint32_t e_min, uint32_t key_k) {
+  return kept_mass_of(x, mx, cross, e_min, key_k);
 }
 
 // First bin at which the running sum over the bins (counts, or masses) reaches `target`, and the sum before it; the
@@ -246,9 +348,18 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sample_rows(SamplePar
   }
   Row<T> r;
   r.init(reinterpret_cast<const T*>(p.logits) + (size_t)row * p.ldl, p.V);
-  r.inv_t = p.inv_temperature;
+  r.flat = p.inv_temperature == 0.f;
+  r.inv_t = r.flat ? 1.f : p.inv_temperature;
   r.penalty = p.penalty;
   r.bits = nullptr;
+  // the first loads of the row are on their way while the penalty's bits are set
+  constexpr int VEC = Row<T>::VEC;
+  const int per = (r.groups + NT / 32 - 1) / (NT / 32);
+  const int g0 = warp * per, g1 = min(r.groups, (warp + 1) * per);      // this warp's stretch
+  uint4 ahead[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (g0 + lane + 32 * k < g1) ahead[k] = r.raw(g0 + lane + 32 * k);
   if (hrow >= 0 && p.penalty != 1.0f) {
     uint32_t* bm = p.bitmaps ? p.bitmaps + (size_t)row * p.bitmap_words : reinterpret_cast<uint32_t*>(dyn_smem);
     for (int i = tid; i < p.bitmap_words; i += NT) bm[i] = 0u;
@@ -262,43 +373,95 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sample_rows(SamplePar
     }
     r.bits = bm;
   }
-  if (tid == 0) { sc->n_list = 0; sc->chosen = 0x7fffffff; sc->last_kept = -1; }
+  if (tid == 0) { sc->n_list = sc->n_item = 0; sc->chosen = 0x7fffffff; sc->last_kept = -1; }
   __syncthreads();
-
-  // ---- pass 1: the maximum, and every thread's own
-  float mine = -INFINITY;
-  for_each<NT>(r, [&](int, const float (&x)[Row<T>::VEC]) {
-#pragma unroll
-    for (int j = 0; j < Row<T>::VEC; ++j) mine = fmaxf(mine, x[j]);
-  });
-  const float mx = block_max<NT>(mine, sc);
 
   const bool use_k = p.top_k > 0 && p.top_k < p.V;
   const bool use_p = p.top_p > 0.f && p.top_p < 1.f;
+  // ---- pass 1: the maximum, every thread's own, and (small top-k) that of each of its blocks: `steps` groups, 32 apart
+  const bool want_list = use_k && p.top_k <= SAMPLE_LIST_TOP_K;
+  const int most = SAMPLE_BLOCKS / NT, lane_groups = (per + 31) / 32;
+  const int steps = (lane_groups + 4 * most - 1) / (4 * most) * 4, n_blocks = (lane_groups + steps - 1) / steps;
+  float mine = -INFINITY, marked = -INFINITY;
+  for (int b = 0; b < n_blocks; ++b) {
+    RawMax<T> best;
+    for (int k0 = 0; k0 < steps; k0 += 4) {
+      const int g = g0 + lane + 32 * (b * steps + k0);
+      uint4 u[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {        // the next four are requested before these are looked at
+        u[k] = ahead[k];
+        if (g + 32 * (4 + k) < g1) ahead[k] = r.raw(g + 32 * (4 + k));
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (g + 32 * k < g1) best.add(r.plain(g + 32 * k, u[k]));
+    }
+    const float v = best.value() * r.inv_t;       // (rounding is monotone: the scaled maximum is the maximum of the scaled)
+    if (want_list || use_p) sc->blocks.top[b * NT + tid] = v;
+    mine = fmaxf(mine, v);
+  }
+  for_marked<NT>(r, [&](int, float x) { marked = fmaxf(marked, x); });
+  mine = fmaxf(mine, marked);
+  const float mx = block_max<NT>(mine, sc);
+
   const float u = p.uniforms[row];
   float kept_mass = 0.f, kept_count = 0.f, z = 0.f;
   int pick = 0;
   bool listed = false;
 
-  if (use_k && p.top_k <= SAMPLE_LIST_TOP_K) {
-    // k-th largest of the threads' maxima, to its leading 20 bits (rounded down: still a lower bound)
+  if (want_list) {
+    // k-th largest of the threads' maxima, to its leading 20 bits (rounded down: still a lower bound), by one warp
     const uint32_t my_key = order_key(mine);
-    uint32_t bound = 0;
-    for (int b = 31; b >= 12; --b) {
-      const uint32_t t = bound | (1u << b);
-      if (__syncthreads_count(my_key >= t) >= p.top_k) bound = t;
-    }
-    if (__any_sync(0xffffffffu, my_key >= bound)) {       // most warps hold no value of the list: they skip the pass
-      const float floor_x = key_value(bound);
-      const bool all = bound <= 0x007fffffu;         // fewer than k threads hold a finite value
-      for_each<NT>(r, [&](int i0, const float (&x)[Row<T>::VEC]) {
+    sc->key[tid] = my_key;
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t keys[NT / 32], found = 0;
 #pragma unroll
-        for (int j = 0; j < Row<T>::VEC; ++j)
-          if ((all || x[j] >= floor_x) && (unsigned)(i0 + j) < (unsigned)r.V) list_add(sc, order_key(x[j]), i0 + j);
-      });
+      for (int c = 0; c < NT / 32; ++c) keys[c] = sc->key[c * 32 + lane];
+      for (int b = 31; b >= 12; --b) {
+        const uint32_t t = found | (1u << b);
+        int n = 0;
+#pragma unroll
+        for (int c = 0; c < NT / 32; ++c) n += keys[c] >= t;
+        if (__reduce_add_sync(0xffffffffu, n) >= p.top_k) found = t;
+      }
+      if (lane == 0) sc->limit = found;
     }
     __syncthreads();
-    const int m = sc->n_list;
+    const uint32_t bound = sc->limit;
+    const float floor_x = key_value(bound);
+    const bool all = bound <= 0x007fffffu;           // fewer than k threads hold a finite value: every element is listed
+    if (all) {
+      for_each<NT, true>(r, [&](int i, float x) {
+        if ((unsigned)i < (unsigned)r.V) list_add(sc, order_key(x), i);
+      });
+    } else {
+      for (int b = 0; b < n_blocks; ++b)
+        if (sc->blocks.top[b * NT + tid] >= floor_x) {
+          const int at = atomicAdd(&sc->n_item, 1);
+          if (at < SAMPLE_ITEMS) sc->blocks.item[at] = b * NT + tid;
+        }
+      if (marked >= floor_x)
+        for_marked<NT>(r, [&](int i, float x) {
+          if (x >= floor_x) list_add(sc, order_key(x), i);
+        });
+      __syncthreads();
+      const int n_item = min(sc->n_item, SAMPLE_ITEMS);
+      for (int e = tid; e < n_item * steps; e += NT) {      // a group of a block for each thread
+        const int it = sc->blocks.item[e / steps], b = it / NT, t = it - b * NT, w = t >> 5;
+        const int g = w * per + (t & 31) + 32 * (b * steps + e % steps);
+        if (g < min(r.groups, (w + 1) * per)) {
+          float x[VEC];
+          r.scaled(r.plain(g, r.raw(g)), x);
+#pragma unroll
+          for (int j = 0; j < VEC; ++j)
+            if (x[j] >= floor_x) list_add(sc, order_key(x[j]), g * VEC - r.lead + j);
+        }
+      }
+    }
+    __syncthreads();
+    const int m = sc->n_item > SAMPLE_ITEMS ? SAMPLE_LIST + 1 : sc->n_list;
     listed = m <= SAMPLE_LIST;                             // block-uniform
     if (listed) {
       const int m4 = (m + 3) & ~3;
@@ -317,7 +480,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sample_rows(SamplePar
             const uint4 o = *reinterpret_cast<const uint4*>(&sc->key[i]);
             above += (o.x > key) + (o.y > key) + (o.z > key) + (o.w > key);
           }
-          if (above < p.top_k && __expf(key_value(key) - mx) > 0.f) kk[c] = key;
+          if (above < p.top_k && mass_of(key_value(key), mx) > 0.f) kk[c] = key;
         }
       }
       __syncthreads();
@@ -338,7 +501,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sample_rows(SamplePar
             const int4 q = *reinterpret_cast<const int4*>(&sc->idx[i]);
             before += (o.x && q.x < idx) + (o.y && q.y < idx) + (o.z && q.z < idx) + (o.w && q.w < idx);
           }
-          sc->sorted.e[before] = __expf(key_value(kk[c]) - mx);
+          sc->sorted.e[before] = mass_of(key_value(kk[c]), mx);
           sc->sorted.idx[before] = idx;
         }
       }
@@ -402,23 +565,21 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sample_rows(SamplePar
     uint32_t key_k = 0u;                     // top-k: keep keys >= key_k
     int cross = SAMPLE_BINS;                 // top-p: keep bins < cross, and in bin `cross` the masses >= e_min
     uint32_t e_min = 1u;                     //        (cross == SAMPLE_BINS: e_min alone decides)
+    float bin_lo = -INFINITY, bin_hi = INFINITY;      // below / above: the bin is certainly a later / an earlier one
+    float all_mass = 0.f;
     if (use_k) {
       for (int b = tid; b < SAMPLE_BINS; b += NT) sc->bins[0][b] = 0u;
       if (tid == 0) sc->n_list = 0;
       __syncthreads();
-      for_each<NT>(r, [&](int i0, const float (&x)[Row<T>::VEC]) {
-#pragma unroll
-        for (int j = 0; j < Row<T>::VEC; ++j)
-          if ((unsigned)(i0 + j) < (unsigned)r.V) atomicAdd(&sc->bins[0][bin_of(x[j], mx)], 1u);
+      for_each<NT, true>(r, [&](int i, float x) {
+        if ((unsigned)i < (unsigned)r.V) atomicAdd(&sc->bins[0][bin_of(x, mx)], 1u);
       });
       __syncthreads();
       find_crossing<NT, false>(sc, (double)p.top_k, 0.0, 0.0);
       const int cb = sc->cross_bin;
       const int need = p.top_k - (int)sc->cross_before;      // values to keep inside the bin
-      for_each<NT>(r, [&](int i0, const float (&x)[Row<T>::VEC]) {
-#pragma unroll
-        for (int j = 0; j < Row<T>::VEC; ++j)
-          if ((unsigned)(i0 + j) < (unsigned)r.V && bin_of(x[j], mx) == cb) list_add(sc, order_key(x[j]), i0 + j);
+      for_each<NT, true>(r, [&](int i, float x) {
+        if ((unsigned)i < (unsigned)r.V && bin_of(x, mx) == cb) list_add(sc, order_key(x), i);
       });
       if (tid == 0) sc->limit = 0xffffffffu;
       __syncthreads();
@@ -436,45 +597,58 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sample_rows(SamplePar
         for (int b = 31; b >= 0; --b) {
           const uint32_t t = key_k | (1u << b);
           double c = 0.0;
-          for_each<NT>(r, [&](int i0, const float (&x)[Row<T>::VEC]) {
-#pragma unroll
-            for (int j = 0; j < Row<T>::VEC; ++j)
-              if ((unsigned)(i0 + j) < (unsigned)r.V && order_key(x[j]) >= t) c += 1.0;
+          for_each<NT, true>(r, [&](int i, float x) {
+            if ((unsigned)i < (unsigned)r.V && order_key(x) >= t) c += 1.0;
           });
           if (block_sum<NT>(c, sc) >= (double)p.top_k) key_k = t;
         }
       }
     }
     if (use_p) {
-      for (int b = tid; b < SAMPLE_BINS; b += NT) sc->bins[1][b] = sc->bins[2][b] = 0u;
-      __syncthreads();
-      if (tid == 0) sc->n_list = 0;
-      double zz = 0.0;
       const uint32_t half_mask = (1u << p.mass_half) - 1u;
       const float one = (float)(1u << (2 * p.mass_half));            // the integer that stands for e = 1
       const double unit = 1.0 / (double)one;
-      for_each<NT>(r, [&](int, const float (&x)[Row<T>::VEC]) {
-#pragma unroll
-        for (int j = 0; j < Row<T>::VEC; ++j) {
-          const float e = order_key(x[j]) >= key_k ? __expf(x[j] - mx) : 0.f;
-          const uint32_t q = __float2uint_rn(e * one);
-          const int b = bin_of(x[j], mx);
-          if (q & half_mask) atomicAdd(&sc->bins[1][b], q & half_mask);
-          if (q >> p.mass_half) atomicAdd(&sc->bins[2][b], q >> p.mass_half);
-          zz += (double)q;
+      // Values whose integer is at most `least` need no bin: all V of them together weigh less than (1 - top_p) of the
+      // largest values of the blocks alone, so the nucleus closes before the first of them (and every bin in front of the one
+      // it closes in is complete).  Two thirds of a row of 50 k normal logits.
+      uint32_t least = 0u;
+      if (!use_k) {
+        unsigned long long some = 0ull;
+        for (int b = 0; b < n_blocks; ++b) some += __float2uint_rn(mass_of(sc->blocks.top[b * NT + tid], mx) * one);
+        const double share = (1.0 - (double)p.top_p) * block_sum<NT>((double)some, sc) / (double)p.V;
+        if (share >= 2.0) least = (uint32_t)fmin(share, 1e9) - 1u;
+      }
+      for (int b = tid; b < SAMPLE_BINS; b += NT) sc->bins[1][b] = sc->bins[2][b] = 0u;
+      __syncthreads();
+      if (tid == 0) sc->n_list = 0;
+      unsigned long long zz = 0ull;
+      auto add_mass = [&](float x) {
+        const float e = !use_k || order_key(x) >= key_k ? mass_of(x, mx) : 0.f;
+        const uint32_t q = __float2uint_rn(e * one);
+        zz += q;
+        all_mass += e;
+        if (q > least) {
+          const int b = bin_of(x, mx);
+          atomicAdd(&sc->bins[1][b], q & half_mask);
+          if (q > half_mask) atomicAdd(&sc->bins[2][b], q >> p.mass_half);
         }
-      });
-      const double zq = block_sum<NT>(zz, sc) * unit;     // exact: integers below 2^53
+      };
+      for_each<NT, false>(r, [&](int, float x) { add_mass(x); });
+      for_marked<NT>(r, [&](int, float x) { add_mass(x); });
+      const double zq = block_sum<NT>((double)zz, sc) * unit;     // exact: integers below 2^53
       const double target = (double)p.top_p * zq;
       find_crossing<NT, true>(sc, target, unit, unit * (double)(half_mask + 1u));
       cross = sc->cross_bin;
       const double before = sc->cross_before;
-      for_each<NT>(r, [&](int i0, const float (&x)[Row<T>::VEC]) {
-#pragma unroll
-        for (int j = 0; j < Row<T>::VEC; ++j)
-          if (bin_of(x[j], mx) == cross && order_key(x[j]) >= key_k && __expf(x[j] - mx) > 0.f)
-            list_add(sc, __float_as_uint(__expf(x[j] - mx)), i0 + j);
-      });
+      // rough edges of the bin, wider than it by more than the rounding of mx - x and of the edges themselves (2^-23 of either)
+      const float slack = 1e-6f * (fabsf(mx) + 33.f);
+      if (cross > 0) bin_hi = mx - (float)cross * (1.f / SAMPLE_BINS_PER_UNIT) + slack;
+      if (cross < SAMPLE_BINS - 1) bin_lo = mx - (float)(cross + 1) * (1.f / SAMPLE_BINS_PER_UNIT) - slack;
+      auto add_bin = [&](int i, float x) {
+        if (x >= bin_lo && x <= bin_hi) list_bin_value(sc, x, mx, i, cross, key_k);
+      };
+      for_each<NT, false>(r, add_bin);
+      for_marked<NT>(r, add_bin);
       if (tid == 0) sc->limit = 0xffffffffu;
       __syncthreads();
       const int m = sc->n_list;
@@ -496,38 +670,35 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sample_rows(SamplePar
         for (int b = 29; b >= 0; --b) {
           const uint32_t t = e_min | (1u << b);
           double c = 0.0;
-          for_each<NT>(r, [&](int, const float (&x)[Row<T>::VEC]) {
-#pragma unroll
-            for (int j = 0; j < Row<T>::VEC; ++j) {
-              const float e = order_key(x[j]) >= key_k ? __expf(x[j] - mx) : 0.f;
-              if (__float_as_uint(e) >= t) c += (double)__float2uint_rn(e * one);
-            }
+          for_each<NT, true>(r, [&](int, float x) {
+            const float e = order_key(x) >= key_k ? mass_of(x, mx) : 0.f;
+            if (__float_as_uint(e) >= t) c += (double)__float2uint_rn(e * one);
           });
           if (block_sum<NT>(c, sc) * unit >= target) e_min = t;
         }
         e_min = max(e_min, 1u);
       }
     }
-    auto keep = [&](float x) -> float {      // unnormalised probability of a kept value, 0 for a dropped one
-      const float e = order_key(x) >= key_k ? __expf(x - mx) : 0.f;
-      if (cross < SAMPLE_BINS) {
-        const int b = bin_of(x, mx);
-        return b < cross || (b == cross && __float_as_uint(e) >= e_min) ? e : 0.f;
-      }
-      return __float_as_uint(e) >= e_min ? e : 0.f;
-    };
+    auto keep = [&](float x) { return kept_mass_of(x, mx, cross, e_min, key_k); };
     // ---- masses of the warps' stretches (vocabulary order), then the stretch that holds the target is walked again
-    float acc = 0.f, all = 0.f;
+    float acc = 0.f;
     int cnt = 0;
-    for_each<NT>(r, [&](int, const float (&x)[Row<T>::VEC]) {
-#pragma unroll
-      for (int j = 0; j < Row<T>::VEC; ++j) {
-        const float e = keep(x[j]);
+    auto add_up = [&](auto kept) {
+      auto add = [&](int, float x) {
+        const float e = kept(x);
         acc += e;
         cnt += e > 0.f;
-        if (use_p) all += order_key(x[j]) >= key_k ? __expf(x[j] - mx) : 0.f;
-      }
-    });
+      };
+      for_each<NT, false>(r, add);
+      for_marked<NT>(r, add);
+    };
+    if (!use_k && !use_p) add_up([&](float x) { return mass_of(x, mx); });
+    else if (!use_k)
+      add_up([&](float x) {
+        const float e = mass_of(x, mx);
+        return x < bin_lo ? 0.f : x > bin_hi ? e : kept_mass_slow(x, mx, cross, e_min, 0u);
+      });
+    else add_up(keep);
     for (int o = 16; o; o >>= 1) {
       acc += __shfl_xor_sync(0xffffffffu, acc, o);
       cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
@@ -549,43 +720,50 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sample_rows(SamplePar
     }
     const bool past_end = own < 0;           // u * total rounded up to the total: the last kept token
     if (past_end) own = last;
-    z = use_p ? (float)block_sum<NT>((double)all, sc) : kept_mass;
-    if (warp == own) {
-      const int per = (r.groups + NT / 32 - 1) / (NT / 32);
-      const int g0 = warp * per, g1 = min(r.groups, (warp + 1) * per);
-      int found = 0x7fffffff, last_i = -1;
-      for (int g = g0; g < g1; g += 32) {    // 32 groups at a time: prefix over the lanes, then inside the lane
-        float x[Row<T>::VEC], e[Row<T>::VEC], s = 0.f;
-        const bool on = g + lane < g1;
-        if (on) r.values(g + lane, r.raw(g + lane), x);
+    z = use_p ? (float)block_sum<NT>((double)all_mass, sc) : kept_mass;
+    // the stretch that holds the target, by the whole CTA: 16-byte groups in order, a running sum over them, then inside a group
+    const int w0 = max(own, 0) * per, w1 = own < 0 ? 0 : min(r.groups, w0 + per);
+    int last_i = -1;
+    for (int base = w0; base < w1; base += NT) {      // (one round up to 50 k bf16 values)
+      const int g = base + tid;
+      float x[VEC], e[VEC], s = 0.f;
+      if (g < w1) r.values(g, r.raw(g), x);
 #pragma unroll
-        for (int j = 0; j < Row<T>::VEC; ++j) {
-          e[j] = on ? keep(x[j]) : 0.f;
-          s += e[j];
-          if (e[j] > 0.f) last_i = (g + lane) * Row<T>::VEC - r.lead + j;
-        }
-        float inc = s;
-        for (int o = 1; o < 32; o <<= 1) {
-          const float t = __shfl_up_sync(0xffffffffu, inc, o);
-          if (lane >= o) inc += t;
-        }
-        if (!past_end) {
-          float c = before + (inc - s);
+      for (int j = 0; j < VEC; ++j) {
+        e[j] = g < w1 ? keep(x[j]) : 0.f;
+        s += e[j];
+        if (e[j] > 0.f) last_i = g * VEC - r.lead + j;
+      }
+      float inc = s;
+      for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+      }
+      __syncthreads();
+      if (lane == 31) sc->warp_f[warp] = inc;
+      __syncthreads();
+      float c = before, round = 0.f;
+      for (int w = 0; w < NT / 32; ++w) {
+        if (w == warp) c += round;
+        round += sc->warp_f[w];
+      }
+      c += inc - s;
+      before += round;
+      if (!past_end) {
+        int found = 0x7fffffff;
 #pragma unroll
-          for (int j = 0; j < Row<T>::VEC; ++j) {
-            c += e[j];
-            if (e[j] > 0.f && c > target) found = min(found, (g + lane) * Row<T>::VEC - r.lead + j);
-          }
-          if (__any_sync(0xffffffffu, found != 0x7fffffff)) break;
+        for (int j = VEC - 1; j >= 0; --j) {
+          float upto = c;
+#pragma unroll
+          for (int i = 0; i <= j; ++i) upto += e[i];
+          if (e[j] > 0.f && upto > target) found = g * VEC - r.lead + j;
         }
-        before += __shfl_sync(0xffffffffu, inc, 31);
+        if (found != 0x7fffffff) atomicMin(&sc->chosen, found);
       }
-      for (int o = 16; o; o >>= 1) {
-        found = min(found, __shfl_xor_sync(0xffffffffu, found, o));
-        last_i = max(last_i, __shfl_xor_sync(0xffffffffu, last_i, o));
-      }
-      if (lane == 0) sc->chosen = found != 0x7fffffff ? found : last_i;
     }
+    if (last_i >= 0) atomicMax(&sc->last_kept, last_i);
+    __syncthreads();
+    if (tid == 0 && sc->chosen == 0x7fffffff) sc->chosen = sc->last_kept;
     __syncthreads();
     pick = sc->chosen;
     if (pick < 0 || pick >= p.V) pick = 0;

@@ -120,3 +120,44 @@ def test_bad_arguments_are_refused():
         ops.sample_logits(logits, torch.zeros(3, device=DEV))
     with pytest.raises(QPamError):
         ops.sample_logits(logits, append=True)
+
+
+@pytest.mark.parametrize("n,V,dtype,shift,cfg", [
+    (3, 5, "fp32", 1, dict(top_k=2, top_p=0.9, repetition_penalty=1.3)),           # fewer groups than lanes
+    (150, 333, "bf16", 3, dict(top_k=50, top_p=0.9, repetition_penalty=1.1)),      # 512 threads a row; rows start anywhere
+    (150, 5003, "fp32", 0, dict(top_k=384, top_p=0.95, repetition_penalty=1.1)),   # the largest top-k of the list
+    (4, 5003, "fp32", 2, dict(top_k=385, top_p=0.95, repetition_penalty=1.1)),     # the first beyond it
+    (150, 5003, "bf16", 1, dict(top_k=0, top_p=0.9, repetition_penalty=1.1)),
+    (2, 700001, "fp32", 1, dict(top_k=50, top_p=0.9, repetition_penalty=1.1)),     # a block is more than four groups
+    (2, 700001, "bf16", 0, dict(top_k=0, top_p=0.6, repetition_penalty=1.1)),
+    (4, 50261, "bf16", 0, dict(top_k=0, top_p=0.999, repetition_penalty=1.0)),
+    (4, 4096, "fp32", 0, dict(top_k=0, top_p=1e-6, repetition_penalty=1.0)),       # the largest value alone
+])
+def test_blocks_stretches_and_marks(n, V, dtype, shift, cfg):
+    """Where the passes can go wrong: rows off 16 bytes, blocks of several steps, both widths of a CTA, every route, penalised
+    tokens (the row's largest among them, and tokens on the edges of the warps' stretches)."""
+    g = torch.Generator().manual_seed(V + n)
+    wide = (torch.randn(n, V + 5, generator=g) * 3.0)
+    wide = wide.bfloat16() if dtype == "bf16" else wide
+    logits = wide.to(DEV)[:, shift:shift + V]
+    hist = torch.randint(0, V, (n, 40), generator=g)
+    hist[:, 0] = logits.float().argmax(1).cpu()
+    hist[:, 1], hist[:, 2], hist[:, 3] = 0, V - 1, V // 2
+    hist[:, 4] = hist[:, 0]                       # the penalty applies once
+    u = torch.rand(n, generator=g)
+    cfg = dict(temperature=0.8, **cfg)
+    ids, stats = ops.sample_logits(logits, u.to(DEV), history=hist.to(DEV), return_stats=True, **cfg)
+    _check_rows(logits, hist.numpy(), None, u.numpy(), ids.cpu().numpy(), stats.cpu().numpy(), cfg, count_exact=dtype == "fp32")
+
+
+def test_infinite_temperature_and_masked_logits():
+    V = 1000
+    logits = torch.randn(3, V, device=DEV)
+    u = torch.tensor([0.0, 0.5, 0.9999], device=DEV)
+    ids, stats = ops.sample_logits(logits, u, temperature=float("inf"), history=torch.zeros(3, 4, dtype=torch.int64, device=DEV),
+                                   repetition_penalty=1.1, return_stats=True)
+    assert (stats[:, 2] == V).all() and ids.tolist() == [0, 500, 999]      # uniform over the vocabulary
+    logits[:, 10:] = float("-inf")
+    for cfg in (dict(top_k=20), dict(top_p=0.9), dict()):
+        ids, stats = ops.sample_logits(logits, u, return_stats=True, **cfg)
+        assert (ids < 10).all() and (stats[:, 2] <= 10).all()
