@@ -38,6 +38,8 @@ __global__ void __launch_bounds__(512) k_act_gate_packed(const T* __restrict__ g
                                                          const float* __restrict__ bias,
                                                          const float* __restrict__ beta, T* __restrict__ out,
                                                          int64_t N, int C) {
+  pdl_wait();
+  pdl_trigger();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (C >> 2)) return;
   float b4[4], be4[4];
@@ -81,6 +83,8 @@ __global__ void __launch_bounds__(128) k_residual_cnorm(T* __restrict__ z, const
                                                         const float* __restrict__ res_scale,
                                                         const float* __restrict__ norm_scale, T* __restrict__ xn,
                                                         T* __restrict__ mag_out, int64_t N, int D, float eps) {
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -148,6 +152,8 @@ __global__ void __launch_bounds__(1024) k_residual_cnorm_row(T* __restrict__ z, 
                                                              T* __restrict__ xn, T* __restrict__ mag_out, int D,
                                                              float eps) {
   __shared__ float s_part[32];
+  pdl_wait();
+  pdl_trigger();
   const int64_t row = blockIdx.x;
   const int g = threadIdx.x, groups = D >> 2;
   const bool on = g < groups;
@@ -213,6 +219,8 @@ constexpr int FRONT_U = 1;  // tokens per tile (one keeps the streaming warps at
 // runs beside the streaming warps instead of at their tail.
 template <typename T>
 __global__ void __launch_bounds__(512) k_pam_front(FrontParams fp, int main_threads) {
+  pdl_wait();
+  pdl_trigger();
   const qpam_front_args& a = fp.a;
   const int H = a.H, K = a.K, d = a.d;
   const int gph = d >> 2;
@@ -327,8 +335,8 @@ extern "C" int qpam_act_gate_packed_fwd(const void* gate_up, int64_t ld, int32_t
   const int groups = C / 4, threads = pick_threads(groups), xb = (groups + threads - 1) / threads;
   dim3 grid(xb, (unsigned)std::min<int64_t>((N + 1) / 2, std::max(1, (sm_count() * 2048) / (xb * threads))));
 #define QPAM_AG(T)                                                                                                  \
-  if (beta) k_act_gate_packed<T, true><<<grid, threads, 0, st>>>((const T*)gate_up, ld, bias, beta, (T*)out, N, C); \
-  else k_act_gate_packed<T, false><<<grid, threads, 0, st>>>((const T*)gate_up, ld, bias, beta, (T*)out, N, C);
+  if (beta) launch_after(k_act_gate_packed<T, true>, grid, threads, 0, st, (const T*)gate_up, ld, bias, beta, (T*)out, N, C); \
+  else launch_after(k_act_gate_packed<T, false>, grid, threads, 0, st, (const T*)gate_up, ld, bias, beta, (T*)out, N, C);
   if (dtype == QPAM_F32) { QPAM_AG(float) } else { QPAM_AG(__nv_bfloat16) }
 #undef QPAM_AG
   QPAM_LAUNCH_CHECK("k_act_gate_packed");
@@ -347,18 +355,18 @@ extern "C" int qpam_residual_cnorm_fwd(void* z, const void* delta, const float* 
   if (N <= sm_count() * 8 && D <= 4096) {  // few rows: a CTA per row keeps every SM busy
     const int threads = (D / 4 + 31) / 32 * 32;
     if (dtype == QPAM_F32)
-      k_residual_cnorm_row<float><<<(unsigned)N, threads, 0, st>>>((float*)z, (const float*)delta, res_scale, norm_scale, (float*)xn, (float*)mag, D, eps);
+      launch_after(k_residual_cnorm_row<float>, (unsigned)N, threads, 0, st, (float*)z, (const float*)delta, res_scale, norm_scale, (float*)xn, (float*)mag, D, eps);
     else
-      k_residual_cnorm_row<__nv_bfloat16><<<(unsigned)N, threads, 0, st>>>((__nv_bfloat16*)z, (const __nv_bfloat16*)delta, res_scale, norm_scale,
+      launch_after(k_residual_cnorm_row<__nv_bfloat16>, (unsigned)N, threads, 0, st, (__nv_bfloat16*)z, (const __nv_bfloat16*)delta, res_scale, norm_scale,
                                                                             (__nv_bfloat16*)xn, (__nv_bfloat16*)mag, D, eps);
     QPAM_LAUNCH_CHECK("k_residual_cnorm_row");
     return QPAM_OK;
   }
   const int blocks = (int)std::min<int64_t>((N + 3) / 4, sm_count() * 8);
   if (dtype == QPAM_F32)
-    k_residual_cnorm<float><<<blocks, 128, 0, st>>>((float*)z, (const float*)delta, res_scale, norm_scale, (float*)xn, (float*)mag, N, D, eps);
+    launch_after(k_residual_cnorm<float>, blocks, 128, 0, st, (float*)z, (const float*)delta, res_scale, norm_scale, (float*)xn, (float*)mag, N, D, eps);
   else
-    k_residual_cnorm<__nv_bfloat16><<<blocks, 128, 0, st>>>((__nv_bfloat16*)z, (const __nv_bfloat16*)delta, res_scale, norm_scale,
+    launch_after(k_residual_cnorm<__nv_bfloat16>, blocks, 128, 0, st, (__nv_bfloat16*)z, (const __nv_bfloat16*)delta, res_scale, norm_scale,
                                                             (__nv_bfloat16*)xn, (__nv_bfloat16*)mag, N, D, eps);
   QPAM_LAUNCH_CHECK("k_residual_cnorm");
   return QPAM_OK;
@@ -383,8 +391,8 @@ extern "C" int qpam_pam_front_fwd(const qpam_front_args* a, void* stream) {
   const int gate_threads = std::min((FRONT_U * a->H * a->K + 31) / 32 * 32, 128);
   const int threads = main_threads + gate_threads;
   const int grid = (int)std::min<int64_t>(((int64_t)a->B * a->T + FRONT_U - 1) / FRONT_U, (sm_count() * 2048) / threads);
-  if (a->io_dtype == QPAM_F32) k_pam_front<float><<<grid, threads, 0, st>>>(fp, main_threads);
-  else k_pam_front<__nv_bfloat16><<<grid, threads, 0, st>>>(fp, main_threads);
+  if (a->io_dtype == QPAM_F32) launch_after(k_pam_front<float>, grid, threads, 0, st, fp, main_threads);
+  else launch_after(k_pam_front<__nv_bfloat16>, grid, threads, 0, st, fp, main_threads);
   QPAM_LAUNCH_CHECK("k_pam_front");
   return QPAM_OK;
 }

@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(256) k_decode_step(DecodeParams p) {
   constexpr int PASSES = D / RPP;
   __shared__ float2 sq[D], sk[D], sv[D];
   const int tid = threadIdx.x;
+  pdl_wait();
   const int seq = blockIdx.x / p.H, h = blockIdx.x - seq * p.H;
   const int slot = p.slot_ids[seq];
   const size_t vb = ((size_t)seq * p.H + h) * D * 2;
@@ -145,6 +146,10 @@ __device__ __forceinline__ void bulk_store(void* gdst, const void* smem_src, uin
                : "memory");
 }
 
+__device__ __forceinline__ void bulk_prefetch(const void* gsrc, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes) : "memory");
+}
+
 constexpr int DEC_BULK_STATE_BYTES = 64 * 64 * 2 * 2;  // one bf16 state
 
 template <typename T>
@@ -155,14 +160,22 @@ __global__ void __launch_bounds__(256) k_decode_step_bulk(DecodeParams p) {
   __shared__ __align__(8) uint64_t bar[QPAM_MAX_STATES];   // one per state: work on state k starts when it has landed
   const int tid = threadIdx.x;
   const int seq = blockIdx.x / p.H, h = blockIdx.x - seq * p.H;
-  const int slot = p.slot_ids[seq];
+  const size_t state_elems = (size_t)D * D * 2;
+  __nv_bfloat16* pool = reinterpret_cast<__nv_bfloat16*>(p.pool);
+  // While the predecessor (the kernel that forms q, k, v) ends, the states are asked into L2.  Nothing is read: should something
+  // still write the slot or its index, it is the wait that orders the loads behind it.
+  if (tid < p.K) {
+    const int hint = __ldcg(p.slot_ids + seq);
+    if (hint >= 0 && hint < p.n_slots)
+      bulk_prefetch(pool + ((((size_t)hint * p.L + p.layer) * p.K + tid) * p.H + h) * state_elems, DEC_BULK_STATE_BYTES);
+  }
+  pdl_wait();
+  const int slot = __ldcg(p.slot_ids + seq);
   const size_t vb = ((size_t)seq * p.H + h) * D * 2;
   if (slot < 0 || slot >= p.n_slots) {        // padded / retired entry (whole CTA): no state, but a defined output -- the row goes on
     if (tid < D) IO<T>::st2(reinterpret_cast<T*>(p.y) + vb + 2 * tid, make_float2(0.f, 0.f));      // through the step to an id
     return;
   }
-  __nv_bfloat16* pool = reinterpret_cast<__nv_bfloat16*>(p.pool);
-  const size_t state_elems = (size_t)D * D * 2;
   const size_t base = (((size_t)slot * p.L + p.layer) * p.K) * p.H + h;  // + k * H per state
   if (tid == 0) {
     for (int k = 0; k < p.K; ++k) umma::mbar_init(&bar[k], 1);
@@ -249,7 +262,7 @@ static int launch_decode_bulk(const DecodeParams& p, cudaStream_t st) {
   auto kern = k_decode_step_bulk<T>;
   const int rc = allow_smem(reinterpret_cast<const void*>(kern), smem);
   if (rc) return rc;
-  kern<<<p.n * p.H, 256, smem, st>>>(p);
+  launch_after(kern, p.n * p.H, 256, smem, st, p);
   QPAM_LAUNCH_CHECK("k_decode_step_bulk");
   return QPAM_OK;
 }
@@ -263,7 +276,7 @@ template <int D, typename ST, typename T>
 static int launch_decode(const DecodeParams& p, cudaStream_t st) {
   constexpr int NC = StateVec<ST>::NC;
   constexpr int NTH = (D * D / NC) < 256 ? (D * D / NC) : 256;
-  k_decode_step<D, ST, T><<<p.n * p.H, NTH, 0, st>>>(p);
+  launch_after(k_decode_step<D, ST, T>, p.n * p.H, NTH, 0, st, p);
   QPAM_LAUNCH_CHECK("k_decode_step");
   return QPAM_OK;
 }
