@@ -146,10 +146,6 @@ __device__ __forceinline__ void bulk_store(void* gdst, const void* smem_src, uin
                : "memory");
 }
 
-__device__ __forceinline__ void bulk_prefetch(const void* gsrc, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes) : "memory");
-}
-
 constexpr int DEC_BULK_STATE_BYTES = 64 * 64 * 2 * 2;  // one bf16 state
 
 template <typename T>
@@ -167,7 +163,7 @@ __global__ void __launch_bounds__(256) k_decode_step_bulk(DecodeParams p) {
   if (tid < p.K) {
     const int hint = __ldcg(p.slot_ids + seq);
     if (hint >= 0 && hint < p.n_slots)
-      bulk_prefetch(pool + ((((size_t)hint * p.L + p.layer) * p.K + tid) * p.H + h) * state_elems, DEC_BULK_STATE_BYTES);
+      umma::bulk_prefetch_l2(pool + ((((size_t)hint * p.L + p.layer) * p.K + tid) * p.H + h) * state_elems, DEC_BULK_STATE_BYTES);
   }
   pdl_wait();
   const int slot = __ldcg(p.slot_ids + seq);

@@ -47,16 +47,14 @@ __device__ __forceinline__ void issue_rows(uint32_t t, uint32_t acc, uint32_t x_
   using namespace umma;
   constexpr uint32_t id = idesc_bf16(128, 64, false, true);
   constexpr uint32_t idn = idesc_bf16_nega(128, 64, false, true);
+  constexpr uint32_t id2 = idesc_bf16(128, 128, false, true);      // (both planes of X2 as one B operand: N blocks 16 KB apart)
   const uint32_t x_i = x_r + 16384;
 #pragma unroll
   for (int kk = 0; kk < 8; ++kk)
-    mma_bf16_ts(acc, t + 16 * kk, smem_desc_sw128(x_r + kk * 2048, 16, 1024), id, kk > 0);
+    mma_bf16_ts(acc, t + 16 * kk, smem_desc_sw128(x_r + kk * 2048, 16384, 1024), id2, kk > 0);
 #pragma unroll
   for (int kk = 0; kk < 8; ++kk)
     mma_bf16_ts(acc, t + 16 * kk + 8, smem_desc_sw128(x_i + kk * 2048, 16, 1024), idn, true);
-#pragma unroll
-  for (int kk = 0; kk < 8; ++kk)
-    mma_bf16_ts(acc + 64, t + 16 * kk, smem_desc_sw128(x_i + kk * 2048, 16, 1024), id, kk > 0);
 #pragma unroll
   for (int kk = 0; kk < 8; ++kk)
     mma_bf16_ts(acc + 64, t + 16 * kk + 8, smem_desc_sw128(x_r + kk * 2048, 16, 1024), id, true);
@@ -186,11 +184,12 @@ __device__ __forceinline__ void pass_b16(uint32_t tl, int c0, int q4, int r, con
 }
 
 // carried state (fp32 [64][64] re, im) -> bf16 planes of a slot; a warp's 512 consecutive bytes are one row
-__device__ __forceinline__ void stage_state(unsigned char* slot, const float2* __restrict__ state, int tid) {
+__device__ __forceinline__ void state_load(float4 (&v)[4], const float2* state, int tid) {
   const float4* sg = reinterpret_cast<const float4*>(state);
-  float4 v[4];
 #pragma unroll
   for (int it = 0; it < 4; ++it) v[it] = ld_dependent(sg + tid + BT * it);
+}
+__device__ __forceinline__ void state_stage(unsigned char* slot, const float4 (&v)[4], int tid) {
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
     const int i = (tid + BT * it) >> 5, c = tid & 31;      // row i, columns 2c and 2c + 1
@@ -280,6 +279,10 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
       tma_load_2d(TY + kb * 16384, &maps.dy, &bars[B_VY], dx + kb * 64, dr);
       tma_load_2d(TV + kb * 16384, &maps.v, &bars[B_VY], kb * 64, row0);
     }
+    if (has_s) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) bulk_prefetch_l2(p.states + state_base(p, k, h, L.slot0 + L.c, TD), 32768);
+    }
     mbar_arrive_expect_tx(&bars[B_QK], 4 * 16384);
 #pragma unroll
     for (int kb = 0; kb < 2; ++kb) {
@@ -328,9 +331,14 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   const uint32_t q_r = smem_u32(TQ), k_r = smem_u32(TK), v_r = smem_u32(TV), y_r = smem_u32(TY), sl = smem_u32(SL);
   const bool issuer = warp == 0 && elect_one();
   // the states entering the chunk, while the tiles are on their way
-  if (has_s) {
+  if (has_s) {          // (the next state's loads in flight while one is staged)
+    float4 sv[2][4];
+    state_load(sv[0], p.states + state_base(p, 0, h, L.slot0 + L.c, TD), tid);
 #pragma unroll
-    for (int k = 0; k < K; ++k) stage_state(SL + k * 16384, p.states + state_base(p, k, h, L.slot0 + L.c, TD), tid);
+    for (int k = 0; k < K; ++k) {
+      if (k + 1 < K) state_load(sv[(k + 1) & 1], p.states + state_base(p, k + 1, h, L.slot0 + L.c, TD), tid);
+      state_stage(SL + k * 16384, sv[k & 1], tid);
+    }
   }
   // de-interleave dy and v, start X; then q and k, start Y
   bool ok = mbar_wait(&bars[B_VY], 0, 251);
@@ -367,6 +375,10 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
 #pragma unroll
   for (int k = 0; k < K; ++k) ar[k] = tb.A[k * TC + r];
 
+  if (tid == 0 && has_ds) {      // (a hint: the reverse carry may still be writing them)
+#pragma unroll
+    for (int k = 0; k < K; ++k) bulk_prefetch_l2(p.dstates + state_base(p, k, h, L.slot0 + L.c + 1, TD), 32768);
+  }
   // ---- pass A: rows t
   float2 wk[K], zs[K];
 #pragma unroll
@@ -455,7 +467,9 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   __syncthreads();
   const bool storing = warp >= 8 && lane == 0 && len == TC && ok;
   if (storing) store_box(&maps.dq, SL, warp - 8, row0);
-  auto stage_grad = [&](int k) { stage_state(SL + ((k + 2) & 3) * 16384, p.dstates + state_base(p, k, h, L.slot0 + L.c + 1, TD), tid); };
+  float4 gv[2][4];
+  auto load_grad = [&](int k) { state_load(gv[k & 1], p.dstates + state_base(p, k, h, L.slot0 + L.c + 1, TD), tid); };
+  auto stage_grad = [&](int k) { state_stage(SL + ((k + 2) & 3) * 16384, gv[k & 1], tid); };
   // the gradients of the states and the anchors are the reverse carry's; everything above is the call's inputs and the forward
   // states, which are older (see launch_after)
   pdl_wait();
@@ -465,8 +479,12 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
     an1 = __ldcg(ap + lane + 32);
   }
   if (has_ds) {
+    load_grad(0);
+    load_grad(1);
     stage_grad(0);
+    if (K > 2) load_grad(2);
     stage_grad(1);
+    if (K > 3) load_grad(3);
   }
   if (K > 2) {
     if (storing) tma_store_wait_read();

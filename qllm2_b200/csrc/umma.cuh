@@ -115,6 +115,10 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
                : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// Asks `bytes` (a multiple of 16, 16-byte aligned) into L2.  A hint: nothing is read.
+__device__ __forceinline__ void bulk_prefetch_l2(const void* gsrc, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes) : "memory");
+}
 // TMA store of one box from shared memory (128-byte swizzled like the loads) to global memory; coordinates must not
 // be negative, x times the element size a multiple of 16 bytes.  The issuing thread commits the group and, before the
 // shared-memory block is written again, waits until the engine has read it.
