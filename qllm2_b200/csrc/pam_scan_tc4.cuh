@@ -22,10 +22,10 @@
 //
 //   TMEM        [0,128)              [128,256)           [256,384)            [384,512)
 //   scores      X real               X imaginary         Y real               Y imaginary
-//   dq          G X (bf16)           dq accumulator      (S^0)^H dy           (S^1)^H dy     (then states 2, 3)
+//   dq          G X (bf16)           dq accumulator      (S^0)^H dy           (S^1)^H dy     (then state 2 in [0,128), 3 in [256,384))
 //   scores      X^H real             X^H imaginary       Y^H real             Y^H imaginary
 //   dk, dv      conj(G X)^T (bf16)   dk accumulator      (G conj Y)^T (bf16)  dv accumulator
-//   carried     (dS^0)^H v                               dS^0 k                              (then states 1, 2; then 3)
+//   carried     (dS^0)^H v           (dS^1)^H v          dS^0 k               dS^1 k         (then states 2, 3)
 //
 // Decay: D factors as e^{A_t - A_m} e^{A_m - A_s} around the middle of the chunk; a state whose chunk decays by more than
 // e^-80 takes one exponential per score instead (see pam_scan_tc2.cuh).
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   float2* dcp = reinterpret_cast<float2*>(tb.row + KMAX * TC);      // [4 channel groups][K][128] shares of dc
   float* kdp = reinterpret_cast<float*>(SL + 2 * 16384);            // [4][K][128] shares of Re<k, dk>, once no MMA reads the slots
   uint64_t* bars = reinterpret_cast<uint64_t*>(dcp + 4 * KMAX * TC);
-  enum { B_VY, B_QK, B_SA, B_SB, B_DQ, B_U2, B_DKV, B_C0, B_C1, B_C2, N_BARS };
+  enum { B_VY, B_QK, B_SA, B_SB, B_DQ, B_U2, B_U3, B_DKV, B_C0, B_C1, B_C2, B_C3, N_BARS };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + N_BARS);
   int* failed = reinterpret_cast<int*>(tmem_slot + 1);
   float* wsum = reinterpret_cast<float*>(failed + 1);               // [K][4]
@@ -331,14 +331,12 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   const uint32_t q_r = smem_u32(TQ), k_r = smem_u32(TK), v_r = smem_u32(TV), y_r = smem_u32(TY), sl = smem_u32(SL);
   const bool issuer = warp == 0 && elect_one();
   // the states entering the chunk, while the tiles are on their way
-  if (has_s) {          // (the next state's loads in flight while one is staged)
-    float4 sv[2][4];
-    state_load(sv[0], p.states + state_base(p, 0, h, L.slot0 + L.c, TD), tid);
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      if (k + 1 < K) state_load(sv[(k + 1) & 1], p.states + state_base(p, k + 1, h, L.slot0 + L.c, TD), tid);
-      state_stage(SL + k * 16384, sv[k & 1], tid);
-    }
+  // the carried states of two states are in flight while the tiles are de-interleaved, the others while those are staged
+  float4 sv[2][4];
+  auto load_state = [&](int k) { state_load(sv[k & 1], p.states + state_base(p, k, h, L.slot0 + L.c, TD), tid); };
+  if (has_s) {
+    load_state(0);
+    load_state(1);
   }
   // de-interleave dy and v, start X; then q and k, start Y
   bool ok = mbar_wait(&bars[B_VY], 0, 251);
@@ -353,6 +351,12 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
     __syncthreads();
     if (issuer) bw_issue_scores(tmem, y_r, v_r);
     __syncwarp();
+    if (has_s) {
+      state_stage(SL, sv[0], tid);
+      if (K > 2) load_state(2);
+      state_stage(SL + 16384, sv[1], tid);
+      if (K > 3) load_state(3);
+    }
     ok = mbar_wait(&bars[B_QK], 0, 252) && ok;
     tile = tid < 256 ? TQ : TK;
     deint_read(tile, row, hb, ra);
@@ -365,6 +369,10 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
       mma_commit(&bars[B_SA]);
     }
     __syncwarp();
+    if (has_s) {
+      if (K > 2) state_stage(SL + 2 * 16384, sv[0], tid);
+      if (K > 3) state_stage(SL + 3 * 16384, sv[1], tid);
+    }
   }
   const int q4 = warp & 3, cq = warp >> 2;
   const int r = q4 * 32 + lane;                                   // this thread's row (TMEM lane)
@@ -406,6 +414,10 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
       issue_state<true>(tmem + 384, y_r, sl + 16384);
     }
     mma_commit(&bars[B_DQ]);
+    if (K > 2 && has_s && mbar_wait(&bars[B_DQ], 0, 254)) {        // the packed scores have been consumed: state 2 takes their columns
+      issue_state<true>(tmem, y_r, sl + 2 * 16384);
+      mma_commit(&bars[B_U2]);
+    }
   }
   __syncwarp();
   ok = mbar_wait(&bars[B_DQ], 0, 254) && ok;
@@ -416,20 +428,21 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
     if (has_s) {
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        if (k == 2) {                       // both accumulators have been read: states 2 and 3
+        if (K > 3 && k == 1) {              // state 0's accumulator has been read: state 3 takes it
           tc_fence_before();
           __syncthreads();
           if (issuer) {
             tc_fence_after();
-            issue_state<true>(tmem + 256, y_r, sl + 2 * 16384);
-            if (K > 3) issue_state<true>(tmem + 384, y_r, sl + 3 * 16384);
-            mma_commit(&bars[B_U2]);
+            issue_state<true>(tmem + 256, y_r, sl + 3 * 16384);
+            mma_commit(&bars[B_U3]);
           }
           __syncwarp();
-          ok = mbar_wait(&bars[B_U2], 0, 255) && ok;
+        }
+        if (k >= 2) {
+          ok = mbar_wait(&bars[k == 2 ? B_U2 : B_U3], 0, 255) && ok;
           tc_fence_after();
         }
-        const uint32_t at = tl + 256 + 128 * (k & 1) + 16 * cq;
+        const uint32_t at = tl + (k == 2 ? 0 : k == 1 ? 384 : 256) + 16 * cq;
         float ur[16], ui[16], xr[16], xi[16];
         tmem_ld16x2(at, ur, at + 64, ui);
         row16(TQ, r, cq, xr, xi);
@@ -535,28 +548,25 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
 #pragma unroll
     for (int k = 0; k < K; ++k) cs[k] *= ck[k];
     if (has_ds) {
+      // a state's products run while the one before it is read: state k + 1 is issued once every warp has read what holds its
+      // columns (dk and dv for state 1, state k - 1 after that)
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        if (k == 1 || k == 3) {                     // every accumulator has been read: the next states
+        if (k + 1 < K) {
           tc_fence_before();
           __syncthreads();
           if (issuer) {
             tc_fence_after();
-            issue_state<true>(tmem, v_r, sl + ((k + 2) & 3) * 16384);
-            issue_state<false>(tmem + 256, k_r, sl + ((k + 2) & 3) * 16384);
-            if (k == 1 && K > 2) {
-              issue_state<true>(tmem + 128, v_r, sl);
-              issue_state<false>(tmem + 384, k_r, sl);
-            }
-            mma_commit(&bars[k == 1 ? B_C1 : B_C2]);
+            const uint32_t s1 = sl + ((k + 3) & 3) * 16384, c1 = tmem + 128 * ((k + 1) & 1);
+            issue_state<true>(c1, v_r, s1);
+            issue_state<false>(c1 + 256, k_r, s1);
+            mma_commit(&bars[B_C1 + k]);
           }
           __syncwarp();
         }
-        if (k != 2) {
-          ok = mbar_wait(&bars[k == 0 ? B_C0 : k == 1 ? B_C1 : B_C2], 0, 258) && ok;
-          tc_fence_after();
-        }
-        const uint32_t at = tl + (k == 2 ? 128u : 0u) + 16 * cq;
+        ok = mbar_wait(&bars[B_C0 + k], 0, 258) && ok;
+        tc_fence_after();
+        const uint32_t at = tl + 128 * (k & 1) + 16 * cq;
         const float e = __expf(fminf(0.f, tb.A[k * TC + TC - 1] - ar[k]));
         float ur[16], ui[16];
         {
