@@ -273,12 +273,8 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
     tc_fence_after();
     constexpr uint32_t idesc = idesc_bf16(128, 64, true, true);
     const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk)      // D1 = A^T Br: k-step = 16 tokens = 2048 bytes in either operand
-      mma_bf16(tmem, smem_desc_sw128(a0 + kk * 2048, 16384, 1024), smem_desc_sw128(b0 + kk * 2048, 16, 1024), idesc, kk > 0);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk)      // D2 = A^T Bi
-      mma_bf16(tmem + 64, smem_desc_sw128(a0 + kk * 2048, 16384, 1024), smem_desc_sw128(b0 + 16384 + kk * 2048, 16, 1024), idesc, kk > 0);
+    mma_run(tmem, smem_desc_sw128(a0, 16384, 1024), smem_desc_sw128(b0, 16, 1024), 128, 128, idesc, 8, false);      // D1 = A^T Br: k-step = 16 tokens = 2048 bytes in either operand
+    mma_run(tmem + 64, smem_desc_sw128(a0, 16384, 1024), smem_desc_sw128(b0 + 16384, 16, 1024), 128, 128, idesc, 8, false);      // D2 = A^T Bi
     mma_commit(&bar[0]);
   }
   __syncwarp();
@@ -443,12 +439,8 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
       tc_fence_after();
       constexpr uint32_t idesc = idesc_bf16(128, 64, true, true);
       const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
-#pragma unroll
-      for (int kk = 0; kk < 8; ++kk)      // D1 = A^T Br
-        mma_bf16(tmem, smem_desc_sw128(a0 + kk * 2048, 16384, 1024), smem_desc_sw128(b0 + kk * 2048, 16, 1024), idesc, kk > 0);
-#pragma unroll
-      for (int kk = 0; kk < 8; ++kk)      // D2 = A^T Bi
-        mma_bf16(tmem + 64, smem_desc_sw128(a0 + kk * 2048, 16384, 1024), smem_desc_sw128(b0 + 16384 + kk * 2048, 16, 1024), idesc, kk > 0);
+      mma_run(tmem, smem_desc_sw128(a0, 16384, 1024), smem_desc_sw128(b0, 16, 1024), 128, 128, idesc, 8, false);      // D1 = A^T Br
+      mma_run(tmem + 64, smem_desc_sw128(a0, 16384, 1024), smem_desc_sw128(b0 + 16384, 16, 1024), 128, 128, idesc, 8, false);      // D2 = A^T Bi
       mma_commit(&bar[k]);
     }
     __syncwarp();

@@ -82,53 +82,32 @@ __device__ __forceinline__ void bw_issue_scores(uint32_t slot, uint32_t a_r, uin
   using namespace umma;
   constexpr uint32_t id = idesc_bf16(128, 128, false, false);
   constexpr uint32_t idn = idesc_bf16_nega(128, 128, false, false);
-  const uint32_t a_i = a_r + 16384, b_i = b_r + 16384;
-#pragma unroll
-  for (int kk = 0; kk < 4; ++kk)
-    mma_bf16(slot, smem_desc_sw128(a_r + kk * 32, 16, 1024), smem_desc_sw128(b_r + kk * 32, 16, 1024), id, kk > 0);
-#pragma unroll
-  for (int kk = 0; kk < 4; ++kk)
-    mma_bf16(slot, smem_desc_sw128(a_i + kk * 32, 16, 1024), smem_desc_sw128(b_i + kk * 32, 16, 1024), id, true);
+  const uint64_t ar = smem_desc_sw128(a_r, 16, 1024), ai = smem_desc_sw128(a_r + 16384, 16, 1024);
+  const uint64_t br = smem_desc_sw128(b_r, 16, 1024), bi = smem_desc_sw128(b_r + 16384, 16, 1024);
+  mma_run(slot, ar, br, 2, 2, id, 4, false);
+  mma_run(slot, ai, bi, 2, 2, id, 4, true);
   if (!IMAG_SWAPPED) {
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-      mma_bf16(slot + 128, smem_desc_sw128(a_i + kk * 32, 16, 1024), smem_desc_sw128(b_r + kk * 32, 16, 1024), id, kk > 0);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-      mma_bf16(slot + 128, smem_desc_sw128(a_r + kk * 32, 16, 1024), smem_desc_sw128(b_i + kk * 32, 16, 1024), idn, true);
+    mma_run(slot + 128, ai, br, 2, 2, id, 4, false);
+    mma_run(slot + 128, ar, bi, 2, 2, idn, 4, true);
   } else {
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-      mma_bf16(slot + 128, smem_desc_sw128(a_r + kk * 32, 16, 1024), smem_desc_sw128(b_i + kk * 32, 16, 1024), idn, kk > 0);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-      mma_bf16(slot + 128, smem_desc_sw128(a_i + kk * 32, 16, 1024), smem_desc_sw128(b_r + kk * 32, 16, 1024), id, true);
+    mma_run(slot + 128, ar, bi, 2, 2, idn, 4, false);
+    mma_run(slot + 128, ai, br, 2, 2, id, 4, true);
   }
 }
 
 // TMEM column of the packed bf16 scores of k-step kk (16 score columns = 8 TMEM columns): the thread that
-// owns score columns [32 cq, 32 cq + 32) of a row writes  Tr(2cq) Tr(2cq+1) Ti(2cq) Ti(2cq+1)  over them.
-__device__ __forceinline__ uint32_t bw_tr_col(int kk) { return (uint32_t)(32 * (kk >> 1) + 8 * (kk & 1)); }
-__device__ __forceinline__ uint32_t bw_ti_col(int kk) { return bw_tr_col(kk) + 16u; }
+// owns score columns [32 cq, 32 cq + 32) of a row writes  Tr(2cq) Tr(2cq+1) Ti(2cq) Ti(2cq+1)  over them, so the real parts
+// are at 0, 8, 32, 40, 64, ... and the imaginary parts 16 further on.
 
-// acc = T X2 : out_r = Tr x2r - Ti x2i, out_i = Tr x2i + Ti x2r   (X2 planes MN-major, K = 128 tokens)
+// acc = T X2 : out_r = Tr x2r - Ti x2i, out_i = Tr x2i + Ti x2r   (X2 planes MN-major, K = 128 tokens).  The real scores multiply
+// both planes at once (one B operand of 128 columns, its halves 16 KB apart).
 __device__ __forceinline__ void bw_issue_out(uint32_t slot, uint32_t x_r, bool accumulate = false) {
   using namespace umma;
-  constexpr uint32_t id = idesc_bf16(128, 64, false, true);
+  constexpr uint32_t id = idesc_bf16(128, 64, false, true), id2 = idesc_bf16(128, 128, false, true);
   constexpr uint32_t idn = idesc_bf16_nega(128, 64, false, true);
-  const uint32_t x_i = x_r + 16384, Or = slot + 128, Oi = slot + 192;
-#pragma unroll
-  for (int kk = 0; kk < 8; ++kk)
-    mma_bf16_ts(Or, slot + bw_tr_col(kk), smem_desc_sw128(x_r + kk * 2048, 16, 1024), id, accumulate || kk > 0);
-#pragma unroll
-  for (int kk = 0; kk < 8; ++kk)
-    mma_bf16_ts(Or, slot + bw_ti_col(kk), smem_desc_sw128(x_i + kk * 2048, 16, 1024), idn, true);
-#pragma unroll
-  for (int kk = 0; kk < 8; ++kk)
-    mma_bf16_ts(Oi, slot + bw_tr_col(kk), smem_desc_sw128(x_i + kk * 2048, 16, 1024), id, accumulate || kk > 0);
-#pragma unroll
-  for (int kk = 0; kk < 8; ++kk)
-    mma_bf16_ts(Oi, slot + bw_ti_col(kk), smem_desc_sw128(x_r + kk * 2048, 16, 1024), id, true);
+  mma_run_ts(slot + 128, slot, smem_desc_sw128(x_r, 16384, 1024), 8, 24, 128, id2, 8, accumulate);
+  mma_run_ts(slot + 128, slot + 16, smem_desc_sw128(x_r + 16384, 16, 1024), 8, 24, 128, idn, 8, true);
+  mma_run_ts(slot + 192, slot + 16, smem_desc_sw128(x_r, 16, 1024), 8, 24, 128, id, 8, true);
 }
 
 // acc (+)= A1 (.) state planes [64 rows i][64 j]:  OP_H == false: out[r][i] = sum_j a[r][j] S[i][j];
@@ -136,30 +115,11 @@ __device__ __forceinline__ void bw_issue_out(uint32_t slot, uint32_t x_r, bool a
 template <bool OP_H>
 __device__ __forceinline__ void bw_issue_state(uint32_t slot, uint32_t a_r, uint32_t s_r, bool accumulate) {
   using namespace umma;
-  const uint32_t a_i = a_r + 16384, s_i = s_r + 8192, Or = slot + 128, Oi = slot + 192;
-  if (!OP_H) {
-    constexpr uint32_t k3 = idesc_bf16(128, 64, false, false), k3n = idesc_bf16_nega(128, 64, false, false);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      const uint64_t ar = smem_desc_sw128(a_r + kk * 32, 16, 1024), ai = smem_desc_sw128(a_i + kk * 32, 16, 1024);
-      const uint64_t sr = smem_desc_sw128(s_r + kk * 32, 16, 1024), si = smem_desc_sw128(s_i + kk * 32, 16, 1024);
-      mma_bf16(Or, ar, sr, k3, accumulate || kk > 0);    // + a_r S_r^T
-      mma_bf16(Or, ai, si, k3n, true);                   // - a_i S_i^T
-      mma_bf16(Oi, ar, si, k3, accumulate || kk > 0);    // + a_r S_i^T
-      mma_bf16(Oi, ai, sr, k3, true);                    // + a_i S_r^T
-    }
-  } else {
-    constexpr uint32_t k3 = idesc_bf16(128, 64, false, true), k3n = idesc_bf16_nega(128, 64, false, true);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      const uint64_t ar = smem_desc_sw128(a_r + kk * 32, 16, 1024), ai = smem_desc_sw128(a_i + kk * 32, 16, 1024);
-      const uint64_t sr = smem_desc_sw128(s_r + kk * 2048, 16, 1024), si = smem_desc_sw128(s_i + kk * 2048, 16, 1024);
-      mma_bf16(Or, ar, sr, k3, accumulate || kk > 0);    // + a_r S_r
-      mma_bf16(Or, ai, si, k3, true);                    // + a_i S_i
-      mma_bf16(Oi, ai, sr, k3, accumulate || kk > 0);    // + a_i S_r
-      mma_bf16(Oi, ar, si, k3n, true);                   // - a_r S_i
-    }
-  }
+  const uint64_t ar = smem_desc_sw128(a_r, 16, 1024), ai = smem_desc_sw128(a_r + 16384, 16, 1024);
+  const uint64_t sr = smem_desc_sw128(s_r, 16, 1024), si = smem_desc_sw128(s_r + 8192, 16, 1024);
+  constexpr uint32_t id = idesc_bf16(128, 64, false, OP_H), idn = idesc_bf16_nega(128, 64, false, OP_H);
+  if (!OP_H) mma_run_complex(slot + 128, slot + 192, ar, ai, sr, si, 2, 2, id, idn, id, true, 4, accumulate);      // a_r S_r - a_i S_i; a_r S_i + a_i S_r
+  else mma_run_complex(slot + 128, slot + 192, ar, ai, sr, si, 2, 128, id, id, idn, false, 4, accumulate);         // a_r S_r + a_i S_i; a_i S_r - a_r S_i
 }
 
 // ---- epilogue 1: decay-masked scores of this thread's row, columns [32 cb, 32 cb + 32), as packed bf16 ------

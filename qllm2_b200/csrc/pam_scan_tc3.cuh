@@ -125,20 +125,7 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   const uint32_t x_r = smem_u32(RC), x_i = x_r + 16384;
   if (warp == 0 && elect_one()) {
     tc_fence_after();
-    constexpr uint32_t id = idesc_bf16(128, 128, false, false);
-    constexpr uint32_t idn = idesc_bf16_nega(128, 128, false, false);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-      mma_bf16(tmem, smem_desc_sw128(a_r + kk * 32, 16, 1024), smem_desc_sw128(b_r + kk * 32, 16, 1024), id, kk > 0);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-      mma_bf16(tmem, smem_desc_sw128(a_i + kk * 32, 16, 1024), smem_desc_sw128(b_i + kk * 32, 16, 1024), id, true);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-      mma_bf16(tmem + 128, smem_desc_sw128(a_i + kk * 32, 16, 1024), smem_desc_sw128(b_r + kk * 32, 16, 1024), id, kk > 0);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-      mma_bf16(tmem + 128, smem_desc_sw128(a_r + kk * 32, 16, 1024), smem_desc_sw128(b_i + kk * 32, 16, 1024), idn, true);
+    bw_issue_scores(tmem, a_r, b_r);
     mma_commit(&bars[1]);
   }
   __syncwarp();
@@ -263,18 +250,11 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
     tc_fence_after();
     constexpr uint32_t id = idesc_bf16(128, 64, false, true);        // A: TMEM, B: MN-major plane
     constexpr uint32_t idn = idesc_bf16_nega(128, 64, false, true);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk)
-      mma_bf16_ts(Or, Tr + kk * 8, smem_desc_sw128(x_r + kk * 2048, 16, 1024), id, kk > 0);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk)
-      mma_bf16_ts(Or, Ti + kk * 8, smem_desc_sw128(x_i + kk * 2048, 16, 1024), idn, true);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk)
-      mma_bf16_ts(Oi, Tr + kk * 8, smem_desc_sw128(x_i + kk * 2048, 16, 1024), id, kk > 0);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk)
-      mma_bf16_ts(Oi, Ti + kk * 8, smem_desc_sw128(x_r + kk * 2048, 16, 1024), id, true);
+    const uint64_t xr = smem_desc_sw128(x_r, 16, 1024), xi = smem_desc_sw128(x_i, 16, 1024);
+    mma_run_ts(Or, Tr, xr, 8, 8, 128, id, 8, false);
+    mma_run_ts(Or, Ti, xi, 8, 8, 128, idn, 8, true);
+    mma_run_ts(Oi, Tr, xi, 8, 8, 128, id, 8, false);
+    mma_run_ts(Oi, Ti, xr, 8, 8, 128, id, 8, true);
     mma_commit(&bars[2]);
   }
   __syncwarp();

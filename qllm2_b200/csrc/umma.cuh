@@ -309,6 +309,43 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
       : "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate)
       : "memory");
 }
+// n MMAs of one accumulator, operands advancing by da, db (descriptor units of 16 bytes) each.  A loop, not n copies: the
+// descriptors' arithmetic made the issue of a chunk job's products tens of KB of code that one thread walks once, missing the
+// instruction cache at every line.
+__device__ __forceinline__ void mma_run(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t da, uint32_t db, uint32_t idesc, int n, bool accumulate) {
+#pragma unroll 1
+  for (int i = 0; i < n; ++i) {
+    mma_bf16(d_tmem, a, b, idesc, accumulate);
+    accumulate = true;
+    a += da;
+    b += db;
+  }
+}
+// the same with A in tensor memory, its column advancing by da0 and da1 in turn
+__device__ __forceinline__ void mma_run_ts(uint32_t d_tmem, uint32_t a, uint64_t b, uint32_t da0, uint32_t da1, uint32_t db, uint32_t idesc, int n,
+                                        bool accumulate) {
+#pragma unroll 1
+  for (int i = 0; i < n; ++i) {
+    mma_bf16_ts(d_tmem, a, b, idesc, accumulate);
+    accumulate = true;
+    a += (i & 1) ? da1 : da0;
+    b += db;
+  }
+}
+// Complex product of interleaved chains: per step  r += ar br, r += ai bi (id_rr, id_ii), i += ax bx', i += ay by' in the order given
+__device__ __forceinline__ void mma_run_complex(uint32_t dr, uint32_t di, uint64_t ar, uint64_t ai, uint64_t br, uint64_t bi, uint32_t da, uint32_t db,
+                                             uint32_t id, uint32_t id_second_r, uint32_t id_second_i, bool i_starts_with_ar, int n, bool accumulate) {
+#pragma unroll 1
+  for (int i = 0; i < n; ++i) {
+    mma_bf16(dr, ar, br, id, accumulate);
+    mma_bf16(dr, ai, bi, id_second_r, true);
+    mma_bf16(di, i_starts_with_ar ? ar : ai, i_starts_with_ar ? bi : br, id, accumulate);
+    mma_bf16(di, i_starts_with_ar ? ai : ar, i_starts_with_ar ? br : bi, id_second_i, true);
+    accumulate = true;
+    ar += da; ai += da;
+    br += db; bi += db;
+  }
+}
 // mbarrier arrives once all MMAs issued so far by this thread have completed
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
