@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
   }
 }
 
-enum ChunkMode { M_FWD = 0, M_DQ = 1, M_DV = 2, M_DK = 3 };
+enum ChunkMode { M_FWD = 0, M_DQ = 1, M_DV = 2, M_DK = 3, M_ANY = 4 };
 
 struct ChunkMaps {
   CUtensorMap a1, b1, x2;  // [B*H*T rows][128 bf16], boxes of 64 x 128, 128-byte swizzle

@@ -74,11 +74,10 @@ __device__ __forceinline__ void deint_write(unsigned char* tile, int row, int hb
 
 // ---- MMA issue (one thread) -----------------------------------------------------------------------------
 // X = A1 conj(B1)^T : Xr = ar br^T + ai bi^T, Xi = ai br^T - ar bi^T  (planes K-major, K = 64)
-// IMAG_SWAPPED: the two halves of Xi are accumulated in the other order, so that the job whose operands are swapped
+// imag_swapped: the two halves of Xi are accumulated in the other order, so that the job whose operands are swapped
 // (dk: v dy^H against dq: dy v^H) adds the same numbers in the same order and gets the negated imaginary part bit
 // for bit.
-template <bool IMAG_SWAPPED = false>
-__device__ __forceinline__ void bw_issue_scores(uint32_t slot, uint32_t a_r, uint32_t b_r) {
+__device__ __forceinline__ void bw_issue_scores(uint32_t slot, uint32_t a_r, uint32_t b_r, const bool imag_swapped = false) {
   using namespace umma;
   constexpr uint32_t id = idesc_bf16(128, 128, false, false);
   constexpr uint32_t idn = idesc_bf16_nega(128, 128, false, false);
@@ -86,13 +85,8 @@ __device__ __forceinline__ void bw_issue_scores(uint32_t slot, uint32_t a_r, uin
   const uint64_t br = smem_desc_sw128(b_r, 16, 1024), bi = smem_desc_sw128(b_r + 16384, 16, 1024);
   mma_run(slot, ar, br, 2, 2, id, 4, false);
   mma_run(slot, ai, bi, 2, 2, id, 4, true);
-  if (!IMAG_SWAPPED) {
-    mma_run(slot + 128, ai, br, 2, 2, id, 4, false);
-    mma_run(slot + 128, ar, bi, 2, 2, idn, 4, true);
-  } else {
-    mma_run(slot + 128, ar, bi, 2, 2, idn, 4, false);
-    mma_run(slot + 128, ai, br, 2, 2, id, 4, true);
-  }
+  mma_run(slot + 128, imag_swapped ? ar : ai, imag_swapped ? bi : br, 2, 2, imag_swapped ? idn : id, 4, false);
+  mma_run(slot + 128, imag_swapped ? ai : ar, imag_swapped ? br : bi, 2, 2, imag_swapped ? id : idn, 4, true);
 }
 
 // TMEM column of the packed bf16 scores of k-step kk (16 score columns = 8 TMEM columns): the thread that
@@ -110,29 +104,29 @@ __device__ __forceinline__ void bw_issue_out(uint32_t slot, uint32_t x_r, bool a
   mma_run_ts(slot + 192, slot + 16, smem_desc_sw128(x_r, 16, 1024), 8, 24, 128, id, 8, true);
 }
 
-// acc (+)= A1 (.) state planes [64 rows i][64 j]:  OP_H == false: out[r][i] = sum_j a[r][j] S[i][j];
-// OP_H == true: out[r][j] = sum_i conj(S[i][j]) a[r][i].
-template <bool OP_H>
-__device__ __forceinline__ void bw_issue_state(uint32_t slot, uint32_t a_r, uint32_t s_r, bool accumulate) {
+// acc (+)= A1 (.) state planes [64 rows i][64 j]:  op_h == false: out[r][i] = sum_j a[r][j] S[i][j]  (a_r S_r - a_i S_i; a_r S_i + a_i S_r);
+// op_h == true: out[r][j] = sum_i conj(S[i][j]) a[r][i]  (a_r S_r + a_i S_i; a_i S_r - a_r S_i).
+__device__ __forceinline__ void bw_issue_state(const bool op_h, uint32_t slot, uint32_t a_r, uint32_t s_r, bool accumulate) {
   using namespace umma;
   const uint64_t ar = smem_desc_sw128(a_r, 16, 1024), ai = smem_desc_sw128(a_r + 16384, 16, 1024);
   const uint64_t sr = smem_desc_sw128(s_r, 16, 1024), si = smem_desc_sw128(s_r + 8192, 16, 1024);
-  constexpr uint32_t id = idesc_bf16(128, 64, false, OP_H), idn = idesc_bf16_nega(128, 64, false, OP_H);
-  if (!OP_H) mma_run_complex(slot + 128, slot + 192, ar, ai, sr, si, 2, 2, id, idn, id, true, 4, accumulate);      // a_r S_r - a_i S_i; a_r S_i + a_i S_r
-  else mma_run_complex(slot + 128, slot + 192, ar, ai, sr, si, 2, 128, id, id, idn, false, 4, accumulate);         // a_r S_r + a_i S_i; a_i S_r - a_r S_i
+  const uint32_t id = idesc_bf16(128, 64, false, op_h), idn = idesc_bf16_nega(128, 64, false, op_h);
+  mma_run_complex(slot + 128, slot + 192, ar, ai, sr, si, 2, op_h ? 128 : 2, id, op_h ? id : idn, op_h ? idn : id, !op_h, 4, accumulate);
 }
 
 // ---- epilogue 1: decay-masked scores of this thread's row, columns [32 cb, 32 cb + 32), as packed bf16 ------
 // fast path: T = [mask] cfac[col] X;  slow path (STRONG): T = [mask] scale exp(-|A_row - A_col|) X.
-// ROWW: the row's own factor `rowf` multiplies the weight before the score is rounded (see chunk_job).
-template <bool LOWER, bool STRONG, bool ROWW>
-__device__ __forceinline__ void bw_epi_scores_t(uint32_t tlane_slot, int q4, int cb, int r, int len,
+// The row's own factor `rowf` (1 where it is applied later) multiplies the weight before the score is rounded (see chunk_job).
+template <bool STRONG>
+__device__ __forceinline__ void bw_epi_scores_t(const bool lower, uint32_t tlane_slot, int q4, int cb, int r, int len,
                                                 const float* __restrict__ cfac, const float* __restrict__ Acum,
                                                 float scale, float rowf) {
   using namespace umma;
   const int c0 = 32 * cb;
-  const bool dead = LOWER ? (c0 > q4 * 32 + 31) : (c0 + 31 < q4 * 32);      // warp-uniform
-  const bool full = LOWER ? (c0 + 31 <= q4 * 32) : (c0 >= q4 * 32 + 31);    // no triangle inside the block
+  const bool dead = lower ? (c0 > q4 * 32 + 31) : (c0 + 31 < q4 * 32);      // warp-uniform
+  const bool full = lower ? (c0 + 31 <= q4 * 32) : (c0 >= q4 * 32 + 31);    // no triangle inside the block
+  // columns that count: [0, r] below the diagonal, [r, 128) above it, all of them without a diagonal in the block
+  const int first = full || lower ? 0 : r, last = full || !lower ? TC - 1 : r;
   uint32_t tr[16], ti[16];
   if (dead) {
 #pragma unroll
@@ -149,10 +143,9 @@ __device__ __forceinline__ void bw_epi_scores_t(uint32_t tlane_slot, int q4, int
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int c = c0 + 16 * hh + j + e;
-          bool on = full || (LOWER ? (c <= r) : (c >= r));
-          if (!LOWER && STRONG) on = on && (c < len);      // (the column factors of the fast path are zero past `len`)
-          const float w = STRONG ? scale * __expf(fminf(0.f, LOWER ? a_r - Acum[c] : Acum[c] - a_r))
-                                 : (ROWW ? rowf * cfac[c] : cfac[c]);
+          bool on = (unsigned)(c - first) <= (unsigned)(last - first);
+          if (STRONG && !lower) on = on && (c < len);      // (the column factors of the fast path are zero past `len`)
+          const float w = STRONG ? scale * __expf(fminf(0.f, lower ? a_r - Acum[c] : Acum[c] - a_r)) : rowf * cfac[c];
           d[e] = on ? w : 0.f;
         }
         const float r0 = __uint_as_float(hh ? xr1[j] : xr0[j]), r1 = __uint_as_float(hh ? xr1[j + 1] : xr0[j + 1]);
@@ -166,20 +159,19 @@ __device__ __forceinline__ void bw_epi_scores_t(uint32_t tlane_slot, int q4, int
   tmem_st16(tlane_slot + c0, tr);
   tmem_st16(tlane_slot + c0 + 16, ti);
 }
-template <bool LOWER, bool ROWW = false>
-__device__ __forceinline__ void bw_epi_scores(uint32_t tlane_slot, int q4, int cb, int r, int len, bool strong,
+__device__ __forceinline__ void bw_epi_scores(const bool lower, uint32_t tlane_slot, int q4, int cb, int r, int len, bool strong,
                                               const float* __restrict__ cfac, const float* __restrict__ Acum,
-                                              float scale, float rowf = 1.f) {
-  if (strong) bw_epi_scores_t<LOWER, true, false>(tlane_slot, q4, cb, r, len, cfac, Acum, scale, 1.f);
-  else bw_epi_scores_t<LOWER, false, ROWW>(tlane_slot, q4, cb, r, len, cfac, Acum, scale, rowf);
+                                              float scale, float rowf) {
+  if (strong) bw_epi_scores_t<true>(lower, tlane_slot, q4, cb, r, len, cfac, Acum, scale, 1.f);
+  else bw_epi_scores_t<false>(lower, tlane_slot, q4, cb, r, len, cfac, Acum, scale, rowf);
 }
 
 // ---- epilogue 2: out[r][16 cb .. 16 cb + 16) = rf * acc -> global; optional part of Re<x_r, out_r>, x_r given as the
 // four 16-byte pieces of the interleaved bf16 row that cover these channels ------------------------------------
 // `stage` != nullptr: the 16-byte pieces go to this row of a 128-byte-swizzled staging block (piece index
 // 4 * (cb & 1) + g, row & 7 = `sw`) instead of global memory; a TMA store moves the block afterwards.
-template <bool DOT, bool ADD = false>
-__device__ __forceinline__ float bw_epi_out(uint32_t tlane_slot, int cb, float rf, __nv_bfloat16* __restrict__ orow,
+template <bool ADD = false>
+__device__ __forceinline__ float bw_epi_out(const bool want_dot, uint32_t tlane_slot, int cb, float rf, __nv_bfloat16* __restrict__ orow,
                                             const uint4 (&xg)[4], bool valid, unsigned char* stage = nullptr, int sw = 0) {
   using namespace umma;
   float vr[16], vi[16];
@@ -210,7 +202,7 @@ __device__ __forceinline__ float bw_epi_out(uint32_t tlane_slot, int cb, float r
       } else {
         *reinterpret_cast<uint4*>(orow + g * 8) = pk;
       }
-      if (DOT) {
+      if (want_dot) {
         const uint32_t xw[4] = {xg[g].x, xg[g].y, xg[g].z, xg[g].w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -245,15 +237,18 @@ __device__ __forceinline__ void rescale_acc_half(uint32_t tlane_slot, int hf, fl
 // ---------------------------------------------------------------------------------------------
 // One job of one chunk (256 threads; the caller's CTA holds nothing else).
 // ---------------------------------------------------------------------------------------------
-template <int MODE, bool ACC = false>      // ACC: the output is added to what the buffer holds (gradients only)
-__device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, const CUtensorMap* __restrict__ mb1,
+// MODE: M_FWD, or M_ANY: one of the three gradients, which one told by `mode`.  (One body for the three: an SM runs all of them side by
+// side, and three copies of it did not fit the instruction cache, 465 misses a job.)
+// ACC: the output is added to what the buffer holds (gradients only).
+template <int MODE, bool ACC = false>
+__device__ __forceinline__ void chunk_job(const int mode, const CUtensorMap* __restrict__ ma1, const CUtensorMap* __restrict__ mb1,
                                           const CUtensorMap* __restrict__ mx2, const CUtensorMap* __restrict__ mout,
                                           const CUtensorMap* __restrict__ mdot, const ScanParams& p, int chunk_x, int h,
                                           unsigned char* smem) {
   using namespace umma;
-  constexpr bool LOWER = (MODE == M_FWD || MODE == M_DQ);       // mask col <= row
-  constexpr bool OP_H = (MODE == M_DQ || MODE == M_DK);         // carried operand conj-transposed
-  constexpr bool DOT = (MODE == M_DQ || MODE == M_DK);          // also leaves Re<x_row, out_row>, x = q (dq) or k (dk): mdot
+  const bool LOWER = MODE == M_FWD || mode == M_DQ;                            // mask col <= row
+  const bool OP_H = MODE != M_FWD && (mode == M_DQ || mode == M_DK);           // carried operand conj-transposed
+  const bool DOT = OP_H;                                                       // also leaves Re<x_row, out_row>, x = q (dq) or k (dk): mdot
   // The decay gradient is a running sum of Re<q_t, dq_t> - Re<k_t, dk_t> over the chunk, in which the contribution of
   // every (t, s) pair cancels -- exactly only if dq and dk are built from the SAME rounded scores.  So these two jobs
   // put the whole weight e^{A_t - A_s} (row factor x column factor) into a score before it is rounded to bf16, which
@@ -261,7 +256,7 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
   // factor from the A1 rows, rescaled between stage 1 and stage 3.  (With the row factor applied in epilogue 2 the two
   // jobs rounded different numbers and the noise of up to 128 tokens piled up in the sum: 1-3 % of dgamma at decays
   // around 0.5 per token.)  The forward and the dv job keep the row factor in epilogue 2.
-  constexpr bool ROWW = DOT;
+  const bool ROWW = DOT;
   unsigned char* RA = smem;                  // A1: real plane, imaginary plane  (2 x [128 rows][128 B])
   unsigned char* RB = RA + 32768;            // B1 planes; after stage 1: carried state planes (2 x [64 rows][128 B])
   unsigned char* RC = RB + 32768;            // X2 planes
@@ -346,7 +341,7 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
   const uint32_t a_r = smem_u32(RA), b_r = smem_u32(RB), x_r = smem_u32(RC);
   if (warp == 0 && elect_one()) {
     tc_fence_after();
-    bw_issue_scores<MODE == M_DK>(tmem, a_r, b_r);
+    bw_issue_scores(tmem, a_r, b_r, MODE != M_FWD && mode == M_DK);
     mma_commit(&bars[1]);
   }
   __syncwarp();
@@ -369,7 +364,7 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
   // epilogue 1: masked, decayed scores of columns [64 hf, 64 hf + 64) as packed bf16 pairs
 #pragma unroll 1
   for (int cb = 2 * hf; cb < 2 * hf + 2; ++cb)
-    bw_epi_scores<LOWER, ROWW>(tl, q4, cb, r, L.len, strong, cfac, Acum, p.q_scale, ROWW ? rfac[r] : 1.f);
+    bw_epi_scores(LOWER, tl, q4, cb, r, L.len, strong, cfac, Acum, p.q_scale, ROWW ? rfac[r] : 1.f);
   tmem_st_wait();
   if (ROWW && has_state && !strong) {
     // stage 1 was the last reader of the unscaled A1 rows: thread (row r, plane hf) multiplies its 128 bytes by the
@@ -426,7 +421,7 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
     // slow path: the carried-state product alone, then every row rescaled by its own decay in TMEM
     if (warp == 0 && elect_one()) {
       tc_fence_after();
-      bw_issue_state<OP_H>(tmem, a_r, b_r, false);
+      bw_issue_state(OP_H, tmem, a_r, b_r, false);
       mma_commit(&bars[3]);
     }
     __syncwarp();
@@ -441,7 +436,7 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
     tc_fence_after();
     const bool state_now = has_state && !strong;
     if (state_now) {        // the carried-state product first: it is the last reader of the A1 planes
-      bw_issue_state<OP_H>(tmem, a_r, b_r, false);
+      bw_issue_state(OP_H, tmem, a_r, b_r, false);
       if (DOT) mma_commit(&bars[3]);
     }
     bw_issue_out(tmem, x_r, two_step || state_now);
@@ -460,7 +455,7 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
   }
   __syncwarp();
   {
-    void* outp = MODE == M_FWD ? p.y : MODE == M_DQ ? p.dq : MODE == M_DV ? p.dv : p.dk;
+    void* outp = MODE == M_FWD ? p.y : mode == M_DQ ? p.dq : mode == M_DV ? p.dv : p.dk;
     const size_t rbase = token_base(p, L.b, h, L.t0 + r, TD) + hf * 64;   // channels [32 hf, 32 hf + 32)
     const size_t obase = (MODE == M_FWD && p.y_token_major)
                              ? (((size_t)L.b * p.T + L.t0 + r) * p.H + h) * (size_t)(TD * 2) + hf * 64 : rbase;
@@ -485,7 +480,7 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
     float dot = 0.f;
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc)
-      dot += bw_epi_out<DOT, accum>(tl, 2 * hf + cc, rf, orow + cc * 32, dpre[cc], valid && ok,
+      dot += bw_epi_out<accum>(DOT, tl, 2 * hf + cc, rf, orow + cc * 32, dpre[cc], valid && ok,
                                     bulk ? wbox + lane * 128 : nullptr, lane & 7);
     if (bulk) {
       fence_proxy_async();
@@ -502,7 +497,7 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
       if (tid < L.len && ok) {
         const float d2 = dots[tid] + dots[TC + tid];
         const size_t gi = gamma_base(p, 0, L.b, h, L.t0 + tid);
-        if (MODE == M_DQ) p.dgamma[gi] = d2; else p.dA_k[gi] = d2;   // combined by k_tc_dgamma_finalize
+        if (mode == M_DQ) p.dgamma[gi] = d2; else p.dA_k[gi] = d2;   // combined by k_tc_dgamma_finalize
       }
     }
   }
@@ -519,7 +514,7 @@ __device__ __forceinline__ void chunk_job(const CUtensorMap* __restrict__ ma1, c
 __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwd(const __grid_constant__ ChunkMaps maps, ScanParams p) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  chunk_job<M_FWD>(&maps.a1, &maps.b1, &maps.x2, &maps.out, &maps.a1, p, blockIdx.x, blockIdx.y, smem);
+  chunk_job<M_FWD>(M_FWD, &maps.a1, &maps.b1, &maps.x2, &maps.out, &maps.a1, p, blockIdx.x, blockIdx.y, smem);
 }
 
 // the three gradients: grid = (3 * chunks, H); CTA x works on chunk x / 3, job x % 3 (dq, dv, dk), so the CTAs that
@@ -530,9 +525,9 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_bwd(const __grid_constant__
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int chunk_x = blockIdx.x / 3, job = blockIdx.x - 3 * chunk_x;
-  if (job == 0) chunk_job<M_DQ, ACC>(&maps.dy, &maps.v, &maps.k, &maps.dq, &maps.q, p, chunk_x, blockIdx.y, smem);
-  else if (job == 1) chunk_job<M_DV, ACC>(&maps.k, &maps.q, &maps.dy, &maps.dv, &maps.k, p, chunk_x, blockIdx.y, smem);
-  else chunk_job<M_DK, ACC>(&maps.v, &maps.dy, &maps.q, &maps.dk, &maps.k, p, chunk_x, blockIdx.y, smem);
+  const CUtensorMap *a1 = job == 0 ? &maps.dy : job == 1 ? &maps.k : &maps.v, *b1 = job == 0 ? &maps.v : job == 1 ? &maps.q : &maps.dy;
+  const CUtensorMap *x2 = job == 0 ? &maps.k : job == 1 ? &maps.dy : &maps.q, *out = job == 0 ? &maps.dq : job == 1 ? &maps.dv : &maps.dk;
+  chunk_job<M_ANY, ACC>(job == 0 ? M_DQ : job == 1 ? M_DV : M_DK, a1, b1, x2, out, job == 0 ? &maps.q : &maps.k, p, chunk_x, blockIdx.y, smem);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -40,7 +40,7 @@ constexpr size_t BWDK_SMEM = 1024 + 4 * 32768 + 4 * 16384 + KMAX * TC * (4 + 4 +
 
 // acc (real parts at acc, imaginary at acc + 64) = A (.) state planes, as bw_issue_state
 template <bool OP_H>
-__device__ __forceinline__ void issue_state(uint32_t acc, uint32_t a_r, uint32_t s_r) { bw_issue_state<OP_H>(acc - 128, a_r, s_r, false); }
+__device__ __forceinline__ void issue_state(uint32_t acc, uint32_t a_r, uint32_t s_r) { bw_issue_state(OP_H, acc - 128, a_r, s_r, false); }
 
 // acc = T X2, T's packed scores in the columns its fp32 scores had: of every 16 columns the first 8 hold the real parts
 __device__ __forceinline__ void issue_rows(uint32_t t, uint32_t acc, uint32_t x_r) {
