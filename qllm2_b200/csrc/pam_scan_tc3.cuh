@@ -14,12 +14,16 @@
 // with the state planes e^{A^k_m} S^k_c, accumulating into the same output tile -- two states per pass.
 //
 //   stage 1  X = Q conj(K)^T                         Xr: cols [0,128)   Xi: cols [128,256)
-//   epi 1    T = [s <= t] G (.) X  -> bf16           Tr: cols [0,64)    Ti: cols [128,192)
-//   stage 2  acc = T V                               acc_r: cols [64,128)  acc_i: cols [192,256)
-//   pass p   T'_k -> cols [32 s, 32 s + 32) of the Tr / Ti ranges (s = slot of state k in the pass)
+//   epi 1    T = [s <= t] G (.) X  -> bf16           over the thread's own Xr columns, as in pam_scan_tc2.cuh
+//   stage 2  acc = T V                               acc_r: cols [128,192)  acc_i: cols [192,256)
+//   pass p   T'_k -> cols [64 s, 64 s + 64), real half, imaginary half (s = slot of state k in the pass)
 //            acc += T'_k (e^{A^k_m} S^k)^T
+// (Weights and states are formed in loops that are not unrolled over column groups: straight-line code missed the instruction
+// cache 460 times a job.  8 x 6 x 2048, three states: 76 -> 66 us; 48 chat prompts: 187 -> 163.)
 //   epi 2    y = acc
 #pragma once
+#include <type_traits>
+
 #include "pam_scan_tc2.cuh"
 
 namespace qpam {
@@ -121,8 +125,7 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   }
   fence_proxy_async();
   __syncthreads();
-  const uint32_t a_r = smem_u32(RA), a_i = a_r + 16384, b_r = smem_u32(RB), b_i = b_r + 16384;
-  const uint32_t x_r = smem_u32(RC), x_i = x_r + 16384;
+  const uint32_t a_r = smem_u32(RA), b_r = smem_u32(RB), x_r = smem_u32(RC);
   if (warp == 0 && elect_one()) {
     tc_fence_after();
     bw_issue_scores(tmem, a_r, b_r);
@@ -159,84 +162,52 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   };
 
   {
-    // epilogue 1: weighted, masked scores of columns [64 hf, 64 hf + 64) as packed bf16 pairs
-    uint32_t tr[32], ti[32];
-#pragma unroll
-    for (int cc = 0; cc < 4; ++cc) {
-      const int c0 = hf * 64 + cc * 16;
-      const bool dead = c0 > q4 * 32 + 31;   // warp-uniform: the whole block lies above the diagonal
+    // epilogue 1: weighted, masked scores of columns [64 hf, 64 hf + 64), 32 at a time, as packed bf16 pairs over the columns they
+    // came from
+#pragma unroll 1
+    for (int cb = 2 * hf; cb < 2 * hf + 2; ++cb) {
+      uint32_t out[2][16];                      // 16 columns of the real parts and 16 of the imaginary parts (two columns a word)
+      const bool dead = cb * 32 > q4 * 32 + 31;      // warp-uniform: the whole block lies above the diagonal
       if (dead) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) tr[cc * 8 + j] = ti[cc * 8 + j] = 0u;
+        for (int j = 0; j < 16; ++j) out[0][j] = out[1][j] = 0u;
       } else {
-        float xr[16], xi[16];
-        tmem_ld16(tlane + c0, xr);
-        tmem_ld16(tlane + 128 + c0, xi);
-        // (the two loops differ only in how a state's column factor is formed: the common case -- no state of this
+        uint32_t x0[16], x1[16], y0[16], y1[16];
+        tmem_ld16x4(tlane + cb * 32, x0, tlane + cb * 32 + 16, x1, tlane + 128 + cb * 32, y0, tlane + 128 + cb * 32 + 16, y1);
+        // (the two forms differ only in how a state's column factor is formed: the common case -- no state of this
         // chunk decays strongly, CTA-uniform -- keeps the exponentials out of the per-score code)
-        if (strong_mask == 0u) {
+        auto weigh = [&](auto any_strong) {
 #pragma unroll
-          for (int j = 0; j < 16; j += 2) {
+          for (int j = 0; j < 32; j += 2) {
             float wr[2], wi[2];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const int c = c0 + j + e;
+              const int c = cb * 32 + j + e;
               float gr = 0.f, gi = 0.f;
 #pragma unroll
               for (int k = 0; k < KMAX; ++k)
                 if (k < K) {
-                  const float cf = cfac[k * TC + c];
+                  const float cf = decltype(any_strong)::value && ((strong_mask >> k) & 1u) ? __expf(fminf(0.f, Acum[k * TC + r] - Acum[k * TC + c]))
+                                                                                            : cfac[k * TC + c];
                   gr = fmaf(rk[k].x, cf, gr);
                   gi = fmaf(rk[k].y, cf, gi);
                 }
               if (c > r) gr = gi = 0.f;
-              wr[e] = xr[j + e] * gr - xi[j + e] * gi;
-              wi[e] = xr[j + e] * gi + xi[j + e] * gr;
+              const float xr = __uint_as_float(j < 16 ? x0[(j + e) & 15] : x1[(j + e) & 15]), xi = __uint_as_float(j < 16 ? y0[(j + e) & 15] : y1[(j + e) & 15]);
+              wr[e] = xr * gr - xi * gi;
+              wi[e] = xr * gi + xi * gr;
             }
-            tr[cc * 8 + (j >> 1)] = pack_bf162(wr[0], wr[1]);
-            ti[cc * 8 + (j >> 1)] = pack_bf162(wi[0], wi[1]);
+            out[0][j >> 1] = pack_bf162(wr[0], wr[1]);
+            out[1][j >> 1] = pack_bf162(wi[0], wi[1]);
           }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            float wr[2], wi[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int c = c0 + j + e;
-              float gr = 0.f, gi = 0.f;
-#pragma unroll
-              for (int k = 0; k < KMAX; ++k)
-                if (k < K) {
-                  const float cf = ((strong_mask >> k) & 1u) ? __expf(fminf(0.f, Acum[k * TC + r] - Acum[k * TC + c]))
-                                                             : cfac[k * TC + c];
-                  gr = fmaf(rk[k].x, cf, gr);
-                  gi = fmaf(rk[k].y, cf, gi);
-                }
-              if (c > r) gr = gi = 0.f;
-              wr[e] = xr[j + e] * gr - xi[j + e] * gi;
-              wi[e] = xr[j + e] * gi + xi[j + e] * gr;
-            }
-            tr[cc * 8 + (j >> 1)] = pack_bf162(wr[0], wr[1]);
-            ti[cc * 8 + (j >> 1)] = pack_bf162(wi[0], wi[1]);
-          }
-        }
+        };
+        if (strong_mask == 0u) weigh(std::false_type());
+        else weigh(std::true_type());
       }
+      tmem_st16(tlane + cb * 32, out[0]);
+      tmem_st16(tlane + cb * 32 + 16, out[1]);
     }
-    tc_fence_before();
-    __syncthreads();          // every warp has read its scores: their columns may be overwritten
-    tc_fence_after();
-    {
-      uint32_t lo[16], hi[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) { lo[j] = tr[j]; hi[j] = tr[16 + j]; }
-      tmem_st16(tlane + hf * 32, lo);
-      tmem_st16(tlane + hf * 32 + 16, hi);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) { lo[j] = ti[j]; hi[j] = ti[16 + j]; }
-      tmem_st16(tlane + 128 + hf * 32, lo);
-      tmem_st16(tlane + 128 + hf * 32 + 16, hi);
-      tmem_st_wait();
-    }
+    tmem_st_wait();
     if (has_state) {          // the K planes are no longer needed: states 0 and 1 take their place
       stage_state(0, 0);
       if (K > 1) stage_state(1, 1);
@@ -245,16 +216,9 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   fence_proxy_async();
   tc_fence_before();
   __syncthreads();
-  const uint32_t Tr = tmem, Ti = tmem + 128, Or = tmem + 64, Oi = tmem + 192;
   if (warp == 0 && elect_one()) {
     tc_fence_after();
-    constexpr uint32_t id = idesc_bf16(128, 64, false, true);        // A: TMEM, B: MN-major plane
-    constexpr uint32_t idn = idesc_bf16_nega(128, 64, false, true);
-    const uint64_t xr = smem_desc_sw128(x_r, 16, 1024), xi = smem_desc_sw128(x_i, 16, 1024);
-    mma_run_ts(Or, Tr, xr, 8, 8, 128, id, 8, false);
-    mma_run_ts(Or, Ti, xi, 8, 8, 128, idn, 8, true);
-    mma_run_ts(Oi, Tr, xi, 8, 8, 128, id, 8, false);
-    mma_run_ts(Oi, Ti, xr, 8, 8, 128, id, 8, true);
+    bw_issue_out(tmem, x_r);
     mma_commit(&bars[2]);
   }
   __syncwarp();
@@ -278,28 +242,24 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
           rr.x *= ea;
           rr.y *= ea;
         }
-        uint32_t wr[32], wi[32];
+#pragma unroll 1
+        for (int g = 0; g < 2; ++g) {                // 32 channels at a time: 16 columns of reals, 16 of imaginaries
+          uint32_t wr[16], wi[16];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const uint4 qr = *reinterpret_cast<const uint4*>(RA + sw128(r, c));
-          const uint4 qi = *reinterpret_cast<const uint4*>(RA + 16384 + sw128(r, c));
-          const uint32_t qrw[4] = {qr.x, qr.y, qr.z, qr.w}, qiw[4] = {qi.x, qi.y, qi.z, qi.w};
+          for (int c = 0; c < 4; ++c) {
+            const uint4 qr = *reinterpret_cast<const uint4*>(RA + sw128(r, 4 * g + c));
+            const uint4 qi = *reinterpret_cast<const uint4*>(RA + 16384 + sw128(r, 4 * g + c));
+            const uint32_t qrw[4] = {qr.x, qr.y, qr.z, qr.w}, qiw[4] = {qi.x, qi.y, qi.z, qi.w};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 a = unpack_bf162(qrw[e]), b = unpack_bf162(qiw[e]);   // two consecutive channels
-            wr[c * 4 + e] = pack_bf162(a.x * rr.x - b.x * rr.y, a.y * rr.x - b.y * rr.y);
-            wi[c * 4 + e] = pack_bf162(a.x * rr.y + b.x * rr.x, a.y * rr.y + b.y * rr.x);
+            for (int e = 0; e < 4; ++e) {
+              const float2 a = unpack_bf162(qrw[e]), b = unpack_bf162(qiw[e]);   // two consecutive channels
+              wr[c * 4 + e] = pack_bf162(a.x * rr.x - b.x * rr.y, a.y * rr.x - b.y * rr.y);
+              wi[c * 4 + e] = pack_bf162(a.x * rr.y + b.x * rr.x, a.y * rr.y + b.y * rr.x);
+            }
           }
+          tmem_st16(tlane + hf * 64 + g * 16, wr);
+          tmem_st16(tlane + hf * 64 + 32 + g * 16, wi);
         }
-        uint32_t lo[16], hi[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) { lo[j] = wr[j]; hi[j] = wr[16 + j]; }
-        tmem_st16(tlane + hf * 32, lo);
-        tmem_st16(tlane + hf * 32 + 16, hi);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) { lo[j] = wi[j]; hi[j] = wi[16 + j]; }
-        tmem_st16(tlane + 128 + hf * 32, lo);
-        tmem_st16(tlane + 128 + hf * 32 + 16, hi);
         tmem_st_wait();
       }
       fence_proxy_async();
@@ -308,16 +268,18 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
       if (warp == 0 && elect_one()) {
         tc_fence_after();
         constexpr uint32_t k3 = idesc_bf16(128, 64, false, false), k3n = idesc_bf16_nega(128, 64, false, false);
+#pragma unroll 1
         for (int s = 0; s < 2 && pass * 2 + s < K; ++s) {
-          const uint32_t s_r = b_r + s * 16384, s_i = s_r + 8192;   // [64 rows i][64 j] planes of this slot
-          const uint32_t tr_ = Tr + s * 32, ti_ = Ti + s * 32;
-#pragma unroll
+          uint64_t sr = smem_desc_sw128(b_r + s * 16384, 16, 1024), si = smem_desc_sw128(b_r + s * 16384 + 8192, 16, 1024);   // [64 rows i][64 j] planes of this slot
+          uint32_t tr_ = tmem + s * 64, ti_ = tr_ + 32;
+#pragma unroll 1
           for (int kk = 0; kk < 4; ++kk) {
-            const uint64_t sr = smem_desc_sw128(s_r + kk * 32, 16, 1024), si = smem_desc_sw128(s_i + kk * 32, 16, 1024);
-            mma_bf16_ts(Or, tr_ + kk * 8, sr, k3, true);    // + T'r Sr^T
-            mma_bf16_ts(Or, ti_ + kk * 8, si, k3n, true);   // - T'i Si^T
-            mma_bf16_ts(Oi, tr_ + kk * 8, si, k3, true);    // + T'r Si^T
-            mma_bf16_ts(Oi, ti_ + kk * 8, sr, k3, true);    // + T'i Sr^T
+            mma_bf16_ts(tmem + 128, tr_, sr, k3, true);    // + T'r Sr^T
+            mma_bf16_ts(tmem + 128, ti_, si, k3n, true);   // - T'i Si^T
+            mma_bf16_ts(tmem + 192, tr_, si, k3, true);    // + T'r Si^T
+            mma_bf16_ts(tmem + 192, ti_, sr, k3, true);    // + T'i Sr^T
+            tr_ += 8; ti_ += 8;
+            sr += 2; si += 2;
           }
         }
         mma_commit(&bars[3 + pass]);
@@ -338,7 +300,7 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc) {
       float vr[16], vi[16];
-      tmem_ld16(tlane + 64 + hf * 32 + cc * 16, vr);
+      tmem_ld16(tlane + 128 + hf * 32 + cc * 16, vr);
       tmem_ld16(tlane + 192 + hf * 32 + cc * 16, vi);
       if (ok && r < L.len) {
 #pragma unroll
