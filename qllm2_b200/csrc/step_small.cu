@@ -486,13 +486,6 @@ __global__ void __launch_bounds__(1024) k_step_norm(bf16* __restrict__ z, const 
   V4<bf16>::st(xn + row * D * 2 + g * 8, re, im);
 }
 
-// Out of line: the routine is long, and a state's read-out weight is one call (unrolled over the states it was four copies).
-__device__ __noinline__ float2 cos_sin(float x) {
-  float sn, cs;
-  sincosf(x, &sn, &cs);
-  return make_float2(cs, sn);
-}
-
 struct StepRecur {
   void* pool;
   const int32_t* slots;
@@ -573,8 +566,9 @@ struct RecurRows {
       float2 cf = make_float2(1.f, 0.f);
       if (p.c_phase >= 0) {
         const float w = p.c_score >= 0 ? sc[k] / wsum * (float)p.K : 1.f;
-        const float2 cs = cos_sin(ph[k]);
-        cf = make_float2(w * cs.x, w * cs.y);
+        float sn, cs;
+        sincosf(ph[k], &sn, &cs);
+        cf = make_float2(w * cs, w * sn);
       }
       float sr[4], si[4];
       S* cell = base + k * step;
@@ -658,7 +652,8 @@ struct OneUnit {
   int kb;                       // K blocks
 };
 
-template <typename S>
+// PAIR: at most two sequences, a unit of a projection back is 8 weight rows and their halves of K
+template <typename S, bool PAIR>
 struct One {
   const OneParams& p;
   const OneLayers& layers;
@@ -771,14 +766,14 @@ struct One {
   }
   __device__ __forceinline__ OneUnit unit_back(const void* w_, int kblocks, int u) const {    // a projection back to D rows
     const int64_t ld = (int64_t)kblocks * 32;
-    if (p.n <= 2) {
+    if (PAIR) {
       const bf16* w = (const bf16*)w_ + 2 * (int64_t)(u * 8 + (lane >> 2)) * ld;
       return {w, w + (ld >> 1), kblocks >> 1};
     }
     const bf16* w = (const bf16*)w_ + 2 * (int64_t)(u * 16 + (lane >> 2)) * ld;
     return {w, w + 16 * ld, kblocks};
   }
-  __device__ __forceinline__ int units_back() const { return p.n <= 2 ? p.D / 8 : p.D / 16; }
+  __device__ __forceinline__ int units_back() const { return PAIR ? p.D / 8 : p.D / 16; }
   __device__ __forceinline__ void request_back(const void* w, int kblocks) {
     if ((int)blockIdx.x < units_back()) request(unit_back(w, kblocks, blockIdx.x), warp, 16);
   }
@@ -892,8 +887,7 @@ struct One {
       const OneUnit un = unit_back(w, kblocks, u);
       if (u != (int)blockIdx.x) request(un, warp, 16);
       float acc[4];
-      if (p.n <= 2) accumulate<true>(un, rows, ld, warp, 16, acc);
-      else accumulate<false>(un, rows, ld, warp, 16, acc);
+      accumulate<PAIR>(un, rows, ld, warp, 16, acc);
       __syncthreads();
       red[warp * 32 + lane] = make_float4(acc[0], acc[1], acc[2], acc[3]);
       __syncthreads();
@@ -906,7 +900,7 @@ struct One {
         }
         const int seq = lane & 3;
         uint32_t* o = reinterpret_cast<uint32_t*>(out);
-        if (p.n <= 2) {                 // (x, y) of columns 0..3 and (z, w) of columns 4..7 are the halves of K
+        if (PAIR) {                     // (x, y) of columns 0..3 and (z, w) of columns 4..7 are the halves of K
           const float re = s.x + __shfl_xor_sync(0xffffffffu, s.z, 2), im = s.y + __shfl_xor_sync(0xffffffffu, s.w, 2);
           const int row = u * 8 + (lane >> 2);
           if (seq < p.n) store_row(o, seq, row, re, im, bias);
@@ -928,13 +922,13 @@ struct One {
   }
 };
 
-template <typename S>
+template <typename S, bool PAIR>
 __global__ void __launch_bounds__(ONE_THREADS, 1) k_step_one(const __grid_constant__ OneParams p, const __grid_constant__ OneLayers layers) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ float ssum[16];
   __shared__ bool last_s;
   __shared__ unsigned long long cand[16][4];
-  One<S> m{p, layers};
+  One<S, PAIR> m{p, layers};
   const int tid = threadIdx.x, lane = tid & 31;
   m.tid = tid; m.lane = lane; m.warp = tid >> 5; m.grp = tid >> 8; m.gtid = tid & 255; m.gwarp = m.gtid >> 5;
   m.gidx = m.grp * gridDim.x + blockIdx.x; m.ngroups = 2 * gridDim.x;
@@ -1221,7 +1215,9 @@ int launch_one(const qpam_step_args* a, const StepWs& w, cudaStream_t st) {
   const size_t smem = ((size_t)4 * 2 * a->D + 4 * row_ld(a->D >> 4) + rows_in) * sizeof(bf16) + (size_t)16 * 32 * sizeof(float4);
   QPAM_CUDA(cudaMemsetAsync(w.best, 0, (size_t)a->n * 8 + 256, st));
   void* args[] = {&p, &layers};
-  auto kern = a->state_dtype == QPAM_F32 ? (const void*)k_step_one<float> : (const void*)k_step_one<bf16>;
+  const bool pair = a->n <= 2;
+  auto kern = a->state_dtype == QPAM_F32 ? pair ? (const void*)k_step_one<float, true> : (const void*)k_step_one<float, false>
+                                         : pair ? (const void*)k_step_one<bf16, true> : (const void*)k_step_one<bf16, false>;
   const int rc = allow_smem(kern, smem);
   if (rc) return rc;
   QPAM_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(ONE_THREADS), args, smem, st));
