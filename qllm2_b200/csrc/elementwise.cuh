@@ -77,8 +77,25 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 // Approximate reciprocal / square root (about 2 ulp): the IEEE forms cost several times more issue slots, and
 // these kernels do ~10 of them per 8 bytes moved.
-__device__ __forceinline__ float frcp_(float x) { return __fdividef(1.f, x); }
-__device__ __forceinline__ float fsqrt_(float x) { return x * rsqrtf(x); }  // x >= 1e-8 here, never 0
+// The .ftz forms: the others wrap the instruction in two to four more that take care of denormal operands and results, which do not
+// occur here (sums of squares carry 1e-8, the exponential is added to 1, what is inverted is at least 1), a fifth of an
+// activation kernel's instructions.  The same bits everywhere else.
+__device__ __forceinline__ float frcp_(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float frsqrt_(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float fexp_(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+  return y;
+}
+__device__ __forceinline__ float fsqrt_(float x) { return x * frsqrt_(x); }  // x >= 1e-8 here, never 0
 // |z|, 1/(|z| + 1e-8) and 1/|z| of m2 = re^2 + im^2 + 1e-8 from ONE special-function instruction:
 // with rs = rsqrt(m2):  |z| = m2 rs,  1/(|z| + e) = rs / (1 + e rs) = rs (1 - t + t^2 - ...), t = e rs <= 1e-4
 // (m2 >= 1e-8), so the two kept terms leave an error below 1e-12.  These kernels are otherwise bound by the
@@ -87,7 +104,7 @@ struct MagInv {
   float mag, inv, rmag;
 };
 __device__ __forceinline__ MagInv mag_inv(float m2) {
-  const float rs = rsqrtf(m2);
+  const float rs = frsqrt_(m2);
   const float t = MAG_EPS * rs;
   return {m2 * rs, rs * (1.f - t + t * t), rs};
 }
@@ -97,7 +114,7 @@ __device__ __forceinline__ float sigmoid_approx(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(0.5f * x));
   return fmaf(0.5f, y, 0.5f);
 }
-__device__ __forceinline__ float sigmoidf_(float x) { return frcp_(1.f + __expf(-x)); }
+__device__ __forceinline__ float sigmoidf_(float x) { return frcp_(1.f + fexp_(-x)); }
 
 // Threads per CTA for kernels whose threads each own one group of 4 channels: the largest multiple of 32
 // (up to 256) that divides the group count, so that no CTA runs mostly idle; 256 when none does.  Up to

@@ -30,6 +30,9 @@ static cudaError_t launch_pairs(void (*kern)(KArgs...), dim3 grid, size_t smem, 
 }
 
 // ------------------------------------------------------------------ plan
+// Rows of one backward chunk: 1.65 GB of probabilities at V = 50261.  A batch of one chunk needs no fp32 buffers of dW, which
+// leaves the accumulators as bf16 (16384 rows in two chunks: two fp32 passes of 154 MB and a pass that adds them).
+constexpr int64_t CE_CHUNK_ROWS = 16384;
 CETcPlan ce_tc_plan(const qpam_ce_args* a) {
   CETcPlan pl{};
   pl.enabled = a->io_dtype == QPAM_BF16 && (a->F % 8) == 0 && a->N > 0;
@@ -54,7 +57,7 @@ CETcPlan ce_tc_plan(const qpam_ce_args* a) {
   pl.nsplit = best;
   pl.tiles_per_split = (pl.n_tiles + best - 1) / best;
   int64_t rows = ((a->N + tc::BM - 1) / tc::BM) * tc::BM;
-  if (rows > 8192) rows = 8192;
+  if (rows > CE_CHUNK_ROWS) rows = CE_CHUNK_ROWS;
   if (rows < tc::BM) rows = tc::BM;
   pl.chunk_rows = rows;
   const int64_t f_tiles = (a->F + 255) / 256;

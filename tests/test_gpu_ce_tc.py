@@ -159,3 +159,25 @@ def test_weight_gradient_tile_walk(N, D, V):
     p /= N
     assert_close(w.grad.double().cpu().numpy(), (p.T @ hd).cpu().numpy(), 2e-2, "dW")
     assert_close(h.grad.double().cpu().numpy(), (p @ wd).cpu().numpy(), 2e-2, "dH")
+
+
+@pytest.mark.parametrize("N", [16384, 16384 + 300, 4 * 16384 + 200])
+def test_row_chunks_of_the_backward(N):
+    """The largest single chunk, two, and a fifth that adds into the first one's dW."""
+    D, V = 32, 520
+    c = synthetic.ce_inputs(N, D, V, seed=12, dtype=torch.bfloat16)
+    w_host = (c.w.float() * 20).bfloat16()
+    h, w, t = c.h.to(DEV).requires_grad_(True), w_host.to(DEV).requires_grad_(True), c.targets.to(DEV)
+    loss = fused_ce.fused_linear_cross_entropy(h, w, t)
+    loss.backward()
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    hd, wd = h.detach().double(), w.detach().double()
+    z = hd @ wd.T
+    want = torch.nn.functional.cross_entropy(z, t)
+    assert abs(float(loss.detach()) - float(want)) <= 1e-5 * float(want)
+    p = torch.softmax(z, 1)
+    p[torch.arange(N, device=DEV), t] -= 1.0
+    p /= N
+    assert_close(w.grad.double().cpu().numpy(), (p.T @ hd).cpu().numpy(), 2e-2, "dW")
+    assert_close(h.grad.double().cpu().numpy(), (p @ wd).cpu().numpy(), 2e-2, "dH")
