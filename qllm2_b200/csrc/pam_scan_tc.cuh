@@ -106,7 +106,7 @@ struct FinalDest {
 //   Re U[i][j] = D1[2j][i] + D2[2j+1][i],   Im U[i][j] = D2[2j][i] - D1[2j+1][i]:  neighbouring TMEM lanes, one shuffle.
 // grid = (chunks, H, K); 256 threads; 66 KB shared memory, 128 TMEM columns: three CTAs per SM.
 // ---------------------------------------------------------------------------------------------
-constexpr size_t OUTER_SMEM = 1024 + 32768 + 32768 + 1024;
+constexpr size_t OUTER_SMEM = 1024 + 32768 + 32768 + 1536;
 
 // DSTATE == true computes the gradient counterpart  G = sum_t scale e^{A_t} dy_t (x) conj(q_t)  (dy in
 // place of v, q in place of k) into dstate slot c.
@@ -205,7 +205,8 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
   unsigned char* sA = smem;            // key tile: [2 boxes of 64 columns][128 rows][128 B]
   unsigned char* sB = smem + 32768;    // value tile, then [256 rows][128 B]: rows s = w Re v_s, rows 128 + s = w Im v_s
   float* Acum = reinterpret_cast<float*>(smem + 65536);          // [128]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(Acum + TC);       // [0] MMAs  [1] token tiles
+  float* wrow = Acum + TC;                                      // [128] weights of the tokens (each is read by 16 threads)
+  uint64_t* bar = reinterpret_cast<uint64_t*>(wrow + TC);       // [0] MMAs  [1] token tiles
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr bool CARRY = MODE == OUTER_CARRY;
@@ -237,25 +238,25 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const float a_last = Acum[TC - 1];
+  if (tid < TC) wrow[tid] = DSTATE ? p.q_scale * __expf(Acum[tid]) : __expf(fminf(0.f, a_last - Acum[tid]));      // (read behind the next barrier)
   const bool tiles_ok = mbar_wait(&bar[1], 0, 202);
   // this thread's 16-byte pieces of the value tile (rows past the chunk's end belong to someone else: their zeros
   // also cancel whatever the key tile holds in those rows)
+  // (rows 16 apart: 2 KB apart in the tile, with the same swizzle)
+  const int row0_ = tid >> 4, c16 = tid & 15;
+  const unsigned char* src = sB + (c16 >> 3) * 16384 + sw128(row0_, c16 & 7);
   uint4 vxa[8];
 #pragma unroll
   for (int it = 0; it < 8; ++it) {
-    const int idx = tid + 256 * it;
-    const int row = idx >> 4, c16 = idx & 15;
     vxa[it] = make_uint4(0, 0, 0, 0);
-    if (row < L.len) vxa[it] = *reinterpret_cast<const uint4*>(sB + (c16 >> 3) * 16384 + sw128(row, c16 & 7));
+    if (row0_ + 16 * it < L.len) vxa[it] = *reinterpret_cast<const uint4*>(src + 2048 * it);
   }
   __syncthreads();      // every piece has been read: the planes may overwrite the tile
+  unsigned char* dst_planes = sB + sw128(row0_, c16 >> 1) + (c16 & 1) * 8;
 #pragma unroll
   for (int it = 0; it < 8; ++it) {
-    const int idx = tid + 256 * it;
-    const int row = idx >> 4, c16 = idx & 15;
-    const uint4 vx = vxa[it];
-    const float w = DSTATE ? p.q_scale * __expf(Acum[row]) : __expf(fminf(0.f, a_last - Acum[row]));
-    const uint32_t vw[4] = {vx.x, vx.y, vx.z, vx.w};
+    const float w = wrow[row0_ + 16 * it];
+    const uint32_t vw[4] = {vxa[it].x, vxa[it].y, vxa[it].z, vxa[it].w};
     float vr[4], vi[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -263,9 +264,8 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
       vr[e] = w * vv.x;
       vi[e] = w * vv.y;
     }
-    const uint32_t boff = (c16 & 1) * 8;
-    *reinterpret_cast<uint2*>(sB + sw128(row, c16 >> 1) + boff) = make_uint2(pack_bf162(vr[0], vr[1]), pack_bf162(vr[2], vr[3]));
-    *reinterpret_cast<uint2*>(sB + sw128(128 + row, c16 >> 1) + boff) = make_uint2(pack_bf162(vi[0], vi[1]), pack_bf162(vi[2], vi[3]));
+    *reinterpret_cast<uint2*>(dst_planes + 2048 * it) = make_uint2(pack_bf162(vr[0], vr[1]), pack_bf162(vr[2], vr[3]));
+    *reinterpret_cast<uint2*>(dst_planes + 16384 + 2048 * it) = make_uint2(pack_bf162(vi[0], vi[1]), pack_bf162(vi[2], vi[3]));
   }
   fence_proxy_async();
   __syncthreads();
@@ -387,9 +387,11 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
   pdl_trigger();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  if (DSTATE) {
-    for (int e = tid; e < K * TC; e += 256) {          // (read after the barrier in front of the first planes)
-      const int k = e / TC, t = e - k * TC;
+  for (int e = tid; e < K * TC; e += 256) {          // (read after the barrier in front of the first planes)
+    const int k = e / TC, t = e - k * TC;
+    if (!DSTATE) {
+      wrow[e].x = __expf(fminf(0.f, Acum[k * TC + TC - 1] - Acum[e]));
+    } else {
       float2 c = make_float2(1.f, 0.f);
       if (p.coef != nullptr && t < L.len) c = __ldg(reinterpret_cast<const float2*>(p.coef + gamma_base(p, k, L.b, h, L.t0 + t) * 2));
       const float f = p.q_scale * __expf(Acum[e]);
@@ -399,13 +401,15 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
   bool ok = mbar_wait(&bar[KMAX], 0, 206);
   // this thread's 16-byte pieces of the value tile (rows past the chunk's end: zeros, which also cancel whatever the
   // key tile holds in those rows)
+  // (rows 16 apart: 2 KB apart in the tile, with the same swizzle)
+  const int row0_ = tid >> 4, c16 = tid & 15;
+  const unsigned char* src = sB + (c16 >> 3) * 16384 + sw128(row0_, c16 & 7);
+  unsigned char* dst_planes = sB + sw128(row0_, c16 >> 1) + (c16 & 1) * 8;
   uint4 vxa[8];
 #pragma unroll
   for (int it = 0; it < 8; ++it) {
-    const int idx = tid + 256 * it;
-    const int row = idx >> 4, c16 = idx & 15;
     vxa[it] = make_uint4(0, 0, 0, 0);
-    if (row < L.len) vxa[it] = *reinterpret_cast<const uint4*>(sB + (c16 >> 3) * 16384 + sw128(row, c16 & 7));
+    if (row0_ + 16 * it < L.len) vxa[it] = *reinterpret_cast<const uint4*>(src + 2048 * it);
   }
   const int q4 = warp & 3, cc = warp >> 2;   // epilogue: TMEM lane quarter, column half
   const bool even = (lane & 1) == 0;
@@ -417,10 +421,8 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
     const float a_last = Acum[k * TC + TC - 1];
 #pragma unroll
     for (int it = 0; it < 8; ++it) {
-      const int idx = tid + 256 * it;
-      const int row = idx >> 4, c16 = idx & 15;
       const uint4 vx = vxa[it];
-      const float2 w = DSTATE ? wrow[k * TC + row] : make_float2(__expf(fminf(0.f, a_last - Acum[k * TC + row])), 0.f);
+      const float2 w = DSTATE ? wrow[k * TC + row0_ + 16 * it] : make_float2(wrow[k * TC + row0_ + 16 * it].x, 0.f);
       const uint32_t vw[4] = {vx.x, vx.y, vx.z, vx.w};
       float vr[4], vi[4];
 #pragma unroll
@@ -429,9 +431,8 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
         vr[e] = DSTATE ? w.x * vv.x - w.y * vv.y : w.x * vv.x;
         vi[e] = DSTATE ? w.x * vv.y + w.y * vv.x : w.x * vv.y;
       }
-      const uint32_t boff = (c16 & 1) * 8;
-      *reinterpret_cast<uint2*>(sB + sw128(row, c16 >> 1) + boff) = make_uint2(pack_bf162(vr[0], vr[1]), pack_bf162(vr[2], vr[3]));
-      *reinterpret_cast<uint2*>(sB + sw128(128 + row, c16 >> 1) + boff) = make_uint2(pack_bf162(vi[0], vi[1]), pack_bf162(vi[2], vi[3]));
+      *reinterpret_cast<uint2*>(dst_planes + 2048 * it) = make_uint2(pack_bf162(vr[0], vr[1]), pack_bf162(vr[2], vr[3]));
+      *reinterpret_cast<uint2*>(dst_planes + 16384 + 2048 * it) = make_uint2(pack_bf162(vi[0], vi[1]), pack_bf162(vi[2], vi[3]));
     }
     fence_proxy_async();
     __syncthreads();
