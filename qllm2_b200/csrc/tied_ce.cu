@@ -109,7 +109,7 @@ static int ce_partial_t(const qpam_ce_args* a, const CELayout& L, float* row_max
   const int64_t nrt = (a->N + CE_TM - 1) / CE_TM;
   k_ce_partial<T><<<dim3(L.nsplit, (unsigned)nrt), 256, 0, st>>>(p);
   QPAM_LAUNCH_CHECK("k_ce_partial");
-  k_ce_merge<<<(unsigned)((a->N + 255) / 256), 256, 0, st>>>(p, row_max, row_sumexp, row_tgt, row_argmax);
+  k_ce_merge<<<(unsigned)((a->N + MERGE_ROWS - 1) / MERGE_ROWS), 256, 0, st>>>(p, row_max, row_sumexp, row_tgt, row_argmax);
   QPAM_LAUNCH_CHECK("k_ce_merge");
   return QPAM_OK;
 }
@@ -178,7 +178,7 @@ extern "C" int qpam_ce_partial(const qpam_ce_args* a, float* row_max, float* row
     if (rc) return rc;
     CEParams p = ce_params(a, L);
     p.nsplit = L.tc.nsplit;
-    launch_after(k_ce_merge, (unsigned)((a->N + 255) / 256), 256, 0, st, p, row_max, row_sumexp, row_tgt, row_argmax);
+    launch_after(k_ce_merge, (unsigned)((a->N + MERGE_ROWS - 1) / MERGE_ROWS), 256, 0, st, p, row_max, row_sumexp, row_tgt, row_argmax);
     QPAM_LAUNCH_CHECK("k_ce_merge");
     return QPAM_OK;
   }

@@ -168,25 +168,48 @@ __global__ void __launch_bounds__(256) k_ce_partial(CEParams p) {
   }
 }
 
-__global__ void k_ce_merge(CEParams p, float* row_max, float* row_sumexp, float* row_tgt, int64_t* row_argmax) {
+// A CTA folds the vocabulary splits of 32 rows, eight threads a row.  A thread a row walked up to 197 splits one after another, which
+// was a third of a greedy head's time: head of 256 rows x 768 x 50261 34.0 -> 25.2 us, 17 rows 36.3 -> 26.2, 4096 rows 205.3 -> 204.3.
+constexpr int MERGE_ROWS = 32;
+__global__ void __launch_bounds__(256) k_ce_merge(CEParams p, float* row_max, float* row_sumexp, float* row_tgt, int64_t* row_argmax) {
+  __shared__ float sm[8][MERGE_ROWS], ss[8][MERGE_ROWS], st_[8][MERGE_ROWS], sb[8][MERGE_ROWS];
+  __shared__ int si[8][MERGE_ROWS];
   pdl_trigger();
   pdl_wait();
-  const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= p.N) return;
-  float M = -INFINITY;
-  for (int s = 0; s < p.nsplit; ++s) M = fmaxf(M, p.pm[(size_t)s * p.N + n]);
-  float S = 0.f, tz = 0.f, best = -INFINITY;
+  const int r = threadIdx.x & 31, part = threadIdx.x >> 5;
+  const int64_t n = (int64_t)blockIdx.x * MERGE_ROWS + r;
+  float M = -INFINITY, S = 0.f, tz = 0.f, best = -INFINITY;
   int bi = 0x7fffffff;
-  for (int s = 0; s < p.nsplit; ++s) {
-    const size_t o = (size_t)s * p.N + n;
-    S += p.ps[o] * expf(p.pm[o] - M);
-    tz += p.pt[o];
-    const float b = p.pbest[o];
-    const int i = p.pidx[o];
-    if (b > best || (b == best && i < bi)) {
-      best = b;
-      bi = i;
+  if (n < p.N)
+    for (int s = part; s < p.nsplit; s += 8) M = fmaxf(M, p.pm[(size_t)s * p.N + n]);
+  sm[part][r] = M;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) M = fmaxf(M, sm[q][r]);
+  if (n < p.N)
+    for (int s = part; s < p.nsplit; s += 8) {
+      const size_t o = (size_t)s * p.N + n;
+      S += p.ps[o] * expf(p.pm[o] - M);
+      tz += p.pt[o];
+      const float b = p.pbest[o];
+      const int i = p.pidx[o];
+      if (b > best || (b == best && i < bi)) {
+        best = b;
+        bi = i;
+      }
     }
+  ss[part][r] = S;
+  st_[part][r] = tz;
+  sb[part][r] = best;
+  si[part][r] = bi;
+  __syncthreads();
+  if (part != 0 || n >= p.N) return;
+#pragma unroll
+  for (int q = 1; q < 8; ++q) {
+    S += ss[q][r];
+    tz += st_[q][r];
+    const float b = sb[q][r];
+    if (b > best || (b == best && si[q][r] < bi)) { best = b; bi = si[q][r]; }
   }
   if (row_max) row_max[n] = M;
   if (row_sumexp) row_sumexp[n] = S;

@@ -97,3 +97,29 @@ def test_empty_batch():
     loss = fused_ce.fused_linear_cross_entropy(h, w, t)
     loss.backward()
     assert float(loss) == 0.0 and float(w.grad.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("dtype,N,V", [(torch.float32, 1, 5), (torch.float32, 33, 2000), (torch.bfloat16, 31, 700), (torch.bfloat16, 257, 9001)])
+def test_row_statistics_merge_over_splits(dtype, N, V):
+    """The vocabulary splits' statistics of a row folded by eight threads: equal best logits in several splits give the lowest id, a
+    row of NaN the first one; max and sum of exponentials against float64 (the logits are exact: one 1 per row, powers of two)."""
+    h = torch.zeros(N, 8, device=DEV, dtype=dtype)
+    h[:, 0] = 1
+    h[N // 2, 1] = 1
+    w = torch.zeros(V, 8, device=DEV, dtype=dtype)
+    w[:, 0] = torch.arange(V, device=DEV).remainder(4).to(dtype) * -0.5          # many equal logits of 0
+    w[V // 2, 1] = w[V - 1, 1] = w[V // 3, 1] = 4
+    w[V // 3, 0] = w[V // 2, 0] = w[V - 1, 0] = 0                             # row N // 2: three equal best logits
+    if N > 1:
+        h[N - 1] = float("nan")
+    t = torch.full((N,), V - 1, device=DEV)
+    m, s, tz, arg = ops.ce_row_stats(h, w, t)
+    z = h.double() @ w.double().T
+    ok = slice(0, N - 1 if N > 1 else N)
+    assert torch.equal(m[ok].double(), z[ok].max(1).values) and torch.equal(tz[ok].double(), z[ok, V - 1])
+    want = torch.exp(z[ok] - z[ok].max(1, keepdim=True).values).sum(1)
+    assert float(((s[ok] - want) / want).abs().max()) < 2e-5
+    assert int(arg[N // 2]) == (V // 3 if N // 2 != N - 1 or N == 1 else 0)
+    assert torch.equal(arg[: N // 2], torch.zeros_like(arg[: N // 2]))
+    if N > 1:
+        assert int(arg[N - 1]) == 0
