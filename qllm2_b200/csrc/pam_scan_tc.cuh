@@ -413,28 +413,66 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
   }
   const int q4 = warp & 3, cc = warp >> 2;   // epilogue: TMEM lane quarter, column half
   const bool even = (lane & 1) == 0;
-  for (int k = 0; k < K; ++k) {
-    // every piece has been read (k = 0) / the previous state's MMAs have read the planes and its epilogue the
-    // accumulators (k > 0: every thread waited for them below)
-    tc_fence_before();
-    __syncthreads();
-    const float a_last = Acum[k * TC + TC - 1];
+  __syncthreads();      // every piece has been read
+  // A state's planes are written as soon as the previous one's MMAs have read theirs, and the previous one's sums leave the accumulators
+  // after that: one barrier a state, and the passes of different warps overlap.  With the sums in groups of 8 columns (the value tile
+  // stays in registers beside them) 48 chat prompts took 310 instead of 322 us, 8 x 6 x 2048 with three states 395 instead of 398.
+#pragma unroll 1
+  for (int k = 0; k <= K; ++k) {
+    if (k < K) {
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      const uint4 vx = vxa[it];
-      const float2 w = DSTATE ? wrow[k * TC + row0_ + 16 * it] : make_float2(wrow[k * TC + row0_ + 16 * it].x, 0.f);
-      const uint32_t vw[4] = {vx.x, vx.y, vx.z, vx.w};
-      float vr[4], vi[4];
+      for (int it = 0; it < 8; ++it) {
+        const uint4 vx = vxa[it];
+        const float2 w = DSTATE ? wrow[k * TC + row0_ + 16 * it] : make_float2(wrow[k * TC + row0_ + 16 * it].x, 0.f);
+        const uint32_t vw[4] = {vx.x, vx.y, vx.z, vx.w};
+        float vr[4], vi[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 vv = unpack_bf162(vw[e]);
-        vr[e] = DSTATE ? w.x * vv.x - w.y * vv.y : w.x * vv.x;
-        vi[e] = DSTATE ? w.x * vv.y + w.y * vv.x : w.x * vv.y;
+        for (int e = 0; e < 4; ++e) {
+          const float2 vv = unpack_bf162(vw[e]);
+          vr[e] = DSTATE ? w.x * vv.x - w.y * vv.y : w.x * vv.x;
+          vi[e] = DSTATE ? w.x * vv.y + w.y * vv.x : w.x * vv.y;
+        }
+        *reinterpret_cast<uint2*>(dst_planes + 2048 * it) = make_uint2(pack_bf162(vr[0], vr[1]), pack_bf162(vr[2], vr[3]));
+        *reinterpret_cast<uint2*>(dst_planes + 16384 + 2048 * it) = make_uint2(pack_bf162(vi[0], vi[1]), pack_bf162(vi[2], vi[3]));
       }
-      *reinterpret_cast<uint2*>(dst_planes + 2048 * it) = make_uint2(pack_bf162(vr[0], vr[1]), pack_bf162(vr[2], vr[3]));
-      *reinterpret_cast<uint2*>(dst_planes + 16384 + 2048 * it) = make_uint2(pack_bf162(vi[0], vi[1]), pack_bf162(vi[2], vi[3]));
     }
+    if (k > 0) {
+      // Re U = D1[2j] + D2[2j+1], Im U = D2[2j] - D1[2j+1]: lane n' = 2j+c holds column i, state[i][j][c] at i*128 + n'
+      float2* slot = DSTATE ? p.dstates + state_base(p, k - 1, h, L.slot0 + L.c, TD) : p.states + state_base(p, k - 1, h, L.slot0 + L.c + 1, TD);
+      float* dst = reinterpret_cast<float*>(slot) + (q4 * 32 + lane);
+      const bool final_now = !DSTATE && (p.fwd_only || p.single) && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
+#pragma unroll 1
+      for (int hh = 0; hh < 4; ++hh) {          // 8 columns at a time
+        float d1[8], d2[8];
+        const uint32_t col = (uint32_t)(cc * 32 + hh * 8);
+        tmem_ld8x2(tmem + ((uint32_t)(q4 * 32) << 16) + col, d1, tmem + ((uint32_t)(q4 * 32) << 16) + 64 + col, d2);
+        if (final_now) {
+          FinalDest fin;
+          fin.init(p, L.seq, k - 1, h);
+#pragma unroll
+          for (int i = 0; i < 8; i += 2) {
+            const float o0 = __shfl_xor_sync(0xffffffffu, d2[i], 1), o1 = __shfl_xor_sync(0xffffffffu, d2[i + 1], 1);
+            const float u0 = even ? d1[i] + o0 : o0 - d1[i], u1 = even ? d1[i + 1] + o1 : o1 - d1[i + 1];
+            fin.store2(p, (int)(col + i) * 128 + q4 * 32 + lane, u0, u1, even, ok);
+            if (p.single && ok) {
+              dst[(size_t)(col + i) * 128] = u0;
+              dst[(size_t)(col + i + 1) * 128] = u1;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float other = __shfl_xor_sync(0xffffffffu, d2[i], 1);
+            const float u = even ? d1[i] + other : other - d1[i];
+            if (ok) dst[(size_t)(col + i) * 128] = u;
+          }
+        }
+      }
+      if (ok && !DSTATE && tid == 0) p.chunk_decay[((size_t)(k - 1) * p.H + h) * p.nslots + L.slot0 + L.c + 1] = __expf(Acum[(k - 1) * TC + TC - 1]);
+    }
+    if (k == K) break;
     fence_proxy_async();
+    tc_fence_before();
     __syncthreads();
     if (warp == 0 && elect_one()) {
       tc_fence_after();
@@ -447,38 +485,6 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
     __syncwarp();
     ok = mbar_wait(&bar[k], 0, 205) && ok;
     tc_fence_after();
-    // Re U = D1[2j] + D2[2j+1], Im U = D2[2j] - D1[2j+1]: lane n' = 2j+c holds column i, state[i][j][c] at i*128 + n'
-    float2* slot = DSTATE ? p.dstates + state_base(p, k, h, L.slot0 + L.c, TD) : p.states + state_base(p, k, h, L.slot0 + L.c + 1, TD);
-    float* dst = reinterpret_cast<float*>(slot) + (q4 * 32 + lane);
-    const bool final_now = !DSTATE && (p.fwd_only || p.single) && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
-#pragma unroll 1
-    for (int hh = 0; hh < 2; ++hh) {          // 16 columns at a time: the value tile stays in registers beside them
-      float d1[16], d2[16];
-      const uint32_t col = (uint32_t)(cc * 32 + hh * 16);
-      tmem_ld16x2(tmem + ((uint32_t)(q4 * 32) << 16) + col, d1, tmem + ((uint32_t)(q4 * 32) << 16) + 64 + col, d2);
-      if (final_now) {
-        FinalDest fin;
-        fin.init(p, L.seq, k, h);
-#pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          const float o0 = __shfl_xor_sync(0xffffffffu, d2[i], 1), o1 = __shfl_xor_sync(0xffffffffu, d2[i + 1], 1);
-          const float u0 = even ? d1[i] + o0 : o0 - d1[i], u1 = even ? d1[i + 1] + o1 : o1 - d1[i + 1];
-          fin.store2(p, (int)(col + i) * 128 + q4 * 32 + lane, u0, u1, even, ok);
-          if (p.single && ok) {
-            dst[(size_t)(col + i) * 128] = u0;
-            dst[(size_t)(col + i + 1) * 128] = u1;
-          }
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float other = __shfl_xor_sync(0xffffffffu, d2[i], 1);
-          const float u = even ? d1[i] + other : other - d1[i];
-          if (ok) dst[(size_t)(col + i) * 128] = u;
-        }
-      }
-    }
-    if (ok && !DSTATE && tid == 0) p.chunk_decay[((size_t)k * p.H + h) * p.nslots + L.slot0 + L.c + 1] = __expf(a_last);
   }
   tc_fence_before();
   __syncthreads();
