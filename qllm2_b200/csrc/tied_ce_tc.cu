@@ -30,9 +30,39 @@ static cudaError_t launch_pairs(void (*kern)(KArgs...), dim3 grid, size_t smem, 
 }
 
 // ------------------------------------------------------------------ plan
-// Rows of one backward chunk: 1.65 GB of probabilities at V = 50261.  A batch of one chunk needs no fp32 buffers of dW, which
-// leaves the accumulators as bf16 (16384 rows in two chunks: two fp32 passes of 154 MB and a pass that adds them).
-constexpr int64_t CE_CHUNK_ROWS = 16384;
+// Rows of one backward chunk.  Chunks of 8192 rows run their products at the tensor rate (0.82 GB of probabilities at V = 50261);
+// what several of them cost is dW, which goes through one fp32 buffer a chunk and a pass that adds those (one chunk: bf16
+// straight from the accumulators).  So more rows than that are one chunk where that takes no more scratch than the chunks and
+// their buffers (up to about 8192 + 4 F rows), and no call needs more than with chunks of 8192.  V = 50261, F = 768, forward and
+// backward, one chunk / two: 10240 rows 2.60 ms and 1.16 GB / 2.74 ms and 1.30 GB; 16384 rows 3.55 ms and 1.91 GB / 3.61 ms and
+// 1.32 GB, which is why those are two.
+constexpr int64_t CE_CHUNK_ROWS = 8192;
+
+// Chunks of `rows` rows: split-K of dH, fp32 buffers of dW; returns the bytes of scratch that depend on them.
+static int64_t plan_chunks(const qpam_ce_args* a, int64_t rows, CETcPlan& pl) {
+  const int sms = sm_count();
+  const int64_t f_tiles = (a->F + 255) / 256;
+  pl.chunk_rows = rows;
+  // split-K of dH: one CTA per SM, so the cost is (waves of CTAs) x (K blocks per split), in K blocks of ~0.55 us, and the
+  // fp32 partials of a split are written and read once more (~5 TB/s).  Few rows take many splits: 509 rows x 768 use 48 of
+  // 148 SMs with eight (77 us) and all of them with 24 (38 us).
+  const int64_t kb_total = (a->V + tc::BK - 1) / tc::BK;
+  int64_t ks = 1, ks_cost = -1;
+  for (int64_t s = 1; s <= 48 && s <= kb_total; ++s) {
+    const int64_t ctas = f_tiles * ((rows + 2 * tc::BM - 1) / (2 * tc::BM)) * s;     // CTAs of two row tiles
+    const int64_t cost = ((ctas + sms - 1) / sms) * ((kb_total + s - 1) / s + 8) +      // + 8: prologue and epilogue of a CTA
+                         s * rows * a->F * 8 / 2750000;
+    if (ks_cost < 0 || cost < ks_cost) { ks_cost = cost; ks = s; }
+  }
+  pl.ksplit = (int32_t)ks;
+  // every row chunk (up to 4) sums its dW into a buffer of its own: adding into one buffer made the epilogue
+  // of the later chunks read what it writes (+50 % on that launch); the final bf16 pass adds the buffers
+  const int64_t n_chunks = (a->N + rows - 1) / rows;
+  // (one row chunk needs none: its dW leaves the accumulators as bf16)
+  pl.dw_bufs = (int32_t)(n_chunks <= 1 ? 0 : (n_chunks > 4 ? 4 : n_chunks));
+  return rows * ((a->V + 63) & ~(int64_t)63) * 2 + ks * rows * a->F * 4 + pl.dw_bufs * a->V * a->F * 4;
+}
+
 CETcPlan ce_tc_plan(const qpam_ce_args* a) {
   CETcPlan pl{};
   pl.enabled = a->io_dtype == QPAM_BF16 && (a->F % 8) == 0 && a->N > 0;
@@ -57,27 +87,12 @@ CETcPlan ce_tc_plan(const qpam_ce_args* a) {
   pl.nsplit = best;
   pl.tiles_per_split = (pl.n_tiles + best - 1) / best;
   int64_t rows = ((a->N + tc::BM - 1) / tc::BM) * tc::BM;
-  if (rows > CE_CHUNK_ROWS) rows = CE_CHUNK_ROWS;
   if (rows < tc::BM) rows = tc::BM;
-  pl.chunk_rows = rows;
-  const int64_t f_tiles = (a->F + 255) / 256;
-  // split-K of dH: one CTA per SM, so the cost is (waves of CTAs) x (K blocks per split), in K blocks of ~0.55 us, and the
-  // fp32 partials of a split are written and read once more (~5 TB/s).  Few rows take many splits: 509 rows x 768 use 48 of
-  // 148 SMs with eight (77 us) and all of them with 24 (38 us).
-  const int64_t kb_total = (a->V + tc::BK - 1) / tc::BK;
-  int64_t ks = 1, ks_cost = -1;
-  for (int64_t s = 1; s <= 48 && s <= kb_total; ++s) {
-    const int64_t ctas = f_tiles * ((rows + 2 * tc::BM - 1) / (2 * tc::BM)) * s;     // CTAs of two row tiles
-    const int64_t cost = ((ctas + sms - 1) / sms) * ((kb_total + s - 1) / s + 8) +      // + 8: prologue and epilogue of a CTA
-                         s * rows * a->F * 8 / 2750000;
-    if (ks_cost < 0 || cost < ks_cost) { ks_cost = cost; ks = s; }
+  const int64_t all = plan_chunks(a, rows, pl);
+  if (rows > CE_CHUNK_ROWS) {
+    CETcPlan chunks = pl;
+    if (plan_chunks(a, CE_CHUNK_ROWS, chunks) < all) pl = chunks;
   }
-  pl.ksplit = (int32_t)ks;
-  // every row chunk (up to 4) sums its dW into a buffer of its own: adding into one buffer made the epilogue
-  // of the later chunks read what it writes (+50 % on that launch); the final bf16 pass adds the buffers
-  const int64_t n_chunks = (a->N + rows - 1) / rows;
-  // (one row chunk needs none: its dW leaves the accumulators as bf16)
-  pl.dw_bufs = (int32_t)(n_chunks <= 1 ? 0 : (n_chunks > 4 ? 4 : n_chunks));
   return pl;
 }
 

@@ -92,6 +92,25 @@ def test_workspace_sizes(lib):
     assert lib.qpam_ce_workspace_bytes(C.byref(ce), 1) > lib.qpam_ce_workspace_bytes(C.byref(ce), 0) > 0
 
 
+@pytest.mark.parametrize("F", [32, 256, 768, 1536])
+@pytest.mark.parametrize("V", [32000, 50261, 262144])
+def test_loss_scratch_is_bounded_by_chunks_of_8192_rows(lib, V, F):
+    """However many rows a loss has, its backward needs no more scratch than the probabilities, the split sums of dH and the (at
+    most four) fp32 dW of chunks of 8192 rows: what a batch of 8192 takes, and those buffers.  (Below some 16 thousand words the
+    256 MB that the CUDA-core path may ask for are more.)"""
+    from qllm2_b200 import _lib
+
+    def scratch(N):
+        ce = _lib.CEArgs()
+        ce.N, ce.V, ce.F, ce.io_dtype = N, V, F, _lib.QPAM_BF16
+        return lib.qpam_ce_workspace_bytes(C.byref(ce), 1) - lib.qpam_ce_workspace_bytes(C.byref(ce), 0)
+
+    for N in (8193, 8192 + 128, 10240, 8192 + 4 * F, 16384, 16385, 20000, 40000, 65536):
+        assert scratch(N) <= scratch(8192) + min(4, -(-N // 8192)) * V * F * 4 + 4096, N
+    if F > 256:       # one chunk where that is the smaller: no fp32 dW beside it
+        assert scratch(10240) < scratch(8192) + 2 * V * F * 4
+
+
 def test_ops_fail_loudly_without_cuda():
     import torch
     from qllm2_b200 import _lib, ops

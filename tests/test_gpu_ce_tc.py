@@ -141,7 +141,7 @@ def test_head_logits_bf16_tiles(N, F, V):
 
 @pytest.mark.parametrize("N,D,V", [
     (65, 260, 20001),           # 79 x 3 tiles of dW, more than pairs of SMs: ragged in both directions
-    (8192 + 65, 260, 20001),    # the same over two row chunks (fp32 sums)
+    (12000, 260, 20001),        # the same over two row chunks (fp32 sums)
     (70, 130, 257),             # fewer tiles than pairs; the second row tile of the last pair has one row
 ])
 def test_weight_gradient_tile_walk(N, D, V):
@@ -161,10 +161,12 @@ def test_weight_gradient_tile_walk(N, D, V):
     assert_close(h.grad.double().cpu().numpy(), (p @ wd).cpu().numpy(), 2e-2, "dH")
 
 
-@pytest.mark.parametrize("N", [16384, 16384 + 300, 4 * 16384 + 200])
-def test_row_chunks_of_the_backward(N):
-    """The largest single chunk, two, and a fifth that adds into the first one's dW."""
-    D, V = 32, 520
+@pytest.mark.parametrize("N,D,V", [
+    (8192, 32, 520),           # the largest batch that is one chunk whatever its width
+    (11600, 384, 20001),       # one: less scratch than two with their fp32 dW
+    (12000, 260, 20001),       # two
+])
+def test_row_chunks_of_the_backward(N, D, V):
     c = synthetic.ce_inputs(N, D, V, seed=12, dtype=torch.bfloat16)
     w_host = (c.w.float() * 20).bfloat16()
     h, w, t = c.h.to(DEV).requires_grad_(True), w_host.to(DEV).requires_grad_(True), c.targets.to(DEV)
@@ -181,3 +183,22 @@ def test_row_chunks_of_the_backward(N):
     p /= N
     assert_close(w.grad.double().cpu().numpy(), (p.T @ hd).cpu().numpy(), 2e-2, "dW")
     assert_close(h.grad.double().cpu().numpy(), (p @ wd).cpu().numpy(), 2e-2, "dH")
+
+
+def test_weight_gradient_of_one_chunk_and_of_two():
+    """10000 rows of 768 columns are one chunk (one chain of fp32 sums, to bf16 at its end), of 192 two (two chains added in fp32).
+    Columns of zeros change neither the logits nor the others' sums: both are as far from float64, to a tenth."""
+    N, V, wide = 10000, 20001, 768
+    c = synthetic.ce_inputs(N, 96, V, seed=3, dtype=torch.bfloat16)
+    h, w, t = c.h.to(DEV), (c.w.float() * 20).bfloat16().to(DEV), c.targets.to(DEV)
+    F = h.shape[1]
+    p = torch.softmax(h.double() @ w.double().T, 1)
+    p[torch.arange(N, device=DEV), t] -= 1.0
+    want = (p.T @ h.double()) / N
+    far = []
+    for width in (F, wide):
+        hw, ww = (torch.nn.functional.pad(x, (0, width - F)).requires_grad_(True) for x in (h, w))
+        fused_ce.fused_linear_cross_entropy(hw, ww, t).backward()
+        assert not ww.grad[:, F:].any()
+        far.append(float((ww.grad[:, :F].double() - want).norm() / want.norm()))
+    assert far[0] <= 2e-2 and far[1] <= 1.1 * far[0], far
