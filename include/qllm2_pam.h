@@ -251,6 +251,8 @@ int qpam_head_logits(const qpam_ce_args* args, void* logits, int64_t ld, void* s
  * without a host round trip.  The draw is the inverse CDF in vocabulary order of uniforms[row] in [0,1), which
  * the caller supplies (the reference draws with torch.multinomial: same distribution, different stream of random
  * numbers).  top_k == 0 and top_p == 0 (or >= 1) switch the filters off, repetition_penalty == 1 the penalty.
+ * Masses are fp32 numbers relative to the largest, e^(x - max): a token more than about 103 below the maximum (in
+ * units of the temperature) has none, is not counted and cannot be drawn.
  *   logits      [n, V] (row stride ld_logits), fp32 or bf16
  *   history     optional int64 [n_hist_rows, ld_hist]: token ids of every sequence so far; row r of the logits
  *               uses history row slot_ids[r] (or r when slot_ids is NULL; a slot outside [0, n_hist_rows) marks a

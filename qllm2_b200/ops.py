@@ -316,7 +316,8 @@ def sample_logits(logits, uniforms=None, *, temperature: float = 1.0, top_k: int
     repetition penalty over `history` (int64 [rows, cols] token ids; `hist_len` int32 [rows] valid entries per
     row, `slot_ids` int32 [n] maps logits rows to history rows), top-k, top-p, then the inverse-CDF draw of
     `uniforms` [n] (default: torch.rand on the logits' device, i.e. torch's generator).  `append=True` also writes
-    the drawn id behind the row's history and advances `hist_len`.  Returns ids int64 [n] (and, with
+    the drawn id behind the row's history and advances `hist_len`.  Masses are float32, e^((x - max) / temperature): a
+    token more than about 103 temperatures below the maximum has none.  Returns ids int64 [n] (and, with
     `return_stats`, float32 [n,4] = (max, kept mass, kept count, mass after top-k))."""
     L = _lib.lib()
     _require_cuda(logits)

@@ -161,3 +161,25 @@ def test_infinite_temperature_and_masked_logits():
     for cfg in (dict(top_k=20), dict(top_p=0.9), dict()):
         ids, stats = ops.sample_logits(logits, u, return_stats=True, **cfg)
         assert (ids < 10).all() and (stats[:, 2] <= 10).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("cfg", [dict(), dict(top_k=20), dict(top_k=500), dict(repetition_penalty=1.2)])
+def test_tokens_far_below_the_maximum_at_a_low_temperature(dtype, cfg):
+    """At temperature 0.05 a logit 4.5 below the maximum has the mass e^-90, a denormal number: it is counted and can be drawn
+    (fp32 masses reach down to e^-103), whichever way the row takes; beyond that a token has no mass."""
+    V = 1000
+    gaps = torch.full((V,), 130.0)
+    gaps[:12] = torch.tensor([95.0, 0.0, 20.0, 50.0, 86.0, 88.5, 91.0, 99.0, 100.5, 106.0, 107.0, 110.0])
+    gaps[V - 1] = 98.0
+    logits = (gaps * -0.05).to(dtype).to(DEV)[None].expand(3, V).contiguous()
+    scaled = logits[0].double().cpu() / 0.05
+    far = scaled.max() - scaled
+    assert not ((far > 102.5) & (far < 104.5)).any()            # e^-102.5 is above the smallest number, e^-104.5 below its half
+    massive = far < 103.5
+    u = torch.tensor([0.0, 0.5, 1.0 - 2.0 ** -24], device=DEV)
+    hist = torch.tensor([[V - 2]] * 3, device=DEV)              # (a token without mass, whatever the penalty)
+    ids, stats = ops.sample_logits(logits, u, temperature=0.05, history=hist, return_stats=True, **cfg)
+    assert (stats[:, 2] == int(massive.sum())).all(), (stats[:, 2], int(massive.sum()))
+    assert ids.tolist() == [0, 1, 1]                            # u = 0: the first token with any mass
+    assert torch.allclose(stats[:, 1].double().cpu(), torch.exp(-far).sum().expand(3), rtol=1e-6)
