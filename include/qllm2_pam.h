@@ -524,6 +524,11 @@ int qpam_device_status(int32_t* status, int32_t clear);
  * library, exercised without hanging or faulting anything.  (No counterpart in the reference.) */
 int qpam_selftest_wait_expiry(int64_t limit_ns, void* stream);
 
+/* Diagnostic: y[i] = f(x[i]) for one of the approximate special functions that the element-wise kernels and the sampler
+ * are built on: 0 e^x with results below 2^-126 as zero, 1 1/x, 2 1/sqrt(x), 3 the logistic function, 4 e^x with gradual
+ * underflow.  x, y: n floats.  (No counterpart in the reference.) */
+int qpam_selftest_special(int32_t which, const float* x, float* y, int64_t n, void* stream);
+
 const char* qpam_last_error(void);
 /* "qllm2_pam_b200 <version> sm_100a" */
 const char* qpam_version(void);

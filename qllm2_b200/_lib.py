@@ -152,6 +152,7 @@ SIGNATURES = {
     "qpam_profile_end": (c_int32, [C.c_char_p, c_size_t]),
     "qpam_device_status": (c_int32, [C.POINTER(c_int32), c_int32]),
     "qpam_selftest_wait_expiry": (c_int32, [c_int64, c_void_p]),
+    "qpam_selftest_special": (c_int32, [c_int32, c_void_p, c_void_p, c_int64, c_void_p]),
     "qpam_last_error": (C.c_char_p, []),
     "qpam_version": (C.c_char_p, []),
 }

@@ -1059,3 +1059,23 @@ extern "C" int qpam_state_combine_tokens_bwd(const void* const* yk, const float*
   QPAM_REQUIRE(B > 0 && H > 0 && T > 0, "state_combine_tokens: empty shape");
   return state_combine(true, yk, dyk, coef, const_cast<void*>(dy), dcoef, dtype, K, (int64_t)B * H * T, d, stream, H, T);
 }
+
+namespace qpam {
+namespace {
+// the special functions of elementwise.cuh over an array
+__global__ void __launch_bounds__(256) k_special_selftest(int which, const float* __restrict__ x, float* __restrict__ y, int64_t n) {
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+    const float v = x[i];
+    y[i] = which == 0 ? fexp_(v) : which == 1 ? frcp_(v) : which == 2 ? frsqrt_(v) : which == 3 ? sigmoidf_(v) : fexp_gradual_(v);
+  }
+}
+}  // namespace
+}  // namespace qpam
+
+extern "C" int qpam_selftest_special(int32_t which, const float* x, float* y, int64_t n, void* stream) {
+  QPAM_REQUIRE(which >= 0 && which <= 4 && x && y && n > 0, "special-function self-test: which outside [0, 4], NULL pointer or no element");
+  cudaStream_t st = (cudaStream_t)stream;
+  k_special_selftest<<<(unsigned)std::min<int64_t>((n + 255) / 256, sm_count() * 8), 256, 0, st>>>(which, x, y, n);
+  QPAM_LAUNCH_CHECK("k_special_selftest");
+  return QPAM_OK;
+}

@@ -29,7 +29,7 @@
 // 256 rows x 50261 bf16 logits with a penalty over 16..513 tokens (a call, device): top-k 50 + top-p 0.9 34.8 -> 20.8 us; top-p 0.9 alone
 // 124 -> 82; neither 54 -> 29.  One row: 19 -> 16.7, 66 -> 51, 29 -> 19.8.  (Before: eight tests and a division for every group of
 // a pass, the small top-k reading the whole row twice, one warp walking the stretch of the draw.)
-#include "common.cuh"
+#include "elementwise.cuh"
 
 namespace qpam {
 namespace {
@@ -268,14 +268,10 @@ __device__ __forceinline__ int bin_of(float x, float mx) {      // (the conversi
 }
 // Unnormalised probability e^(x - mx): fp32 with gradual underflow, so a token counts (and can be drawn) down to about 103 below the
 // maximum.
-__device__ __forceinline__ float mass_of(float x, float mx) { return __expf(x - mx); }
-// The same where it is only a term of a sum that also holds the maximum's 1, as e^y = 2^(y log2 e) with results below 2^-126
-// taken as zero: they vanish in such a sum.  Top-p without top-k, 256 rows: 82 us against 86.
-__device__ __forceinline__ float mass_term(float x, float mx) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"((x - mx) * 1.4426950408889634f));
-  return y;
-}
+__device__ __forceinline__ float mass_of(float x, float mx) { return ew::fexp_gradual_(x - mx); }
+// The same where it is only a term of a sum that also holds the maximum's 1: results below 2^-126 are zero, as they vanish in such
+// a sum.  Top-p without top-k, 256 rows: 82 us against 86.
+__device__ __forceinline__ float mass_term(float x, float mx) { return ew::fexp_(x - mx); }
 // What few elements of a pass need stays out of line: 32 copies of it in a loop that jumps over them cost more than the pass.
 __device__ __noinline__ void list_bin_value(Scratch* sc, float x, float mx, int i, int cross, uint32_t key_k) {
   if (bin_of(x, mx) != cross || order_key(x) < key_k) return;

@@ -358,3 +358,43 @@ def test_state_combine_token_major_with_gradients():
     gb = torch.autograd.grad((y.transpose(1, 2).reshape(B, T, H * d, 2) * dy).sum(), [coef] + yks)
     for a, b in zip(ga, gb):
         assert torch.allclose(a, b, rtol=1e-5, atol=1e-5)
+
+
+EPS = 2.0 ** -22        # largest relative error of the approximate instructions (documented: 2^-22, 2^-23 over [1, 2), 2^-22.4)
+
+
+@pytest.mark.parametrize("which,name,lo,hi,fn,bound", [
+    # e^x = 2^(x log2 e): the product is rounded and so is its constant, together below |x| 2^-23 of the result
+    (0, "exp", -87.3, 88.0, torch.exp, lambda x, y: EPS + x.abs() * 2.0 ** -23),
+    (1, "reciprocal", 1.0, 2.0 ** 126, torch.reciprocal, lambda x, y: torch.full_like(x, EPS)),
+    (2, "reciprocal root", 1e-8, 1e30, torch.rsqrt, lambda x, y: torch.full_like(x, EPS)),
+    # 1 / (1 + e^-x): the exponential's error times its share of the sum, the sum's rounding, the reciprocal
+    (3, "logistic", -87.0, 100.0, torch.sigmoid, lambda x, y: 2 * EPS + 2.0 ** -24 + (1 - y) * x.abs() * 2.0 ** -23),
+    # with gradual underflow: half a denormal step besides
+    (4, "exp to denormals", -103.0, 0.0, torch.exp, lambda x, y: EPS + x.abs() * 2.0 ** -23 + 2.0 ** -150 / y),
+])
+def test_special_functions_against_float64(which, name, lo, hi, fn, bound):
+    from qllm2_b200 import _lib
+    n = 1 << 20
+    g = torch.Generator(device=DEV).manual_seed(which)
+    r = torch.rand(n, device=DEV, generator=g, dtype=torch.float64)
+    x = (torch.exp(np.log(lo) + r * np.log(hi / lo)) if lo > 0 else lo + r * (hi - lo)).float().clamp(lo, hi)
+    x[0], x[1] = lo, hi
+    y = torch.empty_like(x)
+    _lib.check(_lib.lib().qpam_selftest_special(which, x.data_ptr(), y.data_ptr(), n, _lib.stream_ptr()), name)
+    want = fn(x.double())
+    err = (y.double() - want).abs() / want
+    assert bool((err <= bound(x.double(), want) * (1 + 1e-6)).all()), (name, float(err.max()), float((err / bound(x.double(), want)).max()))
+
+
+def test_special_functions_at_their_ends():
+    """Where the flushing forms end: e^x below 2^-126 and the reciprocal of more than 2^126 are zero, infinities and NaN pass."""
+    from qllm2_b200 import _lib
+    inf, nan = float("inf"), float("nan")
+    for which, xs, want in ((0, [-inf, -90.0, 0.0, inf, nan], [0.0, 0.0, 1.0, inf, nan]),
+                            (1, [inf, 3e38, nan], [0.0, 0.0, nan]), (2, [inf, nan], [0.0, nan]),
+                            (3, [-inf, -200.0, 0.0, 200.0, inf, nan], [0.0, 0.0, 0.5, 1.0, 1.0, nan]), (4, [-inf, -105.0, 0.0, nan], [0.0, 0.0, 1.0, nan])):
+        x = torch.tensor(xs, device=DEV)
+        y = torch.empty_like(x)
+        _lib.check(_lib.lib().qpam_selftest_special(which, x.data_ptr(), y.data_ptr(), len(xs), _lib.stream_ptr()), str(which))
+        assert torch.equal(y.nan_to_num(nan=-1.0, posinf=2.0), torch.tensor(want, device=DEV).nan_to_num(nan=-1.0, posinf=2.0)), (which, y)
