@@ -67,9 +67,9 @@ __device__ __forceinline__ float4 ld_dependent(const float4* p) {
   return v;                                                                                       // stores; volatile keeps them behind the wait)
 }
 
-// `first`: an ordinary launch, for a kernel that begins a call and reads its inputs without waiting.
+// `ordinary`: begins when everything before it has completed (a kernel that does not wait).
 template <typename... Params, typename... Args>
-static inline void launch_kernel(bool first, void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+static inline void launch_kernel(bool ordinary, void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
@@ -79,7 +79,7 @@ static inline void launch_kernel(bool first, void (*kern)(Params...), dim3 grid,
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = first ? 0 : 1;
+  cfg.numAttrs = ordinary ? 0 : 1;
   cudaLaunchKernelEx(&cfg, kern, args...);      // (an error is found by the QPAM_LAUNCH_CHECK behind every launch)
 }
 template <typename... Params, typename... Args>

@@ -165,9 +165,9 @@ static int set_smem(KernelT kern, size_t bytes) { return allow_smem(reinterpret_
 // 48 chat prompts of three states 370 -> 357.  The carries start ordinarily: they have nothing to do before their
 // predecessor's sums, and waiting beside its last chunks they took what they saved (three states 444, the prompts 367).  So do the
 // FFMA chunk sums: a few hundred compute-bound CTAs that fill whichever SMs are free first instead of spreading (4 x 6 x 700
-// fp32, d = 32: 145 us against 131).
+// fp32, d = 32: 145 us against 131).  Kernels launched this way do not wait: all before them is complete when they begin.
 template <typename... Args>
-static inline void launch_carry(Args&&... args) { launch_kernel(true, std::forward<Args>(args)...); }
+static inline void launch_ordinary(Args&&... args) { launch_kernel(true, std::forward<Args>(args)...); }
 
 template <int D>
 constexpr size_t outer_smem() { return sizeof(float2) * 2 * CH * (D + 1) + sizeof(float) * CH; }
@@ -183,11 +183,11 @@ static int launch_states(const ScanParams& p, const ScanLayout& L, const qpam_sc
     auto kern = k_chunk_outer<D, T, false>;
     int rc = set_smem(kern, outer_smem<D>());
     if (rc) return rc;
-    launch_carry(kern, dim3(L.grid_chunks, a->H, a->K), NT, outer_smem<D>(), st, p);
+    launch_ordinary(kern, dim3(L.grid_chunks, a->H, a->K), NT, outer_smem<D>(), st, p);
     QPAM_LAUNCH_CHECK("k_chunk_outer<state>");
   }
   const int n4 = D * D / 2;
-  launch_carry(k_state_scan<false>, dim3(a->S, a->H * a->K, (n4 + 255) / 256), 256, 0, st, p, D);
+  launch_ordinary(k_state_scan<false>, dim3(a->S, a->H * a->K, (n4 + 255) / 256), 256, 0, st, p, D);
   QPAM_LAUNCH_CHECK("k_state_scan<fwd>");
   return QPAM_OK;
 }
@@ -310,7 +310,7 @@ static int tc_states(const ScanParams& p0, const ScanLayout& L, const qpam_scan_
     QPAM_LAUNCH_CHECK("k_tc_chunk_outer<state>");
   }
   if (single) return QPAM_OK;
-  launch_carry(k_state_scan<false>, dim3(a->S, a->H * a->K, (64 * 64 / 2 + 255) / 256), 256, 0, st, p, 64);
+  launch_ordinary(k_state_scan<false>, dim3(a->S, a->H * a->K, (64 * 64 / 2 + 255) / 256), 256, 0, st, p, 64);
   QPAM_LAUNCH_CHECK("k_state_scan<fwd>");
   return QPAM_OK;
 }
@@ -463,7 +463,7 @@ static int scan_bwd_tc(const qpam_scan_args* a, const ScanLayout& L, const void*
     QPAM_LAUNCH_CHECK("k_tc_chunk_outer<dstate>");
   }
   if (!alone) {
-    launch_carry(tcs::k_tc_state_scan_rev, dim3(a->S, a->H, 64 * 64 / 2 / 256), 256, 0, st, p, anchors);
+    launch_ordinary(tcs::k_tc_state_scan_rev, dim3(a->S, a->H, 64 * 64 / 2 / 256), 256, 0, st, p, anchors);
     QPAM_LAUNCH_CHECK("k_tc_state_scan_rev");
   }
   if (L.grid_chunks > 0) {
@@ -541,7 +541,7 @@ static int scan_bwd_tcK(const qpam_scan_args* a, const ScanLayout& L, const void
   if (alone) {
     anchors = nullptr;
   } else {
-    launch_carry(tcs::k_tc_state_scan_rev, dim3(a->S, a->H, 8 * a->K), 256, 0, st, p, anchors);
+    launch_ordinary(tcs::k_tc_state_scan_rev, dim3(a->S, a->H, 8 * a->K), 256, 0, st, p, anchors);
     QPAM_LAUNCH_CHECK("k_tc_state_scan_rev");
   }
   if (L.grid_chunks == 0) return QPAM_OK;
@@ -571,12 +571,12 @@ static int scan_bwd_t(const qpam_scan_args* a, const ScanLayout& L, const void* 
     auto kern = k_chunk_outer<D, T, true>;
     rc = set_smem(kern, outer_smem<D>());
     if (rc) return rc;
-    launch_carry(kern, dim3(L.grid_chunks, a->H, a->K), NT, outer_smem<D>(), st, p);
+    launch_ordinary(kern, dim3(L.grid_chunks, a->H, a->K), NT, outer_smem<D>(), st, p);
     QPAM_LAUNCH_CHECK("k_chunk_outer<dstate>");
   }
   const int n4 = D * D / 2;
   if (!alone) {
-    launch_carry(k_state_scan<true>, dim3(a->S, a->H * a->K, (n4 + 255) / 256), 256, 0, st, p, D);
+    launch_ordinary(k_state_scan<true>, dim3(a->S, a->H * a->K, (n4 + 255) / 256), 256, 0, st, p, D);
     QPAM_LAUNCH_CHECK("k_state_scan<rev>");
   }
   if (L.grid_chunks > 0) {

@@ -173,8 +173,6 @@ __global__ void __launch_bounds__(NT) k_chunk_outer(ScanParams p) {
   float2* Ys = Xs + CH * LD;                           // [CH][LD]  k (or q~)
   float* A = reinterpret_cast<float*>(Ys + CH * LD);   // [CH]
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  pdl_wait();
-  pdl_trigger();
   const ChunkLoc L = locate_chunk(p.geom, blockIdx.x);
   if (!L.valid) return;
   const int h = blockIdx.y, k = blockIdx.z;
@@ -233,8 +231,7 @@ __global__ void __launch_bounds__(NT) k_chunk_outer(ScanParams p) {
 // ---------------------------------------------------------------------------------------------
 template <bool REVERSE>
 __global__ void __launch_bounds__(256) k_state_scan(ScanParams p, int D) {
-  pdl_trigger();
-  pdl_wait();
+  pdl_trigger();      // (launched ordinarily: its predecessor has completed)
   const int seq = blockIdx.x;
   const int hk = blockIdx.y;
   const int k = hk / p.H, h = hk - k * p.H;

@@ -548,8 +548,7 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_bwd(const __grid_constant__
 // grid = (S, H, 8 K), 256 threads: every thread owns one float4 (two complex entries) of the state.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_tc_state_scan_rev(ScanParams p, float* __restrict__ anchor_parts) {
-  pdl_trigger();
-  pdl_wait();
+  pdl_trigger();      // (launched ordinarily: its predecessor has completed)
   const int seq = blockIdx.x, h = blockIdx.y, k = blockIdx.z >> 3, z = blockIdx.z & 7;
   const int e4 = z * 256 + threadIdx.x;
   constexpr int n4 = TD * TD / 2;
