@@ -481,15 +481,14 @@ def main():
 # DRAM bytes (read + written) per launch of the dominant kernels at the headline shape, from an ncu capture of
 # THIS build (one kernel, one launch): the figure the `traffic` field of the roofline reports
 NCU_TRAFFIC = {
-    "k_tc_chunk<dq,dv,dk>": {"bytes": 148378624 + 53239552, "source": "ncu --set full of this kernel, one launch (summary kept under profiles/); a constant of this build, not measured in this run"},
-    "k_tc_chunk<fwd>": {"bytes": 99545856 + 5786368, "source": "ncu --set full of this kernel, one launch (summary kept under profiles/); a constant of this build, not measured in this run"},
+    "k_tc_chunk<dq,dv,dk>": {"bytes": 148352000 + 51937792, "source": "ncu of this kernel, one launch (summary kept under profiles/); a constant of this build, not measured in this run"},
+    "k_tc_chunk<fwd>": {"bytes": 99540480 + 6555648, "source": "ncu of this kernel, one launch (summary kept under profiles/); a constant of this build, not measured in this run"},
 }
 
 
 def scan_k3(dev, B, H, T, d, C, rank, iters=10):
-    """Scan forward + backward with K = 3 phase-routed states on the headline shape: the fused K-state output
-    kernel does not keep what a backward needs, so training runs the states as single-state scans combined by
-    the read-out weights (ops.pam_scan)."""
+    """Scan forward + backward with K = 3 phase-routed states and their read-out weights on the headline shape, through the
+    fused K-state kernels."""
     from qllm2_b200 import ops, synthetic
     K = 3
     inp = synthetic.scan_inputs(B, H, T, d, seed=700 + rank, dtype=torch.bfloat16)

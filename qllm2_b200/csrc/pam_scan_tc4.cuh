@@ -14,7 +14,7 @@
 // the weight G, its sums of Z and its carried-state products.  dc and the decay gradient come from the fp32 scores (no
 // per-state output is needed, and the contribution of every (t, s) pair to Re<q,dq> - Re<k,dk> cancels to fp32 rounding).
 // (One state keeps the three-job kernel of pam_scan_tc2.cuh: two CTAs on an SM hide each other's waits there, 102-106 us against
-// 118 us here at 8 x 6 x 2048; three states took 420 us that way, read-out weights included, and take 230-235 us.)
+// 118 us here at 8 x 6 x 2048 (93 now); three states took 420 us that way, read-out weights included, and take 214 us.)
 //
 // Every score is formed twice, once per direction of the sum (a row of the tile is a TMEM lane, so sums along a row stay
 // inside threads): pass A has tokens t as rows (dq, dc), pass B tokens s (dk, dv, Re<k,dk>).  512 threads: a thread owns a

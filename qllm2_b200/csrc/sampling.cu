@@ -26,9 +26,9 @@
 //                 row into a dozen bins, whose atomics serialise), the bin in which the k-th value / the nucleus closes,
 //                 and the exact threshold from the elements of that bin.  Masses are accumulated in fixed point: the
 //                 sums do not depend on the order of the atomics.
-// 256 rows x 50261 bf16 logits with a penalty over 16..513 tokens (a call, device): top-k 50 + top-p 0.9 34.8 -> 20.8 us; top-p 0.9 alone
-// 124 -> 82; neither 54 -> 29.  One row: 19 -> 16.7, 66 -> 51, 29 -> 19.8.  (Before: eight tests and a division for every group of
-// a pass, the small top-k reading the whole row twice, one warp walking the stretch of the draw.)
+// 256 rows x 50261 bf16 logits with a penalty over 16..513 tokens (captured calls back to back): top-k 50 + top-p 0.9 33.7 -> 20.4 us;
+// top-p 0.9 alone 121 -> 78; neither 51.9 -> 28.6.  One row: 17.2 -> 15.2, 58.3 -> 47.8, 22.9 -> 18.5.  (Before: eight tests and a
+// division for every group of a pass, the small top-k reading the whole row twice, one warp walking the stretch of the draw.)
 #include "elementwise.cuh"
 
 namespace qpam {
@@ -270,7 +270,8 @@ __device__ __forceinline__ int bin_of(float x, float mx) {      // (the conversi
 // maximum.
 __device__ __forceinline__ float mass_of(float x, float mx) { return ew::fexp_gradual_(x - mx); }
 // The same where it is only a term of a sum that also holds the maximum's 1: results below 2^-126 are zero, as they vanish in such
-// a sum.  Top-p without top-k, 256 rows: 82 us against 86.
+// a sum.  (Top-p without top-k is 5 % faster for it.  With it everywhere a row without filters takes 27.4 us, not 28.6, and loses
+// its tokens beyond 87.)
 __device__ __forceinline__ float mass_term(float x, float mx) { return ew::fexp_(x - mx); }
 // What few elements of a pass need stays out of line: 32 copies of it in a loop that jumps over them cost more than the pass.
 __device__ __noinline__ void list_bin_value(Scratch* sc, float x, float mx, int i, int cross, uint32_t key_k) {

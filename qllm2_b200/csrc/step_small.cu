@@ -15,7 +15,7 @@
 // and the sequences as the 8 columns: tcgen05 would need its 128-row tiles staged through shared memory for the same
 // bytes, and they would give the D-row projections 12 CTAs.
 // Step of that model, replayed from a graph, K = 3 states (library GEMMs on the packed matrices, ~160 launches, before):
-// n = 1 760 -> 274 us, n = 4 780 -> 329 us, n = 8 -> 448 us, n = 16 820 -> 516 us; at n = 32 the library route is as fast.
+// n = 1 760 -> 267 us, n = 4 780 -> 329 us, n = 8 -> 448 us, n = 16 820 -> 516 us; at n = 32 the library route is as fast.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -947,7 +947,7 @@ __global__ void __launch_bounds__(ONE_THREADS, 1) k_step_one(const __grid_consta
   m.embed();
   m.template norm_rows<false, false>(nullptr, nullptr, layers.l[0].n1);
   // Half a layer at a time (gated unit, sequence mixing): both are a norm, a wide projection and one back to D rows.  One copy of
-  // that code serves both and stays in the instruction cache; written out per layer it missed 620 times a layer, now 370 (a step of one sequence 279 -> 267 us).
+  // that code serves both and stays in the instruction cache; written out per layer it missed 620 times a layer, now 385 (a step of one sequence 279 -> 267 us).
 #pragma unroll 1
   for (int half = 0; half < 2 * p.L; ++half) {
     const int l = half >> 1;

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(1024) k_ce_finalize(CEParams p, const float* r
 // k_ce_merge + k_ce_finalize of an unsharded head in one launch: a CTA folds the vocabulary splits of 32 rows (eight
 // threads per row, neighbouring rows on neighbouring lanes), forms lse and loss, and leaves its four sums; the CTA that
 // arrives last adds the CTAs' sums in their order.  (The two kernels and the five fills around them took 24 us at 8192
-// rows and 23 us at 509; this one 5 and 4.)
+// rows and 23 us at 509; this one 5 and 4, cold 10 and 12.)
 constexpr int CE_ROWS = 32;
 __global__ void __launch_bounds__(256) k_ce_rows(CEParams p, float* lse, float* loss, float* per_token, float* denom, float* loss_sum, float* correct,
                                                  float* tokens, double* block_sums, unsigned int* arrived) {
