@@ -139,18 +139,26 @@ def test_head_logits_bf16_tiles(N, F, V):
     assert err <= 2.0 ** -8, err
 
 
-@pytest.mark.parametrize("N,D,V", [
-    (65, 260, 20001),           # 79 x 3 tiles of dW, more than pairs of SMs: ragged in both directions
-    (12000, 260, 20001),        # the same over two row chunks (fp32 sums)
-    (70, 130, 257),             # fewer tiles than pairs; the second row tile of the last pair has one row
+def _backward_chunks(loss):
+    """Run the backward; returns the number of its row chunks (one dW product each)."""
+    torch.cuda.synchronize()
+    _lib.profile_begin()
+    loss.backward()
+    return _lib.profile_end()["k_tc_gemm<dW>"][0]
+
+
+@pytest.mark.parametrize("N,D,V,chunks", [
+    (65, 260, 20001, 1),        # 79 x 3 tiles of dW, more than pairs of SMs: ragged in both directions
+    (12000, 260, 20001, 2),     # the same over two row chunks (fp32 sums)
+    (70, 132, 385, 1),          # fewer tiles than pairs; the second row tile of the last pair has one row
 ])
-def test_weight_gradient_tile_walk(N, D, V):
+def test_weight_gradient_tile_walk(N, D, V, chunks):
     c = synthetic.ce_inputs(N, D, V, seed=N, dtype=torch.bfloat16)
     w_host = (c.w.float() * 20).bfloat16()
     h = c.h.to(DEV).requires_grad_(True)
     w = w_host.to(DEV).requires_grad_(True)
     loss = fused_ce.fused_linear_cross_entropy(h, w, c.targets.to(DEV))
-    loss.backward()
+    assert _backward_chunks(loss) == chunks
     torch.cuda.synchronize()
     assert _lib.device_status() == 0
     hd, wd, t = h.detach().double(), w.detach().double(), c.targets.to(DEV)
@@ -161,17 +169,17 @@ def test_weight_gradient_tile_walk(N, D, V):
     assert_close(h.grad.double().cpu().numpy(), (p @ wd).cpu().numpy(), 2e-2, "dH")
 
 
-@pytest.mark.parametrize("N,D,V", [
-    (8192, 32, 520),           # the largest batch that is one chunk whatever its width
-    (11600, 384, 20001),       # one: less scratch than two with their fp32 dW
-    (12000, 260, 20001),       # two
+@pytest.mark.parametrize("N,D,V,chunks", [
+    (8192, 32, 520, 1),        # the largest batch that is one chunk whatever its width
+    (11600, 384, 20001, 1),    # one: less scratch than two with their fp32 dW
+    (12000, 260, 20001, 2),
 ])
-def test_row_chunks_of_the_backward(N, D, V):
+def test_row_chunks_of_the_backward(N, D, V, chunks):
     c = synthetic.ce_inputs(N, D, V, seed=12, dtype=torch.bfloat16)
     w_host = (c.w.float() * 20).bfloat16()
     h, w, t = c.h.to(DEV).requires_grad_(True), w_host.to(DEV).requires_grad_(True), c.targets.to(DEV)
     loss = fused_ce.fused_linear_cross_entropy(h, w, t)
-    loss.backward()
+    assert _backward_chunks(loss) == chunks
     torch.cuda.synchronize()
     assert _lib.device_status() == 0
     hd, wd = h.detach().double(), w.detach().double()
@@ -196,9 +204,9 @@ def test_weight_gradient_of_one_chunk_and_of_two():
     p[torch.arange(N, device=DEV), t] -= 1.0
     want = (p.T @ h.double()) / N
     far = []
-    for width in (F, wide):
+    for width, chunks in ((F, 2), (wide, 1)):
         hw, ww = (torch.nn.functional.pad(x, (0, width - F)).requires_grad_(True) for x in (h, w))
-        fused_ce.fused_linear_cross_entropy(hw, ww, t).backward()
+        assert _backward_chunks(fused_ce.fused_linear_cross_entropy(hw, ww, t)) == chunks
         assert not ww.grad[:, F:].any()
         far.append(float((ww.grad[:, :F].double() - want).norm() / want.norm()))
     assert far[0] <= 2e-2 and far[1] <= 1.1 * far[0], far

@@ -398,3 +398,13 @@ def test_special_functions_at_their_ends():
         y = torch.empty_like(x)
         _lib.check(_lib.lib().qpam_selftest_special(which, x.data_ptr(), y.data_ptr(), len(xs), _lib.stream_ptr()), str(which))
         assert torch.equal(y.nan_to_num(nan=-1.0, posinf=2.0), torch.tensor(want, device=DEV).nan_to_num(nan=-1.0, posinf=2.0)), (which, y)
+
+
+def test_the_two_exponentials_agree_above_underflow():
+    """The sampler forms sums with the one and single masses with the other: the same bits from 2^-126 on."""
+    from qllm2_b200 import _lib
+    x = torch.linspace(-87.3, 0.0, 1 << 21, device=DEV)
+    out = [torch.empty_like(x) for _ in range(2)]
+    for which, y in zip((0, 4), out):
+        _lib.check(_lib.lib().qpam_selftest_special(which, x.data_ptr(), y.data_ptr(), x.numel(), _lib.stream_ptr()), str(which))
+    assert torch.equal(*out)
