@@ -7,6 +7,7 @@
 #include "pam_scan_tc2.cuh"
 #include "pam_scan_tc3.cuh"
 #include "pam_scan_tc4.cuh"
+#include "pam_scan_walk.cuh"
 #include "tma_host.cuh"
 
 namespace qpam {
@@ -105,8 +106,8 @@ static ScanLayout scan_layout(const qpam_scan_args* a, int ch) {
   off += align256(sizeof(float2) * (size_t)a->K * a->H * L.nslots * dd);
   L.off_decay = off;
   off += align256(sizeof(float) * (size_t)a->K * a->H * L.nslots);
-  L.off_jobs = off;      // ticket counter, then the jobs of the carrying chunk sums (packed calls)
-  if (a->cu_seqlens != nullptr) off += align256(256 + sizeof(ChunkJob) * (size_t)L.grid_chunks);
+  L.off_jobs = off;      // packed calls: the counters and the list of a forward that walks, an entry a chunk at most
+  if (a->cu_seqlens != nullptr) off += align256(256 + sizeof(WalkJob) * (size_t)L.grid_chunks);
   L.total_fwd = off;
   L.off_dstates = off;
   off += align256(sizeof(float2) * (size_t)a->K * a->H * L.nslots * dd);
@@ -223,93 +224,35 @@ static ScanParams one_state_view(const ScanParams& pK, const qpam_scan_args* a, 
   return p;
 }
 
-// Jobs of the carrying chunk sums: CTA s places the chunks of sequence s.  Chunk c of nc sits at (c + 1/2) / nc of the way, so
-// that all sequences end together and the chunks of the longest are as far apart as they can be.  The rank of a chunk is the
-// number of chunks before that point, plus the earlier sequences that have one at the same point.
-// A link of a chain takes ~2.2 us and the chip does 67 jobs a us, so the sums carry (ticket[1]) where the longest sequence has at
-// most 1/CARRY_WIDTH of all jobs; a pass of its own for the carry costs ~9 ns a job.
-// Clears the flags and the ticket counter.
-constexpr int CARRY_WIDTH = 160;
-__global__ void __launch_bounds__(256) k_chunk_jobs(ScanParams p, ChunkJob* jobs) {
-  pdl_wait();
-  pdl_trigger();
-  const int s = blockIdx.x, S = p.geom.S;
-  const int32_t *cu = p.geom.cu_seqlens, *pre = p.geom.chunk_prefix;
-  if (s == 0) {
-    int longest = 1;
-    for (int o = threadIdx.x; o < S; o += 256) longest = max(longest, pre[o + 1] - pre[o]);
-    const bool narrow = __syncthreads_or((int64_t)pre[S] * p.H < (int64_t)longest * CARRY_WIDTH);
-    if (threadIdx.x == 0) {
-      p.ticket[0] = 0u;
-      p.ticket[1] = narrow ? 0u : 1u;
-    }
-  }
-  const int64_t flags = (int64_t)p.K * p.H * p.nslots;
-  for (int64_t i = (int64_t)s * 256 + threadIdx.x; i < flags; i += (int64_t)S * 256) p.ready[i] = 0u;
-  const int nc = pre[s + 1] - pre[s], a = cu[s], len = cu[s + 1] - a;
-  for (int c = threadIdx.x; c < nc; c += 256) {
-    int rank = 0;
-    for (int o = 0; o < S; ++o) {
-      const int n = pre[o + 1] - pre[o];            // chunks x of o with (2x + 1) / n < (2c + 1) / nc
-      int up;
-      bool tie;
-      if (pre[S] <= 32768) {
-        const uint32_t at = (uint32_t)(2 * c + 1) * (uint32_t)n;
-        up = (int)((at + (uint32_t)nc - 1u) / (uint32_t)nc);
-        tie = (uint32_t)up * (uint32_t)nc == at;
-      } else {
-        const int64_t at = (int64_t)(2 * c + 1) * n;
-        up = (int)((at + nc - 1) / nc);
-        tie = (int64_t)up * nc == at;
-      }
-      rank += up >> 1;
-      if (o < s && (up & 1) && tie) ++rank;
-    }
-    jobs[rank] = ChunkJob{s, c, nc, a + c * p.geom.ch, min(p.geom.ch, len - c * p.geom.ch), pre[s] + s, {0, 0}};
-  }
-}
-
-// chunk-local state sums on tensor cores, then the carry over the chunk axis
-static int tc_states(const ScanParams& p0, const ScanLayout& L, const qpam_scan_args* a, cudaStream_t st) {
-  ScanParams p = p0;
-  // Where the carry is likely to pay: the lengths are on the device, so by their average (eight chunks and more: short
-  // sequences have few links to save) and by how many sequences and heads run side by side (of 384, with lengths anywhere
-  // up to the longest, about 190 on average).  Drawing jobs costs 10 % of the chunk sums if the device then decides against it.
-  // every sequence one chunk, from zero: its sums are its final state, and nothing is left for the carry
-  const bool single = a->cu_seqlens == nullptr && L.nc_uniform == 1 && p.s0 == nullptr;
-  p.single = single && !p.fwd_only;
-  const bool carry = a->cu_seqlens != nullptr && a->K == 1 && p.fwd_only && p.s0 == nullptr && a->T >= (int64_t)8 * tcs::TC * a->S &&
-                     (int64_t)a->S * a->H >= 384;
-  if (carry) {
-    char* ws = reinterpret_cast<char*>(a->workspace);
-    ChunkJob* jobs = reinterpret_cast<ChunkJob*>(ws + L.off_jobs + 256);
-    p.jobs = jobs;
-    p.ticket = reinterpret_cast<unsigned int*>(ws + L.off_jobs);
-    p.ready = reinterpret_cast<unsigned int*>(p.chunk_decay);
-    launch_after(k_chunk_jobs, a->S, 256, 0, st, p, jobs);
-    QPAM_LAUNCH_CHECK("k_chunk_jobs");
-  }
-  if (L.grid_chunks > 0 && a->K > 1) {      // all states from one load of the key / value tiles
-    int rc = set_smem(tcs::k_tc_chunk_outerK<false>, tcs::OUTERK_SMEM);
-    if (rc) return rc;
-    CUtensorMap mk, mv;
-    const int64_t rows = (int64_t)a->B * a->H * a->T;
-    if ((rc = make_map(&mk, a->k, 128, rows, 128, 64, 128))) return rc;
-    if ((rc = make_map(&mv, a->v, 128, rows, 128, 64, 128))) return rc;
+// chunk-local state sums on tensor cores; done: every sequence is one chunk from zero, its sums are its final state
+static int tc_sums(ScanParams& p, const ScanLayout& L, const qpam_scan_args* a, cudaStream_t st, bool& done) {
+  done = a->cu_seqlens == nullptr && L.nc_uniform == 1 && p.s0 == nullptr;
+  p.single = done;
+  if (L.grid_chunks == 0) return QPAM_OK;
+  CUtensorMap mk, mv;
+  const int64_t rows = (int64_t)a->B * a->H * a->T;
+  int rc;
+  if ((rc = make_map(&mk, a->k, 128, rows, 128, 64, 128))) return rc;
+  if ((rc = make_map(&mv, a->v, 128, rows, 128, 64, 128))) return rc;
+  if (a->K > 1) {      // all states from one load of the key / value tiles
+    if ((rc = set_smem(tcs::k_tc_chunk_outerK<false>, tcs::OUTERK_SMEM))) return rc;
     launch_after(tcs::k_tc_chunk_outerK<false>, dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st, mk, mv, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outerK");
-  } else if (L.grid_chunks > 0) {
-    const auto kern = carry ? tcs::k_tc_chunk_outer<false, tcs::OUTER_CARRY> : p.fwd_only || single ? tcs::k_tc_chunk_outer<false, tcs::OUTER_FWD_ONLY> : tcs::k_tc_chunk_outer<false>;
-    int rc = set_smem(kern, tcs::OUTER_SMEM);
-    if (rc) return rc;
-    CUtensorMap mk, mv;
-    const int64_t rows = (int64_t)a->B * a->H * a->T;
-    if ((rc = make_map(&mk, a->k, 128, rows, 128, 64, 128))) return rc;
-    if ((rc = make_map(&mv, a->v, 128, rows, 128, 64, 128))) return rc;
+  } else {
+    const auto kern = done ? tcs::k_tc_chunk_outer<false, true> : tcs::k_tc_chunk_outer<false>;
+    if ((rc = set_smem(kern, tcs::OUTER_SMEM))) return rc;
     launch_after(kern, dim3(L.grid_chunks, a->H, a->K), 256, tcs::OUTER_SMEM, st, mk, mv, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outer<state>");
   }
-  if (single) return QPAM_OK;
+  return QPAM_OK;
+}
+
+// the same, then the carry over the chunk axis
+static int tc_states(const ScanParams& p0, const ScanLayout& L, const qpam_scan_args* a, cudaStream_t st) {
+  ScanParams p = p0;
+  bool done;
+  const int rc = tc_sums(p, L, a, st, done);
+  if (rc || done) return rc;
   launch_ordinary(k_state_scan<false>, dim3(a->S, a->H * a->K, (64 * 64 / 2 + 255) / 256), 256, 0, st, p, 64);
   QPAM_LAUNCH_CHECK("k_state_scan<fwd>");
   return QPAM_OK;
@@ -322,15 +265,6 @@ struct PoolDest {
   int64_t n_slots;
   int32_t dtype, L, layer;
 };
-// A workspace without room for the backward's part cannot be handed to one (qpam_scan_bwd refuses it): forward only.
-static void set_forward_only(ScanParams& p, const qpam_scan_args* a, const ScanLayout& L, const PoolDest* dest) {
-  p.fwd_only = dest != nullptr || a->workspace_bytes < L.total_bwd;
-  if (dest) {
-    p.pool = dest->pool; p.slot_ids = dest->slot_ids; p.n_slots = dest->n_slots;
-    p.pool_bf16 = dest->dtype == QPAM_BF16; p.pool_L = dest->L; p.pool_layer = dest->layer;
-  }
-}
-
 // Output tensor as the target of the chunk kernels' TMA stores (boxes of 64 elements x 32 rows): [B*H*T rows][128], or
 // for the token-major layout [B*T rows][H*128].
 static int make_out_map(CUtensorMap* m, const qpam_scan_args* a, bool token_major) {
@@ -338,55 +272,117 @@ static int make_out_map(CUtensorMap* m, const qpam_scan_args* a, bool token_majo
   return make_map(m, a->y, 128, (int64_t)a->B * a->H * a->T, 128, 64, 32);
 }
 
-// bf16 / d = 64 / one state: tensor-core kernels on 128-token chunks
-static int scan_fwd_tc(const qpam_scan_args* a, const ScanLayout& L, cudaStream_t st, bool token_major = false, const PoolDest* dest = nullptr) {
-  ScanParams p = make_params(a, L);
-  p.y_token_major = token_major ? 1 : 0;
-  set_forward_only(p, a, L, dest);
-  if (a->cu_seqlens != nullptr) {
-    launch_after(k_chunk_prefix_checked, 1, 256, 0, st, a->cu_seqlens, const_cast<int32_t*>(p.geom.chunk_prefix), a->S, L.ch, a->T);
-    QPAM_LAUNCH_CHECK("k_chunk_prefix");
-  }
+// The output kernel of all chunks, by its number of states
+static int tc_outputs(const ScanParams& p, const ScanLayout& L, const qpam_scan_args* a, bool token_major, cudaStream_t st) {
+  if (L.grid_chunks == 0 || a->y == nullptr) return QPAM_OK;
+  tcs::ChunkMaps maps;
+  const int64_t rows = (int64_t)a->B * a->H * a->T;
   int rc;
-  rc = tc_states(p, L, a, st);
-  if (rc) return rc;
-  if (L.grid_chunks > 0 && a->y != nullptr) {
-    tcs::ChunkMaps maps;
-    const int64_t rows = (int64_t)a->B * a->H * a->T;
-    if ((rc = make_map(&maps.a1, a->q, 128, rows, 128, 64, 128))) return rc;
-    if ((rc = make_map(&maps.b1, a->k, 128, rows, 128, 64, 128))) return rc;
-    if ((rc = make_map(&maps.x2, a->v, 128, rows, 128, 64, 128))) return rc;
-    if ((rc = make_out_map(&maps.out, a, token_major))) return rc;
-    if ((rc = set_smem(tcs::k_tc_chunk_fwd, tcs::CHUNK2_SMEM))) return rc;
-    launch_after(tcs::k_tc_chunk_fwd, dim3(L.grid_chunks, a->H), 256, tcs::CHUNK2_SMEM, st, maps, p);
+  if ((rc = make_map(&maps.a1, a->q, 128, rows, 128, 64, 128))) return rc;
+  if ((rc = make_map(&maps.b1, a->k, 128, rows, 128, 64, 128))) return rc;
+  if ((rc = make_map(&maps.x2, a->v, 128, rows, 128, 64, 128))) return rc;
+  if ((rc = make_out_map(&maps.out, a, token_major))) return rc;
+  const auto kern = a->K == 1 ? tcs::k_tc_chunk_fwd : a->K == 2 ? tcs::k_tc_chunk_fwdK<2> : a->K == 3 ? tcs::k_tc_chunk_fwdK<3> : tcs::k_tc_chunk_fwdK<4>;
+  const size_t smem = a->K == 1 ? tcs::CHUNK2_SMEM : tcs::CHUNKK_SMEM;
+  if ((rc = set_smem(kern, smem))) return rc;
+  launch_after(kern, dim3(L.grid_chunks, a->H), 256, smem, st, maps, p);
+  if (a->K > 1) {
+    QPAM_LAUNCH_CHECK("k_tc_chunk_fwdK");
+  } else {
     QPAM_LAUNCH_CHECK("k_tc_chunk<fwd>");
   }
   return QPAM_OK;
 }
 
-// bf16 / d = 64 / K = 2..4 states: state sums and carry per state, then ONE fused output kernel
-static int scan_fwd_tcK(const qpam_scan_args* a, const ScanLayout& L, cudaStream_t st, bool token_major = false, const PoolDest* dest = nullptr) {
+// Whether a forward-only call walks (pam_scan_walk.cuh): it wants more sequences and heads than the chip holds CTAs, and more still for
+// one state, whose three passes cost less; lengths of packed sequences are on the device, so by their number.  Measured (us, three passes
+// -> walking; packed lengths anywhere between the two given): K = 1, 32 x 512..16384, 16 heads 1614 -> 1442, 19 x 108..649, 16 heads
+// 69 -> 70, 24 x 326..5999, 12 heads 400 -> 469; K = 3, 48 x 32..1024, 12 heads 311 -> 245, 22 x 448..2034, 16 heads 517 -> 418,
+// 24 x 17..1482, 12 heads 262 -> 262, 5 x 170..2570, 6 heads 64 -> 94.  Of equal lengths the last round of CTAs has to be four fifths full.
+static bool walk_pays(const qpam_scan_args* a, int ctas) {
+  const int64_t units = (int64_t)a->S * a->H;
+  if (a->y == nullptr || a->T == 0) return false;
+  if (a->cu_seqlens != nullptr) return units >= (a->K == 1 ? 384 : 320);
+  return units * 5 >= (units + ctas - 1) / ctas * ctas * 4;
+}
+
+template <int K>
+static int scan_walk(ScanParams& p, const qpam_scan_args* a, const ScanLayout& L, cudaStream_t st, bool token_major, int ctas) {
+  tcs::ChunkMaps maps{};
+  const int64_t rows = (int64_t)a->B * a->H * a->T;
+  int rc;
+  if ((rc = make_map(&maps.a1, a->q, 128, rows, 128, 64, 128))) return rc;
+  if ((rc = make_map(&maps.b1, a->k, 128, rows, 128, 64, 128))) return rc;
+  if ((rc = make_map(&maps.x2, a->v, 128, rows, 128, 64, 128))) return rc;
+  if ((rc = make_out_map(&maps.out, a, token_major))) return rc;
+  if (a->cu_seqlens != nullptr) {
+    char* ws = reinterpret_cast<char*>(a->workspace);
+    WalkJob* jobs = reinterpret_cast<WalkJob*>(ws + L.off_jobs + 256);
+    p.jobs = jobs;
+    p.ticket = reinterpret_cast<unsigned int*>(ws + L.off_jobs);
+    launch_after(tcs::k_walk_plan, 1, 1024, 0, st, p, const_cast<int32_t*>(p.geom.chunk_prefix), jobs, ctas, QPAM_DEV_BAD_CU_SEQLENS);
+    QPAM_LAUNCH_CHECK("k_walk_plan");
+    // (sums and carry of split sequences: they start with empty hands when every sequence is walked)
+    const auto kern = tcs::k_tc_walk<K, false>;
+    if ((rc = set_smem(kern, tcs::walk_smem(K, false)))) return rc;
+    launch_after(kern, 3 * ctas / 2, 256, tcs::walk_smem(K, false), st, maps, p);
+    QPAM_LAUNCH_CHECK("k_tc_walk<sums>");
+    launch_after(tcs::k_walk_carry, 4 * ctas, 256, 0, st, p);
+    QPAM_LAUNCH_CHECK("k_walk_carry");
+  }
+  const auto kern = tcs::k_tc_walk<K, true>;
+  if ((rc = set_smem(kern, tcs::walk_smem(K, true)))) return rc;
+  launch_after(kern, ctas, 256, tcs::walk_smem(K, true), st, maps, p);
+  QPAM_LAUNCH_CHECK("k_tc_walk");
+  return QPAM_OK;
+}
+
+// A forward of which no backward will read the states (a workspace without room for the backward's part cannot be handed to one:
+// qpam_scan_bwd refuses it)
+static bool forward_only(const qpam_scan_args* a, const ScanLayout& L, const PoolDest* dest) { return dest != nullptr || a->workspace_bytes < L.total_bwd; }
+
+static int scan_forward_only(const qpam_scan_args* a, const ScanLayout& L, cudaStream_t st, bool token_major, const PoolDest* dest) {
   ScanParams p = make_params(a, L);
   p.y_token_major = token_major ? 1 : 0;
-  set_forward_only(p, a, L, dest);
+  if (dest) {
+    p.pool = dest->pool; p.slot_ids = dest->slot_ids; p.n_slots = dest->n_slots;
+    p.pool_bf16 = dest->dtype == QPAM_BF16; p.pool_L = dest->L; p.pool_layer = dest->layer;
+  }
+  const int ctas = 2 * sm_count();
+  if (walk_pays(a, ctas)) {
+    switch (a->K) {
+      case 1: return scan_walk<1>(p, a, L, st, token_major, ctas);
+      case 2: return scan_walk<2>(p, a, L, st, token_major, ctas);
+      case 3: return scan_walk<3>(p, a, L, st, token_major, ctas);
+      default: return scan_walk<4>(p, a, L, st, token_major, ctas);
+    }
+  }
   if (a->cu_seqlens != nullptr) {
     launch_after(k_chunk_prefix_checked, 1, 256, 0, st, a->cu_seqlens, const_cast<int32_t*>(p.geom.chunk_prefix), a->S, L.ch, a->T);
     QPAM_LAUNCH_CHECK("k_chunk_prefix");
   }
-  int rc = tc_states(p, L, a, st);
+  bool done;
+  int rc = tc_sums(p, L, a, st, done);
   if (rc) return rc;
-  if (L.grid_chunks > 0 && a->y != nullptr) {
-    tcs::ChunkMaps maps;
-    const int64_t rows = (int64_t)a->B * a->H * a->T;
-    if ((rc = make_map(&maps.a1, a->q, 128, rows, 128, 64, 128))) return rc;
-    if ((rc = make_map(&maps.b1, a->k, 128, rows, 128, 64, 128))) return rc;
-    if ((rc = make_map(&maps.x2, a->v, 128, rows, 128, 64, 128))) return rc;
-    if ((rc = make_out_map(&maps.out, a, token_major))) return rc;
-    if ((rc = set_smem(tcs::k_tc_chunk_fwdK, tcs::CHUNKK_SMEM))) return rc;
-    launch_after(tcs::k_tc_chunk_fwdK, dim3(L.grid_chunks, a->H), 256, tcs::CHUNKK_SMEM, st, maps, p);
-    QPAM_LAUNCH_CHECK("k_tc_chunk_fwdK");
+  if (!done) {
+    const int64_t items = (int64_t)a->S * a->H * a->K * (64 * 64 / 2 / 256);
+    launch_ordinary(tcs::k_walk_carry, (unsigned)(items < 4 * ctas ? items : 4 * ctas), 256, 0, st, p);
+    QPAM_LAUNCH_CHECK("k_walk_carry");
   }
-  return QPAM_OK;
+  return tc_outputs(p, L, a, token_major, st);
+}
+
+// bf16 / d = 64: state sums of all states and their carry, then ONE output kernel, on 128-token chunks
+static int scan_fwd_tc(const qpam_scan_args* a, const ScanLayout& L, cudaStream_t st, bool token_major = false, const PoolDest* dest = nullptr) {
+  if (forward_only(a, L, dest)) return scan_forward_only(a, L, st, token_major, dest);
+  ScanParams p = make_params(a, L);
+  p.y_token_major = token_major ? 1 : 0;
+  if (a->cu_seqlens != nullptr) {
+    launch_after(k_chunk_prefix_checked, 1, 256, 0, st, a->cu_seqlens, const_cast<int32_t*>(p.geom.chunk_prefix), a->S, L.ch, a->T);
+    QPAM_LAUNCH_CHECK("k_chunk_prefix");
+  }
+  const int rc = tc_states(p, L, a, st);
+  return rc ? rc : tc_outputs(p, L, a, token_major, st);
 }
 
 // bf16 / d = 64 / K = 2..4 states, training form: the state sums of all states from ONE load of the key / value tiles
@@ -646,7 +642,7 @@ static int scan_fwd_any(const qpam_scan_args* a, void* stream, bool token_major)
   }
   QPAM_REQUIRE(a->y != nullptr || a->s_final != nullptr, "scan fwd: both y and s_final are NULL");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (L.ch == tcs::TC) return tc_fwdK_eligible(a) ? scan_fwd_tcK(a, L, st, token_major) : scan_fwd_tc(a, L, st, token_major);
+  if (L.ch == tcs::TC) return scan_fwd_tc(a, L, st, token_major);
   if (token_major) {
     set_error("scan fwd: the token-major output exists on the tensor-core path only (bf16, d = 64)");
     return QPAM_EUNSUPPORTED;
@@ -676,7 +672,7 @@ extern "C" int qpam_scan_prefill(const qpam_scan_args* a, void* pool, int32_t st
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const PoolDest dest{pool, slot_ids, n_slots, state_dtype, L_, layer};
-  return tc_fwdK_eligible(a) ? scan_fwd_tcK(a, L, st, true, &dest) : scan_fwd_tc(a, L, st, true, &dest);
+  return scan_fwd_tc(a, L, st, true, &dest);
 }
 
 static int scan_bwd_any(const qpam_scan_args* a, const void* dy, void* dq, void* dk, void* dv, float* dgamma, float* dcoef, const float* ds_final,

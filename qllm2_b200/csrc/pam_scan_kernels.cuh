@@ -89,10 +89,10 @@ __device__ __forceinline__ void warp_chunk_cumsum(float* A, const float* __restr
   A[t + 1] = excl + x0 + x1;
 }
 
-// One chunk of a packed batch as a job of the carrying chunk sums (pam_scan_tc.cuh)
-struct ChunkJob {
-  int32_t seq, c, nc, t0, len, slot0;
-  int32_t pad[2];
+// An entry of the list of a forward-only call (pam_scan_walk.cuh): chunks [c0, c1) of a sequence of nc, its tokens [a, e) of row b, its
+// first state slot, and the pool slot of its final state (-1: none)
+struct __align__(16) WalkJob {
+  int32_t seq, c0, c1, nc, a, e, slot0, pool_slot;
 };
 
 struct ScanParams {
@@ -116,20 +116,16 @@ struct ScanParams {
   float q_scale, eps;
   int32_t y_token_major;   // tensor-core forward kernels only: y laid out [B,T,H,d,2] instead of [B,H,T,d,2]
   int32_t dy_tokens;       // K-state tensor-core backward only: the same for dy
-  // Tensor-core forward of which no backward will read the states: what only a backward needs is not written (see
-  // k_state_scan), and the final states may go to slots of a state pool [n_slots,L,K,H,D,D,2] instead of s_final.
-  int32_t fwd_only;
-  int32_t single;          // a backward may follow, but every sequence is one chunk from zero: the chunk sums write s_final as well
+  int32_t single;          // every sequence is one chunk from zero: the chunk sums write s_final as well
+  // Tensor-core forward of which no backward will read the states: the final states may go to slots of a state pool
+  // [n_slots,L,K,H,D,D,2] instead of s_final.
   int32_t pool_bf16, pool_L, pool_layer;
   void* pool;
   const int32_t* slot_ids;
   int64_t n_slots;
-  // Packed forward-only calls from zero states: jobs[0 .. chunk_prefix[S]) in an order in which a sequence's chunks follow one
-  // another; the tickets drawn so far, [1]: whether the chunk sums carry; a flag for every state slot, set once the state is
-  // there.
-  const ChunkJob* jobs;
+  // The same calls, packed, where they walk: list and counters.
+  const WalkJob* jobs;
   unsigned int* ticket;
-  unsigned int* ready;     // [K,H,nslots] (in the place of chunk_decay)
 };
 
 __device__ __forceinline__ size_t token_base(const ScanParams& p, int b, int h, int t, int D) {
@@ -142,10 +138,14 @@ __device__ __forceinline__ size_t state_base(const ScanParams& p, int k, int h, 
   return (((size_t)k * p.H + h) * p.nslots + slot) * (size_t)(D * D);
 }
 
-// Slot-pool element of (sequence, state, head): index of its first scalar, or -1 when the sequence has no valid slot.
-__device__ __forceinline__ int64_t pool_base(const ScanParams& p, int seq, int k, int h, int D) {
+// Slot of a sequence's final state in the pool, or -1 when it has no valid one.
+__device__ __forceinline__ int pool_slot_of(const ScanParams& p, int seq) {
+  if (p.pool == nullptr) return -1;
   const int slot = p.slot_ids[seq];
-  if (slot < 0 || slot >= p.n_slots) return -1;
+  return slot < 0 || slot >= p.n_slots ? -1 : slot;
+}
+// First scalar of (slot, state, head) in the pool.
+__device__ __forceinline__ int64_t pool_block(const ScanParams& p, int slot, int k, int h, int D) {
   return ((((int64_t)slot * p.pool_L + p.pool_layer) * p.K + k) * p.H + h) * (int64_t)(D * D) * 2;
 }
 __device__ __forceinline__ void store_final4(const ScanParams& p, int64_t at, float4 v) {   // four scalars from `at` on
@@ -223,11 +223,6 @@ __global__ void __launch_bounds__(NT) k_chunk_outer(ScanParams p) {
 // reads U_c, applies S <- g_c S + U_c and writes S back to the same slot.  Loads of the next
 // chunks do not depend on the recurrence, so they are issued ahead of the FMA chain.
 // grid = (S, H*K, ceil(D*D/2/256)).  REVERSE runs the adjoint recurrence for the backward pass.
-//
-// fwd_only (no backward will follow): the output kernel of a chunk reads the state BEFORE it, and none where that is zero,
-// so slot 0 is not written, slot 1 of a sequence without s0 already holds its state (the first chunk's sums) and the last
-// slot is not written either; a one-chunk sequence without s0 has been finished by the chunk-sum kernel.  48 chat prompts of
-// 32..1024 tokens, H = 12, K = 3: 98 -> 73 us.
 // ---------------------------------------------------------------------------------------------
 template <bool REVERSE>
 __global__ void __launch_bounds__(256) k_state_scan(ScanParams p, int D) {
@@ -245,9 +240,6 @@ __global__ void __launch_bounds__(256) k_state_scan(ScanParams p, int D) {
     nc = p.geom.chunk_prefix[seq + 1] - p.geom.chunk_prefix[seq];
     slot0 = (int64_t)p.geom.chunk_prefix[seq] + seq;
   }
-  const bool from_zero = !REVERSE && p.s0 == nullptr;
-  if (!REVERSE && p.fwd_only && nc == 1 && from_zero) return;
-  if (!REVERSE && p.jobs != nullptr && p.ticket[1] != 0u && nc > 1) return;      // the chunk sums have carried already
   const int e4 = blockIdx.z * 256 + threadIdx.x;  // float4 index within the D*D*2 floats
   if (e4 >= n4) return;
   float4* st = reinterpret_cast<float4*>((REVERSE ? p.dstates : p.states) + state_base(p, k, h, slot0, D)) + e4;
@@ -258,17 +250,8 @@ __global__ void __launch_bounds__(256) k_state_scan(ScanParams p, int D) {
   if (init != nullptr) cur = reinterpret_cast<const float4*>(init)[ext];
   constexpr int UN = 4;
   if (!REVERSE) {
-    int first = 0;
-    if (!p.fwd_only) {
-      st[0] = cur;
-    } else if (from_zero && nc > 0) {
-      cur = st[n4];
-      first = 1;
-    } else {
-      st[0] = cur;                                // (a given initial state is read through slot 0)
-    }
-    const int last_slot = p.fwd_only ? nc - 1 : nc;
-    for (int c = first; c < nc; c += UN) {
+    st[0] = cur;
+    for (int c = 0; c < nc; c += UN) {
       float4 u[UN];
       float g[UN];
 #pragma unroll
@@ -284,14 +267,10 @@ __global__ void __launch_bounds__(256) k_state_scan(ScanParams p, int D) {
           cur.y = fmaf(g[i], cur.y, u[i].y);
           cur.z = fmaf(g[i], cur.z, u[i].z);
           cur.w = fmaf(g[i], cur.w, u[i].w);
-          if (c + i + 1 <= last_slot) st[(size_t)(c + i + 1) * n4] = cur;
+          st[(size_t)(c + i + 1) * n4] = cur;
         }
     }
     if (p.s_final != nullptr) reinterpret_cast<float4*>(p.s_final)[ext] = cur;
-    if (p.pool != nullptr) {
-      const int64_t at = pool_base(p, seq, k, h, D);
-      if (at >= 0) store_final4(p, at + (int64_t)e4 * 4, cur);
-    }
   } else {
     st[(size_t)nc * n4] = cur;
     for (int c = nc - 1; c >= 0; c -= UN) {

@@ -69,30 +69,33 @@ __device__ __forceinline__ void warp_cumsum128(float* A, const float* __restrict
   warp_cumsum128_finish(A, g, len, eps, lane);
 }
 
-// Where a chunk's sums go when they are a sequence's final state already (fwd_only, one chunk, no initial state): s_final
-// and / or the sequence's pool slot.  A lane holds one column (n' = q4 * 32 + lane) of every row.
+// Where a sequence's final state goes: s_final and / or the sequence's pool slot.  A lane holds one column (n' = q4 * 32 + lane) of every row.
 struct FinalDest {
   float* f;                 // s_final block, or null
   int64_t pool;             // first scalar of the pool block, or -1
-  __device__ __forceinline__ void init(const ScanParams& p, int seq, int k, int h) {
+  __device__ __forceinline__ void init(const ScanParams& p, int seq, int pool_slot, int k, int h) {
     f = p.s_final ? p.s_final + (((size_t)k * p.geom.S + seq) * p.H + h) * (size_t)(TD * TD) * 2 : nullptr;
-    pool = p.pool ? pool_base(p, seq, k, h, TD) : -1;
+    pool = pool_slot >= 0 ? pool_block(p, pool_slot, k, h, TD) : -1;
   }
-  // rows i and i + 1 (u0, u1) of the lane's column; off: the scalar of row i
-  __device__ __forceinline__ void store2(const ScanParams& p, int off, float u0, float u1, bool even, bool ok) const {
+  // rows i .. i + N - 1 of the lane's column; off: the scalar of row i
+  template <int N>
+  __device__ __forceinline__ void store(const ScanParams& p, int off, const float (&u)[N], bool even, bool ok) const {
     if (f && ok) {
-      f[off] = u0;
-      f[off + 2 * TD] = u1;
+#pragma unroll
+      for (int i = 0; i < N; ++i) f[off + i * 2 * TD] = u[i];
     }
-    if (pool >= 0) {
-      if (p.pool_bf16) {         // the even lane of a pair takes both columns of row i, the odd lane those of row i + 1
-        const float x = __shfl_xor_sync(0xffffffffu, even ? u1 : u0, 1);
-        const int at = even ? off : off - 1 + 2 * TD;
-        if (ok) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.pool) + pool + at) = even ? pack_bf162(u0, x) : pack_bf162(x, u1);
-      } else if (ok) {
-        reinterpret_cast<float*>(p.pool)[pool + off] = u0;
-        reinterpret_cast<float*>(p.pool)[pool + off + 2 * TD] = u1;
+    if (pool < 0) return;
+    if (p.pool_bf16) {           // the even lane of a pair takes both columns of row i, the odd lane those of row i + 1
+      __nv_bfloat16* at = reinterpret_cast<__nv_bfloat16*>(p.pool) + pool + (even ? off : off - 1 + 2 * TD);
+#pragma unroll
+      for (int i = 0; i < N; i += 2) {
+        const float x = __shfl_xor_sync(0xffffffffu, even ? u[i + 1] : u[i], 1);
+        if (ok) *reinterpret_cast<uint32_t*>(at + i * 2 * TD) = even ? pack_bf162(u[i], x) : pack_bf162(x, u[i + 1]);
       }
+    } else if (ok) {
+      float* at = reinterpret_cast<float*>(p.pool) + pool + off;
+#pragma unroll
+      for (int i = 0; i < N; ++i) at[i * 2 * TD] = u[i];
     }
   }
 };
@@ -113,90 +116,8 @@ constexpr size_t OUTER_SMEM = 1024 + 32768 + 32768 + 1536;
 // The two token tiles (k and v, or q and dy; maps of [B*H*T rows][128 bf16], boxes of 64 x 128, 128-byte swizzle)
 // arrive by TMA; the value tile lands in the region its planes are then built in: every thread reads its pieces, a
 // barrier, and the planes are written over them.
-// CARRY (packed forward-only calls of one state from zero): the carry over the chunk axis happens here, S_c+1 = e^{A_last} S_c + U,
-// so that the chunk states cross HBM once as what the output kernel reads instead of being written as sums, read and written
-// by a pass of their own and read again.  A CTA draws the next job; a sequence's chunks are spread evenly over the order
-// (k_chunk_jobs), so the predecessor of a job is usually done; a job only ever waits for a smaller ticket, whose CTA has
-// started, so the waiting ends (and is bounded like every other wait).  ticket[1] == 0: too few sequences side by side for
-// that, the sums are left to k_state_scan.
-// 32 documents of 512..16384 tokens (241,740 in all), 16 heads: 676 us where the sums and a carry of its own take 516 + 334.  (K
-// states take their links one after the other in a CTA; with three the pass of its own was as fast.)
-enum OuterMode { OUTER_PLAIN = 0, OUTER_FWD_ONLY = 1, OUTER_CARRY = 2 };
-
-__device__ __forceinline__ bool wait_ready(const unsigned int* flag) {
-  uint64_t t0 = 0;
-  for (uint32_t it = 0;; ++it) {
-    unsigned int v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
-    if (v) return true;
-    if ((it & 63) == 63) {
-      const uint64_t now = umma::global_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > umma::WAIT_NS) break;
-      if (umma::device_error_now() != 0) break;
-    }
-  }
-  umma::record_device_error(208);
-  return false;
-}
-__device__ __forceinline__ void set_ready(unsigned int* flag) {      // one thread, behind a CTA barrier that follows the stores
-  __threadfence();
-  asm volatile("st.release.gpu.global.u32 [%0], 1;" ::"l"(flag) : "memory");
-}
-// The job of this CTA: the next one (through `slot` in shared memory, a word of its own), or (not CARRY) the one its block index
-// names.
-template <bool CARRY>
-__device__ __forceinline__ ChunkLoc take_job(const ScanParams& p, unsigned int* slot, int& h) {
-  if (!CARRY) {
-    h = blockIdx.y;
-    return locate_chunk(p.geom, blockIdx.x);
-  }
-  if (threadIdx.x == 0) *slot = umma::device_error_now() != 0 ? 0xffffffffu : atomicAdd(p.ticket, 1u);      // after a failure: no new work
-  __syncthreads();
-  const unsigned int t = *slot;
-  ChunkLoc L;
-  L.valid = t < (unsigned int)p.geom.chunk_prefix[p.geom.S] * (unsigned int)p.H;
-  if (!L.valid) return L;
-  const unsigned int j = t / (unsigned int)p.H;
-  h = (int)(t - j * (unsigned int)p.H);
-  const ChunkJob& job = p.jobs[j];
-  L.seq = job.seq; L.c = job.c; L.nc = job.nc; L.b = 0; L.t0 = job.t0; L.len = job.len; L.slot0 = job.slot0;
-  return L;
-}
-
-// S_c+1 = g S_c + U of this CTA's accumulators, to the next slot or, after the last chunk, to the final destination (without
-// `carry`: U alone).
-__device__ __forceinline__ void carry_out(const ScanParams& p, const ChunkLoc& L, int k, int h, uint32_t tmem, int warp, int lane, float g, bool carry,
-                                          bool ok) {
-  const int q4 = warp & 3, cc = warp >> 2, n = q4 * 32 + lane;
-  const bool even = (lane & 1) == 0, last = carry ? L.c + 1 == L.nc : L.nc == 1;
-  const float* prev = reinterpret_cast<const float*>(p.states + state_base(p, k, h, L.slot0 + L.c, TD)) + n;
-  float* next = reinterpret_cast<float*>(p.states + state_base(p, k, h, L.slot0 + L.c + 1, TD)) + n;
-  FinalDest fin;
-  if (last) fin.init(p, L.seq, k, h);
-#pragma unroll 1
-  for (int hh = 0; hh < 2; ++hh) {
-    const int col = cc * 32 + hh * 16;
-    float pv[16], d1[16], d2[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) pv[i] = carry && L.c > 0 && ok ? __ldcg(prev + (size_t)(col + i) * 128) : 0.f;
-    umma::tmem_ld16x2(tmem + ((uint32_t)(q4 * 32) << 16) + col, d1, tmem + ((uint32_t)(q4 * 32) << 16) + 64 + col, d2);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float o = __shfl_xor_sync(0xffffffffu, d2[i], 1);
-      pv[i] = fmaf(g, pv[i], even ? d1[i] + o : o - d1[i]);
-    }
-    if (last) {
-#pragma unroll
-      for (int i = 0; i < 16; i += 2) fin.store2(p, (col + i) * 128 + n, pv[i], pv[i + 1], even, ok);
-    } else if (ok) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) next[(size_t)(col + i) * 128] = pv[i];
-    }
-  }
-}
-
-template <bool DSTATE, int MODE = OUTER_PLAIN>
+// SINGLE: every sequence is one chunk from zero, its sums are its final state as well.
+template <bool DSTATE, bool SINGLE = false>
 __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant__ CUtensorMap mk,
                                                            const __grid_constant__ CUtensorMap mv, ScanParams p) {
   using namespace umma;
@@ -209,11 +130,10 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
   uint64_t* bar = reinterpret_cast<uint64_t*>(wrow + TC);       // [0] MMAs  [1] token tiles
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr bool CARRY = MODE == OUTER_CARRY;
   pdl_wait();
-  int h;
-  const ChunkLoc L = take_job<CARRY>(p, tmem_slot + 1, h);
+  const ChunkLoc L = locate_chunk(p.geom, blockIdx.x);
   if (!L.valid) return;
+  const int h = blockIdx.y;
   const int kst = blockIdx.z;                 // state (its decay weights the rows); grid z = K
   float graw[4] = {1.f, 1.f, 1.f, 1.f};
   if (warp == 1) warp_cumsum128_load(graw, p.gamma + gamma_base(p, kst, L.b, h, L.t0), L.len, lane);
@@ -280,21 +200,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
   __syncwarp();
   bool ok = mbar_wait(&bar[0], 0, 201) && tiles_ok;
   tc_fence_after();
-  if constexpr (CARRY) {
-    unsigned int* ready = p.ready + ((size_t)kst * p.H + h) * p.nslots + L.slot0 + L.c;
-    const bool carry = p.ticket[1] != 0u;
-    if (carry) {
-      if (L.c > 0 && tid == 64) ok = wait_ready(ready) && ok;
-      ok = __syncthreads_and(ok);
-    }
-    carry_out(p, L, kst, h, tmem, warp, lane, __expf(a_last), carry, ok);
-    if (!carry) {
-      if (tid == 0 && ok) reinterpret_cast<float*>(ready)[1] = __expf(a_last);      // the chunk's decay, for k_state_scan
-    } else if (L.c + 1 < L.nc) {
-      __syncthreads();
-      if (tid == 0 && ok) set_ready(ready + 1);
-    }
-  } else {
+  {
     // lane n' = 2j+c of the tile holds column i: state[i][j][c] sits at float offset i*128 + n'
     float2* slot = DSTATE ? p.dstates + state_base(p, kst, h, L.slot0 + L.c, TD)
                           : p.states + state_base(p, kst, h, L.slot0 + L.c + 1, TD);
@@ -304,20 +210,16 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + cc * 32, d1);
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + 64 + cc * 32, d2);
     const bool even = (lane & 1) == 0;
-    const bool final_now = MODE == OUTER_FWD_ONLY && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform (fwd_only or single)
-    if (final_now) {
+    if (SINGLE) {
       FinalDest fin;
-      fin.init(p, L.seq, kst, h);
+      fin.init(p, L.seq, pool_slot_of(p, L.seq), kst, h);
 #pragma unroll
-      for (int i = 0; i < 32; i += 2) {
-        const float o0 = __shfl_xor_sync(0xffffffffu, d2[i], 1), o1 = __shfl_xor_sync(0xffffffffu, d2[i + 1], 1);
-        const float u0 = even ? d1[i] + o0 : o0 - d1[i], u1 = even ? d1[i + 1] + o1 : o1 - d1[i + 1];
-        fin.store2(p, (cc * 32 + i) * 128 + q4 * 32 + lane, u0, u1, even, ok);
-        if (p.single && ok) {
-          dst[(size_t)(cc * 32 + i) * 128] = u0;
-          dst[(size_t)(cc * 32 + i + 1) * 128] = u1;
-        }
+      for (int i = 0; i < 32; ++i) {
+        const float o = __shfl_xor_sync(0xffffffffu, d2[i], 1);
+        d1[i] = even ? d1[i] + o : o - d1[i];
+        if (ok) dst[(size_t)(cc * 32 + i) * 128] = d1[i];
       }
+      fin.store(p, cc * 32 * 128 + q4 * 32 + lane, d1, even, ok);
     } else {
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
@@ -440,7 +342,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
       // Re U = D1[2j] + D2[2j+1], Im U = D2[2j] - D1[2j+1]: lane n' = 2j+c holds column i, state[i][j][c] at i*128 + n'
       float2* slot = DSTATE ? p.dstates + state_base(p, k - 1, h, L.slot0 + L.c, TD) : p.states + state_base(p, k - 1, h, L.slot0 + L.c + 1, TD);
       float* dst = reinterpret_cast<float*>(slot) + (q4 * 32 + lane);
-      const bool final_now = !DSTATE && (p.fwd_only || p.single) && L.nc == 1 && p.s0 == nullptr;      // CTA-uniform
+      const bool final_now = !DSTATE && p.single;
 #pragma unroll 1
       for (int hh = 0; hh < 4; ++hh) {          // 8 columns at a time
         float d1[8], d2[8];
@@ -448,17 +350,14 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
         tmem_ld8x2(tmem + ((uint32_t)(q4 * 32) << 16) + col, d1, tmem + ((uint32_t)(q4 * 32) << 16) + 64 + col, d2);
         if (final_now) {
           FinalDest fin;
-          fin.init(p, L.seq, k - 1, h);
+          fin.init(p, L.seq, pool_slot_of(p, L.seq), k - 1, h);
 #pragma unroll
-          for (int i = 0; i < 8; i += 2) {
-            const float o0 = __shfl_xor_sync(0xffffffffu, d2[i], 1), o1 = __shfl_xor_sync(0xffffffffu, d2[i + 1], 1);
-            const float u0 = even ? d1[i] + o0 : o0 - d1[i], u1 = even ? d1[i + 1] + o1 : o1 - d1[i + 1];
-            fin.store2(p, (int)(col + i) * 128 + q4 * 32 + lane, u0, u1, even, ok);
-            if (p.single && ok) {
-              dst[(size_t)(col + i) * 128] = u0;
-              dst[(size_t)(col + i + 1) * 128] = u1;
-            }
+          for (int i = 0; i < 8; ++i) {
+            const float o = __shfl_xor_sync(0xffffffffu, d2[i], 1);
+            d1[i] = even ? d1[i] + o : o - d1[i];
+            if (ok) dst[(size_t)(col + i) * 128] = d1[i];
           }
+          fin.store(p, (int)col * 128 + q4 * 32 + lane, d1, even, ok);
         } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {

@@ -89,9 +89,8 @@ __device__ __forceinline__ void bw_issue_scores(uint32_t slot, uint32_t a_r, uin
   mma_run(slot + 128, imag_swapped ? ai : ar, imag_swapped ? br : bi, 2, 2, imag_swapped ? id : idn, 4, true);
 }
 
-// TMEM column of the packed bf16 scores of k-step kk (16 score columns = 8 TMEM columns): the thread that
-// owns score columns [32 cq, 32 cq + 32) of a row writes  Tr(2cq) Tr(2cq+1) Ti(2cq) Ti(2cq+1)  over them, so the real parts
-// are at 0, 8, 32, 40, 64, ... and the imaginary parts 16 further on.
+// TMEM columns of the packed bf16 scores of k-step kk (16 score columns): a thread writes the 8 words of the real parts to 16 kk and
+// the 8 of the imaginary parts behind them, over the 16 Xr columns they came from.
 
 // acc = T X2 : out_r = Tr x2r - Ti x2i, out_i = Tr x2i + Ti x2r   (X2 planes MN-major, K = 128 tokens).  The real scores multiply
 // both planes at once (one B operand of 128 columns, its halves 16 KB apart).
@@ -99,9 +98,9 @@ __device__ __forceinline__ void bw_issue_out(uint32_t slot, uint32_t x_r, bool a
   using namespace umma;
   constexpr uint32_t id = idesc_bf16(128, 64, false, true), id2 = idesc_bf16(128, 128, false, true);
   constexpr uint32_t idn = idesc_bf16_nega(128, 64, false, true);
-  mma_run_ts(slot + 128, slot, smem_desc_sw128(x_r, 16384, 1024), 8, 24, 128, id2, 8, accumulate);
-  mma_run_ts(slot + 128, slot + 16, smem_desc_sw128(x_r + 16384, 16, 1024), 8, 24, 128, idn, 8, true);
-  mma_run_ts(slot + 192, slot + 16, smem_desc_sw128(x_r, 16, 1024), 8, 24, 128, id, 8, true);
+  mma_run_ts(slot + 128, slot, smem_desc_sw128(x_r, 16384, 1024), 16, 128, id2, 8, accumulate);
+  mma_run_ts(slot + 128, slot + 8, smem_desc_sw128(x_r + 16384, 16, 1024), 16, 128, idn, 8, true);
+  mma_run_ts(slot + 192, slot + 8, smem_desc_sw128(x_r, 16, 1024), 16, 128, id, 8, true);
 }
 
 // acc (+)= A1 (.) state planes [64 rows i][64 j]:  op_h == false: out[r][i] = sum_j a[r][j] S[i][j]  (a_r S_r - a_i S_i; a_r S_i + a_i S_r);
@@ -114,56 +113,52 @@ __device__ __forceinline__ void bw_issue_state(const bool op_h, uint32_t slot, u
   mma_run_complex(slot + 128, slot + 192, ar, ai, sr, si, 2, op_h ? 128 : 2, id, op_h ? id : idn, op_h ? idn : id, !op_h, 4, accumulate);
 }
 
-// ---- epilogue 1: decay-masked scores of this thread's row, columns [32 cb, 32 cb + 32), as packed bf16 ------
+// ---- epilogue 1: decay-masked scores of this thread's row, columns [64 hf, 64 hf + 64), 16 at a time, as packed bf16 ------
 // fast path: T = [mask] cfac[col] X;  slow path (STRONG): T = [mask] scale exp(-|A_row - A_col|) X.
 // The row's own factor `rowf` (1 where it is applied later) multiplies the weight before the score is rounded (see chunk_job).
+// (A rolled loop of 16 columns: written out for 64 the two forms were 20 KB of code.)
 template <bool STRONG>
-__device__ __forceinline__ void bw_epi_scores_t(const bool lower, uint32_t tlane_slot, int q4, int cb, int r, int len,
+__device__ __forceinline__ void bw_epi_scores_t(const bool lower, uint32_t tlane_slot, int q4, int hf, int r, int len,
                                                 const float* __restrict__ cfac, const float* __restrict__ Acum,
                                                 float scale, float rowf) {
   using namespace umma;
-  const int c0 = 32 * cb;
-  const bool dead = lower ? (c0 > q4 * 32 + 31) : (c0 + 31 < q4 * 32);      // warp-uniform
-  const bool full = lower ? (c0 + 31 <= q4 * 32) : (c0 >= q4 * 32 + 31);    // no triangle inside the block
-  // columns that count: [0, r] below the diagonal, [r, 128) above it, all of them without a diagonal in the block
-  const int first = full || lower ? 0 : r, last = full || !lower ? TC - 1 : r;
-  uint32_t tr[16], ti[16];
-  if (dead) {
+  const float a_r = STRONG ? Acum[r] : 0.f;
+#pragma unroll 1
+  for (int c0 = 64 * hf; c0 < 64 * hf + 64; c0 += 16) {
+    const bool dead = lower ? (c0 > q4 * 32 + 31) : (c0 + 15 < q4 * 32);      // warp-uniform
+    const bool full = lower ? (c0 + 15 <= q4 * 32) : (c0 >= q4 * 32 + 31);    // no triangle inside the block
+    // columns that count: [0, r] below the diagonal, [r, 128) above it, all of them without a diagonal in the block
+    const int first = full || lower ? 0 : r, last = full || !lower ? TC - 1 : r;
+    uint32_t out[16];
+    if (dead) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) tr[j] = ti[j] = 0u;
-  } else {
-    const float a_r = STRONG ? Acum[r] : 0.f;
-    uint32_t xr0[16], xr1[16], xi0[16], xi1[16];
-    tmem_ld16x4(tlane_slot + c0, xr0, tlane_slot + c0 + 16, xr1, tlane_slot + 128 + c0, xi0, tlane_slot + 128 + c0 + 16, xi1);
-#pragma unroll
-    for (int hh = 0; hh < 2; ++hh) {
+      for (int j = 0; j < 16; ++j) out[j] = 0u;
+    } else {
+      float xr[16], xi[16];
+      tmem_ld16x2(tlane_slot + c0, xr, tlane_slot + 128 + c0, xi);
 #pragma unroll
       for (int j = 0; j < 16; j += 2) {
         float d[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int c = c0 + 16 * hh + j + e;
+          const int c = c0 + j + e;
           bool on = (unsigned)(c - first) <= (unsigned)(last - first);
           if (STRONG && !lower) on = on && (c < len);      // (the column factors of the fast path are zero past `len`)
           const float w = STRONG ? scale * __expf(fminf(0.f, lower ? a_r - Acum[c] : Acum[c] - a_r)) : rowf * cfac[c];
           d[e] = on ? w : 0.f;
         }
-        const float r0 = __uint_as_float(hh ? xr1[j] : xr0[j]), r1 = __uint_as_float(hh ? xr1[j + 1] : xr0[j + 1]);
-        const float i0 = __uint_as_float(hh ? xi1[j] : xi0[j]), i1 = __uint_as_float(hh ? xi1[j + 1] : xi0[j + 1]);
-        tr[hh * 8 + (j >> 1)] = pack_bf162(d[0] * r0, d[1] * r1);
-        ti[hh * 8 + (j >> 1)] = pack_bf162(d[0] * i0, d[1] * i1);
+        out[j >> 1] = pack_bf162(d[0] * xr[j], d[1] * xr[j + 1]);
+        out[8 + (j >> 1)] = pack_bf162(d[0] * xi[j], d[1] * xi[j + 1]);
       }
     }
+    tmem_st16(tlane_slot + c0, out);      // (the loads of these columns have completed)
   }
-  // every load of this thread has completed: its own 32 Xr columns take the packed scores
-  tmem_st16(tlane_slot + c0, tr);
-  tmem_st16(tlane_slot + c0 + 16, ti);
 }
-__device__ __forceinline__ void bw_epi_scores(const bool lower, uint32_t tlane_slot, int q4, int cb, int r, int len, bool strong,
+__device__ __forceinline__ void bw_epi_scores(const bool lower, uint32_t tlane_slot, int q4, int hf, int r, int len, bool strong,
                                               const float* __restrict__ cfac, const float* __restrict__ Acum,
                                               float scale, float rowf) {
-  if (strong) bw_epi_scores_t<true>(lower, tlane_slot, q4, cb, r, len, cfac, Acum, scale, 1.f);
-  else bw_epi_scores_t<false>(lower, tlane_slot, q4, cb, r, len, cfac, Acum, scale, rowf);
+  if (strong) bw_epi_scores_t<true>(lower, tlane_slot, q4, hf, r, len, cfac, Acum, scale, 1.f);
+  else bw_epi_scores_t<false>(lower, tlane_slot, q4, hf, r, len, cfac, Acum, scale, rowf);
 }
 
 // ---- epilogue 2: out[r][16 cb .. 16 cb + 16) = rf * acc -> global; optional part of Re<x_r, out_r>, x_r given as the
@@ -371,9 +366,7 @@ __device__ __forceinline__ void chunk_job(const int mode, const CUtensorMap* __r
   const int r = q4 * 32 + lane;                               // this thread's row (TMEM lane)
   const uint32_t tl = tmem + ((uint32_t)(q4 * 32) << 16);
   // epilogue 1: masked, decayed scores of columns [64 hf, 64 hf + 64) as packed bf16 pairs
-#pragma unroll 1
-  for (int cb = 2 * hf; cb < 2 * hf + 2; ++cb)
-    bw_epi_scores(LOWER, tl, q4, cb, r, L.len, strong, cfac, Acum, p.q_scale, ROWW ? rfac[r] : 1.f);
+  bw_epi_scores(LOWER, tl, q4, hf, r, L.len, strong, cfac, Acum, p.q_scale, ROWW ? rfac[r] : 1.f);
   tmem_st_wait();
   if (ROWW && has_state && !strong) {
     // stage 1 was the last reader of the unscaled A1 rows: thread (row r, plane hf) multiplies its 128 bytes by the

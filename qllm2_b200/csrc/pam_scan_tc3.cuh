@@ -18,12 +18,10 @@
 //   stage 2  acc = T V                               acc_r: cols [128,192)  acc_i: cols [192,256)
 //   pass p   T'_k -> cols [64 s, 64 s + 64), real half, imaginary half (s = slot of state k in the pass)
 //            acc += T'_k (e^{A^k_m} S^k)^T
-// (Weights and states are formed in loops that are not unrolled over column groups: straight-line code missed the instruction
-// cache 460 times a job.  8 x 6 x 2048, three states: 76 -> 66 us; 48 chat prompts: 187 -> 163.)
+// (Weights and states are formed in loops that are not unrolled over column groups, and the number of states is a template argument:
+// straight-line code missed the instruction cache 460 times a job.  8 x 6 x 2048, three states: 76 -> 66 us; 48 chat prompts: 187 -> 163.)
 //   epi 2    y = acc
 #pragma once
-#include <type_traits>
-
 #include "pam_scan_tc2.cuh"
 
 namespace qpam {
@@ -31,6 +29,131 @@ namespace tcs {
 
 constexpr size_t CHUNKK_SMEM = 1024 + 3 * 32768 + 9216;
 
+// ---- pieces of a K-state chunk job, shared with the walking form (pam_scan_walk.cuh)
+// epilogue 1: weighted, masked scores of columns [64 hf, 64 hf + 64), 16 at a time, as packed bf16 pairs over the columns they came from
+template <int K, bool STRONG>
+__device__ __forceinline__ void kstate_scores_t(uint32_t tlane, int q4, int hf, int r, uint32_t strong_mask, const float2 (&rk)[K],
+                                                const float* __restrict__ cfac, const float* __restrict__ Acum) {
+  using namespace umma;
+#pragma unroll 1
+  for (int c0 = 64 * hf; c0 < 64 * hf + 64; c0 += 16) {
+    uint32_t out[16];
+    if (c0 > q4 * 32 + 31) {                  // warp-uniform: the whole block lies above the diagonal
+#pragma unroll
+      for (int j = 0; j < 16; ++j) out[j] = 0u;
+    } else {
+      float xr[16], xi[16];
+      tmem_ld16x2(tlane + c0, xr, tlane + 128 + c0, xi);
+#pragma unroll
+      for (int j = 0; j < 16; j += 2) {
+        // the weights of two columns, and their products with the scores, two numbers an instruction
+        const int c = c0 + j;
+        float2 gr = make_float2(0.f, 0.f), gi = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          float2 cf = *reinterpret_cast<const float2*>(cfac + k * TC + c);
+          if (STRONG && ((strong_mask >> k) & 1u)) {
+            const float a = Acum[k * TC + r];
+            cf = make_float2(__expf(fminf(0.f, a - Acum[k * TC + c])), __expf(fminf(0.f, a - Acum[k * TC + c + 1])));
+          }
+          gr = ffma2(make_float2(rk[k].x, rk[k].x), cf, gr);
+          gi = ffma2(make_float2(rk[k].y, rk[k].y), cf, gi);
+        }
+        if (c > r) gr.x = gi.x = 0.f;
+        if (c + 1 > r) gr.y = gi.y = 0.f;
+        const float2 x = make_float2(xr[j], xr[j + 1]), y = make_float2(xi[j], xi[j + 1]);
+        const float2 wr = ffma2(x, gr, fmul2(make_float2(-y.x, -y.y), gi)), wi = ffma2(x, gi, fmul2(y, gr));
+        out[j >> 1] = pack_bf162(wr.x, wr.y);
+        out[8 + (j >> 1)] = pack_bf162(wi.x, wi.y);
+      }
+    }
+    tmem_st16(tlane + c0, out);
+  }
+  tmem_st_wait();
+}
+// (the two forms differ only in how a state's column factor is formed: the common case -- no state of this chunk decays strongly,
+// CTA-uniform -- keeps the exponentials out of the per-score code)
+template <int K>
+__device__ __forceinline__ void kstate_scores(uint32_t tlane, int q4, int hf, int r, uint32_t strong_mask, const float2 (&rk)[K],
+                                              const float* __restrict__ cfac, const float* __restrict__ Acum) {
+  if (strong_mask == 0u) kstate_scores_t<K, false>(tlane, q4, hf, r, strong_mask, rk, cfac, Acum);
+  else kstate_scores_t<K, true>(tlane, q4, hf, r, strong_mask, rk, cfac, Acum);
+}
+// the chunk constant e^{A_m} of a state (1 where its rows carry the whole decay)
+__device__ __forceinline__ float state_const(const float* Acum, uint32_t strong_mask, int k) {
+  return ((strong_mask >> k) & 1u) ? 1.f : __expf(Acum[k * TC + TC / 2 - 1]);
+}
+// planes of a carried state (fp32 [i][j] (re, im)), times its chunk constant, into 16 KB at `dstp`
+__device__ __forceinline__ void kstate_planes(unsigned char* dstp, const void* state, float cst, int tid) {
+  const float4* sg = reinterpret_cast<const float4*>(state);
+  float4 v[8];                               // all of them requested before the first is used
+#pragma unroll
+  for (int it = 0; it < 8; ++it) v[it] = ld_dependent(sg + (tid + 256 * (it >> 1)) * 2 + (it & 1));
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int idx = tid + 256 * it;          // (i, c16): state[i][4*c16 .. +3]
+    const float4 s01 = v[2 * it], s23 = v[2 * it + 1];
+    const int i = idx >> 4, c16 = idx & 15;
+    const uint32_t off = sw128(i, c16 >> 1) + (c16 & 1) * 8;
+    *reinterpret_cast<uint2*>(dstp + off) = make_uint2(pack_bf162(cst * s01.x, cst * s01.z), pack_bf162(cst * s23.x, cst * s23.z));
+    *reinterpret_cast<uint2*>(dstp + 8192 + off) = make_uint2(pack_bf162(cst * s01.y, cst * s01.w), pack_bf162(cst * s23.y, cst * s23.w));
+  }
+}
+// T'[r][j] = rho_k[r] q_r[j], j = 0..63, as packed bf16 pairs: 32 columns of reals, 32 of imaginaries (slot hf of the pass)
+template <int K>
+__device__ __forceinline__ void kstate_rows(uint32_t tlane, const unsigned char* RA, int hf, int r, int k_mine, uint32_t strong_mask, const float2 (&rk)[K],
+                                            const float* __restrict__ Acum) {
+  using namespace umma;
+  float2 rr = rk[0];                           // (a select chain keeps rk in registers)
+#pragma unroll
+  for (int k = 1; k < K; ++k)
+    if (k_mine == k) rr = rk[k];
+  if ((strong_mask >> k_mine) & 1u) {          // unfactored state: the row's own decay goes here
+    const float ea = __expf(Acum[k_mine * TC + r]);
+    rr.x *= ea;
+    rr.y *= ea;
+  }
+#pragma unroll 1
+  for (int g = 0; g < 2; ++g) {                // 32 channels at a time: 16 columns of reals, 16 of imaginaries
+    uint32_t wr[16], wi[16];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint4 qr = *reinterpret_cast<const uint4*>(RA + sw128(r, 4 * g + c));
+      const uint4 qi = *reinterpret_cast<const uint4*>(RA + 16384 + sw128(r, 4 * g + c));
+      const uint32_t qrw[4] = {qr.x, qr.y, qr.z, qr.w}, qiw[4] = {qi.x, qi.y, qi.z, qi.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 a = unpack_bf162(qrw[e]), b = unpack_bf162(qiw[e]);   // two consecutive channels
+        wr[c * 4 + e] = pack_bf162(a.x * rr.x - b.x * rr.y, a.y * rr.x - b.y * rr.y);
+        wi[c * 4 + e] = pack_bf162(a.x * rr.y + b.x * rr.x, a.y * rr.y + b.y * rr.x);
+      }
+    }
+    tmem_st16(tlane + hf * 64 + g * 16, wr);
+    tmem_st16(tlane + hf * 64 + 32 + g * 16, wi);
+  }
+  tmem_st_wait();
+}
+// acc += T' S^T of the states in `n` slots (one thread)
+__device__ __forceinline__ void kstate_issue(uint32_t tmem, uint32_t b_r, int n) {
+  using namespace umma;
+  constexpr uint32_t k3 = idesc_bf16(128, 64, false, false), k3n = idesc_bf16_nega(128, 64, false, false);
+#pragma unroll 1
+  for (int s = 0; s < n; ++s) {
+    uint64_t sr = smem_desc_sw128(b_r + s * 16384, 16, 1024), si = smem_desc_sw128(b_r + s * 16384 + 8192, 16, 1024);   // [64 rows i][64 j] planes of this slot
+    uint32_t tr_ = tmem + s * 64, ti_ = tr_ + 32;
+#pragma unroll 1
+    for (int kk = 0; kk < 4; ++kk) {
+      mma_bf16_ts(tmem + 128, tr_, sr, k3, true);    // + T'r Sr^T
+      mma_bf16_ts(tmem + 128, ti_, si, k3n, true);   // - T'i Si^T
+      mma_bf16_ts(tmem + 192, tr_, si, k3, true);    // + T'r Si^T
+      mma_bf16_ts(tmem + 192, ti_, sr, k3, true);    // + T'i Sr^T
+      tr_ += 8; ti_ += 8;
+      sr += 2; si += 2;
+    }
+  }
+}
+
+template <int K>
 __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant__ ChunkMaps maps, ScanParams p) {
   using namespace umma;
   extern __shared__ unsigned char smem_raw[];
@@ -52,7 +175,6 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   }
   if (tid == 160) *failed = device_error_now();
   const int h = blockIdx.y;
-  const int K = p.K;
   const bool has_state = (L.c > 0) || (p.s0 != nullptr);
   const int row0 = (L.b * p.H + h) * p.T + L.t0;
   if (tid == 0) {
@@ -96,8 +218,8 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   // scores get exp(A_t - A_s) one by one and its carried-state rows their own e^{A_t}
   uint32_t strong_mask = 0;
 #pragma unroll
-  for (int k = 0; k < KMAX; ++k)
-    if (k < K && Acum[k * TC + TC - 1] < STRONG_DECAY) strong_mask |= 1u << k;
+  for (int k = 0; k < K; ++k)
+    if (Acum[k * TC + TC - 1] < STRONG_DECAY) strong_mask |= 1u << k;
 #pragma unroll
   for (int m = 0; m < 2; ++m) {          // KMAX * TC = 512 entries, two per thread
     const int e = tid + 256 * m;
@@ -146,79 +268,19 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   const int q4 = warp & 3, hf = warp >> 2;
   const int r = q4 * 32 + lane;                               // this thread's row (TMEM lane)
   const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);
-  float2 rk[KMAX];                                            // rho_k of this row
+  float2 rk[K];                                               // rho_k of this row
 #pragma unroll
-  for (int k = 0; k < KMAX; ++k) rk[k] = (k < K) ? rho[k * TC + r] : make_float2(0.f, 0.f);
+  for (int k = 0; k < K; ++k) rk[k] = rho[k * TC + r];
 
-  // carried-state planes of state k (times its chunk constant e^{A^k_m}) into slot s of the K-plane region
   auto stage_state = [&](int k, int s) {
-    const float cst = ((strong_mask >> k) & 1u) ? 1.f : __expf(Acum[k * TC + TC / 2 - 1]);
-    const float4* sg = reinterpret_cast<const float4*>(p.states + state_base(p, k, h, L.slot0 + L.c, TD));
-    unsigned char* dstp = RB + s * 16384;
-    float4 v[8];                               // all of them requested before the first is used
-#pragma unroll
-    for (int it = 0; it < 8; ++it) v[it] = ld_dependent(sg + (tid + 256 * (it >> 1)) * 2 + (it & 1));
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int idx = tid + 256 * it;          // (i, c16): state[i][4*c16 .. +3]
-      const float4 s01 = v[2 * it], s23 = v[2 * it + 1];
-      const int i = idx >> 4, c16 = idx & 15;
-      const uint32_t off = sw128(i, c16 >> 1) + (c16 & 1) * 8;
-      *reinterpret_cast<uint2*>(dstp + off) = make_uint2(pack_bf162(cst * s01.x, cst * s01.z), pack_bf162(cst * s23.x, cst * s23.z));
-      *reinterpret_cast<uint2*>(dstp + 8192 + off) = make_uint2(pack_bf162(cst * s01.y, cst * s01.w), pack_bf162(cst * s23.y, cst * s23.w));
-    }
+    kstate_planes(RB + s * 16384, p.states + state_base(p, k, h, L.slot0 + L.c, TD), state_const(Acum, strong_mask, k), tid);
   };
 
   {
-    // epilogue 1: weighted, masked scores of columns [64 hf, 64 hf + 64), 32 at a time, as packed bf16 pairs over the columns they
-    // came from
-#pragma unroll 1
-    for (int cb = 2 * hf; cb < 2 * hf + 2; ++cb) {
-      uint32_t out[2][16];                      // 16 columns of the real parts and 16 of the imaginary parts (two columns a word)
-      const bool dead = cb * 32 > q4 * 32 + 31;      // warp-uniform: the whole block lies above the diagonal
-      if (dead) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) out[0][j] = out[1][j] = 0u;
-      } else {
-        uint32_t x0[16], x1[16], y0[16], y1[16];
-        tmem_ld16x4(tlane + cb * 32, x0, tlane + cb * 32 + 16, x1, tlane + 128 + cb * 32, y0, tlane + 128 + cb * 32 + 16, y1);
-        // (the two forms differ only in how a state's column factor is formed: the common case -- no state of this
-        // chunk decays strongly, CTA-uniform -- keeps the exponentials out of the per-score code)
-        auto weigh = [&](auto any_strong) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            float wr[2], wi[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int c = cb * 32 + j + e;
-              float gr = 0.f, gi = 0.f;
-#pragma unroll
-              for (int k = 0; k < KMAX; ++k)
-                if (k < K) {
-                  const float cf = decltype(any_strong)::value && ((strong_mask >> k) & 1u) ? __expf(fminf(0.f, Acum[k * TC + r] - Acum[k * TC + c]))
-                                                                                            : cfac[k * TC + c];
-                  gr = fmaf(rk[k].x, cf, gr);
-                  gi = fmaf(rk[k].y, cf, gi);
-                }
-              if (c > r) gr = gi = 0.f;
-              const float xr = __uint_as_float(j < 16 ? x0[(j + e) & 15] : x1[(j + e) & 15]), xi = __uint_as_float(j < 16 ? y0[(j + e) & 15] : y1[(j + e) & 15]);
-              wr[e] = xr * gr - xi * gi;
-              wi[e] = xr * gi + xi * gr;
-            }
-            out[0][j >> 1] = pack_bf162(wr[0], wr[1]);
-            out[1][j >> 1] = pack_bf162(wi[0], wi[1]);
-          }
-        };
-        if (strong_mask == 0u) weigh(std::false_type());
-        else weigh(std::true_type());
-      }
-      tmem_st16(tlane + cb * 32, out[0]);
-      tmem_st16(tlane + cb * 32 + 16, out[1]);
-    }
-    tmem_st_wait();
+    kstate_scores<K>(tlane, q4, hf, r, strong_mask, rk, cfac, Acum);
     if (has_state) {          // the K planes are no longer needed: states 0 and 1 take their place
-      stage_state(0, 0);
-      if (K > 1) stage_state(1, 1);
+#pragma unroll 1
+      for (int k = 0; k < 2; ++k) stage_state(k, k);
     }
   }
   fence_proxy_async();
@@ -233,63 +295,20 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   ok = mbar_wait(&bars[2], 0, 233) && ok;
   tc_fence_after();
   if (has_state) {
+#pragma unroll 1
     for (int pass = 0; pass * 2 < K; ++pass) {
       const int k_mine = pass * 2 + hf;                 // the state whose rows this half of the CTA writes
       if (pass > 0) {                                   // the previous pass has finished with both slots
-        stage_state(pass * 2, 0);
-        if (pass * 2 + 1 < K) stage_state(pass * 2 + 1, 1);
-      }
-      if (k_mine < K) {
-        // T'[r][j] = rho_k[r] q_r[j], j = 0..63, as packed bf16 pairs: 32 columns of reals, 32 of imaginaries
-        float2 rr = rk[0];                           // (a select chain keeps rk in registers)
-#pragma unroll
-        for (int k = 1; k < KMAX; ++k)
-          if (k_mine == k) rr = rk[k];
-        if ((strong_mask >> k_mine) & 1u) {          // unfactored state: the row's own decay goes here
-          const float ea = __expf(Acum[k_mine * TC + r]);
-          rr.x *= ea;
-          rr.y *= ea;
-        }
 #pragma unroll 1
-        for (int g = 0; g < 2; ++g) {                // 32 channels at a time: 16 columns of reals, 16 of imaginaries
-          uint32_t wr[16], wi[16];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint4 qr = *reinterpret_cast<const uint4*>(RA + sw128(r, 4 * g + c));
-            const uint4 qi = *reinterpret_cast<const uint4*>(RA + 16384 + sw128(r, 4 * g + c));
-            const uint32_t qrw[4] = {qr.x, qr.y, qr.z, qr.w}, qiw[4] = {qi.x, qi.y, qi.z, qi.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 a = unpack_bf162(qrw[e]), b = unpack_bf162(qiw[e]);   // two consecutive channels
-              wr[c * 4 + e] = pack_bf162(a.x * rr.x - b.x * rr.y, a.y * rr.x - b.y * rr.y);
-              wi[c * 4 + e] = pack_bf162(a.x * rr.y + b.x * rr.x, a.y * rr.y + b.y * rr.x);
-            }
-          }
-          tmem_st16(tlane + hf * 64 + g * 16, wr);
-          tmem_st16(tlane + hf * 64 + 32 + g * 16, wi);
-        }
-        tmem_st_wait();
+        for (int k = pass * 2; k < K && k < pass * 2 + 2; ++k) stage_state(k, k & 1);
       }
+      if (k_mine < K) kstate_rows<K>(tlane, RA, hf, r, k_mine, strong_mask, rk, Acum);
       fence_proxy_async();
       tc_fence_before();
       __syncthreads();
       if (warp == 0 && elect_one()) {
         tc_fence_after();
-        constexpr uint32_t k3 = idesc_bf16(128, 64, false, false), k3n = idesc_bf16_nega(128, 64, false, false);
-#pragma unroll 1
-        for (int s = 0; s < 2 && pass * 2 + s < K; ++s) {
-          uint64_t sr = smem_desc_sw128(b_r + s * 16384, 16, 1024), si = smem_desc_sw128(b_r + s * 16384 + 8192, 16, 1024);   // [64 rows i][64 j] planes of this slot
-          uint32_t tr_ = tmem + s * 64, ti_ = tr_ + 32;
-#pragma unroll 1
-          for (int kk = 0; kk < 4; ++kk) {
-            mma_bf16_ts(tmem + 128, tr_, sr, k3, true);    // + T'r Sr^T
-            mma_bf16_ts(tmem + 128, ti_, si, k3n, true);   // - T'i Si^T
-            mma_bf16_ts(tmem + 192, tr_, si, k3, true);    // + T'r Si^T
-            mma_bf16_ts(tmem + 192, ti_, sr, k3, true);    // + T'i Sr^T
-            tr_ += 8; ti_ += 8;
-            sr += 2; si += 2;
-          }
-        }
+        kstate_issue(tmem, b_r, pass * 2 + 1 < K ? 2 : 1);
         mma_commit(&bars[3 + pass]);
       }
       __syncwarp();

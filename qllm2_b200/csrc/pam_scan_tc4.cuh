@@ -48,9 +48,9 @@ __device__ __forceinline__ void issue_rows(uint32_t t, uint32_t acc, uint32_t x_
   constexpr uint32_t id = idesc_bf16(128, 64, false, true);
   constexpr uint32_t idn = idesc_bf16_nega(128, 64, false, true);
   constexpr uint32_t id2 = idesc_bf16(128, 128, false, true);      // (both planes of X2 as one B operand: N blocks 16 KB apart)
-  mma_run_ts(acc, t, smem_desc_sw128(x_r, 16384, 1024), 16, 16, 128, id2, 8, false);
-  mma_run_ts(acc, t + 8, smem_desc_sw128(x_r + 16384, 16, 1024), 16, 16, 128, idn, 8, true);
-  mma_run_ts(acc + 64, t + 8, smem_desc_sw128(x_r, 16, 1024), 16, 16, 128, id, 8, true);
+  mma_run_ts(acc, t, smem_desc_sw128(x_r, 16384, 1024), 16, 128, id2, 8, false);
+  mma_run_ts(acc, t + 8, smem_desc_sw128(x_r + 16384, 16, 1024), 16, 128, idn, 8, true);
+  mma_run_ts(acc + 64, t + 8, smem_desc_sw128(x_r, 16, 1024), 16, 128, id, 8, true);
 }
 
 struct BwdTables {

@@ -337,14 +337,14 @@ __device__ __forceinline__ void mma_run(uint32_t d_tmem, uint64_t a, uint64_t b,
     b += db;
   }
 }
-// the same with A in tensor memory, its column advancing by da0 and da1 in turn
-__device__ __forceinline__ void mma_run_ts(uint32_t d_tmem, uint32_t a, uint64_t b, uint32_t da0, uint32_t da1, uint32_t db, uint32_t idesc, int n,
+// the same with A in tensor memory, da columns a step
+__device__ __forceinline__ void mma_run_ts(uint32_t d_tmem, uint32_t a, uint64_t b, uint32_t da, uint32_t db, uint32_t idesc, int n,
                                         bool accumulate) {
 #pragma unroll 1
   for (int i = 0; i < n; ++i) {
     mma_bf16_ts(d_tmem, a, b, idesc, accumulate);
     accumulate = true;
-    a += (i & 1) ? da1 : da0;
+    a += da;
     b += db;
   }
 }
