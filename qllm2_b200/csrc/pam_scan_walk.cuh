@@ -243,8 +243,48 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
     if (sums) {
       constexpr int G = OUT ? 16 : 8;          // columns at a time (three CTAs per SM have fewer registers)
       float pv[G];                             // that many of the thread's elements of the entering state, ahead of their use
+      // the sums of state k leave the accumulators: S' = g S + U, U as in k_tc_chunk_outer
+      auto sums_out = [&](int k) {
+        const uint32_t from = tl + (OUT ? (uint32_t)(k & 1) * 128u : 0u);
+        // lane n' = 2j+c holds column i, state[i][j][c] at i*128 + n'
+        const float g = __expf(Acum[k * TC + TC - 1]);
+        const float* prev = has_state ? entering(k) + hf * 4096 + r : nullptr;
+        float* next = reinterpret_cast<float*>(p.states + state_base(p, k, s.h, to_slot, TD)) + hf * 4096 + r;
+        FinalDest fin;
+        if (to_final) fin.init(p, s.job.seq, s.job.pool_slot, k, s.h);
+#pragma unroll 1
+        for (int hh = 0; hh < 32 / G; ++hh) {
+          float d1[G], d2[G];
+          const uint32_t col = (uint32_t)(hf * 32 + hh * G);
+          if constexpr (OUT) tmem_ld16x2(from + col, d1, from + 64 + col, d2);
+          else tmem_ld8x2(from + col, d1, from + 64 + col, d2);
+#pragma unroll
+          for (int i = 0; i < G; i += 2) {      // two columns an instruction
+            const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, d2[i], 1), __shfl_xor_sync(0xffffffffu, d2[i + 1], 1));
+            float2 u = ffma2(make_float2(sign, sign), make_float2(d1[i], d1[i + 1]), o);
+            if (has_state) u = ffma2(make_float2(g, g), make_float2(pv[i], pv[i + 1]), u);
+            d1[i] = u.x;
+            d1[i + 1] = u.y;
+          }
+          if (has_state) {
+            if (OUT && hh == 0) {
+#pragma unroll
+              for (int i = 0; i < G; ++i) pv[i] = __ldcg(prev + 2048 + i * 128);
+            }
+          }
+          if (to_final) {
+            fin.store(p, (int)col * 128 + r, d1, even, ok);
+          } else if (ok) {
+#pragma unroll
+            for (int i = 0; i < G; ++i) next[i * 128] = d1[i];
+            next += 128 * G;
+          }
+        }
+        if (!OUT && ok && tid == 0) p.chunk_decay[((size_t)k * p.H + s.h) * p.nslots + s.job.slot0 + s.c + 1] = g;
+      };
 #pragma unroll 1
       for (int k = 0; k <= K; ++k) {
+        if (!OUT && k > 0) sums_out(k - 1);
         if (k < K) {
 #pragma unroll
           for (int it = 0; it < 8; ++it) {
@@ -256,57 +296,22 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
             *reinterpret_cast<uint2*>(planes + 2048 * it) = make_uint2(pack_bf162(x[0].x, x[1].x), pack_bf162(x[2].x, x[3].x));
             *reinterpret_cast<uint2*>(planes + 16384 + 2048 * it) = make_uint2(pack_bf162(x[0].y, x[1].y), pack_bf162(x[2].y, x[3].y));
           }
-        }
-        if (k > 0) {
-          // S' = g S + U, U as in k_tc_chunk_outer: lane n' = 2j+c holds column i, state[i][j][c] at i*128 + n'
-          const float g = __expf(Acum[(k - 1) * TC + TC - 1]);
-          const float* prev = has_state ? entering(k - 1) + hf * 4096 + r : nullptr;
-          float* next = reinterpret_cast<float*>(p.states + state_base(p, k - 1, s.h, to_slot, TD)) + hf * 4096 + r;
-          FinalDest fin;
-          if (to_final) fin.init(p, s.job.seq, s.job.pool_slot, k - 1, s.h);
-#pragma unroll 1
-          for (int hh = 0; hh < 32 / G; ++hh) {
-            float d1[G], d2[G];
-            const uint32_t col = (uint32_t)(hf * 32 + hh * G);
-            if constexpr (OUT) tmem_ld16x2(tl + col, d1, tl + 64 + col, d2);
-            else tmem_ld8x2(tl + col, d1, tl + 64 + col, d2);
-#pragma unroll
-            for (int i = 0; i < G; i += 2) {      // two columns an instruction
-              const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, d2[i], 1), __shfl_xor_sync(0xffffffffu, d2[i + 1], 1));
-              float2 u = ffma2(make_float2(sign, sign), make_float2(d1[i], d1[i + 1]), o);
-              if (has_state) u = ffma2(make_float2(g, g), make_float2(pv[i], pv[i + 1]), u);
-              d1[i] = u.x;
-              d1[i + 1] = u.y;
-            }
-            if (has_state) {
-              if (OUT && hh == 0) {
-#pragma unroll
-                for (int i = 0; i < G; ++i) pv[i] = __ldcg(prev + 2048 + i * 128);
-              }
-            }
-            if (to_final) {
-              fin.store(p, (int)col * 128 + r, d1, even, ok);
-            } else if (ok) {
-#pragma unroll
-              for (int i = 0; i < G; ++i) next[i * 128] = d1[i];
-              next += 128 * G;
-            }
+          fence_proxy_async();
+          tc_fence_before();
+          __syncthreads();
+          if (warp == 0 && elect_one()) {
+            tc_fence_after();
+            if (OUT && k == 0) mbar_wait(&bars[1], ph_tile, 243);
+            const uint32_t d = tmem + (OUT ? (uint32_t)(k & 1) * 128u : 0u);
+            constexpr uint32_t idesc = idesc_bf16(128, 64, true, true);
+            mma_run(d, smem_desc_sw128(b_r, 16384, 1024), smem_desc_sw128(x_r, 16, 1024), 128, 128, idesc, 8, false);      // D1 = k'^T (w Re v)
+            mma_run(d + 64, smem_desc_sw128(b_r, 16384, 1024), smem_desc_sw128(x_r + 16384, 16, 1024), 128, 128, idesc, 8, false);      // D2 = k'^T (w Im v)
+            mma_commit(&bars[2]);
           }
-          if (!OUT && ok && tid == 0) p.chunk_decay[((size_t)(k - 1) * p.H + s.h) * p.nslots + s.job.slot0 + s.c + 1] = g;
+          __syncwarp();
         }
+        if (OUT && k > 0) sums_out(k - 1);      // (beside this state's products: they go to the other half of the accumulators)
         if (k == K) break;
-        fence_proxy_async();
-        tc_fence_before();
-        __syncthreads();
-        if (warp == 0 && elect_one()) {
-          tc_fence_after();
-          if (OUT && k == 0) mbar_wait(&bars[1], ph_tile, 243);
-          constexpr uint32_t idesc = idesc_bf16(128, 64, true, true);
-          mma_run(tmem, smem_desc_sw128(b_r, 16384, 1024), smem_desc_sw128(x_r, 16, 1024), 128, 128, idesc, 8, false);      // D1 = k'^T (w Re v)
-          mma_run(tmem + 64, smem_desc_sw128(b_r, 16384, 1024), smem_desc_sw128(x_r + 16384, 16, 1024), 128, 128, idesc, 8, false);      // D2 = k'^T (w Im v)
-          mma_commit(&bars[2]);
-        }
-        __syncwarp();
         if (has_state) {
           const float* prev = entering(k) + hf * 4096 + r;
 #pragma unroll
