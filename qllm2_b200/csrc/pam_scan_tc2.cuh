@@ -147,8 +147,9 @@ __device__ __forceinline__ void bw_epi_scores_t(const bool lower, uint32_t tlane
           const float w = STRONG ? scale * __expf(fminf(0.f, lower ? a_r - Acum[c] : Acum[c] - a_r)) : rowf * cfac[c];
           d[e] = on ? w : 0.f;
         }
-        out[j >> 1] = pack_bf162(d[0] * xr[j], d[1] * xr[j + 1]);
-        out[8 + (j >> 1)] = pack_bf162(d[0] * xi[j], d[1] * xi[j + 1]);
+        const float2 w = make_float2(d[0], d[1]), a = fmul2(w, make_float2(xr[j], xr[j + 1])), b = fmul2(w, make_float2(xi[j], xi[j + 1]));
+        out[j >> 1] = pack_bf162(a.x, a.y);
+        out[8 + (j >> 1)] = pack_bf162(b.x, b.y);
       }
     }
     tmem_st16(tlane_slot + c0, out);      // (the loads of these columns have completed)

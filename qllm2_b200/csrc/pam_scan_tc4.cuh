@@ -57,13 +57,14 @@ struct BwdTables {
   float* A;        // [K][128] cumulative log decay
   float* col;      // [K][128] e^{A_m - A_s}                       (strong: 1)
   float* row;      // [K][128] sigma e^{A_t - A_m}, 0 past the end (strong: sigma)
-  float2* w;       // [K][128] conj(c_t) row_t
+  float *wr, *wi;  // [K][128] conj(c_t) row_t
 };
 
-// Pass A for 16 columns of row r: T = G X over the columns of X, sums of col_s D Z over the columns into zs.
+// Pass A for 16 columns of row r: T = G X over the columns of X, sums of col_s D Z over the columns into zs (real and imaginary, even
+// and odd columns apart).
 template <int K, bool STRONG>
 __device__ __forceinline__ void pass_a16(uint32_t tl, int c0, int q4, int r, const BwdTables& tb, uint32_t strong, const float2 (&wk)[K],
-                                         const float (&ar)[K], float2 (&zs)[K]) {
+                                         float2 (&zs)[K][2]) {
   using namespace umma;
   uint32_t out[16];
   if (c0 > q4 * 32 + 31) {                  // warp-uniform: above the diagonal
@@ -74,43 +75,31 @@ __device__ __forceinline__ void pass_a16(uint32_t tl, int c0, int q4, int r, con
     tmem_ld16x4(tl + c0, xr, tl + 128 + c0, xi, tl + 256 + c0, yr, tl + 384 + c0, yi);
     const int last = c0 + 15 <= q4 * 32 ? TC : r;      // no diagonal inside the block: every column counts
 #pragma unroll
-    for (int j4 = 0; j4 < 16; j4 += 4) {
-      float cf[K][4];
+    for (int j = 0; j < 16; j += 2) {          // two columns an instruction
+      const int c1 = c0 + j;
+      const float2 x = make_float2(__uint_as_float(xr[j]), __uint_as_float(xr[j + 1])), y = make_float2(__uint_as_float(xi[j]), __uint_as_float(xi[j + 1]));
+      const float2 u = make_float2(__uint_as_float(yr[j]), __uint_as_float(yr[j + 1])), v = make_float2(__uint_as_float(yi[j]), __uint_as_float(yi[j + 1]));
+      float2 cf[K], gr = make_float2(0.f, 0.f), gi = gr;
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        const float4 v = *reinterpret_cast<const float4*>(tb.col + k * TC + c0 + j4);
-        cf[k][0] = v.x; cf[k][1] = v.y; cf[k][2] = v.z; cf[k][3] = v.w;
-        if (STRONG && ((strong >> k) & 1u)) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) cf[k][e] = __expf(fminf(0.f, ar[k] - tb.A[k * TC + c0 + j4 + e]));
-        }
+        cf[k] = *reinterpret_cast<const float2*>(tb.col + k * TC + c1);
+        if (STRONG && ((strong >> k) & 1u)) cf[k] = make_float2(__expf(fminf(0.f, tb.A[k * TC + r] - tb.A[k * TC + c1])), __expf(fminf(0.f, tb.A[k * TC + r] - tb.A[k * TC + c1 + 1])));
+        gr = ffma2(make_float2(wk[k].x, wk[k].x), cf[k], gr);
+        gi = ffma2(make_float2(wk[k].y, wk[k].y), cf[k], gi);
       }
-      float tr[4], ti[4];
+      const float2 xv = fmul2(x, v);
+      float2 zr = ffma2(x, u, fmul2(y, v)), zi = ffma2(y, u, make_float2(-xv.x, -xv.y));
+      if (c1 > last) gr.x = gi.x = zr.x = zi.x = 0.f;
+      if (c1 + 1 > last) gr.y = gi.y = zr.y = zi.y = 0.f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int j = j4 + e;
-        const bool on = c0 + j <= last;
-        const float a = __uint_as_float(xr[j]), b = __uint_as_float(xi[j]), c = __uint_as_float(yr[j]), d = __uint_as_float(yi[j]);
-        float gr = 0.f, gi = 0.f;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-          gr = fmaf(wk[k].x, cf[k][e], gr);
-          gi = fmaf(wk[k].y, cf[k][e], gi);
-        }
-        float zr = fmaf(a, c, b * d), zi = fmaf(b, c, -(a * d));
-        if (!on) gr = gi = zr = zi = 0.f;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-          zs[k].x = fmaf(cf[k][e], zr, zs[k].x);
-          zs[k].y = fmaf(cf[k][e], zi, zs[k].y);
-        }
-        tr[e] = gr * a - gi * b;
-        ti[e] = gr * b + gi * a;
+      for (int k = 0; k < K; ++k) {
+        zs[k][0] = ffma2(cf[k], zr, zs[k][0]);
+        zs[k][1] = ffma2(cf[k], zi, zs[k][1]);
       }
-      out[j4 >> 1] = pack_bf162(tr[0], tr[1]);
-      out[(j4 >> 1) + 1] = pack_bf162(tr[2], tr[3]);
-      out[8 + (j4 >> 1)] = pack_bf162(ti[0], ti[1]);
-      out[8 + (j4 >> 1) + 1] = pack_bf162(ti[2], ti[3]);
+      const float2 iy = fmul2(gi, y);
+      const float2 tr = ffma2(gr, x, make_float2(-iy.x, -iy.y)), ti = ffma2(gr, y, fmul2(gi, x));
+      out[j >> 1] = pack_bf162(tr.x, tr.y);
+      out[8 + (j >> 1)] = pack_bf162(ti.x, ti.y);
     }
   }
   tmem_st16(tl + c0, out);
@@ -120,7 +109,7 @@ __device__ __forceinline__ void pass_a16(uint32_t tl, int c0, int q4, int r, con
 // of sigma e^{A_t - A_m} Re(conj(c) Z) into cs.
 template <int K, bool STRONG>
 __device__ __forceinline__ void pass_b16(uint32_t tl, int c0, int q4, int r, const BwdTables& tb, uint32_t strong, const float (&ck)[K],
-                                         const float (&ar)[K], float (&cs)[K]) {
+                                         float2 (&cs)[K]) {
   using namespace umma;
   uint32_t ox[16], oy[16];
   if (c0 + 15 < q4 * 32) {
@@ -131,45 +120,36 @@ __device__ __forceinline__ void pass_b16(uint32_t tl, int c0, int q4, int r, con
     tmem_ld16x4(tl + c0, xr, tl + 128 + c0, xi, tl + 256 + c0, yr, tl + 384 + c0, yi);
     const int first = c0 >= q4 * 32 + 31 ? 0 : r;
 #pragma unroll
-    for (int j2 = 0; j2 < 16; j2 += 2) {
-      float2 w[K][2];
+    for (int j = 0; j < 16; j += 2) {          // two columns an instruction
+      const int c1 = c0 + j;
+      const float2 x = make_float2(__uint_as_float(xr[j]), __uint_as_float(xr[j + 1])), y = make_float2(__uint_as_float(xi[j]), __uint_as_float(xi[j + 1]));
+      const float2 u = make_float2(__uint_as_float(yr[j]), __uint_as_float(yr[j + 1])), v = make_float2(__uint_as_float(yi[j]), __uint_as_float(yi[j + 1]));
+      float2 wr[K], wi[K], gr = make_float2(0.f, 0.f), gi = gr;
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        const float4 v = *reinterpret_cast<const float4*>(tb.w + k * TC + c0 + j2);
-        w[k][0] = make_float2(v.x, v.y);
-        w[k][1] = make_float2(v.z, v.w);
+        wr[k] = *reinterpret_cast<const float2*>(tb.wr + k * TC + c1);
+        wi[k] = *reinterpret_cast<const float2*>(tb.wi + k * TC + c1);
         if (STRONG && ((strong >> k) & 1u)) {
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float f = __expf(fminf(0.f, tb.A[k * TC + c0 + j2 + e] - ar[k]));
-            w[k][e].x *= f;
-            w[k][e].y *= f;
-          }
+          const float2 f = make_float2(__expf(fminf(0.f, tb.A[k * TC + c1] - tb.A[k * TC + r])), __expf(fminf(0.f, tb.A[k * TC + c1 + 1] - tb.A[k * TC + r])));
+          wr[k] = fmul2(wr[k], f);
+          wi[k] = fmul2(wi[k], f);
         }
+        gr = ffma2(wr[k], make_float2(ck[k], ck[k]), gr);
+        gi = ffma2(wi[k], make_float2(ck[k], ck[k]), gi);
       }
-      float xo[2], xp[2], yo[2], yp[2];
+      const float2 xv = fmul2(x, v);
+      float2 zr = ffma2(x, u, fmul2(y, v)), zn = ffma2(y, u, make_float2(-xv.x, -xv.y));      // conj(X^H) Y^H: the real part, the imaginary part negated
+      if (c1 < first) gr.x = gi.x = zr.x = zn.x = 0.f;
+      if (c1 + 1 < first) gr.y = gi.y = zr.y = zn.y = 0.f;
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int j = j2 + e;
-        const bool on = c0 + j >= first;
-        const float a = __uint_as_float(xr[j]), b = __uint_as_float(xi[j]), c = __uint_as_float(yr[j]), d = __uint_as_float(yi[j]);
-        float gr = 0.f, gi = 0.f;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-          gr = fmaf(w[k][e].x, ck[k], gr);
-          gi = fmaf(w[k][e].y, ck[k], gi);
-        }
-        float zr = fmaf(a, c, b * d), zi = fmaf(a, d, -(b * c));      // conj(X^H) Y^H
-        if (!on) gr = gi = zr = zi = 0.f;
-#pragma unroll
-        for (int k = 0; k < K; ++k) cs[k] = fmaf(w[k][e].x, zr, fmaf(-w[k][e].y, zi, cs[k]));
-        xo[e] = gr * a + gi * b; xp[e] = gr * b - gi * a;
-        yo[e] = gr * c - gi * d; yp[e] = gr * d + gi * c;
-      }
-      ox[j2 >> 1] = pack_bf162(xo[0], xo[1]);
-      ox[8 + (j2 >> 1)] = pack_bf162(xp[0], xp[1]);
-      oy[j2 >> 1] = pack_bf162(yo[0], yo[1]);
-      oy[8 + (j2 >> 1)] = pack_bf162(yp[0], yp[1]);
+      for (int k = 0; k < K; ++k) cs[k] = ffma2(wr[k], zr, ffma2(wi[k], zn, cs[k]));
+      const float2 ix = fmul2(gi, x), iv = fmul2(gi, v);
+      const float2 xo = ffma2(gr, x, fmul2(gi, y)), xp = ffma2(gr, y, make_float2(-ix.x, -ix.y));
+      const float2 yo = ffma2(gr, u, make_float2(-iv.x, -iv.y)), yp = ffma2(gr, v, fmul2(gi, u));
+      ox[j >> 1] = pack_bf162(xo.x, xo.y);
+      ox[8 + (j >> 1)] = pack_bf162(xp.x, xp.y);
+      oy[j >> 1] = pack_bf162(yo.x, yo.y);
+      oy[8 + (j >> 1)] = pack_bf162(yp.x, yp.y);
     }
   }
   tmem_st16(tl + c0, ox);
@@ -239,8 +219,9 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   BwdTables tb;
   tb.A = reinterpret_cast<float*>(SL + 4 * 16384);
   tb.col = tb.A + KMAX * TC;
-  tb.w = reinterpret_cast<float2*>(tb.col + KMAX * TC);
-  tb.row = reinterpret_cast<float*>(tb.w + KMAX * TC);
+  tb.wr = tb.col + KMAX * TC;
+  tb.wi = tb.wr + KMAX * TC;
+  tb.row = tb.wi + KMAX * TC;
   float2* dcp = reinterpret_cast<float2*>(tb.row + KMAX * TC);      // [4 channel groups][K][128] shares of dc
   float* kdp = reinterpret_cast<float*>(SL + 2 * 16384);            // [4][K][128] shares of Re<k, dk>, once no MMA reads the slots
   uint64_t* bars = reinterpret_cast<uint64_t*>(dcp + 4 * KMAX * TC);
@@ -319,7 +300,8 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
     const float rf = et < len ? p.q_scale * (st ? 1.f : __expf(a - a_mid)) : 0.f;
     tb.col[ek * TC + et] = st ? 1.f : __expf(a_mid - a);
     tb.row[ek * TC + et] = rf;
-    tb.w[ek * TC + et] = make_float2(c_e.x * rf, -c_e.y * rf);
+    tb.wr[ek * TC + et] = c_e.x * rf;
+    tb.wi[ek * TC + et] = -c_e.y * rf;
   }
   const uint32_t q_r = smem_u32(TQ), k_r = smem_u32(TK), v_r = smem_u32(TV), y_r = smem_u32(TY), sl = smem_u32(SL);
   const bool issuer = warp == 0 && elect_one();
@@ -372,29 +354,28 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
   const uint32_t tl = tmem + ((uint32_t)(q4 * 32) << 16);
   const bool valid = r < len;
   const size_t obase = token_base(p, L.b, h, L.t0 + r, TD);
-  float ar[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) ar[k] = tb.A[k * TC + r];
 
   if (tid == 0 && has_ds) {      // (a hint: the reverse carry may still be writing them)
 #pragma unroll
     for (int k = 0; k < K; ++k) bulk_prefetch_l2(p.dstates + state_base(p, k, h, L.slot0 + L.c + 1, TD), 32768);
   }
   // ---- pass A: rows t
-  float2 wk[K], zs[K];
+  float2 wk[K], zp[K][2], zs[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    wk[k] = tb.w[k * TC + r];
-    zs[k] = make_float2(0.f, 0.f);
+    wk[k] = make_float2(tb.wr[k * TC + r], tb.wi[k * TC + r]);
+    zp[k][0] = zp[k][1] = make_float2(0.f, 0.f);
   }
   ok = mbar_wait(&bars[B_SA], 0, 253) && ok;
   tc_fence_after();
 #pragma unroll 1
   for (int hh = 0; hh < 2; ++hh) {
     const int c0 = cq * 32 + hh * 16;
-    if (strong == 0u) pass_a16<K, false>(tl, c0, q4, r, tb, 0u, wk, ar, zs);
-    else pass_a16<K, true>(tl, c0, q4, r, tb, strong, wk, ar, zs);
+    if (strong == 0u) pass_a16<K, false>(tl, c0, q4, r, tb, 0u, wk, zp);
+    else pass_a16<K, true>(tl, c0, q4, r, tb, strong, wk, zp);
   }
+#pragma unroll
+  for (int k = 0; k < K; ++k) zs[k] = make_float2(zp[k][0].x + zp[k][0].y, zp[k][1].x + zp[k][1].y);
   tmem_st_wait();
   fence_proxy_async();
   tc_fence_before();
@@ -439,18 +420,22 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
         float ur[16], ui[16], xr[16], xi[16];
         tmem_ld16x2(at, ur, at + 64, ui);
         row16(TQ, r, cq, xr, xi);
-        const float f = __expf(((strong >> k) & 1u) ? ar[k] : tb.A[k * TC + TC / 2 - 1]);      // row_t f = sigma e^{A_t}
+        const float f = __expf(((strong >> k) & 1u) ? tb.A[k * TC + r] : tb.A[k * TC + TC / 2 - 1]);      // row_t f = sigma e^{A_t}
         const float wr = wk[k].x * f, wi = wk[k].y * f;
-        float er = 0.f, ei = 0.f;
+        float2 er = make_float2(0.f, 0.f), ei = er, en = er;      // (two channels an instruction; ei - en is the imaginary part)
+        const float2 wr2 = make_float2(wr, wr), wi2 = make_float2(wi, wi), wn2 = make_float2(-wi, -wi);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          er = fmaf(xr[j], ur[j], fmaf(xi[j], ui[j], er));
-          ei = fmaf(xr[j], ui[j], fmaf(-xi[j], ur[j], ei));
-          vr[j] += wr * ur[j] - wi * ui[j];
-          vi[j] += wr * ui[j] + wi * ur[j];
+        for (int j = 0; j < 16; j += 2) {
+          const float2 a = make_float2(ur[j], ur[j + 1]), b = make_float2(ui[j], ui[j + 1]), c = make_float2(xr[j], xr[j + 1]), d = make_float2(xi[j], xi[j + 1]);
+          er = ffma2(c, a, ffma2(d, b, er));
+          ei = ffma2(c, b, ei);
+          en = ffma2(d, a, en);
+          const float2 o = ffma2(wr2, a, ffma2(wn2, b, make_float2(vr[j], vr[j + 1]))), p2 = ffma2(wr2, b, ffma2(wi2, a, make_float2(vi[j], vi[j + 1])));
+          vr[j] = o.x; vr[j + 1] = o.y;
+          vi[j] = p2.x; vi[j + 1] = p2.y;
         }
-        zs[k].x = fmaf(f, er, zs[k].x);
-        zs[k].y = fmaf(f, ei, zs[k].y);
+        zs[k].x = fmaf(f, er.x + er.y, zs[k].x);
+        zs[k].y = fmaf(f, (ei.x - en.x) + (ei.y - en.y), zs[k].y);
       }
     }
 #pragma unroll
@@ -503,18 +488,19 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
 
   // ---- pass B: rows s
   float ck[K], cs[K];
+  float2 cp[K];                             // even and odd columns apart
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     ck[k] = tb.col[k * TC + r];
-    cs[k] = 0.f;
+    cp[k] = make_float2(0.f, 0.f);
   }
   ok = mbar_wait(&bars[B_SB], 0, 256) && ok;
   tc_fence_after();
 #pragma unroll 1
   for (int hh = 0; hh < 2; ++hh) {
     const int c0 = cq * 32 + hh * 16;
-    if (strong == 0u) pass_b16<K, false>(tl, c0, q4, r, tb, 0u, ck, ar, cs);
-    else pass_b16<K, true>(tl, c0, q4, r, tb, strong, ck, ar, cs);
+    if (strong == 0u) pass_b16<K, false>(tl, c0, q4, r, tb, 0u, ck, cp);
+    else pass_b16<K, true>(tl, c0, q4, r, tb, strong, ck, cp);
   }
   tmem_st_wait();
   fence_proxy_async();
@@ -539,7 +525,7 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
     tmem_ld16x2(tl + 128 + 16 * cq, kr, tl + 192 + 16 * cq, ki);
     tmem_ld16x2(tl + 384 + 16 * cq, vr, tl + 448 + 16 * cq, vi);
 #pragma unroll
-    for (int k = 0; k < K; ++k) cs[k] *= ck[k];
+    for (int k = 0; k < K; ++k) cs[k] = (cp[k].x + cp[k].y) * ck[k];
     if (has_ds) {
       // a state's products run while the one before it is read: state k + 1 is issued once every warp has read what holds its
       // columns (dk and dv for state 1, state k - 1 after that)
@@ -560,26 +546,30 @@ __global__ void __launch_bounds__(BT, 1) k_tc_scan_bwdK(const __grid_constant__ 
         ok = mbar_wait(&bars[B_C0 + k], 0, 258) && ok;
         tc_fence_after();
         const uint32_t at = tl + 128 * (k & 1) + 16 * cq;
-        const float e = __expf(fminf(0.f, tb.A[k * TC + TC - 1] - ar[k]));
+        const float e = __expf(fminf(0.f, tb.A[k * TC + TC - 1] - tb.A[k * TC + r]));
         float ur[16], ui[16];
         {
           float xr[16], xi[16];
           tmem_ld16x2(at, ur, at + 64, ui);
           row16(TK, r, cq, xr, xi);
-          float d = 0.f;
+          float2 d = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            d = fmaf(xr[j], ur[j], fmaf(xi[j], ui[j], d));
-            kr[j] = fmaf(e, ur[j], kr[j]);
-            ki[j] = fmaf(e, ui[j], ki[j]);
+          for (int j = 0; j < 16; j += 2) {
+            const float2 a = make_float2(ur[j], ur[j + 1]), b = make_float2(ui[j], ui[j + 1]);
+            d = ffma2(make_float2(xr[j], xr[j + 1]), a, ffma2(make_float2(xi[j], xi[j + 1]), b, d));
+            const float2 o = ffma2(make_float2(e, e), a, make_float2(kr[j], kr[j + 1])), p2 = ffma2(make_float2(e, e), b, make_float2(ki[j], ki[j + 1]));
+            kr[j] = o.x; kr[j + 1] = o.y;
+            ki[j] = p2.x; ki[j + 1] = p2.y;
           }
-          cs[k] = fmaf(e, d, cs[k]);
+          cs[k] = fmaf(e, d.x + d.y, cs[k]);
         }
         tmem_ld16x2(at + 256, ur, at + 320, ui);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          vr[j] = fmaf(e, ur[j], vr[j]);
-          vi[j] = fmaf(e, ui[j], vi[j]);
+        for (int j = 0; j < 16; j += 2) {
+          const float2 o = ffma2(make_float2(e, e), make_float2(ur[j], ur[j + 1]), make_float2(vr[j], vr[j + 1]));
+          const float2 p2 = ffma2(make_float2(e, e), make_float2(ui[j], ui[j + 1]), make_float2(vi[j], vi[j + 1]));
+          vr[j] = o.x; vr[j + 1] = o.y;
+          vi[j] = p2.x; vi[j + 1] = p2.y;
         }
       }
     }
