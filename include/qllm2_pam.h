@@ -363,6 +363,19 @@ struct qpam_front_bwd_args {
 };
 int qpam_pam_front_fwd(const qpam_front_args* args, void* stream);
 
+/* qpam_pam_front_fwd and qpam_decode_step of one token each in one launch (bf16 tensors and pool, d = 64): q, k, v, the decays and
+ * the read-out weights are formed where they are used (f.q, f.k, f.v, f.gamma, f.coef, f.B, f.T are not looked at; the rows of f.qkv
+ * are the n sequences).  A gate whose pointer in f is NULL may be a projection of mag [n,D] instead: mag_row[i] is its first row
+ * in w_mag [rows,D] (i = 0 dt, 1 pg, 2 phase, 3 score; rows as the columns of the gate), -1: it is not. */
+typedef struct qpam_decode_front_args {
+  qpam_front_args f;
+  const void *mag, *w_mag, *b_mag;
+  int32_t mag_row[4];
+  int32_t D;
+} qpam_decode_front_args;
+int qpam_decode_front(void* state_pool, int64_t n_slots, int32_t L, int32_t layer, const int32_t* slot_ids,
+                      const qpam_decode_front_args* args, void* y, int32_t n, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Training-step fusions of a block (bf16 activations, fp32 parameters): the element-wise work of
  * V11Block.forward (v11/model.py:1021-1049) and its backward around the library GEMMs and the scan.

@@ -53,6 +53,10 @@ class FrontArgs(C.Structure):
     ]
 
 
+class DecodeFrontArgs(C.Structure):
+    _fields_ = [("f", FrontArgs), ("mag", c_void_p), ("w_mag", c_void_p), ("b_mag", c_void_p), ("mag_row", c_int32 * 4), ("D", c_int32)]
+
+
 class StepLayer(C.Structure):
     _fields_ = [(n, c_void_p) for n in ("w_gu", "w_down", "w_front", "b_front", "w_mag", "b_mag", "w_o", "n1", "n2", "act_bias", "act_beta",
                                         "cgu_scale", "pam_scale", "dt_bias", "dt_off")] + \
@@ -125,6 +129,7 @@ SIGNATURES = {
     "qpam_residual_cnorm_fwd": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int64,
                                           c_int32, C.c_float, c_void_p]),
     "qpam_pam_front_fwd": (c_int32, [C.POINTER(FrontArgs), c_void_p]),
+    "qpam_decode_front": (c_int32, [c_void_p, c_int64, c_int32, c_int32, c_void_p, C.POINTER(DecodeFrontArgs), c_void_p, c_int32, c_void_p]),
     "qpam_pack_block": (c_int32, [c_void_p, c_int32, c_void_p]),
     "qpam_unpack_block": (c_int32, [c_void_p, c_int32, c_void_p]),
     "qpam_colsum": (c_int32, [c_void_p, c_int32, c_void_p]),

@@ -7,6 +7,7 @@
 // shuffles.  Continuous batching: `slot_ids` picks the slot of every live sequence, so sequences
 // join and leave by editing that index vector only.
 #include "common.cuh"
+#include "elementwise.cuh"
 #include "umma.cuh"
 
 namespace qpam {
@@ -148,11 +149,94 @@ __device__ __forceinline__ void bulk_store(void* gdst, const void* smem_src, uin
 
 constexpr int DEC_BULK_STATE_BYTES = 64 * 64 * 2 * 2;  // one bf16 state
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_decode_step_bulk(DecodeParams p) {
+// q, k, v, decay and read-out weights of one token and head, from the outputs of the layer's input projections: what k_pam_front
+// writes for the whole batch, formed here by the CTA that uses it while its states are on their way.  The gates that read |x| (one
+// to ten rows of D for a head) are products of this CTA too, a warp each.  Two launches less a layer where there are such gates, one
+// where not: a step of the 12-layer model with three states, 128 / 48 / 20 sequences: 1010 -> 966, 773 -> 716, 688 -> 629 us; with one
+// state, 256 / 20: 938 -> 939, 598 -> 581 (256: bound by the states, and k_pam_front ran beside their first loads).
+struct FrontOut {
+  float2 q[64], k[64], v[64];
+  float gate[2 + 2 * QPAM_MAX_STATES];      // dt | protect | phases | scores
+  float gamma[QPAM_MAX_STATES];
+  float2 coef[QPAM_MAX_STATES];
+};
+__device__ __forceinline__ void decode_front(const qpam_decode_front_args& a, int seq, int h, FrontOut& o) {
+  typedef __nv_bfloat16 bf16;
+  const qpam_front_args& f = a.f;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K = f.K;
+  float2 x[3], rot = make_float2(1.f, 0.f);
+  if (tid < 64) {
+    const bf16* src = reinterpret_cast<const bf16*>(f.qkv) + (int64_t)seq * f.ld_qkv + (h * 64 + tid) * 2;
+#pragma unroll
+    for (int w = 0; w < 3; ++w) x[w] = IO<bf16>::ld2(src + (int64_t)w * f.H * 128);
+    if (f.rope) {
+      int64_t pos = f.positions ? f.positions[seq] : f.offset;
+      pos = pos < 0 ? 0 : (pos >= f.rope_len ? f.rope_len - 1 : pos);
+      rot = *reinterpret_cast<const float2*>(f.rope + (pos * 64 + tid) * 2);
+    }
+  } else {
+    for (int i = warp - 2; i < 2 + 2 * K; i += 6) {
+      const int what = i < 2 ? i : i < 2 + K ? 2 : 3, at = what < 2 ? h : h * K + (i - 2) % K;
+      const void* raw = what == 0 ? f.dt : what == 1 ? f.pg : what == 2 ? f.phase : f.score;
+      const int64_t ld = what == 0 ? f.ld_dt : what == 1 ? f.ld_pg : what == 2 ? f.ld_phase : f.ld_score;
+      float v = 0.f;
+      if (raw) {
+        v = __bfloat162float(reinterpret_cast<const bf16*>(raw)[seq * ld + at]);
+      } else if (a.mag_row[what] >= 0) {
+        const int row = a.mag_row[what] + at;
+        const uint4* m = reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(a.mag) + (int64_t)seq * a.D);
+        const uint4* w = reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(a.w_mag) + (int64_t)row * a.D);
+        for (int g = lane; g < a.D / 8; g += 32) {
+          const uint4 p = m[g], r = w[g];
+          const uint32_t pw[4] = {p.x, p.y, p.z, p.w}, rw[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            v = fmaf(__uint_as_float(pw[e] << 16), __uint_as_float(rw[e] << 16), v);
+            v = fmaf(__uint_as_float(pw[e] & 0xffff0000u), __uint_as_float(rw[e] & 0xffff0000u), v);
+          }
+        }
+        v = ew::warp_sum(v) + __bfloat162float(reinterpret_cast<const bf16*>(a.b_mag)[row]);
+        v = __bfloat162float(__float2bfloat16_rn(v));
+      }
+      if (lane == 0) o.gate[i] = v;
+    }
+  }
+  __syncthreads();
+  const bool has_pg = f.pg != nullptr || a.mag_row[1] >= 0, has_phase = f.phase != nullptr || a.mag_row[2] >= 0, has_score = f.score != nullptr || a.mag_row[3] >= 0;
+  const float prot = has_pg ? ew::sigmoidf_(o.gate[1]) : 0.f;
+  if (tid < 64) {
+    auto store = [&](float2& at, float re, float im) { at = __bfloat1622float2(__floats2bfloat162_rn(re, im)); };      // (as they are stored otherwise)
+    store(o.q[tid], (x[0].x * rot.x - x[0].y * rot.y) * f.q_scale, (x[0].x * rot.y + x[0].y * rot.x) * f.q_scale);
+    store(o.k[tid], x[1].x * rot.x - x[1].y * rot.y, x[1].x * rot.y + x[1].y * rot.x);
+    const float keep = 1.f - prot;
+    store(o.v[tid], x[2].x * keep, x[2].y * keep);
+  } else if (tid < 64 + K) {
+    const int k = tid - 64;
+    float base = ew::sigmoidf_(-(o.gate[0] + f.dt_bias[h] + (f.state_dt_offset ? f.state_dt_offset[k] : 0.f)));      // exp(-softplus(x))
+    if (f.gamma_floor > 0.f) base = f.gamma_floor + (1.f - f.gamma_floor) * base;
+    o.gamma[k] = base * (1.f - prot) + prot;
+    float w = 1.f, sn = 0.f, cs = 1.f;
+    if (K > 1) {
+      if (has_score) {
+        const float* s = o.gate + 2 + K;
+        float top = -INFINITY, sum = 0.f;
+        for (int i = 0; i < K; ++i) top = fmaxf(top, s[i]);
+        for (int i = 0; i < K; ++i) sum += __expf(s[i] - top);
+        w = __expf(s[k] - top) / sum * (float)K;
+      }
+      if (has_phase) sincosf(o.gate[2 + k], &sn, &cs);
+    }
+    o.coef[k] = make_float2(w * cs, w * sn);
+  }
+  __syncthreads();
+}
+
+// FRONT: q, k, v, gamma and coef come from `decode_front` instead of memory.
+template <typename T, bool FRONT>
+__global__ void __launch_bounds__(256) k_decode_step_bulk(DecodeParams p, const __grid_constant__ qpam_decode_front_args front) {
   constexpr int D = 64, NC = 4, LPR = D / NC, RPP = 256 / LPR, PASSES = D / RPP;
   extern __shared__ __align__(128) unsigned char dec_smem[];
-  __shared__ float2 sq[D], sk[D], sv[D];
+  __shared__ FrontOut in;
   __shared__ __align__(8) uint64_t bar[QPAM_MAX_STATES];   // one per state: work on state k starts when it has landed
   const int tid = threadIdx.x;
   const int seq = blockIdx.x / p.H, h = blockIdx.x - seq * p.H;
@@ -182,19 +266,23 @@ __global__ void __launch_bounds__(256) k_decode_step_bulk(DecodeParams p) {
                 DEC_BULK_STATE_BYTES, &bar[k]);
     }
   }
-  if (tid < D) {
-    sq[tid] = IO<T>::ld2(reinterpret_cast<const T*>(p.q) + vb + 2 * tid);
-    sk[tid] = IO<T>::ld2(reinterpret_cast<const T*>(p.k) + vb + 2 * tid);
-    sv[tid] = IO<T>::ld2(reinterpret_cast<const T*>(p.v) + vb + 2 * tid);
+  if constexpr (FRONT) {
+    decode_front(front, seq, h, in);
+  } else {
+    if (tid < D) {
+      in.q[tid] = IO<T>::ld2(reinterpret_cast<const T*>(p.q) + vb + 2 * tid);
+      in.k[tid] = IO<T>::ld2(reinterpret_cast<const T*>(p.k) + vb + 2 * tid);
+      in.v[tid] = IO<T>::ld2(reinterpret_cast<const T*>(p.v) + vb + 2 * tid);
+    }
+    __syncthreads();  // (here as in decode_front: it also publishes the barriers' initialisation to the waiters)
   }
-  __syncthreads();  // also publishes the barriers' initialisation to the waiters
   bool arrived = true;
   const int row0 = tid / LPR, j0 = (tid % LPR) * NC;
   float2 kq[NC], qq[NC], yacc[PASSES];
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
-    kq[c] = sk[j0 + c];
-    qq[c] = sq[j0 + c];
+    kq[c] = in.k[j0 + c];
+    qq[c] = in.q[j0 + c];
   }
 #pragma unroll
   for (int r = 0; r < PASSES; ++r) yacc[r] = make_float2(0.f, 0.f);
@@ -204,9 +292,10 @@ __global__ void __launch_bounds__(256) k_decode_step_bulk(DecodeParams p) {
       arrived = umma::mbar_wait(&bar[k], 0, 31) && arrived;
       __nv_bfloat16* S = reinterpret_cast<__nv_bfloat16*>(dec_smem + (size_t)k * DEC_BULK_STATE_BYTES);
       const size_t gi = ((size_t)k * p.n + seq) * p.H + h;
-      const float g = p.gamma[gi];
+      const float g = FRONT ? in.gamma[k] : p.gamma[gi];
       float2 cf = make_float2(1.f, 0.f);
-      if (p.coef != nullptr) cf = *reinterpret_cast<const float2*>(p.coef + gi * 2);
+      if (FRONT) cf = in.coef[k];
+      else if (p.coef != nullptr) cf = *reinterpret_cast<const float2*>(p.coef + gi * 2);
 #pragma unroll
       for (int r = 0; r < PASSES; ++r) {
         if (!arrived) break;
@@ -214,7 +303,7 @@ __global__ void __launch_bounds__(256) k_decode_step_bulk(DecodeParams p) {
         uint4* cell = reinterpret_cast<uint4*>(S + ((size_t)row * D + j0) * 2);
         uint4 raw = *cell;
         __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&raw);
-        const float2 vi = sv[row];
+        const float2 vi = in.v[row];
         float2 part = make_float2(0.f, 0.f);
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
@@ -252,13 +341,13 @@ __global__ void __launch_bounds__(256) k_decode_step_bulk(DecodeParams p) {
   }
 }
 
-template <typename T>
-static int launch_decode_bulk(const DecodeParams& p, cudaStream_t st) {
+template <typename T, bool FRONT = false>
+static int launch_decode_bulk(const DecodeParams& p, cudaStream_t st, const qpam_decode_front_args& front = {}) {
   const size_t smem = (size_t)p.K * DEC_BULK_STATE_BYTES;
-  auto kern = k_decode_step_bulk<T>;
+  auto kern = k_decode_step_bulk<T, FRONT>;
   const int rc = allow_smem(reinterpret_cast<const void*>(kern), smem);
   if (rc) return rc;
-  launch_after(kern, p.n * p.H, 256, smem, st, p);
+  launch_after(kern, p.n * p.H, 256, smem, st, p, front);
   QPAM_LAUNCH_CHECK("k_decode_step_bulk");
   return QPAM_OK;
 }
@@ -319,6 +408,25 @@ extern "C" int qpam_decode_step(void* state_pool, int32_t state_dtype, int64_t n
   if (d == 32) { QPAM_DEC(32) }
   QPAM_DEC(64)
 #undef QPAM_DEC
+}
+
+extern "C" int qpam_decode_front(void* state_pool, int64_t n_slots, int32_t L, int32_t layer, const int32_t* slot_ids,
+                                 const qpam_decode_front_args* a, void* y, int32_t n, void* stream) {
+  QPAM_REQUIRE(state_pool && slot_ids && a && y && a->f.qkv && a->f.dt_bias, "decode front: NULL pointer argument");
+  const qpam_front_args& f = a->f;
+  QPAM_REQUIRE(f.d == 64 && f.io_dtype == QPAM_BF16, "decode front: offered for bf16 and head dim 64");
+  QPAM_REQUIRE(f.K >= 1 && f.K <= QPAM_MAX_STATES && f.H >= 1, "decode front: bad H/K = %d/%d", f.H, f.K);
+  QPAM_REQUIRE(n >= 0 && L >= 1 && layer >= 0 && layer < L, "decode front: bad n/L/layer");
+  QPAM_REQUIRE(((uintptr_t)state_pool & 15) == 0 && (((uintptr_t)f.qkv | (uintptr_t)y) & 3) == 0 && f.ld_qkv % 2 == 0, "decode front: unaligned pointer");
+  QPAM_REQUIRE(f.dt != nullptr || a->mag_row[0] >= 0, "decode front: no decay projection");
+  QPAM_REQUIRE(!f.rope || f.rope_len > 0, "decode front: empty rotary table");
+  bool from_mag = false;
+  for (int i = 0; i < 4; ++i) from_mag = from_mag || a->mag_row[i] >= 0;
+  QPAM_REQUIRE(!from_mag || (a->mag && a->w_mag && a->b_mag && a->D >= 8 && a->D % 8 == 0 && (((uintptr_t)a->mag | (uintptr_t)a->w_mag) & 15) == 0),
+               "decode front: gates of |x| need mag, w_mag (16-byte aligned rows) and b_mag");
+  if (n == 0) return QPAM_OK;
+  const DecodeParams p{state_pool, slot_ids, nullptr, nullptr, nullptr, nullptr, nullptr, y, n_slots, L, layer, n, f.H, f.K};
+  return launch_decode_bulk<__nv_bfloat16, true>(p, reinterpret_cast<cudaStream_t>(stream), *a);
 }
 
 extern "C" int qpam_pool_store(void* state_pool, int32_t state_dtype, int64_t n_slots, int32_t L,

@@ -155,21 +155,14 @@ class FusedForward:
                                                  dtype_code(z.dtype), N, self.D, 1e-6, stream_ptr()), "qpam_residual_cnorm_fwd")
         return xn, mag
 
-    def _front(self, L, raw, rawm, B, T, positions, offset, q_scale):
-        H, d, K = self.H, self.d, self.K
-        dev, dt = raw.device, raw.dtype
-        q, k, v = (torch.empty(B, H, T, d, 2, dtype=dt, device=dev) for _ in range(3))
-        gamma = torch.empty(K, B, H, T, dtype=torch.float32, device=dev)
-        coef = torch.empty(K, B, H, T, 2, dtype=torch.float32, device=dev) if K > 1 else None
-        a = _lib.FrontArgs()
+    def _front_args(self, a, L, raw, rawm, positions, offset, q_scale):
+        """The operands of the gate / head-split kernels: raw, rawm are the outputs of w_front and w_mag (rawm None: not formed)."""
         es = raw.element_size()
 
         def col(name):
-            if name not in L.cols:
-                return None, 0
-            src, off = L.cols[name]
-            base = raw if src == "a" else rawm
-            return base.data_ptr() + off * es, base.shape[1]
+            src, off = L.cols.get(name, ("", 0))
+            base = raw if src == "a" else rawm if src == "m" else None
+            return (None, 0) if base is None else (base.data_ptr() + off * es, base.shape[1])
 
         a.qkv, a.ld_qkv = raw.data_ptr(), raw.shape[1]
         a.dt, a.ld_dt = col("dt")
@@ -179,18 +172,49 @@ class FusedForward:
         a.dt_bias, a.state_dt_offset = ptr(L.dt_bias), ptr(L.dt_off)
         a.rope, a.rope_len = ptr(self.rope), 0 if self.rope is None else self.rope.shape[0]
         a.positions, a.offset = ptr(positions), int(offset)
-        a.q, a.k, a.v, a.gamma, a.coef = ptr(q), ptr(k), ptr(v), ptr(gamma), ptr(coef)
         a.gamma_floor, a.q_scale = L.gamma_floor, float(q_scale)
-        a.B, a.T, a.H, a.d, a.K, a.io_dtype = B, T, H, d, K, dtype_code(dt)
+        a.H, a.d, a.K, a.io_dtype = self.H, self.d, self.K, dtype_code(raw.dtype)
+
+    def _front(self, L, raw, rawm, B, T, positions, offset, q_scale):
+        H, d, K = self.H, self.d, self.K
+        dev, dt = raw.device, raw.dtype
+        q, k, v = (torch.empty(B, H, T, d, 2, dtype=dt, device=dev) for _ in range(3))
+        gamma = torch.empty(K, B, H, T, dtype=torch.float32, device=dev)
+        coef = torch.empty(K, B, H, T, 2, dtype=torch.float32, device=dev) if K > 1 else None
+        a = _lib.FrontArgs()
+        self._front_args(a, L, raw, rawm, positions, offset, q_scale)
+        a.q, a.k, a.v, a.gamma, a.coef = ptr(q), ptr(k), ptr(v), ptr(gamma), ptr(coef)
+        a.B, a.T = B, T
         check(_lib.lib().qpam_pam_front_fwd(a, stream_ptr()), "qpam_pam_front_fwd")
         return q, k, v, gamma, coef
+
+    def _decodes_in_place(self, mix, T) -> bool:
+        """Whether one launch forms q, k, v and the gates of a token and does the recurrent step on the pool of `mix`."""
+        pool = getattr(mix, "pool", None)
+        return (T == 1 and pool is not None and self.dtype == pool.dtype == torch.bfloat16 and self.d == 64 and self.D % 8 == 0 and
+                pool.is_contiguous() and pool.data_ptr() % 16 == 0 and tuple(pool.shape[1:]) == (len(self.layers), self.K, self.H, 64, 64, 2))
+
+    def _decode(self, li, L, raw, mag, positions, offset, mix):
+        n = raw.shape[0]
+        if mix.slots.dtype != torch.int32 or mix.slots.numel() != n or mix.slots.device != raw.device:
+            raise _lib.QPamError("decode: int32 slot ids, one per sequence, expected")
+        slots = mix.slots.contiguous()
+        a = _lib.DecodeFrontArgs()
+        self._front_args(a.f, L, raw, None, positions, offset, mix.q_scale)
+        a.mag_row[:] = [L.cols[name][1] if L.cols.get(name, "?")[0] == "m" else -1 for name in ("dt", "pg", "phase", "score")]
+        a.mag, a.w_mag, a.b_mag, a.D = ptr(mag), ptr(L.w_mag), ptr(L.b_mag), self.D
+        y = torch.empty(n, self.inner * 2, dtype=raw.dtype, device=raw.device)
+        check(_lib.lib().qpam_decode_front(mix.pool.data_ptr(), mix.pool.shape[0], mix.pool.shape[1], li, ptr(slots), a, ptr(y), n, stream_ptr()),
+              "qpam_decode_front")
+        return y
 
     # ---------------------------------------------------------------------------------- forward
     @torch.no_grad()
     def hidden(self, ids: torch.Tensor, mix, positions: Optional[torch.Tensor] = None, offset: int = 0):
         """Run the blocks over ids [B, T]; `mix(layer, q, k, v, gamma, coef) -> y [B*T, inner*2]` is the
-        sequence-mixing step (a scan at prefill, the recurrent step at decode).  Returns the final
-        residual stream normalised by output_norm, [B*T, D, 2]."""
+        sequence-mixing step (a scan at prefill, the recurrent step at decode; a mix with a `pool` and `slots` is the
+        latter, and may be done in one launch with what it takes).  Returns the final residual stream normalised by
+        output_norm, [B*T, D, 2]."""
         m, D = self.model, self.D
         B, T = ids.shape
         N = B * T
@@ -202,6 +226,7 @@ class FusedForward:
         z, _ = self._res_norm(z, None, None, self.embed_scale)          # embed_norm
         xn, _ = self._res_norm(z, None, None, self.layers[0].n1)
         lib = _lib.lib()
+        in_place = self._decodes_in_place(mix, T)
         for li, L in enumerate(self.layers):
             gu = F.linear(xn.view(N, 2 * D), L.w_gu)                      # [N, 4*hidden]
             gated = torch.empty(N, L.hidden, 2, dtype=z.dtype, device=z.device)
@@ -210,9 +235,12 @@ class FusedForward:
             dn = F.linear(gated.view(N, 2 * L.hidden), L.w_down)
             xn2, mag = self._res_norm(z, dn, L.cgu_scale, L.n2, want_mag=L.w_mag is not None)
             raw = F.linear(xn2.view(N, 2 * D), L.w_front, L.b_front)
-            rawm = F.linear(mag, L.w_mag, L.b_mag) if L.w_mag is not None else None
-            q, k, v, gamma, coef = self._front(L, raw, rawm, B, T, positions, offset, mix.q_scale)
-            y = mix(li, q, k, v, gamma, coef)                              # [N, inner*2]
+            if in_place:
+                y = self._decode(li, L, raw, mag, positions, offset, mix)      # [N, inner*2]
+            else:
+                rawm = F.linear(mag, L.w_mag, L.b_mag) if L.w_mag is not None else None
+                q, k, v, gamma, coef = self._front(L, raw, rawm, B, T, positions, offset, mix.q_scale)
+                y = mix(li, q, k, v, gamma, coef)
             o = F.linear(y, L.w_o)
             nxt = self.layers[li + 1].n1 if li + 1 < len(self.layers) else self.out_scale
             xn, _ = self._res_norm(z, o, L.pam_scale, nxt)

@@ -155,13 +155,13 @@ class _DecodeMix:
     """Sequence mixing at decode: one recurrent step in place on the slots of the live sequences."""
 
     def __init__(self, eng, slots):
-        self.eng, self.slots = eng, slots
+        self.pool, self.slots = eng.pool, slots
         self.q_scale = eng.model.config.head_dim ** -0.5
 
     def __call__(self, layer, q, k, v, gamma, coef):
         n, H, _, d, _ = q.shape
         K = gamma.shape[0]
-        y = ops.pam_decode_step(self.eng.pool, self.slots, q.view(n, H, d, 2), k.view(n, H, d, 2), v.view(n, H, d, 2),
+        y = ops.pam_decode_step(self.pool, self.slots, q.view(n, H, d, 2), k.view(n, H, d, 2), v.view(n, H, d, 2),
                                 gamma.view(K, n, H), None if coef is None else coef.view(K, n, H, 2), layer=layer)
         return y.view(n, -1)
 
