@@ -191,6 +191,10 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
   request_weights(steps[0]);
   form_factors(steps[0], 0);
   __syncthreads();
+  // One state: it stays in registers, column r of rows [32 hf, 32 hf + 32) (as the sums leave the accumulators).  (In slots, as K
+  // states do it, 32 stores, 32 loads and a copy into shared memory a step: 22 k clocks instead of @@.)
+  constexpr bool HELD = OUT && !MULTI;
+  float S[HELD ? 32 : 1];
 
 #pragma unroll 1
   while (steps[cur].valid) {
@@ -217,6 +221,13 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
       return s.c == 0 ? p.s0 + (((size_t)k * p.geom.S + s.job.seq) * p.H + s.h) * (size_t)(TD * TD) * 2
                       : reinterpret_cast<const float*>(p.states + state_base(p, k, s.h, from_slot, TD));
     };
+    if constexpr (HELD) {
+      if (s.c == s.job.c0) {                 // a job begins: the state that enters its first chunk
+        const float* prev = has_state ? entering(0) + hf * 4096 + r : nullptr;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) S[i] = prev ? __ldcg(prev + i * 128) : 0.f;
+      }
+    }
     bool ok = mbar_wait(&bars[0], ph_tile, 241);
     // this thread's 16-byte pieces of the value tile (rows past the chunk's end: zeros, which also cancel whatever the key tile
     // holds in those rows), as in k_tc_chunk_outer
@@ -240,11 +251,45 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
     } else {
       __syncthreads();
     }
+    // the entering state as words of its bf16 planes, times the chunk constant (two columns a word: a lane takes row i or i + 2 for itself
+    // and the lane two further on); they go to the k region once the scores have been formed
+    uint32_t sw[HELD ? 16 : 1];
+    if constexpr (HELD) {
+      const float cst = state_const(Acum, strong_mask, 0);
+      const bool upper = lane & 2;
+#pragma unroll
+      for (int m = 0; m < 16; ++m) {
+        const int i = (m >> 1) * 4 + (m & 1);
+        const float mine = upper ? S[i + 2] : S[i], got = __shfl_xor_sync(0xffffffffu, upper ? S[i] : S[i + 2], 2);
+        sw[m] = upper ? pack_bf162(cst * got, cst * mine) : pack_bf162(cst * mine, cst * got);
+      }
+    }
     if (sums) {
       constexpr int G = OUT ? 16 : 8;          // columns at a time (three CTAs per SM have fewer registers)
       float pv[G];                             // that many of the thread's elements of the entering state, ahead of their use
       // the sums of state k leave the accumulators: S' = g S + U, U as in k_tc_chunk_outer
       auto sums_out = [&](int k) {
+        if constexpr (HELD) {
+          const float g = __expf(Acum[TC - 1]);
+#pragma unroll
+          for (int hh = 0; hh < 4; ++hh) {
+            float d1[8], d2[8];
+            tmem_ld8x2(tl + hf * 32 + hh * 8, d1, tl + 64 + hf * 32 + hh * 8, d2);
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+              const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, d2[i], 1), __shfl_xor_sync(0xffffffffu, d2[i + 1], 1));
+              const float2 u = ffma2(make_float2(g, g), make_float2(S[hh * 8 + i], S[hh * 8 + i + 1]), ffma2(make_float2(sign, sign), make_float2(d1[i], d1[i + 1]), o));
+              S[hh * 8 + i] = u.x;
+              S[hh * 8 + i + 1] = u.y;
+            }
+          }
+          if (to_final) {
+            FinalDest fin;
+            fin.init(p, s.job.seq, s.job.pool_slot, 0, s.h);
+            fin.store(p, hf * 4096 + r, S, even, ok);
+          }
+          return;
+        }
         const uint32_t from = tl + (OUT ? (uint32_t)(k & 1) * 128u : 0u);
         // lane n' = 2j+c holds column i, state[i][j][c] at i*128 + n'
         const float g = __expf(Acum[k * TC + TC - 1]);
@@ -312,7 +357,7 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
         }
         if (OUT && k > 0) sums_out(k - 1);      // (beside this state's products: they go to the other half of the accumulators)
         if (k == K) break;
-        if (has_state) {
+        if (MULTI && has_state) {
           const float* prev = entering(k) + hf * 4096 + r;
 #pragma unroll
           for (int i = 0; i < G; ++i) pv[i] = __ldcg(prev + i * 128);
@@ -321,7 +366,6 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
         ph_sum ^= 1;
         tc_fence_after();
       }
-      if (OUT && !MULTI && !to_final) asm volatile("fence.proxy.async;" ::: "memory");      // (the next step reads the state by a bulk copy)
     }
     if (tid == 0) {                          // the step after this one (known to all behind the next barrier)
       if (!job_ends) {
@@ -369,39 +413,13 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
       if constexpr (!MULTI) {
         // one state: as chunk_job<M_FWD>
         const bool strong = strong_mask != 0;
-        if (has_state && tid == 0) {
-          mbar_arrive_expect_tx(&bars[5], 32768);
-          bulk_load_1d(RB, entering(0), 32768, &bars[5]);
+        if (has_state) {
+          unsigned char* plane = RB + (lane & 1) * 8192 + ((r >> 2) & 3) * 4;      // columns j0 = 2 (r / 4) and j0 + 1 of plane re or im
+#pragma unroll
+          for (int m = 0; m < 16; ++m) *reinterpret_cast<uint32_t*>(plane + sw128(hf * 32 + (m >> 1) * 4 + (m & 1) + (lane & 2), r >> 4)) = sw[m];
         }
         bw_epi_scores(true, tl, q4, hf, r, s.len, strong, cfac, Acum, p.q_scale, 1.f);
         tmem_st_wait();
-        if (has_state) {
-          ok = mbar_wait(&bars[5], ph_state, 245) && ok;
-          ph_state ^= 1;
-          const float st_cst = strong ? 1.f : __expf(Acum[TC / 2 - 1]);
-          const int flip = (lane >> 2) & 1;
-          uint32_t st_r[4][2], st_i[4][2];
-#pragma unroll
-          for (int it = 0; it < 4; ++it) {
-            const int idx = tid + 256 * it;          // (i, c16): state[i][4*c16 .. +3]
-            const float4 a = *reinterpret_cast<const float4*>(RB + idx * 32 + flip * 16);
-            const float4 b = *reinterpret_cast<const float4*>(RB + idx * 32 + (flip ^ 1) * 16);
-            const float4 s01 = flip ? b : a, s23 = flip ? a : b;
-            st_r[it][0] = pack_bf162(st_cst * s01.x, st_cst * s01.z);
-            st_r[it][1] = pack_bf162(st_cst * s23.x, st_cst * s23.z);
-            st_i[it][0] = pack_bf162(st_cst * s01.y, st_cst * s01.w);
-            st_i[it][1] = pack_bf162(st_cst * s23.y, st_cst * s23.w);
-          }
-          __syncthreads();
-#pragma unroll
-          for (int it = 0; it < 4; ++it) {
-            const int idx = tid + 256 * it;
-            const int i = idx >> 4, c4 = idx & 15;
-            const uint32_t off = sw128(i, c4 >> 1) + (c4 & 1) * 8;
-            *reinterpret_cast<uint2*>(RB + off) = make_uint2(st_r[it][0], st_r[it][1]);
-            *reinterpret_cast<uint2*>(RB + 8192 + off) = make_uint2(st_i[it][0], st_i[it][1]);
-          }
-        }
         fence_proxy_async();
         tc_fence_before();
         __syncthreads();
