@@ -294,15 +294,16 @@ static int tc_outputs(const ScanParams& p, const ScanLayout& L, const qpam_scan_
   return QPAM_OK;
 }
 
-// Whether a forward-only call walks (pam_scan_walk.cuh): it wants more sequences and heads than the chip holds CTAs, and more still for
-// one state, whose three passes cost less; lengths of packed sequences are on the device, so by their number.  Measured (us, three passes
-// -> walking; packed lengths anywhere between the two given): K = 1, 32 x 512..16384, 16 heads 1614 -> 1442, 19 x 108..649, 16 heads
-// 69 -> 70, 24 x 326..5999, 12 heads 400 -> 469; K = 3, 48 x 32..1024, 12 heads 311 -> 245, 22 x 448..2034, 16 heads 517 -> 418,
-// 24 x 17..1482, 12 heads 262 -> 262, 5 x 170..2570, 6 heads 64 -> 94.  Of equal lengths the last round of CTAs has to be four fifths full.
+// Whether a forward-only call walks (pam_scan_walk.cuh): it wants more sequences and heads than the chip holds CTAs (296); lengths of
+// packed sequences are on the device, so by their number.  Measured (us, three passes -> walking; packed lengths anywhere between the
+// two given): one state, 32 x 512..16384, 16 heads 1772 -> 1247, 27 x 512..8192, 12 heads 751 -> 635, 19 x 108..649, 16 heads 74 -> 70,
+// 24 x 326..5999, 12 heads 420 -> 422, 23 x 44..11396, 12 heads 591 -> 747; three states, 48 x 32..1024, 12 heads 311 -> 242,
+// 21 x 80..2261, 16 heads 349 -> 315, 24 x 17..1482, 12 heads 256 -> 270, 5 x 170..2570, 6 heads 64 -> 94.  Of equal lengths the last
+// round of CTAs has to be four fifths full.
 static bool walk_pays(const qpam_scan_args* a, int ctas) {
   const int64_t units = (int64_t)a->S * a->H;
   if (a->y == nullptr || a->T == 0) return false;
-  if (a->cu_seqlens != nullptr) return units >= (a->K == 1 ? 384 : 320);
+  if (a->cu_seqlens != nullptr) return units >= (a->K == 1 ? 300 : 320);
   return units * 5 >= (units + ctas - 1) / ctas * ctas * 4;
 }
 

@@ -1,12 +1,12 @@
 // Forward scan of which no backward will read the states (bf16, d = 64, 1..4 states): a CTA takes a sequence and a head and WALKS
 // over its chunks.  A chunk's tiles are loaded once; they give the state the next chunk starts from and the output, and the
-// state stays with the CTA (two fp32 slots of 32 KB a state, written and read by the same SM, so in L2).
+// state stays with the CTA (one state in registers, several in two fp32 slots each, written and read by the same SM, so in L2).
 //
 // What bounds it: the chain of phases of a chunk (tiles, weighted planes, state sums, de-interleave, scores, masks, products, stores),
-// 22 k clocks for one state and 45 k for three with two CTAs per SM: a quarter of it the sums' way out of the accumulators, 42 % of the
-// issue slots taken.  The form it replaces, chunk sums -> carry -> outputs as three passes over all chunks, ran three such chains, read
+// 18 k clocks for one state and 45 k for three with two CTAs per SM (three: a quarter of it the sums' way out of the accumulators, 42 %
+// of the issue slots taken).  The form it replaces, chunk sums -> carry -> outputs as three passes over all chunks, ran three such chains, read
 // k and v twice and moved every chunk's state (K * 32 KB for 48-96 KB of tokens and output) through HBM two to four times.  32 documents
-// of 512..16384 tokens, 16 heads, one state: 1842 -> 1490 us; 48 chat prompts of 32..1024, 12 heads, three states: 324 -> 241; 256 prompts
+// of 512..16384 tokens, 16 heads, one state: 1842 -> 1285 us; 48 chat prompts of 32..1024, 12 heads, three states: 324 -> 241; 256 prompts
 // of 70, 12 heads, three states: 339 -> 213.
 // Code is kept short (rolled loops, 16 columns at a time): the first version, written out, was 216 KB for three states, spilled, and
 // missed the instruction cache; its score epilogue took 8.8 k clocks instead of 1.9 k.
@@ -17,7 +17,7 @@
 // A sequence that is long beside what the batch gives every SM to do would leave the chip to a few CTAs.  Its chunks are taken in the
 // three passes instead (`split`): sums of every chunk by this kernel without its output part, the carry, and one-chunk jobs whose state
 // is read from its slot, at the end of the same list.  Both ways give the same bits (the carry is the same sequence of fused multiply-adds).
-// (One sequence of 60000 tokens among 32 short ones: 673 us, 586 with kernels of their own for the three passes.)
+// (One sequence of 60000 tokens among 32 short ones: 715 us, 586 with kernels of their own for the three passes.)
 // Batches with few sequences and heads take the three passes as kernels of their own (scan_forward_only, pam_scan.cu).
 #pragma once
 #include "pam_scan_tc3.cuh"
@@ -34,11 +34,12 @@ __host__ __device__ constexpr size_t walk_smem(int K, bool out) { return 1024 + 
 enum { WT_OUT = 0, WT_SUM = 1, WT_JOBS = 2, WT_SPLIT_JOBS = 3, WT_CARRY = 4, WT_SPLIT = 5 };
 constexpr int WALK_MIN = 2;            // a sequence of at most so many chunks is always walked
 
-// Sequences of more chunks than twice what the call has for each CTA that the chip holds are split.  (A chunk costs a quarter more in
-// the three passes; a sequence of up to twice the mean, begun first, ends with the others.  32 documents of 512..16384 tokens, 16
-// heads, split above 0.75 / 1 / 1.25 / 2 / 3 times the mean: 1618 / 1516 / 1475 / 1442 / 1427 us.)
+// Sequences of more chunks than three times what the call has for each CTA that the chip holds are split.  (A chunk costs more in the
+// three passes, and a long sequence, begun first, ends with the others.  32 documents of 512..16384 tokens, 16 heads, split above 1.25 /
+// 1.5 / 2 / 3 times the mean: 1225 / 1296 / 1278 / 1247 us; 18 of 300..16000: 1181 / 1262 / 1080 / 1041; 22 of 400..9000, 12 heads: 658 /
+// 648 / 586 / 572.)
 __host__ __device__ inline int walk_split_above(int64_t chunk_heads, int ctas) {
-  const int64_t m = 2 * ((chunk_heads + ctas - 1) / ctas);
+  const int64_t m = 3 * ((chunk_heads + ctas - 1) / ctas);
   return (int)(m < WALK_MIN ? WALK_MIN : m > 0x3fffffff ? 0x3fffffff : m);
 }
 
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
   form_factors(steps[0], 0);
   __syncthreads();
   // One state: it stays in registers, column r of rows [32 hf, 32 hf + 32) (as the sums leave the accumulators).  (In slots, as K
-  // states do it, 32 stores, 32 loads and a copy into shared memory a step: 22 k clocks instead of @@.)
+  // states do it, 32 stores, 32 loads and a copy into shared memory a step: 22 k clocks instead of 18.)
   constexpr bool HELD = OUT && !MULTI;
   float S[HELD ? 32 : 1];
 
