@@ -83,12 +83,13 @@ __device__ __forceinline__ void kstate_scores(uint32_t tlane, int q4, int hf, in
 __device__ __forceinline__ float state_const(const float* Acum, uint32_t strong_mask, int k) {
   return ((strong_mask >> k) & 1u) ? 1.f : __expf(Acum[k * TC + TC / 2 - 1]);
 }
-// planes of a carried state (fp32 [i][j] (re, im)), times its chunk constant, into 16 KB at `dstp`
-__device__ __forceinline__ void kstate_planes(unsigned char* dstp, const void* state, float cst, int tid) {
+// planes of a carried state (fp32 [i][j] (re, im)), times its chunk constant, into 16 KB at `dstp`: requested, and written
+__device__ __forceinline__ void kstate_load(float4 (&v)[8], const void* state, int tid) {
   const float4* sg = reinterpret_cast<const float4*>(state);
-  float4 v[8];                               // all of them requested before the first is used
 #pragma unroll
   for (int it = 0; it < 8; ++it) v[it] = ld_dependent(sg + (tid + 256 * (it >> 1)) * 2 + (it & 1));
+}
+__device__ __forceinline__ void kstate_store(unsigned char* dstp, const float4 (&v)[8], float cst, int tid) {
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
     const int idx = tid + 256 * it;          // (i, c16): state[i][4*c16 .. +3]
@@ -98,6 +99,19 @@ __device__ __forceinline__ void kstate_planes(unsigned char* dstp, const void* s
     *reinterpret_cast<uint2*>(dstp + off) = make_uint2(pack_bf162(cst * s01.x, cst * s01.z), pack_bf162(cst * s23.x, cst * s23.z));
     *reinterpret_cast<uint2*>(dstp + 8192 + off) = make_uint2(pack_bf162(cst * s01.y, cst * s01.w), pack_bf162(cst * s23.y, cst * s23.w));
   }
+}
+__device__ __forceinline__ void kstate_planes(unsigned char* dstp, const void* state, float cst, int tid) {
+  float4 v[8];                               // all of them requested before the first is used
+  kstate_load(v, state, tid);
+  kstate_store(dstp, v, cst, tid);
+}
+// two of them into neighbouring slots, both on their way at once (48 chat prompts, three states: 242 -> 236 us)
+__device__ __forceinline__ void kstate_planes2(unsigned char* dstp, const void* state0, const void* state1, float cst0, float cst1, int tid) {
+  float4 v0[8], v1[8];
+  kstate_load(v0, state0, tid);
+  kstate_load(v1, state1, tid);
+  kstate_store(dstp, v0, cst0, tid);
+  kstate_store(dstp + 16384, v1, cst1, tid);
 }
 // T'[r][j] = rho_k[r] q_r[j], j = 0..63, as packed bf16 pairs: 32 columns of reals, 32 of imaginaries (slot hf of the pass)
 template <int K>
@@ -279,8 +293,8 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
   {
     kstate_scores<K>(tlane, q4, hf, r, strong_mask, rk, cfac, Acum);
     if (has_state) {          // the K planes are no longer needed: states 0 and 1 take their place
-#pragma unroll 1
-      for (int k = 0; k < 2; ++k) stage_state(k, k);
+      kstate_planes2(RB, p.states + state_base(p, 0, h, L.slot0 + L.c, TD), p.states + state_base(p, 1, h, L.slot0 + L.c, TD), state_const(Acum, strong_mask, 0),
+                     state_const(Acum, strong_mask, 1), tid);
     }
   }
   fence_proxy_async();

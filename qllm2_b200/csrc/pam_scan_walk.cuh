@@ -6,8 +6,8 @@
 // 18 k clocks for one state and 45 k for three with two CTAs per SM (three: a quarter of it the sums' way out of the accumulators, 42 %
 // of the issue slots taken).  The form it replaces, chunk sums -> carry -> outputs as three passes over all chunks, ran three such chains, read
 // k and v twice and moved every chunk's state (K * 32 KB for 48-96 KB of tokens and output) through HBM two to four times.  32 documents
-// of 512..16384 tokens, 16 heads, one state: 1842 -> 1285 us; 48 chat prompts of 32..1024, 12 heads, three states: 324 -> 241; 256 prompts
-// of 70, 12 heads, three states: 339 -> 213.
+// of 512..16384 tokens, 16 heads, one state: 1842 -> 1299 us; 48 chat prompts of 32..1024, 12 heads, three states: 324 -> 236; 256 prompts
+// of 70, 12 heads, three states: 339 -> 203.
 // Code is kept short (rolled loops, 16 columns at a time): the first version, written out, was 216 KB for three states, spilled, and
 // missed the instruction cache; its score epilogue took 8.8 k clocks instead of 1.9 k.
 //
@@ -29,7 +29,7 @@ namespace tcs {
 // (four states have room for one)
 __host__ __device__ constexpr int walk_sets(int K) { return K <= 3 ? 2 : 1; }
 __host__ __device__ constexpr size_t walk_smem(int K, bool out) { return 1024 + (out ? 3 : 2) * 32768 + (size_t)walk_sets(K) * K * TC * 20 + 512; }
-// ScanParams::ticket: [0] outputs drawn  [1] sums drawn  [2] entries of the list  [3] how many of them, at its end, are chunks of split
+// ScanParams::ticket: [0] next job of the outputs  [1] of the sums  [2] entries of the list  [3] how many of them, at its end, are chunks of split
 // sequences: the jobs of the sums  [4] any sequence for the carry  [5] sequences of more chunks are split
 enum { WT_OUT = 0, WT_SUM = 1, WT_JOBS = 2, WT_SPLIT_JOBS = 3, WT_CARRY = 4, WT_SPLIT = 5 };
 constexpr int WALK_MIN = 2;            // a sequence of at most so many chunks is always walked
@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
   const WalkJob* jobs = p.jobs;
   if (packed) {
     entries = p.ticket[OUT ? WT_JOBS : WT_SPLIT_JOBS];
+    if (entries == 0u) return;               // (the sums of a call without split sequences)
     if (!OUT) jobs += p.ticket[WT_JOBS] - entries;
   }
   const unsigned int total = entries * (unsigned int)p.H;
@@ -157,7 +158,7 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
 #pragma unroll
     for (int i = 0; i < 6; ++i) mbar_init(&bars[i], 1);
     fence_barrier_init();
-    const unsigned int t = packed ? atomicAdd(p.ticket + (OUT ? WT_OUT : WT_SUM), 1u) : blockIdx.x;
+    const unsigned int t = blockIdx.x;       // (the counters start behind the grid)
     steps[0].valid = 0;
     if (t < total && *failed == 0) {
       steps[0].job = packed ? jobs[t / (unsigned int)p.H] : walk_uniform_job(p, (int)(t / (unsigned int)p.H));
@@ -456,10 +457,7 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
 #pragma unroll
         for (int k = 0; k < K; ++k) rk[k] = rho[k * TC + r];
         kstate_scores<K>(tl, q4, hf, r, strong_mask, rk, cfac, Acum);
-        if (has_state) {
-#pragma unroll 1
-          for (int k = 0; k < 2; ++k) kstate_planes(RB + k * 16384, entering(k), state_const(Acum, strong_mask, k), tid);
-        }
+        if (has_state) kstate_planes2(RB, entering(0), entering(1), state_const(Acum, strong_mask, 0), state_const(Acum, strong_mask, 1), tid);
         fence_proxy_async();
         tc_fence_before();
         __syncthreads();
@@ -586,17 +584,24 @@ __global__ void __launch_bounds__(1024) k_walk_plan(ScanParams p, int32_t* __res
     __syncthreads();
     return inc;
   };
+  int first = 0, end = 0, slot = -1, before_me = 0;      // of sequence tid (all of a call's, if there are no more than threads)
   for (int base = 0; base < S; base += 1024) {
     const int s = base + tid;
     int n = 0;
     if (s < S) {
       const int a = cu[s], e = cu[s + 1];
+      if (base == 0) {
+        first = a;
+        end = e;
+        slot = pool_slot_of(p, s);
+      }
       if (!(e >= a && e <= p.T)) bad_s = 1;
       n = (max(0, e - a) + TC - 1) / TC;
     }
     int all;
     const int inc = scan(n, all), before = carry_s;
     if (s < S) prefix[s + 1] = before + inc;
+    if (base == 0) before_me = inc - n;
     __syncthreads();
     if (tid == 0) carry_s = before + all;
     __syncthreads();
@@ -611,8 +616,9 @@ __global__ void __launch_bounds__(1024) k_walk_plan(ScanParams p, int32_t* __res
     return;
   }
   const int above = walk_split_above((int64_t)C * p.H, ctas);
+  auto chunks_of = [&](int s) { return s < 1024 ? (end - first + TC - 1) / TC : prefix[s + 1] - prefix[s]; };
   for (int s = tid; s < S; s += 1024) {
-    const int nc = prefix[s + 1] - prefix[s];
+    const int nc = chunks_of(s);
     if (nc > 0 && nc <= above) atomicAdd(&hist[min(nc, 1023)], 1);
     else special_s = 1;
   }
@@ -622,8 +628,10 @@ __global__ void __launch_bounds__(1024) k_walk_plan(ScanParams p, int32_t* __res
   hist[1023 - tid] = inc - mine;
   __syncthreads();
   for (int s = tid; s < S; s += 1024) {
-    const int nc = prefix[s + 1] - prefix[s];
-    if (nc > 0 && nc <= above) jobs[atomicAdd(&hist[min(nc, 1023)], 1)] = WalkJob{s, 0, nc, nc, cu[s], cu[s + 1], prefix[s] + s, pool_slot_of(p, s)};
+    const int nc = chunks_of(s);
+    if (nc > 0 && nc <= above)
+      jobs[atomicAdd(&hist[min(nc, 1023)], 1)] = s < 1024 ? WalkJob{s, 0, nc, nc, first, end, before_me + s, slot}
+                                                          : WalkJob{s, 0, nc, nc, cu[s], cu[s + 1], prefix[s] + s, pool_slot_of(p, s)};
   }
   if (special_s)
     for (int x = tid; x < C; x += 1024) {
@@ -640,7 +648,8 @@ __global__ void __launch_bounds__(1024) k_walk_plan(ScanParams p, int32_t* __res
     }
   __syncthreads();
   if (tid == 0) {
-    p.ticket[WT_OUT] = p.ticket[WT_SUM] = 0u;
+    p.ticket[WT_OUT] = (unsigned int)ctas;               // (behind the grids of the two: a CTA's first job is its index)
+    p.ticket[WT_SUM] = (unsigned int)(3 * ctas / 2);
     p.ticket[WT_JOBS] = (unsigned int)(walked + split_s);
     p.ticket[WT_SPLIT_JOBS] = (unsigned int)split_s;
     p.ticket[WT_CARRY] = (unsigned int)special_s;
