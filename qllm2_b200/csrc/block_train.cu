@@ -43,6 +43,8 @@ __device__ __forceinline__ float2 unpack2(uint32_t w) { return make_float2(__uin
 // A CTA takes 256 groups of four source columns of one item.
 template <bool UNPACK>
 __global__ void __launch_bounds__(256) k_pack_block(const __grid_constant__ PackList L) {
+  pdl_wait();
+  pdl_trigger();
   int i = 0;
   while (i + 1 < L.n && (int)blockIdx.x >= L.first_block[i + 1]) ++i;
   const qpam_pack_item& t = L.it[i];
@@ -107,6 +109,8 @@ template <int MAXV>
 __global__ void __launch_bounds__(128) k_norm_train(const bf16* __restrict__ z, const bf16* __restrict__ delta, const float* __restrict__ s_ptr,
                                                     const float* __restrict__ scale, bf16* __restrict__ z_out, bf16* __restrict__ xn,
                                                     bf16* __restrict__ mag_out, int64_t N, int D, float eps) {
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31, groups = D >> 2;
   const float s = delta ? *s_ptr : 0.f;
   for (int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5); row < N; row += (int64_t)gridDim.x * 4) {
@@ -161,6 +165,8 @@ __global__ void __launch_bounds__(128) k_norm_train(const bf16* __restrict__ z, 
 template <bool SWISH>
 __global__ void __launch_bounds__(512) k_act_gate_train(const bf16* __restrict__ gate, const bf16* __restrict__ up, const float* __restrict__ bias,
                                                         const float* __restrict__ beta, bf16* __restrict__ out, int64_t N, int C) {
+  pdl_wait();
+  pdl_trigger();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (C >> 2)) return;
   float b4[4], be4[4];
@@ -193,6 +199,8 @@ __global__ void __launch_bounds__(512) k_act_gate_train(const bf16* __restrict__
 template <bool SWISH>
 __global__ void __launch_bounds__(512) k_act_gate_bwd(const bf16* __restrict__ gate, const bf16* __restrict__ up, const bf16* __restrict__ dout,
                                                       const float* __restrict__ bias, const float* __restrict__ beta, bf16* __restrict__ dgu, float* __restrict__ part, int64_t N, int C) {
+  pdl_wait();
+  pdl_trigger();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (C >> 2)) return;
   float b4[4], be4[4], ab[4] = {0.f, 0.f, 0.f, 0.f}, abe[4] = {0.f, 0.f, 0.f, 0.f};
@@ -275,6 +283,8 @@ __global__ void __launch_bounds__(128) k_cnorm_res_bwd(const bf16* __restrict__ 
                                                        const bf16* __restrict__ dmag, const bf16* __restrict__ dres, const bf16* __restrict__ delta,
                                                        const float* __restrict__ s_ptr, bf16* __restrict__ dz, bf16* __restrict__ ddelta,
                                                        float* __restrict__ part, int64_t N, int D, float eps) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ float sh[];               // [4][D + 1]
   const int lane = threadIdx.x & 31, w4 = threadIdx.x >> 5;
   const int64_t warp = (int64_t)blockIdx.x * 4 + w4, nwarps = (int64_t)gridDim.x * 4;
@@ -406,6 +416,8 @@ __global__ void __launch_bounds__(128) k_cnorm_res_bwd(const bf16* __restrict__ 
 // tokens, while another CTA of the SM streams (112 us with tiles of four tokens, 47 us
 // so; 27 us of traffic).
 __global__ void __launch_bounds__(1024) k_front_bwd(const __grid_constant__ qpam_front_bwd_args p, int per_tok_pad, int tile_tok) {
+  pdl_wait();
+  pdl_trigger();
   const qpam_front_args& a = p.f;
   extern __shared__ float domp[];             // [tile_tok][H], then the CTA's sums [tile_tok * H][3K + 1]
   const int H = a.H, K = a.K, d = a.d, gph = d >> 2, tid = threadIdx.x;
@@ -559,6 +571,8 @@ struct SumList {
 };
 // out[c] = sum_p part[p][c]; a CTA takes 32 columns, 32 threads each.
 __global__ void __launch_bounds__(1024) k_colsum(const __grid_constant__ SumList L) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float sh[32][33];
   int i = 0;
   while (i + 1 < L.n && (int)blockIdx.x >= L.first_block[i + 1]) ++i;
@@ -618,7 +632,7 @@ int pack_launch(const qpam_pack_item* items, int32_t n, void* stream) {
   }
   L.first_block[n] = blocks;
   cudaStream_t st = (cudaStream_t)stream;
-  k_pack_block<UNPACK><<<blocks, 256, 0, st>>>(L);
+  launch_after(k_pack_block<UNPACK>, blocks, 256, 0, st, L);
   QPAM_LAUNCH_CHECK("k_pack_block");
   return QPAM_OK;
 }
@@ -645,7 +659,7 @@ extern "C" int qpam_colsum(const qpam_colsum_item* items, int32_t n, void* strea
   }
   L.first_block[n] = blocks;
   cudaStream_t st = (cudaStream_t)stream;
-  k_colsum<<<blocks, 1024, 0, st>>>(L);
+  launch_after(k_colsum, blocks, 1024, 0, st, L);
   QPAM_LAUNCH_CHECK("k_colsum");
   return QPAM_OK;
 }
@@ -657,7 +671,7 @@ extern "C" int qpam_norm_train_fwd(const void* z, const void* delta, const float
   cudaStream_t st = (cudaStream_t)stream;
   const int blocks = (int)std::min<int64_t>((N + 3) / 4, sm_count() * 16);
 #define QPAM_NT(MV) \
-  k_norm_train<MV><<<blocks, 128, 0, st>>>((const bf16*)z, (const bf16*)delta, s, scale, (bf16*)z_out, (bf16*)xn, (bf16*)mag, N, D, eps)
+  launch_after(k_norm_train<MV>, blocks, 128, 0, st, (const bf16*)z, (const bf16*)delta, s, scale, (bf16*)z_out, (bf16*)xn, (bf16*)mag, N, D, eps)
   if (D <= 384) QPAM_NT(3);
   else QPAM_NT(6);
 #undef QPAM_NT
@@ -671,8 +685,8 @@ extern "C" int qpam_act_gate_train_fwd(const void* gate, const void* up, const f
   cudaStream_t st = (cudaStream_t)stream;
   const int groups = C / 4, threads = pick_threads(groups), xb = (groups + threads - 1) / threads;
   dim3 grid(xb, (unsigned)std::min<int64_t>(N, std::max(1, (sm_count() * 2048) / (xb * threads))));
-  if (beta) k_act_gate_train<true><<<grid, threads, 0, st>>>((const bf16*)gate, (const bf16*)up, bias, beta, (bf16*)out, N, C);
-  else k_act_gate_train<false><<<grid, threads, 0, st>>>((const bf16*)gate, (const bf16*)up, bias, beta, (bf16*)out, N, C);
+  if (beta) launch_after(k_act_gate_train<true>, grid, threads, 0, st, (const bf16*)gate, (const bf16*)up, bias, beta, (bf16*)out, N, C);
+  else launch_after(k_act_gate_train<false>, grid, threads, 0, st, (const bf16*)gate, (const bf16*)up, bias, beta, (bf16*)out, N, C);
   QPAM_LAUNCH_CHECK("k_act_gate_train");
   return QPAM_OK;
 }
@@ -688,8 +702,8 @@ extern "C" int qpam_act_gate_bwd(const void* gate, const void* up, const void* d
   cudaStream_t st = (cudaStream_t)stream;
   const int groups = C / 4, threads = pick_threads(groups);
   dim3 grid((groups + threads - 1) / threads, P);
-  if (beta) k_act_gate_bwd<true><<<grid, threads, 0, st>>>((const bf16*)gate, (const bf16*)up, (const bf16*)dout, bias, beta, (bf16*)dgate_up, part, N, C);
-  else k_act_gate_bwd<false><<<grid, threads, 0, st>>>((const bf16*)gate, (const bf16*)up, (const bf16*)dout, bias, beta, (bf16*)dgate_up, part, N, C);
+  if (beta) launch_after(k_act_gate_bwd<true>, grid, threads, 0, st, (const bf16*)gate, (const bf16*)up, (const bf16*)dout, bias, beta, (bf16*)dgate_up, part, N, C);
+  else launch_after(k_act_gate_bwd<false>, grid, threads, 0, st, (const bf16*)gate, (const bf16*)up, (const bf16*)dout, bias, beta, (bf16*)dgate_up, part, N, C);
   QPAM_LAUNCH_CHECK("k_act_gate_bwd");
   return QPAM_OK;
 }
@@ -701,7 +715,7 @@ extern "C" int qpam_cnorm_res_bwd(const void* z, const float* scale, const void*
   cudaStream_t st = (cudaStream_t)stream;
   const size_t smem = (size_t)4 * (D + 1) * sizeof(float);
 #define QPAM_NRB(MV)                                                                                                                      \
-  k_cnorm_res_bwd<MV><<<P, 128, smem, st>>>((const bf16*)z, scale, (const bf16*)dxn, (const bf16*)dmag, (const bf16*)dres, (const bf16*)delta, s, \
+  launch_after(k_cnorm_res_bwd<MV>, P, 128, smem, st, (const bf16*)z, scale, (const bf16*)dxn, (const bf16*)dmag, (const bf16*)dres, (const bf16*)delta, s, \
                                             (bf16*)dz, (bf16*)ddelta, part, N, D, eps)
   if (D <= 384) QPAM_NRB(3);
   else QPAM_NRB(6);
@@ -726,7 +740,7 @@ extern "C" int qpam_pam_front_bwd(const qpam_front_bwd_args* p, void* stream) {
   const int tile = (int)std::min<int64_t>(most, (share + slots - 1) / slots * slots);
   const size_t smem = (size_t)tile * a.H * (3 * a.K + 1) * sizeof(float);
   cudaStream_t st = (cudaStream_t)stream;
-  k_front_bwd<<<p->P, threads, smem, st>>>(*p, per_tok, tile);
+  launch_after(k_front_bwd, p->P, threads, smem, st, *p, per_tok, tile);
   QPAM_LAUNCH_CHECK("k_front_bwd");
   return QPAM_OK;
 }
