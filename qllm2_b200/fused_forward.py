@@ -41,6 +41,21 @@ def _is_table(m) -> bool:
             not _has_any_global_hook() and w.is_contiguous() and w.data_ptr() % 16 == 0)
 
 
+class PoolDecodeMix:
+    """Sequence mixing at decode, as `FusedForward.hidden` takes it: one recurrent step in place on the pool slots of the live
+    sequences.  slots [n]: integers of any type, those that name no slot are idle rows."""
+
+    def __init__(self, pool, slots, head_dim):
+        self.pool, self.slots, self.q_scale = pool, slots, head_dim ** -0.5
+
+    def __call__(self, layer, q, k, v, gamma, coef):
+        n, H, _, d, _ = q.shape
+        K = gamma.shape[0]
+        y = ops.pam_decode_step(self.pool, self.slots, q.view(n, H, d, 2), k.view(n, H, d, 2), v.view(n, H, d, 2),
+                                gamma.view(K, n, H), None if coef is None else coef.view(K, n, H, 2), layer=layer)
+        return y.view(n, -1)
+
+
 class FusedForward:
     def __init__(self, model: V11LM, max_position: int = 8192):
         cfg = model.config
@@ -189,16 +204,16 @@ class FusedForward:
         return q, k, v, gamma, coef
 
     def _decodes_in_place(self, mix, T) -> bool:
-        """Whether one launch forms q, k, v and the gates of a token and does the recurrent step on the pool of `mix`."""
-        pool = getattr(mix, "pool", None)
-        return (T == 1 and pool is not None and self.dtype == pool.dtype == torch.bfloat16 and self.d == 64 and self.D % 8 == 0 and
+        """Whether one launch forms q, k, v and the gates of a token and does the recurrent step on the pool of `mix`.  Only for
+        `PoolDecodeMix` itself: any other object, a subclass too, may do something else when it is called."""
+        if T != 1 or type(mix) is not PoolDecodeMix:
+            return False
+        pool = mix.pool
+        return (pool.device == self.device and self.dtype == pool.dtype == torch.bfloat16 and self.d == 64 and self.D % 8 == 0 and
                 pool.is_contiguous() and pool.data_ptr() % 16 == 0 and tuple(pool.shape[1:]) == (len(self.layers), self.K, self.H, 64, 64, 2))
 
-    def _decode(self, li, L, raw, mag, positions, offset, mix):
+    def _decode(self, li, L, raw, mag, positions, offset, mix, slots):
         n = raw.shape[0]
-        if mix.slots.dtype != torch.int32 or mix.slots.numel() != n or mix.slots.device != raw.device:
-            raise _lib.QPamError("decode: int32 slot ids, one per sequence, expected")
-        slots = mix.slots.contiguous()
         a = _lib.DecodeFrontArgs()
         self._front_args(a.f, L, raw, None, positions, offset, mix.q_scale)
         a.mag_row[:] = [L.cols[name][1] if L.cols.get(name, "?")[0] == "m" else -1 for name in ("dt", "pg", "phase", "score")]
@@ -212,8 +227,8 @@ class FusedForward:
     @torch.no_grad()
     def hidden(self, ids: torch.Tensor, mix, positions: Optional[torch.Tensor] = None, offset: int = 0):
         """Run the blocks over ids [B, T]; `mix(layer, q, k, v, gamma, coef) -> y [B*T, inner*2]` is the
-        sequence-mixing step (a scan at prefill, the recurrent step at decode; a mix with a `pool` and `slots` is the
-        latter, and may be done in one launch with what it takes).  Returns the final residual stream normalised by
+        sequence-mixing step (a scan at prefill, the recurrent step at decode; `PoolDecodeMix` is the latter, and may be
+        done in one launch with what it takes instead of being called).  Returns the final residual stream normalised by
         output_norm, [B*T, D, 2]."""
         m, D = self.model, self.D
         B, T = ids.shape
@@ -226,7 +241,11 @@ class FusedForward:
         z, _ = self._res_norm(z, None, None, self.embed_scale)          # embed_norm
         xn, _ = self._res_norm(z, None, None, self.layers[0].n1)
         lib = _lib.lib()
-        in_place = self._decodes_in_place(mix, T)
+        slots = None                                                    # of a step that is done in one launch with what it takes
+        if self._decodes_in_place(mix, T):
+            slots = mix.slots.to(device=self.device, dtype=torch.int32).contiguous()
+            if slots.numel() != N:
+                raise _lib.QPamError("slot_ids must have one entry per sequence")
         for li, L in enumerate(self.layers):
             gu = F.linear(xn.view(N, 2 * D), L.w_gu)                      # [N, 4*hidden]
             gated = torch.empty(N, L.hidden, 2, dtype=z.dtype, device=z.device)
@@ -235,8 +254,8 @@ class FusedForward:
             dn = F.linear(gated.view(N, 2 * L.hidden), L.w_down)
             xn2, mag = self._res_norm(z, dn, L.cgu_scale, L.n2, want_mag=L.w_mag is not None)
             raw = F.linear(xn2.view(N, 2 * D), L.w_front, L.b_front)
-            if in_place:
-                y = self._decode(li, L, raw, mag, positions, offset, mix)      # [N, inner*2]
+            if slots is not None:
+                y = self._decode(li, L, raw, mag, positions, offset, mix, slots)      # [N, inner*2]
             else:
                 rawm = F.linear(mag, L.w_mag, L.b_mag) if L.w_mag is not None else None
                 q, k, v, gamma, coef = self._front(L, raw, rawm, B, T, positions, offset, mix.q_scale)

@@ -20,7 +20,7 @@ from typing import Deque, Dict, Iterable, List, Optional
 import torch
 
 from . import _lib, ops
-from .fused_forward import FusedForward
+from .fused_forward import FusedForward, PoolDecodeMix as _PoolDecodeMix
 from .model import V11LM
 
 
@@ -149,21 +149,6 @@ def _captured():
             graph.capture_end()
     finally:
         torch.cuda.current_stream().wait_stream(side)
-
-
-class _DecodeMix:
-    """Sequence mixing at decode: one recurrent step in place on the slots of the live sequences."""
-
-    def __init__(self, eng, slots):
-        self.pool, self.slots = eng.pool, slots
-        self.q_scale = eng.model.config.head_dim ** -0.5
-
-    def __call__(self, layer, q, k, v, gamma, coef):
-        n, H, _, d, _ = q.shape
-        K = gamma.shape[0]
-        y = ops.pam_decode_step(self.pool, self.slots, q.view(n, H, d, 2), k.view(n, H, d, 2), v.view(n, H, d, 2),
-                                gamma.view(K, n, H), None if coef is None else coef.view(K, n, H, 2), layer=layer)
-        return y.view(n, -1)
 
 
 class ContinuousBatcher:
@@ -366,7 +351,7 @@ class ContinuousBatcher:
             out = self.ff.step(ids, positions, slots, self.pool, logits=self.sampling is not None)
             return out if self.sampling is None else self._draw(out, slots)
         if self.ff is not None:
-            xn = self.ff.hidden(ids, _DecodeMix(self, slots), positions=positions)
+            xn = self.ff.hidden(ids, _PoolDecodeMix(self.pool, slots, self.model.config.head_dim), positions=positions)
             return self._pick(self.ff.head_hidden(xn), slots)
         m = self.model
         n = ids.shape[0]
@@ -465,18 +450,6 @@ class ContinuousBatcher:
 
 
 # ------------------------------------------------------------------------------------ V11LM.generate
-class _PoolDecodeMix:
-    def __init__(self, pool, slots, head_dim):
-        self.pool, self.slots, self.q_scale = pool, slots, head_dim ** -0.5
-
-    def __call__(self, layer, q, k, v, gamma, coef):
-        n, H, _, d, _ = q.shape
-        K = gamma.shape[0]
-        y = ops.pam_decode_step(self.pool, self.slots, q.view(n, H, d, 2), k.view(n, H, d, 2), v.view(n, H, d, 2),
-                                gamma.view(K, n, H), None if coef is None else coef.view(K, n, H, 2), layer=layer)
-        return y.view(n, -1)
-
-
 def _fused_forward_of(model: V11LM, need_positions: int) -> FusedForward:
     """The model's packed forward, rebuilt when a parameter changed or longer positions are needed."""
     key = (tuple(p._version for p in model.parameters()), next(model.parameters()).dtype, next(model.parameters()).device)

@@ -63,3 +63,50 @@ def test_decode_front_against_separate_kernels(name, n):
     untouched = torch.ones(n + 3, dtype=torch.bool, device=DEV)
     untouched[slots[(slots >= 0) & (slots < n + 3)].long()] = False
     assert torch.equal(p2[untouched], pool[untouched])
+
+
+def _small():
+    torch.manual_seed(5)
+    cfg = M.V11Config(vocab_size=101, head_dim=64, n_layers=2, dropout=0.0, gradient_checkpointing=False, max_seq_len=64, **CONFIGS["k3_content"])
+    ff = FusedForward(M.V11LM(cfg).to(DEV).bfloat16().eval(), 64)
+    pool = torch.randn(5, 2, 3, 2, 64, 64, 2, device=DEV, generator=torch.Generator(device=DEV).manual_seed(2)).bfloat16()
+    return ff, pool, torch.tensor([[3], [8], [1]], device=DEV), torch.tensor([2, 0, 4], device=DEV, dtype=torch.int32)
+
+
+class _Scaled(_PoolDecodeMix):
+    def __call__(self, *args):
+        return super().__call__(*args) * 256
+
+
+class _Own:
+    """Anything with a pool, slots and a q_scale; its mixing is its own."""
+
+    def __init__(self, pool, slots):
+        self.pool, self.slots, self.q_scale, self.calls = pool, slots, 0.125, []
+
+    def __call__(self, layer, q, k, v, gamma, coef):
+        self.calls.append((layer, tuple(q.shape)))
+        return v[:, :, 0].reshape(v.shape[0], -1)
+
+
+def test_a_callers_mix_is_called():
+    ff, pool, ids, slots = _small()
+    plain = ff.hidden(ids, _PoolDecodeMix(pool.clone(), slots, 64))
+    scaled = ff.hidden(ids, _Scaled(pool.clone(), slots, 64))
+    assert torch.equal(scaled, ff.hidden(ids, _Separate(_Scaled(pool.clone(), slots, 64)))) and not torch.equal(scaled, plain)
+    own, before = _Own(pool, slots), pool.clone()
+    got = ff.hidden(ids, own)
+    assert own.calls == [(0, (3, 2, 1, 64, 2)), (1, (3, 2, 1, 64, 2))] and torch.equal(pool, before)
+    assert torch.equal(got, ff.hidden(ids, _Separate(own)))
+
+
+def test_slot_ids_and_pools_as_the_separate_step_takes_them():
+    ff, pool, ids, slots = _small()
+    want_pool = pool.clone()
+    want = ff.hidden(ids, _Separate(_PoolDecodeMix(want_pool, slots, 64)))
+    for other in (slots.long(), slots.cpu(), slots.short(), torch.stack([slots, slots], 1)[:, 0]):
+        p = pool.clone()
+        assert torch.equal(ff.hidden(ids, _PoolDecodeMix(p, other, 64)), want) and torch.equal(p, want_pool)
+    for mix in (_PoolDecodeMix(pool, slots[:2], 64), _PoolDecodeMix(pool.cpu(), slots, 64), _PoolDecodeMix(pool.transpose(0, 1), slots, 64)):
+        with pytest.raises(_lib.QPamError):
+            ff.hidden(ids, mix)

@@ -170,3 +170,17 @@ def test_scheduler_chunked_prefill_plan():
     assert [(st, n) for _, st, n in w.plan_prefill()] == [(0, 10), (0, 10)]
     with pytest.raises(ValueError):
         SlotScheduler(1, max_prefill_tokens=0)
+
+
+def test_decode_in_one_launch_only_on_the_models_device():
+    """The one-launch decode step gets the pool as a pointer: a pool elsewhere takes the operator, which refuses it."""
+    from types import SimpleNamespace
+
+    from qllm2_b200.fused_forward import FusedForward
+    from qllm2_b200.serving import _PoolDecodeMix
+    ff = SimpleNamespace(device=torch.device("cuda:0"), dtype=torch.bfloat16, d=64, D=64, H=2, K=1, layers=[None])
+    pool = torch.zeros(2, 1, 1, 2, 64, 64, 2, dtype=torch.bfloat16)
+    mix = _PoolDecodeMix(pool, torch.zeros(1, dtype=torch.int32), 64)
+    assert not FusedForward._decodes_in_place(ff, mix, 1)
+    ff.device = torch.device("cpu")
+    assert FusedForward._decodes_in_place(ff, mix, 1) and not FusedForward._decodes_in_place(ff, mix, 2)
