@@ -532,9 +532,9 @@ int qpam_profile_end(char* buf, size_t buf_bytes);
  * synchronise anyway (once per optimizer step, once per decode step).  (No counterpart in the reference.) */
 int qpam_device_status(int32_t* status, int32_t clear);
 
-/* Diagnostic: launches one thread that waits on an mbarrier nobody arrives at and gives up after limit_ns
- * (0 < limit_ns <= 1e8), leaving 299 in the status word -- the give-up path of every bounded wait in this
- * library, exercised without hanging or faulting anything.  (No counterpart in the reference.) */
+/* Diagnostic: launches one warp half of whose lanes wait on an mbarrier nobody arrives at and give up after limit_ns
+ * (0 < limit_ns <= 1e8), leaving 299 in the status word (298 if the warp's lanes do not agree that the wait failed) -- the
+ * give-up path of every bounded wait in this library, exercised without hanging or faulting anything.  (No counterpart in the reference.) */
 int qpam_selftest_wait_expiry(int64_t limit_ns, void* stream);
 
 /* Diagnostic: y[i] = f(x[i]) for one of the approximate special functions that the element-wise kernels and the sampler

@@ -591,15 +591,17 @@ static int scan_bwd_t(const qpam_scan_args* a, const ScanLayout& L, const void* 
 }  // namespace qpam
 
 namespace qpam {
-// one thread waits on an mbarrier nobody arrives at, with a short limit: exercises the give-up path of every
-// bounded wait (status word, return) without hanging anything
+// one warp waits on an mbarrier nobody arrives at, its even lanes for a phase that never ends, with a short limit, its odd
+// lanes for the phase before it, which has ended: exercises the give-up path of every bounded wait (status word, return)
+// without hanging anything.  A lane that is told the wait succeeded says so in the status.
 __global__ void k_wait_selftest(unsigned long long limit_ns) {
   __shared__ uint64_t bar;
   if (threadIdx.x == 0) {
     umma::mbar_init(&bar, 1);
     umma::fence_barrier_init();
-    umma::mbar_wait(&bar, 0, QPAM_DEV_WAIT_SELFTEST, limit_ns);
   }
+  __syncwarp();
+  if (umma::mbar_wait_warp(&bar, threadIdx.x & 1, QPAM_DEV_WAIT_SELFTEST, limit_ns)) atomicExch(&umma::g_device_error, QPAM_DEV_WAIT_SELFTEST - 1);
 }
 int scan_tc_device_status(int* value, bool clear) {
   QPAM_CUDA(umma::read_device_error(value, clear));

@@ -476,7 +476,7 @@ __device__ __forceinline__ void chunk_job(const int mode, const CUtensorMap* __r
     // A full chunk leaves through the X2 region, which every MMA has finished reading: each warp stages its 32 rows
     // x 128 bytes there and one TMA store moves the block (whole 128-byte lines instead of 16 bytes per lane and
     // row).  A ragged chunk (its rows past `len` belong to someone else) stores per lane.
-    const bool bulk = ok && L.len == TC;                                             // CTA-uniform
+    const bool bulk = warp_agrees(ok) && L.len == TC;
     const bool tok = MODE == M_FWD && p.y_token_major;     // [B, T, H, d, 2]: the map's rows are tokens, a row holds all heads
     constexpr bool accum = ACC && MODE != M_FWD;             // gradients of several scans over the same q, k, v add up
     unsigned char* wbox = RC + hf * 16384 + q4 * 4096;                               // this warp's 32 x 128 B block

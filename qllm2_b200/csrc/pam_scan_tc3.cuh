@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(256, 2) k_tc_chunk_fwdK(const __grid_constant_
     __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.y) + rbase;
     // a full chunk leaves through the X2 region (no MMA reads it any more): 32 rows x 128 bytes per warp, one TMA
     // store each; a ragged chunk stores per lane
-    const bool bulk = ok && L.len == TC;                                             // CTA-uniform
+    const bool bulk = warp_agrees(ok) && L.len == TC;
     unsigned char* wrow = RC + hf * 16384 + (warp & 3) * 4096 + lane * 128;
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc) {

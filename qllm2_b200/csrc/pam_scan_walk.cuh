@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
       if (tid == 0 && nx.valid) request_tiles(nx);
       // ---- the output leaves through the k region: 32 rows x 128 bytes a warp, one TMA store each; a ragged chunk (its rows past
       // the end belong to someone else) stores per lane
-      const bool bulk = ok && s.len == TC;                                             // CTA-uniform
+      const bool bulk = warp_agrees(ok) && s.len == TC;
       const float rf = MULTI || strong_mask != 0 ? 1.f : rho[r].x;
       __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.y) + (p.y_token_major ? (((size_t)s.b * p.T + s.t0 + r) * p.H + s.h) * (size_t)(TD * 2)
                                                                                      : token_base(p, s.b, s.h, s.t0 + r, TD)) + hf * 64;

@@ -283,7 +283,7 @@ k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
         const int n = tile_n(nn), m_tile = tile_m(nn);
         const int buf = it % C::NBUF;
         const uint32_t bphase = (it / C::NBUF) & 1;
-        if (!mbar_wait(&tfull[buf], bphase, 104)) { ok = false; break; }
+        if (!mbar_wait_warp(&tfull[buf], bphase, 104)) { ok = false; break; }
         tc_fence_after();
         const int64_t col0 = (int64_t)n * BN;
         if constexpr (EPI == EPI_PROBS || EPI == EPI_STORE_BF16) {

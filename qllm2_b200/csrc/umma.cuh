@@ -91,6 +91,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int co
   atomicCAS(&g_device_error, 0, code);
   return false;
 }
+// When a wait gives up, by its time limit or because of the error word, some lanes of a warp may and others may not: what a warp does
+// together afterwards (a tcgen05 load in a loop that the give-up leaves, a branch with a __syncwarp) must not depend on a lane's own
+// answer.  The answers of a warp's waits, agreed on:
+__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok); }
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int code, uint64_t limit_ns = WAIT_NS) {
+  return warp_agrees(mbar_wait(bar, parity, code, limit_ns));
+}
 
 // Kernels read the error word once at their start (one thread, into shared memory) and return without touching
 // their outputs when an earlier launch has recorded a failure: results stay as the caller left them until the
