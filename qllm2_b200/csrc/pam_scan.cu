@@ -326,7 +326,7 @@ static int scan_walk(ScanParams& p, const qpam_scan_args* a, const ScanLayout& L
     // (sums and carry of split sequences: they start with empty hands when every sequence is walked)
     const auto kern = tcs::k_tc_walk<K, false>;
     if ((rc = set_smem(kern, tcs::walk_smem(K, false)))) return rc;
-    launch_after(kern, 3 * ctas / 2, 256, tcs::walk_smem(K, false), st, maps, p);
+    launch_after(kern, ctas, 256, tcs::walk_smem(K, false), st, maps, p);
     QPAM_LAUNCH_CHECK("k_tc_walk<sums>");
     launch_after(tcs::k_walk_carry, 4 * ctas, 256, 0, st, p);
     QPAM_LAUNCH_CHECK("k_walk_carry");
@@ -349,7 +349,7 @@ static int scan_forward_only(const qpam_scan_args* a, const ScanLayout& L, cudaS
     p.pool = dest->pool; p.slot_ids = dest->slot_ids; p.n_slots = dest->n_slots;
     p.pool_bf16 = dest->dtype == QPAM_BF16; p.pool_L = dest->L; p.pool_layer = dest->layer;
   }
-  const int ctas = 2 * sm_count();
+  const int ctas = tcs::WALK_PER_SM * sm_count();
   if (walk_pays(a, ctas)) {
     switch (a->K) {
       case 1: return scan_walk<1>(p, a, L, st, token_major, ctas);

@@ -29,6 +29,14 @@ namespace tcs {
 // (four states have room for one)
 __host__ __device__ constexpr int walk_sets(int K) { return K <= 3 ? 2 : 1; }
 __host__ __device__ constexpr size_t walk_smem(int K, bool out) { return 1024 + (out ? 3 : 2) * 32768 + (size_t)walk_sets(K) * K * TC * 20 + 512; }
+// Both forms are built and launched for two CTAs per SM.  (The sums were built for three, of which two fitted for K = 2 and 3: 80 registers,
+// 196 bytes spilled, eight columns at a time, and a third of the grid began behind the others' last jobs.  60000 tokens among 32 short
+// sequences, 12 heads, all of them split: one state 501 -> 460 us, three 948 -> 865.)
+constexpr int WALK_PER_SM = 2;
+constexpr size_t SM_SMEM = 228 * 1024, CTA_RESERVED = 1024;
+template <int K>
+constexpr bool walk_fits() { return WALK_PER_SM * (walk_smem(K, true) + CTA_RESERVED) <= SM_SMEM && WALK_PER_SM * (walk_smem(K, false) + CTA_RESERVED) <= SM_SMEM; }
+static_assert(walk_fits<1>() && walk_fits<2>() && walk_fits<3>() && walk_fits<KMAX>(), "CTAs per SM of the walking kernels");
 // ScanParams::ticket: [0] next job of the outputs  [1] of the sums  [2] entries of the list  [3] how many of them, at its end, are chunks of split
 // sequences: the jobs of the sums  [4] any sequence for the carry  [5] sequences of more chunks are split
 enum { WT_OUT = 0, WT_SUM = 1, WT_JOBS = 2, WT_SPLIT_JOBS = 3, WT_CARRY = 4, WT_SPLIT = 5 };
@@ -72,7 +80,7 @@ __device__ __forceinline__ void walk_request_entry(WalkJob* smem_dst, const Walk
 }
 
 template <int K, bool OUT>
-__global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_constant__ ChunkMaps maps, ScanParams p) {
+__global__ void __launch_bounds__(256, WALK_PER_SM) k_tc_walk(const __grid_constant__ ChunkMaps maps, ScanParams p) {
   using namespace umma;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -267,7 +275,7 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
       }
     }
     if (sums) {
-      constexpr int G = OUT ? 16 : 8;          // columns at a time (three CTAs per SM have fewer registers)
+      constexpr int G = 16;                    // columns at a time
       float pv[G];                             // that many of the thread's elements of the entering state, ahead of their use
       // the sums of state k leave the accumulators: S' = g S + U, U as in k_tc_chunk_outer
       auto sums_out = [&](int k) {
@@ -303,8 +311,7 @@ __global__ void __launch_bounds__(256, OUT ? 2 : 3) k_tc_walk(const __grid_const
         for (int hh = 0; hh < 32 / G; ++hh) {
           float d1[G], d2[G];
           const uint32_t col = (uint32_t)(hf * 32 + hh * G);
-          if constexpr (OUT) tmem_ld16x2(from + col, d1, from + 64 + col, d2);
-          else tmem_ld8x2(from + col, d1, from + 64 + col, d2);
+          tmem_ld16x2(from + col, d1, from + 64 + col, d2);
 #pragma unroll
           for (int i = 0; i < G; i += 2) {      // two columns an instruction
             const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, d2[i], 1), __shfl_xor_sync(0xffffffffu, d2[i + 1], 1));
@@ -649,7 +656,7 @@ __global__ void __launch_bounds__(1024) k_walk_plan(ScanParams p, int32_t* __res
   __syncthreads();
   if (tid == 0) {
     p.ticket[WT_OUT] = (unsigned int)ctas;               // (behind the grids of the two: a CTA's first job is its index)
-    p.ticket[WT_SUM] = (unsigned int)(3 * ctas / 2);
+    p.ticket[WT_SUM] = (unsigned int)ctas;
     p.ticket[WT_JOBS] = (unsigned int)(walked + split_s);
     p.ticket[WT_SPLIT_JOBS] = (unsigned int)split_s;
     p.ticket[WT_CARRY] = (unsigned int)special_s;
