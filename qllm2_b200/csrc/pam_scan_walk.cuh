@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256, WALK_PER_SM) k_tc_walk(const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_trigger();
+  if (OUT) pdl_trigger();                    // (the sums: by their end, see k_walk_carry)
   const uint32_t tmem = *tmem_slot;
   // thread 0: the entry to walk after the current one, drawn when the current one's last chunk is the next step (equally long
   // sequences: every gridDim.x-th entry)
@@ -668,6 +668,8 @@ __global__ void __launch_bounds__(1024) k_walk_plan(ScanParams p, int32_t* __res
 // S_c+1 = g_c S_c + U_c, in place over the slots, as k_state_scan; the last state goes to its destination only, the first is written
 // where it is given.  CTAs take (sequence, head and state, eighth of a state) in turn: a grid with one for each took 78 us to find
 // out that there was nothing to do (256 short prompts, 36 heads and states).
+// Where sums are formed before it, it is called by their end, not by their start: a long chain is only a few CTAs, and called early these
+// piled up on the SMs that were free first (60000 tokens among 32 short sequences, 12 heads, one state: 547 -> 453 us; three, 893 -> 838).
 __global__ void __launch_bounds__(256) k_walk_carry(ScanParams p) {
   pdl_wait();
   pdl_trigger();
