@@ -224,10 +224,11 @@ static ScanParams one_state_view(const ScanParams& pK, const qpam_scan_args* a, 
   return p;
 }
 
-// chunk-local state sums on tensor cores; done: every sequence is one chunk from zero, its sums are its final state
-static int tc_sums(ScanParams& p, const ScanLayout& L, const qpam_scan_args* a, cudaStream_t st, bool& done) {
+// chunk-local state sums on tensor cores; done: every sequence is one chunk from zero, its sums are its final state.  `only`: no backward
+// will read the states
+static int tc_sums(ScanParams& p, const ScanLayout& L, const qpam_scan_args* a, cudaStream_t st, bool only, bool& done) {
   done = a->cu_seqlens == nullptr && L.nc_uniform == 1 && p.s0 == nullptr;
-  p.single = done;
+  p.finish = p.s0 != nullptr ? FIN_NONE : only ? FIN_ONLY : done ? FIN_ALSO : FIN_NONE;
   if (L.grid_chunks == 0) return QPAM_OK;
   CUtensorMap mk, mv;
   const int64_t rows = (int64_t)a->B * a->H * a->T;
@@ -239,7 +240,7 @@ static int tc_sums(ScanParams& p, const ScanLayout& L, const qpam_scan_args* a, 
     launch_after(tcs::k_tc_chunk_outerK<false>, dim3(L.grid_chunks, a->H), 256, tcs::OUTERK_SMEM, st, mk, mv, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outerK");
   } else {
-    const auto kern = done ? tcs::k_tc_chunk_outer<false, true> : tcs::k_tc_chunk_outer<false>;
+    const auto kern = p.finish != FIN_NONE ? tcs::k_tc_chunk_outer<false, true> : tcs::k_tc_chunk_outer<false>;
     if ((rc = set_smem(kern, tcs::OUTER_SMEM))) return rc;
     launch_after(kern, dim3(L.grid_chunks, a->H, a->K), 256, tcs::OUTER_SMEM, st, mk, mv, p);
     QPAM_LAUNCH_CHECK("k_tc_chunk_outer<state>");
@@ -251,7 +252,7 @@ static int tc_sums(ScanParams& p, const ScanLayout& L, const qpam_scan_args* a, 
 static int tc_states(const ScanParams& p0, const ScanLayout& L, const qpam_scan_args* a, cudaStream_t st) {
   ScanParams p = p0;
   bool done;
-  const int rc = tc_sums(p, L, a, st, done);
+  const int rc = tc_sums(p, L, a, st, false, done);
   if (rc || done) return rc;
   launch_ordinary(k_state_scan<false>, dim3(a->S, a->H * a->K, (64 * 64 / 2 + 255) / 256), 256, 0, st, p, 64);
   QPAM_LAUNCH_CHECK("k_state_scan<fwd>");
@@ -363,7 +364,7 @@ static int scan_forward_only(const qpam_scan_args* a, const ScanLayout& L, cudaS
     QPAM_LAUNCH_CHECK("k_chunk_prefix");
   }
   bool done;
-  int rc = tc_sums(p, L, a, st, done);
+  int rc = tc_sums(p, L, a, st, true, done);
   if (rc) return rc;
   if (!done) {
     const int64_t items = (int64_t)a->S * a->H * a->K * (64 * 64 / 2 / 256);

@@ -95,6 +95,11 @@ struct __align__(16) WalkJob {
   int32_t seq, c0, c1, nc, a, e, slot0, pool_slot;
 };
 
+// ScanParams::finish.  FIN_ALSO: beside the slot, which a backward may read (every sequence is one chunk: there is no carry).  FIN_ONLY:
+// in the slot's place, and the carry passes such sequences by (20 prompts of 60..128 tokens, 12 heads, one state: carry 5.8 -> 2.9 us, the
+// call 35.8 -> 33.8; three states 13.2 -> 6.9 and 56 -> 52).
+enum { FIN_NONE = 0, FIN_ALSO = 1, FIN_ONLY = 2 };
+
 struct ScanParams {
   const void *q, *k, *v, *dy;
   const float* gamma;   // [K,B,H,T]
@@ -116,7 +121,7 @@ struct ScanParams {
   float q_scale, eps;
   int32_t y_token_major;   // tensor-core forward kernels only: y laid out [B,T,H,d,2] instead of [B,H,T,d,2]
   int32_t dy_tokens;       // K-state tensor-core backward only: the same for dy
-  int32_t single;          // every sequence is one chunk from zero: the chunk sums write s_final as well
+  int32_t finish;          // chunk sums of a one-chunk sequence from zero are its final state: FIN_ALSO / FIN_ONLY that one is written
   // Tensor-core forward of which no backward will read the states: the final states may go to slots of a state pool
   // [n_slots,L,K,H,D,D,2] instead of s_final.
   int32_t pool_bf16, pool_L, pool_layer;

@@ -116,8 +116,8 @@ constexpr size_t OUTER_SMEM = 1024 + 32768 + 32768 + 1536;
 // The two token tiles (k and v, or q and dy; maps of [B*H*T rows][128 bf16], boxes of 64 x 128, 128-byte swizzle)
 // arrive by TMA; the value tile lands in the region its planes are then built in: every thread reads its pieces, a
 // barrier, and the planes are written over them.
-// SINGLE: every sequence is one chunk from zero, its sums are its final state as well.
-template <bool DSTATE, bool SINGLE = false>
+// FINISH: as p.finish says; the sequences start from zero.
+template <bool DSTATE, bool FINISH = false>
 __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant__ CUtensorMap mk,
                                                            const __grid_constant__ CUtensorMap mv, ScanParams p) {
   using namespace umma;
@@ -210,14 +210,14 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outer(const __grid_constant
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + cc * 32, d1);
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + 64 + cc * 32, d2);
     const bool even = (lane & 1) == 0;
-    if (SINGLE) {
+    if (FINISH && L.nc == 1) {                  // CTA-uniform
       FinalDest fin;
       fin.init(p, L.seq, pool_slot_of(p, L.seq), kst, h);
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
         const float o = __shfl_xor_sync(0xffffffffu, d2[i], 1);
         d1[i] = even ? d1[i] + o : o - d1[i];
-        if (ok) dst[(size_t)(cc * 32 + i) * 128] = d1[i];
+        if (ok && p.finish == FIN_ALSO) dst[(size_t)(cc * 32 + i) * 128] = d1[i];
       }
       fin.store(p, cc * 32 * 128 + q4 * 32 + lane, d1, even, ok);
     } else {
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
       // Re U = D1[2j] + D2[2j+1], Im U = D2[2j] - D1[2j+1]: lane n' = 2j+c holds column i, state[i][j][c] at i*128 + n'
       float2* slot = DSTATE ? p.dstates + state_base(p, k - 1, h, L.slot0 + L.c, TD) : p.states + state_base(p, k - 1, h, L.slot0 + L.c + 1, TD);
       float* dst = reinterpret_cast<float*>(slot) + (q4 * 32 + lane);
-      const bool final_now = !DSTATE && p.single;
+      const bool final_now = !DSTATE && p.finish != FIN_NONE && L.nc == 1;
 #pragma unroll 1
       for (int hh = 0; hh < 4; ++hh) {          // 8 columns at a time
         float d1[8], d2[8];
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(256, 3) k_tc_chunk_outerK(const __grid_constan
           for (int i = 0; i < 8; ++i) {
             const float o = __shfl_xor_sync(0xffffffffu, d2[i], 1);
             d1[i] = even ? d1[i] + o : o - d1[i];
-            if (ok) dst[(size_t)(col + i) * 128] = d1[i];
+            if (ok && p.finish == FIN_ALSO) dst[(size_t)(col + i) * 128] = d1[i];
           }
           fin.store(p, (int)col * 128 + q4 * 32 + lane, d1, even, ok);
         } else {

@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(256) k_walk_carry(ScanParams p) {
     const int64_t sh = it / (n4 / 256);
     const int seq = (int)(sh / (p.H * p.K)), hk = (int)(sh - (int64_t)seq * (p.H * p.K)), k = hk / p.H, h = hk - k * p.H;
     const int nc = packed ? p.geom.chunk_prefix[seq + 1] - p.geom.chunk_prefix[seq] : p.geom.nc_uniform;
-    if (nc > 0 && nc <= above) continue;
+    if ((nc > 0 && nc <= above) || (nc == 1 && p.finish == FIN_ONLY)) continue;
     const int64_t slot0 = packed ? (int64_t)p.geom.chunk_prefix[seq] + seq : (int64_t)seq * (nc + 1);
     const int e4 = (int)(it % (n4 / 256)) * 256 + threadIdx.x;
     float4* st = reinterpret_cast<float4*>(p.states + state_base(p, k, h, slot0, TD)) + e4;

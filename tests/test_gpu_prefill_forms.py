@@ -1,0 +1,70 @@
+"""Which form a packed forward-only scan takes, told by what it leaves in its workspace: short batches that finish one-chunk sequences in
+the chunk sums, batches that walk, and the sequences that are split among them; with the states that each form puts into pool slots."""
+import ctypes as C
+
+import pytest
+import torch
+
+from qllm2_b200 import _lib, ops
+from qllm2_b200._lib import check, dtype_code, ptr, stream_ptr
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+LONGEST_BIN = 1023
+
+
+def _inputs(K, H, lens, with_s0=False):
+    g = torch.Generator(device=DEV).manual_seed(K * 11 + H)
+    T = sum(lens)
+    q, k, v = ((torch.randn(1, H, T, 64, 2, device=DEV, generator=g) * 0.1).bfloat16() for _ in range(3))
+    gamma = torch.sigmoid(torch.randn(K, 1, H, T, device=DEV, generator=g) + 2)
+    coef = torch.randn(K, 1, H, T, 2, device=DEV, generator=g) if K > 1 else None
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).int()
+    s0 = torch.randn(K, len(lens), H, 64, 64, 2, device=DEV, generator=g) if with_s0 else None
+    return q, k, v, gamma, coef, cu, s0
+
+
+def _align(n):
+    return (n + 255) // 256 * 256
+
+
+def _prefill(K, H, lens, x, dtype):
+    """y, the pool, the workspace's state slots as bytes, and the six counters of a call that walks."""
+    q, k, v, gamma, coef, cu, s0 = x
+    n, T = len(lens), sum(lens)
+    pool = torch.full((n + 1, 1, K, H, 64, 64, 2), 7.0, device=DEV, dtype=dtype)
+    slots = torch.arange(n, device=DEV, dtype=torch.int32)
+    y = torch.empty(1, T, H * 64, 2, device=DEV, dtype=torch.bfloat16)
+    a = _lib.ScanArgs()
+    a.q, a.k, a.v, a.gamma, a.coef, a.s0, a.cu_seqlens, a.y = (ptr(t) for t in (q, k, v, gamma, coef, s0, cu, y))
+    a.B, a.H, a.T, a.d, a.K, a.S, a.chunk, a.io_dtype, a.q_scale, a.gamma_eps = 1, H, T, 64, K, n, 64, 1, 0.125, 1e-6
+    total = _lib.lib().qpam_scan_workspace_bytes(C.byref(a), 0)
+    ws = torch.full((total,), 0x5A, dtype=torch.uint8, device=DEV)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    n0 = _lib.launch_count()
+    check(_lib.lib().qpam_scan_prefill(C.byref(a), pool.data_ptr(), dtype_code(dtype), n + 1, 1, 0, ptr(slots), stream_ptr()), "qpam_scan_prefill")
+    launches = _lib.launch_count() - n0
+    first, state_slots = _align(4 * (n + 1)), K * H * (T // 128 + 2 * n)      # chunk prefix | state slots | decays | counters and list
+    jobs = first + _align(state_slots * 64 * 64 * 8) + _align(state_slots * 4)
+    states = ws[first:first + state_slots * 64 * 64 * 8]
+    assert bool((pool[n] == 7).all()) and _lib.device_status() == 0
+    return y, pool[:n, 0], states, ws[jobs:jobs + 24].view(torch.int32).tolist(), launches
+
+
+def _training_form(K, x):
+    q, k, v, gamma, coef, cu, s0 = x
+    return ops.pam_scan(q, k, v, gamma.clone().requires_grad_(True), coef=coef, cu_seqlens=cu, s0=s0, token_major=True)
+
+
+@pytest.mark.parametrize("K", [1, 3])
+@pytest.mark.parametrize("with_s0", [False, True])
+def test_one_chunk_sequences_finish_in_the_sums(K, with_s0):
+    """Few short prompts: their sums go to the pool and nowhere else; a state before them takes the carry."""
+    lens, H = [1, 128, 64, 0, 127], 2
+    x = _inputs(K, H, lens, with_s0)
+    y_ref, s_ref = _training_form(K, x)
+    for dtype in (torch.float32, torch.bfloat16):
+        y, pool, states, _, launches = _prefill(K, H, lens, x, dtype)
+        assert launches == 4
+        assert torch.equal(y, y_ref.detach()) and torch.equal(pool, s_ref.detach().transpose(0, 1).to(dtype))
+        assert bool((states == 0x5A).all()) != with_s0
