@@ -17,7 +17,8 @@
 // A sequence that is long beside what the batch gives every SM to do would leave the chip to a few CTAs.  Its chunks are taken in the
 // three passes instead (`split`): sums of every chunk by this kernel without its output part, the carry, and one-chunk jobs whose state
 // is read from its slot, at the end of the same list.  Both ways give the same bits (the carry is the same sequence of fused multiply-adds).
-// (One sequence of 60000 tokens among 32 short ones: 715 us, 586 with kernels of their own for the three passes.)
+// (One sequence of 60000 tokens among 32 short ones, 12 heads, as it is split now / as kernels of their own for the three passes: one state
+// 438 / 450 us, three 821 / 839.)
 // Batches with few sequences and heads take the three passes as kernels of their own (scan_forward_only, pam_scan.cu).
 #pragma once
 #include "pam_scan_tc3.cuh"
@@ -40,15 +41,21 @@ static_assert(walk_fits<1>() && walk_fits<2>() && walk_fits<3>() && walk_fits<KM
 // ScanParams::ticket: [0] next job of the outputs  [1] of the sums  [2] entries of the list  [3] how many of them, at its end, are chunks of split
 // sequences: the jobs of the sums  [4] any sequence for the carry  [5] sequences of more chunks are split
 enum { WT_OUT = 0, WT_SUM = 1, WT_JOBS = 2, WT_SPLIT_JOBS = 3, WT_CARRY = 4, WT_SPLIT = 5 };
-constexpr int WALK_MIN = 2;            // a sequence of at most so many chunks is always walked
+constexpr int WALK_BINS = 1024;        // sequences are counted by their chunks, the longest (1023 and more) together
 
-// Sequences of more chunks than three times what the call has for each CTA that the chip holds are split.  (A chunk costs more in the
-// three passes, and a long sequence, begun first, ends with the others.  32 documents of 512..16384 tokens, 16 heads, split above 1.25 /
-// 1.5 / 2 / 3 times the mean: 1225 / 1296 / 1278 / 1247 us; 18 of 300..16000: 1181 / 1262 / 1080 / 1041; 22 of 400..9000, 12 heads: 658 /
-// 648 / 586 / 572.)
-__host__ __device__ inline int walk_split_above(int64_t chunk_heads, int ctas) {
-  const int64_t m = 3 * ((chunk_heads + ctas - 1) / ctas);
-  return (int)(m < WALK_MIN ? WALK_MIN : m > 0x3fffffff ? 0x3fffffff : m);
+// What a call takes if sequences of more than a given number of chunks are split, in the time of a chunk that is walked with two CTAs on
+// every SM (10 us with one state, 26 with three).  walked, split: chunks of either kind; longest_walked, longest_split: chunks of the
+// longest sequence of either kind; per_cta: heads over the CTAs that the chip holds.  The walks end with the longest of them (0.6 a chunk
+// once it has its SM for itself) or with their share of the work; a split chunk costs 0.7 for its sums before anything else begins and 0.8
+// for its output, a link of the carry 0.01, the two launches 1.
+// The call takes the cheapest split.  Measured over 28 batches and 1..4 states against the best of splitting above 0 / 0.6 / .. / 1.5 / 2 / 3
+// times a CTA's share / never, it is within 2 % of the best on average and within 10 % everywhere; a fixed factor is not: of 48 prompts
+// around 300 tokens (log-normal, deviation 1.5), 12 heads, one state, a split above 1 / 1.5 / 3 times the share takes 213 / 230 / 350 us, of
+// 28 of 512..16384 1200 / 986 / 1130.
+__host__ __device__ inline float walk_cost(float walked, float split, float longest_walked, float longest_split, float per_cta) {
+  const float shared = per_cta * (walked + split);
+  const float t = fmaxf(0.6f * longest_walked + 0.4f * fminf(longest_walked, shared), per_cta * (walked + 0.8f * split));
+  return split > 0.f ? t + 1.f + 0.7f * per_cta * split + 0.01f * longest_split : t;
 }
 
 struct WalkStep {
@@ -549,19 +556,21 @@ __global__ void __launch_bounds__(256, WALK_PER_SM) k_tc_walk(const __grid_const
   }
 }
 
-// The list of a packed call, one CTA: chunks before every sequence (descriptor checked as in k_chunk_prefix_checked), sequences to
-// walk by falling length (counted by length, 1023 and more together), then the chunks of the split ones.
+// The list of a packed call, one CTA: chunks before every sequence (descriptor checked as in k_chunk_prefix_checked), which sequences are
+// split (walk_cost), those to walk by falling length, then the chunks of the split ones.
 __global__ void __launch_bounds__(1024) k_walk_plan(ScanParams p, int32_t* __restrict__ prefix, WalkJob* __restrict__ jobs, int ctas, int bad_code) {
-  __shared__ int hist[1024];
+  __shared__ int hist[WALK_BINS];            // sequences by their chunks, then where those of a length begin in the list
   __shared__ int wsum[32];
-  __shared__ int carry_s, bad_s, special_s, split_s;
+  __shared__ int carry_s, bad_s, special_s, split_s, longest_s;
+  __shared__ unsigned long long best_s;
   pdl_wait();
   pdl_trigger();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, S = p.geom.S;
   const int32_t* cu = p.geom.cu_seqlens;
   hist[tid] = 0;
   if (tid == 0) {
-    carry_s = special_s = split_s = 0;
+    carry_s = special_s = split_s = longest_s = 0;
+    best_s = ~0ull;
     bad_s = cu[0] != 0;
     prefix[0] = 0;
   }
@@ -622,24 +631,42 @@ __global__ void __launch_bounds__(1024) k_walk_plan(ScanParams p, int32_t* __res
     }
     return;
   }
-  const int above = walk_split_above((int64_t)C * p.H, ctas);
   auto chunks_of = [&](int s) { return s < 1024 ? (end - first + TC - 1) / TC : prefix[s + 1] - prefix[s]; };
+  int longest = 0;
   for (int s = tid; s < S; s += 1024) {
     const int nc = chunks_of(s);
-    if (nc > 0 && nc <= above) atomicAdd(&hist[min(nc, 1023)], 1);
+    longest = max(longest, nc);
+    if (nc > 0) atomicAdd(&hist[min(nc, WALK_BINS - 1)], 1);
     else special_s = 1;
   }
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  if (lane == 0 && longest > 0) atomicMax(&longest_s, longest);
   __syncthreads();
+  // thread x looks at a split above x chunks, where there are sequences of so many (x = 0: every one is split)
+  longest = longest_s;
+  const int count = hist[tid];
+  int below_last;
+  const int upto = scan(tid < WALK_BINS - 1 ? count * tid : 0, below_last);
+  if (count > 0 || tid == 0) {
+    const bool all = tid == WALK_BINS - 1;
+    const int walked_chunks = all ? C : upto;
+    const float t = walk_cost((float)walked_chunks, (float)(C - walked_chunks), (float)(all ? longest : tid), (float)longest, (float)p.H / (float)ctas);
+    atomicMin(&best_s, (unsigned long long)__float_as_uint(t) << 32 | (unsigned int)(WALK_BINS - 1 - tid));      // (of equals the one that splits less)
+  }
+  __syncthreads();
+  const int best = WALK_BINS - 1 - (int)(unsigned int)best_s, above = best == WALK_BINS - 1 ? 0x3fffffff : best;
   int walked;
-  const int mine = hist[1023 - tid], inc = scan(mine, walked);      // longest first
-  hist[1023 - tid] = inc - mine;
+  const int bin = WALK_BINS - 1 - tid, mine = bin <= above ? hist[bin] : 0, inc = scan(mine, walked);      // longest first
+  hist[bin] = inc - mine;
   __syncthreads();
   for (int s = tid; s < S; s += 1024) {
     const int nc = chunks_of(s);
-    if (nc > 0 && nc <= above)
-      jobs[atomicAdd(&hist[min(nc, 1023)], 1)] = s < 1024 ? WalkJob{s, 0, nc, nc, first, end, before_me + s, slot}
-                                                          : WalkJob{s, 0, nc, nc, cu[s], cu[s + 1], prefix[s] + s, pool_slot_of(p, s)};
+    if (nc > above) special_s = 1;
+    else if (nc > 0)
+      jobs[atomicAdd(&hist[min(nc, WALK_BINS - 1)], 1)] = s < 1024 ? WalkJob{s, 0, nc, nc, first, end, before_me + s, slot}
+                                                                  : WalkJob{s, 0, nc, nc, cu[s], cu[s + 1], prefix[s] + s, pool_slot_of(p, s)};
   }
+  __syncthreads();
   if (special_s)
     for (int x = tid; x < C; x += 1024) {
       int lo = 0, hi = S;                    // the last s with prefix[s] <= x

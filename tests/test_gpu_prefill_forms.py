@@ -68,3 +68,41 @@ def test_one_chunk_sequences_finish_in_the_sums(K, with_s0):
         assert launches == 4
         assert torch.equal(y, y_ref.detach()) and torch.equal(pool, s_ref.detach().transpose(0, 1).to(dtype))
         assert bool((states == 0x5A).all()) != with_s0
+
+
+@pytest.mark.parametrize("K", [1, 3])
+def test_a_long_sequence_beside_short_ones_keeps_three_passes_for_itself(K):
+    """The final state of a split sequence in its pool slot, behind a list of walked ones."""
+    lens, H = [5, 3000, 0] + [100 + i for i in range(26)], 12
+    x = _inputs(K, H, lens)
+    y_ref, s_ref = _training_form(K, x)
+    for dtype in (torch.float32, torch.bfloat16):
+        y, pool, _, (_, _, jobs, split_jobs, carry, above), launches = _prefill(K, H, lens, x, dtype)
+        assert launches == 4 and carry == 1 and 1 <= above < 24 and jobs - split_jobs == 27 and split_jobs == 24
+        assert torch.equal(y, y_ref.detach()) and torch.equal(pool, s_ref.detach().transpose(0, 1).to(dtype))
+
+
+def _cost(chunks, above, H, ctas):
+    walked, split = [c for c in chunks if c <= above], [c for c in chunks if c > above]
+    per = H / ctas
+    t = max(0.6 * max(walked, default=0) + 0.4 * min(max(walked, default=0), per * sum(chunks)), per * (sum(walked) + 0.8 * sum(split)))
+    return t + 1 + 0.7 * per * sum(split) + 0.01 * max(split) if split else t
+
+
+@pytest.mark.parametrize("K,H,lens", [
+    (1, 16, [128 * (1 + i) for i in range(24)]),                                                   # evenly spread: all of them walk
+    (1, 12, [3000] * 8 + [60] * 24),                                                               # a quarter is long
+    (3, 6, [int(60 * 1.09 ** i) for i in range(56)]),                                              # a tail of ever longer ones
+    (2, 12, [9000, 700] + [90] * 30),
+    (1, 1, [int(1 + (37 * i) % 128) for i in range(1500)] + [128 * 1100, 128 * 1023, 128 * 40]),   # past the last bin, more than threads
+])
+def test_the_cheapest_split(K, H, lens):
+    x = _inputs(K, H, lens)
+    ctas = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert len(lens) * H * 37 >= ctas * 40 or (K == 1 and len(lens) * H > ctas)
+    _, _, _, (_, _, jobs, split_jobs, carry, above), _ = _prefill(K, H, lens, x, torch.bfloat16)
+    chunks = [-(-n // 128) for n in lens]
+    split = [c for c in chunks if c > above]
+    assert split_jobs == sum(split) and jobs == sum(split) + len(chunks) - len(split) and carry == (1 if split else 0)
+    best = min(_cost(chunks, min(c, LONGEST_BIN - 1) if c < LONGEST_BIN else 1 << 29, H, ctas) for c in [0] + chunks)
+    assert _cost(chunks, above, H, ctas) <= best * (1 + 1e-5)      # (fp32 on the device: 24 bits)
