@@ -693,8 +693,9 @@ __global__ void __launch_bounds__(1024) k_walk_plan(ScanParams p, int32_t* __res
 
 // The carry of split sequences (of all of them where no list has been made), and the final states of empty ones:
 // S_c+1 = g_c S_c + U_c, in place over the slots, as k_state_scan; the last state goes to its destination only, the first is written
-// where it is given.  CTAs take (sequence, head and state, eighth of a state) in turn: a grid with one for each took 78 us to find
-// out that there was nothing to do (256 short prompts, 36 heads and states).
+// where it is given, and no slot at all where no output will read them (a call for final states alone).  CTAs take (sequence, head and
+// state, eighth of a state) in turn: a grid with one for each took 78 us to find out that there was nothing to do (256 short prompts, 36
+// heads and states).
 // Where sums are formed before it, it is called by their end, not by their start: a long chain is only a few CTAs, and called early these
 // piled up on the SMs that were free first (60000 tokens among 32 short sequences, 12 heads, one state: 547 -> 453 us; three, 893 -> 838).
 __global__ void __launch_bounds__(256) k_walk_carry(ScanParams p) {
@@ -703,6 +704,7 @@ __global__ void __launch_bounds__(256) k_walk_carry(ScanParams p) {
   const bool packed = p.geom.cu_seqlens != nullptr;
   if (p.ticket != nullptr && p.ticket[WT_CARRY] == 0u) return;
   const int above = p.ticket != nullptr ? (int)p.ticket[WT_SPLIT] : 0;
+  const bool keep = p.y != nullptr;
   constexpr int n4 = TD * TD / 2, UN = 4;
   const int64_t items = (int64_t)p.geom.S * p.H * p.K * (n4 / 256);
   for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
@@ -716,7 +718,7 @@ __global__ void __launch_bounds__(256) k_walk_carry(ScanParams p) {
     const float* dec = p.chunk_decay + ((size_t)k * p.H + h) * p.nslots + slot0;
     const size_t ext = ((((size_t)k * p.geom.S + seq) * p.H + h) * (size_t)(TD * TD)) / 2 + e4;
     float4 cur = p.s0 != nullptr ? reinterpret_cast<const float4*>(p.s0)[ext] : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.s0 != nullptr) st[0] = cur;
+    if (p.s0 != nullptr && keep) st[0] = cur;
     for (int c = 0; c < nc; c += UN) {
       float4 u[UN];
       float g[UN];
@@ -737,7 +739,7 @@ __global__ void __launch_bounds__(256) k_walk_carry(ScanParams p) {
           cur.y = fmaf(g[i], cur.y, u[i].y);
           cur.z = fmaf(g[i], cur.z, u[i].z);
           cur.w = fmaf(g[i], cur.w, u[i].w);
-          if (c + i + 1 < nc) st[(size_t)(c + i + 1) * n4] = cur;
+          if (keep && c + i + 1 < nc) st[(size_t)(c + i + 1) * n4] = cur;
         }
     }
     if (p.s_final != nullptr) reinterpret_cast<float4*>(p.s_final)[ext] = cur;

@@ -106,3 +106,27 @@ def test_the_cheapest_split(K, H, lens):
     assert split_jobs == sum(split) and jobs == sum(split) + len(chunks) - len(split) and carry == (1 if split else 0)
     best = min(_cost(chunks, min(c, LONGEST_BIN - 1) if c < LONGEST_BIN else 1 << 29, H, ctas) for c in [0] + chunks)
     assert _cost(chunks, above, H, ctas) <= best * (1 + 1e-5)      # (fp32 on the device: 24 bits)
+
+
+@pytest.mark.parametrize("K", [1, 3])
+@pytest.mark.parametrize("with_s0", [False, True])
+def test_final_states_alone(K, with_s0):
+    """A call for final states: the carry passes over the chunk sums and writes none of the slots that only an output would read."""
+    lens, H = [300, 1, 0, 128, 513], 2
+    q, k, v, gamma, coef, cu, s0 = x = _inputs(K, H, lens, with_s0)
+    n, T = len(lens), sum(lens)
+    s = torch.empty(K, n, H, 64, 64, 2, device=DEV)
+    a = _lib.ScanArgs()
+    a.q, a.k, a.v, a.gamma, a.s0, a.cu_seqlens, a.s_final = (ptr(t) for t in (q, k, v, gamma, s0, cu, s))
+    a.B, a.H, a.T, a.d, a.K, a.S, a.chunk, a.io_dtype, a.q_scale, a.gamma_eps = 1, H, T, 64, K, n, 64, 1, 0.125, 1e-6
+    ws = torch.full((_lib.lib().qpam_scan_workspace_bytes(C.byref(a), 0),), 0x5A, dtype=torch.uint8, device=DEV)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    check(_lib.lib().qpam_scan_fwd(C.byref(a), stream_ptr()), "qpam_scan_fwd")
+    assert torch.equal(s, _training_form(K, x)[1].detach()) and torch.equal(s, ops.pam_scan_states(k, v, gamma, s0=s0, cu_seqlens=cu))
+    slots = T // 128 + 2 * n
+    first = _align(4 * (n + 1))
+    states = ws[first:first + K * H * slots * 64 * 64 * 8].view(K, H, slots, 64 * 64 * 8)
+    at = 0
+    for length in lens:                                    # a sequence's first slot is the state before it
+        assert bool((states[:, :, at] == 0x5A).all())
+        at += -(-length // 128) + 1
