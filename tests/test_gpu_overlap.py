@@ -230,3 +230,32 @@ def test_statistics_of_a_head():
     want = linear_ce_stats(h, w, t)
     for _ in range(3):
         assert linear_ce_stats(h * 1.0, w * 1.0, t) == want
+
+
+@pytest.mark.parametrize("lengths,H,K,s0", [
+    ([130, 1, 384, 257, 64, 300] * 6, 12, 1, False),      # walked, the list's kernel before them
+    ([130, 1, 384, 257, 64, 300] * 6, 12, 3, False),
+    ([130, 1, 384, 257, 64, 300] * 6, 12, 2, True),
+    ([130, 1, 6000, 257, 64, 300] + [50, 100] * 15, 12, 1, True),      # one of them split: sums, carry and outputs behind the list
+    ([130, 1, 6000, 257, 64, 300] + [50, 100] * 15, 12, 3, False),
+    ([100, 1, 128, 64], 4, 1, False),                     # finished by the chunk sums
+    ([100, 1, 128, 64], 4, 3, False),
+])
+def test_packed_prefill_that_walks(lengths, H, K, s0):
+    x = _scan_inputs(1, H, sum(lengths), K, coef=K > 1, s0=len(lengths) if s0 else 0)
+    x["cu"] = _lengths(lengths)
+    _check(x, lambda x: ops.pam_scan_tokens(x["q"], x["k"], x["v"], x["gamma"], coef=x.get("coef"), s0=x.get("s0"), cu_seqlens=x["cu"]))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,top_k,top_p", [(1, 50, 0.9), (64, 0, 0.9), (200, 0, 0.0)])
+def test_sampler(n, top_k, top_p, dtype):
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x = dict(logits=(torch.randn(n, 5008, device=DEV, generator=g) * 3).to(dtype), u=torch.rand(n, device=DEV, generator=g),
+             history=torch.randint(0, 5003, (n, 40), device=DEV, generator=g), hist_len=torch.randint(0, 41, (n,), device=DEV, generator=g).int())
+
+    def call(x):
+        got = ops.sample_logits(x["logits"][:, :5003], x["u"], temperature=0.8, top_k=top_k, top_p=top_p, repetition_penalty=1.1, history=x["history"],
+                                hist_len=x["hist_len"], return_stats=True)
+        return [t for t in got] if isinstance(got, (tuple, list)) else [*got.values()] if isinstance(got, dict) else [got]
+    _check(x, call)
