@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(1024) k_walk_plan(ScanParams p, int32_t* __res
   if (bad_s) {
     for (int s = tid; s <= S; s += 1024) prefix[s] = 0;
     if (tid == 0) {
-      for (int i = 0; i < 6; ++i) p.ticket[i] = 0u;
+      for (int i = 0; i < 6; ++i) p.ticket[i] = i == WT_CARRY ? 1u : 0u;      // (every sequence is empty now: its final state is its first)
       umma::record_device_error(bad_code);
     }
     return;

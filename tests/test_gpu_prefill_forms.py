@@ -130,3 +130,27 @@ def test_final_states_alone(K, with_s0):
     for length in lens:                                    # a sequence's first slot is the state before it
         assert bool((states[:, :, at] == 0x5A).all())
         at += -(-length // 128) + 1
+
+
+@pytest.mark.parametrize("K", [1, 3])
+@pytest.mark.parametrize("with_s0", [False, True])
+def test_refused_descriptor(K, with_s0):
+    """Lengths that decrease, in a batch that would walk: the status word says so, no token is touched, and every sequence counts as
+    empty, as in the batches that do not walk."""
+    lens, H = [60] * 30, 12
+    q, k, v, gamma, coef, cu, s0 = _inputs(K, H, lens, with_s0)
+    cu[5] = cu[4] - 1
+    n, T = len(lens), sum(lens)
+    y, s = torch.full((1, T, H * 64, 2), 3.0, device=DEV, dtype=torch.bfloat16), torch.full((K, n, H, 64, 64, 2), 3.0, device=DEV)
+    a = _lib.ScanArgs()
+    a.q, a.k, a.v, a.gamma, a.coef, a.s0, a.cu_seqlens, a.y, a.s_final = (ptr(t) for t in (q, k, v, gamma, coef, s0, cu, y, s))
+    a.B, a.H, a.T, a.d, a.K, a.S, a.chunk, a.io_dtype, a.q_scale, a.gamma_eps = 1, H, T, 64, K, n, 64, 1, 0.125, 1e-6
+    ws = torch.empty(_lib.lib().qpam_scan_workspace_bytes(C.byref(a), 0), dtype=torch.uint8, device=DEV)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    assert _lib.device_status() == 0
+    try:
+        check(_lib.lib().qpam_scan_fwd_tokens(C.byref(a), stream_ptr()), "qpam_scan_fwd_tokens")
+        torch.cuda.synchronize()
+    finally:
+        assert _lib.device_status(clear=True) == 301
+    assert bool((y == 3).all()) and torch.equal(s, torch.zeros_like(s) if s0 is None else s0)
