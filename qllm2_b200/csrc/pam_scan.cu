@@ -297,11 +297,12 @@ static int tc_outputs(const ScanParams& p, const ScanLayout& L, const qpam_scan_
 
 // Whether a forward-only call walks (pam_scan_walk.cuh): it wants more sequences and heads than the chip holds CTAs, with several states
 // a twelfth more; lengths of packed sequences are on the device, so here by their number, and the device splits the ones that are long
-// beside the rest (walk_cost).  Three passes -> walking, us, packed lengths anywhere between the two given: one state, 26 x 30..128
-// tokens, 12 heads 40 -> 39; 26 x 30..300, 12 heads 54 -> 47; 19 x 108..649, 16 heads 77 -> 74; 32 x 512..16384, 16 heads 1858 -> 1300;
-// three states, 48 x 32..1024, 12 heads 362 -> 275; 40 x 60..128, 12 heads 83 -> 57; just below the line 19 x 108..649, 16 heads 138 -> 143
-// (four states 171 -> 182), 26 x 30..300, 12 heads 97 -> 80.  (24 x 17..1482, 12 heads, three states, in the passes: 236; walked, with a
-// split above three times the mean, 270.)  Of equal lengths the last round of CTAs has to be four fifths full.
+// beside the rest (walk_cost).  Three passes -> walking, us, single calls with L2 flushed before them, packed lengths anywhere between the
+// two given (longer ones at the head of pam_scan_walk.cuh): one state, 26 x 30..128 tokens, 12 heads 40 -> 39; 26 x 30..300, 12 heads 54 ->
+// 47; 19 x 108..649, 16 heads 77 -> 74; 26 x 44..11396, 12 heads 1003 -> 762; three states, 40 x 60..128, 12 heads 83 -> 57; 64 x 64..4096,
+// 6 heads 826 -> 747; just below the line 19 x 108..649, 16 heads 138 -> 143 (four states 171 -> 182), 26 x 30..300, 12 heads 97 -> 80.
+// (24 x 17..1482, 12 heads, three states, in the passes: 236; walked, with a split above three times the mean, 270.)  Of equal lengths
+// the last round of CTAs has to be four fifths full.
 static bool walk_pays(const qpam_scan_args* a, int ctas) {
   const int64_t units = (int64_t)a->S * a->H;
   if (a->y == nullptr || a->T == 0) return false;

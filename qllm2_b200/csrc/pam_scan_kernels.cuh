@@ -96,8 +96,8 @@ struct __align__(16) WalkJob {
 };
 
 // ScanParams::finish.  FIN_ALSO: beside the slot, which a backward may read (every sequence is one chunk: there is no carry).  FIN_ONLY:
-// in the slot's place, and the carry passes such sequences by (20 prompts of 60..128 tokens, 12 heads, one state: carry 5.8 -> 2.9 us, the
-// call 35.8 -> 33.8; three states 13.2 -> 6.9 and 56 -> 52).
+// in the slot's place, and the carry passes such sequences by (20 prompts of 60..128 tokens, 12 heads: one state, carry 5.8 -> 3.0 us;
+// three, carry 13.2 -> 5.0, the call 56 -> 50).
 enum { FIN_NONE = 0, FIN_ALSO = 1, FIN_ONLY = 2 };
 
 struct ScanParams {

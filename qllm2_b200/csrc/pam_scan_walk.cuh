@@ -6,7 +6,7 @@
 // 18 k clocks for one state and 45 k for three with two CTAs per SM (three: a quarter of it the sums' way out of the accumulators, 42 %
 // of the issue slots taken).  The form it replaces, chunk sums -> carry -> outputs as three passes over all chunks, ran three such chains, read
 // k and v twice and moved every chunk's state (K * 32 KB for 48-96 KB of tokens and output) through HBM two to four times.  32 documents
-// of 512..16384 tokens, 16 heads, one state: 1842 -> 1299 us; 48 chat prompts of 32..1024, 12 heads, three states: 324 -> 236; 256 prompts
+// of 512..16384 tokens, 16 heads, one state: 1853 -> 1295 us; 48 chat prompts of 32..1024, 12 heads, three states: 327 -> 239; 256 prompts
 // of 70, 12 heads, three states: 339 -> 203.
 // Code is kept short (rolled loops, 16 columns at a time): the first version, written out, was 216 KB for three states, spilled, and
 // missed the instruction cache; its score epilogue took 8.8 k clocks instead of 1.9 k.
@@ -17,7 +17,7 @@
 // A sequence that is long beside what the batch gives every SM to do would leave the chip to a few CTAs.  Its chunks are taken in the
 // three passes instead (`split`): sums of every chunk by this kernel without its output part, the carry, and one-chunk jobs whose state
 // is read from its slot, at the end of the same list.  Both ways give the same bits (the carry is the same sequence of fused multiply-adds).
-// (One sequence of 60000 tokens among 32 short ones, 12 heads, as it is split now / as kernels of their own for the three passes: one state
+// (One sequence of 60000 tokens among 32 of 100..300, 12 heads, as it is split / as kernels of their own for the three passes: one state
 // 438 / 450 us, three 821 / 839.)
 // Batches with few sequences and heads take the three passes as kernels of their own (scan_forward_only, pam_scan.cu).
 #pragma once
@@ -48,7 +48,7 @@ constexpr int WALK_BINS = 1024;        // sequences are counted by their chunks,
 // longest sequence of either kind; per_cta: heads over the CTAs that the chip holds.  The walks end with the longest of them (0.6 a chunk
 // once it has its SM for itself) or with their share of the work; a split chunk costs 0.7 for its sums before anything else begins and 0.8
 // for its output, a link of the carry 0.01, the two launches 1.
-// The call takes the cheapest split.  Measured over 28 batches and 1..4 states against the best of splitting above 0 / 0.6 / .. / 1.5 / 2 / 3
+// The call takes the cheapest split.  Measured over 32 batches and 1..4 states against the best of splitting above 0 / 0.6 / .. / 1.5 / 2 / 3
 // times a CTA's share / never, it is within 2 % of the best on average and within 10 % everywhere; a fixed factor is not: of 48 prompts
 // around 300 tokens (log-normal, deviation 1.5), 12 heads, one state, a split above 1 / 1.5 / 3 times the share takes 213 / 230 / 350 us, of
 // 28 of 512..16384 1200 / 986 / 1130.
