@@ -300,7 +300,7 @@ static int tc_outputs(const ScanParams& p, const ScanLayout& L, const qpam_scan_
 // beside the rest (walk_cost).  Three passes -> walking, us, single calls with L2 flushed before them, packed lengths anywhere between the
 // two given (longer ones at the head of pam_scan_walk.cuh): one state, 26 x 30..128 tokens, 12 heads 40 -> 39; 26 x 30..300, 12 heads 54 ->
 // 47; 19 x 108..649, 16 heads 77 -> 74; 26 x 44..11396, 12 heads 1003 -> 762; three states, 40 x 60..128, 12 heads 83 -> 57; 64 x 64..4096,
-// 6 heads 826 -> 747; just below the line 19 x 108..649, 16 heads 138 -> 143 (four states 171 -> 182), 26 x 30..300, 12 heads 97 -> 80.
+// 6 heads 826 -> 747; just below the line 19 x 108..649, 16 heads 138 -> 143 (four states 171 -> 182), 26 x 30..300, 12 heads 85 -> 80.
 // (24 x 17..1482, 12 heads, three states, in the passes: 236; walked, with a split above three times the mean, 270.)  Of equal lengths
 // the last round of CTAs has to be four fifths full.
 static bool walk_pays(const qpam_scan_args* a, int ctas) {
